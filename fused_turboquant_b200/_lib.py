@@ -74,6 +74,29 @@ def load() -> ctypes.CDLL:
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The compiled host path (csrc/ftq_torch.cpp), bound to this library's entry points."""
+    global _native
+    if _native is None:
+        lib = load()
+        import torch  # noqa: F401  (the module links against torch's libraries)
+        try:
+            from . import _native as ext
+        except ImportError as e:
+            raise RuntimeError(
+                "fused_turboquant_b200/_native.so is missing or does not load: build it with "
+                f"`python -m fused_turboquant_b200.build` ({e})") from e
+        from . import kernels
+
+        ext.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in SIGNATURES},
+                 check, kernels.get_workspace, kernels._workspaces)
+        _native = ext
+    return _native
+
+
 def is_available() -> bool:
     """True when the CUDA library is built and a CUDA device is visible."""
     import torch

@@ -24,6 +24,9 @@ LIB_PATH = os.path.join(PKG_DIR, "libftq_b200.so")
 # never issued and the poll limit is small), so that a bounded wait runs out and the give-up path
 # (NaN rows, status word, the context stays usable) executes.  Never loaded by the package.
 TEST_LIB_PATH = os.path.join(PKG_DIR, "libftq_b200_waittest.so")
+# The tensor-level host path (csrc/ftq_torch.cpp): a CPython module compiled with the host compiler
+# against torch's headers; it gets the C ABI's addresses at import and links nothing of ours.
+NATIVE_PATH = os.path.join(PKG_DIR, "_native.so")
 TEST_UNIT = ("ftq_attn_inst.cu", "attn_d128_waittest",
              ["-DFTQ_D=128", "-DFTQ_ONLY_BITS=4", "-DFTQ_TEST_WAIT_EXPIRY"])
 
@@ -49,6 +52,27 @@ def _nvcc() -> str:
         if cand and os.path.exists(cand):
             return cand
     raise RuntimeError("nvcc not found: cannot build libftq_b200.so")
+
+
+def _build_native() -> None:
+    import sysconfig
+
+    import torch
+    src = os.path.join(CSRC, "ftq_torch.cpp")
+    if not _unit_stale("ftq_torch.cpp", NATIVE_PATH):
+        return
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(root, "include"),
+           "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I" + os.path.join(cuda, "include"), src, "-o", NATIVE_PATH,
+           "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10",
+           "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {src}:\n{r.stdout}\n{r.stderr}")
 
 
 def _sources_mtime() -> float:
@@ -86,7 +110,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     """Compile and link the library (and the wait-expiry test library) if missing or older than
     the sources."""
     if not force and all(os.path.exists(l) and os.path.getmtime(l) >= _sources_mtime()
-                         for l in (LIB_PATH, TEST_LIB_PATH)):
+                         for l in (LIB_PATH, TEST_LIB_PATH, NATIVE_PATH)):
         return LIB_PATH
     nvcc = _nvcc()
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -106,7 +130,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return obj
 
     with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
+        native = ex.submit(_build_native)
         objs = list(ex.map(compile_one, UNITS + [TEST_UNIT]))
+        native.result()
     test_obj = objs.pop()
     for lib, members in ((LIB_PATH, objs),
                          (TEST_LIB_PATH, [test_obj if o.endswith("attn_d128.o") else o for o in objs])):

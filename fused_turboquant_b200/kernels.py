@@ -94,61 +94,20 @@ def get_workspace(device: torch.device, nbytes: int) -> torch.Tensor:
 def fused_encode(x: torch.Tensor, signs, boundaries, bits: int):
     """RHT + norm + Lloyd-Max + pack in one launch -> (packed u8 (..., pd), norms f16 (...))."""
     _require_cuda(x, "x")
-    if x.dtype not in _DT:
-        x = x.float()
-    d = x.shape[-1]
-    lead = x.shape[:-1]
-    pd = packed_dim(d, bits)
-    x2 = x.contiguous().view(-1, d)
-    n = x2.shape[0]
-    packed = torch.empty((n, pd), dtype=torch.uint8, device=x.device)
-    norms = torch.empty((n,), dtype=torch.float16, device=x.device)
-    with torch.cuda.device(x.device):
-        rc = _lib.load().ftq_encode(_ptr(x2), _DT[x2.dtype], n, d, d, bits,
-                                    _lib.fptr(_host_table(signs)),
-                                    _lib.fptr(_host_table(boundaries)), _ptr(packed), _ptr(norms),
-                                    _stream(x.device))
-    _lib.check(rc, "ftq_encode")
-    return packed.view(*lead, pd), norms.view(lead)
+    return _lib.native().encode(x, signs, boundaries, bits)
 
 
 def fused_decode(packed_indices: torch.Tensor, norms: torch.Tensor, levels, signs, bits: int,
                  original_dim: int) -> torch.Tensor:
     """unpack + dequant + denorm + inverse RHT -> fp32 (..., original_dim)."""
     _require_cuda(packed_indices, "packed_indices")
-    d = original_dim
-    pd = packed_dim(d, bits)
-    p2 = packed_indices.contiguous().view(-1, pd)
-    nflat = norms.contiguous().view(-1)
-    if nflat.dtype not in (torch.float16, torch.float32):
-        nflat = nflat.float()
-    n = nflat.shape[0]
-    out = torch.empty((n, d), dtype=torch.float32, device=packed_indices.device)
-    with torch.cuda.device(out.device):
-        rc = _lib.load().ftq_decode_dense(_ptr(p2), _ptr(nflat), _DT[nflat.dtype], n, d, bits,
-                                          _lib.fptr(_host_table(levels)),
-                                          _lib.fptr(_host_table(signs)), _ptr(out),
-                                          _stream(out.device))
-    _lib.check(rc, "ftq_decode_dense")
-    return out.view(*norms.shape, d)
+    return _lib.native().decode_dense(packed_indices, norms, levels, signs, bits, original_dim)
 
 
 def rht(x: torch.Tensor, signs, inverse: bool = False) -> torch.Tensor:
     """Randomized Hadamard transform (forward or inverse), same shape and dtype out."""
     _require_cuda(x, "x")
-    orig_dtype = x.dtype
-    if x.dtype not in _DT:
-        x = x.float()
-    d = x.shape[-1]
-    x2 = x.contiguous().view(-1, d)
-    y = torch.empty_like(x2)
-    with torch.cuda.device(x.device):
-        rc = _lib.load().ftq_rht(_ptr(x2), _ptr(y), _DT[x2.dtype], x2.shape[0], d,
-                                 _lib.fptr(_host_table(signs)), int(bool(inverse)),
-                                 _stream(x.device))
-    _lib.check(rc, "ftq_rht")
-    y = y.view(x.shape)
-    return y if y.dtype == orig_dtype else y.to(orig_dtype)
+    return _lib.native().rht(x, signs, inverse)
 
 
 # --------------------------------------------------------------- attention
@@ -189,28 +148,9 @@ def flash_decode_compressed(q_rotated: torch.Tensor, k_indices: torch.Tensor,
     ``out_dtype`` says otherwise).  ``seq_lens`` is honoured.
     """
     _require_cuda(q_rotated, "q_rotated")
-    B, Hq, q_len, d = q_rotated.shape
-    if q_len != 1:
-        raise ValueError("flash_decode_compressed handles one query token per sequence")
-    _, Hkv, S, _ = k_indices.shape
-    q = q_rotated.contiguous()
-    if q.dtype not in _DT:
-        q = q.float()
-    out_dtype = out_dtype or torch.float32
-    out = torch.empty((B, Hq, 1, d), dtype=out_dtype, device=q.device)
-    ki, vi = k_indices.contiguous(), v_indices.contiguous()
-    kn, vn = k_norms.contiguous().half(), v_norms.contiguous().half()
-    sl = None if seq_lens is None else seq_lens.to(device=q.device, dtype=torch.int32).contiguous()
-    need = workspace_bytes(B, Hq, Hkv, d, S, 1)
-    ws = workspace if workspace is not None else get_workspace(q.device, need)
-    with torch.cuda.device(q.device):
-        rc = _lib.load().ftq_flash_decode(
-            _ptr(q), _DT[q.dtype], int(bool(q_is_rotated)), _ptr(ki), _ptr(kn), _ptr(vi), _ptr(vn),
-            _lib.fptr(_host_table(k_centroids)), _lib.fptr(_host_table(v_centroids)),
-            _lib.fptr(_host_table(signs)), float(scale), bits_k, bits_v, _ptr(sl), B, Hq, Hkv, S,
-            d, _ptr(out), _DT[out_dtype], _ptr(ws), ws.numel(), _stream(q.device))
-    _lib.check(rc, "ftq_flash_decode")
-    return out
+    return _lib.native().flash_decode(q_rotated, k_indices, k_norms, v_indices, v_norms, k_centroids,
+                                      v_centroids, signs, scale, bits_k, bits_v, seq_lens,
+                                      q_is_rotated, out_dtype, workspace)
 
 
 # names the reference's modules export

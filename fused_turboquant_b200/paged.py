@@ -73,24 +73,10 @@ class PagedKVPool:
         slot_mapping: [n_tokens] int64, slot = block * 16 + offset; negative = skip.
         """
         _require_cuda(key, "key")
-        if key.dtype not in _DT:
-            key, value = key.float(), value.float()
-        key, value = key.contiguous(), value.contiguous().to(key.dtype)
-        sm = slot_mapping.to(device=key.device, dtype=torch.int64).contiguous()
-        if layer is None:
-            L, n_tokens = key.shape[0], key.shape[1]
-            pool = self.pool
-        else:
-            L, n_tokens = 1, key.shape[0]
-            pool = self.pool[layer]
-        D, H = self.head_dim, self.num_kv_heads
-        with torch.cuda.device(key.device), _trace.nvtx("ftq.store"):
-            rc = _lib.load().ftq_paged_store(
-                _ptr(key), _ptr(value), _DT[key.dtype], n_tokens, H, D, H * D, D, self.key_bits,
-                self.value_bits, _lib.fptr(self.signs), _lib.fptr(self.bounds_k),
-                _lib.fptr(self.bounds_v), _ptr(pool), self.num_blocks, _ptr(sm), L,
-                n_tokens * H * D, self.layer_stride, _stream(key.device))
-        _lib.check(rc, "ftq_paged_store")
+        if _trace.ENABLED:
+            with _trace.nvtx("ftq.store"):
+                return _lib.native().paged_store(self, key, value, slot_mapping, layer)
+        _lib.native().paged_store(self, key, value, slot_mapping, layer)
 
     def workspace_bytes(self, batch: int, num_q_heads: int, max_seq_len: int,
                         n_layers: int = 1) -> int:
@@ -108,32 +94,12 @@ class PagedKVPool:
         No host synchronisation; graph-capturable when out/workspace are passed in.
         """
         _require_cuda(q, "q")
-        if q.dtype not in _DT:
-            q = q.float()
-        q = q.contiguous()
-        if layer is None:
-            L, B, Hq, D = q.shape
-            pool = self.pool
-        else:
-            L = 1
-            B, Hq, D = q.shape
-            pool = self.pool[layer]
-        scale = (D ** -0.5) if scale is None else scale
-        out = torch.empty_like(q) if out is None else out
-        bt = block_table.to(device=q.device, dtype=torch.int32).contiguous()
-        sl = seq_lens.to(device=q.device, dtype=torch.int32).contiguous()
-        need = self.workspace_bytes(B, Hq, max_seq_len, L)
-        ws = workspace if workspace is not None else kernels.get_workspace(q.device, need)
-        with torch.cuda.device(q.device), _trace.nvtx("ftq.decode"):
-            rc = _lib.load().ftq_paged_decode_attn(
-                _ptr(q), _DT[q.dtype], _ptr(out), _DT[out.dtype], _ptr(pool), self.num_blocks,
-                self.layer_stride, L, _ptr(bt), bt.shape[1], _ptr(sl), int(max_seq_len), B, Hq,
-                self.num_kv_heads, D, self.key_bits, self.value_bits, _lib.fptr(self.levels_k),
-                _lib.fptr(self.levels_v), _lib.fptr(self.signs), float(scale), _ptr(ws),
-                ws.numel(), _stream(q.device))
-        _lib.check(rc, "ftq_paged_decode_attn")
-        self._last_decode = (ws, B, Hq, int(max_seq_len), L, q.device)
-        return out
+        if _trace.ENABLED:
+            with _trace.nvtx("ftq.decode"):
+                return _lib.native().paged_decode(self, q, block_table, seq_lens, max_seq_len, scale,
+                                                  layer, out, workspace)
+        return _lib.native().paged_decode(self, q, block_table, seq_lens, max_seq_len, scale, layer,
+                                          out, workspace)
 
     def decode_status(self) -> int:
         """Status bits of this pool's last ``decode_attention`` call (0: nothing to report;

@@ -21,7 +21,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib
-from .kernels import _DT, _host_table, _ptr, _require_cuda, _stream, rht
+from .kernels import _DT, _require_cuda, rht
 
 
 @dataclass(frozen=True)
@@ -113,20 +113,6 @@ def _key_bits(tq_config) -> int:
     return kb
 
 
-def _table_ptr(table, fp8: bool):
-    # FP8 keys have no key codebook: whatever table the caller holds (the reference sizes it for the
-    # values then) is not read
-    return None if fp8 else _lib.fptr(_host_table(table))
-
-
-def _cache_strides(kv_cache: torch.Tensor) -> tuple[int, int, int]:
-    if kv_cache.dtype != torch.uint8:
-        kv_cache = kv_cache.view(torch.uint8)
-    if kv_cache.dim() != 4 or kv_cache.stride(3) != 1:
-        raise ValueError("kv_cache must be [num_blocks, block_size, num_kv_heads, slot] with a dense last dim")
-    return kv_cache.stride(0), kv_cache.stride(1), kv_cache.stride(2)
-
-
 def launch_store(key: torch.Tensor, value: torch.Tensor, kv_cache: torch.Tensor,
                  slot_mapping: torch.Tensor, midpoints, tq_config: TurboQuantSlotConfig,
                  head_size: int | None = None, v_rotate: bool = False,
@@ -146,41 +132,22 @@ def launch_store(key: torch.Tensor, value: torch.Tensor, kv_cache: torch.Tensor,
     layered = key.dim() == 4
     if layered != (kv_cache.dim() == 5):
         raise ValueError("key/value [L, N, Hkv, D] go with a cache [L, num_blocks, block_size, Hkv, slot]")
-    n_layers = key.shape[0] if layered else 1
-    if layered and kv_cache.shape[0] != n_layers:
-        raise ValueError("key/value and kv_cache disagree on the number of layers")
-    n, hkv, d = key.shape[-3:]
+    d = key.shape[-1]
     if head_size is not None and head_size != d:
         raise ValueError(f"head_size {head_size} does not match key.shape[-1] {d}")
     if d != tq_config.head_dim:
         raise ValueError(f"key head size {d} does not match the config ({tq_config.head_dim})")
     if value.shape != key.shape:
         raise ValueError("key and value must have the same shape")
-    if key.dtype not in _DT:
-        key = key.float()
-    if value.dtype != key.dtype:
-        value = value.to(key.dtype)
-    rotate_in_kernel = bool(v_rotate) and tq_config.value_quant_bits != 8
-    if v_rotate and not rotate_in_kernel:
+    vb = tq_config.value_quant_bits
+    if v_rotate and vb == 8:
         # 8-bit values: rotate here (the kernel fuses the rotation for 1..4-bit values only)
-        value = rht(value.float().contiguous(), None).to(key.dtype)
-    if key.stride(-1) != 1 or value.stride() != key.stride():
-        key, value = key.contiguous(), value.contiguous()
-    if kv_cache.dtype != torch.uint8:
-        kv_cache = kv_cache.view(torch.uint8)
-    sb, sp, sh = _cache_strides(kv_cache[0] if layered else kv_cache)
-    if kv_cache.shape[-1] < tq_config.slot_size:
-        raise ValueError(f"kv_cache slots of {kv_cache.shape[-1]} bytes are smaller than {tq_config.slot_size}")
-    sm = slot_mapping.to(device=key.device, dtype=torch.int64).contiguous()
-    kb = _key_bits(tq_config)
-    with torch.cuda.device(key.device):
-        rc = _lib.load().ftq_tq_store_layers(
-            _ptr(key), _ptr(value), _DT[key.dtype], n, hkv, d, key.stride(-3), key.stride(-2),
-            kb, tq_config.value_quant_bits, int(rotate_in_kernel),
-            int(bool(v_lloyd_max)), _table_ptr(midpoints, kb == 8), _ptr(kv_cache), sb, sp, sh,
-            kv_cache.shape[-3], _ptr(sm), n_layers, key.stride(0) if layered else 0,
-            kv_cache.stride(0) if layered else 0, kv_cache.shape[-4], _stream(key.device))
-    _lib.check(rc, "ftq_tq_store_layers")
+        if key.dtype not in _DT:
+            key = key.float()
+        value = rht(value.to(key.dtype).float().contiguous(), None).to(key.dtype)
+        v_rotate = False
+    _lib.native().tq_store(key, value, kv_cache, slot_mapping, midpoints, _key_bits(tq_config), vb,
+                           v_rotate, v_lloyd_max)
 
 
 def decode_attention(query: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Tensor,
@@ -208,66 +175,10 @@ def decode_attention(query: torch.Tensor, kv_cache: torch.Tensor, block_table: t
     """
     _require_cuda(query, "query")
     _require_cuda(kv_cache, "kv_cache")
-    if kv_cache.dtype != torch.uint8:
-        kv_cache = kv_cache.view(torch.uint8)
-    n_layers, layer_stride, lead = 1, 0, ()
-    if query.dim() == 4:
-        if kv_cache.dim() != 5 or kv_cache.shape[0] != query.shape[0]:
-            raise ValueError("a [L, B, Hq, D] query needs a [L, num_blocks, block_size, Hkv, slot] cache")
-        n_layers, lead = query.shape[0], (query.shape[0],)
-        layer_stride = kv_cache.stride(0)
-        query = query.reshape(-1, *query.shape[2:])
-        kv_cache = kv_cache[0]
-    B, hq, d = query.shape
-    B //= n_layers
-    rows = B * n_layers
-    if d != tq_config.head_dim:
-        raise ValueError(f"query head size {d} does not match the config ({tq_config.head_dim})")
-    if query.dtype not in _DT:
-        query = query.float()
-    query = query.contiguous()
-    sb, sp, sh = _cache_strides(kv_cache)
-    hkv = kv_cache.shape[2]
-    dev = query.device
-    bt = block_table.to(device=dev, dtype=torch.int32).contiguous()
-    sl = seq_lens.to(device=dev, dtype=torch.int32).contiguous()
-    ks = None if kv_start_offset is None else kv_start_offset.to(device=dev, dtype=torch.int32).contiguous()
-    if mid_o is None:
-        mid_o = torch.empty((rows, hq, num_kv_splits, d + 1), dtype=torch.float32, device=dev)
-    elif mid_o.numel() != rows * hq * num_kv_splits * (d + 1) or mid_o.dtype != torch.float32 or \
-            not mid_o.is_contiguous():
-        raise ValueError("mid_o must be a contiguous fp32 [(L,) B, Hq, num_kv_splits, D+1] tensor")
-    odt = out_dtype or query.dtype
-    if output is None:
-        output = torch.empty(lead + (B, hq, d), dtype=odt, device=dev)
-    elif output.shape != lead + (B, hq, d) or not output.is_contiguous() or output.dtype not in _DT:
-        raise ValueError("output must be a contiguous [(L,) B, Hq, D] tensor of a supported dtype")
-    if lse is not None and (lse.dtype != torch.float32 or not lse.is_contiguous() or
-                            lse.numel() != rows * hq or lse.device != dev):
-        raise ValueError("lse must be a contiguous fp32 [(L,) B, Hq] tensor on the query's device")
-    if (prefix_output is None) != (prefix_lse is None):
-        raise ValueError("prefix_output and prefix_lse go together")
-    if prefix_output is not None:
-        _require_cuda(prefix_output, "prefix_output")
-        if prefix_output.shape != lead + (B, hq, d) or prefix_lse.shape != lead + (B, hq):
-            raise ValueError("prefix_output must be [(L,) B, Hq, D] and prefix_lse [(L,) B, Hq]")
-        if prefix_output.dtype not in _DT:
-            prefix_output = prefix_output.float()
-        prefix_output = prefix_output.contiguous()
-        prefix_lse = prefix_lse.to(device=dev, dtype=torch.float32).contiguous()
-    kb = _key_bits(tq_config)
-    with torch.cuda.device(dev):
-        rc = _lib.load().ftq_tq_decode_layers(
-            _ptr(query), _DT[query.dtype], B, hq, hkv, d, _ptr(kv_cache), sb, sp, sh,
-            kv_cache.shape[1], _ptr(bt), bt.shape[1], _ptr(sl), _ptr(ks),
-            kb, tq_config.value_quant_bits, int(tq_config.norm_correction),
-            int(v_rotate), int(bool(v_lloyd_max)), _table_ptr(centroids, kb == 8), float(scale),
-            num_kv_splits,
-            _ptr(mid_o), _ptr(output), _DT[output.dtype], _ptr(lse), _ptr(prefix_output),
-            _DT[prefix_output.dtype] if prefix_output is not None else 0, _ptr(prefix_lse),
-            n_layers, layer_stride, kv_cache.shape[0], _stream(dev))
-    _lib.check(rc, "ftq_tq_decode_layers")
-    return output
+    return _lib.native().tq_decode(
+        query, kv_cache, block_table, seq_lens, kv_start_offset, centroids, _key_bits(tq_config),
+        tq_config.value_quant_bits, tq_config.norm_correction, v_rotate, v_lloyd_max, scale,
+        num_kv_splits, mid_o, output, out_dtype, lse, prefix_output, prefix_lse, tq_config.head_dim)
 
 
 def continuation_attention(query: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Tensor,

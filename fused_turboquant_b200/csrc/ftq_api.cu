@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cfloat>
+#include <climits>
 #include <atomic>
 #include <cstdint>
 #include <cstring>
@@ -60,74 +61,55 @@ int pack_levels(const float* levels_host, int bits, ftq::Codebook* out) {
 
 float rsqrt_dim(int d) { return static_cast<float>(std::pow(static_cast<double>(d), -0.5)); }
 
-int make_encode_tables(int d, int bits, const float* signs_host, const float* boundaries_host,
-                       ftq::EncodeTables* tab) {
+// One tensor's share of an encode call (source and sink are the caller's).
+int make_encode_job(int bits, const float* boundaries_host, ftq::EncodeJob* job) {
     if (!boundaries_host) return fail(FTQ_ERR_INVALID, "boundaries table is NULL");
     const int nb = (1 << bits) + 1;
     for (int i = 1; i < nb; i++)
         if (!(boundaries_host[i - 1] <= boundaries_host[i]))
             return fail(FTQ_ERR_INVALID, "boundaries must be ascending");
-    memset(tab, 0, sizeof(*tab));
-    const int rc = pack_signs(signs_host, d, &tab->signs);
-    if (rc) return rc;
+    job->bits = bits;
     // code = clamp(#{b < x} - 1, 0, 2^bits - 1) = #{interior boundaries < x}
-    for (int j = 1; j < nb - 1; j++) tab->bounds[j - 1] = boundaries_host[j];
-    tab->rsqrt_d = rsqrt_dim(d);
+    for (int j = 1; j < nb - 1; j++) job->bounds[j - 1] = boundaries_host[j];
     return FTQ_OK;
 }
 
-// Table quantizer of the throughput encode kernel: x is mapped to a cell of [-1, 1] by
-// the same single-precision FMA the kernel uses; usable when no cell holds two boundaries
+// The throughput kernel maps x to a cell of [-1, 1]: usable when no cell holds two boundaries
 // and no boundary is so close to zero that a 2^100 scaling cannot separate it from x.
-uint32_t quant_cell(float x) {
-    const float v = fmaf(x, ftq::kCellScale, ftq::kCellMagic);
-    uint32_t bits;
-    memcpy(&bits, &v, 4);
-    return (bits & 0xFF80u) >> 7;
-}
-
-bool make_encode2_tables(const ftq::EncodeTables& tab, int bits, ftq::Encode2Tables* out) {
-    const int nb = (1 << bits) - 1;  // interior boundaries, ascending
-    out->signs = tab.signs;
-    out->rsqrt_d = tab.rsqrt_d;
-    for (int c = 0; c < ftq::kQuantCells; c++) {
-        out->cells[c].neg_thr_scaled = -FLT_MAX;
-        out->cells[c].base = 0.f;
-    }
+bool table_quantizer_takes(const ftq::EncodeJob& job) {
+    const int nb = (1 << job.bits) - 1;  // interior boundaries, ascending
     uint32_t prev = 0xffffffffu;
     for (int j = 0; j < nb; j++) {
-        const float b = tab.bounds[j];
-        if (!(b > -1.0f && b < 1.0f) || (j > 0 && !(tab.bounds[j - 1] < b))) return false;
+        const float b = job.bounds[j];
+        if (!(b > -1.0f && b < 1.0f) || (j > 0 && !(job.bounds[j - 1] < b))) return false;
         if (std::fabs(b) < 1e-20f) return false;
-        const uint32_t c = quant_cell(b);
+        const uint32_t c = ftq::quant_cell(b);
         if (c == prev || c >= static_cast<uint32_t>(ftq::kQuantCells)) return false;
         prev = c;
-        out->cells[c].neg_thr_scaled = -b * ftq::kStepScale;
-        for (uint32_t k = c + 1; k < static_cast<uint32_t>(ftq::kQuantCells); k++)
-            out->cells[k].base += 1.f;
     }
     return true;
 }
 
-cudaError_t dispatch_encode(int d, int bits, int dtype, const ftq::EncodeSource& src_in,
-                            const ftq::EncodeSink& sink_in, const ftq::EncodeTables& tab,
-                            int64_t n_vec, int n_layers, cudaStream_t st) {
+cudaError_t dispatch_encode(int d, int dtype, ftq::EncodeJobs& jobs, int n_jobs, int n_layers,
+                            cudaStream_t st) {
     // vector indices are split into (token, head) with 31-bit arithmetic in the kernels (the
     // public entry points reject larger counts, which no resident input can reach)
-    if (n_vec >= (1ll << 31) || src_in.n_inner <= 0 || sink_in.Hkv <= 0) return cudaErrorInvalidValue;
-    ftq::EncodeSource src = src_in;
-    ftq::EncodeSink sink = sink_in;
-    src.div_inner = ftq::make_fastdiv(static_cast<uint32_t>(src.n_inner));
-    sink.div_hkv = ftq::make_fastdiv(static_cast<uint32_t>(sink.Hkv));
-    // A handful of vectors (a decode step) is launch-bound either way: the simple kernel
-    // skips the table set-up.  Bulk encodes take the throughput kernel when the codebook allows.
-    ftq::Encode2Tables tab2;
-    const bool fast = n_vec >= 2048 && make_encode2_tables(tab, bits, &tab2);
-    const ftq::Encode2Tables* t2 = fast ? &tab2 : nullptr;
+    if (jobs.n_vec >= (1ll << 31)) return cudaErrorInvalidValue;
+    jobs.rsqrt_d = rsqrt_dim(d);
+    // A handful of vectors (a decode step) is latency-bound: the warp-per-vector kernel.  From 2048
+    // on the SMs have enough vectors for the throughput kernel's octets, when the codebooks allow.
+    bool bulk = jobs.n_vec >= 2048;
+    for (int i = 0; i < n_jobs; i++) {
+        ftq::EncodeJob& j = jobs.job[i];
+        if (j.src.n_inner <= 0 || j.sink.Hkv <= 0) return cudaErrorInvalidValue;
+        j.src.div_inner = ftq::make_fastdiv(static_cast<uint32_t>(j.src.n_inner));
+        j.sink.div_hkv = ftq::make_fastdiv(static_cast<uint32_t>(j.sink.Hkv));
+        bulk = bulk && table_quantizer_takes(j);
+    }
     switch (d) {
-        case 64: return ftq::launch_encode_d64(bits, dtype, src, sink, tab, t2, n_vec, n_layers, st);
-        case 128: return ftq::launch_encode_d128(bits, dtype, src, sink, tab, t2, n_vec, n_layers, st);
-        case 256: return ftq::launch_encode_d256(bits, dtype, src, sink, tab, t2, n_vec, n_layers, st);
+        case 64: return ftq::launch_encode_d64(dtype, jobs, n_jobs, bulk, n_layers, st);
+        case 128: return ftq::launch_encode_d128(dtype, jobs, n_jobs, bulk, n_layers, st);
+        case 256: return ftq::launch_encode_d256(dtype, jobs, n_jobs, bulk, n_layers, st);
     }
     return cudaErrorInvalidValue;
 }
@@ -313,6 +295,37 @@ ftq::SplitPlan make_split(const ChunkPlan& pl, int64_t units, bool tensor_core) 
     return sp;
 }
 
+// Plans are pure functions of a few sizes, and finding one walks up to a thousand candidates (up
+// to 60 us on the host for a 128k context): each thread keeps the last ones it made.  Contexts are
+// rounded up to the planners' granularity of 64 tokens first, so that a decode loop, whose
+// context grows by one token a step, makes a new plan every 64 steps only.
+struct PlanKey {
+    int kind, B, Hq, Hkv, d, seq, layers, slots;
+    bool operator==(const PlanKey& o) const {
+        return kind == o.kind && B == o.B && Hq == o.Hq && Hkv == o.Hkv && d == o.d && seq == o.seq &&
+               layers == o.layers && slots == o.slots;
+    }
+};
+int round_seq(int max_seq_len) {
+    return max_seq_len <= 0 ? 0 : max_seq_len > INT_MAX - 64 ? max_seq_len : (max_seq_len + 63) / 64 * 64;
+}
+template <class Value, class Make>
+Value remembered(const PlanKey& k, Make make) {
+    constexpr int kSlots = 32;   // (power of two; a slot is overwritten by the next key that maps to it)
+    struct Entry { PlanKey key{}; Value value; bool used = false; };
+    static thread_local Entry memo[kSlots];
+    uint32_t h = 2166136261u;
+    for (int v : {k.kind, k.B, k.Hq, k.Hkv, k.d, k.seq / 64, k.layers, k.slots})
+        h = (h ^ static_cast<uint32_t>(v)) * 16777619u;
+    Entry& e = memo[(h ^ (h >> 15)) % kSlots];
+    if (!e.used || !(e.key == k)) {
+        e.value = make();
+        e.key = k;
+        e.used = true;
+    }
+    return e.value;
+}
+
 // Split the context so that the grid fills the GPU a few times over.
 ChunkPlan plan_chunks(int B, int Hq, int Hkv, int d, int max_seq_len, int n_layers) {
     const int gh = 64 / (d / 8);
@@ -409,9 +422,11 @@ ChunkPlan plan_two_regions(int64_t units, int64_t slots, int max_seq_len, double
 // CTA-wide barriers) weighs about 15 pages for a 16-warp CTA and 30 for an 8-warp one (fitted to
 // measured step times of the uniform benchmark shapes).
 ChunkPlan plan_chunks_mma(int B, int Hkv, int max_seq_len, int n_layers, int ctas_per_sm) {
-    return plan_two_regions(static_cast<int64_t>(B) * Hkv * n_layers,
-                            static_cast<int64_t>(ftq::sm_count()) * ctas_per_sm, max_seq_len,
-                            ctas_per_sm == 1 ? 15.0 : 30.0);
+    const int seq = round_seq(max_seq_len), slots = ftq::sm_count() * ctas_per_sm;
+    return remembered<ChunkPlan>({1, B, 0, Hkv, ctas_per_sm, seq, n_layers, slots}, [&] {
+        return plan_two_regions(static_cast<int64_t>(B) * Hkv * n_layers, slots, seq,
+                                ctas_per_sm == 1 ? 15.0 : 30.0);
+    });
 }
 
 // The streaming kernel.  Measured on B200 (Llama-shaped K4V4 batches of 37..111
@@ -419,8 +434,10 @@ ChunkPlan plan_chunks_mma(int B, int Hkv, int max_seq_len, int n_layers, int cta
 // service warps' smaller page share, the publish / fold / prepare hand-overs), so long chunks
 // pay -- but whole waves of them rarely match the unit count, hence the two regions.
 ChunkPlan plan_chunks_stream(int B, int Hkv, int max_seq_len, int n_layers, int ctas_per_sm) {
-    return plan_two_regions(static_cast<int64_t>(B) * Hkv * n_layers,
-                            static_cast<int64_t>(ftq::sm_count()) * ctas_per_sm, max_seq_len, 74.0);
+    const int seq = round_seq(max_seq_len), slots = ftq::sm_count() * ctas_per_sm;
+    return remembered<ChunkPlan>({2, B, 0, Hkv, 0, seq, n_layers, slots}, [&] {
+        return plan_two_regions(static_cast<int64_t>(B) * Hkv * n_layers, slots, seq, 74.0);
+    });
 }
 
 int attn_mma_stream_ctas(int d, int bits_k, int bits_v, int group) {
@@ -569,17 +586,18 @@ int ftq_encode(const void* x, int dtype, int64_t n_vec, int head_dim, int64_t ro
         return fail(FTQ_ERR_INVALID, "input rows must be 16-byte aligned");
     if (!aligned(packed, 4) || !aligned(norms_f16, 2))
         return fail(FTQ_ERR_INVALID, "outputs must be 4-byte (codes) / 2-byte (norms) aligned");
-    ftq::EncodeTables tab;
-    int rc = make_encode_tables(head_dim, bits, signs_host, boundaries_host, &tab);
+    ftq::EncodeJobs jobs{};
+    int rc = pack_signs(signs_host, head_dim, &jobs.signs);
+    if (rc == FTQ_OK) rc = make_encode_job(bits, boundaries_host, &jobs.job[0]);
     if (rc) return rc;
-    ftq::EncodeSource src{x, 1, row_stride, 0, 0};
-    ftq::EncodeSink sink{};
+    jobs.n_vec = n_vec;
+    jobs.job[0].src = ftq::EncodeSource{x, 1, row_stride, 0, 0, {}};
+    ftq::EncodeSink& sink = jobs.job[0].sink;
     sink.mode = ftq::kSinkFlat;
     sink.codes = packed;
     sink.norms = norms_f16;
     sink.Hkv = 1;
-    cudaError_t e = dispatch_encode(head_dim, bits, dtype, src, sink, tab, n_vec, 1,
-                                    static_cast<cudaStream_t>(stream));
+    cudaError_t e = dispatch_encode(head_dim, dtype, jobs, 1, 1, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_encode launch");
 }
 
@@ -735,22 +753,20 @@ static size_t counter_bytes(int B, int Hkv, int n_layers) {
 size_t ftq_decode_workspace_bytes(int B, int Hq, int Hkv, int head_dim, int max_seq_len,
                                   int n_layers) {
     if (!dim_ok(head_dim) || B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || n_layers <= 0) return 0;
-    // the larger of the two paths' needs, so one buffer serves whichever kernel runs
-    const ChunkPlan a = plan_chunks(B, Hq, Hkv, head_dim, max_seq_len, n_layers);
-    const ChunkPlan m1 = plan_chunks_mma(B, Hkv, max_seq_len, n_layers, 1);
-    const ChunkPlan m2 = plan_chunks_mma(B, Hkv, max_seq_len, n_layers, 2);
-    const ChunkPlan m3 = plan_chunks_stream(B, Hkv, max_seq_len, n_layers, 1);
-    const ChunkPlan m4 = plan_chunks_stream(B, Hkv, max_seq_len, n_layers, 2);
-    size_t n = partial_bytes(a, B, Hq, head_dim, n_layers);
-    const size_t n3 = partial_bytes(m3, B, Hq, head_dim, n_layers);
-    const size_t n4 = partial_bytes(m4, B, Hq, head_dim, n_layers);
-    if (n3 > n) n = n3;
-    if (n4 > n) n = n4;
-    const size_t n1 = partial_bytes(m1, B, Hq, head_dim, n_layers);
-    const size_t n2 = partial_bytes(m2, B, Hq, head_dim, n_layers);
-    if (n1 > n) n = n1;
-    if (n2 > n) n = n2;
-    return n + counter_bytes(B, Hkv, n_layers);
+    // the larger of the paths' needs, so one buffer serves whichever kernel runs
+    const int seq = round_seq(max_seq_len);
+    return remembered<size_t>({0, B, Hq, Hkv, head_dim, seq, n_layers, ftq::sm_count()}, [&] {
+        size_t n = 0;
+        for (const ChunkPlan& pl : {plan_chunks(B, Hq, Hkv, head_dim, seq, n_layers),
+                                    plan_chunks_mma(B, Hkv, seq, n_layers, 1),
+                                    plan_chunks_mma(B, Hkv, seq, n_layers, 2),
+                                    plan_chunks_stream(B, Hkv, seq, n_layers, 1),
+                                    plan_chunks_stream(B, Hkv, seq, n_layers, 2)}) {
+            const size_t m = partial_bytes(pl, B, Hq, head_dim, n_layers);
+            n = m > n ? m : n;
+        }
+        return n;
+    }) + counter_bytes(B, Hkv, n_layers);
 }
 
 static int check_attn_common(int B, int Hq, int Hkv, int head_dim, int bits_k, int bits_v,
@@ -781,7 +797,7 @@ int ftq_flash_decode(const void* q, int q_dtype, int q_is_rotated, const uint8_t
     if (!aligned(q, 16) || !aligned(out, 4)) return fail(FTQ_ERR_INVALID, "q must be 16-byte aligned");
     if (!aligned(k_codes, 4) || !aligned(v_codes, 4) || !aligned(k_norms, 2) || !aligned(v_norms, 2))
         return fail(FTQ_ERR_INVALID, "misaligned K/V tensor");
-    const ChunkPlan pl = plan_chunks(B, Hq, Hkv, head_dim, S, 1);
+    const ChunkPlan pl = plan_chunks(B, Hq, Hkv, head_dim, round_seq(S), 1);
     const size_t need = partial_bytes(pl, B, Hq, head_dim, 1);
     if (!workspace || workspace_bytes < need)
         return fail(FTQ_ERR_WORKSPACE, "workspace needs %zu bytes, got %zu", need, workspace_bytes);
@@ -835,14 +851,14 @@ int ftq_paged_store(const void* key, const void* value, int dtype, int64_t n_tok
         return fail(FTQ_ERR_INVALID, "pool must be 16-byte aligned");
     const int pdk = ftq::packed_dim(head_dim, bits_k), pdv = ftq::packed_dim(head_dim, bits_v);
     const int64_t page = ftq_page_bytes(head_dim, bits_k, bits_v);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    for (int which = 0; which < 2; which++) {
-        ftq::EncodeTables tab;
-        int rc = make_encode_tables(head_dim, which ? bits_v : bits_k, signs_host,
-                                    which ? boundaries_v_host : boundaries_k_host, &tab);
-        if (rc) return rc;
-        ftq::EncodeSource src{which ? value : key, Hkv, token_stride, head_stride, kv_layer_stride};
-        ftq::EncodeSink sink{};
+    ftq::EncodeJobs jobs{};
+    int rc = pack_signs(signs_host, head_dim, &jobs.signs);
+    jobs.n_vec = n_tokens * Hkv;
+    for (int which = 0; which < 2 && rc == FTQ_OK; which++) {
+        ftq::EncodeJob& job = jobs.job[which];
+        rc = make_encode_job(which ? bits_v : bits_k, which ? boundaries_v_host : boundaries_k_host, &job);
+        job.src = ftq::EncodeSource{which ? value : key, Hkv, token_stride, head_stride, kv_layer_stride, {}};
+        ftq::EncodeSink& sink = job.sink;
         sink.mode = ftq::kSinkPaged;
         sink.codes = pool;
         sink.slot_mapping = slot_mapping;
@@ -854,11 +870,10 @@ int ftq_paged_store(const void* key, const void* value, int dtype, int64_t n_tok
                                : FTQ_PAGE_TOKENS * pdk;
         sink.layer_stride = pool_layer_stride;
         sink.swap_halves = which;  // V rows only (see the page layout in ftq_b200.h)
-        cudaError_t e = dispatch_encode(head_dim, which ? bits_v : bits_k, dtype, src, sink, tab,
-                                        n_tokens * Hkv, n_layers, st);
-        if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_store launch");
     }
-    return FTQ_OK;
+    if (rc) return rc;
+    const cudaError_t e = dispatch_encode(head_dim, dtype, jobs, 2, n_layers, static_cast<cudaStream_t>(stream));
+    return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_paged_store launch");
 }
 
 int ftq_paged_decode_attn(const void* q, int q_dtype, void* out, int out_dtype,
@@ -889,7 +904,7 @@ int ftq_paged_decode_attn(const void* q, int q_dtype, void* out, int out_dtype,
     const bool streams = stream_ctas > 0;
     const ChunkPlan pl = streams ? plan_chunks_stream(B, Hkv, max_seq_len, n_layers, stream_ctas)
                          : mma   ? plan_chunks_mma(B, Hkv, max_seq_len, n_layers, mma_ctas)
-                                 : plan_chunks(B, Hq, Hkv, head_dim, max_seq_len, n_layers);
+                                 : plan_chunks(B, Hq, Hkv, head_dim, round_seq(max_seq_len), n_layers);
     const size_t need = ftq_decode_workspace_bytes(B, Hq, Hkv, head_dim, max_seq_len, n_layers);
     if (!workspace || workspace_bytes < need)
         return fail(FTQ_ERR_WORKSPACE, "workspace needs %zu bytes, got %zu", need, workspace_bytes);
@@ -974,14 +989,14 @@ int ftq_v0_store(const void* key, const void* value, int dtype, int64_t n_tokens
     if (!aligned(key, 16) || !aligned(value, 16) || (token_stride * es) % 16 || (head_stride * es) % 16)
         return fail(FTQ_ERR_INVALID, "key/value rows must be 16-byte aligned");
     if (!aligned(kv_cache, 4)) return fail(FTQ_ERR_INVALID, "kv_cache must be 4-byte aligned");
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    for (int which = 0; which < 2; which++) {
-        ftq::EncodeTables tab;
-        int rc = make_encode_tables(head_dim, which ? bits_v : bits_k, signs_host,
-                                    which ? boundaries_v_host : boundaries_k_host, &tab);
-        if (rc) return rc;
-        ftq::EncodeSource src{which ? value : key, Hkv, token_stride, head_stride, 0};
-        ftq::EncodeSink sink{};
+    ftq::EncodeJobs jobs{};
+    int rc = pack_signs(signs_host, head_dim, &jobs.signs);
+    jobs.n_vec = n_tokens * Hkv;
+    for (int which = 0; which < 2 && rc == FTQ_OK; which++) {
+        ftq::EncodeJob& job = jobs.job[which];
+        rc = make_encode_job(which ? bits_v : bits_k, which ? boundaries_v_host : boundaries_k_host, &job);
+        job.src = ftq::EncodeSource{which ? value : key, Hkv, token_stride, head_stride, 0, {}};
+        ftq::EncodeSink& sink = job.sink;
         sink.mode = ftq::kSinkV0;
         sink.codes = kv_cache;
         sink.slot_mapping = slot_mapping;
@@ -990,11 +1005,10 @@ int ftq_v0_store(const void* key, const void* value, int dtype, int64_t n_tokens
         sink.slot_limit = num_blocks * block_size;
         sink.elem_size = elem_size;
         sink.plane_off = static_cast<int64_t>(which) * num_blocks * block_size * Hkv * elem_size;
-        cudaError_t e = dispatch_encode(head_dim, which ? bits_v : bits_k, dtype, src, sink, tab,
-                                        n_tokens * Hkv, 1, st);
-        if (e != cudaSuccess) return cuda_fail(e, "ftq_v0_store launch");
     }
-    return FTQ_OK;
+    if (rc) return rc;
+    const cudaError_t e = dispatch_encode(head_dim, dtype, jobs, 2, 1, static_cast<cudaStream_t>(stream));
+    return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_v0_store launch");
 }
 
 int ftq_v0_gather(const uint8_t* kv_cache, int64_t num_blocks, int block_size, int Hkv,

@@ -75,9 +75,8 @@ static cudaError_t run_mma_nh(const AttnParams& p, int n_lb, cudaStream_t stream
     constexpr int D = FTQ_D;
     if constexpr (use_stream_kernel<BK, BV, NH>()) {
         using S = StreamCfg<D, BK, BV, NH>;
-        auto kern = attn_stream_kernel<D, BK, BV, SHARED, NH>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             S::SMEM_BYTES);
+        constexpr auto kern = attn_stream_kernel<D, BK, BV, SHARED, NH>;
+        cudaError_t e = allow_smem<kern>(S::SMEM_BYTES);
         if (e != cudaSuccess) return e;
         const int64_t items = p.split.total_items;
         const int64_t slots = static_cast<int64_t>(sm_count()) * S::CTAS_PER_SM;
@@ -106,9 +105,8 @@ static cudaError_t run_mma_nh(const AttnParams& p, int n_lb, cudaStream_t stream
     *merged = false;
     using C = MmaCfg<D, BK, BV, NH>;
     static_assert(C::SMEM_BYTES <= 227 * 1024, "shared memory budget");
-    auto kern = attn_mma_kernel<D, BK, BV, SHARED, NH>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         C::SMEM_BYTES);
+    constexpr auto kern = attn_mma_kernel<D, BK, BV, SHARED, NH>;
+    cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     const int64_t items = p.split.total_items;
     const int64_t slots = static_cast<int64_t>(sm_count()) * C::CTAS_PER_SM;

@@ -21,6 +21,10 @@
 //    floating point (exact below 2^24).
 #pragma once
 
+#include <cfloat>
+#include <cmath>
+#include <cstring>
+
 #include "ftq_encode.cuh"
 
 namespace ftq {
@@ -30,16 +34,17 @@ constexpr float kCellScale = 128.0f;                 // cells per unit of x
 constexpr float kCellMagic = 98304.0f + 128.0f;      // 1.5 * 2^16 + scale: ulp = 2^-7
 constexpr float kStepScale = 1.2676506002282294e30f; // 2^100
 
-struct QuantCell {
-    float neg_thr_scaled;  // -boundary * 2^100, or -FLT_MAX when the cell holds no boundary
-    float base;            // number of interior boundaries in lower cells
-};
-
-struct Encode2Tables {
-    SignBits signs;
-    float rsqrt_d;
-    QuantCell cells[kQuantCells];
-};
+// Cell of x in the table quantizer (the kernel applies the same single-precision FMA).
+__host__ __device__ __forceinline__ uint32_t quant_cell(float x) {
+    const float v = fmaf(x, kCellScale, kCellMagic);
+#ifdef __CUDA_ARCH__
+    const uint32_t bits = __float_as_uint(v);
+#else
+    uint32_t bits;
+    memcpy(&bits, &v, 4);
+#endif
+    return (bits & 0xFF80u) >> 7;
+}
 
 typedef unsigned long long u64;
 
@@ -159,9 +164,14 @@ __host__ __device__ constexpr int encode2_smem_bytes(int D, int warps) {
 
 __host__ __device__ constexpr int encode2_threads(int D) { return D >= 256 ? 512 : 256; }
 
+// One (neg_thr_scaled, base) pair per cell, 16 copies so that lane column = bank pair:
+// -boundary * 2^100 of the boundary inside the cell (-FLT_MAX: none) and the number of interior
+// boundaries in lower cells.
+typedef float2 QuantTable[kQuantCells][16];
+
 template <int D, int BITS, typename T>
-__global__ void __launch_bounds__(encode2_threads(D), 512 / encode2_threads(D))
-encode2_kernel(EncodeSource src, EncodeSink sink, const Encode2Tables tab, int64_t n_vec) {
+__device__ __forceinline__ void encode2_body(const EncodeJobs& jobs, const EncodeJob& job,
+                                             QuantTable& lut, float* tbuf) {
     constexpr int E = D / kOctet;
     constexpr int NCH = E / 8;
     constexpr int SLOT = encode2_slot_floats(D);
@@ -170,18 +180,26 @@ encode2_kernel(EncodeSource src, EncodeSink sink, const Encode2Tables tab, int64
     constexpr int CPF = 24 / BITS;                          // codes per fp32 accumulator
     constexpr int FPW = (IPW + CPF - 1) / CPF;              // accumulators per word
     constexpr bool NARROW = sizeof(T) == 2;                 // bf16 / fp16 input
-
-    // the quantiser table is a static array: its shared-memory offset is then an immediate of
-    // the load and the per-element address is one bit-select (cell row | lane column)
-    __shared__ __align__(128) float2 lut[kQuantCells * 16];            // [257][16]
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    float* tbuf = reinterpret_cast<float*>(smem_raw);                  // [warps][4][SLOT]
+    const EncodeSource& src = job.src;
+    const EncodeSink& sink = job.sink;
+    const int64_t n_vec = jobs.n_vec;
 
     const int tid = threadIdx.x;
     const int lane = tid & 31, wip = tid >> 5;
     const int t = lane & 7, sub = lane >> 3;
-    for (int i = tid; i < kQuantCells * 16; i += blockDim.x)
-        lut[i] = make_float2(tab.cells[i >> 4].neg_thr_scaled, tab.cells[i >> 4].base);
+    for (int c = tid; c < kQuantCells; c += blockDim.x) {
+        float thr = -FLT_MAX, base = 0.f;
+#pragma unroll
+        for (int j = 0; j < (1 << BITS) - 1; j++) {
+            const float b = job.bounds[j];
+            const int cb = static_cast<int>(quant_cell(b));
+            if (cb == c) thr = -b * kStepScale;
+            if (cb < c) base += 1.f;
+        }
+        // (staggered by the cell: the copies of neighbouring threads go to different banks)
+#pragma unroll
+        for (int i = 0; i < 16; i++) lut[c][(i + c) & 15] = make_float2(thr, base);
+    }
     __syncthreads();
     const uint32_t lut_col = (lane & 15) * 8;
     float* slot = tbuf + (wip * 4 + sub) * SLOT;
@@ -198,12 +216,12 @@ encode2_kernel(EncodeSource src, EncodeSink sink, const Encode2Tables tab, int64
 #pragma unroll
     for (int r = 0; r < NSGN; r++) {
         if constexpr (NARROW)
-            sgn[r] = (sign_mask(tab.signs, load_coord(t, 2 * r)) >> 16) |
-                     sign_mask(tab.signs, load_coord(t, 2 * r + 1));
+            sgn[r] = (sign_mask(jobs.signs, load_coord(t, 2 * r)) >> 16) |
+                     sign_mask(jobs.signs, load_coord(t, 2 * r + 1));
         else
-            sgn[r] = sign_mask(tab.signs, load_coord(t, r));
+            sgn[r] = sign_mask(jobs.signs, load_coord(t, r));
     }
-    const u64 scale2 = pk2(tab.rsqrt_d, tab.rsqrt_d);
+    const u64 scale2 = pk2(jobs.rsqrt_d, jobs.rsqrt_d);
     const u64 cs2 = pk2(kCellScale, kCellScale), cm2 = pk2(kCellMagic, kCellMagic);
     const TransposeConsts<BITS> tc = transpose_consts<BITS>(lane);
 
@@ -335,8 +353,8 @@ encode2_kernel(EncodeSource src, EncodeSink sink, const Encode2Tables tab, int64
             {
                 const uint32_t oA = (__float_as_uint(cA) & 0xFF80u) | lut_col;
                 const uint32_t oB = (__float_as_uint(cB) & 0xFF80u) | lut_col;
-                eA = *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(lut) + oA);
-                eB = *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(lut) + oB);
+                eA = *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(&lut) + oA);
+                eB = *reinterpret_cast<const float2*>(reinterpret_cast<const uint8_t*>(&lut) + oB);
             }
             const float stA = fma_sat(qA, kStepScale, eA.x);
             const float stB = fma_sat(qB, kStepScale, eB.x);
@@ -367,6 +385,22 @@ encode2_kernel(EncodeSource src, EncodeSink sink, const Encode2Tables tab, int64
         if constexpr (!NARROW) {
             if (base + n_warps * 8 < n_vec) issue_loads(base + n_warps * 8);
         }
+    }
+}
+
+template <int D, typename T>
+__global__ void __launch_bounds__(encode2_threads(D), 512 / encode2_threads(D))
+encode2_kernel(const __grid_constant__ EncodeJobs jobs) {
+    // the quantiser table is a static array: its shared-memory offset is then an immediate of
+    // the load and the per-element address is one bit-select (cell row | lane column)
+    __shared__ __align__(128) QuantTable lut;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    float* tbuf = reinterpret_cast<float*>(smem_raw);                  // [warps][4][SLOT]
+    const EncodeJob& job = jobs.job[blockIdx.z];
+    switch (job.bits) {
+        case 2: encode2_body<D, 2, T>(jobs, job, lut, tbuf); break;
+        case 3: encode2_body<D, 3, T>(jobs, job, lut, tbuf); break;
+        case 4: encode2_body<D, 4, T>(jobs, job, lut, tbuf); break;
     }
 }
 

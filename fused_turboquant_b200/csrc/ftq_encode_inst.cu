@@ -9,59 +9,39 @@
 
 namespace ftq {
 
-// Throughput kernel (needs the table quantizer; see ftq_encode2.cuh).
-template <int BITS, typename T>
-static cudaError_t run2(const EncodeSource& src, const EncodeSink& sink, const Encode2Tables& tab,
-                        int64_t n_vec, int n_layers, cudaStream_t stream) {
-    // 16 warps per SM: two CTAs of 8 warps, or one of 16 where two transpose areas would not
-    // fit next to two copies of the quantiser table (head_dim 256); a warp pass = 8 vectors
-    constexpr int threads = encode2_threads(FTQ_D);
-    constexpr int ctas_per_sm = 512 / threads;
-    constexpr int smem = encode2_smem_bytes(FTQ_D, threads / 32);
-    auto kern = encode2_kernel<FTQ_D, BITS, T>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    const int64_t want = (n_vec + threads / 4 - 1) / (threads / 4);
-    const int64_t cap = static_cast<int64_t>(sm_count()) * ctas_per_sm;   // persistent grid
-    const unsigned gx = static_cast<unsigned>(want < 1 ? 1 : (want < cap ? want : cap));
-    kern<<<dim3(gx, n_layers), threads, smem, stream>>>(src, sink, tab, n_vec);
-    return cudaGetLastError();
-}
-
-template <int BITS, typename T>
-static cudaError_t run(const EncodeSource& src, const EncodeSink& sink, const EncodeTables& tab,
-                       const Encode2Tables* tab2, int64_t n_vec, int n_layers,
-                       cudaStream_t stream) {
-    if (tab2) return run2<BITS, T>(src, sink, *tab2, n_vec, n_layers, stream);
-    constexpr int threads = 256;                       // 8 warps, 32 vectors per CTA pass
-    const int64_t want = (n_vec + 31) / 32;
-    const int64_t cap = static_cast<int64_t>(sm_count()) * 8;  // persistent-style grid
-    const unsigned gx = static_cast<unsigned>(want < 1 ? 1 : (want < cap ? want : cap));
-    encode_kernel<FTQ_D, BITS, T><<<dim3(gx, n_layers), threads, 0, stream>>>(src, sink, tab, n_vec);
-    return cudaGetLastError();
-}
-
-template <int BITS>
-static cudaError_t by_dtype(int dtype, const EncodeSource& src, const EncodeSink& sink,
-                            const EncodeTables& tab, const Encode2Tables* tab2, int64_t n_vec,
-                            int n_layers, cudaStream_t stream) {
-    switch (dtype) {
-        case kF32: return run<BITS, float>(src, sink, tab, tab2, n_vec, n_layers, stream);
-        case kF16: return run<BITS, __half>(src, sink, tab, tab2, n_vec, n_layers, stream);
-        case kBF16:
-            return run<BITS, __nv_bfloat16>(src, sink, tab, tab2, n_vec, n_layers, stream);
+template <typename T>
+static cudaError_t run(const EncodeJobs& jobs, int n_jobs, bool bulk, int n_layers, cudaStream_t stream) {
+    const int64_t n = jobs.n_vec;
+    if (bulk) {
+        // 16 warps per SM: two CTAs of 8 warps, or one of 16 where two transpose areas would not
+        // fit next to two copies of the quantiser table (head_dim 256); a warp pass = 8 vectors.
+        // Persistent: the jobs and layers share one wave of CTAs.
+        constexpr int threads = encode2_threads(FTQ_D);
+        constexpr int smem = encode2_smem_bytes(FTQ_D, threads / 32);
+        constexpr auto kern = encode2_kernel<FTQ_D, T>;
+        const cudaError_t e = allow_smem<kern>(smem);
+        if (e != cudaSuccess) return e;
+        const int64_t want = (n + threads / 4 - 1) / (threads / 4);
+        const int64_t share = static_cast<int64_t>(sm_count()) * (512 / threads) / (n_jobs * n_layers);
+        const int64_t cap = share > 1 ? share : 1;
+        const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), n_layers, n_jobs);
+        kern<<<grid, threads, smem, stream>>>(jobs);
+        return cudaGetLastError();
     }
-    return cudaErrorInvalidValue;
+    constexpr int threads = 128;                       // 4 warps, a vector each
+    const int64_t want = (n + threads / 32 - 1) / (threads / 32);
+    const int64_t cap = static_cast<int64_t>(sm_count()) * 64;
+    const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), n_layers, n_jobs);
+    encode_kernel<FTQ_D, T><<<grid, threads, 0, stream>>>(jobs);
+    return cudaGetLastError();
 }
 
-cudaError_t FTQ_CAT(launch_encode_d, FTQ_D)(int bits, int dtype, const EncodeSource& src,
-                                            const EncodeSink& sink, const EncodeTables& tab,
-                                            const Encode2Tables* tab2, int64_t n_vec, int n_layers,
-                                            cudaStream_t stream) {
-    switch (bits) {
-        case 2: return by_dtype<2>(dtype, src, sink, tab, tab2, n_vec, n_layers, stream);
-        case 3: return by_dtype<3>(dtype, src, sink, tab, tab2, n_vec, n_layers, stream);
-        case 4: return by_dtype<4>(dtype, src, sink, tab, tab2, n_vec, n_layers, stream);
+cudaError_t FTQ_CAT(launch_encode_d, FTQ_D)(int dtype, const EncodeJobs& jobs, int n_jobs, bool bulk,
+                                            int n_layers, cudaStream_t stream) {
+    switch (dtype) {
+        case kF32: return run<float>(jobs, n_jobs, bulk, n_layers, stream);
+        case kF16: return run<__half>(jobs, n_jobs, bulk, n_layers, stream);
+        case kBF16: return run<__nv_bfloat16>(jobs, n_jobs, bulk, n_layers, stream);
     }
     return cudaErrorInvalidValue;
 }

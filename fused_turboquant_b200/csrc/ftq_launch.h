@@ -4,16 +4,16 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "ftq_attn.cuh"
 #include "ftq_encode2.cuh"
 
 namespace ftq {
 
 #define FTQ_DECLARE_LAUNCHERS(DD)                                                              \
-    cudaError_t launch_encode_d##DD(int bits, int dtype, const EncodeSource& src,               \
-                                    const EncodeSink& sink, const EncodeTables& tab,            \
-                                    const Encode2Tables* tab2, int64_t n_vec, int n_layers,     \
-                                    cudaStream_t stream);                                       \
+    cudaError_t launch_encode_d##DD(int dtype, const EncodeJobs& jobs, int n_jobs, bool bulk,   \
+                                    int n_layers, cudaStream_t stream);                         \
     cudaError_t launch_attn_split_d##DD(int bits_k, int bits_v, bool paged, const AttnParams& p, \
                                         int n_lb, cudaStream_t stream);                         \
     cudaError_t launch_attn_mma_d##DD(int bits_k, int bits_v, bool shared_lut, const AttnParams& p, \
@@ -31,5 +31,22 @@ FTQ_DECLARE_LAUNCHERS(256)
 
 // number of SMs of the current device (cached per device)
 int sm_count();
+
+namespace {   // (internal linkage: every library that holds these kernels keeps its own record)
+// Allows `kern` more than 48 KB of dynamic shared memory, once per device (the attribute call costs
+// the host about half a microsecond, which every launch used to pay).
+template <auto kern>
+inline cudaError_t allow_smem(int bytes) {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+    const cudaError_t r = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (r == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return r;
+}
+}  // namespace
 
 }  // namespace ftq

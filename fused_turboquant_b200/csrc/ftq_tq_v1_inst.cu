@@ -135,8 +135,8 @@ template <int KB, int VB, int NH>
 static cudaError_t mma_run(const TqDecodeParams& p, int n_items, cudaStream_t stream) {
     using C = TqMmaCfg<FTQ_D, KB, VB, NH>;
     static_assert(C::SMEM_BYTES <= 227 * 1024, "shared memory budget");
-    auto kern = tq_mma_kernel<FTQ_D, KB, VB, NH>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    constexpr auto kern = tq_mma_kernel<FTQ_D, KB, VB, NH>;
+    cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     const int64_t slots = static_cast<int64_t>(sm_count()) * C::CTAS_PER_SM;
     const unsigned gx = static_cast<unsigned>(n_items < slots ? n_items : slots);

@@ -32,8 +32,7 @@
 // dropped into bits 8..15 of the lane's base address.  3- and 2-bit codes use
 // 128-byte rows in a table aligned to its own size (shift + and/or).
 //
-// Fragment maps for one 16-token page (lane = 4*g + tg), query heads handled in
-// halves of 4 (NH = 1 for a GQA group <= 4, else 2):
+// Fragment maps for one 16-token page (lane = 4*g + tg), GQA group <= 4 (NH = 1):
 //   S = K.Q^T :  A = K [16 tokens x 16 coords]: rows g / g+8 = page tokens rho(g) / rho(g)+2,
 //                    k-block kb covers coordinates (D/4)*tg + 4*kb + {0..3}
 //                B = Q^T[16 coords x 8]: column n = head n>>1 (each head twice)
@@ -45,8 +44,18 @@
 //                A[row = d-pair][k = (token, parity)] = V[token][2*pair + parity]
 //                B[k = (token, parity)][n = (head n>>1, parity n&1)] = p or 0
 //                C[d-pair][(head tg, parity)]: lane (g,tg) owns O[head tg][(D/8)g .. +D/8)
-//   so a lane dequantises the K slices (D/4 coordinates) of two tokens and the V
-//   slices (D/8 coordinates) of four tokens per page, all contiguous bytes, every
+// GQA group 5 .. 8 (NH = 2): the eight columns are eight heads,
+//   S:  B column n = head n;  C[token][heads 2tg, 2tg + 1]; the two weights of a token are packed
+//                into one fp16 pair, and movmatrix turns the packed scores of tokens rho(0..7)
+//                (rho(0..7) + 2) straight into the B registers of P.V: head g, tokens 4tg, 4tg + 1
+//                (4tg + 2, 4tg + 3);
+//   O^T += V^T.P^T with k = token:  A[row g / g+8 = coordinate (D/8)g + 2mt / + 1][k = token]: the
+//                pairs of two tokens' look-ups are exchanged with two byte-permutes;
+//                C[coordinate pair][heads 2tg, 2tg + 1].
+//   Against two passes of the 4-head map this halves the MMAs and the softmax bookkeeping for one
+//   byte-permute per value look-up.
+// In both maps a lane dequantises the K slices (D/4 coordinates) of two tokens and the V
+// slices (D/8 coordinates) of four tokens per page, all contiguous bytes, every
 //   code exactly once per KV head.
 #pragma once
 
@@ -90,6 +99,9 @@ __device__ __forceinline__ uint2 lut64(uint32_t addr) {
     return v;
 }
 
+#ifndef FTQ_MMA_PIPE
+#define FTQ_MMA_PIPE (!C::QSMEM && WARPS <= 16)
+#endif
 #ifndef FTQ_LAZY_SLACK
 #define FTQ_LAZY_SLACK 3
 #endif
@@ -107,6 +119,12 @@ __device__ __forceinline__ void mma_16816_z(float (&c)[4], uint32_t a0, uint32_t
 __device__ __forceinline__ uint32_t f2h_sat(float x) {
     unsigned short h;
     asm("cvt.rn.satfinite.f16.f32 %0, %1;\n" : "=h"(h) : "f"(x));
+    return h;
+}
+
+__device__ __forceinline__ uint32_t f2h2_sat(float lo, float hi) {
+    uint32_t h;
+    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;\n" : "=r"(h) : "f"(hi), "f"(lo));
     return h;
 }
 
@@ -174,43 +192,42 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     return v;
 }
 
-// Load slice `idx` (SB bytes each, slices back to back starting at the 4-byte aligned shared
-// address `row`) of a staged page into ceil(SB/4) words.  Slices whose size is not a multiple
-// of 4 are cut out of the enclosing aligned chunk with funnel shifts.
+// A lane's slice of SB packed bytes into ceil(SB/4) words.  `addr` is the 4-byte aligned address at
+// or below the slice's start and `sh` 8 * the bytes between the two (both are lane constants, see
+// slice_word / slice_shift; whole-word slices ignore `sh`).  Slices of 6 and 3 bytes come out of
+// two words with funnel shifts; bits beyond the slice are junk that pair_index masks (the second
+// word of a row's last slice may lie behind the row, never behind the page).
 template <int SB>
-__device__ __forceinline__ void lds_slice(uint32_t row, int idx, uint32_t (&w)[(SB + 3) / 4]) {
+__device__ __forceinline__ constexpr uint32_t slice_word(int idx) { return (SB * idx) & ~3; }
+template <int SB>
+__device__ __forceinline__ constexpr uint32_t slice_shift(int idx) { return 8 * ((SB * idx) & 3); }
+template <int SB>
+__device__ __forceinline__ void lds_slice(uint32_t addr, uint32_t sh, uint32_t (&w)[(SB + 3) / 4]) {
     if constexpr (SB % 16 == 0) {
 #pragma unroll
         for (int i = 0; i < SB / 16; i++) {
-            const uint4 v = lds128(row + idx * SB + 16 * i);
+            const uint4 v = lds128(addr + 16 * i);
             w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
         }
     } else if constexpr (SB % 8 == 0) {
 #pragma unroll
         for (int i = 0; i < SB / 8; i++) {
-            const uint2 v = lds64(row + idx * SB + 8 * i);
+            const uint2 v = lds64(addr + 8 * i);
             w[2 * i] = v.x; w[2 * i + 1] = v.y;
         }
     } else if constexpr (SB % 4 == 0) {
 #pragma unroll
-        for (int i = 0; i < SB / 4; i++) w[i] = lds32(row + idx * SB + 4 * i);
+        for (int i = 0; i < SB / 4; i++) w[i] = lds32(addr + 4 * i);
     } else if constexpr (SB == 6) {
-        const uint32_t c = row + (idx >> 1) * 12;
-        const uint32_t x0 = lds32(c), x1 = lds32(c + 4), x2 = lds32(c + 8);
-        const bool odd = idx & 1;
-        w[0] = odd ? __funnelshift_r(x1, x2, 16) : x0;
-        w[1] = odd ? (x2 >> 16) : (x1 & 0xffffu);
+        const uint32_t x0 = lds32(addr), x1 = lds32(addr + 4);
+        w[0] = __funnelshift_r(x0, x1, sh);
+        w[1] = x1 >> sh;
     } else if constexpr (SB == 3) {
-        const uint32_t c = row + (idx >> 2) * 12;
-        const uint32_t x0 = lds32(c), x1 = lds32(c + 4), x2 = lds32(c + 8);
-        const int q = idx & 3;
-        const uint32_t lo = q == 0 ? x0 : (q == 1 ? __funnelshift_r(x0, x1, 24)
-                                                  : (q == 2 ? __funnelshift_r(x1, x2, 16) : (x2 >> 8)));
-        w[0] = lo & 0xffffffu;
+        const uint32_t x0 = lds32(addr), x1 = lds32(addr + 4);
+        w[0] = __funnelshift_r(x0, x1, sh);
     } else {
         static_assert(SB == 2, "unsupported slice size");
-        const uint32_t x = lds32(row + (idx >> 1) * 4);
-        w[0] = (idx & 1) ? (x >> 16) : (x & 0xffffu);
+        w[0] = lds32(addr) >> sh;
     }
 }
 
@@ -262,6 +279,9 @@ struct MmaCfg {
     static constexpr int SMALL_ALIGN = TKS > TVS ? TKS : TVS;
     static constexpr int SMALL_BYTES = TKS + TVS + SMALL_ALIGN;  // incl. alignment slack
     static constexpr int STATE_F4 = NH * NMT;                    // float4 items per lane
+    static constexpr bool H8 = NH == 2;       // eight heads in the N dimension (see the fragment maps)
+    static constexpr int HL = H8 ? 2 : 1;     // heads whose softmax state a lane keeps: HL * tg + {0 ..}
+    static constexpr int NPB = H8 ? 1 : 2;    // P.V steps per page
     // per-warp ring of pages staged by bulk copies (TMA), one mbarrier per buffer
     static constexpr int RING = 2;
     static constexpr int BASE_A = SMALL_BYTES + 8 * (D + 16) * 4 + kMmaMaxChunkPages * 4 + 64;
@@ -383,26 +403,27 @@ attn_mma_kernel(const AttnParams p, int n_items) {
     const int g = lane >> 2, tg = lane & 3;
     const bool odd = g & 1;
     const int group = p.Hq / p.Hkv;  // <= 4 * NH
+    constexpr bool H8 = C::H8;
+    constexpr int NO = C::STATE_F4;  // accumulator tiles per lane
+    constexpr int HL = C::HL;
     // byte selectors (source 4 = a zero byte): a lane's own fp16 of a packed pair, and the
     // placement of a weight in the low (even g) or high (odd g) half of a B register
     uint32_t sel_own = odd ? 0x4432u : 0x4410u;
     uint32_t sel_plo = odd ? 0x1044u : 0x4410u;
     uint32_t sel_phi = odd ? 0x3244u : 0x4432u;
     // Lane constants of the page reads: byte offset of the key row rho(g) and of the norm quad;
-    // per value register j the row of page token 4tg + ((j + tg) & 3) (plus the slice where
-    // slices are whole words) and the slice index otherwise (slice g, halves exchanged for tokens
-    // with bit 1 set).  (The streaming kernel pins these in registers; here that measured no gain.)
-    uint32_t koff = (4 * (g >> 1) + (g & 1)) * MmaCfg<D, BK, BV, NH>::PDK;
-    uint32_t noff = MmaCfg<D, BK, BV, NH>::OFF_KN + 8 * (g >> 1);
+    // per value register j the first word of slice g in the row of page token 4tg + ((j + tg) & 3)
+    // (halves exchanged for tokens with bit 1 set).  (The streaming kernel pins these in registers; here that measured no gain.)
+    uint32_t koff = (4 * (g >> 1) + (g & 1)) * C::PDK + slice_word<C::KSB>(tg);
+    const uint32_t ksh = slice_shift<C::KSB>(tg);
+    uint32_t noff = C::OFF_KN + 8 * (g >> 1);
     uint32_t vrow[4];
-    int vidx[4];
+    const uint32_t vsh = slice_shift<C::VSB>(g);   // (the same for the exchanged slice g ^ 4)
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        using CC = MmaCfg<D, BK, BV, NH>;
         const int u = (j + tg) & 3;
         const int slice = g ^ ((u & 2) << 1);
-        vrow[j] = CC::OFF_VC + (4 * tg + u) * CC::PDV + (CC::VSB % 4 == 0 ? slice * CC::VSB : 0);
-        vidx[j] = CC::VSB % 4 == 0 ? 0 : slice;
+        vrow[j] = C::OFF_VC + (4 * tg + u) * C::PDV + slice_word<C::VSB>(slice);
     }
 
     // ---- once per CTA: dequantisation tables
@@ -558,7 +579,7 @@ attn_mma_kernel(const AttnParams p, int n_items) {
     };
     // warps that fold the per-warp states into the partial rows; when at least two warps are
     // left over they run the next item's prologue at the same time
-    constexpr int NRED = (NH * NMT <= WARPS - 2) ? NH * NMT : WARPS;
+    constexpr int NRED = (NO <= WARPS - 2) ? NO : WARPS;
 
 #ifdef FTQ_TEST_WAIT_EXPIRY
     bool test_drop = blockIdx.x == 0 && warp == 5;
@@ -585,34 +606,32 @@ attn_mma_kernel(const AttnParams p, int n_items) {
         const int next = s_next[slot];
         slot ^= 1;
 
-        // Q^T fragments: column n = g is head 4*hh + (g >> 1); k-block kb covers coordinates
+        // Q^T fragments: column n = g is head g >> 1 (NH = 1) or g (NH = 2); k-block kb covers coordinates
         // (D/4)*tg + 4*kb + {0,1} (b0) and + {2,3} (b1)
-        uint32_t qb[C::QSMEM ? 1 : NH][C::QSMEM ? 1 : NKB][2];
-        // shared-memory copy of the fragments (QSMEM): [hh][kb][lane] x 8 bytes, in place of the
+        uint32_t qb[C::QSMEM ? 1 : NKB][2];
+        // shared-memory copy of the fragments (QSMEM): [kb][lane] x 8 bytes, in place of the
         // fp32 queries, which nobody reads again before the next item's prologue rewrites them
         const uint32_t qfrag = static_cast<uint32_t>(__cvta_generic_to_shared(qs));
         if constexpr (!C::QSMEM) {
 #pragma unroll
-            for (int hh = 0; hh < NH; hh++)
-#pragma unroll
-                for (int kb = 0; kb < NKB; kb++) {
-                    const float4 q4 = *reinterpret_cast<const float4*>(
-                        qs + qs_index(4 * hh + (g >> 1), (D / 4) * tg + 4 * kb));
-                    const __half2 lo = __floats2half2_rn(q4.x, q4.y);
-                    const __half2 hi = __floats2half2_rn(q4.z, q4.w);
-                    qb[hh][kb][0] = *reinterpret_cast<const uint32_t*>(&lo);
-                    qb[hh][kb][1] = *reinterpret_cast<const uint32_t*>(&hi);
-                }
+            for (int kb = 0; kb < NKB; kb++) {
+                const float4 q4 = *reinterpret_cast<const float4*>(
+                    qs + qs_index(H8 ? g : g >> 1, (D / 4) * tg + 4 * kb));
+                const __half2 lo = __floats2half2_rn(q4.x, q4.y);
+                const __half2 hi = __floats2half2_rn(q4.z, q4.w);
+                qb[kb][0] = *reinterpret_cast<const uint32_t*>(&lo);
+                qb[kb][1] = *reinterpret_cast<const uint32_t*>(&hi);
+            }
         } else {
-            constexpr int NE = NH * NKB * 32, PER = (NE + THREADS - 1) / THREADS;
+            constexpr int NE = NKB * 32, PER = (NE + THREADS - 1) / THREADS;
             uint2 frag[PER];
 #pragma unroll
             for (int i = 0; i < PER; i++) {
                 const int e = tid + i * THREADS;
-                const int ln = e & 31, kb = (e >> 5) % NKB, hh = (e >> 5) / NKB;
+                const int ln = e & 31, kb = e >> 5;
                 if (e < NE) {
                     const float4 q4 = *reinterpret_cast<const float4*>(
-                        qs + qs_index(4 * hh + (ln >> 3), (D / 4) * (ln & 3) + 4 * kb));
+                        qs + qs_index(H8 ? ln >> 2 : ln >> 3, (D / 4) * (ln & 3) + 4 * kb));
                     const __half2 lo = __floats2half2_rn(q4.x, q4.y);
                     const __half2 hi = __floats2half2_rn(q4.z, q4.w);
                     frag[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo),
@@ -633,17 +652,14 @@ attn_mma_kernel(const AttnParams p, int n_items) {
             p.pool + layer * p.pool_layer_stride + static_cast<int64_t>(hkv) * C::PAGE_BYTES;
         const uint32_t blk_stride = static_cast<uint32_t>(p.Hkv) * C::PAGE_BYTES;
 
-        // per lane: softmax state of head 4*hh + tg, O[head][(D/8)*g .. + D/8)
-        float m_run[NH], l_run[NH], oacc[NH][NMT][4];
+        // per lane: softmax state of heads HL*tg + {0 .. HL-1}, O[head][(D/8)*g .. + D/8)
+        float m_run[HL], l_run[HL], oacc[NO][4];
 #pragma unroll
-        for (int hh = 0; hh < NH; hh++) {
-            m_run[hh] = -INFINITY;
-            l_run[hh] = 0.f;
+        for (int i = 0; i < HL; i++) { m_run[i] = -INFINITY; l_run[i] = 0.f; }
 #pragma unroll
-            for (int mt = 0; mt < NMT; mt++)
+        for (int mt = 0; mt < NO; mt++)
 #pragma unroll
-                for (int i = 0; i < 4; i++) oacc[hh][mt][i] = 0.f;
-        }
+            for (int i = 0; i < 4; i++) oacc[mt][i] = 0.f;
 
         const uint32_t my_bars = bars + warp * C::RING * 8;
         const uint32_t my_ring = ring + warp * C::RING * C::PAGE_BYTES;
@@ -675,8 +691,8 @@ attn_mma_kernel(const AttnParams p, int n_items) {
         // every lane copies its slices of the staged page into registers
         auto read_page = [&](Regs& r, int rb) {
             const uint32_t page = my_ring + rb * C::PAGE_BYTES;
-            lds_slice<C::KSB>(page + koff, tg, r.k[0]);
-            lds_slice<C::KSB>(page + koff + 2 * C::PDK, tg, r.k[1]);
+            lds_slice<C::KSB>(page + koff, ksh, r.k[0]);
+            lds_slice<C::KSB>(page + koff + 2 * C::PDK, ksh, r.k[1]);
             // register j holds page token 4tg + ((j + tg) & 3): the four lanes of a quad then read
             // rows of alternating parity in one instruction (2-way instead of 4-way bank conflict);
             // the P.V k-slots of a lane may hold its tokens in any order as long as the weights
@@ -684,43 +700,39 @@ attn_mma_kernel(const AttnParams p, int n_items) {
             // with its two halves exchanged for tokens with bit 1 set, so that the four rows a quad
             // reads in one instruction fall into distinct bank groups.
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if constexpr (C::VSB % 4 == 0) lds_slice<C::VSB>(page + vrow[j], 0, r.v[j]);
-                else lds_slice<C::VSB>(page + vrow[j], vidx[j], r.v[j]);
-            }
+            for (int j = 0; j < 4; j++) lds_slice<C::VSB>(page + vrow[j], vsh, r.v[j]);
             r.kn = lds64(page + noff);
             r.vn = lds64(page + noff + (C::OFF_VN - C::OFF_KN));
         };
 
-        // S = K.Q^T of one page (two accumulator chains per head half)
-        auto qk_scores = [&](const Regs& r, float (&c)[NH][2][4]) {
+        // S = K.Q^T of one page (two accumulator chains)
+        auto qk_scores = [&](const Regs& r, float (&c)[2][4]) {
 #pragma unroll
             for (int kb = 0; kb < NKB; kb++) {
                 const uint32_t a0 = lut32(entry_addr<C::IWK>(r.k[0], 2 * kb, lk_lane));
                 const uint32_t a1 = lut32(entry_addr<C::IWK>(r.k[1], 2 * kb, lk_lane));
                 const uint32_t a2 = lut32(entry_addr<C::IWK>(r.k[0], 2 * kb + 1, lk_lane));
                 const uint32_t a3 = lut32(entry_addr<C::IWK>(r.k[1], 2 * kb + 1, lk_lane));
-#pragma unroll
-                for (int hh = 0; hh < NH; hh++) {
-                    uint32_t b0, b1;
-                    if constexpr (C::QSMEM) {
-                        const uint2 qv = lds64(qfrag + ((hh * NKB + kb) * 32 + lane) * 8);
-                        b0 = qv.x; b1 = qv.y;
-                    } else {
-                        b0 = qb[hh][kb][0]; b1 = qb[hh][kb][1];
-                    }
-                    // (the first MMA of each of the two accumulator chains starts from zero)
-                    if (kb < 2) mma_16816_z(c[hh][kb & 1], a0, a1, a2, a3, b0, b1);
-                    else mma_16816(c[hh][kb & 1], a0, a1, a2, a3, b0, b1);
+                uint32_t b0, b1;
+                if constexpr (C::QSMEM) {
+                    const uint2 qv = lds64(qfrag + (kb * 32 + lane) * 8);
+                    b0 = qv.x; b1 = qv.y;
+                } else {
+                    b0 = qb[kb][0]; b1 = qb[kb][1];
                 }
+                // (the first MMA of each of the two accumulator chains starts from zero)
+                if (kb < 2) mma_16816_z(c[kb & 1], a0, a1, a2, a3, b0, b1);
+                else mma_16816(c[kb & 1], a0, a1, a2, a3, b0, b1);
             }
         };
 
-        // online softmax per head (4*hh + tg) over the page's scores (base-2 exponent domain:
-        // the queries carry log2(e)); the weights p * vnorm are rounded to fp16 and transposed
-        // into the B operand of P.V.  FULL = all 16 tokens of the page are valid.
-        auto softmax_update = [&](auto full_tag, const Regs& r, int pg, const float (&c)[NH][2][4],
-                                  uint32_t (&pb)[NH][2][2]) {
+        // online softmax per head over the page's scores (base-2 exponent domain: the queries
+        // carry log2(e)); the weights p * vnorm are rounded to fp16 and transposed into the B
+        // operand of P.V: pb[ks] = k-slots {2tg, 2tg+1} and {2tg+8, 2tg+9} of MMA step ks (one step
+        // of 16 tokens for NH = 2, two of 8 (token, parity) pairs for NH = 1).
+        // FULL = all 16 tokens of the page are valid.
+        auto softmax_update = [&](auto full_tag, const Regs& r, int pg, const float (&c)[2][4],
+                                  uint32_t (&pb)[C::NPB][2]) {
             constexpr bool FULL = decltype(full_tag)::value;
             bool okA = true, okB = true;
             if constexpr (!FULL) {
@@ -737,81 +749,118 @@ attn_mma_kernel(const AttnParams p, int n_items) {
                 vna = okA ? vna : 0.f;
                 vnb = okB ? vnb : 0.f;
             }
+            // columns 2tg, 2tg + 1: two heads (NH = 2) or one head twice
+            float sa[HL], sb[HL];
+            bool above = false;
 #pragma unroll
-            for (int hh = 0; hh < NH; hh++) {
-                float sa = (c[hh][0][0] + c[hh][1][0]) * kna;
-                float sb = (c[hh][0][2] + c[hh][1][2]) * knb;
+            for (int i = 0; i < HL; i++) {
+                sa[i] = (c[0][i] + c[1][i]) * kna;
+                sb[i] = (c[0][2 + i] + c[1][2 + i]) * knb;
                 if constexpr (!FULL) {
-                    sa = okA ? sa : -INFINITY;
-                    sb = okB ? sb : -INFINITY;
+                    sa[i] = okA ? sa[i] : -INFINITY;
+                    sb[i] = okB ? sb[i] : -INFINITY;
                 }
-                // Lazy reference maximum: the cross-lane maximum and the rescale run only when a
-                // score exceeds the reference by more than kLazyMaxSlack (always on the first
-                // page of an item, where it is -inf); weights stay below 2^kLazyMaxSlack.
-                const float mloc = fmaxf(sa, sb);
-                if (__any_sync(0xffffffffu, mloc > m_run[hh] + kLazyMaxSlack)) {
-                    float mx = mloc;
+                above |= fmaxf(sa[i], sb[i]) > m_run[i] + kLazyMaxSlack;
+            }
+            // Lazy reference maximum: the cross-lane maximum and the rescale run only when a
+            // score exceeds the reference by more than kLazyMaxSlack (always on the first
+            // page of an item, where it is -inf); weights stay below 2^kLazyMaxSlack.
+            if (__any_sync(0xffffffffu, above)) {
+                float corr[HL];
+#pragma unroll
+                for (int i = 0; i < HL; i++) {
+                    float mx = fmaxf(sa[i], sb[i]);
                     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
                     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
                     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                    const float m_new = fmaxf(m_run[hh], mx);  // finite: page token 0 is valid
-                    const float corr = fast_exp2(m_run[hh] - m_new);  // 1 if unchanged, 0 from -inf
-                    l_run[hh] *= corr;
-#pragma unroll
-                    for (int mt = 0; mt < NMT; mt++)
-#pragma unroll
-                        for (int i = 0; i < 4; i++) oacc[hh][mt][i] *= corr;
-                    m_run[hh] = m_new;
+                    const float m_new = fmaxf(m_run[i], mx);  // finite: page token 0 is valid
+                    corr[i] = fast_exp2(m_run[i] - m_new);    // 1 if unchanged, 0 from -inf
+                    l_run[i] *= corr[i];
+                    m_run[i] = m_new;
                 }
-                const float pa = fast_exp2(sa - m_run[hh]);  // exp2(-inf) = 0 for masked tokens
-                const float pbv = fast_exp2(sb - m_run[hh]);
-                l_run[hh] += pa + pbv;
-                const uint32_t ha = f2h_sat(pa * vna);
-                const uint32_t hb = f2h_sat(pbv * vnb);
+#pragma unroll
+                for (int mt = 0; mt < NO; mt++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) oacc[mt][i] *= corr[H8 ? (i & 1) : 0];
+            }
+            float wa[HL], wb[HL];
+#pragma unroll
+            for (int i = 0; i < HL; i++) {
+                const float pa = fast_exp2(sa[i] - m_run[i]);  // exp2(-inf) = 0 for masked tokens
+                const float pbv = fast_exp2(sb[i] - m_run[i]);
+                l_run[i] += pa + pbv;
+                wa[i] = pa * vna;
+                wb[i] = pbv * vnb;
+            }
+            uint32_t t0w, t1w;
+            if constexpr (H8) {
+                t0w = movmatrix_trans(f2h2_sat(wa[0], wa[1]));
+                t1w = movmatrix_trans(f2h2_sat(wb[0], wb[1]));
+            } else {
                 // M[token row][column n], both columns of a head equal; transposed, lane (g, tg)
                 // receives head g>>1, page tokens 4tg, 4tg+1 (first) and 4tg+2, 4tg+3 (second)
-                uint32_t t0w = movmatrix_trans(__byte_perm(ha, 0u, 0x1010u));
-                uint32_t t1w = movmatrix_trans(__byte_perm(hb, 0u, 0x1010u));
-                // rotate the four 16-bit weights by tg positions to match the V register order
-                if (tg & 2) { const uint32_t x = t0w; t0w = t1w; t1w = x; }
-                {
-                    const uint32_t sh = (tg & 1) * 16;
-                    const uint32_t lo = __funnelshift_r(t0w, t1w, sh);
-                    const uint32_t hi = __funnelshift_r(t1w, t0w, sh);
-                    t0w = lo;
-                    t1w = hi;
-                }
+                t0w = movmatrix_trans(__byte_perm(f2h_sat(wa[0]), 0u, 0x1010u));
+                t1w = movmatrix_trans(__byte_perm(f2h_sat(wb[0]), 0u, 0x1010u));
+            }
+            // rotate the four 16-bit weights by tg positions to match the V register order
+            if (tg & 2) { const uint32_t x = t0w; t0w = t1w; t1w = x; }
+            {
+                const uint32_t sh = (tg & 1) * 16;
+                const uint32_t lo = __funnelshift_r(t0w, t1w, sh);
+                const uint32_t hi = __funnelshift_r(t1w, t0w, sh);
+                t0w = lo;
+                t1w = hi;
+            }
+            if constexpr (H8) {
+                pb[0][0] = t0w;
+                pb[0][1] = t1w;
+            } else {
                 // column n = (head, parity): an even g keeps the weight in the low half (parity 0
                 // rows of the k index), an odd g in the high half; the other half is zero
-                pb[hh][0][0] = __byte_perm(t0w, 0u, sel_plo);
-                pb[hh][0][1] = __byte_perm(t0w, 0u, sel_phi);
-                pb[hh][1][0] = __byte_perm(t1w, 0u, sel_plo);
-                pb[hh][1][1] = __byte_perm(t1w, 0u, sel_phi);
+                pb[0][0] = __byte_perm(t0w, 0u, sel_plo);
+                pb[0][1] = __byte_perm(t0w, 0u, sel_phi);
+                pb[1][0] = __byte_perm(t1w, 0u, sel_plo);
+                pb[1][1] = __byte_perm(t1w, 0u, sel_phi);
             }
         };
 
-        // O^T += V^T.P^T : rows = d-pairs (D/16)*g + 2*mt + {0,1}, k = (token, parity)
-        auto pv_accum = [&](const uint32_t (&v)[4][(C::VSB + 3) / 4], const uint32_t (&pb)[NH][2][2]) {
+        // values of the code pairs (coordinates (D/8)g + 2 * pair + {0, 1}) of register v[j]
+        auto v_pairs = [&](const uint32_t (&v)[(C::VSB + 3) / 4], int mt, uint32_t& x, uint32_t& y) {
+            if constexpr (C::V2BYTE) {
+                const uint2 e = lut64(entry_addr<8>(v, mt, lv_lane));   // byte mt = pairs 2mt, 2mt + 1
+                x = e.x; y = e.y;
+            } else {
+                x = lut32(entry_addr<C::IWV>(v, 2 * mt, lv_lane));
+                y = lut32(entry_addr<C::IWV>(v, 2 * mt + 1, lv_lane));
+            }
+        };
+        auto pv_accum = [&](const uint32_t (&v)[4][(C::VSB + 3) / 4], const uint32_t (&pb)[C::NPB][2]) {
+            if constexpr (H8) {
+                // O^T += V^T.P^T : rows = coordinates (D/8)g + 2mt, + 1, k = tokens
 #pragma unroll
-            for (int ks = 0; ks < 2; ks++)
+                for (int m2 = 0; m2 < NMT; m2++) {
+                    uint32_t x[4], y[4];
 #pragma unroll
-                for (int mt = 0; mt < NMT; mt++) {
-                    uint32_t a0, a1, a2, a3;
-                    if constexpr (C::V2BYTE) {
-                        // byte mt of a token's slice = its d-pairs 2mt and 2mt + 1
-                        const uint2 lo = lut64(entry_addr<8>(v[2 * ks], mt, lv_lane));
-                        const uint2 hi = lut64(entry_addr<8>(v[2 * ks + 1], mt, lv_lane));
-                        a0 = lo.x; a1 = lo.y; a2 = hi.x; a3 = hi.y;
-                    } else {
-                        a0 = lut32(entry_addr<C::IWV>(v[2 * ks], 2 * mt, lv_lane));
-                        a1 = lut32(entry_addr<C::IWV>(v[2 * ks], 2 * mt + 1, lv_lane));
-                        a2 = lut32(entry_addr<C::IWV>(v[2 * ks + 1], 2 * mt, lv_lane));
-                        a3 = lut32(entry_addr<C::IWV>(v[2 * ks + 1], 2 * mt + 1, lv_lane));
-                    }
-#pragma unroll
-                    for (int hh = 0; hh < NH; hh++)
-                        mma_16816(oacc[hh][mt], a0, a1, a2, a3, pb[hh][ks][0], pb[hh][ks][1]);
+                    for (int j = 0; j < 4; j++) v_pairs(v[j], m2, x[j], y[j]);
+                    mma_16816(oacc[2 * m2], __byte_perm(x[0], x[1], 0x5410u), __byte_perm(x[0], x[1], 0x7632u),
+                              __byte_perm(x[2], x[3], 0x5410u), __byte_perm(x[2], x[3], 0x7632u),
+                              pb[0][0], pb[0][1]);
+                    mma_16816(oacc[2 * m2 + 1], __byte_perm(y[0], y[1], 0x5410u),
+                              __byte_perm(y[0], y[1], 0x7632u), __byte_perm(y[2], y[3], 0x5410u),
+                              __byte_perm(y[2], y[3], 0x7632u), pb[0][0], pb[0][1]);
                 }
+            } else {
+                // rows = d-pairs (D/16)*g + 2*mt + {0,1}, k = (token, parity)
+#pragma unroll
+                for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+                    for (int mt = 0; mt < NMT; mt++) {
+                        uint32_t a0, a1, a2, a3;
+                        v_pairs(v[2 * ks], mt, a0, a1);
+                        v_pairs(v[2 * ks + 1], mt, a2, a3);
+                        mma_16816(oacc[mt], a0, a1, a2, a3, pb[ks][0], pb[ks][1]);
+                    }
+            }
         };
 
         // ---- main loop: the warp's pages; RING bulk copies stay in flight during the math.
@@ -840,18 +889,16 @@ attn_mma_kernel(const AttnParams p, int n_items) {
                 if (lane == 0 && nxt < n_pages && !stalled) issue_page(nxt, rb);
             };
             // all pages but possibly the last one of the chunk are full (warp-uniform branch)
-            auto softmax_page = [&](const Regs& r, int pg2, const float (&c2)[NH][2][4],
-                                    uint32_t (&pb2)[NH][2][2]) {
+            auto softmax_page = [&](const Regs& r, int pg2, const float (&c2)[2][4],
+                                    uint32_t (&pb2)[C::NPB][2]) {
                 if ((pg2 + 1) * kPageTokens <= t1 - t0) softmax_update(std::true_type{}, r, pg2, c2, pb2);
                 else softmax_update(std::false_type{}, r, pg2, c2, pb2);
             };
             Regs ra, rb_;
-            uint32_t pba[NH][2][2], pbb[NH][2][2];
-            float c[NH][2][4];
+            uint32_t pba[C::NPB][2], pbb[C::NPB][2];
+            float c[2][4];
             int pg = warp;
-            // (two head halves already give the scheduler independent work and the extra live
-            // registers would spill: plain order there)
-            constexpr bool kPipelined = (NH == 1 || (D == 256 && !C::QSMEM)) && !C::QSMEM && WARPS <= 16;
+            constexpr bool kPipelined = FTQ_MMA_PIPE;
             if constexpr (!kPipelined) {
                 for (; pg < n_pages; pg += WARPS) {
                     fetch(ra, pg);
@@ -899,67 +946,90 @@ attn_mma_kernel(const AttnParams p, int n_items) {
 
         // ---- fold the warps' states: every warp publishes (m, l, O), NRED warps reduce
 #pragma unroll
-        for (int hh = 0; hh < NH; hh++) {
-            l_run[hh] += __shfl_xor_sync(0xffffffffu, l_run[hh], 4);
-            l_run[hh] += __shfl_xor_sync(0xffffffffu, l_run[hh], 8);
-            l_run[hh] += __shfl_xor_sync(0xffffffffu, l_run[hh], 16);
+        for (int i = 0; i < HL; i++) {
+            l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 4);
+            l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 8);
+            l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 16);
         }
         // a warp whose copy never arrived poisons its state (NaN propagates to the output)
         if (stalled) {
 #pragma unroll
-            for (int hh = 0; hh < NH; hh++) m_run[hh] = __int_as_float(0x7fc00000);
+            for (int i = 0; i < HL; i++) m_run[i] = __int_as_float(0x7fc00000);
             if (lane == 0) atomicOr(p.work_counter + kStatusWord, kStatusWaitExpired);
         }
         __syncthreads();  // every warp is done with the ring: it becomes the exchange area
 #pragma unroll
-        for (int hh = 0; hh < NH; hh++) {
+        for (int mt = 0; mt < NO; mt++)
+            xchg[(warp * NO + mt) * 32 + lane] = make_float4(oacc[mt][0], oacc[mt][1], oacc[mt][2], oacc[mt][3]);
+        if (g == 0) {
 #pragma unroll
-            for (int mt = 0; mt < NMT; mt++)
-                xchg[((warp * NH + hh) * NMT + mt) * 32 + lane] = make_float4(
-                    oacc[hh][mt][0], oacc[hh][mt][1], oacc[hh][mt][2], oacc[hh][mt][3]);
-            if (g == 0) {
-                xml[((warp * NH + hh) * 2 + 0) * 4 + tg] = m_run[hh];
-                xml[((warp * NH + hh) * 2 + 1) * 4 + tg] = l_run[hh];
+            for (int i = 0; i < HL; i++) {
+                xml[(warp * 2 + 0) * (4 * NH) + HL * tg + i] = m_run[i];
+                xml[(warp * 2 + 1) * (4 * NH) + HL * tg + i] = l_run[i];
             }
         }
         __syncthreads();
         if (warp < NRED) {
             float* prow = partial_row(cur);
-            for (int j = tid; j < NH * NMT * 32; j += NRED * 32) {
-                const int ln = j & 31, mt = (j >> 5) % NMT, hh = j / (32 * NMT);
+            for (int j = tid; j < NO * 32; j += NRED * 32) {
+                const int ln = j & 31, mt = j >> 5;
                 const int tg_ = ln & 3, g_ = ln >> 2;
-                float M = -INFINITY;
-                bool nan = bad_item;
+                float M[HL], l[HL];
+                bool nan[HL];
 #pragma unroll
-                for (int w2 = 0; w2 < WARPS; w2++) {
-                    const float mw = xml[((w2 * NH + hh) * 2 + 0) * 4 + tg_];
-                    nan |= mw != mw;   // (fmaxf drops a NaN operand)
-                    M = fmaxf(M, mw);
+                for (int i = 0; i < HL; i++) {
+                    M[i] = -INFINITY;
+                    l[i] = 0.f;
+                    nan[i] = bad_item;
+#pragma unroll
+                    for (int w2 = 0; w2 < WARPS; w2++) {
+                        const float mw = xml[(w2 * 2 + 0) * (4 * NH) + HL * tg_ + i];
+                        nan[i] |= mw != mw;   // (fmaxf drops a NaN operand)
+                        M[i] = fmaxf(M[i], mw);
+                    }
                 }
                 float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-                float l = 0.f;
 #pragma unroll
                 for (int w2 = 0; w2 < WARPS; w2++) {
-                    const float mw = xml[((w2 * NH + hh) * 2 + 0) * 4 + tg_];
-                    if (mw != -INFINITY) {  // (NaN compares unequal: poison goes through)
-                        const float f = fast_exp2(mw - M);
-                        const float4 o = xchg[((w2 * NH + hh) * NMT + mt) * 32 + ln];
-                        a.x = fmaf(o.x, f, a.x);
-                        a.y = fmaf(o.y, f, a.y);
-                        a.z = fmaf(o.z, f, a.z);
-                        a.w = fmaf(o.w, f, a.w);
-                        l = fmaf(xml[((w2 * NH + hh) * 2 + 1) * 4 + tg_], f, l);
+                    float f[HL];
+                    bool some = false;
+#pragma unroll
+                    for (int i = 0; i < HL; i++) {
+                        const float mw = xml[(w2 * 2 + 0) * (4 * NH) + HL * tg_ + i];
+                        const bool has = mw != -INFINITY;  // (NaN compares unequal: poison goes through)
+                        f[i] = has ? fast_exp2(mw - M[i]) : 0.f;
+                        some |= has;
+                        l[i] = fmaf(has ? xml[(w2 * 2 + 1) * (4 * NH) + HL * tg_ + i] : 0.f, f[i], l[i]);
+                    }
+                    if (some) {
+                        const float4 o = xchg[(w2 * NO + mt) * 32 + ln];
+                        a.x = fmaf(o.x, f[0], a.x);
+                        a.y = fmaf(o.y, f[HL - 1], a.y);
+                        a.z = fmaf(o.z, f[0], a.z);
+                        a.w = fmaf(o.w, f[HL - 1], a.w);
                     }
                 }
-                const int h = 4 * hh + tg_;
-                if (h < group) {
-                    float* dst = prow + h * prow_head_stride;
-                    *reinterpret_cast<float4*>(dst + (D / 8) * g_ + 4 * mt) = a;
+                auto put_state = [&](float* dst, int i) {
                     if (g_ == 0 && mt == 0) {
                         // the partial rows carry natural-log maxima; NaN marks a poisoned item
-                        dst[D] = nan ? __int_as_float(0x7fc00000) : M * kLn2;
-                        dst[D + 1] = l;
+                        dst[D] = nan[i] ? __int_as_float(0x7fc00000) : M[i] * kLn2;
+                        dst[D + 1] = l[i];
                     }
+                };
+                if constexpr (H8) {
+                    const float2 o2[2] = {make_float2(a.x, a.z), make_float2(a.y, a.w)};
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        if (2 * tg_ + i < group) {
+                            float* dst = prow + (2 * tg_ + i) * prow_head_stride;
+                            *reinterpret_cast<float2*>(dst + (D / 8) * g_ + 2 * mt) = o2[i];
+                            put_state(dst, i);
+                        }
+                    }
+                } else if (tg_ < group) {
+                    float* dst = prow + tg_ * prow_head_stride;
+                    *reinterpret_cast<float4*>(dst + (D / 8) * g_ + 4 * mt) = a;
+                    put_state(dst, 0);
                 }
             }
         }

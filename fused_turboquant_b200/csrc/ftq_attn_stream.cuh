@@ -638,36 +638,33 @@ attn_stream_kernel(const AttnParams p, int n_items) {
     // Lane constants of the page reads (like the table bases and byte selectors above) are made
     // opaque to the compiler -- an empty asm that "modifies" them: left alone it recomputes them
     // for every page rather than spend registers on them, ~25 instructions per page (measured +4 %).
-    uint32_t koff = (4 * (g >> 1) + (g & 1)) * C::PDK;   // key row rho(g)
+    uint32_t koff = (4 * (g >> 1) + (g & 1)) * C::PDK + slice_word<C::KSB>(tg);   // key row rho(g)
+    const uint32_t ksh = slice_shift<C::KSB>(tg);
     uint32_t noff = C::OFF_KN + 8 * (g >> 1);
     asm volatile("" : "+r"(koff), "+r"(noff));
     auto read_keys = [&](Regs& r, uint32_t page) {
-        lds_slice<C::KSB>(page + koff, tg, r.k[0]);
-        lds_slice<C::KSB>(page + koff + 2 * C::PDK, tg, r.k[1]);
+        lds_slice<C::KSB>(page + koff, ksh, r.k[0]);
+        lds_slice<C::KSB>(page + koff + 2 * C::PDK, ksh, r.k[1]);
         r.kn = lds64(page + noff);
         r.vn = lds64(page + noff + (C::OFF_VN - C::OFF_KN));
     };
     // this lane's four value slices inside a page: register j holds page token 4tg + ((j + tg) & 3),
     // slice g with its halves exchanged for tokens with bit 1 set (the rotation by tg and the
-    // exchanged halves keep the quad's reads conflict-free).  vrow = byte offset of the token's
-    // row (plus the slice where slices are whole words), vidx = slice index otherwise.
+    // exchanged halves keep the quad's reads conflict-free).  vrow = byte offset of the slice's
+    // first word, vsh = its shift (slices that are not whole words).
     uint32_t vrow[4];
-    int vidx[4];
+    uint32_t vsh = slice_shift<C::VSB>(g);
+    if constexpr (C::VSB % 4 != 0) asm volatile("" : "+r"(vsh));
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const int u = (j + tg) & 3;
         const int slice = g ^ ((u & 2) << 1);
-        vrow[j] = C::OFF_VC + (4 * tg + u) * C::PDV + (C::VSB % 4 == 0 ? slice * C::VSB : 0);
-        vidx[j] = C::VSB % 4 == 0 ? 0 : slice;
+        vrow[j] = C::OFF_VC + (4 * tg + u) * C::PDV + slice_word<C::VSB>(slice);
         asm volatile("" : "+r"(vrow[j]));
-        if constexpr (C::VSB % 4 != 0) asm volatile("" : "+r"(vidx[j]));
     }
     auto read_values = [&](Regs& r, uint32_t page) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            if constexpr (C::VSB % 4 == 0) lds_slice<C::VSB>(page + vrow[j], 0, r.v[j]);
-            else lds_slice<C::VSB>(page + vrow[j], vidx[j], r.v[j]);
-        }
+        for (int j = 0; j < 4; j++) lds_slice<C::VSB>(page + vrow[j], vsh, r.v[j]);
     };
 
     // S = K.Q^T of one page (two accumulator chains per head half, the first MMA of a chain

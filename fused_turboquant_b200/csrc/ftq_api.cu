@@ -418,17 +418,6 @@ ChunkPlan plan_two_regions(int64_t units, int64_t slots, int max_seq_len, double
     return pl;
 }
 
-// attn_mma_kernel: the fixed cost of an item (publish / fold / next item's queries between
-// CTA-wide barriers) weighs about 15 pages for a 16-warp CTA and 30 for an 8-warp one (fitted to
-// measured step times of the uniform benchmark shapes).
-ChunkPlan plan_chunks_mma(int B, int Hkv, int max_seq_len, int n_layers, int ctas_per_sm) {
-    const int seq = round_seq(max_seq_len), slots = ftq::sm_count() * ctas_per_sm;
-    return remembered<ChunkPlan>({1, B, 0, Hkv, ctas_per_sm, seq, n_layers, slots}, [&] {
-        return plan_two_regions(static_cast<int64_t>(B) * Hkv * n_layers, slots, seq,
-                                ctas_per_sm == 1 ? 15.0 : 30.0);
-    });
-}
-
 // The streaming kernel.  Measured on B200 (Llama-shaped K4V4 batches of 37..111
 // sequences, forced chunk counts): an item costs about 74 pages on top of its own pages (the
 // service warps' smaller page share, the publish / fold / prepare hand-overs), so long chunks
@@ -747,7 +736,7 @@ static unsigned long long next_epoch() {
 static size_t counter_bytes(int B, int Hkv, int n_layers) {
     const size_t units = static_cast<size_t>(n_layers > 0 ? n_layers : 0) * (B > 0 ? B : 0) *
                          (Hkv > 0 ? Hkv : 0);
-    return (256 + units * sizeof(int) + 255) / 256 * 256;
+    return (256 + 2 * units * sizeof(int) + 255) / 256 * 256;
 }
 
 size_t ftq_decode_workspace_bytes(int B, int Hq, int Hkv, int head_dim, int max_seq_len,
@@ -758,14 +747,14 @@ size_t ftq_decode_workspace_bytes(int B, int Hq, int Hkv, int head_dim, int max_
     return remembered<size_t>({0, B, Hq, Hkv, head_dim, seq, n_layers, ftq::sm_count()}, [&] {
         size_t n = 0;
         for (const ChunkPlan& pl : {plan_chunks(B, Hq, Hkv, head_dim, seq, n_layers),
-                                    plan_chunks_mma(B, Hkv, seq, n_layers, 1),
-                                    plan_chunks_mma(B, Hkv, seq, n_layers, 2),
                                     plan_chunks_stream(B, Hkv, seq, n_layers, 1),
                                     plan_chunks_stream(B, Hkv, seq, n_layers, 2)}) {
             const size_t m = partial_bytes(pl, B, Hq, head_dim, n_layers);
             n = m > n ? m : n;
         }
-        return n;
+        // the equal-share kernel: two blocks of rows per CTA, at most two CTAs per SM
+        const size_t flow = static_cast<size_t>(ftq::sm_count()) * 4 * (Hq / Hkv) * (head_dim + 4) * sizeof(float);
+        return flow > n ? flow : n;
     }) + counter_bytes(B, Hkv, n_layers);
 }
 
@@ -898,12 +887,10 @@ int ftq_paged_decode_attn(const void* q, int q_dtype, void* out, int out_dtype,
     // 16-bit queries with a GQA group of at most 8 take the tensor-core kernel; fp32 queries
     // (and larger groups) take the fp32 kernel.
     const bool mma = use_mma_path(Hq, Hkv, q_dtype);
-    // one CTA per SM (16 warps) when a 4-bit byte table is in use, else two (8 warps each)
-    const int mma_ctas = (bits_k == 4 || bits_v == 4) ? 1 : 2;
     const int stream_ctas = mma ? attn_mma_stream_ctas(head_dim, bits_k, bits_v, Hq / Hkv) : 0;
     const bool streams = stream_ctas > 0;
     const ChunkPlan pl = streams ? plan_chunks_stream(B, Hkv, max_seq_len, n_layers, stream_ctas)
-                         : mma   ? plan_chunks_mma(B, Hkv, max_seq_len, n_layers, mma_ctas)
+                         : mma   ? ChunkPlan{}
                                  : plan_chunks(B, Hq, Hkv, head_dim, round_seq(max_seq_len), n_layers);
     const size_t need = ftq_decode_workspace_bytes(B, Hq, Hkv, head_dim, max_seq_len, n_layers);
     if (!workspace || workspace_bytes < need)
@@ -946,12 +933,13 @@ int ftq_paged_decode_attn(const void* q, int q_dtype, void* out, int out_dtype,
         p.out = out;
         p.out_dtype = out_dtype;
         p.num_blocks = num_blocks;
-        p.div_chunks = ftq::make_fastdiv(static_cast<uint32_t>(p.n_chunks));
         p.div_hkv = ftq::make_fastdiv(static_cast<uint32_t>(Hkv));
         p.div_b = ftq::make_fastdiv(static_cast<uint32_t>(B));
         p.n_units = n_layers * B * Hkv;
         p.epoch = next_epoch();
-        p.split = make_split(pl, p.n_units, true);
+        p.n_layers = n_layers;
+        p.max_seq = max_seq_len;
+        if (streams) p.split = make_split(pl, p.n_units, true);
         bool merged = false;
         e = dispatch_mma(head_dim, bits_k, bits_v, shared_lut, p, n_layers * B, st, &merged);
         if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_decode_attn launch");

@@ -90,10 +90,14 @@ struct AttnParams {
     int* unit_counter;          // [n_units = L*B*Hkv] chunks delivered per unit
     int n_units;
     unsigned long long epoch;
+    // equal-share tensor-core kernel: sequences b0 .. b0 + B - 1 of the batch's B_stride, n_layers
+    // layers; context lengths are cut to max_seq; pages per CTA at least min_share; unit_counter
+    // holds two counters per unit
+    int n_layers, b0, B_stride, max_seq, min_share;
     void* out;                  // [L*B, Hq, D]
     int out_dtype;
     int64_t num_blocks;         // block ids are checked against it
-    FastDiv div_chunks, div_hkv, div_b;  // divisions by n_chunks, Hkv, B
+    FastDiv div_hkv, div_b;     // divisions by Hkv, B
     Codebook lk, lv;
     SignBits signs;
     float rsqrt_d;

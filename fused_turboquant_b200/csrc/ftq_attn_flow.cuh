@@ -1,0 +1,896 @@
+// Paged decode attention on the tensor cores: every CTA owns an equal share of the batch's pages.
+//
+// Arithmetic, tables, page layout and fragment maps: ftq_attn_mma.cuh (the fused formulation of
+// src/fused_turboquant/kernels/triton_flash_decode.py:33-324 of the reference, with the query
+// rotation of hf/fused_cache.py:579-581 and the page-table walk of vllm_plugin/cache_ops.py:151-205
+// folded in).  This file: how the work is split and put together again.
+//
+// The pages of all (layer, sequence, KV head) units lie in one line, unit after unit, and CTA c of
+// the persistent grid takes pages [c * share, (c + 1) * share): all CTAs have the same amount of
+// work whatever the lengths of the sequences are, a CTA's share crosses unit borders in at most
+// units / CTAs + 2 pieces, and a unit is cut only where a share ends.  (Cutting every unit into
+// equal chunks instead left the last wave of chunks up to half empty and paid the fixed cost of a
+// piece -- rotate the queries, fold the warps' states, about as long as 30 pages -- for every
+// chunk: 1.4 to 1.8 ms per 1000 pages and SM against 1.0 to 1.2 here.)  The partition needs the
+// prefix sums of the page counts, which every CTA computes from seq_lens at its start.
+//
+// A piece is walked by the CTA's warps in stages of NP consecutive pages, dealt round-robin.  A
+// warp keeps RING stages in flight (1-D bulk copies, TMA); block ids are read straight from the
+// block table, a batch of 32 per warp, one batch ahead.  The first stages of the next piece are
+// requested before this piece's states are folded.
+//
+// Pieces of a cut unit leave (O, m, l) rows in the workspace (two row blocks per CTA: a CTA's first
+// and last piece can be parts of units) and count themselves in; whoever arrives last merges the
+// rows, rotates back (core/hadamard.py:93-100) and stores.  A unit that one piece covers is
+// finished from shared memory.  Nobody waits for anybody.  The counters are cleared by CTA 0 under
+// the launch's epoch, as described at AttnParams.
+//
+// Every wait is bounded (mbar_wait, the epoch); a wait that runs out turns the unit's rows into NaN
+// and sets a bit of the status word.  Block ids outside [0, num_blocks) are never dereferenced.
+#pragma once
+
+#include "ftq_attn_mma.cuh"
+
+namespace ftq {
+
+constexpr int kEpochSpinLimit = 1 << 22;
+
+// A piece of a CTA's share: pages [page0, page0 + n_pages) of one unit (n_pages = 0: none left).
+struct FlowPiece {
+    int64_t unit_start;   // first page of the unit on the line of all pages
+    int64_t next;         // where the next piece starts
+    int unit_pages, layer, b, hkv, page0, n_pages, tokens;
+};
+
+template <int D, int BK, int BV, bool SHARED_LUT, int NH>
+__global__ void __launch_bounds__(MmaCfg<D, BK, BV, NH>::THREADS, MmaCfg<D, BK, BV, NH>::CTAS_PER_SM)
+attn_flow_kernel(const __grid_constant__ AttnParams p) {
+    using C = MmaCfg<D, BK, BV, NH>;
+    constexpr int NKB = C::NKB, NMT = C::NMT, WARPS = C::WARPS, THREADS = C::THREADS, NP = C::NP;
+    constexpr int E = D / kOctet;
+    constexpr int ROW = D + 4;
+    constexpr int IDS = 32 / NP;   // stages per batch of block ids
+
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw));
+    // ---- carve shared memory (addresses in the shared window): the byte table needs a
+    // 64 KB-aligned window; the other objects go first-fit before or after it
+    uint32_t window = 0, free0 = sbase, end0 = sbase, free1 = sbase;
+    if constexpr (C::BYTE) {
+        window = (sbase + 65535u) & ~65535u;
+        end0 = window;
+        free1 = window + 65536u;
+    }
+    auto take = [&](uint32_t bytes) {
+        uint32_t a = (free0 + 127u) & ~127u;
+        if (a + bytes <= end0) { free0 = a + bytes; return a; }
+        a = (free1 + 127u) & ~127u;
+        free1 = a + bytes;
+        return a;
+    };
+    auto gptr = [&](uint32_t saddr) { return smem_raw + (saddr - sbase); };
+    const uint32_t misc = take(C::MISC_BYTES + WARPS * C::XML);
+    uint32_t tk_small = 0, tv_small = 0, cur_addr = misc;
+    if constexpr (C::SMALL_ALIGN > 0) {
+        cur_addr = (misc + C::SMALL_ALIGN - 1) & ~static_cast<uint32_t>(C::SMALL_ALIGN - 1);
+        if (C::TKS >= C::TVS) { tk_small = cur_addr; tv_small = cur_addr + C::TKS; }
+        else { tv_small = cur_addr; tk_small = cur_addr + C::TVS; }
+        cur_addr += C::TKS + C::TVS;
+        if (SHARED_LUT) tv_small = tk_small;
+    }
+    cur_addr = (cur_addr + 15u) & ~15u;
+    float* qs = reinterpret_cast<float*>(gptr(cur_addr));             // [8][D + 16] rotated queries
+    float* folded = qs + 8 * (D + 16);                                // [4 * NH][ROW] the piece's (O, m, l)
+    int* prefix = reinterpret_cast<int*>(folded + 4 * NH * ROW);      // [B + 1] page counts, summed up
+    float* xml = reinterpret_cast<float*>(prefix + kFlowMaxSeqs + 4); // [WARPS][2][4 * NH]
+    const uint32_t bars = cur_addr + 8 * (D + 16) * 4 + 4 * NH * ROW * 4 + (kFlowMaxSeqs + 4) * 4 +
+                          WARPS * C::XML;                             // [WARPS][RING] x 8 bytes
+    uint32_t* ring_at = reinterpret_cast<uint32_t*>(gptr(bars + WARPS * C::RING * 8));  // [WARPS]
+    const uint32_t xarea = C::SEP ? take(WARPS * C::XSLOT) : 0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < WARPS; w++) ring_at[w] = take(C::ring_bytes(NP, C::SEP));
+    // warp w's share of the merge exchange area
+    auto xchg = [&](int w) {
+        return reinterpret_cast<float4*>(gptr(C::SEP ? xarea + w * C::XSLOT : ring_at[w]));
+    };
+
+    // the next kernel of the stream may start its own set-up as soon as every CTA got here
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const int tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, tg = lane & 3;
+    const bool odd = g & 1;
+    const int group = p.Hq / p.Hkv;  // <= 4 * NH
+    constexpr bool H8 = C::H8;
+    constexpr int NO = C::STATE_F4;  // accumulator tiles per lane
+    constexpr int HL = C::HL;
+    // byte selectors (source 4 = a zero byte): a lane's own fp16 of a packed pair, and the
+    // placement of a weight in the low (even g) or high (odd g) half of a B register
+    uint32_t sel_own = odd ? 0x4432u : 0x4410u;
+    uint32_t sel_plo = odd ? 0x1044u : 0x4410u;
+    uint32_t sel_phi = odd ? 0x3244u : 0x4432u;
+    // Lane constants of the page reads: byte offset of the key row rho(g) and of the norm quad;
+    // per value register j the first word of slice g in the row of page token 4tg + ((j + tg) & 3)
+    // (halves exchanged for tokens with bit 1 set).
+    uint32_t koff = (4 * (g >> 1) + (g & 1)) * C::PDK + slice_word<C::KSB>(tg);
+    const uint32_t ksh = slice_shift<C::KSB>(tg);
+    uint32_t noff = C::OFF_KN + 8 * (g >> 1);
+    uint32_t vrow[4];
+    const uint32_t vsh = slice_shift<C::VSB>(g);   // (the same for the exchanged slice g ^ 4)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int u = C::ROT ? (j + tg) & 3 : j;
+        const int slice = g ^ ((u & 2) << 1);
+        vrow[j] = C::OFF_VC + (4 * tg + u) * C::PDV + slice_word<C::VSB>(slice);
+    }
+
+    // ---- once per CTA: dequantisation tables.  A lane keeps one level of each codebook; a row (32
+    // copies of an entry) is two shuffles, a conversion and one store.
+    {
+        const float lev_k = p.lk.v[lane & 15], lev_v = p.lv_scaled.v[lane & 15];
+        auto pair = [&](float lev, int lo, int hi) {
+            const __half2 h = __floats2half2_rn(__shfl_sync(0xffffffffu, lev, lo), __shfl_sync(0xffffffffu, lev, hi));
+            return *reinterpret_cast<const uint32_t*>(&h);
+        };
+        if constexpr (C::BYTE) {
+            uint32_t* tb = reinterpret_cast<uint32_t*>(gptr(window));
+#pragma unroll 4
+            for (int e = warp; e < 256; e += WARPS) {
+                if constexpr (BK == 4) tb[e * 64 + lane] = pair(lev_k, e & 15, e >> 4);
+                if constexpr (BV == 4 && !SHARED_LUT) tb[e * 64 + 32 + lane] = pair(lev_v, e & 15, e >> 4);
+                if constexpr (C::V2BYTE) {
+                    const uint32_t x = pair(lev_v, e & 3, (e >> 2) & 3), y = pair(lev_v, (e >> 4) & 3, e >> 6);
+                    tb[e * 64 + 32 + lane] = (lane & 1) ? y : x;
+                }
+            }
+        }
+        if constexpr (BK != 4) {
+            uint32_t* t = reinterpret_cast<uint32_t*>(gptr(tk_small));
+            for (int e = warp; e < (1 << C::IWK); e += WARPS)
+                t[e * 32 + lane] = pair(lev_k, e & ((1 << BK) - 1), e >> BK);
+        }
+        if constexpr (BV != 4 && !SHARED_LUT && !C::V2BYTE) {
+            uint32_t* t = reinterpret_cast<uint32_t*>(gptr(tv_small));
+            for (int e = warp; e < (1 << C::IWV); e += WARPS)
+                t[e * 32 + lane] = pair(lev_v, e & ((1 << BV) - 1), e >> BV);
+        }
+    }
+    const uint32_t lk_lane = (BK == 4 ? window : tk_small) | (lane * 4);
+    const uint32_t lv_lane =
+        C::V2BYTE ? (window | 128u | ((lane & 15) * 8))
+                  : ((BV == 4 ? (window | (SHARED_LUT ? 0u : 128u)) : tv_small) | (lane * 4));
+    // one mbarrier per ring buffer (a single arrival + the copies' bytes)
+    const uint32_t my_bars = bars + warp * C::RING * 8;
+    if (lane == 0) {
+#pragma unroll
+        for (int r = 0; r < C::RING; r++) mbar_init(my_bars + r * 8, 1);
+    }
+    mbar_fence_init();
+    __shared__ int s_bad[3];   // by piece number mod 3: a block id of the piece was out of range
+    if (tid < 3) s_bad[tid] = 0;
+
+    // Everything up to here touched shared memory only.  From here on the kernel reads and writes
+    // global memory that the kernel before it in the stream may still be using.
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    unsigned long long* epoch_word = reinterpret_cast<unsigned long long*>(p.work_counter + 2);
+    if (blockIdx.x == 0) {
+        for (int i = tid; i < 2 * p.n_units; i += THREADS) p.unit_counter[i] = 0;
+        if (tid == 0) {
+            p.work_counter[1] = 0;
+            p.work_counter[kStatusWord] = 0;
+        }
+    }
+    // prefix sums of the page counts (lengths beyond the host's bound are cut to it)
+    auto tokens_of = [&](int b) { return max(0, min(p.seq_lens[b], p.max_seq)); };
+    if (warp == 0) {
+        int carry = 0;
+        for (int b0 = 0; b0 < p.B; b0 += 32) {
+            const int b = b0 + lane;
+            int x = b < p.B ? (tokens_of(b) + kPageTokens - 1) / kPageTokens : 0;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d) x += y;
+            }
+            if (b < p.B) prefix[b + 1] = carry + x;
+            carry += __shfl_sync(0xffffffffu, x, 31);
+        }
+        if (lane == 0) prefix[0] = 0;
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && tid == 0) {
+        __threadfence();
+        asm volatile("st.release.gpu.global.u64 [%0], %1;\n" ::"l"(epoch_word), "l"(p.epoch) : "memory");
+    }
+    bool stalled = false; // a wait of this warp ran out: no more waiting, its results become NaN
+    bool epoch_seen = false;
+    // the counters and the status word are valid once CTA 0 has published this launch's epoch (by the
+    // time anybody asks it has normally been there for long)
+    auto await_epoch = [&]() {
+        if (epoch_seen) return;
+        epoch_seen = true;
+        for (int i = 0; i < kEpochSpinLimit; i++) {
+            unsigned long long v;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(epoch_word) : "memory");
+            if (v == p.epoch) return;
+            __nanosleep(100);
+        }
+        stalled = true;
+    };
+
+    // ---- this CTA's share of the pages, and the piece that starts at a given page
+    const int per_layer = prefix[p.B] * p.Hkv;
+    const int64_t total = static_cast<int64_t>(per_layer) * p.n_layers;
+    int64_t share = (total + gridDim.x - 1) / gridDim.x;
+    share = share > p.min_share ? share : p.min_share;
+    const int64_t first = share * blockIdx.x;
+    const int64_t end = first + share < total ? first + share : total;
+    auto locate = [&](int64_t pos) {
+        FlowPiece it{};
+        it.next = pos;
+        if (pos >= end) return it;
+        int r;
+        if (p.n_layers == 1) {
+            it.layer = 0;
+            r = static_cast<int>(pos);
+        } else {
+            it.layer = static_cast<int>(pos / per_layer);
+            r = static_cast<int>(pos - static_cast<int64_t>(it.layer) * per_layer);
+        }
+        int lo = 0, hi = p.B;    // prefix[lo] * Hkv <= r < prefix[hi] * Hkv
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (prefix[mid] * p.Hkv <= r) lo = mid; else hi = mid;
+        }
+        it.b = lo;
+        it.unit_pages = prefix[lo + 1] - prefix[lo];
+        r -= prefix[lo] * p.Hkv;
+        it.hkv = r / it.unit_pages;
+        it.page0 = r - it.hkv * it.unit_pages;
+        it.unit_start = pos - it.page0;
+        const int64_t room = end - pos;
+        it.n_pages = it.unit_pages - it.page0;
+        if (it.n_pages > room) it.n_pages = static_cast<int>(room);
+        it.tokens = min(tokens_of(lo) - it.page0 * kPageTokens, it.n_pages * kPageTokens);
+        it.next = pos + it.n_pages;
+        return it;
+    };
+    // The pieces of the share, by number mod 3: this one, the next one and the one after are known (one
+    // thread looks for them, between two barriers).
+    __shared__ FlowPiece s_piece[3];
+    if (tid == 0) {
+        s_piece[0] = locate(first);
+        s_piece[1] = locate(s_piece[0].next);
+    }
+    __syncthreads();
+
+    // ---- pages: block ids and bulk copies
+    const uint32_t my_ring = ring_at[warp];
+    const uint32_t blk_stride = static_cast<uint32_t>(p.Hkv) * C::PAGE_BYTES;
+    const uint64_t page_policy = l2_evict_first_policy();   // (pages are read once per step)
+    uint32_t phase = 0;   // bit r = parity the next wait on ring buffer r expects
+    int ring_it = 0;      // stages this warp has taken from its ring so far (buffer = ring_it % RING)
+#ifdef FTQ_TEST_WAIT_EXPIRY
+    bool test_drop = blockIdx.x == 0 && warp == 5;
+#endif
+    // stages of a piece that are this warp's: warp, warp + WARPS, ...
+    auto my_stages = [&](const FlowPiece& it) {
+        const int n = (it.n_pages + NP - 1) / NP - warp;
+        return n > 0 ? (n + WARPS - 1) / WARPS : 0;
+    };
+    // block ids of this warp's stages k0 .. k0 + IDS - 1: lane NP * j + i holds page i of stage k0 + j
+    // (an id outside the pool is replaced by 0 and remembered)
+    auto load_ids = [&](const FlowPiece& it, int k0, int slot) {
+        const int pg = (warp + (k0 + lane / NP) * WARPS) * NP + lane % NP;
+        int id = 0;
+        if (pg < it.n_pages) {
+            id = __ldg(p.block_table + static_cast<int64_t>(it.b) * p.max_blocks + it.page0 + pg);
+            if (static_cast<uint32_t>(id) >= static_cast<uint64_t>(p.num_blocks)) {
+                id = 0;
+                s_bad[slot] = 1;
+            }
+        }
+        return id;
+    };
+    auto head_base = [&](const FlowPiece& it) {
+        return p.pool + it.layer * p.pool_layer_stride + static_cast<int64_t>(it.hkv) * C::PAGE_BYTES;
+    };
+    // start the copies of the warp's stage k into ring buffer rb: lane i copies page i, lane 0
+    // announces the bytes of all of them
+    auto issue_stage = [&](const uint8_t* base, int ids, int n_pages, int k, int rb) {
+        const int here = min(NP, n_pages - (warp + k * WARPS) * NP);
+        const uint32_t id = __shfl_sync(0xffffffffu, ids, (k % IDS) * NP + lane % NP);
+        if (lane == 0) mbar_expect_tx(my_bars + rb * 8, here * C::PAGE_BYTES);
+        __syncwarp();
+#ifdef FTQ_TEST_WAIT_EXPIRY
+        if (test_drop) {   // (see kMbarSpinLimit)
+            test_drop = false;
+            if (lane == 0) return;
+        }
+#endif
+        if (lane < here)
+            bulk_g2s_hint(my_ring + rb * C::STAGE_BYTES + lane * C::PAGE_BYTES,
+                          base + static_cast<uint64_t>(id) * blk_stride, C::PAGE_BYTES, my_bars + rb * 8,
+                          page_policy);
+    };
+
+    // ---- queries: rotated, pre-scaled, in shared memory: head rows of D + 16 floats, each quarter of
+    // a row padded by 4, so that the 16 distinct float4 a fragment load touches are 2-way at worst
+    auto qs_index = [](int head, int coord) {
+        return head * (D + 16) + (coord / (D / 4)) * (D / 4 + 4) + coord % (D / 4);
+    };
+    auto head_row = [&](const FlowPiece& it) {   // first query head of the piece, as a row of q and out
+        return (static_cast<int64_t>(it.layer) * p.B_stride + p.b0 + it.b) * p.Hq + it.hkv * group;
+    };
+    // run by warps w0 and w0 + 1 (8 octets rotate the at most 8 heads)
+    auto rotate_queries = [&](const FlowPiece& it, int w0) {
+        if (warp < w0 || warp - w0 >= NH) return;
+        const int t8 = lane & 7, o = lane >> 3;
+        const int hh = (warp - w0) * 4 + o;
+        const bool hv = hh < group;
+        const int64_t qoff = (head_row(it) + (hv ? hh : 0)) * D;
+        float a[E];
+#pragma unroll
+        for (int i = 0; i < E / 8; i++) {
+            float tmp[8];
+            const int64_t eo = qoff + 8 * (t8 + 8 * i);
+            if (p.q_dtype == kBF16) load8<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.q) + eo, tmp);
+            else load8<__half>(static_cast<const __half*>(p.q) + eo, tmp);
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                a[8 * i + c] = __uint_as_float(
+                    __float_as_uint(tmp[c]) ^ sign_mask(p.signs, load_coord(t8, 8 * i + c)));
+        }
+        octet_fwht<E>(a, lane);
+#pragma unroll
+        for (int k = 0; k < E; k++)
+            qs[qs_index(hh, t8 + 8 * k)] = hv ? a[k] * p.rsqrt_d * (p.scale * kLog2e) : 0.f;
+    };
+
+    // ---- per-piece arithmetic state of a lane: query fragments, softmax state of heads
+    // HL*tg + {0 .. HL-1}, O[head][(D/8)*g .. + D/8)
+    uint32_t qb[C::QSMEM ? 1 : NKB][2];
+    const uint32_t qfrag = static_cast<uint32_t>(__cvta_generic_to_shared(qs));   // [kb][lane] x 8 bytes (QSMEM)
+    float m_run[HL], l_run[HL], oacc[NO][4];
+
+    // a lane's slices of the staged page at `page`
+    auto read_keys = [&](uint32_t (&k)[2][C::KW], uint32_t page) {
+        lds_slice<C::KSB>(page + koff, ksh, k[0]);
+        lds_slice<C::KSB>(page + koff + 2 * C::PDK, ksh, k[1]);
+    };
+    auto read_values = [&](uint32_t (&v)[4][C::VW], uint32_t page) {
+        // register j holds page token 4tg + ((j + tg) & 3) where ROT is set: the four lanes of a
+        // quad then read rows of alternating parity in one instruction; the P.V k-slots of a lane may hold its tokens in any order as long as the weights
+        // follow (see the rotation of the transposed weights below).  The pool stores a V row
+        // with its two halves exchanged for tokens with bit 1 set, so that the four rows a quad
+        // reads in one instruction fall into distinct bank groups.
+#pragma unroll
+        for (int j = 0; j < 4; j++) lds_slice<C::VSB>(page + vrow[j], vsh, v[j]);
+    };
+
+    // S = K.Q^T of NP pages (two accumulator chains each)
+    auto qk_scores = [&](const uint32_t (&k)[C::NP][2][C::KW], float (&c)[C::NP][2][4]) {
+#pragma unroll
+        for (int kb = 0; kb < NKB; kb++) {
+            uint32_t b0, b1;
+            if constexpr (C::QSMEM) {
+                const uint2 qv = lds64(qfrag + (kb * 32 + lane) * 8);
+                b0 = qv.x; b1 = qv.y;
+            } else {
+                b0 = qb[kb][0]; b1 = qb[kb][1];
+            }
+#pragma unroll
+            for (int i = 0; i < NP; i++) {
+                const uint32_t a0 = lut32(entry_addr<C::IWK>(k[i][0], 2 * kb, lk_lane));
+                const uint32_t a1 = lut32(entry_addr<C::IWK>(k[i][1], 2 * kb, lk_lane));
+                const uint32_t a2 = lut32(entry_addr<C::IWK>(k[i][0], 2 * kb + 1, lk_lane));
+                const uint32_t a3 = lut32(entry_addr<C::IWK>(k[i][1], 2 * kb + 1, lk_lane));
+                // (the first MMA of each of the two accumulator chains starts from zero)
+                if (kb < 2) mma_16816_z(c[i][kb & 1], a0, a1, a2, a3, b0, b1);
+                else mma_16816(c[i][kb & 1], a0, a1, a2, a3, b0, b1);
+            }
+        }
+    };
+
+    // online softmax per head over the scores of NP pages (base-2 exponent domain: the queries
+    // carry log2(e)); the weights p * vnorm are rounded to fp16 and transposed into the B
+    // operand of P.V: pb[i][ks] = k-slots {2tg, 2tg+1} and {2tg+8, 2tg+9} of page i's MMA step ks
+    // (one step of 16 tokens for NH = 2, two of 8 (token, parity) pairs for NH = 1).
+    // FULL = all tokens of the pages are valid.
+    auto softmax_update = [&](auto full_tag, const uint2 (&kn)[C::NP], const uint2 (&vn)[C::NP], int st, int tokens,
+                              const float (&c)[C::NP][2][4], uint32_t (&pb)[C::NP][C::NPB][2]) {
+        constexpr bool FULL = decltype(full_tag)::value;
+        // columns 2tg, 2tg + 1: two heads (NH = 2) or one head twice
+        float sa[C::NP][HL], sb[C::NP][HL];
+        bool okA[C::NP], okB[C::NP];
+        float mx[HL];
+#pragma unroll
+        for (int h = 0; h < HL; h++) mx[h] = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < NP; i++) {
+            if constexpr (!FULL) {
+                const int ntok = tokens - (st * NP + i) * kPageTokens;
+                const int tokA = 4 * (g >> 1) + (g & 1);  // rows g, g+8 of S: tokens tokA, tokA + 2
+                okA[i] = tokA < ntok;
+                okB[i] = tokA + 2 < ntok;
+            }
+            const float kna = half_bits_to_float(__byte_perm(kn[i].x, 0u, sel_own));
+            const float knb = half_bits_to_float(__byte_perm(kn[i].y, 0u, sel_own));
+#pragma unroll
+            for (int h = 0; h < HL; h++) {
+                sa[i][h] = (c[i][0][h] + c[i][1][h]) * kna;
+                sb[i][h] = (c[i][0][2 + h] + c[i][1][2 + h]) * knb;
+                if constexpr (!FULL) {
+                    sa[i][h] = okA[i] ? sa[i][h] : -INFINITY;
+                    sb[i][h] = okB[i] ? sb[i][h] : -INFINITY;
+                }
+                mx[h] = fmaxf(mx[h], fmaxf(sa[i][h], sb[i][h]));
+            }
+        }
+        bool above = false;
+#pragma unroll
+        for (int h = 0; h < HL; h++) above |= mx[h] > m_run[h] + kLazyMaxSlack;
+        // Lazy reference maximum: the cross-lane maximum and the rescale run only when a
+        // score exceeds the reference by more than kLazyMaxSlack (always on the first
+        // stage of an item, where it is -inf); weights stay below 2^kLazyMaxSlack.
+        if (__any_sync(0xffffffffu, above)) {
+            float corr[HL];
+#pragma unroll
+            for (int h = 0; h < HL; h++) {
+                float m = mx[h];
+                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+                const float m_new = fmaxf(m_run[h], m);   // finite: the stage's token 0 is valid
+                corr[h] = fast_exp2(m_run[h] - m_new);    // 1 if unchanged, 0 from -inf
+                l_run[h] *= corr[h];
+                m_run[h] = m_new;
+            }
+#pragma unroll
+            for (int mt = 0; mt < NO; mt++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) oacc[mt][i] *= corr[H8 ? (i & 1) : 0];
+        }
+#pragma unroll
+        for (int i = 0; i < NP; i++) {
+        float vna = half_bits_to_float(__byte_perm(vn[i].x, 0u, sel_own));
+        float vnb = half_bits_to_float(__byte_perm(vn[i].y, 0u, sel_own));
+        if constexpr (!FULL) {
+            vna = okA[i] ? vna : 0.f;
+            vnb = okB[i] ? vnb : 0.f;
+        }
+        float wa[HL], wb[HL];
+#pragma unroll
+        for (int h = 0; h < HL; h++) {
+            const float pa = fast_exp2(sa[i][h] - m_run[h]);  // exp2(-inf) = 0 for masked tokens
+            const float pbv = fast_exp2(sb[i][h] - m_run[h]);
+            l_run[h] += pa + pbv;
+            wa[h] = pa * vna;
+            wb[h] = pbv * vnb;
+        }
+        uint32_t t0w, t1w;
+        if constexpr (H8) {
+            t0w = movmatrix_trans(f2h2_sat(wa[0], wa[1]));
+            t1w = movmatrix_trans(f2h2_sat(wb[0], wb[1]));
+        } else {
+            // M[token row][column n], both columns of a head equal; transposed, lane (g, tg)
+            // receives head g>>1, page tokens 4tg, 4tg+1 (first) and 4tg+2, 4tg+3 (second)
+            t0w = movmatrix_trans(__byte_perm(f2h_sat(wa[0]), 0u, 0x1010u));
+            t1w = movmatrix_trans(__byte_perm(f2h_sat(wb[0]), 0u, 0x1010u));
+        }
+        // rotate the four 16-bit weights by tg positions to match the V register order
+        if constexpr (C::ROT) {
+            if (tg & 2) { const uint32_t x = t0w; t0w = t1w; t1w = x; }
+            const uint32_t sh = (tg & 1) * 16;
+            const uint32_t lo = __funnelshift_r(t0w, t1w, sh);
+            const uint32_t hi = __funnelshift_r(t1w, t0w, sh);
+            t0w = lo;
+            t1w = hi;
+        }
+        if constexpr (H8) {
+            pb[i][0][0] = t0w;
+            pb[i][0][1] = t1w;
+        } else {
+            // column n = (head, parity): an even g keeps the weight in the low half (parity 0
+            // rows of the k index), an odd g in the high half; the other half is zero
+            pb[i][0][0] = __byte_perm(t0w, 0u, sel_plo);
+            pb[i][0][1] = __byte_perm(t0w, 0u, sel_phi);
+            pb[i][1][0] = __byte_perm(t1w, 0u, sel_plo);
+            pb[i][1][1] = __byte_perm(t1w, 0u, sel_phi);
+        }
+        }
+    };
+
+    // values of the code pairs (coordinates (D/8)g + 2 * pair + {0, 1}) of register v[j]
+    auto v_pairs = [&](const uint32_t (&v)[C::VW], int mt, uint32_t& x, uint32_t& y) {
+        if constexpr (C::V2BYTE) {
+            const uint2 e = lut64(entry_addr<8>(v, mt, lv_lane));   // byte mt = pairs 2mt, 2mt + 1
+            x = e.x; y = e.y;
+        } else {
+            x = lut32(entry_addr<C::IWV>(v, 2 * mt, lv_lane));
+            y = lut32(entry_addr<C::IWV>(v, 2 * mt + 1, lv_lane));
+        }
+    };
+    auto pv_accum = [&](const uint32_t (&v)[4][C::VW], const uint32_t (&pb)[C::NPB][2]) {
+        if constexpr (H8) {
+            // O^T += V^T.P^T : rows = coordinates (D/8)g + 2mt, + 1, k = tokens
+#pragma unroll
+            for (int m2 = 0; m2 < NMT; m2++) {
+                uint32_t x[4], y[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) v_pairs(v[j], m2, x[j], y[j]);
+                mma_16816(oacc[2 * m2], __byte_perm(x[0], x[1], 0x5410u), __byte_perm(x[0], x[1], 0x7632u),
+                          __byte_perm(x[2], x[3], 0x5410u), __byte_perm(x[2], x[3], 0x7632u),
+                          pb[0][0], pb[0][1]);
+                mma_16816(oacc[2 * m2 + 1], __byte_perm(y[0], y[1], 0x5410u),
+                          __byte_perm(y[0], y[1], 0x7632u), __byte_perm(y[2], y[3], 0x5410u),
+                          __byte_perm(y[2], y[3], 0x7632u), pb[0][0], pb[0][1]);
+            }
+        } else {
+            // rows = d-pairs (D/16)*g + 2*mt + {0,1}, k = (token, parity)
+#pragma unroll
+            for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+                for (int mt = 0; mt < NMT; mt++) {
+                    uint32_t a0, a1, a2, a3;
+                    v_pairs(v[2 * ks], mt, a0, a1);
+                    v_pairs(v[2 * ks + 1], mt, a2, a3);
+                    mma_16816(oacc[mt], a0, a1, a2, a3, pb[ks][0], pb[ks][1]);
+                }
+        }
+    };
+
+    // warps that fold the per-warp states; when enough warps are left over they rotate the next
+    // piece's queries at the same time
+    constexpr int NRED = (NO <= WARPS - 2) ? NO : WARPS;
+    constexpr int FINISH = NH;   // warps that finish a piece (four heads each)
+
+    // Finish warp w's heads of a folded piece: normalise, rotate back and store when the piece is the
+    // whole unit; else put its rows beside the unit's others, and finish the unit when they were the
+    // last ones missing.
+    auto finish_piece = [&](const FlowPiece& it, bool first_of_cta) {
+        const int t = lane & 7, h = warp * 4 + (lane >> 3);
+        const bool valid = h < group;
+        const float* row0 = folded + (valid ? h : 0) * ROW;
+        float a[E];
+#pragma unroll
+        for (int i = 0; i < E / 8; i++) {
+            const float4 u = *reinterpret_cast<const float4*>(row0 + 8 * (t + 8 * i));
+            const float4 v = *(reinterpret_cast<const float4*>(row0 + 8 * (t + 8 * i)) + 1);
+            a[8 * i] = u.x; a[8 * i + 1] = u.y; a[8 * i + 2] = u.z; a[8 * i + 3] = u.w;
+            a[8 * i + 4] = v.x; a[8 * i + 5] = v.y; a[8 * i + 6] = v.z; a[8 * i + 7] = v.w;
+        }
+        float m = row0[D], l = row0[D + 1];
+        bool nan = m != m;
+        const int64_t c0 = it.unit_start / share, c1 = (it.unit_start + it.unit_pages - 1) / share;
+        if (c0 != c1) {
+            // row block 0 of a CTA: the piece its share starts with; 1: its last one
+            auto row_of = [&](int64_t c, int block) {
+                return p.partials + ((2 * c + block) * group + (valid ? h : 0)) * ROW;
+            };
+            float* mine = row_of(blockIdx.x, first_of_cta ? 0 : 1);
+            if (valid) {
+#pragma unroll
+                for (int i = 0; i < E / 8; i++) {
+                    float4* dst = reinterpret_cast<float4*>(mine + 8 * (t + 8 * i));
+                    __stcg(dst, make_float4(a[8 * i], a[8 * i + 1], a[8 * i + 2], a[8 * i + 3]));
+                    __stcg(dst + 1, make_float4(a[8 * i + 4], a[8 * i + 5], a[8 * i + 6], a[8 * i + 7]));
+                }
+                if (t == 0) {
+                    __stcg(mine + D, m);
+                    __stcg(mine + D + 1, l);
+                }
+            }
+            __threadfence();
+            __syncwarp();
+            await_epoch();
+            int old = 0;
+            if (lane == 0) {
+                const int64_t unit = (static_cast<int64_t>(it.layer) * p.B + it.b) * p.Hkv + it.hkv;
+                old = atomicAdd(p.unit_counter + 2 * unit + warp, 1);
+            }
+            if (__shfl_sync(0xffffffffu, old, 0) != static_cast<int>(c1 - c0)) return;
+            __threadfence();
+            // (the order of the sum is the order of the CTAs, whoever merges)
+            m = -INFINITY;
+            for (int64_t c = c0; c <= c1; c++) {
+                const float mc = __ldcg(row_of(c, c * share >= it.unit_start ? 0 : 1) + D);
+                nan |= mc != mc;   // (fmaxf drops a NaN operand)
+                m = fmaxf(m, mc);
+            }
+            l = 0.f;
+#pragma unroll
+            for (int r = 0; r < E; r++) a[r] = 0.f;
+            for (int64_t c = c0; c <= c1; c++) {
+                const float* row = row_of(c, c * share >= it.unit_start ? 0 : 1);
+                const float f = fast_exp2(__ldcg(row + D) - m);
+                l = fmaf(__ldcg(row + D + 1), f, l);
+#pragma unroll
+                for (int i = 0; i < E / 4; i++) {
+                    const float4 x = __ldcg(reinterpret_cast<const float4*>(row + 8 * (t + 8 * (i / 2))) + (i & 1));
+                    a[4 * i] = fmaf(x.x, f, a[4 * i]);
+                    a[4 * i + 1] = fmaf(x.y, f, a[4 * i + 1]);
+                    a[4 * i + 2] = fmaf(x.z, f, a[4 * i + 2]);
+                    a[4 * i + 3] = fmaf(x.w, f, a[4 * i + 3]);
+                }
+            }
+        }
+        float inv = l > 0.f ? 1.f / l : 0.f;
+        if (nan) inv = __int_as_float(0x7fc00000);
+#pragma unroll
+        for (int r = 0; r < E; r++) a[r] *= inv;
+        octet_fwht<E>(a, lane);
+        if (valid) {
+            const int64_t at = (head_row(it) + h) * D;
+#pragma unroll
+            for (int k = 0; k < E; k++) {
+                const float r = a[k] * p.rsqrt_d;
+                const float s = __uint_as_float(__float_as_uint(r) ^ sign_mask(p.signs, t + 8 * k));
+                const int64_t idx = at + t + 8 * k;
+                if (p.out_dtype == kBF16) static_cast<__nv_bfloat16*>(p.out)[idx] = __float2bfloat16_rn(s);
+                else if (p.out_dtype == kF16) static_cast<__half*>(p.out)[idx] = __float2half_rn(s);
+                else static_cast<float*>(p.out)[idx] = s;
+            }
+        }
+    };
+
+    // sequences without tokens: no CTA meets their units, their outputs are zero (softmax over nothing)
+    for (int i = blockIdx.x; i < p.n_layers * p.B; i += gridDim.x) {
+        const int layer = i / p.B, b = i - layer * p.B;
+        if (prefix[b + 1] != prefix[b]) continue;
+        const int per_seq = p.Hq * D;
+        const int64_t at = (static_cast<int64_t>(layer) * p.B_stride + p.b0 + b) * per_seq;
+        for (int d = tid; d < per_seq; d += THREADS) {
+            if (p.out_dtype == kF32) static_cast<float*>(p.out)[at + d] = 0.f;
+            else static_cast<uint16_t*>(p.out)[at + d] = 0;   // (fp16 and bf16 zero)
+        }
+    }
+
+    // ---- the pieces of this CTA's share
+    int slot = 0;                // piece number mod 3
+    int ids = 0, ids_next = 0;   // block ids: the batch the next request takes, and the one after
+    bool primed = false;         // the first RING stages of the current piece were requested early
+    bool any = false, prev_first = true;   // a folded piece is waiting; it was the CTA's first
+    if (s_piece[0].n_pages > 0) {
+        ids = load_ids(s_piece[0], 0, 0);
+        rotate_queries(s_piece[0], 0);
+    }
+    while (s_piece[slot].n_pages > 0) {
+        const FlowPiece& cur = s_piece[slot];
+        const int slot1 = slot == 2 ? 0 : slot + 1, slot2 = slot == 0 ? 2 : slot - 1;   // next, after next
+        const int n_pages = cur.n_pages, tokens = cur.tokens;
+        const int n_mine = my_stages(cur);
+        const uint8_t* base = head_base(cur);
+        ids_next = load_ids(cur, IDS, slot);
+        __syncthreads();         // C: queries, the next piece visible; `folded` holds the piece before
+        int ids_piece = 0;       // first batch of the next piece
+        if (s_piece[slot1].n_pages > 0) ids_piece = load_ids(s_piece[slot1], 0, slot1);
+        // (a warp whose wait has run out requests nothing any more: the mbarrier of the lost copy
+        // never completes its phase, and arriving on it again would be an error)
+        if (!primed && !stalled) {
+            // (when the exchange area aliases the ring, the fold used it with ordinary accesses)
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+#pragma unroll
+            for (int r = 0; r < C::RING; r++)
+                if (r < n_mine) issue_stage(base, ids, n_pages, r, (ring_it + r) % C::RING);
+        }
+
+        // Q^T fragments: column n = g is head g >> 1 (NH = 1) or g (NH = 2); k-block kb covers
+        // coordinates (D/4)*tg + 4*kb + {0,1} (b0) and + {2,3} (b1)
+        if constexpr (!C::QSMEM) {
+#pragma unroll
+            for (int kb = 0; kb < NKB; kb++) {
+                const float4 q4 = *reinterpret_cast<const float4*>(
+                    qs + qs_index(H8 ? g : g >> 1, (D / 4) * tg + 4 * kb));
+                const __half2 lo = __floats2half2_rn(q4.x, q4.y);
+                const __half2 hi = __floats2half2_rn(q4.z, q4.w);
+                qb[kb][0] = *reinterpret_cast<const uint32_t*>(&lo);
+                qb[kb][1] = *reinterpret_cast<const uint32_t*>(&hi);
+            }
+        } else {
+            // shared-memory copy of the fragments, in place of the fp32 queries, which nobody reads
+            // again before the next piece's are rotated
+            constexpr int NE = NKB * 32, PER = (NE + THREADS - 1) / THREADS;
+            uint2 frag[PER];
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                const int e = tid + i * THREADS;
+                const int ln = e & 31, kb = e >> 5;
+                if (e < NE) {
+                    const float4 q4 = *reinterpret_cast<const float4*>(
+                        qs + qs_index(H8 ? ln >> 2 : ln >> 3, (D / 4) * (ln & 3) + 4 * kb));
+                    const __half2 lo = __floats2half2_rn(q4.x, q4.y);
+                    const __half2 hi = __floats2half2_rn(q4.z, q4.w);
+                    frag[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo),
+                                         *reinterpret_cast<const uint32_t*>(&hi));
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < PER; i++) {
+                const int e = tid + i * THREADS;
+                if (e < NE) reinterpret_cast<uint2*>(qs)[e] = frag[i];
+            }
+            __syncthreads();
+        }
+        if (any && warp < FINISH) finish_piece(s_piece[slot2], prev_first);
+
+#pragma unroll
+        for (int i = 0; i < HL; i++) { m_run[i] = -INFINITY; l_run[i] = 0.f; }
+#pragma unroll
+        for (int mt = 0; mt < NO; mt++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) oacc[mt][i] = 0.f;
+
+        // ---- the warp's stages.  NP pages at a time share the wait, the hand-over of the buffer, the
+        // query fragments and the look at the reference maximum, and their chains of look-ups and
+        // MMAs overlap.
+        for (int k = 0; k < n_mine; k++) {
+            const int rb = ring_it % C::RING;
+            ring_it++;
+            if (!stalled && !mbar_wait(my_bars + rb * 8, (phase >> rb) & 1u)) stalled = true;
+            phase ^= 1u << rb;
+            const uint32_t page = my_ring + rb * C::STAGE_BYTES;
+            uint32_t kw[C::NP][2][C::KW], v[4][C::VW], pb[C::NP][C::NPB][2];
+            uint2 kn[C::NP], vn[C::NP];
+            float c[C::NP][2][4];
+#pragma unroll
+            for (int i = 0; i < NP; i++) {
+                read_keys(kw[i], page + i * C::PAGE_BYTES);
+                kn[i] = lds64(page + i * C::PAGE_BYTES + noff);
+                vn[i] = lds64(page + i * C::PAGE_BYTES + noff + (C::OFF_VN - C::OFF_KN));
+            }
+            qk_scores(kw, c);
+            // all stages but possibly the piece's last one are full (warp-uniform branch)
+            const int st = warp + k * WARPS;
+            if ((st + 1) * NP * kPageTokens <= tokens) softmax_update(std::true_type{}, kn, vn, st, tokens, c, pb);
+            else softmax_update(std::false_type{}, kn, vn, st, tokens, c, pb);
+#pragma unroll
+            for (int i = 0; i < NP; i++) {
+                read_values(v, page + i * C::PAGE_BYTES);
+                pv_accum(v, pb[i]);
+            }
+            __syncwarp();  // every lane has its slices: the buffer may be refilled
+            const int req = k + C::RING;
+            if (req < n_mine && !stalled) {
+                if (req % IDS == 0) {
+                    ids = ids_next;
+                    ids_next = load_ids(cur, req + IDS, slot);
+                }
+                issue_stage(base, ids, n_pages, req, rb);
+            }
+        }
+
+        // ---- this warp's ring is drained: request the first stages of the next piece now, so that
+        // they arrive while this one is folded (when the fold has its own exchange area)
+        ids = ids_piece;
+        primed = false;
+        if constexpr (C::SEP) {
+            const FlowPiece& nx = s_piece[slot1];
+            if (nx.n_pages > 0) {
+                primed = true;
+                const int n = my_stages(nx);
+                if (!stalled) {
+#pragma unroll
+                    for (int r = 0; r < C::RING; r++)
+                        if (r < n) issue_stage(head_base(nx), ids, nx.n_pages, r, (ring_it + r) % C::RING);
+                }
+            }
+        }
+
+        // ---- fold the warps' states: every warp publishes (m, l, O), NRED warps reduce
+#pragma unroll
+        for (int i = 0; i < HL; i++) {
+            l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 4);
+            l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 8);
+            l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 16);
+        }
+        // a warp whose copy never arrived poisons its state (NaN propagates to the output)
+        if (stalled) {
+#pragma unroll
+            for (int i = 0; i < HL; i++) m_run[i] = __int_as_float(0x7fc00000);
+        }
+        __syncthreads();  // A: every warp is done with the ring, the queries and `folded`
+#pragma unroll
+        for (int mt = 0; mt < NO; mt++)
+            // (the factor that undoes the scaling of the value centroids is applied once per piece)
+            xchg(warp)[mt * 32 + lane] =
+                make_float4(oacc[mt][0] * p.inv_v_scale, oacc[mt][1] * p.inv_v_scale,
+                            oacc[mt][2] * p.inv_v_scale, oacc[mt][3] * p.inv_v_scale);
+        if (g == 0) {
+#pragma unroll
+            for (int i = 0; i < HL; i++) {
+                xml[(warp * 2 + 0) * (4 * NH) + HL * tg + i] = m_run[i];
+                xml[(warp * 2 + 1) * (4 * NH) + HL * tg + i] = l_run[i];
+            }
+        }
+        __syncthreads();  // B: all states are published
+        if (warp < NRED) {
+            const bool bad = s_bad[slot] != 0;
+            for (int j = tid; j < NO * 32; j += NRED * 32) {
+                const int ln = j & 31, mt = j >> 5;
+                const int tg_ = ln & 3, g_ = ln >> 2;
+                float M[HL], l[HL];
+                bool nan[HL];
+#pragma unroll
+                for (int i = 0; i < HL; i++) {
+                    M[i] = -INFINITY;
+                    l[i] = 0.f;
+                    nan[i] = bad;
+#pragma unroll
+                    for (int w2 = 0; w2 < WARPS; w2++) {
+                        const float mw = xml[(w2 * 2 + 0) * (4 * NH) + HL * tg_ + i];
+                        nan[i] |= mw != mw;   // (fmaxf drops a NaN operand)
+                        M[i] = fmaxf(M[i], mw);
+                    }
+                }
+                float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int w2 = 0; w2 < WARPS; w2++) {
+                    float f[HL];
+                    bool some = false;
+#pragma unroll
+                    for (int i = 0; i < HL; i++) {
+                        const float mw = xml[(w2 * 2 + 0) * (4 * NH) + HL * tg_ + i];
+                        const bool has = mw != -INFINITY;  // (NaN compares unequal: poison goes through)
+                        f[i] = has ? fast_exp2(mw - M[i]) : 0.f;
+                        some |= has;
+                        l[i] = fmaf(has ? xml[(w2 * 2 + 1) * (4 * NH) + HL * tg_ + i] : 0.f, f[i], l[i]);
+                    }
+                    if (some) {
+                        const float4 o = xchg(w2)[mt * 32 + ln];
+                        o4.x = fmaf(o.x, f[0], o4.x);
+                        o4.y = fmaf(o.y, f[HL - 1], o4.y);
+                        o4.z = fmaf(o.z, f[0], o4.z);
+                        o4.w = fmaf(o.w, f[HL - 1], o4.w);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < HL; i++) {
+                    float* dst = folded + (HL * tg_ + i) * ROW;
+                    if constexpr (H8)
+                        *reinterpret_cast<float2*>(dst + (D / 8) * g_ + 2 * mt) =
+                            i == 0 ? make_float2(o4.x, o4.z) : make_float2(o4.y, o4.w);
+                    else
+                        *reinterpret_cast<float4*>(dst + (D / 8) * g_ + 4 * mt) = o4;
+                    if (g_ == 0 && mt == 0) {
+                        dst[D] = nan[i] ? __int_as_float(0x7fc00000) : M[i];   // NaN marks a poisoned piece
+                        dst[D + 1] = l[i];
+                    }
+                }
+            }
+            if (bad && tid == 0) {
+                await_epoch();
+                atomicOr(p.work_counter + kStatusWord, kStatusBadBlock);
+            }
+        }
+        if (s_piece[slot1].n_pages > 0) rotate_queries(s_piece[slot1], NRED < WARPS ? NRED : 0);
+        if (tid == THREADS - 1) {
+            s_piece[slot2] = locate(s_piece[slot1].next);
+            s_bad[slot2] = 0;
+        }
+        any = true;
+        prev_first = cur.unit_start + cur.page0 == first;
+        slot = slot1;
+        __syncwarp();
+        if (s_piece[slot].n_pages == 0) break;
+    }
+    __syncthreads();
+    if (any && warp < FINISH) finish_piece(s_piece[slot == 0 ? 2 : slot - 1], prev_first);
+    if (stalled) {
+        await_epoch();
+        if (lane == 0) atomicOr(p.work_counter + kStatusWord, kStatusWaitExpired);
+    }
+    // the last CTA to leave takes the epoch out of the workspace: a replay of this very launch (a
+    // captured graph) must not find its own epoch there before CTA 0 has cleared the counters
+    __syncthreads();
+    if (warp == 0) {
+        await_epoch();
+        if (lane == 0 && atomicAdd(p.work_counter + 1, 1) == static_cast<int>(gridDim.x) - 1) {
+            __threadfence();
+            asm volatile("st.release.gpu.global.u64 [%0], %1;\n" ::"l"(epoch_word), "l"(0ull) : "memory");
+        }
+    }
+}
+
+}  // namespace ftq

@@ -1,4 +1,5 @@
 // Instantiates the split-KV decode attention kernels for one head_dim (FTQ_D).
+#include "ftq_attn_flow.cuh"
 #include "ftq_attn_stream.cuh"
 #include "ftq_launch.h"
 
@@ -71,6 +72,43 @@ constexpr bool use_stream_kernel() {
 }
 
 template <int BK, int BV, bool SHARED, int NH>
+static cudaError_t run_flow(const AttnParams& p_in, cudaStream_t stream, bool* merged) {
+    using C = MmaCfg<FTQ_D, BK, BV, NH>;
+    static_assert(C::SMEM_BYTES <= C::LIMIT, "shared memory budget");
+    constexpr auto kern = attn_flow_kernel<FTQ_D, BK, BV, SHARED, NH>;
+    cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    *merged = true;
+    AttnParams p = p_in;
+    // a CTA's share is at least one stage per warp: less would only cut units into more rows to merge
+    p.min_share = C::WARPS * C::NP;
+    p.B_stride = p_in.B;
+    for (p.b0 = 0; p.b0 < p_in.B; p.b0 += kFlowMaxSeqs) {
+        p.B = p_in.B - p.b0 < kFlowMaxSeqs ? p_in.B - p.b0 : kFlowMaxSeqs;
+        p.seq_lens = p_in.seq_lens + p.b0;
+        p.block_table = p_in.block_table + static_cast<int64_t>(p.b0) * p.max_blocks;
+        p.n_units = p.n_layers * p.B * p.Hkv;
+        const int64_t most = static_cast<int64_t>(p.n_units) * ((static_cast<int64_t>(p.max_seq) + kPageTokens - 1) / kPageTokens);
+        const int64_t want = (most + p.min_share - 1) / p.min_share;
+        const int64_t slots = static_cast<int64_t>(sm_count()) * C::CTAS_PER_SM;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(static_cast<unsigned>(want < 1 ? 1 : want < slots ? want : slots));
+        cfg.blockDim = dim3(C::THREADS);
+        cfg.dynamicSmemBytes = C::SMEM_BYTES;
+        cfg.stream = stream;
+        // (programmatic stream serialisation: the tables are built while the kernel before drains)
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, kern, p);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+template <int BK, int BV, bool SHARED, int NH>
 static cudaError_t run_mma_nh(const AttnParams& p, int n_lb, cudaStream_t stream, bool* merged) {
     constexpr int D = FTQ_D;
     if constexpr (use_stream_kernel<BK, BV, NH>()) {
@@ -102,19 +140,7 @@ static cudaError_t run_mma_nh(const AttnParams& p, int n_lb, cudaStream_t stream
         *merged = true;
         return cudaLaunchKernelEx(&cfg, kern, p, static_cast<int>(items));
     } else {
-    *merged = false;
-    using C = MmaCfg<D, BK, BV, NH>;
-    static_assert(C::SMEM_BYTES <= 227 * 1024, "shared memory budget");
-    constexpr auto kern = attn_mma_kernel<D, BK, BV, SHARED, NH>;
-    cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    const int64_t items = p.split.total_items;
-    const int64_t slots = static_cast<int64_t>(sm_count()) * C::CTAS_PER_SM;
-    const unsigned grid = static_cast<unsigned>(items < slots ? items : slots);
-    e = cudaMemsetAsync(p.work_counter, 0, 256, stream);   // this kernel counts from a zeroed word
-    if (e != cudaSuccess) return e;
-    kern<<<grid, C::THREADS, C::SMEM_BYTES, stream>>>(p, static_cast<int>(items));
-    return cudaGetLastError();
+        return run_flow<BK, BV, SHARED, NH>(p, stream, merged);
     }
 }
 

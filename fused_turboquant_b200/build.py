@@ -43,6 +43,7 @@ for _d in (256, 128, 64):
     UNITS.append(("ftq_tq_v1_inst.cu", f"tq_v1_decode_d{_d}", [f"-DFTQ_D={_d}", "-DFTQ_TQ_PART=1"]))
 for _d in (256, 128, 64):
     UNITS.append(("ftq_attn_inst.cu", f"attn_d{_d}", [f"-DFTQ_D={_d}"]))
+    UNITS.append(("ftq_attn_chunk_inst.cu", f"attn_chunk_d{_d}", [f"-DFTQ_D={_d}"]))
     UNITS.append(("ftq_encode_inst.cu", f"encode_d{_d}", [f"-DFTQ_D={_d}"]))
 UNITS.append(("ftq_api.cu", "api", []))
 

@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cfloat>
 #include <climits>
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstring>
@@ -752,8 +753,8 @@ size_t ftq_decode_workspace_bytes(int B, int Hq, int Hkv, int head_dim, int max_
             const size_t m = partial_bytes(pl, B, Hq, head_dim, n_layers);
             n = m > n ? m : n;
         }
-        // the equal-share kernel: two blocks of rows per CTA, at most two CTAs per SM
-        const size_t flow = static_cast<size_t>(ftq::sm_count()) * 4 * (Hq / Hkv) * (head_dim + 4) * sizeof(float);
+        // the equal-share kernel (groups of at most 8): two blocks of rows per CTA, at most two CTAs per SM
+        const size_t flow = Hq / Hkv > 8 ? 0 : static_cast<size_t>(ftq::sm_count()) * 4 * (Hq / Hkv) * (head_dim + 4) * sizeof(float);
         return flow > n ? flow : n;
     }) + counter_bytes(B, Hkv, n_layers);
 }
@@ -1112,6 +1113,107 @@ extern "C" int ftq_paged_decode_status(const void* workspace, int B, int Hq, int
     return fail(FTQ_ERR_DEVICE, "the last decode call on this workspace reported%s%s",
                 (bits & FTQ_STATUS_BAD_BLOCK_ID) ? " a block id outside the pool" : "",
                 (bits & FTQ_STATUS_WAIT_EXPIRED) ? " a wait that ran out" : "");
+}
+
+// ------------------------------------------------------------------ causal attention of a chunk
+
+namespace {
+// The tiles of a row tile's context are cut into as many parts as give the shortest schedule: waves of
+// CTAs (one per SM) x (tiles of a part + what a CTA costs besides its tiles: tables, queries and the
+// pipeline's start and end take about as long as 6 tiles, measured on parts of 4 to 64 tiles).
+int chunk_splits(int B, int q_len, int Hq, int Hkv, int d, int max_seq) {
+    const int slots = d == 256 ? 1 : 2, kt = d == 256 ? 32 : 64;
+    const int64_t rows = static_cast<int64_t>(q_len) * (Hq / Hkv);
+    const int64_t units = static_cast<int64_t>(B) * Hkv * ((rows + 128 * slots - 1) / (128 * slots));
+    const int tiles = std::max(1, (max_seq + kt - 1) / kt), sms = ftq::sm_count();
+    int best = 1;
+    double cost = -1.0;
+    for (int s = 1; s <= 32 && s <= tiles; s++) {
+        const double c = static_cast<double>((units * s + sms - 1) / sms) * ((tiles + s - 1) / s + 6.0);
+        if (cost < 0.0 || c < cost * 0.98) {
+            cost = c;
+            best = s;
+        }
+    }
+    return best;
+}
+}  // namespace
+
+extern "C" size_t ftq_paged_chunk_workspace_bytes(int B, int q_len, int Hq, int Hkv, int head_dim,
+                                                  int max_seq_len) {
+    if (B <= 0 || q_len <= 0) return 0;
+    const size_t head = ftq_decode_workspace_bytes(1, Hq, Hkv, head_dim, max_seq_len, 1);
+    if (head == 0) return 0;
+    const int seq = round_seq(max_seq_len);
+    return (head + 255) / 256 * 256 +
+           static_cast<size_t>(B) * q_len * Hq * chunk_splits(B, q_len, Hq, Hkv, head_dim, seq) *
+               (head_dim + 4) * sizeof(float);
+}
+
+extern "C" int ftq_paged_chunk_attn(const void* q, int q_dtype, void* out, int out_dtype,
+                                    const uint8_t* pool, int64_t num_blocks, const int32_t* block_table,
+                                    int max_blocks, const int32_t* seq_lens, int max_seq_len, int B,
+                                    int q_len, int Hq, int Hkv, int head_dim, int bits_k, int bits_v,
+                                    const float* levels_k_host, const float* levels_v_host,
+                                    const float* signs_host, float scale, void* workspace,
+                                    size_t workspace_bytes, void* stream) {
+    int rc = check_attn_common(B, Hq, Hkv, head_dim, bits_k, bits_v, q_dtype, out_dtype);
+    if (rc) return rc;
+    if (q_dtype == FTQ_F32 || Hq / Hkv > 8)
+        return fail(FTQ_ERR_UNSUPPORTED, "chunk attention takes 16-bit queries and GQA groups of at most 8");
+    if (q_len <= 0 || max_blocks <= 0 || max_seq_len < 0 || num_blocks < 0)
+        return fail(FTQ_ERR_INVALID, "bad shape q_len=%d max_blocks=%d max_seq_len=%d", q_len, max_blocks, max_seq_len);
+    if (B == 0) return FTQ_OK;
+    const int64_t rows = static_cast<int64_t>(q_len) * (Hq / Hkv);
+    if (B > 65535 || rows > (1 << 24) || static_cast<int64_t>(Hkv) * ((rows + 127) / 128) > 65535)
+        return fail(FTQ_ERR_UNSUPPORTED, "too many sequences or queries for one call");
+    if (!q || !out || !pool || !block_table || !seq_lens) return fail(FTQ_ERR_INVALID, "NULL tensor pointer");
+    if (static_cast<int64_t>(max_blocks) * FTQ_PAGE_TOKENS < max_seq_len)
+        return fail(FTQ_ERR_INVALID, "block_table too narrow: %d blocks < max_seq_len %d", max_blocks, max_seq_len);
+    if (!aligned(q, 16) || !aligned(out, 4) || !aligned(pool, 16))
+        return fail(FTQ_ERR_INVALID, "q and pool must be 16-byte aligned");
+    const size_t need = ftq_paged_chunk_workspace_bytes(B, q_len, Hq, Hkv, head_dim, max_seq_len);
+    if (!workspace || workspace_bytes < need)
+        return fail(FTQ_ERR_WORKSPACE, "workspace needs %zu bytes, got %zu", need, workspace_bytes);
+    if (!aligned(workspace, 16)) return fail(FTQ_ERR_WORKSPACE, "workspace must be 16-byte aligned");
+    ftq::ChunkAttnParams p{};
+    rc = pack_levels(levels_k_host, bits_k, &p.lk);
+    if (rc == FTQ_OK) rc = pack_levels(levels_v_host, bits_v, &p.lv);
+    if (rc == FTQ_OK) rc = pack_signs(signs_host, head_dim, &p.signs);
+    if (rc) return rc;
+    const float ks = choose_k_scale(levels_k_host, bits_k, head_dim);
+    for (int i = 0; i < (1 << bits_k); i++) p.lk.v[i] = levels_k_host[i] * ks;
+    const float vs = choose_v_scale(levels_v_host, bits_v, head_dim);
+    for (int i = 0; i < (1 << bits_v); i++) p.lv.v[i] = levels_v_host[i] * vs;
+    p.inv_v_scale = 1.0f / vs;
+    p.q_scale = rsqrt_dim(head_dim) * (scale / ks * ftq::kLog2e);
+    p.q = q; p.q_dtype = q_dtype;
+    p.pool = pool; p.num_blocks = num_blocks;
+    p.block_table = block_table; p.max_blocks = max_blocks;
+    p.seq_lens = seq_lens; p.max_seq = max_seq_len;
+    p.q_len = q_len; p.Hq = Hq; p.Hkv = Hkv;
+    p.splits = chunk_splits(B, q_len, Hq, Hkv, head_dim, round_seq(max_seq_len));
+    // the workspace begins as that of a decode call of one sequence, so that ftq_paged_decode_status
+    // finds the status word; the rows follow
+    uint8_t* const ws = static_cast<uint8_t*>(workspace);
+    const size_t head = ftq_decode_workspace_bytes(1, Hq, Hkv, head_dim, max_seq_len, 1);
+    p.status = reinterpret_cast<int*>(ws + head - counter_bytes(1, Hkv, 1)) + ftq::kStatusWord;
+    p.partials = reinterpret_cast<float*>(ws + (head + 255) / 256 * 256);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    cudaError_t e = cudaMemsetAsync(p.status, 0, sizeof(int), st);
+    if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_chunk_attn status reset");
+    switch (head_dim) {
+        case 64: e = ftq::launch_attn_chunk_d64(bits_k, bits_v, p, B, st); break;
+        case 128: e = ftq::launch_attn_chunk_d128(bits_k, bits_v, p, B, st); break;
+        default: e = ftq::launch_attn_chunk_d256(bits_k, bits_v, p, B, st); break;
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_chunk_attn launch");
+    ChunkPlan pl{};
+    pl.n_chunks = p.splits;
+    pl.chunk_tokens = 1;
+    e = dispatch_merge(head_dim, out_dtype, p.partials, out, nullptr, p.splits, B, Hq, Hkv, pl,
+                       ftq::SplitPlan{}, static_cast<int64_t>(B) * q_len * Hq, p.signs, st);
+    return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_paged_chunk_attn merge launch");
 }
 
 // ------------------------------------------------------------------ vLLM-v1 slot format

@@ -6,7 +6,7 @@
 
 #include <atomic>
 
-#include "ftq_attn.cuh"
+#include "ftq_attn_chunk.cuh"
 #include "ftq_encode2.cuh"
 
 namespace ftq {
@@ -18,6 +18,8 @@ namespace ftq {
                                         int n_lb, cudaStream_t stream);                         \
     cudaError_t launch_attn_mma_d##DD(int bits_k, int bits_v, bool shared_lut, const AttnParams& p, \
                                       int n_lb, cudaStream_t stream, bool* merged);            \
+    cudaError_t launch_attn_chunk_d##DD(int bits_k, int bits_v, const ChunkAttnParams& p, int B, \
+                                        cudaStream_t stream);                                   \
     int attn_mma_stream_ctas_d##DD(int bits_k, int bits_v, int group);                          \
     cudaError_t launch_attn_merge_d##DD(int out_dtype, const float* partials, void* out,        \
                                         const int32_t* seq_lens, int S, int B, int Hq,          \

@@ -33,7 +33,7 @@ namespace {
 #define FTQ_BOUND(X)                                                                       \
     X(ftq_encode) X(ftq_decode_dense) X(ftq_rht) X(ftq_decode_workspace_bytes)             \
     X(ftq_flash_decode) X(ftq_paged_store) X(ftq_paged_decode_attn) X(ftq_tq_store_layers) \
-    X(ftq_tq_decode_layers)
+    X(ftq_tq_decode_layers) X(ftq_paged_chunk_workspace_bytes) X(ftq_paged_chunk_attn)
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
     FTQ_BOUND(X)
@@ -344,6 +344,42 @@ PyObject* paged_decode(PyObject* const* a) {
     return THPVariable_Wrap(out);
 }
 
+// paged_chunk(self, q, block_table, seq_lens, max_seq_len, scale, layer)
+PyObject* paged_chunk(PyObject* const* a) {
+    PyObject* self = a[0];
+    at::Tensor q = cuda_tensor(a[1], "q");
+    if (!q.is_contiguous()) q = q.contiguous();
+    const Pool p(self);
+    const int64_t B = q.size(0), q_len = q.size(1), Hq = q.size(2), D = q.size(3);
+    const double scale = a[5] == Py_None ? std::pow(static_cast<double>(D), -0.5) : as_double(a[5]);
+    const at::Device dev = q.device();
+    const at::Tensor bt = as_i32(a[2], "block_table", dev), sl = as_i32(a[3], "seq_lens", dev);
+    const long long max_seq = as_int(a[4]);
+    const c10::cuda::CUDAGuard guard(dev);
+    const at::Tensor out = empty(q.sizes(), q.scalar_type(), dev);
+    void* st = stream_of(dev);
+    const at::Tensor ws = workspace(Py_None, dev, st, api.ftq_paged_chunk_workspace_bytes(
+                                                          B, q_len, Hq, p.hkv, p.d, max_seq));
+    uint8_t* base = p.base(a[6]);
+    Ref so(PyObject_GetAttr(self, names.signs)), ko(PyObject_GetAttr(self, names.levels_k)),
+        vo(PyObject_GetAttr(self, names.levels_v));
+    const Table signs(so.o), lk(ko.o), lv(vo.o);
+    int rc;
+    {
+        NoGil nogil;
+        rc = api.ftq_paged_chunk_attn(
+            ptr<void>(q), dtype_code(q.scalar_type()), mptr<void>(out), dtype_code(out.scalar_type()), base,
+            p.num_blocks, ptr<int32_t>(bt), bt.size(1), ptr<int32_t>(sl), max_seq, B, q_len, Hq, p.hkv, D,
+            p.kb, p.vb, lk.p, lv.p, signs.p, static_cast<float>(scale), mptr<void>(ws), ws.numel(), st);
+    }
+    check(rc, "ftq_paged_chunk_attn");
+    // (the status word lies where a decode call of one sequence has it)
+    Ref w(THPVariable_Wrap(ws)), d(THPDevice_New(dev));
+    Ref last(Py_BuildValue("(OLLLLO)", w.o, 1ll, static_cast<long long>(Hq), max_seq, 1ll, d.o));
+    if (PyObject_SetAttr(self, names._last_decode, last.o) < 0) throw PyError{};
+    return THPVariable_Wrap(out);
+}
+
 int64_t packed_dim(int64_t d, long long bits) {
     if (bits < 2 || bits > 4)
         raise(PyExc_ValueError, "bits must be 2, 3, or 4, got " + std::to_string(bits));
@@ -649,6 +685,7 @@ PyMethodDef methods[] = {
     FTQ_ENTRY(bind, 4),
     FTQ_ENTRY(paged_store, 5),
     FTQ_ENTRY(paged_decode, 9),
+    FTQ_ENTRY(paged_chunk, 7),
     FTQ_ENTRY(encode, 4),
     FTQ_ENTRY(decode_dense, 6),
     FTQ_ENTRY(rht, 3),

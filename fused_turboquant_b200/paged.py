@@ -154,17 +154,32 @@ class PagedKVPool:
         v_norms = rows(off_vn, 2).contiguous().view(torch.float16).reshape(H, -1)[:, :S].contiguous()
         return k_codes, k_norms, v_codes, v_norms
 
+    def _takes_chunk_kernel(self, q, block_table, seq_lens, layer) -> bool:
+        B, q_len, Hq, D = q.shape
+        H = self.num_kv_heads
+        return (q.is_cuda and q.dtype in (torch.float16, torch.bfloat16) and layer is not None and
+                min(B, q_len, Hq) > 0 and Hq % H == 0 and Hq // H <= 8 and D == self.head_dim and
+                B <= 65535 and H * -(-q_len * (Hq // H) // 128) <= 65535 and
+                block_table.dim() == 2 and block_table.shape[0] == B and seq_lens.shape == (B,))
+
     def continuation_attention(self, q: torch.Tensor, block_table: torch.Tensor,
                                seq_lens: torch.Tensor, max_seq_len: int, scale: float | None = None,
                                layer: int = 0) -> torch.Tensor:
         """Causal attention of ``q_len`` new tokens per sequence whose keys/values are already stored.
 
         q: [B, q_len, Hq, D]; seq_lens: [B] totals INCLUDING the new tokens.  Query i of a sequence
-        attends positions < seq_len - q_len + i + 1.  Same device-side formulation as the reference's
-        continuation chunk (vllm_plugin/v1_backend.py:1359-1384): the decode kernel run on one
-        synthetic sequence per query with its own length; no host synchronisation.
+        attends positions < seq_len - q_len + i + 1 (reference: vllm_plugin/v1_backend.py:1359-1384).
+        16-bit queries with a GQA group of at most 8 take the chunk kernel, which dequantises a page
+        once for all queries; the others run the decode kernel on one synthetic sequence per query with
+        its own length.  No host synchronisation.
         """
         B, q_len, Hq, D = q.shape
+        if self._takes_chunk_kernel(q, block_table, seq_lens, layer):
+            if _trace.ENABLED:
+                with _trace.nvtx("ftq.decode"):
+                    return _lib.native().paged_chunk(self, q, block_table, seq_lens, max_seq_len, scale,
+                                                     layer)
+            return _lib.native().paged_chunk(self, q, block_table, seq_lens, max_seq_len, scale, layer)
         synth_bt, synth_sl = synthetic_decode_batch(block_table, seq_lens, q_len)
         out = self.decode_attention(q.reshape(B * q_len, Hq, D), synth_bt, synth_sl, max_seq_len,
                                     scale, layer=layer)

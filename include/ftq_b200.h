@@ -246,6 +246,29 @@ int ftq_paged_decode_attn_static(const void *q, int q_dtype, void *out, int out_
 int ftq_paged_decode_status(const void *workspace, int B, int Hq, int Hkv, int head_dim,
                             int max_seq_len, int n_layers, void *stream, int *status_bits);
 
+/*
+ * Causal attention of q_len new tokens per sequence, whose keys and values are
+ * already stored, over one layer of the pool (chunked prefill, speculative
+ * verification; reference: vllm_plugin/v1_backend.py:1359-1384, which runs the
+ * decode kernel on one synthetic sequence per query).
+ *
+ * q / out: [B, q_len, Hq, head_dim], 16-bit queries, Hq / Hkv at most 8;
+ * seq_lens: [B], the new tokens included; query i of a sequence attends the
+ * positions below seq_len - q_len + i + 1 (none: zeros).  The other arguments
+ * are those of ftq_paged_decode_attn.  The workspace holds at least
+ * ftq_paged_chunk_workspace_bytes(...) bytes, 16-byte aligned; the call's
+ * status is read with ftq_paged_decode_status(workspace, 1, Hq, Hkv, head_dim,
+ * max_seq_len, 1, ...).
+ */
+size_t ftq_paged_chunk_workspace_bytes(int B, int q_len, int Hq, int Hkv, int head_dim,
+                                       int max_seq_len);
+int ftq_paged_chunk_attn(const void *q, int q_dtype, void *out, int out_dtype, const uint8_t *pool,
+                         int64_t num_blocks, const int32_t *block_table, int max_blocks,
+                         const int32_t *seq_lens, int max_seq_len, int B, int q_len, int Hq, int Hkv,
+                         int head_dim, int bits_k, int bits_v, const float *levels_k_host,
+                         const float *levels_v_host, const float *signs_host, float scale,
+                         void *workspace, size_t workspace_bytes, void *stream);
+
 /* ------------------------------------------- reference v0 layout adaptors */
 
 /*

@@ -1,0 +1,94 @@
+"""The chunk attention kernel (continuation_attention with 16-bit queries) against the fp32 decode kernel
+run on one synthetic sequence per query."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _pool(d, bk, bv, hkv, lens, seed):
+    from fused_turboquant_b200 import PagedKVPool
+    gen = torch.Generator("cuda").manual_seed(seed)
+    per = [(n + 15) // 16 for n in lens]
+    ids = torch.randperm(sum(per) + 3, device="cuda", generator=gen)
+    table = torch.zeros(len(lens), max(per), dtype=torch.int32, device="cuda")
+    pool = PagedKVPool(sum(per) + 3, hkv, d, bk, bv, n_layers=2, device="cuda")
+    at = 0
+    for b, n in enumerate(lens):
+        table[b, :per[b]] = ids[at:at + per[b]].int()
+        pos = torch.arange(n, device="cuda")
+        slots = ids[at:at + per[b]][pos // 16] * 16 + pos % 16
+        kv = torch.randn(2, n, hkv, d, device="cuda", generator=gen)
+        kv[..., 3] *= 6.0
+        pool.store(kv[0].bfloat16(), kv[1].bfloat16(), slots, layer=1)
+        at += per[b]
+    return pool, table, torch.tensor(lens, dtype=torch.int32, device="cuda"), gen
+
+
+# (sizes around the tiles of 32 / 64 tokens and 128 rows: fewer rows than a tile, one tile, a second
+# one that is partly filled, more than the two of a CTA; contexts shorter than the chunk, one token,
+# remainders of a page and of a tile; one part and many)
+@pytest.mark.parametrize("d,bk,bv,hkv,group,q_len,lens,dtype", [
+    (128, 4, 4, 2, 4, 5, [40, 23], "bf16"),
+    (128, 4, 4, 8, 4, 64, [4096, 777, 63, 65], "bf16"),
+    (128, 3, 3, 2, 8, 33, [1000, 64, 20], "fp16"),
+    (128, 4, 2, 1, 1, 130, [513, 130], "bf16"),
+    (128, 2, 4, 2, 7, 19, [320, 1], "fp16"),
+    (64, 3, 3, 2, 7, 40, [700, 129], "bf16"),
+    (64, 4, 4, 1, 1, 2, [2, 1, 8000], "fp16"),
+    (64, 2, 2, 4, 8, 100, [300], "bf16"),
+    (256, 4, 2, 2, 2, 64, [400, 33, 31], "bf16"),
+    (256, 3, 4, 1, 8, 50, [1111, 95], "fp16"),
+    (256, 4, 4, 8, 1, 3, [50, 2], "bf16"),
+])
+def test_matches_fp32_decode(d, bk, bv, hkv, group, q_len, lens, dtype):
+    pool, table, sl, gen = _pool(d, bk, bv, hkv, lens, d + q_len)
+    dt = torch.bfloat16 if dtype == "bf16" else torch.float16
+    q = torch.randn(len(lens), q_len, hkv * group, d, device="cuda", generator=gen).to(dt)
+    assert pool._takes_chunk_kernel(q, table, sl, 1)
+    got = pool.continuation_attention(q, table, sl, max(lens), layer=1)
+    assert pool.decode_status() == 0
+    ref = pool.continuation_attention(q.float(), table, sl, max(lens), layer=1)
+    assert got.dtype == dt and got.shape == q.shape
+    dead = (sl[:, None] - q_len + 1 + torch.arange(q_len, device="cuda")[None]) <= 0
+    assert (got[dead] == 0).all()
+    err = (got.float() - ref).norm(dim=-1) / ref.norm(dim=-1).clamp_min(1e-6)
+    # 16-bit output (2^-9 bf16, 2^-12 fp16) and fp16 operands (queries, centroids, weights: 2^-12
+    # each, of scores of a few units): 4e-3 / 2e-3 per vector with a factor of two to spare
+    assert err[~dead].max().item() < (8e-3 if dtype == "bf16" else 5e-3)
+
+
+def test_other_calls_stay_on_the_decode_kernel():
+    pool, table, sl, gen = _pool(64, 4, 4, 1, [70], 3)
+    q = torch.randn(1, 4, 16, 64, device="cuda", generator=gen).bfloat16()
+    assert not pool._takes_chunk_kernel(q, table, sl, 1)              # group 16
+    assert not pool._takes_chunk_kernel(q.float()[:, :, :8], table, sl, 1)
+    assert not pool._takes_chunk_kernel(q[:, :, :8], table, sl, None)
+
+
+def test_block_id_out_of_range_is_reported():
+    pool, table, sl, gen = _pool(128, 4, 4, 2, [300, 300], 5)
+    q = torch.randn(2, 20, 8, 128, device="cuda", generator=gen).half()
+    good = pool.continuation_attention(q, table, sl, 300, layer=1)
+    table[1, 2] = pool.num_blocks + 5
+    out = pool.continuation_attention(q, table, sl, 300, layer=1)
+    assert pool.decode_status() == 1
+    assert torch.isnan(out[1]).all()
+    assert torch.equal(out[0], good[0])
+    table[1, 2] = 0
+    pool.continuation_attention(q, table, sl, 300, layer=1)
+    assert pool.decode_status() == 0
+
+
+def test_a_captured_call_replays():
+    pool, table, sl, gen = _pool(128, 4, 4, 2, [200], 6)
+    q = torch.randn(1, 16, 8, 128, device="cuda", generator=gen).half()
+    want = pool.continuation_attention(q, table, sl, 200, layer=1)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = pool.continuation_attention(q, table, sl, 200, layer=1)
+    out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy(), want.cpu().numpy())

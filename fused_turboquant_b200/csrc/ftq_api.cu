@@ -346,6 +346,27 @@ ChunkPlan plan_chunks(int B, int Hq, int Hkv, int d, int max_seq_len, int n_laye
     return pl;
 }
 
+// The same for contexts of one known length: no more chunks than above (the workspace is sized for
+// those), but as few as fill the chip's slots (two CTAs per SM) in whole waves.  A CTA costs about
+// three tiles besides its own: tables, queries, the fold of its warps, its rows and their merge.
+ChunkPlan plan_chunks_uniform(int B, int Hq, int Hkv, int d, int seq_len) {
+    ChunkPlan pl = plan_chunks(B, Hq, Hkv, d, round_seq(seq_len), 1);
+    const int tile = ftq::kTilePages * ftq::kPageTokens;
+    const int tiles = (seq_len + tile - 1) / tile, most = pl.n_chunks;
+    const int64_t units = static_cast<int64_t>(B) * Hkv * pl.n_hpass, slots = ftq::sm_count() * 2;
+    int64_t best = INT64_MAX;
+    for (int n = 1; n <= most && n <= tiles; n++) {
+        const int per = (tiles + n - 1) / n, real = (tiles + per - 1) / per;
+        const int64_t cost = (units * real + slots - 1) / slots * (per + 3);
+        if (cost < best) {
+            best = cost;
+            pl.n_chunks = real;
+            pl.chunk_tokens = per * tile;
+        }
+    }
+    return pl;
+}
+
 // Chunking of the tensor-core path (persistent CTAs): few, large chunks keep the per-item
 // fixed costs small, more chunks fill the last wave of CTA slots better; the plan with the
 // lowest modelled cost wins.  Chunks hold at most 8192 tokens (short enough for the dynamic
@@ -466,23 +487,19 @@ cudaError_t dispatch_mma(int d, int bk, int bv, bool shared_lut, const ftq::Attn
 }
 
 cudaError_t dispatch_merge(int d, int out_dtype, const float* partials, void* out,
-                           const int32_t* seq_lens, int S, int B, int Hq, int Hkv,
-                           const ChunkPlan& pl, const ftq::SplitPlan& split, int64_t n_vec,
-                           const ftq::SignBits& signs, cudaStream_t st) {
+                           const int32_t* seq_lens, int S, int B, int Hq, int n_chunks, int chunk_tokens,
+                           int64_t n_vec, const ftq::SignBits& signs, cudaStream_t st) {
     const float r = rsqrt_dim(d);
     switch (d) {
         case 64:
-            return ftq::launch_attn_merge_d64(out_dtype, partials, out, seq_lens, S, B, Hq,
-                                              pl.n_chunks, pl.chunk_tokens, n_vec, signs, r, Hkv,
-                                              split, st);
+            return ftq::launch_attn_merge_d64(out_dtype, partials, out, seq_lens, S, B, Hq, n_chunks,
+                                              chunk_tokens, n_vec, signs, r, st);
         case 128:
-            return ftq::launch_attn_merge_d128(out_dtype, partials, out, seq_lens, S, B, Hq,
-                                               pl.n_chunks, pl.chunk_tokens, n_vec, signs, r, Hkv,
-                                               split, st);
+            return ftq::launch_attn_merge_d128(out_dtype, partials, out, seq_lens, S, B, Hq, n_chunks,
+                                               chunk_tokens, n_vec, signs, r, st);
         case 256:
-            return ftq::launch_attn_merge_d256(out_dtype, partials, out, seq_lens, S, B, Hq,
-                                               pl.n_chunks, pl.chunk_tokens, n_vec, signs, r, Hkv,
-                                               split, st);
+            return ftq::launch_attn_merge_d256(out_dtype, partials, out, seq_lens, S, B, Hq, n_chunks,
+                                               chunk_tokens, n_vec, signs, r, st);
     }
     return cudaErrorInvalidValue;
 }
@@ -787,8 +804,9 @@ int ftq_flash_decode(const void* q, int q_dtype, int q_is_rotated, const uint8_t
     if (!aligned(q, 16) || !aligned(out, 4)) return fail(FTQ_ERR_INVALID, "q must be 16-byte aligned");
     if (!aligned(k_codes, 4) || !aligned(v_codes, 4) || !aligned(k_norms, 2) || !aligned(v_norms, 2))
         return fail(FTQ_ERR_INVALID, "misaligned K/V tensor");
-    const ChunkPlan pl = plan_chunks(B, Hq, Hkv, head_dim, round_seq(S), 1);
-    const size_t need = partial_bytes(pl, B, Hq, head_dim, 1);
+    const ChunkPlan most = plan_chunks(B, Hq, Hkv, head_dim, round_seq(S), 1);
+    const ChunkPlan pl = seq_lens ? most : plan_chunks_uniform(B, Hq, Hkv, head_dim, S);
+    const size_t need = partial_bytes(most, B, Hq, head_dim, 1);
     if (!workspace || workspace_bytes < need)
         return fail(FTQ_ERR_WORKSPACE, "workspace needs %zu bytes, got %zu", need, workspace_bytes);
     if (!aligned(workspace, 16)) return fail(FTQ_ERR_WORKSPACE, "workspace must be 16-byte aligned");
@@ -812,8 +830,8 @@ int ftq_flash_decode(const void* q, int q_dtype, int q_is_rotated, const uint8_t
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = dispatch_split(head_dim, bits_k, bits_v, false, p, B, st);
     if (e != cudaSuccess) return cuda_fail(e, "ftq_flash_decode split launch");
-    e = dispatch_merge(head_dim, out_dtype, p.partials, out, seq_lens, S, B, Hq, Hkv, pl,
-                       ftq::SplitPlan{}, static_cast<int64_t>(B) * Hq, p.signs, st);
+    e = dispatch_merge(head_dim, out_dtype, p.partials, out, seq_lens, S, B, Hq, pl.n_chunks,
+                       pl.chunk_tokens, static_cast<int64_t>(B) * Hq, p.signs, st);
     return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_flash_decode merge launch");
 }
 
@@ -951,8 +969,8 @@ int ftq_paged_decode_attn(const void* q, int q_dtype, void* out, int out_dtype,
         e = dispatch_split(head_dim, bits_k, bits_v, true, p, n_layers * B, st);
     }
     if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_decode_attn split launch");
-    e = dispatch_merge(head_dim, out_dtype, p.partials, out, seq_lens, 0, B, Hq, Hkv, pl,
-                       p.split, static_cast<int64_t>(n_layers) * B * Hq, p.signs, st);
+    e = dispatch_merge(head_dim, out_dtype, p.partials, out, seq_lens, 0, B, Hq, pl.n_chunks,
+                       pl.chunk_tokens, static_cast<int64_t>(n_layers) * B * Hq, p.signs, st);
     return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_paged_decode_attn merge launch");
 }
 
@@ -1208,11 +1226,8 @@ extern "C" int ftq_paged_chunk_attn(const void* q, int q_dtype, void* out, int o
         default: e = ftq::launch_attn_chunk_d256(bits_k, bits_v, p, B, st); break;
     }
     if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_chunk_attn launch");
-    ChunkPlan pl{};
-    pl.n_chunks = p.splits;
-    pl.chunk_tokens = 1;
-    e = dispatch_merge(head_dim, out_dtype, p.partials, out, nullptr, p.splits, B, Hq, Hkv, pl,
-                       ftq::SplitPlan{}, static_cast<int64_t>(B) * q_len * Hq, p.signs, st);
+    e = dispatch_merge(head_dim, out_dtype, p.partials, out, nullptr, p.splits, B, Hq, p.splits, 1,
+                       static_cast<int64_t>(B) * q_len * Hq, p.signs, st);
     return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_paged_chunk_attn merge launch");
 }
 

@@ -336,19 +336,23 @@ attn_split_kernel(const AttnParams p) {
     }
     __syncthreads();
 
-    float qr[GH][E];
+    // queries and accumulators as pairs of adjacent coordinates: packed fp32 FMAs (two independent IEEE
+    // FMAs per instruction)
+    constexpr int EP = E / 2;
+    u64 qr[GH][EP], acc[GH][EP];
 #pragma unroll
     for (int h = 0; h < GH; h++)
 #pragma unroll
-        for (int r = 0; r < E; r++) qr[h][r] = qs[h * D + t * E + r];
+        for (int i = 0; i < EP; i++)
+            qr[h][i] = pk2(qs[h * D + t * E + 2 * i], qs[h * D + t * E + 2 * i + 1]);
 
-    float m_run[GH], l_run[GH], acc[GH][E];
+    float m_run[GH], l_run[GH];
 #pragma unroll
     for (int h = 0; h < GH; h++) {
         m_run[h] = -INFINITY;
         l_run[h] = 0.f;
 #pragma unroll
-        for (int r = 0; r < E; r++) acc[h][r] = 0.f;
+        for (int i = 0; i < EP; i++) acc[h][i] = pk2(0.f, 0.f);
     }
 
     // ---- main loop over 64-token tiles, double buffered
@@ -374,14 +378,18 @@ attn_split_kernel(const AttnParams p) {
                 load_code_bytes<NBK>(page + tk * PDK + t * NBK, w);
                 const float kn =
                     __half2float(reinterpret_cast<const __half*>(page + OFF_KN)[tk]);
-                float kv[E];
+                u64 kv[EP];
 #pragma unroll
-                for (int r = 0; r < E; r++) kv[r] = lutk[extract_code<BK>(w, r)];
+                for (int i = 0; i < EP; i++)
+                    kv[i] = pk2(lutk[extract_code<BK>(w, 2 * i)], lutk[extract_code<BK>(w, 2 * i + 1)]);
 #pragma unroll
                 for (int h = 0; h < GH; h++) {
-                    float d = 0.f;
+                    u64 d2 = pk2(0.f, 0.f);
 #pragma unroll
-                    for (int r = 0; r < E; r++) d = fmaf(qr[h][r], kv[r], d);
+                    for (int i = 0; i < EP; i++) d2 = fma2(qr[h][i], kv[i], d2);
+                    float d0, d1;
+                    upk2(d2, d0, d1);
+                    float d = d0 + d1;
                     d += __shfl_xor_sync(0xffffffffu, d, 1);
                     d += __shfl_xor_sync(0xffffffffu, d, 2);
                     d += __shfl_xor_sync(0xffffffffu, d, 4);
@@ -406,8 +414,9 @@ attn_split_kernel(const AttnParams p) {
                     wp[step][h] = pe;
                 }
                 l_run[h] = l_run[h] * corr + ls;
+                const u64 corr2 = pk2(corr, corr);
 #pragma unroll
-                for (int r = 0; r < E; r++) acc[h][r] *= corr;
+                for (int i = 0; i < EP; i++) acc[h][i] = mul2(acc[h][i], corr2);
             }
 
 #pragma unroll
@@ -419,14 +428,16 @@ attn_split_kernel(const AttnParams p) {
                 load_code_bytes<NBV>(page + OFF_VC + tk * PDV + vt * NBV, w);
                 const float vn = tk < ntok
                     ? __half2float(reinterpret_cast<const __half*>(page + OFF_VN)[tk]) : 0.f;
-                float vv[E];
+                u64 vv[EP];
 #pragma unroll
-                for (int r = 0; r < E; r++) vv[r] = lutv[extract_code<BV>(w, r)];
+                for (int i = 0; i < EP; i++)
+                    vv[i] = pk2(lutv[extract_code<BV>(w, 2 * i)], lutv[extract_code<BV>(w, 2 * i + 1)]);
 #pragma unroll
                 for (int h = 0; h < GH; h++) {
                     const float wgt = tk < ntok ? wp[step][h] * vn : 0.f;
+                    const u64 wgt2 = pk2(wgt, wgt);
 #pragma unroll
-                    for (int r = 0; r < E; r++) acc[h][r] = fmaf(wgt, vv[r], acc[h][r]);
+                    for (int i = 0; i < EP; i++) acc[h][i] = fma2(wgt2, vv[i], acc[h][i]);
                 }
             }
         }
@@ -439,9 +450,9 @@ attn_split_kernel(const AttnParams p) {
         l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 8);
         l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 16);
 #pragma unroll
-        for (int r = 0; r < E; r++) {
-            acc[h][r] += __shfl_xor_sync(0xffffffffu, acc[h][r], 8);
-            acc[h][r] += __shfl_xor_sync(0xffffffffu, acc[h][r], 16);
+        for (int i = 0; i < EP; i++) {
+            acc[h][i] = add2(acc[h][i], __shfl_xor_sync(0xffffffffu, acc[h][i], 8));
+            acc[h][i] = add2(acc[h][i], __shfl_xor_sync(0xffffffffu, acc[h][i], 16));
         }
     }
     float* wacc = reinterpret_cast<float*>(tiles);   // [4][GH][D]   (tiles are free now)
@@ -451,7 +462,8 @@ attn_split_kernel(const AttnParams p) {
 #pragma unroll
         for (int h = 0; h < GH; h++) {
 #pragma unroll
-            for (int r = 0; r < E; r++) wacc[(warp * GH + h) * D + t * E + r] = acc[h][r];
+            for (int i = 0; i < EP; i++)
+                *reinterpret_cast<u64*>(wacc + (warp * GH + h) * D + t * E + 2 * i) = acc[h][i];
             if (t == 0) {
                 wm[warp * GH + h] = m_run[h];
                 wl[warp * GH + h] = l_run[h];
@@ -488,66 +500,64 @@ attn_split_kernel(const AttnParams p) {
 
 // Merge the chunk partials of one (layer, sequence, query head), normalise,
 // rotate back to the original space (inverse_randomized_hadamard,
-// core/hadamard.py:93-100) and store.  One octet per output vector.
-template <int D, typename OT>
+// core/hadamard.py:93-100) and store.  OCTETS octets per output vector: each takes every OCTETS-th
+// chunk's row, and their sums are added up with shuffles.  What bounds it is the latency of the
+// rows' loads, so the loop has nothing that keeps the next row's loads from being issued.  (An octet
+// per vector with a branch per row took 23 us of the 65 us of a call with 128 vectors of 32 chunks.)
+template <int D, typename OT, int OCTETS>
 __global__ void __launch_bounds__(128)
 attn_merge_kernel(const float* __restrict__ partials, OT* __restrict__ out,
                   const int32_t* __restrict__ seq_lens, int S, int B, int Hq, int n_chunks,
-                  int chunk_tokens, int64_t n_vec, SignBits signs, float rsqrt_d, int Hkv,
-                  const SplitPlan split) {
+                  int chunk_tokens, int64_t n_vec, SignBits signs, float rsqrt_d) {
     constexpr int E = D / kOctet;
     constexpr int ROW = D + 4;
     const int lane = threadIdx.x & 31;
-    const int t = lane & 7;
-    const int64_t v = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
-    const bool valid = v < n_vec;
-    int nc = 0;
-    if (valid) {
-        const int b = static_cast<int>((v / Hq) % B);
-        const int len = seq_lens ? (S > 0 ? min(seq_lens[b], S) : seq_lens[b]) : S;
-        // the unit's region tells how many chunks it was cut into (split.n_regions == 0: one
-        // split for all units, n_chunks / chunk_tokens)
-        int ncr = n_chunks, ct = chunk_tokens;
-        if (split.n_regions > 0) {
-            const int unit = static_cast<int>((v / Hq) * Hkv + (v % Hq) / (Hq / Hkv));
-            const SplitRegion& rg = region_of_unit(split, unit);
-            ncr = rg.chunks;
-            ct = rg.chunk_tokens;
-        }
-        nc = min(ncr, (len + ct - 1) / ct);
-    }
-    const float* rows =
-        partials + (valid ? v : 0) * (split.n_regions > 0 ? split.row_chunks : n_chunks) * ROW;
+    const int t = lane & 7, o = (lane >> 3) & (OCTETS - 1);
+    const int64_t at = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / (8 * OCTETS);
+    const int64_t v = at < n_vec ? at : n_vec - 1;   // (octets left over repeat the last vector)
+    const int b = static_cast<int>((v / Hq) % B);
+    const int len = seq_lens ? (S > 0 ? min(seq_lens[b], S) : seq_lens[b]) : S;
+    const int nc = min(n_chunks, (len + chunk_tokens - 1) / chunk_tokens);
+    const float* rows = partials + v * n_chunks * ROW;
     float M = -INFINITY;
-    for (int c = 0; c < nc; c++) M = fmaxf(M, rows[c * ROW + D]);
+    for (int c = 8 * o + t; c < nc; c += 8 * OCTETS) M = fmaxf(M, rows[static_cast<int64_t>(c) * ROW + D]);
+#pragma unroll
+    for (int m = 1; m < 8 * OCTETS; m <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, m));
     float a[E];
 #pragma unroll
     for (int r = 0; r < E; r++) a[r] = 0.f;
     float L = 0.f;
-    for (int c = 0; c < nc; c++) {
-        const float mc = rows[c * ROW + D];
-        if (mc == -INFINITY) continue;
-        const float f = __expf(mc - M);
-        L = fmaf(rows[c * ROW + D + 1], f, L);
+#pragma unroll 2
+    for (int c = o; c < nc; c += OCTETS) {
+        const float* row = rows + static_cast<int64_t>(c) * ROW;
+        const float mc = row[D];
+        const bool live = mc != -INFINITY;   // (the vector of a dead chunk's row was never written)
+        const float f = live ? __expf(mc - M) : 0.f;
+        L = live ? fmaf(row[D + 1], f, L) : L;
 #pragma unroll
         for (int i = 0; i < E / 8; i++) {
             float tmp[8];
-            load8<float>(rows + c * ROW + 8 * (t + 8 * i), tmp);
+            load8<float>(row + 8 * (t + 8 * i), tmp);
 #pragma unroll
-            for (int cc = 0; cc < 8; cc++) a[8 * i + cc] = fmaf(tmp[cc], f, a[8 * i + cc]);
+            for (int cc = 0; cc < 8; cc++) a[8 * i + cc] = live ? fmaf(tmp[cc], f, a[8 * i + cc]) : a[8 * i + cc];
         }
+    }
+#pragma unroll
+    for (int m = 8; m < 8 * OCTETS; m <<= 1) {
+        L += __shfl_xor_sync(0xffffffffu, L, m);
+#pragma unroll
+        for (int r = 0; r < E; r++) a[r] += __shfl_xor_sync(0xffffffffu, a[r], m);
     }
     const float inv = L > 0.f ? 1.f / L : 0.f;
 #pragma unroll
     for (int r = 0; r < E; r++) a[r] *= inv;
     octet_fwht<E>(a, lane);
-    if (valid) {
 #pragma unroll
-        for (int k = 0; k < E; k++) {
-            const float r = a[k] * rsqrt_d;
-            out[v * D + t + 8 * k] =
-                from_float<OT>(__uint_as_float(__float_as_uint(r) ^ sign_mask(signs, t + 8 * k)));
-        }
+    for (int k = 0; k < E; k++) {
+        if (at >= n_vec || (k & (OCTETS - 1)) != o) continue;   // (every octet of the vector holds the result and stores its part)
+        const float r = a[k] * rsqrt_d;
+        out[v * D + t + 8 * k] =
+            from_float<OT>(__uint_as_float(__float_as_uint(r) ^ sign_mask(signs, t + 8 * k)));
     }
 }
 

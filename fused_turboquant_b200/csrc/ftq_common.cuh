@@ -30,6 +30,7 @@ namespace ftq {
 constexpr int kOctet = 8;          // lanes per head vector
 constexpr int kPageTokens = 16;    // tokens per page
 constexpr int kMaxLevels = 16;
+constexpr int kWideMerge = 16;     // vectors per SM up to which a merge kernel gives each a whole warp
 
 enum : int { kF32 = 0, kF16 = 1, kBF16 = 2 };
 
@@ -46,6 +47,39 @@ struct SignBits {
 struct Codebook {
     float v[kMaxLevels];  // levels[0 .. 2^bits)  or interior boundaries [1 .. 2^bits) at v[0..]
 };
+
+// ---------------------------------------------------------------- packed fp32 pairs
+
+typedef unsigned long long u64;
+
+__device__ __forceinline__ u64 pk2(float lo, float hi) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void upk2(u64 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+    u64 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 sub2(u64 a, u64 b) {
+    u64 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+    u64 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 
 // ---------------------------------------------------------------- loads
 

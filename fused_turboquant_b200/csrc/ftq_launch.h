@@ -24,8 +24,7 @@ namespace ftq {
     cudaError_t launch_attn_merge_d##DD(int out_dtype, const float* partials, void* out,        \
                                         const int32_t* seq_lens, int S, int B, int Hq,          \
                                         int n_chunks, int chunk_tokens, int64_t n_vec,          \
-                                        const SignBits& signs, float rsqrt_d, int Hkv,          \
-                                        const SplitPlan& split, cudaStream_t stream);
+                                        const SignBits& signs, float rsqrt_d, cudaStream_t stream);
 
 FTQ_DECLARE_LAUNCHERS(64)
 FTQ_DECLARE_LAUNCHERS(128)

@@ -881,10 +881,12 @@ struct TqMergeParams {
     const float* prefix_lse;  // [n_rows]
 };
 
-// Merge the split partials of 4 (sequence, query head) rows per warp: softmax-weighted by lse,
-// optionally Hadamard-transform the result, optionally merge a prefix result in, cast and store.
-// mid_o rows with lse = -inf are skipped.
-template <int D, typename OT>
+// Merge the split partials of a (sequence, query head) row: softmax-weighted by lse, optionally
+// Hadamard-transform the result, optionally merge a prefix result in, cast and store.  mid_o rows with
+// lse = -inf are skipped.  OCTETS octets per row take every OCTETS-th split each and nothing keeps the
+// next split's loads from being issued: the latency of the loads bounds it (an octet per row and a
+// branch per split took 9.6 us for 1024 rows of 8 splits).
+template <int D, typename OT, int OCTETS>
 __global__ void __launch_bounds__(128)
 tq_merge_kernel(const TqMergeParams p) {
     const float* __restrict__ mid_o = p.mid_o;
@@ -895,24 +897,36 @@ tq_merge_kernel(const TqMergeParams p) {
     const float rsqrt_d = p.rsqrt_d;
     constexpr int E = D / kOctet;
     const int lane = threadIdx.x & 31;
-    const int t = lane & 7;
-    const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 8;
-    const bool valid = row < n_rows;
-    const float* base = mid_o + (valid ? row : 0) * static_cast<int64_t>(splits) * (D + 1);
+    const int t = lane & 7, o = (lane >> 3) & (OCTETS - 1);
+    const int64_t at = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / (8 * OCTETS);
+    const int64_t row = at < n_rows ? at : n_rows - 1;   // (octets left over repeat the last row)
+    const float* base = mid_o + row * static_cast<int64_t>(splits) * (D + 1);
     float M = -INFINITY;
-    for (int s = 0; s < splits; s++) M = fmaxf(M, base[static_cast<int64_t>(s) * (D + 1) + D]);
+    for (int s = 8 * o + t; s < splits; s += 8 * OCTETS) M = fmaxf(M, base[static_cast<int64_t>(s) * (D + 1) + D]);
+#pragma unroll
+    for (int m = 1; m < 8 * OCTETS; m <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, m));
     float a[E];
 #pragma unroll
     for (int r = 0; r < E; r++) a[r] = 0.f;
     float l = 0.f;
-    for (int s = 0; s < splits; s++) {
+#pragma unroll 2
+    for (int s = o; s < splits; s += OCTETS) {
         const float* ps = base + static_cast<int64_t>(s) * (D + 1);
         const float ls = ps[D];
-        if (ls == -INFINITY) continue;
-        const float f = __expf(ls - M);
+        const bool live = ls != -INFINITY;
+        const float f = live ? __expf(ls - M) : 0.f;
         l += f;
 #pragma unroll
-        for (int r = 0; r < E; r++) a[r] = fmaf(ps[load_coord(t, r)], f, a[r]);
+        for (int r = 0; r < E; r++) {
+            const float x = ps[load_coord(t, r)];
+            a[r] = live ? fmaf(x, f, a[r]) : a[r];
+        }
+    }
+#pragma unroll
+    for (int m = 8; m < 8 * OCTETS; m <<= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, m);
+#pragma unroll
+        for (int r = 0; r < E; r++) a[r] += __shfl_xor_sync(0xffffffffu, a[r], m);
     }
     const float inv = l > 0.f ? 1.f / l : 0.f;
 #pragma unroll
@@ -922,7 +936,6 @@ tq_merge_kernel(const TqMergeParams p) {
 #pragma unroll
         for (int k = 0; k < E; k++) a[k] *= rsqrt_d;
     }
-    if (!valid) return;
     float lse = l > 0.f ? M + logf(l) : -INFINITY;
     float w_own = 1.f, w_pre = 0.f;
     const bool prefix = p.prefix_out != nullptr;
@@ -942,6 +955,7 @@ tq_merge_kernel(const TqMergeParams p) {
     OT* orow = out + row * D;
 #pragma unroll
     for (int r = 0; r < E; r++) {
+        if (at >= n_rows || (r & (OCTETS - 1)) != o) continue;   // (every octet of the row holds the result and stores its part)
         const int coord = rotate ? t + 8 * r : load_coord(t, r);
         float v = a[r];
         if (prefix) {
@@ -956,7 +970,7 @@ tq_merge_kernel(const TqMergeParams p) {
         else if constexpr (std::is_same<OT, __half>::value) orow[coord] = __float2half_rn(v);
         else orow[coord] = __float2bfloat16_rn(v);
     }
-    if (lse_out && t == 0) lse_out[row] = lse;
+    if (lse_out && t == 0 && o == 0 && at < n_rows) lse_out[row] = lse;
 }
 
 }  // namespace ftq

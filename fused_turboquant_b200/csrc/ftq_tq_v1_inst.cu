@@ -173,16 +173,25 @@ cudaError_t FTQ_CAT(launch_tq_mma_d, FTQ_D)(int kb, int vb, int nh, const TqDeco
     return cudaErrorInvalidValue;
 }
 
+template <typename OT>
+static cudaError_t run_tq_merge(const TqMergeParams& p, cudaStream_t stream) {
+    // (as in the page-layout merge: a warp per row where there are few of them)
+    if (p.n_rows <= 0) return cudaSuccess;
+    const int octets = p.n_rows <= kWideMerge * sm_count() ? 4 : 1;
+    const unsigned grid = static_cast<unsigned>((p.n_rows * octets + 15) / 16);
+    if (octets == 4) tq_merge_kernel<FTQ_D, OT, 4><<<grid, 128, 0, stream>>>(p);
+    else tq_merge_kernel<FTQ_D, OT, 1><<<grid, 128, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
 cudaError_t FTQ_CAT(launch_tq_merge_d, FTQ_D)(int out_dtype, const TqMergeParams& p,
                                              cudaStream_t stream) {
-    const unsigned grid = static_cast<unsigned>((p.n_rows + 15) / 16);  // 128 threads = 16 rows
     switch (out_dtype) {
-        case kF32: tq_merge_kernel<FTQ_D, float><<<grid, 128, 0, stream>>>(p); break;
-        case kF16: tq_merge_kernel<FTQ_D, __half><<<grid, 128, 0, stream>>>(p); break;
-        case kBF16: tq_merge_kernel<FTQ_D, __nv_bfloat16><<<grid, 128, 0, stream>>>(p); break;
-        default: return cudaErrorInvalidValue;
+        case kF32: return run_tq_merge<float>(p, stream);
+        case kF16: return run_tq_merge<__half>(p, stream);
+        case kBF16: return run_tq_merge<__nv_bfloat16>(p, stream);
     }
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 #endif  // FTQ_TQ_DECODE

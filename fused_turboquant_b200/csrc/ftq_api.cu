@@ -1464,7 +1464,17 @@ extern "C" int ftq_tq_decode_layers(const void* q, int q_dtype, int B, int Hq, i
     const bool mma = q_dtype != FTQ_F32 && group <= 8 && key_bits >= 2 && key_bits <= 4 && value_bits >= 2 &&
                      value_bits != 8 && head_dim != 256 && aligned(kv_cache, 4) &&
                      !p.value_lloyd_max;
-    if (mma) {
+    // FP8 keys under the same conditions take a tensor-core kernel of fp32 precision; its copies are
+    // 4-byte words, so every slot has to start on one
+    const int64_t strides = stride_block | stride_pos | stride_head | cache_layer_stride;
+    const bool fp8 = key_fp8 && q_dtype != FTQ_F32 && group <= 8 && value_bits >= 2 && value_bits <= 4 &&
+                     head_dim != 256 && aligned(kv_cache, 4) && strides % 4 == 0 &&
+                     static_cast<int64_t>(B) * Hkv * num_kv_splits < (1ll << 31);
+    if (fp8) {
+        const int items = B * Hkv * num_kv_splits, nh = group <= 4 ? 1 : 2;
+        e = head_dim == 64 ? ftq::launch_tq_fp8_d64(value_bits, nh, p, items, st)
+                           : ftq::launch_tq_fp8_d128(value_bits, nh, p, items, st);
+    } else if (mma) {
         // key centroids scaled for the smallest fp16 rounding error of the table (see
         // choose_k_scale).  With norm correction the factor cancels by itself (the centroid
         // vector is re-normalised with the scaled centroids); without, it goes into the

@@ -1,0 +1,422 @@
+// vLLM-v1 slot format with FP8 keys, decode stage 1 on the tensor cores at fp32 precision.
+//
+// Same result as tq_split_kernel (ftq_tq_v1.cuh), i.e. the reference's
+// `_tq_decode_stage1_offset` (src/fused_turboquant/vllm_plugin/triton_decode_offset.py:42-444), partials
+// in the same [B, Hq, splits, D + 1] layout.  That kernel spends 1500 instructions on a 16-token page
+// (fp32 FMAs per query head, shuffles per score) and was issue bound at 137 us for 16 x 4096 tokens of
+// 8 heads; here both products are m16n8k16 MMAs whose operands lose nothing:
+//   * e4m3 keys and the centred 2- to 4-bit value codes are exact in fp16;
+//   * a rotated query is the sum of two fp16 numbers, hi + lo / 2^11, after scaling by a power of two that
+//     puts the head's largest coordinate in [2^10, 2^11): 23 bits of that coordinate's magnitude;
+//   * a softmax weight (times the value scale) is split the same way.
+// Accumulation is fp32.  With at most four heads the eight columns of an MMA are (head, hi / lo), so the
+// split costs no MMA; with five to eight heads hi and lo are one MMA each.
+//
+// Fragment maps for a page of 16 tokens (lane = 4 g + tg):
+//   S: A rows g, g + 8 = tokens, k-block kb = coordinates (D/4) tg + 4 kb + {0..3} (word kb of the lane's
+//      key slice), C columns 2tg, 2tg + 1 = (head tg, hi / lo) or heads 2tg, 2tg + 1
+//   O^T: A rows g, g + 8 of m-tile mt = coordinates (D/8) g + 2 mt, + 1, k = tokens; B = the weights,
+//      packed per token and transposed by movmatrix
+//
+// Work: persistent CTAs over (split, KV head, sequence) items, the pages of an item dealt to the warps.
+// A warp's copies (cp.async, 4 bytes: slots are only 4-byte aligned; eight lanes per slot) run STAGES - 1
+// pages ahead of its arithmetic and across items.
+#pragma once
+
+#include <cuda_fp8.h>
+
+#include "ftq_attn_mma.cuh"
+#include "ftq_tq_v1.cuh"
+
+namespace ftq {
+
+template <int D, int VB, int NH>
+struct TqFp8Cfg {
+    static constexpr int NKB = D / 16, NMT = D / 16;
+    static constexpr int WARPS = 8, THREADS = 32 * WARPS;
+    static constexpr int PDV = D * VB / 8, VSB = PDV / 8, VW = (VSB + 3) / 4;
+    static constexpr int USED = D + PDV + 4, NW = USED / 4;      // bytes and words of a slot
+    // an odd number of 16-byte units: the rows g, g + 1 of a 16-byte load fall into distinct banks
+    static constexpr int ROWB = ((USED + 15) / 16 | 1) * 16;
+    static constexpr int PAGE = kPageTokens * ROWB;
+    static constexpr int STAGES = NH == 1 ? 3 : 2;
+    static constexpr int HL = NH;                                // heads whose state a lane keeps
+    static constexpr int OL = NMT * 2 * HL;                      // output floats of a lane
+    static constexpr int QS = 8 * (D + 16) * 4;
+    static constexpr int XO = WARPS * 32 * OL * 4, XML = WARPS * 3 * 8 * 4;
+    static constexpr int SMEM_BYTES = WARPS * STAGES * PAGE + QS + 8 * 4 + XO + XML + 64;
+    static_assert(USED % 4 == 0 && 2 * SMEM_BYTES <= 226 * 1024, "two CTAs per SM");
+};
+
+template <int D, int VB, int NH>
+__global__ void __launch_bounds__(TqFp8Cfg<D, VB, NH>::THREADS, 2)
+tq_fp8_kernel(const TqDecodeParams p, int n_items) {
+    using C = TqFp8Cfg<D, VB, NH>;
+    constexpr int NKB = C::NKB, NMT = C::NMT, WARPS = C::WARPS, HL = C::HL, E = D / kOctet;
+    constexpr float kLo = 2048.f, kInvLo = 1.f / 2048.f;
+    // codes are centred and the zero point moved accordingly: the sums of code * scale and of zero would
+    // be large numbers of opposite sign otherwise (a centre half a code off costs a factor of five in
+    // the error of a mean over 500 tokens of 2-bit values)
+    constexpr float kCtr = 0.5f * ((1 << VB) - 1);
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, tg = lane & 3;
+    const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw)) + warp * C::STAGES * C::PAGE;
+    float* qs = reinterpret_cast<float*>(smem_raw + WARPS * C::STAGES * C::PAGE);   // [8][D + 16]
+    float* qmul = qs + 8 * (D + 16);                                               // [8]
+    float* xo = qmul + 8;                                                          // [WARPS][OL][32]
+    float* xml = xo + C::XO / 4;                                                   // [WARPS][3][8]
+    const int group = p.Hq / p.Hkv;
+
+    struct Item { int sid, hkv, b, bs, layer, t0, t1, n_pages; };
+    auto item_info = [&](int item) {
+        Item it;
+        it.sid = item % p.splits;
+        const int r = item / p.splits;
+        it.hkv = r % p.Hkv;
+        it.b = r / p.Hkv;   // (layer, sequence) row
+        it.layer = static_cast<int>(fast_div(static_cast<uint32_t>(it.b), p.div_bseq));
+        it.bs = it.b - it.layer * p.B_seq;
+        const int seq_len = p.seq_lens[it.bs];
+        const int kv_start = p.kv_start ? p.kv_start[it.bs] : 0;
+        const int split_len = (seq_len - kv_start + p.splits - 1) / p.splits;
+        it.t0 = kv_start + split_len * it.sid;
+        it.t1 = min(it.t0 + split_len, seq_len);
+        it.n_pages = it.t1 > it.t0 ? (it.t1 - it.t0 + kPageTokens - 1) / kPageTokens : 0;
+        return it;
+    };
+    auto mid_row = [&](const Item& it, int h) {
+        return p.mid_o + ((static_cast<int64_t>(it.b) * p.Hq + it.hkv * group + h) * p.splits + it.sid) * (D + 1);
+    };
+
+    // ---- copies: the warp's pages of all its items, in the order of the arithmetic below
+    int c_item = blockIdx.x, c_page = warp, c_stage = 0;
+    uint32_t stage_bad = 0;   // bit s: a block id of the page in ring buffer s was out of range
+    Item c_it = item_info(c_item < n_items ? c_item : 0);
+    auto copy_next = [&]() {
+        while (c_item < n_items && c_page >= c_it.n_pages) {
+            c_item += gridDim.x;
+            c_page = warp;
+            if (c_item < n_items) c_it = item_info(c_item);
+        }
+        if (c_item < n_items) {   // (warp-uniform)
+            // tokens past the end of the range re-read the last valid slot (their weight is zero)
+            const int pos = min(c_it.t0 + c_page * kPageTokens + (lane & 15), c_it.t1 - 1);
+            const uint32_t blk = fast_div(static_cast<uint32_t>(pos), p.div_block);
+            const uint32_t off = static_cast<uint32_t>(pos) - blk * p.block_size;
+            int64_t id = p.block_table[static_cast<int64_t>(c_it.bs) * p.max_blocks + blk];
+            const bool bad = p.num_blocks > 0 && static_cast<uint64_t>(id) >= static_cast<uint64_t>(p.num_blocks);
+            if (bad) id = 0;
+            const bool any_bad = __any_sync(0xffffffffu, bad);
+            stage_bad = (stage_bad & ~(1u << c_stage)) | (static_cast<uint32_t>(any_bad) << c_stage);
+            const uint8_t* sp = p.kv_cache + c_it.layer * p.cache_layer_stride + id * p.stride_block +
+                                off * p.stride_pos + c_it.hkv * p.stride_head;
+            const uint32_t dst = ring + c_stage * C::PAGE + 4 * (lane & 7);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int tk = (lane >> 3) + 4 * k;
+                const uint8_t* src = reinterpret_cast<const uint8_t*>(__shfl_sync(
+                                         0xffffffffu, reinterpret_cast<unsigned long long>(sp), tk)) + 4 * (lane & 7);
+#pragma unroll
+                for (int j = 0; j < (C::NW + 7) / 8; j++)
+                    if (8 * j + 7 < C::NW || 8 * j + (lane & 7) < C::NW)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst + tk * C::ROWB + 32 * j),
+                                     "l"(src + 32 * j));
+            }
+            c_page += WARPS;
+        }
+        cp_async_commit();
+        c_stage = c_stage + 1 == C::STAGES ? 0 : c_stage + 1;
+    };
+#pragma unroll
+    for (int i = 0; i < C::STAGES - 1; i++) copy_next();
+    int stage = 0;
+
+    auto qs_index = [](int head, int coord) {
+        return head * (D + 16) + (coord / (D / 4)) * (D / 4 + 4) + coord % (D / 4);
+    };
+    auto pack = [](float lo, float hi) {
+        const __half2 h = __floats2half2_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    };
+    auto residual = [&](float x) { return (x - __half2float(__float2half_rn(x))) * kLo; };
+
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+        const Item it = item_info(item);
+        if (it.n_pages == 0) {   // neutral partial (CTA-uniform): zeros and lse = -inf
+            for (int idx = tid; idx < group * (D + 1); idx += C::THREADS) {
+                const int h = idx / (D + 1), d = idx - h * (D + 1);
+                mid_row(it, h)[d] = d == D ? -INFINITY : 0.f;
+            }
+            continue;
+        }
+        __syncthreads();   // (the item before has been folded)
+        if (warp < NH) {   // rotate (no signs) and normalise the group's queries, an octet per head
+            const int t8 = lane & 7, hh = warp * 4 + (lane >> 3);
+            const bool hv = hh < group;
+            const int64_t qoff = (static_cast<int64_t>(it.b) * p.Hq + it.hkv * group + (hv ? hh : 0)) * D;
+            float a[E];
+#pragma unroll
+            for (int i = 0; i < E / 8; i++) {
+                float tmp[8];
+                const int64_t eo = qoff + 8 * (t8 + 8 * i);
+                if (p.q_dtype == kBF16) load8<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.q) + eo, tmp);
+                else load8<__half>(static_cast<const __half*>(p.q) + eo, tmp);
+#pragma unroll
+                for (int c = 0; c < 8; c++) a[8 * i + c] = tmp[c];
+            }
+            octet_fwht<E>(a, lane);
+            float mx = 0.f;
+#pragma unroll
+            for (int k = 0; k < E; k++) {
+                a[k] *= p.rsqrt_d;
+                mx = fmaxf(mx, fabsf(a[k]));
+            }
+#pragma unroll
+            for (int m = 1; m < 8; m <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, m));
+            // power of two that brings mx into [2^10, 2^11) (1 for zero, infinite or NaN rows)
+            int e = static_cast<int>((__float_as_uint(mx) >> 23) & 255u);
+            e = e == 255 || mx == 0.f ? 0 : min(120, 127 + 10 - e);
+            const float up = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+            const float down = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
+#pragma unroll
+            for (int k = 0; k < E; k++) qs[qs_index(hh, t8 + 8 * k)] = hv ? a[k] * up : 0.f;
+            if (t8 == 0) qmul[hh] = p.scale * kLog2e * down;
+        }
+        __syncthreads();
+
+        // B fragments: column g = (head g >> 1, hi for an even g, lo for an odd one), or head g (hi, lo)
+        uint32_t qb[NH][NKB][2];
+#pragma unroll
+        for (int kb = 0; kb < NKB; kb++) {
+            const float4 q4 = *reinterpret_cast<const float4*>(qs + qs_index(NH == 1 ? g >> 1 : g, (D / 4) * tg + 4 * kb));
+            const uint32_t h0 = pack(q4.x, q4.y), h1 = pack(q4.z, q4.w);
+            const uint32_t l0 = pack(residual(q4.x), residual(q4.y)), l1 = pack(residual(q4.z), residual(q4.w));
+            if constexpr (NH == 1) {
+                qb[0][kb][0] = (g & 1) ? l0 : h0;
+                qb[0][kb][1] = (g & 1) ? l1 : h1;
+            } else {
+                qb[0][kb][0] = h0; qb[0][kb][1] = h1;
+                qb[NH - 1][kb][0] = l0; qb[NH - 1][kb][1] = l1;
+            }
+        }
+        float mul[HL];
+#pragma unroll
+        for (int h = 0; h < HL; h++) mul[h] = qmul[HL * tg + h];
+
+        float m_run[HL], l_run[HL], z_run[HL], oacc[NH][NMT][4];
+#pragma unroll
+        for (int h = 0; h < HL; h++) {
+            m_run[h] = -INFINITY;
+            l_run[h] = z_run[h] = 0.f;
+        }
+#pragma unroll
+        for (int x = 0; x < NH; x++)
+#pragma unroll
+            for (int mt = 0; mt < NMT; mt++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) oacc[x][mt][i] = 0.f;
+        bool bad_block = false;
+
+        for (int pg = warp; pg < it.n_pages; pg += WARPS) {
+            cp_async_wait<C::STAGES - 2>();
+            __syncwarp();   // the page is there for every lane; everybody is done with the one before
+            const uint32_t page = ring + stage * C::PAGE;
+            bad_block |= ((stage_bad >> stage) & 1u) != 0u;
+            copy_next();
+            stage = stage + 1 == C::STAGES ? 0 : stage + 1;
+
+            // ---- scores
+            float c[NH][2][4];
+#pragma unroll
+            for (int x = 0; x < NH; x++)
+#pragma unroll
+                for (int z = 0; z < 2; z++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) c[x][z][i] = 0.f;
+            const uint32_t rowa = page + g * C::ROWB, rowb = rowa + 8 * C::ROWB;
+#pragma unroll
+            for (int q = 0; q < NKB / 4; q++) {
+                const uint4 ka = lds128(rowa + (D / 4) * tg + 16 * q), kb4 = lds128(rowb + (D / 4) * tg + 16 * q);
+                const uint32_t wa[4] = {ka.x, ka.y, ka.z, ka.w}, wb[4] = {kb4.x, kb4.y, kb4.z, kb4.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    auto half2_of = [](uint32_t two) {
+                        const __half2_raw r = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(two), __NV_E4M3);
+                        return static_cast<uint32_t>(r.x) | (static_cast<uint32_t>(r.y) << 16);
+                    };
+                    const uint32_t a0 = half2_of(wa[j] & 0xffffu), a2 = half2_of(wa[j] >> 16);
+                    const uint32_t a1 = half2_of(wb[j] & 0xffffu), a3 = half2_of(wb[j] >> 16);
+#pragma unroll
+                    for (int x = 0; x < NH; x++)
+                        mma_16816(c[x][j & 1], a0, a1, a2, a3, qb[x][4 * q + j][0], qb[x][4 * q + j][1]);
+                }
+            }
+
+            // ---- online softmax (base-2 exponents), the lane's tokens g and g + 8
+            const int ntok = min(kPageTokens, it.t1 - it.t0 - pg * kPageTokens);
+            const bool okA = g < ntok, okB = g + 8 < ntok;
+            const uint32_t ma = lds32(rowa + D + C::PDV), mb = lds32(rowb + D + C::PDV);
+            const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&ma));
+            const float2 fb = __half22float2(*reinterpret_cast<const __half2*>(&mb));
+            const float vsa = okA ? fa.x : 0.f, vsb = okB ? fb.x : 0.f;
+            const float vza = okA ? fmaf(kCtr, fa.x, fa.y) : 0.f;
+            const float vzb = okB ? fmaf(kCtr, fb.x, fb.y) : 0.f;
+            float ra[HL], rb[HL], sa[HL], sb[HL];   // products; scaled scores
+            bool above = false;
+#pragma unroll
+            for (int h = 0; h < HL; h++) {
+                if constexpr (NH == 1) {
+                    ra[h] = fmaf(c[0][0][1] + c[0][1][1], kInvLo, c[0][0][0] + c[0][1][0]);
+                    rb[h] = fmaf(c[0][0][3] + c[0][1][3], kInvLo, c[0][0][2] + c[0][1][2]);
+                } else {
+                    ra[h] = fmaf(c[NH - 1][0][h] + c[NH - 1][1][h], kInvLo, c[0][0][h] + c[0][1][h]);
+                    rb[h] = fmaf(c[NH - 1][0][2 + h] + c[NH - 1][1][2 + h], kInvLo, c[0][0][2 + h] + c[0][1][2 + h]);
+                }
+                sa[h] = okA ? ra[h] * mul[h] : -INFINITY;
+                sb[h] = okB ? rb[h] * mul[h] : -INFINITY;
+                above |= fmaxf(sa[h], sb[h]) > m_run[h];   // (no slack: a weight is at most the value scale)
+            }
+            if (__any_sync(0xffffffffu, above)) {
+                float corr[HL];
+#pragma unroll
+                for (int h = 0; h < HL; h++) {
+                    float m = fmaxf(sa[h], sb[h]);
+                    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+                    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+                    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+                    const float m_new = fmaxf(m_run[h], m);   // finite: the page's first token is valid
+                    corr[h] = fast_exp2(m_run[h] - m_new);
+                    l_run[h] *= corr[h];
+                    z_run[h] *= corr[h];
+                    m_run[h] = m_new;
+                }
+#pragma unroll
+                for (int x = 0; x < NH; x++)
+#pragma unroll
+                    for (int mt = 0; mt < NMT; mt++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) oacc[x][mt][i] *= corr[NH == 1 ? 0 : (i & 1)];
+            }
+            uint32_t pb[NH][2];
+            {
+                float wa[HL], wb[HL];
+#pragma unroll
+                for (int h = 0; h < HL; h++) {
+                    // (the exponent in one rounding)
+                    const float pa = okA ? fast_exp2(fmaf(ra[h], mul[h], -m_run[h])) : 0.f;
+                    const float pbv = okB ? fast_exp2(fmaf(rb[h], mul[h], -m_run[h])) : 0.f;
+                    l_run[h] += pa + pbv;
+                    z_run[h] = fmaf(pa, vza, fmaf(pbv, vzb, z_run[h]));
+                    wa[h] = pa * vsa;
+                    wb[h] = pbv * vsb;
+                }
+                if constexpr (NH == 1) {
+                    pb[0][0] = movmatrix_trans(pack(wa[0], residual(wa[0])));
+                    pb[0][1] = movmatrix_trans(pack(wb[0], residual(wb[0])));
+                } else {
+                    pb[0][0] = movmatrix_trans(pack(wa[0], wa[HL - 1]));
+                    pb[0][1] = movmatrix_trans(pack(wb[0], wb[HL - 1]));
+                    pb[NH - 1][0] = movmatrix_trans(pack(residual(wa[0]), residual(wa[HL - 1])));
+                    pb[NH - 1][1] = movmatrix_trans(pack(residual(wb[0]), residual(wb[HL - 1])));
+                }
+            }
+
+            // ---- O^T += V^T.P^T.  Codes become fp16 arithmetically: or-ed into the mantissa of 1024 a
+            // code at bit s is 1024 + 2^s * code, and one packed FMA scales and centres it exactly (s >= 1:
+            // 2^(10 - s) + centre is then an fp16 number).  A 16-bit half of x holds the next codes of
+            // one token, the other half those of its neighbour.
+            uint32_t v[4][C::VW];
+            const uint32_t vrow = page + D + slice_word<C::VSB>(g) + 2 * tg * C::ROWB;
+            const uint32_t vsh = slice_shift<C::VSB>(g);
+            lds_slice<C::VSB>(vrow, vsh, v[0]);
+            lds_slice<C::VSB>(vrow + C::ROWB, vsh, v[1]);
+            lds_slice<C::VSB>(vrow + 8 * C::ROWB, vsh, v[2]);
+            lds_slice<C::VSB>(vrow + 9 * C::ROWB, vsh, v[3]);
+            constexpr int CPW = VB == 3 ? 5 : 16 / VB;     // whole codes in 16 bits
+            constexpr int CLO = VB == 3 ? 3 : CPW / 2;     // ... of which the first CLO are read from x << 1
+            constexpr int DOWN = VB * CLO - 1;             // the others from x >> DOWN
+            uint32_t h01[D / 8], h23[D / 8];               // [coordinate] tokens 2tg, 2tg + 1 / 2tg + 8, 2tg + 9
+            auto window = [&](const uint32_t (&a)[C::VW], const uint32_t (&b)[C::VW], int bit) {
+                const int j = bit >> 5, sh = bit & 31;
+                const uint32_t hi_a = a[j + 1 < C::VW ? j + 1 : j], hi_b = b[j + 1 < C::VW ? j + 1 : j];
+                const uint32_t x = sh == 0 ? a[j] : sh + 16 <= 32 ? a[j] >> sh : __funnelshift_r(a[j], hi_a, sh);
+                const uint32_t y = sh == 0 ? b[j] : sh + 16 <= 32 ? b[j] >> sh : __funnelshift_r(b[j], hi_b, sh);
+                return __byte_perm(x, y, 0x5410u);
+            };
+            auto code_half2 = [&](uint32_t up, uint32_t down, int i) {
+                const int sh = i < CLO ? VB * i + 1 : VB * i - DOWN;
+                const uint32_t w = ((i < CLO ? up : down) & (((1u << VB) - 1u) * 0x00010001u << sh)) | 0x64006400u;
+                const float inv = 1.f / static_cast<float>(1 << sh), off = -(1024.f * inv + kCtr);
+                const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&w), __floats2half2_rn(inv, inv),
+                                          __floats2half2_rn(off, off));
+                return *reinterpret_cast<const uint32_t*>(&r);
+            };
+#pragma unroll
+            for (int w = 0; w < (D / 8 + CPW - 1) / CPW; w++) {
+                const uint32_t x = window(v[0], v[1], w * CPW * VB), y = window(v[2], v[3], w * CPW * VB);
+#pragma unroll
+                for (int i = 0; i < CPW; i++) {
+                    if (w * CPW + i >= D / 8) break;
+                    h01[w * CPW + i] = code_half2(x << 1, x >> DOWN, i);
+                    h23[w * CPW + i] = code_half2(y << 1, y >> DOWN, i);
+                }
+            }
+#pragma unroll
+            for (int mt = 0; mt < NMT; mt++)
+#pragma unroll
+                for (int x = 0; x < NH; x++)
+                    mma_16816(oacc[x][mt], h01[2 * mt], h01[2 * mt + 1], h23[2 * mt], h23[2 * mt + 1], pb[x][0], pb[x][1]);
+        }
+
+        // ---- fold the warps' states
+#pragma unroll
+        for (int h = 0; h < HL; h++)
+#pragma unroll
+            for (int m = 4; m < 32; m <<= 1) {
+                l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], m);
+                z_run[h] += __shfl_xor_sync(0xffffffffu, z_run[h], m);
+            }
+        // output float (mt, j, h): coordinate (D/8) g + 2 mt + j of head HL * tg + h
+#pragma unroll
+        for (int mt = 0; mt < NMT; mt++)
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int h = 0; h < HL; h++)
+                    xo[(warp * C::OL + (mt * 2 + j) * HL + h) * 32 + lane] =
+                        NH == 1 ? fmaf(oacc[0][mt][2 * j + 1], kInvLo, oacc[0][mt][2 * j])
+                                : fmaf(oacc[NH - 1][mt][2 * j + h], kInvLo, oacc[0][mt][2 * j + h]);
+        if (g == 0) {
+#pragma unroll
+            for (int h = 0; h < HL; h++) {
+                xml[(warp * 3 + 0) * 8 + HL * tg + h] = m_run[h];
+                xml[(warp * 3 + 1) * 8 + HL * tg + h] = l_run[h];
+                xml[(warp * 3 + 2) * 8 + HL * tg + h] = z_run[h];
+            }
+        }
+        const bool any_bad = __syncthreads_or(bad_block) != 0;
+        for (int i = tid; i < C::OL * 32; i += C::THREADS) {
+            const int ln = i & 31, f = i >> 5, h = HL * (ln & 3) + f % HL;
+            if (h >= group) continue;
+            float M = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) M = fmaxf(M, xml[(w * 3 + 0) * 8 + h]);
+            float o = 0.f, l = 0.f, z = 0.f;
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) {
+                const float s = fast_exp2(xml[(w * 3 + 0) * 8 + h] - M);   // (a warp without pages: 0)
+                o = fmaf(xo[(w * C::OL + f) * 32 + ln], s, o);
+                l = fmaf(xml[(w * 3 + 1) * 8 + h], s, l);
+                z = fmaf(xml[(w * 3 + 2) * 8 + h], s, z);
+            }
+            float* dst = mid_row(it, h);
+            const int coord = (D / 8) * (ln >> 2) + f / HL;
+            dst[coord] = (o + z) / l;
+            if (coord == 0) dst[D] = any_bad ? __int_as_float(0x7fc00000) : M * kLn2 + logf(l);
+        }
+    }
+    cp_async_wait<0>();
+}
+
+}  // namespace ftq

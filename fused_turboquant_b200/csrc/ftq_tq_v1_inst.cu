@@ -11,6 +11,7 @@
 #define FTQ_TQ_DECODE 1
 #endif
 #if FTQ_D != 256 && defined(FTQ_TQ_DECODE)
+#include "ftq_tq_v1_fp8.cuh"
 #include "ftq_tq_v1_mma.cuh"
 #endif
 
@@ -159,6 +160,33 @@ static cudaError_t mma_by_vb(int vb, int nh, const TqDecodeParams& p, int n_item
     return cudaErrorInvalidValue;
 }
 #endif
+
+template <int VB, int NH>
+static cudaError_t fp8_run(const TqDecodeParams& p, int n_items, cudaStream_t stream) {
+#if FTQ_D != 256
+    using C = TqFp8Cfg<FTQ_D, VB, NH>;
+    constexpr auto kern = tq_fp8_kernel<FTQ_D, VB, NH>;
+    const cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    const int64_t slots = static_cast<int64_t>(sm_count()) * 2;
+    const unsigned gx = static_cast<unsigned>(n_items < slots ? n_items : slots);
+    kern<<<gx, C::THREADS, C::SMEM_BYTES, stream>>>(p, n_items);
+    return cudaGetLastError();
+#else
+    return cudaErrorInvalidValue;
+#endif
+}
+// Tensor-core stage 1 for FP8 keys (16-bit queries, GQA group <= 8, 2- to 4-bit values, head_dim 64 /
+// 128, 4-byte aligned slots).
+cudaError_t FTQ_CAT(launch_tq_fp8_d, FTQ_D)(int vb, int nh, const TqDecodeParams& p, int n_items,
+                                           cudaStream_t stream) {
+    switch (vb) {
+        case 2: return nh == 1 ? fp8_run<2, 1>(p, n_items, stream) : fp8_run<2, 2>(p, n_items, stream);
+        case 3: return nh == 1 ? fp8_run<3, 1>(p, n_items, stream) : fp8_run<3, 2>(p, n_items, stream);
+        case 4: return nh == 1 ? fp8_run<4, 1>(p, n_items, stream) : fp8_run<4, 2>(p, n_items, stream);
+    }
+    return cudaErrorInvalidValue;
+}
 
 // Tensor-core stage 1 (16-bit queries, GQA group <= 8, value_bits != 8, head_dim 64 / 128).
 cudaError_t FTQ_CAT(launch_tq_mma_d, FTQ_D)(int kb, int vb, int nh, const TqDecodeParams& p,

@@ -1,0 +1,93 @@
+"""Slot-format decode with FP8 keys: the tensor-core kernel (16-bit queries) against 64-bit arithmetic on the
+cache's bytes, and its error against that of the fp32 kernel, which fp32 queries take."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(q, cache, table, lens, d, vb, hkv, scale):
+    """float64, torch on the GPU: [B, Hq, D]."""
+    had = torch.ones(1, 1, dtype=torch.float64, device="cuda")
+    while had.shape[0] < d:
+        had = torch.cat([torch.cat([had, had], 1), torch.cat([had, -had], 1)], 0)
+    qr = q.double() @ (had / d ** 0.5)
+    out = []
+    for b, n in enumerate(lens.tolist()):
+        rows = cache[table[b].long()].reshape(-1, hkv, cache.shape[-1])[:n]
+        k = rows[..., :d].contiguous().view(torch.float8_e4m3fn).double()
+        bits = (rows[..., d:d + d * vb // 8, None].int() >> torch.arange(8, device="cuda")) & 1
+        code = (bits.reshape(n, hkv, d, vb) << torch.arange(vb, device="cuda")).sum(-1).double()
+        meta = rows[..., d + d * vb // 8:d + d * vb // 8 + 4].contiguous().view(torch.float16).double()
+        v = code * meta[..., :1] + meta[..., 1:]
+        group = q.shape[1] // hkv
+        s = torch.einsum("hgd,nhd->hgn", qr[b].view(hkv, group, d), k) * scale
+        out.append(torch.einsum("hgn,nhd->hgd", s.softmax(-1), v).reshape(-1, d))
+    return torch.stack(out)
+
+
+# (one token; less than a page; pages that not every warp has; remainders; groups on both sides of four;
+# splits without tokens; one and several layers of items per CTA)
+@pytest.mark.parametrize("d,vb,hkv,group,lens,splits,dtype", [
+    (128, 4, 2, 4, [1, 15, 16, 17], 8, "bf16"),
+    (128, 4, 8, 4, [1000, 4096, 333], 8, "bf16"),
+    (128, 3, 2, 7, [700, 90], 4, "fp16"),
+    (128, 2, 1, 8, [513], 1, "bf16"),
+    (64, 4, 4, 1, [129, 2000], 8, "fp16"),
+    (64, 3, 2, 8, [40, 300], 3, "bf16"),
+    (64, 2, 1, 3, [77] * 40, 16, "bf16"),
+])
+def test_fp32_precision(d, vb, hkv, group, lens, splits, dtype):
+    from fused_turboquant_b200 import tq_v1
+    gen = torch.Generator("cuda").manual_seed(d + vb + group)
+    cfg = tq_v1.TurboQuantSlotConfig(d, 8, vb, norm_correction=True)
+    per = [(n + 15) // 16 for n in lens]
+    cache = torch.randint(0, 255, (sum(per) + 1, 16, hkv, cfg.slot_size_aligned), dtype=torch.uint8, device="cuda",
+                          generator=gen)       # (unwritten slots hold anything, NaN keys and scales too)
+    ids = torch.randperm(sum(per) + 1, device="cuda", generator=gen)
+    table = torch.zeros(len(lens), max(per), dtype=torch.int32, device="cuda")
+    at = 0
+    for b, n in enumerate(lens):
+        table[b, :per[b]] = ids[at:at + per[b]].int()
+        pos = torch.arange(n, device="cuda")
+        slots = ids[at:at + per[b]][pos // 16] * 16 + pos % 16
+        kv = torch.randn(2, n, hkv, d, device="cuda", generator=gen)
+        kv[..., 1] *= 5.0
+        tq_v1.launch_store(kv[0].bfloat16(), kv[1].bfloat16(), cache, slots, None, cfg)
+        at += per[b]
+    sl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    q = torch.randn(len(lens), hkv * group, d, device="cuda", generator=gen)
+    q = q.to(torch.bfloat16 if dtype == "bf16" else torch.float16)
+
+    def run(x):
+        out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
+        tq_v1.decode_attention(x, cache, table, sl, None, cfg, d ** -0.5, num_kv_splits=splits, output=out)
+        return out
+
+    ref = _exact(q, cache, table, sl, d, vb, hkv, d ** -0.5)
+    new, old = ((run(x).double() - ref).norm().item() / ref.norm().item() for x in (q, q.float()))
+    # fp32 exponentials, sums over up to 4096 tokens: a few 2^-24
+    print(f"relative error: tensor cores {new:.2e}, fp32 kernel {old:.2e}")
+    assert new < 1e-6 and new < 2.0 * old + 1e-7
+
+
+def test_slots_off_the_word_stay_on_the_fp32_kernel():
+    """A cache whose slots start on 2-byte boundaries gives the same result through the other kernel."""
+    from fused_turboquant_b200 import tq_v1
+    d, hkv, n = 128, 2, 50
+    gen = torch.Generator("cuda").manual_seed(1)
+    cfg = tq_v1.TurboQuantSlotConfig(d, 8, 4, norm_correction=True)
+    size = cfg.slot_size_aligned
+    kv = torch.randn(2, n, hkv, d, device="cuda", generator=gen).bfloat16()
+    q = torch.randn(1, 8, d, device="cuda", generator=gen).bfloat16()
+    table = torch.arange(4, dtype=torch.int32, device="cuda")[None]
+    sl = torch.tensor([n], dtype=torch.int32, device="cuda")
+    outs = []
+    for pad in (0, 2):
+        cache = torch.zeros(4, 16, hkv, size + pad, dtype=torch.uint8, device="cuda")[..., :size]
+        tq_v1.launch_store(kv[0], kv[1], cache, torch.arange(n, device="cuda"), None, cfg)
+        out = torch.empty(1, 8, d, dtype=torch.float32, device="cuda")
+        tq_v1.decode_attention(q, cache, table, sl, None, cfg, d ** -0.5, num_kv_splits=4, output=out)
+        outs.append(out.cpu().numpy())
+    assert np.allclose(outs[0], outs[1], rtol=0, atol=2e-6)

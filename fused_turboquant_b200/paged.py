@@ -154,13 +154,23 @@ class PagedKVPool:
         v_norms = rows(off_vn, 2).contiguous().view(torch.float16).reshape(H, -1)[:, :S].contiguous()
         return k_codes, k_norms, v_codes, v_norms
 
-    def _takes_chunk_kernel(self, q, block_table, seq_lens, layer) -> bool:
+    def _takes_chunk_kernel(self, q, block_table, seq_lens, max_seq_len, layer) -> bool:
+        """Whether a continuation call goes to the chunk kernel.
+
+        From 8 queries per sequence on always: its time does not depend on the number of queries until
+        they fill 256 rows, that of the decode kernel grows with it (8 x 8000 tokens, 32 / 8 heads of
+        128: 57, 88, 136 us for 2, 4, 8 queries against 120 us).  Below that while the whole context
+        is at most 12 tiles per SM (under 30 us, where a decode call with its synthetic batch takes 40).
+        """
         B, q_len, Hq, D = q.shape
         H = self.num_kv_heads
-        return (q.is_cuda and q.dtype in (torch.float16, torch.bfloat16) and layer is not None and
+        if not (q.is_cuda and q.dtype in (torch.float16, torch.bfloat16) and layer is not None and
                 min(B, q_len, Hq) > 0 and Hq % H == 0 and Hq // H <= 8 and D == self.head_dim and
                 B <= 65535 and H * -(-q_len * (Hq // H) // 128) <= 65535 and
-                block_table.dim() == 2 and block_table.shape[0] == B and seq_lens.shape == (B,))
+                block_table.dim() == 2 and block_table.shape[0] == B and seq_lens.shape == (B,)):
+            return False
+        tile = 32 if D == 256 else 64
+        return q_len >= 8 or B * H * -(-int(max_seq_len) // tile) <= 12 * 148
 
     def continuation_attention(self, q: torch.Tensor, block_table: torch.Tensor,
                                seq_lens: torch.Tensor, max_seq_len: int, scale: float | None = None,
@@ -170,11 +180,11 @@ class PagedKVPool:
         q: [B, q_len, Hq, D]; seq_lens: [B] totals INCLUDING the new tokens.  Query i of a sequence
         attends positions < seq_len - q_len + i + 1 (reference: vllm_plugin/v1_backend.py:1359-1384).
         16-bit queries with a GQA group of at most 8 take the chunk kernel, which dequantises a page
-        once for all queries; the others run the decode kernel on one synthetic sequence per query with
+        once for all queries (see _takes_chunk_kernel); the others run the decode kernel on one synthetic sequence per query with
         its own length.  No host synchronisation.
         """
         B, q_len, Hq, D = q.shape
-        if self._takes_chunk_kernel(q, block_table, seq_lens, layer):
+        if self._takes_chunk_kernel(q, block_table, seq_lens, max_seq_len, layer):
             if _trace.ENABLED:
                 with _trace.nvtx("ftq.decode"):
                     return _lib.native().paged_chunk(self, q, block_table, seq_lens, max_seq_len, scale,

@@ -46,7 +46,7 @@ def test_matches_fp32_decode(d, bk, bv, hkv, group, q_len, lens, dtype):
     pool, table, sl, gen = _pool(d, bk, bv, hkv, lens, d + q_len)
     dt = torch.bfloat16 if dtype == "bf16" else torch.float16
     q = torch.randn(len(lens), q_len, hkv * group, d, device="cuda", generator=gen).to(dt)
-    assert pool._takes_chunk_kernel(q, table, sl, 1)
+    assert pool._takes_chunk_kernel(q, table, sl, max(lens), 1)
     got = pool.continuation_attention(q, table, sl, max(lens), layer=1)
     assert pool.decode_status() == 0
     ref = pool.continuation_attention(q.float(), table, sl, max(lens), layer=1)
@@ -62,9 +62,14 @@ def test_matches_fp32_decode(d, bk, bv, hkv, group, q_len, lens, dtype):
 def test_other_calls_stay_on_the_decode_kernel():
     pool, table, sl, gen = _pool(64, 4, 4, 1, [70], 3)
     q = torch.randn(1, 4, 16, 64, device="cuda", generator=gen).bfloat16()
-    assert not pool._takes_chunk_kernel(q, table, sl, 1)              # group 16
-    assert not pool._takes_chunk_kernel(q.float()[:, :, :8], table, sl, 1)
-    assert not pool._takes_chunk_kernel(q[:, :, :8], table, sl, None)
+    assert not pool._takes_chunk_kernel(q, table, sl, 70, 1)              # group 16
+    q8 = q[:, :, :8]
+    assert not pool._takes_chunk_kernel(q8.float(), table, sl, 70, 1)
+    assert not pool._takes_chunk_kernel(q8, table, sl, 70, None)
+    # few queries over much context; the limit, and one tile more
+    assert pool._takes_chunk_kernel(q8, table, sl, 64 * 1776, 1)
+    assert not pool._takes_chunk_kernel(q8, table, sl, 64 * 1776 + 1, 1)
+    assert pool._takes_chunk_kernel(q8.repeat(1, 2, 1, 1), table, sl, 64 * 1776 + 1, 1)
 
 
 def test_block_id_out_of_range_is_reported():

@@ -812,7 +812,7 @@ def main():
         enc = {"tokens_per_s": tok_total / (ms * 1e-3), "ms": ms, "tokens": int(tok_total),
                "vectors_per_token": 2 * Hkv_local, "bytes_per_gpu": eb,
                "gbs_per_gpu": eb / (ms * 1e-3) / 1e9, "frac_of_peak": eb / (ms * 1e-3) / 1e9 / peak,
-               "launches": 2}
+               "launches": 1}
         del k, v, epool
 
     peak, peak_src = load_peaks()
@@ -822,16 +822,14 @@ def main():
         value = total_bytes_step / (ms_step * 1e-3) / 1e9
         bytes_call = s.bytes_layer * s.layers_per_call
         traffic, traffic_src = load_traffic(args.workload, s.layers_per_call)
-        # 4-bit keys with a GQA group of at most 4 run the streaming kernel (merge and counter
-        # reset inside the kernel); the other configurations run attn_mma_kernel behind a memset
-        # node, followed by the merge kernel
-        fused = w["bk"] == 4 and w["Hq"] // w["Hkv"] <= 4
-        # Duration of the dominant kernel's launch.  Where a call is this one kernel and a step is
-        # nothing but such calls back to back, it is the timed region divided by its launches
-        # (gaps between launches included).  Otherwise (several nodes per call, or a collective
-        # inside the step) it is the event-timed duration of one call, timed call by call.
+        # one kernel per call (merge and counter reset inside): the streaming kernel for 4-bit keys
+        # with a GQA group of at most 4, the equal-share kernel for the other configurations
+        stream = w["bk"] == 4 and w["Hq"] // w["Hkv"] <= 4
+        # Duration of the kernel's launch.  Where a step is nothing but such calls back to back, it is
+        # the timed region divided by its launches (gaps between launches included).  Otherwise (a
+        # collective inside the step) it is the event-timed duration of one call, timed call by call.
         launch_ms = call_ms
-        if fused and gather is None:
+        if gather is None:
             launch_ms = float(np.median(regions)) / (args.steps * s.n_calls)
         achieved = bytes_call / (launch_ms * 1e-3) / 1e9
         line = {
@@ -848,10 +846,8 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_src,
                          "peak_source": peak_src, "frac_of_nominal_8000": achieved / 8000.0,
-                         "kernel": ("attn_stream_kernel (one ftq_paged_decode_attn call = this one "
-                                    "kernel)" if fused else
-                                    "attn_mma_kernel + attn_merge_kernel behind one memset node "
-                                    "(one ftq_paged_decode_attn call)")
+                         "kernel": ("attn_stream_kernel" if stream else "attn_flow_kernel")
+                                   + " (one ftq_paged_decode_attn call = this one kernel)"
                                    + ", %d layer(s)" % s.layers_per_call,
                          "bytes_per_launch": bytes_call, "ms_per_launch": launch_ms,
                          "ms_per_call_timed_alone": call_ms},
@@ -859,7 +855,7 @@ def main():
                     "h2d_bytes_per_step": int(s.q_host.numel() * 2),
                     "d2h_bytes_per_step": int(s.q_host.numel() * 2 * (world if head_sharded else 1)),
                     "ms_per_step": ms_e2e / args.steps, "copies": copies},
-            "gpu_launches": int(args.steps * len(regions) * s.n_calls * (1 if fused else 2)),
+            "gpu_launches": int(args.steps * len(regions) * s.n_calls),
             "memset_nodes": 0 if fused else int(args.steps * len(regions) * s.n_calls),
             "clocks": clocks, "parity": parity, "encode": enc,
         }

@@ -1,5 +1,5 @@
-// Paged split-KV decode attention on the tensor cores (barrier-synchronised form;
-// ftq_attn_stream.cuh holds the streaming form of the same arithmetic): whole
+// What the tensor-core kernels of paged decode attention share (ftq_attn_flow.cuh: equal
+// shares of pages per CTA; ftq_attn_stream.cuh: streaming warps): whole
 // 16-token pages arrive in a per-warp ring by 1-D bulk copies (TMA), every lane
 // copies its slices to registers, the codes are dequantised through a
 // bank-conflict-free shared-memory table and feed warp-level m16n8k16 fp16 MMAs
@@ -15,15 +15,6 @@
 // by a host-chosen factor in [1, 2) before the rounding (and the weights divided
 // by it): a common rounding bias of the centroids would otherwise add up over
 // all coordinates into one output element through the inverse rotation.
-//
-// Work split: persistent CTAs (one per SM when a 4-bit byte table is in use --
-// 16 warps, or 8 where 16 page rings do not fit beside the table -- else two per
-// SM with 8 warps) loop over work items
-// (KV chunk, KV head, sequence x layer); the dequantisation tables are built once
-// per CTA.  Within an item each warp walks pages warp, warp+W, ... with its own
-// online-softmax state; the states are merged pairwise (registers + a small
-// shared exchange area) and warp 0 writes one partial row per query head (same
-// workspace format as attn_split_kernel, so attn_merge_kernel finishes both).
 //
 // Tables: an entry holds the fp16 centroids of two adjacent codes, replicated
 // for the 32 lanes so that bank = lane (no conflicts whatever the codes are).

@@ -1,6 +1,6 @@
 // Paged split-KV decode attention, streaming form of the tensor-core kernel.
 //
-// Same arithmetic, tables, page layout and fragment maps as attn_mma_kernel
+// Same arithmetic, tables, page layout and fragment maps as attn_flow_kernel
 // (ftq_attn_mma.cuh: the fused formulation of
 // src/fused_turboquant/kernels/triton_flash_decode.py:33-324 of the reference with
 // the query rotation of hf/fused_cache.py:579-581 and the page-table walk of
@@ -283,7 +283,7 @@ attn_stream_kernel(const AttnParams p, int n_items) {
         ctl[kCtlArrived + 1] = 0;
     }
 
-    // ---- once per CTA: dequantisation tables (same contents as attn_mma_kernel's)
+    // ---- once per CTA: dequantisation tables (same contents as attn_flow_kernel's)
     if constexpr (C::BYTE) {
         uint32_t* tb = reinterpret_cast<uint32_t*>(gptr(window));
         for (int i = tid; i < 256 * 64; i += THREADS) {

@@ -856,7 +856,7 @@ def main():
                     "d2h_bytes_per_step": int(s.q_host.numel() * 2 * (world if head_sharded else 1)),
                     "ms_per_step": ms_e2e / args.steps, "copies": copies},
             "gpu_launches": int(args.steps * len(regions) * s.n_calls),
-            "memset_nodes": 0 if fused else int(args.steps * len(regions) * s.n_calls),
+            "memset_nodes": 0,
             "clocks": clocks, "parity": parity, "encode": enc,
         }
     del s

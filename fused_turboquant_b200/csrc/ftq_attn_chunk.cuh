@@ -28,8 +28,11 @@
 // (O, m, l) in the workspace and attn_merge_kernel finishes.
 //
 // Every wait is bounded; one that runs out makes the CTA's rows NaN and sets a bit of the status word.
-// Block ids outside [0, num_blocks) are never dereferenced and have the same effect.
+// Block ids outside [0, num_blocks) are never dereferenced and have the same effect on the rows that attend
+// a token of such a page.
 #pragma once
+
+#include <climits>
 
 #include "ftq_attn_mma.cuh"
 
@@ -174,7 +177,8 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
     }
 
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort;   // bit 0: a block id out of range, bit 1: a wait ran out
+    __shared__ int s_abort;     // a wait ran out
+    __shared__ int s_bad_pos;   // first token on a page whose block id is out of range
     const volatile int* const abort_now = &s_abort;
     const uint32_t bars = sbase + C::OFF_BAR;
     const uint32_t kv_full = bars, kv_empty = bars + 16, s_full = bars + 32, s_free = bars + 48,
@@ -198,7 +202,10 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
         }
         tc_fence_before();
     }
-    if (tid == 0) s_abort = 0;
+    if (tid == 0) {
+        s_abort = 0;
+        s_bad_pos = INT_MAX;
+    }
     // ---- tables: an entry (the fp16 centroids of two adjacent codes) 32 times, bank = lane
     {
         auto build = [&](int off, int bits, const Codebook& cb) {
@@ -254,9 +261,9 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
                 "selp.u32 %0, 1, 0, p;\n}\n"
                 : "=r"(ok) : "r"(bar), "r"(parity & 1u) : "memory");
             if (ok) return true;
-            if ((i & 63) == 63 && (*abort_now & 2)) return false;
+            if ((i & 63) == 63 && *abort_now) return false;
         }
-        atomicOr(&s_abort, 2);
+        s_abort = 1;
         return false;
     };
 
@@ -287,7 +294,8 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
                 const float4* vn = kn + KT / 4;
                 float mx = -INFINITY;
                 const int left = limit - (tile0 + it) * KT;   // tokens of this tile the row attends
-                if (__all_sync(0xffffffffu, left >= KT)) {
+                const bool all_attended = __all_sync(0xffffffffu, left >= KT);
+                if (all_attended) {
 #pragma unroll
                     for (int c = 0; c < KT; c += 4) {
                         const float4 n = kn[c / 4];
@@ -341,16 +349,29 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
                 }
                 const float m_use = m_run == -INFINITY ? 0.f : m_run;   // (nothing attended so far)
                 float l0 = 0.f, l1 = 0.f;
+                // A token that the row does not attend has weight zero whatever its value norm is: an
+                // infinite or NaN norm (a vector longer than fp16 holds, a slot of a rejected draft
+                // token) belongs to the later queries only.
+                auto weights = [&](auto whole) {
 #pragma unroll
-                for (int c = 0; c < KT; c += 4) {
-                    const float4 n = vn[c / 4];
-                    const float p0 = fast_exp2(__uint_as_float(sr[c]) - m_use), p1 = fast_exp2(__uint_as_float(sr[c + 1]) - m_use);
-                    const float p2 = fast_exp2(__uint_as_float(sr[c + 2]) - m_use), p3 = fast_exp2(__uint_as_float(sr[c + 3]) - m_use);
-                    l0 += p0 + p1;
-                    l1 += p2 + p3;
-                    sr[c / 2] = f2h2_sat(p0 * n.x, p1 * n.y);
-                    sr[c / 2 + 1] = f2h2_sat(p2 * n.z, p3 * n.w);
-                }
+                    for (int c = 0; c < KT; c += 4) {
+                        float4 n = vn[c / 4];
+                        if constexpr (!decltype(whole)::value) {
+                            n.x = c < left ? n.x : 0.f;
+                            n.y = c + 1 < left ? n.y : 0.f;
+                            n.z = c + 2 < left ? n.z : 0.f;
+                            n.w = c + 3 < left ? n.w : 0.f;
+                        }
+                        const float p0 = fast_exp2(__uint_as_float(sr[c]) - m_use), p1 = fast_exp2(__uint_as_float(sr[c + 1]) - m_use);
+                        const float p2 = fast_exp2(__uint_as_float(sr[c + 2]) - m_use), p3 = fast_exp2(__uint_as_float(sr[c + 3]) - m_use);
+                        l0 += p0 + p1;
+                        l1 += p2 + p3;
+                        sr[c / 2] = f2h2_sat(p0 * n.x, p1 * n.y);
+                        sr[c / 2 + 1] = f2h2_sat(p2 * n.z, p3 * n.w);
+                    }
+                };
+                if (all_attended) weights(std::true_type{});
+                else weights(std::false_type{});
                 l_run += l0 + l1;
 #pragma unroll
                 for (int c = 0; c < KT / 2; c += 16) tc_st16(tm + C::COL_P + c, sr + c);
@@ -421,7 +442,7 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
             const int pos = (tile0 + it) * KT + t;
             if (it >= n_tiles || pos >= seq) return;
             if (static_cast<uint64_t>(static_cast<int64_t>(id)) >= static_cast<uint64_t>(p.num_blocks)) {
-                atomicOr(&s_abort, 1);
+                atomicMin(&s_bad_pos, pos);
                 return;
             }
             const uint8_t* page = head + id * blk_stride;
@@ -520,13 +541,12 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
     }
     __syncwarp();
     __syncthreads();
-    const int bad = s_abort;
-    if (bad) {   // NaN rows
-        for (int r = row0 + tid; r < row_end; r += C::THREADS) partial_row(r)[D] = __int_as_float(0x7fc00000);
-        if (tid == 0) {
-            if (bad & 1) atomicOr(p.status, kStatusBadBlock);
-            if (bad & 2) atomicOr(p.status, kStatusWaitExpired);
-        }
+    const bool expired = s_abort != 0;
+    const int bad_pos = s_bad_pos;
+    if (expired || bad_pos != INT_MAX) {
+        for (int r = row0 + tid; r < row_end; r += C::THREADS)
+            if (expired || bad_pos < min(p.max_seq, limit0 + r / group)) partial_row(r)[D] = __int_as_float(0x7fc00000);
+        if (tid == 0) atomicOr(p.status, (expired ? kStatusWaitExpired : 0) | (bad_pos != INT_MAX ? kStatusBadBlock : 0));
     }
     if (warp == C::SM_WARPS + C::DQ_WARPS) {
         tc_fence_after();

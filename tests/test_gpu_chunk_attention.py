@@ -97,3 +97,34 @@ def test_a_captured_call_replays():
     g.replay()
     torch.cuda.synchronize()
     assert np.array_equal(out.cpu().numpy(), want.cpu().numpy())
+
+
+@pytest.mark.parametrize("d,bk,bv,group,q_len,n", [(128, 4, 4, 4, 20, 300), (64, 3, 3, 7, 40, 129),
+                                                   (256, 4, 2, 1, 130, 200)])
+@pytest.mark.parametrize("bad", [6e4, float("nan")])
+def test_a_later_token_without_a_finite_value_norm_is_nobody_elses(d, bk, bv, group, q_len, n, bad):
+    """The last two tokens' value vectors are longer than fp16 holds, or NaN: queries before them are bit
+    for bit what they are with ordinary values there."""
+    pool, table, sl, gen = _pool(d, bk, bv, 2, [n], d + q_len)
+    q = torch.randn(1, q_len, 2 * group, d, device="cuda", generator=gen).bfloat16()
+    assert pool._takes_chunk_kernel(q, table, sl, n, 1)
+    good = pool.continuation_attention(q, table, sl, n, layer=1)
+    key = torch.randn(2, 2, d, device="cuda", generator=gen).bfloat16()
+    pos = torch.tensor([n - 2, n - 1], device="cuda")
+    slots = table[0].long()[pos // 16] * 16 + pos % 16
+    pool.store(key, torch.full_like(key, bad), slots, layer=1)
+    got = pool.continuation_attention(q, table, sl, n, layer=1)
+    assert torch.equal(got[:, :-2], good[:, :-2])
+
+
+def test_block_id_out_of_range_concerns_the_queries_that_attend_it():
+    """The chunk's last page has a bad id: the queries whose context ends before it are untouched."""
+    n, q_len = 320, 24                       # the last page holds the last 16 queries' tokens
+    pool, table, sl, gen = _pool(128, 4, 4, 2, [n], 7)
+    q = torch.randn(1, q_len, 8, 128, device="cuda", generator=gen).half()
+    good = pool.continuation_attention(q, table, sl, n, layer=1)
+    table[0, n // 16 - 1] = pool.num_blocks + 1
+    out = pool.continuation_attention(q, table, sl, n, layer=1)
+    assert pool.decode_status() == 1
+    assert torch.equal(out[:, :8], good[:, :8])
+    assert torch.isnan(out[:, 8:]).all()

@@ -177,7 +177,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         for (int i = tid; i < 2 * p.n_units; i += THREADS) p.unit_counter[i] = 0;
         if (tid == 0) {
             p.work_counter[1] = 0;
-            p.work_counter[kStatusWord] = 0;
+            if (p.b0 == 0) p.work_counter[kStatusWord] = 0;   // (the call's: its later launches add to it)
         }
     }
     // prefix sums of the page counts (lengths beyond the host's bound are cut to it)

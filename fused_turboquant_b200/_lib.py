@@ -95,7 +95,7 @@ def native():
         from . import kernels
 
         ext.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in SIGNATURES},
-                 check, kernels.get_workspace, kernels._workspaces)
+                 check, kernels.get_workspace, kernels._workspaces, kernels._host_table)
         _native = ext
     return _native
 

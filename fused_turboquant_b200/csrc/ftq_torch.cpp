@@ -42,6 +42,7 @@ struct Api {
 PyObject* g_check = nullptr;        // _lib.check(rc, name): raises what the status stands for
 PyObject* g_get_workspace = nullptr;  // kernels.get_workspace(device, nbytes)
 PyObject* g_workspaces = nullptr;     // kernels._workspaces
+PyObject* g_host_table = nullptr;     // kernels._host_table: fp32 copy of an array of any type and strides
 
 struct PyError {};  // a Python exception is set
 
@@ -136,8 +137,9 @@ at::Tensor empty(at::IntArrayRef size, at::ScalarType t, const at::Device& d) {
 }
 
 // ------------------------------------------------------------------ small host tables
-// numpy fp32 arrays are read in place; a tensor's values are copied to the host once and kept
-// while the tensor is alive and unmodified (as kernels._host_table does for the other callers).
+// Contiguous fp32 arrays are read in place, other arrays converted; a tensor's values are copied to
+// the host once and kept while the tensor is alive and unmodified (as kernels._host_table does for the
+// other callers).
 struct CachedTable {
     c10::weak_intrusive_ptr<c10::TensorImpl> owner;
     uint32_t version;
@@ -153,21 +155,30 @@ struct Table {
     explicit Table(PyObject* o) {
         if (o == nullptr || o == Py_None) return;
         if (THPVariable_Check(o)) { from_tensor(THPVariable_Unpack(o)); return; }
-        if (PyObject_GetBuffer(o, &view, PyBUF_CONTIG_RO | PyBUF_FORMAT) == 0) {
-            if (view.itemsize == 4 && view.format && view.format[0] == 'f') {
-                p = static_cast<const float*>(view.buf);
-                return;
-            }
-            PyBuffer_Release(&view);
-            view.obj = nullptr;
-        }
-        PyErr_Clear();
-        raise(PyExc_TypeError, "a table must be a float32 array or a tensor");
+        if (from_buffer(o)) return;
+        PyObject* c = PyObject_CallOneArg(g_host_table, o);
+        if (!c) throw PyError{};
+        const bool ok = from_buffer(c);   // (the view holds the array)
+        Py_DECREF(c);
+        if (!ok) raise(PyExc_TypeError, "a table must be an array or a tensor of numbers");
     }
     Table(const Table&) = delete;
     ~Table() { if (view.obj) PyBuffer_Release(&view); }
 
    private:
+    bool from_buffer(PyObject* o) {
+        if (PyObject_GetBuffer(o, &view, PyBUF_CONTIG_RO | PyBUF_FORMAT) != 0) {
+            PyErr_Clear();
+            return false;
+        }
+        if (view.itemsize == 4 && view.format && view.format[0] == 'f') {
+            p = static_cast<const float*>(view.buf);
+            return true;
+        }
+        PyBuffer_Release(&view);
+        view.obj = nullptr;
+        return false;
+    }
     void from_tensor(const at::Tensor& t) {
         const bool keep = !t.is_inference();
         const void* key = t.unsafeGetTensorImpl();
@@ -651,7 +662,7 @@ PyObject* tq_decode(PyObject* const* a) {
     return THPVariable_Wrap(out);
 }
 
-// bind({name: address}, check, get_workspace, workspaces)
+// bind({name: address}, check, get_workspace, workspaces, host_table)
 PyObject* bind(PyObject* const* a) {
 #define X(name)                                                                     \
     {                                                                               \
@@ -664,6 +675,7 @@ PyObject* bind(PyObject* const* a) {
     g_check = Py_NewRef(a[1]);
     g_get_workspace = Py_NewRef(a[2]);
     g_workspaces = Py_NewRef(a[3]);
+    g_host_table = Py_NewRef(a[4]);
     Py_RETURN_NONE;
 }
 
@@ -682,7 +694,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 #define FTQ_ENTRY(name, n) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<name, n>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
-    FTQ_ENTRY(bind, 4),
+    FTQ_ENTRY(bind, 5),
     FTQ_ENTRY(paged_store, 5),
     FTQ_ENTRY(paged_decode, 9),
     FTQ_ENTRY(paged_chunk, 7),

@@ -4,13 +4,21 @@
 // `_tq_decode_stage1_offset` (src/fused_turboquant/vllm_plugin/triton_decode_offset.py:42-444), partials
 // in the same [B, Hq, splits, D + 1] layout.  That kernel spends 1500 instructions on a 16-token page
 // (fp32 FMAs per query head, shuffles per score) and was issue bound at 137 us for 16 x 4096 tokens of
-// 8 heads; here both products are m16n8k16 MMAs whose operands lose nothing:
-//   * e4m3 keys and the centred 2- to 4-bit value codes are exact in fp16;
+// 8 heads; here both products are m16n8k16 MMAs (73 us):
+//   * e4m3 keys and 2- to 4-bit value codes are exact in fp16.  The code nearest to the value 0 is taken off
+//     a token's codes and what it is off by goes through fp32 sums: the sums of code * scale and of the zero
+//     points would be large numbers of opposite sign otherwise;
 //   * a rotated query is the sum of two fp16 numbers, hi + lo / 2^11, after scaling by a power of two that
 //     puts the head's largest coordinate in [2^10, 2^11): 23 bits of that coordinate's magnitude;
-//   * a softmax weight (times the value scale) is split the same way.
-// Accumulation is fp32.  With at most four heads the eight columns of an MMA are (head, hi / lo), so the
-// split costs no MMA; with five to eight heads hi and lo are one MMA each.
+//   * a softmax weight (times the value scale) is split the same way, times the power of two that puts the
+//     largest value scale seen so far at 2^14.
+// An MMA truncates its sums where FMAs round, so chains are short (two k-blocks of a score, one page of the
+// output) and added up in fp32.  Error against 64-bit arithmetic over 72 configurations (64 / 128, 300 to
+// 30000 tokens, values times 1 to 1e-4, shifted by 10, channels ten times larger), mean per vector: 0.57 to
+// 1.02 of the fp32 kernel's, 0.87 in the middle.  With chains over all of a warp's pages, unscaled
+// weights and codes centred at 7.5 it was 0.55 to 4.1 of it, 1.16 in the middle, in 70 us.
+// With at most four heads the eight columns of an MMA are (head, hi / lo), so the split costs no MMA; with
+// five to eight heads hi and lo are one MMA each.
 //
 // Fragment maps for a page of 16 tokens (lane = 4 g + tg):
 //   S: A rows g, g + 8 = tokens, k-block kb = coordinates (D/4) tg + 4 kb + {0..3} (word kb of the lane's
@@ -41,6 +49,7 @@ struct TqFp8Cfg {
     static constexpr int PAGE = kPageTokens * ROWB;
     static constexpr int STAGES = NH == 1 ? 3 : 2;
     static constexpr int HL = NH;                                // heads whose state a lane keeps
+    static constexpr int CHAINS = 4;                             // independent sums of a score
     static constexpr int OL = NMT * 2 * HL;                      // output floats of a lane
     static constexpr int QS = 8 * (D + 16) * 4;
     static constexpr int XO = WARPS * 32 * OL * 4, XML = WARPS * 3 * 8 * 4;
@@ -54,10 +63,6 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
     using C = TqFp8Cfg<D, VB, NH>;
     constexpr int NKB = C::NKB, NMT = C::NMT, WARPS = C::WARPS, HL = C::HL, E = D / kOctet;
     constexpr float kLo = 2048.f, kInvLo = 1.f / 2048.f;
-    // codes are centred and the zero point moved accordingly: the sums of code * scale and of zero would
-    // be large numbers of opposite sign otherwise (a centre half a code off costs a factor of five in
-    // the error of a mean over 500 tokens of 2-bit values)
-    constexpr float kCtr = 0.5f * ((1 << VB) - 1);
     extern __shared__ __align__(16) uint8_t smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tg = lane & 3;
@@ -168,10 +173,7 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
             octet_fwht<E>(a, lane);
             float mx = 0.f;
 #pragma unroll
-            for (int k = 0; k < E; k++) {
-                a[k] *= p.rsqrt_d;
-                mx = fmaxf(mx, fabsf(a[k]));
-            }
+            for (int k = 0; k < E; k++) mx = fmaxf(mx, fabsf(a[k]));
 #pragma unroll
             for (int m = 1; m < 8; m <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, m));
             // power of two that brings mx into [2^10, 2^11) (1 for zero, infinite or NaN rows)
@@ -181,7 +183,9 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
             const float down = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
 #pragma unroll
             for (int k = 0; k < E; k++) qs[qs_index(hh, t8 + 8 * k)] = hv ? a[k] * up : 0.f;
-            if (t8 == 0) qmul[hh] = p.scale * kLog2e * down;
+            // (the transform's factor goes here, not into the coordinates: one rounding for all factors)
+            constexpr double kRotate = D == 64 ? 0.125 : 0.08838834764831845;   // 1 / sqrt(D)
+            if (t8 == 0) qmul[hh] = static_cast<float>(p.scale * (1.4426950408889634 * kRotate)) * down;
         }
         __syncthreads();
 
@@ -204,18 +208,17 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
 #pragma unroll
         for (int h = 0; h < HL; h++) mul[h] = qmul[HL * tg + h];
 
-        float m_run[HL], l_run[HL], z_run[HL], oacc[NH][NMT][4];
+        float m_run[HL], l_run[HL], z_run[HL], oacc[NMT][2 * HL];   // [m-tile][row g or g + 8, head]
+        float s_ref = 0.f, up = 1.f;   // largest value scale so far as a power of two; weights are split times up
 #pragma unroll
         for (int h = 0; h < HL; h++) {
             m_run[h] = -INFINITY;
             l_run[h] = z_run[h] = 0.f;
         }
 #pragma unroll
-        for (int x = 0; x < NH; x++)
+        for (int mt = 0; mt < NMT; mt++)
 #pragma unroll
-            for (int mt = 0; mt < NMT; mt++)
-#pragma unroll
-                for (int i = 0; i < 4; i++) oacc[x][mt][i] = 0.f;
+            for (int i = 0; i < 2 * HL; i++) oacc[mt][i] = 0.f;
         bool bad_block = false;
 
         for (int pg = warp; pg < it.n_pages; pg += WARPS) {
@@ -226,14 +229,10 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
             copy_next();
             stage = stage + 1 == C::STAGES ? 0 : stage + 1;
 
-            // ---- scores
-            float c[NH][2][4];
-#pragma unroll
-            for (int x = 0; x < NH; x++)
-#pragma unroll
-                for (int z = 0; z < 2; z++)
-#pragma unroll
-                    for (int i = 0; i < 4; i++) c[x][z][i] = 0.f;
+            // ---- scores: chains of NKB / CH MMAs (an MMA's sum is truncated, the sums of the chains'
+            // results are rounded)
+            constexpr int CH = C::CHAINS;
+            float c[NH][CH][4];
             const uint32_t rowa = page + g * C::ROWB, rowb = rowa + 8 * C::ROWB;
 #pragma unroll
             for (int q = 0; q < NKB / 4; q++) {
@@ -248,8 +247,11 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
                     const uint32_t a0 = half2_of(wa[j] & 0xffffu), a2 = half2_of(wa[j] >> 16);
                     const uint32_t a1 = half2_of(wb[j] & 0xffffu), a3 = half2_of(wb[j] >> 16);
 #pragma unroll
-                    for (int x = 0; x < NH; x++)
-                        mma_16816(c[x][j & 1], a0, a1, a2, a3, qb[x][4 * q + j][0], qb[x][4 * q + j][1]);
+                    for (int x = 0; x < NH; x++) {
+                        const int kb = 4 * q + j;
+                        if (kb < CH) mma_16816_z(c[x][kb % CH], a0, a1, a2, a3, qb[x][kb][0], qb[x][kb][1]);
+                        else mma_16816(c[x][kb % CH], a0, a1, a2, a3, qb[x][kb][0], qb[x][kb][1]);
+                    }
                 }
             }
 
@@ -260,24 +262,48 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
             const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&ma));
             const float2 fb = __half22float2(*reinterpret_cast<const __half2*>(&mb));
             const float vsa = okA ? fa.x : 0.f, vsb = okB ? fb.x : 0.f;
-            const float vza = okA ? fmaf(kCtr, fa.x, fa.y) : 0.f;
-            const float vzb = okB ? fmaf(kCtr, fb.x, fb.y) : 0.f;
+            // the code nearest to the value 0 and what it is off by
+            auto code0 = [](float2 m) { return fminf(fmaxf(rintf(__fdividef(-m.y, m.x)), 0.f), static_cast<float>((1 << VB) - 1)); };
+            const float ca = code0(fa), cb = code0(fb);
+            const float vza = okA ? fmaf(ca, fa.x, fa.y) : 0.f;
+            const float vzb = okB ? fmaf(cb, fb.x, fb.y) : 0.f;
             float ra[HL], rb[HL], sa[HL], sb[HL];   // products; scaled scores
-            bool above = false;
+            const float s_max = fmaxf(fabsf(vsa), fabsf(vsb));
+            bool above = s_max > s_ref;
 #pragma unroll
             for (int h = 0; h < HL; h++) {
-                if constexpr (NH == 1) {
-                    ra[h] = fmaf(c[0][0][1] + c[0][1][1], kInvLo, c[0][0][0] + c[0][1][0]);
-                    rb[h] = fmaf(c[0][0][3] + c[0][1][3], kInvLo, c[0][0][2] + c[0][1][2]);
-                } else {
-                    ra[h] = fmaf(c[NH - 1][0][h] + c[NH - 1][1][h], kInvLo, c[0][0][h] + c[0][1][h]);
-                    rb[h] = fmaf(c[NH - 1][0][2 + h] + c[NH - 1][1][2 + h], kInvLo, c[0][0][2 + h] + c[0][1][2 + h]);
-                }
+                // sum of a column over the chains
+                auto total = [&](const float (&x)[CH][4], int i) {
+                    float t[CH];
+#pragma unroll
+                    for (int z = 0; z < CH; z++) t[z] = x[z][i];
+#pragma unroll
+                    for (int w = CH / 2; w > 0; w /= 2)
+#pragma unroll
+                        for (int z = 0; z < w; z++) t[z] += t[z + w];
+                    return t[0];
+                };
+                constexpr int LO = NH - 1;   // where the lo parts are: the next column, or the second MMA
+                ra[h] = fmaf(total(c[LO], NH == 1 ? 1 : h), kInvLo, total(c[0], h));
+                rb[h] = fmaf(total(c[LO], NH == 1 ? 3 : 2 + h), kInvLo, total(c[0], 2 + h));
                 sa[h] = okA ? ra[h] * mul[h] : -INFINITY;
                 sb[h] = okB ? rb[h] * mul[h] : -INFINITY;
                 above |= fmaxf(sa[h], sb[h]) > m_run[h];   // (no slack: a weight is at most the value scale)
             }
             if (__any_sync(0xffffffffu, above)) {
+                // the page's largest value scale, rounded up to a power of two, brought to 2^14: no weight
+                // leaves fp16's range, and one below its normal numbers is 2^-28 of the largest possible
+                float top = s_max;
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 4));
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 8));
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+                float shift = 1.f;
+                if (top > s_ref) {   // (warp-uniform; a power of two >= 2^-24)
+                    s_ref = __uint_as_float((__float_as_uint(top) + 0x007fffffu) & 0x7f800000u);
+                    const float was = up;
+                    up = 16384.f / s_ref;
+                    shift = up / was;
+                }
                 float corr[HL];
 #pragma unroll
                 for (int h = 0; h < HL; h++) {
@@ -292,15 +318,14 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
                     m_run[h] = m_new;
                 }
 #pragma unroll
-                for (int x = 0; x < NH; x++)
+                for (int mt = 0; mt < NMT; mt++)
 #pragma unroll
-                    for (int mt = 0; mt < NMT; mt++)
-#pragma unroll
-                        for (int i = 0; i < 4; i++) oacc[x][mt][i] *= corr[NH == 1 ? 0 : (i & 1)];
+                    for (int i = 0; i < 2 * HL; i++) oacc[mt][i] *= corr[i % HL] * shift;
             }
             uint32_t pb[NH][2];
             {
                 float wa[HL], wb[HL];
+                const float sua = vsa * up, sub = vsb * up;   // (exact)
 #pragma unroll
                 for (int h = 0; h < HL; h++) {
                     // (the exponent in one rounding)
@@ -308,8 +333,8 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
                     const float pbv = okB ? fast_exp2(fmaf(rb[h], mul[h], -m_run[h])) : 0.f;
                     l_run[h] += pa + pbv;
                     z_run[h] = fmaf(pa, vza, fmaf(pbv, vzb, z_run[h]));
-                    wa[h] = pa * vsa;
-                    wb[h] = pbv * vsb;
+                    wa[h] = pa * sua;
+                    wb[h] = pbv * sub;
                 }
                 if constexpr (NH == 1) {
                     pb[0][0] = movmatrix_trans(pack(wa[0], residual(wa[0])));
@@ -323,9 +348,12 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
             }
 
             // ---- O^T += V^T.P^T.  Codes become fp16 arithmetically: or-ed into the mantissa of 1024 a
-            // code at bit s is 1024 + 2^s * code, and one packed FMA scales and centres it exactly (s >= 1:
-            // 2^(10 - s) + centre is then an fp16 number).  A 16-bit half of x holds the next codes of
-            // one token, the other half those of its neighbour.
+            // code at bit s is 1024 + 2^s * code, and one packed FMA scales it and takes the token's code of
+            // zero off exactly (s >= 1: 2^(10 - s) + code is then an fp16 number).  A 16-bit half of x holds
+            // the next codes of one token, the other half those of its neighbour.
+            const uint32_t czero = pack(ca, cb);   // tokens g, g + 8
+            const uint32_t c_even = __shfl_sync(0xffffffffu, czero, 9 * tg), c_odd = __shfl_sync(0xffffffffu, czero, 9 * tg + 4);
+            const uint32_t c01 = __byte_perm(c_even, c_odd, 0x5410u), c23 = __byte_perm(c_even, c_odd, 0x7632u);
             uint32_t v[4][C::VW];
             const uint32_t vrow = page + D + slice_word<C::VSB>(g) + 2 * tg * C::ROWB;
             const uint32_t vsh = slice_shift<C::VSB>(g);
@@ -344,12 +372,12 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
                 const uint32_t y = sh == 0 ? b[j] : sh + 16 <= 32 ? b[j] >> sh : __funnelshift_r(b[j], hi_b, sh);
                 return __byte_perm(x, y, 0x5410u);
             };
-            auto code_half2 = [&](uint32_t up, uint32_t down, int i) {
+            auto code_half2 = [&](uint32_t up, uint32_t down, int i, uint32_t zero) {
                 const int sh = i < CLO ? VB * i + 1 : VB * i - DOWN;
                 const uint32_t w = ((i < CLO ? up : down) & (((1u << VB) - 1u) * 0x00010001u << sh)) | 0x64006400u;
-                const float inv = 1.f / static_cast<float>(1 << sh), off = -(1024.f * inv + kCtr);
+                const float inv = 1.f / static_cast<float>(1 << sh), off = -1024.f * inv;
                 const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&w), __floats2half2_rn(inv, inv),
-                                          __floats2half2_rn(off, off));
+                                          __hsub2(__floats2half2_rn(off, off), *reinterpret_cast<const __half2*>(&zero)));
                 return *reinterpret_cast<const uint32_t*>(&r);
             };
 #pragma unroll
@@ -358,15 +386,23 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
 #pragma unroll
                 for (int i = 0; i < CPW; i++) {
                     if (w * CPW + i >= D / 8) break;
-                    h01[w * CPW + i] = code_half2(x << 1, x >> DOWN, i);
-                    h23[w * CPW + i] = code_half2(y << 1, y >> DOWN, i);
+                    h01[w * CPW + i] = code_half2(x << 1, x >> DOWN, i, c01);
+                    h23[w * CPW + i] = code_half2(y << 1, y >> DOWN, i, c23);
                 }
             }
+            // (a page's sum is a new MMA chain, added in fp32: sums over many pages stay rounded, not truncated)
 #pragma unroll
-            for (int mt = 0; mt < NMT; mt++)
+            for (int mt = 0; mt < NMT; mt++) {
+                float o[NH][4];
 #pragma unroll
                 for (int x = 0; x < NH; x++)
-                    mma_16816(oacc[x][mt], h01[2 * mt], h01[2 * mt + 1], h23[2 * mt], h23[2 * mt + 1], pb[x][0], pb[x][1]);
+                    mma_16816_z(o[x], h01[2 * mt], h01[2 * mt + 1], h23[2 * mt], h23[2 * mt + 1], pb[x][0], pb[x][1]);
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+#pragma unroll
+                    for (int h = 0; h < HL; h++)
+                        oacc[mt][j * HL + h] += fmaf(NH == 1 ? o[0][2 * j + 1] : o[NH - 1][2 * j + h], kInvLo, o[0][2 * j + h]);
+            }
         }
 
         // ---- fold the warps' states
@@ -384,9 +420,7 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
             for (int j = 0; j < 2; j++)
 #pragma unroll
                 for (int h = 0; h < HL; h++)
-                    xo[(warp * C::OL + (mt * 2 + j) * HL + h) * 32 + lane] =
-                        NH == 1 ? fmaf(oacc[0][mt][2 * j + 1], kInvLo, oacc[0][mt][2 * j])
-                                : fmaf(oacc[NH - 1][mt][2 * j + h], kInvLo, oacc[0][mt][2 * j + h]);
+                    xo[(warp * C::OL + (mt * 2 + j) * HL + h) * 32 + lane] = oacc[mt][j * HL + h] * (1.f / up);
         if (g == 0) {
 #pragma unroll
             for (int h = 0; h < HL; h++) {

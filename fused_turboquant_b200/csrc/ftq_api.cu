@@ -754,7 +754,7 @@ static unsigned long long next_epoch() {
 static size_t counter_bytes(int B, int Hkv, int n_layers) {
     const size_t units = static_cast<size_t>(n_layers > 0 ? n_layers : 0) * (B > 0 ? B : 0) *
                          (Hkv > 0 ? Hkv : 0);
-    return (256 + 2 * units * sizeof(int) + 255) / 256 * 256;
+    return (256 + units * sizeof(int) + 255) / 256 * 256;
 }
 
 size_t ftq_decode_workspace_bytes(int B, int Hq, int Hkv, int head_dim, int max_seq_len,

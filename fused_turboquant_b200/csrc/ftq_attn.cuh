@@ -91,8 +91,8 @@ struct AttnParams {
     int n_units;
     unsigned long long epoch;
     // equal-share tensor-core kernel: sequences b0 .. b0 + B - 1 of the batch's B_stride, n_layers
-    // layers; context lengths are cut to max_seq; pages per CTA at least min_share; unit_counter
-    // holds two counters per unit
+    // layers; context lengths are cut to max_seq; pages per CTA at least min_share; a unit's counter
+    // holds 16 bits for each warp that finishes pieces
     int n_layers, b0, B_stride, max_seq, min_share;
     void* out;                  // [L*B, Hq, D]
     int out_dtype;

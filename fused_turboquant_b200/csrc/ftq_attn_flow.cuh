@@ -174,7 +174,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     unsigned long long* epoch_word = reinterpret_cast<unsigned long long*>(p.work_counter + 2);
     if (blockIdx.x == 0) {
-        for (int i = tid; i < 2 * p.n_units; i += THREADS) p.unit_counter[i] = 0;
+        for (int i = tid; i < p.n_units; i += THREADS) p.unit_counter[i] = 0;
         if (tid == 0) {
             p.work_counter[1] = 0;
             if (p.b0 == 0) p.work_counter[kStatusWord] = 0;   // (the call's: its later launches add to it)
@@ -584,12 +584,12 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             __threadfence();
             __syncwarp();
             await_epoch();
-            int old = 0;
+            uint32_t old = 0;   // (16 bits of the unit's counter for each finishing warp)
             if (lane == 0) {
                 const int64_t unit = (static_cast<int64_t>(it.layer) * p.B + it.b) * p.Hkv + it.hkv;
-                old = atomicAdd(p.unit_counter + 2 * unit + warp, 1);
+                old = static_cast<uint32_t>(atomicAdd(p.unit_counter + unit, 1 << (16 * warp))) >> (16 * warp) & 0xffffu;
             }
-            if (__shfl_sync(0xffffffffu, old, 0) != static_cast<int>(c1 - c0)) return;
+            if (__shfl_sync(0xffffffffu, old, 0) != static_cast<uint32_t>(c1 - c0)) return;
             __threadfence();
             // (the order of the sum is the order of the CTAs, whoever merges)
             m = -INFINITY;

@@ -80,6 +80,13 @@ def load() -> ctypes.CDLL:
 _native = None
 
 
+def native_tag() -> str:
+    """What the compiled host path is bound to besides its source: torch's and Python's binary interfaces."""
+    import importlib.metadata
+    import sysconfig
+    return f"ftq-native-for torch-{importlib.metadata.version('torch')} {sysconfig.get_config_var('SOABI')}"
+
+
 def native():
     """The compiled host path (csrc/ftq_torch.cpp), bound to this library's entry points."""
     global _native
@@ -92,6 +99,10 @@ def native():
             raise RuntimeError(
                 "fused_turboquant_b200/_native.so is missing or does not load: build it with "
                 f"`python -m fused_turboquant_b200.build` ({e})") from e
+        if ext.BUILT_FOR != native_tag():
+            raise RuntimeError(
+                f"fused_turboquant_b200/_native.so is {ext.BUILT_FOR!r}, this is {native_tag()!r}: build it "
+                "with `python -m fused_turboquant_b200.build`")
         from . import kernels
 
         ext.bind({n: ctypes.cast(getattr(lib, n), ctypes.c_void_p).value for n in SIGNATURES},

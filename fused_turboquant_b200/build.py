@@ -15,6 +15,8 @@ import shutil
 import subprocess
 import sys
 
+from ._lib import native_tag
+
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
@@ -55,32 +57,42 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found: cannot build libftq_b200.so")
 
 
+def _run(cmd: list, out: str, what: str) -> str:
+    """Run a compiler or linker whose output file is `out`; the file appears complete or not at all (another
+    process may have the one before loaded)."""
+    part = f"{out}.{os.getpid()}.part"
+    r = subprocess.run([*cmd, "-o", part], capture_output=True, text=True)
+    if r.returncode != 0:
+        if os.path.exists(part):
+            os.remove(part)
+        raise RuntimeError(f"{what} failed:\n{r.stdout}\n{r.stderr}")
+    os.replace(part, out)
+    return r.stderr
+
+
 def _build_native() -> None:
     import sysconfig
 
     import torch
     src = os.path.join(CSRC, "ftq_torch.cpp")
-    if not _unit_stale("ftq_torch.cpp", NATIVE_PATH):
-        return
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
-           "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(root, "include"),
-           "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
-           "-I" + os.path.join(cuda, "include"), src, "-o", NATIVE_PATH,
-           "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10",
-           "-lc10_cuda"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"g++ failed for {src}:\n{r.stdout}\n{r.stderr}")
+    _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+          f'-DFTQ_BUILT_FOR="{native_tag()}"',
+          "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(root, "include"),
+          "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+          "-I" + os.path.join(cuda, "include"), src,
+          "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10",
+          "-lc10_cuda"], NATIVE_PATH, f"g++ for {src}")
 
 
-def _sources_mtime() -> float:
-    m = os.path.getmtime(os.path.join(PKG_DIR, "..", "include", "ftq_b200.h"))
-    for f in os.listdir(CSRC):
-        m = max(m, os.path.getmtime(os.path.join(CSRC, f)))
-    return m
+def _native_stale() -> bool:
+    """Older than its own sources, or compiled against another torch or Python."""
+    if _older(NATIVE_PATH, _deps(os.path.join(CSRC, "ftq_torch.cpp"))):
+        return True
+    with open(NATIVE_PATH, "rb") as f:
+        return native_tag().encode() not in f.read()
 
 
 _INCLUDE = re.compile(r'^\s*#\s*include\s+"([^"]+)"', re.M)
@@ -100,18 +112,22 @@ def _deps(path: str, seen=None) -> set:
     return seen
 
 
-def _unit_stale(src: str, obj: str) -> bool:
-    if not os.path.exists(obj):
+def _older(out: str, deps) -> bool:
+    """`out` does not exist or is older than one of `deps`."""
+    if not os.path.exists(out):
         return True
-    t = os.path.getmtime(obj)
-    return any(os.path.getmtime(d) > t for d in _deps(os.path.join(CSRC, src)))
+    t = os.path.getmtime(out)
+    return any(os.path.getmtime(d) > t for d in deps)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile and link the library (and the wait-expiry test library) if missing or older than
-    the sources."""
-    if not force and all(os.path.exists(l) and os.path.getmtime(l) >= _sources_mtime()
-                         for l in (LIB_PATH, TEST_LIB_PATH, NATIVE_PATH)):
+    """Compile and link what is missing or older than its own sources: the library, the wait-expiry test
+    library, the host path."""
+    cuda_deps = set().union(*(_deps(os.path.join(CSRC, u[0])) for u in UNITS + [TEST_UNIT]))
+    cuda_stale = force or any(_older(l, cuda_deps) for l in (LIB_PATH, TEST_LIB_PATH))
+    if force or _native_stale():
+        _build_native()
+    if not cuda_stale:
         return LIB_PATH
     nvcc = _nvcc()
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -120,27 +136,19 @@ def build(force: bool = False, verbose: bool = False) -> str:
     def compile_one(unit):
         src, tag, defs = unit
         obj = os.path.join(OBJ_DIR, f"{tag}.o")
-        if not force and not verbose and not _unit_stale(src, obj):
+        if not force and not verbose and not _older(obj, _deps(os.path.join(CSRC, src))):
             return obj      # up to date: only units whose sources changed are recompiled
-        cmd = [nvcc, *NVCC_FLAGS, *extra, *defs, "-c", os.path.join(CSRC, src), "-o", obj]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            raise RuntimeError(f"nvcc failed for {src} {defs}:\n{r.stdout}\n{r.stderr}")
+        err = _run([nvcc, *NVCC_FLAGS, *extra, *defs, "-c", os.path.join(CSRC, src)], obj, f"nvcc for {src} {defs}")
         if verbose:
-            sys.stderr.write(r.stderr)
+            sys.stderr.write(err)
         return obj
 
     with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
-        native = ex.submit(_build_native)
         objs = list(ex.map(compile_one, UNITS + [TEST_UNIT]))
-        native.result()
     test_obj = objs.pop()
     for lib, members in ((LIB_PATH, objs),
                          (TEST_LIB_PATH, [test_obj if o.endswith("attn_d128.o") else o for o in objs])):
-        cmd = [nvcc, "-shared", "-o", lib, *members, "-lcudart"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+        _run([nvcc, "-shared", *members, "-lcudart"], lib, f"link of {lib}")
     return LIB_PATH
 
 

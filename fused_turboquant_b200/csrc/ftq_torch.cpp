@@ -714,5 +714,7 @@ PyMODINIT_FUNC PyInit__native(void) {
 #define X(name) names.name = PyUnicode_InternFromString(#name);
     FTQ_NAMES(X)
 #undef X
-    return PyModule_Create(&module_def);
+    PyObject* m = PyModule_Create(&module_def);
+    if (m && PyModule_AddStringConstant(m, "BUILT_FOR", FTQ_BUILT_FOR) < 0) Py_CLEAR(m);
+    return m;
 }

@@ -1,0 +1,61 @@
+"""What build() recompiles (CPU; the compilers are replaced by a recorder)."""
+import os
+
+import pytest
+
+from fused_turboquant_b200 import build
+
+
+@pytest.fixture
+def outputs(tmp_path, monkeypatch):
+    """Outputs that are up to date, in a folder of their own; the list of outputs build() makes."""
+    made = []
+
+    def fake_run(cmd, **kw):
+        out = cmd[cmd.index("-o") + 1]
+        made.append(out)
+        with open(out, "wb") as f:
+            f.write(" ".join(cmd).encode())
+        return type("R", (), dict(returncode=0, stdout="", stderr=""))
+
+    monkeypatch.setattr(build.subprocess, "run", fake_run)
+    monkeypatch.setattr(build, "_nvcc", lambda: "/usr/local/cuda/bin/nvcc")
+    monkeypatch.setattr(build, "OBJ_DIR", str(tmp_path / "build"))
+    for name in ("LIB_PATH", "TEST_LIB_PATH", "NATIVE_PATH"):
+        monkeypatch.setattr(build, name, str(tmp_path / (name + ".so")))
+    build.build()
+    made.clear()
+    return made
+
+
+def test_up_to_date_outputs_are_left_alone(outputs, monkeypatch):
+    build.build()
+    assert outputs == []
+    # the host path is older than a kernel, which it does not include
+    ages = {build.NATIVE_PATH: 150, build.LIB_PATH: 300, build.TEST_LIB_PATH: 300,
+            os.path.join(build.CSRC, "ftq_attn_flow.cuh"): 200}
+    monkeypatch.setattr(os.path, "getmtime", lambda p: ages.get(p, 100))
+    build.build()
+    assert outputs == []
+
+
+def test_force_rebuilds_everything(outputs):
+    build.build(force=True)
+    text = " ".join(outputs)
+    assert all(os.path.basename(p) in text for p in (build.LIB_PATH, build.TEST_LIB_PATH, build.NATIVE_PATH))
+
+
+def test_another_torch_makes_the_host_path_stale(outputs, monkeypatch):
+    import importlib.metadata
+    real = importlib.metadata.version
+    monkeypatch.setattr(importlib.metadata, "version", lambda n: "99.0" if n == "torch" else real(n))
+    build.build()
+    assert len(outputs) == 1 and os.path.basename(build.NATIVE_PATH) in outputs[0]
+    build.build()
+    assert len(outputs) == 1
+
+
+def test_outputs_appear_complete(outputs):
+    """Nothing is written under an output's own name: a process that has it loaded keeps its file."""
+    build.build(force=True)
+    assert not set(outputs) & {build.LIB_PATH, build.TEST_LIB_PATH, build.NATIVE_PATH}

@@ -67,6 +67,7 @@ struct EncodeJobs {
     SignBits signs;
     float rsqrt_d;                 // fp32(D ** -0.5)
     int64_t n_vec;                 // vectors per job and layer
+    int n_layers;
 };
 
 // Transposition of an 8-lane x (items per word) matrix of BITS-wide items: afterwards lane j

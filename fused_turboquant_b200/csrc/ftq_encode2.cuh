@@ -139,7 +139,12 @@ __host__ __device__ constexpr int encode2_threads(int D) { return D >= 256 ? 512
 // boundaries in lower cells.
 typedef float2 QuantTable[kQuantCells][16];
 
-template <int D, int BITS, typename T>
+// LAYERS: the groups of eight vectors of all layers are one line, dealt to the warps of the grid in turn.
+// (A grid per layer either builds the table once per layer and CTA or leaves SMs idle: 80 layers of 2048
+// tokens, K and V of 8 heads of 128, took 658 us with a wave of CTAs per layer, 764 us with one wave divided
+// among the layers and rounded down; 420 us so.)  With one layer the step is a constant and the layer zero.
+// Vector numbers are below 2^31: 32-bit arithmetic (524288 tokens of one layer: 1330 -> 1301 us).
+template <int D, int BITS, bool LAYERS, typename T>
 __device__ __forceinline__ void encode2_body(const EncodeJobs& jobs, const EncodeJob& job,
                                              QuantTable& lut, float* tbuf) {
     constexpr int E = D / kOctet;
@@ -152,7 +157,7 @@ __device__ __forceinline__ void encode2_body(const EncodeJobs& jobs, const Encod
     constexpr bool NARROW = sizeof(T) == 2;                 // bf16 / fp16 input
     const EncodeSource& src = job.src;
     const EncodeSink& sink = job.sink;
-    const int64_t n_vec = jobs.n_vec;
+    const uint32_t n_vec = static_cast<uint32_t>(jobs.n_vec);   // (below 2^31)
 
     const int tid = threadIdx.x;
     const int lane = tid & 31, wip = tid >> 5;
@@ -174,10 +179,29 @@ __device__ __forceinline__ void encode2_body(const EncodeJobs& jobs, const Encod
     const uint32_t lut_col = (lane & 15) * 8;
     float* slot = tbuf + (wip * 4 + sub) * SLOT;
 
-    const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + tid) >> 5;
-    const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    const T* xbase = static_cast<const T*>(src.base) + blockIdx.y * src.layer_stride;
-    const int64_t sink_layer = blockIdx.y * sink.layer_stride;
+    // (layer, first vector) of the warp's group and the step to its next one
+    const uint32_t warp = (blockIdx.x * blockDim.x + tid) >> 5;
+    const uint32_t n_warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t groups = (n_vec + 7) >> 3;
+    uint32_t layer = 0, step_layers = 0;
+    uint32_t base = 8 * warp, step = 8 * n_warps;
+    if constexpr (LAYERS) {
+        layer = warp / groups;
+        base = 8 * (warp - layer * groups);
+        step_layers = n_warps / groups;
+        step = 8 * (n_warps - step_layers * groups);
+    }
+    auto more = [&]() { return LAYERS ? layer < static_cast<uint32_t>(jobs.n_layers) : base < n_vec; };
+    auto advance = [&]() {
+        base += step;
+        if constexpr (LAYERS) {
+            layer += step_layers;
+            if (base >= n_vec) {
+                base -= 8 * groups;
+                layer++;
+            }
+        }
+    };
 
     // sign masks in the load layout: per element for fp32 input; for 16-bit input one mask per
     // packed pair of elements (bits 15 and 31), applied before the values are widened
@@ -199,8 +223,10 @@ __device__ __forceinline__ void encode2_body(const EncodeJobs& jobs, const Encod
     // stand in for vectors past the end) and fetch the slots their codes go to
     Raw8<T> rawA[NCH], rawB[NCH];
     int64_t slotA = -1, slotB = -1;
-    auto issue_loads = [&](int64_t base) {
-        const int64_t vA = base + sub, vB = base + 4 + sub;
+    auto issue_loads = [&]() {
+        const T* xbase = static_cast<const T*>(src.base);
+        if constexpr (LAYERS) xbase += layer * src.layer_stride;
+        const uint32_t vA = base + sub, vB = base + 4 + sub;
         slotA = load_slot(sink, vA, vA < n_vec);
         slotB = load_slot(sink, vB, vB < n_vec);
         if (vA < n_vec) {
@@ -222,10 +248,12 @@ __device__ __forceinline__ void encode2_body(const EncodeJobs& jobs, const Encod
             for (int i = 0; i < NCH; i++) zero_raw8<T>(rawB[i]);
         }
     };
-    if (warp * 8 < n_vec) issue_loads(warp * 8);
+    if (more()) issue_loads();
 
-    for (int64_t base = warp * 8; base < n_vec; base += n_warps * 8) {
-        const int64_t vA = base + sub, vB = base + 4 + sub;
+    while (more()) {
+        const uint32_t vA = base + sub, vB = base + 4 + sub;
+        const int64_t sink_layer = LAYERS ? layer * sink.layer_stride : 0;
+        advance();
         const bool okA = vA < n_vec, okB = vB < n_vec;
         const int64_t cur_slotA = slotA, cur_slotB = slotB;
         u64 p[E];
@@ -249,7 +277,7 @@ __device__ __forceinline__ void encode2_body(const EncodeJobs& jobs, const Encod
         }
         // next group's loads fly while this one is processed (16-bit inputs: 4 registers per run)
         if constexpr (NARROW) {
-            if (base + n_warps * 8 < n_vec) issue_loads(base + n_warps * 8);
+            if (more()) issue_loads();
         }
         // stages h = 1, 2, 4 on the coordinates inside a run
         stage2<E, 0>(p);
@@ -353,22 +381,22 @@ __device__ __forceinline__ void encode2_body(const EncodeJobs& jobs, const Encod
         emit_vector<D, BITS>(wA, normA, okA, vA, cur_slotA, sink, sink_layer, lane, tc);
         emit_vector<D, BITS>(wB, normB, okB, vB, cur_slotB, sink, sink_layer, lane, tc);
         if constexpr (!NARROW) {
-            if (base + n_warps * 8 < n_vec) issue_loads(base + n_warps * 8);
+            if (more()) issue_loads();
         }
     }
 }
 
-template <int D, typename T>
+template <int D, bool LAYERS, typename T>
 __device__ __forceinline__ void encode2_job(const EncodeJobs& jobs, const EncodeJob& job, QuantTable& lut,
                                             float* tbuf) {
     switch (job.bits) {
-        case 2: encode2_body<D, 2, T>(jobs, job, lut, tbuf); break;
-        case 3: encode2_body<D, 3, T>(jobs, job, lut, tbuf); break;
-        case 4: encode2_body<D, 4, T>(jobs, job, lut, tbuf); break;
+        case 2: encode2_body<D, 2, LAYERS, T>(jobs, job, lut, tbuf); break;
+        case 3: encode2_body<D, 3, LAYERS, T>(jobs, job, lut, tbuf); break;
+        case 4: encode2_body<D, 4, LAYERS, T>(jobs, job, lut, tbuf); break;
     }
 }
 
-template <int D, typename T>
+template <int D, bool LAYERS, typename T>
 __global__ void __launch_bounds__(encode2_threads(D), 512 / encode2_threads(D))
 encode2_kernel(const __grid_constant__ EncodeJobs jobs) {
     // the quantiser table is a static array: its shared-memory offset is then an immediate of
@@ -379,8 +407,8 @@ encode2_kernel(const __grid_constant__ EncodeJobs jobs) {
     // A body per job: the fields of a job that is known at compile time are operands in the constant
     // bank, those of jobs.job[blockIdx.z] took registers and instructions inside the loop (524288 tokens,
     // K and V of 8 heads of 128: 1390 us, 1330 us so).
-    if (blockIdx.z == 0) encode2_job<D, T>(jobs, jobs.job[0], lut, tbuf);
-    else encode2_job<D, T>(jobs, jobs.job[1], lut, tbuf);
+    if (blockIdx.z == 0) encode2_job<D, LAYERS, T>(jobs, jobs.job[0], lut, tbuf);
+    else encode2_job<D, LAYERS, T>(jobs, jobs.job[1], lut, tbuf);
 }
 
 }  // namespace ftq

@@ -10,22 +10,23 @@
 namespace ftq {
 
 template <typename T>
-static cudaError_t run(const EncodeJobs& jobs, int n_jobs, bool bulk, int n_layers, cudaStream_t stream) {
+static cudaError_t run(EncodeJobs jobs, int n_jobs, bool bulk, int n_layers, cudaStream_t stream) {
     const int64_t n = jobs.n_vec;
     if (bulk) {
         // 16 warps per SM: two CTAs of 8 warps, or one of 16 where two transpose areas would not
         // fit next to two copies of the quantiser table (head_dim 256); a warp pass = 8 vectors.
-        // Persistent: the jobs and layers share one wave of CTAs.
+        // Persistent: the jobs share one wave of CTAs, a job's layers share its part of them.
         constexpr int threads = encode2_threads(FTQ_D);
         constexpr int smem = encode2_smem_bytes(FTQ_D, threads / 32);
-        constexpr auto kern = encode2_kernel<FTQ_D, T>;
-        const cudaError_t e = allow_smem<kern>(smem);
+        constexpr auto one = encode2_kernel<FTQ_D, false, T>, many = encode2_kernel<FTQ_D, true, T>;
+        const cudaError_t e = n_layers > 1 ? allow_smem<many>(smem) : allow_smem<one>(smem);
         if (e != cudaSuccess) return e;
-        const int64_t want = (n + threads / 4 - 1) / (threads / 4);
-        const int64_t share = static_cast<int64_t>(sm_count()) * (512 / threads) / (n_jobs * n_layers);
-        const int64_t cap = share > 1 ? share : 1;
-        const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), n_layers, n_jobs);
-        kern<<<grid, threads, smem, stream>>>(jobs);
+        const int64_t want = ((n + 7) / 8 * n_layers + threads / 32 - 1) / (threads / 32);
+        const int64_t cap = static_cast<int64_t>(sm_count()) * (512 / threads) / n_jobs;
+        const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), 1, n_jobs);
+        jobs.n_layers = n_layers;
+        if (n_layers > 1) many<<<grid, threads, smem, stream>>>(jobs);
+        else one<<<grid, threads, smem, stream>>>(jobs);
         return cudaGetLastError();
     }
     constexpr int threads = 128;                       // 4 warps, a vector each

@@ -98,21 +98,33 @@ cudaError_t dispatch_encode(int d, int dtype, ftq::EncodeJobs& jobs, int n_jobs,
     if (jobs.n_vec >= (1ll << 31)) return cudaErrorInvalidValue;
     jobs.rsqrt_d = rsqrt_dim(d);
     // A handful of vectors (a decode step) is latency-bound: the warp-per-vector kernel.  From 2048
-    // on the SMs have enough vectors for the throughput kernel's octets, when the codebooks allow.
-    bool bulk = jobs.n_vec >= 2048;
+    // on the SMs have enough vectors for octets: with the table quantiser when the codebook allows, with
+    // every boundary compared when not (2048 vectors of K and V: 5.9 us against a warp's 6.2, 65536: 52
+    // against 78).
+    ftq::Encode kind[2];
     for (int i = 0; i < n_jobs; i++) {
         ftq::EncodeJob& j = jobs.job[i];
         if (j.src.n_inner <= 0 || j.sink.Hkv <= 0) return cudaErrorInvalidValue;
         j.src.div_inner = ftq::make_fastdiv(static_cast<uint32_t>(j.src.n_inner));
         j.sink.div_hkv = ftq::make_fastdiv(static_cast<uint32_t>(j.sink.Hkv));
-        bulk = bulk && table_quantizer_takes(j);
+        kind[i] = jobs.n_vec < 2048 ? ftq::Encode::kFew : table_quantizer_takes(j) ? ftq::Encode::kTable : ftq::Encode::kAnyCodebook;
     }
-    switch (d) {
-        case 64: return ftq::launch_encode_d64(dtype, jobs, n_jobs, bulk, n_layers, st);
-        case 128: return ftq::launch_encode_d128(dtype, jobs, n_jobs, bulk, n_layers, st);
-        case 256: return ftq::launch_encode_d256(dtype, jobs, n_jobs, bulk, n_layers, st);
-    }
-    return cudaErrorInvalidValue;
+    auto launch = [&](const ftq::EncodeJobs& js, int n, ftq::Encode k) {
+        switch (d) {
+            case 64: return ftq::launch_encode_d64(dtype, js, n, k, n_layers, st);
+            case 128: return ftq::launch_encode_d128(dtype, js, n, k, n_layers, st);
+            case 256: return ftq::launch_encode_d256(dtype, js, n, k, n_layers, st);
+        }
+        return cudaErrorInvalidValue;
+    };
+    if (n_jobs == 1 || kind[0] == kind[1]) return launch(jobs, n_jobs, kind[0]);
+    // One of K and V has a codebook for the table: a launch each, unless they are so small that the launches
+    // show (K and V of 4096 tokens, 8 heads of 128: 26.8 us as two, 28.8 as one; of 512 tokens: 12.6, 7.6).
+    if (jobs.n_vec * n_layers < 32768) return launch(jobs, 2, ftq::Encode::kAnyCodebook);
+    const cudaError_t e = launch(jobs, 1, kind[0]);
+    if (e != cudaSuccess) return e;
+    jobs.job[0] = jobs.job[1];
+    return launch(jobs, 1, kind[1]);
 }
 
 // fp32 -> fp16 -> fp32 with round to nearest even (host side).

@@ -211,8 +211,8 @@ __device__ __forceinline__ void emit_vector(const uint32_t (&w)[NW], float norm,
     }
 }
 
-// Encode of a handful of vectors (a decode step's new tokens), and of codebooks that the table
-// quantiser of encode2_kernel cannot take.  Latency is what counts: a WARP takes one vector, so
+// Encode of a handful of vectors (a decode step's new tokens).  Latency is what counts: a WARP takes one
+// vector, so
 // that a lane carries D/32 values through the chain load -> butterfly -> norm -> division ->
 // bucketise.  One token of 8 KV heads, bf16, 4 bits: an octet per vector (D/8 values per lane) and
 // a launch per tensor took 8.3 us at D = 128 and 14.9 us at 256; this takes 2.5 and 3.0 us for
@@ -338,6 +338,86 @@ __global__ void __launch_bounds__(256) encode_kernel(const __grid_constant__ Enc
         case 3: encode_body<D, 3, T>(jobs, job); break;
         case 4: encode_body<D, 4, T>(jobs, job); break;
     }
+}
+
+// Bulk encode with a codebook that the table quantiser of encode2_kernel cannot take: an octet of lanes per
+// vector, four vectors a warp, every boundary compared.  32768 tokens, K and V of 8 heads of 128, 4 bits:
+// 191 us; 295 us with a warp per vector, which exchanges two more butterfly stages between lanes and has a
+// quarter of the vectors in flight.
+template <int D, int BITS, typename T>
+__device__ __forceinline__ void encode_octet_body(const EncodeJobs& jobs, const EncodeJob& job) {
+    constexpr int E = D / kOctet;                           // values per lane
+    constexpr int NW = BITS == 2 ? (E + 15) / 16 : E / 8;   // words of packed items per lane
+    const int lane = threadIdx.x & 31, t = lane & 7, sub = lane >> 3;
+    const int64_t n_vec = jobs.n_vec;
+    const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    const EncodeSource& src = job.src;
+    const T* xbase = static_cast<const T*>(src.base) + blockIdx.y * src.layer_stride;
+    const int64_t sink_layer = blockIdx.y * job.sink.layer_stride;
+    uint32_t sgn[E];
+#pragma unroll
+    for (int r = 0; r < E; r++) sgn[r] = sign_mask(jobs.signs, load_coord(t, r));
+    const TransposeConsts<BITS> tc = transpose_consts<BITS>(lane);
+
+    for (int64_t base = warp * 4; base < n_vec; base += n_warps * 4) {
+        const int64_t v = base + sub;
+        const bool valid = v < n_vec;
+        const int64_t slot = load_slot(job.sink, v, valid);
+        const int64_t at = valid ? v : n_vec - 1;   // (octets left over encode the last vector and store nothing)
+        const int64_t outer = fast_div(static_cast<uint32_t>(at), src.div_inner);
+        const T* row = xbase + outer * src.outer_stride + (at - outer * src.n_inner) * src.inner_stride;
+        float y[E];
+#pragma unroll
+        for (int i = 0; i < E / 8; i++) {
+            float tmp[8];
+            load8<T>(row + 8 * (t + 8 * i), tmp);
+#pragma unroll
+            for (int c = 0; c < 8; c++) y[8 * i + c] = __uint_as_float(__float_as_uint(tmp[c]) ^ sgn[8 * i + c]);
+        }
+        octet_fwht<E>(y, lane);
+        // scaled; lane l sums the squares of coordinates l + 8k in order, the octet its eight sums
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            y[k] = __fmul_rn(y[k], jobs.rsqrt_d);
+            acc = __fadd_rn(acc, __fmul_rn(y[k], y[k]));
+        }
+        float s = __shfl_sync(0xffffffffu, acc, 0, 8);
+#pragma unroll
+        for (int l = 1; l < 8; l++) s = __fadd_rn(s, __shfl_sync(0xffffffffu, acc, l, 8));
+        const float norm = __fsqrt_rn(s);
+        const float denom = __fadd_rn(norm, 1e-8f);
+        uint32_t w[NW];
+#pragma unroll
+        for (int i = 0; i < NW; i++) w[i] = 0u;
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const float nv = __fdiv_rn(y[k], denom);
+            uint32_t code = 0;
+#pragma unroll
+            for (int b = 0; b < (1 << BITS) - 1; b++) code += (job.bounds[b] < nv) ? 1u : 0u;
+            if constexpr (BITS == 2) w[k >> 4] |= code << (2 * (((k >> 1) & 7) | ((k & 1) << 3)));
+            else w[k >> 3] |= code << (BITS * (k & 7));
+        }
+        emit_vector<D, BITS>(w, norm, valid, v, slot, job.sink, sink_layer, lane, tc);
+    }
+}
+
+template <int D, typename T>
+__device__ __forceinline__ void encode_octet_job(const EncodeJobs& jobs, const EncodeJob& job) {
+    switch (job.bits) {
+        case 2: encode_octet_body<D, 2, T>(jobs, job); break;
+        case 3: encode_octet_body<D, 3, T>(jobs, job); break;
+        case 4: encode_octet_body<D, 4, T>(jobs, job); break;
+    }
+}
+
+template <int D, typename T>
+__global__ void __launch_bounds__(256) encode_octet_kernel(const __grid_constant__ EncodeJobs jobs) {
+    // (a body per job: its boundaries are constant operands)
+    if (blockIdx.z == 0) encode_octet_job<D, T>(jobs, jobs.job[0]);
+    else encode_octet_job<D, T>(jobs, jobs.job[1]);
 }
 
 }  // namespace ftq

@@ -10,9 +10,9 @@
 namespace ftq {
 
 template <typename T>
-static cudaError_t run(EncodeJobs jobs, int n_jobs, bool bulk, int n_layers, cudaStream_t stream) {
+static cudaError_t run(EncodeJobs jobs, int n_jobs, Encode kind, int n_layers, cudaStream_t stream) {
     const int64_t n = jobs.n_vec;
-    if (bulk) {
+    if (kind == Encode::kTable) {
         // 16 warps per SM: two CTAs of 8 warps, or one of 16 where two transpose areas would not
         // fit next to two copies of the quantiser table (head_dim 256); a warp pass = 8 vectors.
         // Persistent: the jobs share one wave of CTAs, a job's layers share its part of them.
@@ -29,6 +29,14 @@ static cudaError_t run(EncodeJobs jobs, int n_jobs, bool bulk, int n_layers, cud
         else one<<<grid, threads, smem, stream>>>(jobs);
         return cudaGetLastError();
     }
+    if (kind == Encode::kAnyCodebook) {
+        constexpr int threads = 256;                   // 8 warps, four vectors each
+        const int64_t want = (n + threads / 8 - 1) / (threads / 8);
+        const int64_t cap = static_cast<int64_t>(sm_count()) * 8;
+        const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), n_layers, n_jobs);
+        encode_octet_kernel<FTQ_D, T><<<grid, threads, 0, stream>>>(jobs);
+        return cudaGetLastError();
+    }
     constexpr int threads = 128;                       // 4 warps, a vector each
     const int64_t want = (n + threads / 32 - 1) / (threads / 32);
     const int64_t cap = static_cast<int64_t>(sm_count()) * 64;
@@ -37,12 +45,12 @@ static cudaError_t run(EncodeJobs jobs, int n_jobs, bool bulk, int n_layers, cud
     return cudaGetLastError();
 }
 
-cudaError_t FTQ_CAT(launch_encode_d, FTQ_D)(int dtype, const EncodeJobs& jobs, int n_jobs, bool bulk,
+cudaError_t FTQ_CAT(launch_encode_d, FTQ_D)(int dtype, const EncodeJobs& jobs, int n_jobs, Encode kind,
                                             int n_layers, cudaStream_t stream) {
     switch (dtype) {
-        case kF32: return run<float>(jobs, n_jobs, bulk, n_layers, stream);
-        case kF16: return run<__half>(jobs, n_jobs, bulk, n_layers, stream);
-        case kBF16: return run<__nv_bfloat16>(jobs, n_jobs, bulk, n_layers, stream);
+        case kF32: return run<float>(jobs, n_jobs, kind, n_layers, stream);
+        case kF16: return run<__half>(jobs, n_jobs, kind, n_layers, stream);
+        case kBF16: return run<__nv_bfloat16>(jobs, n_jobs, kind, n_layers, stream);
     }
     return cudaErrorInvalidValue;
 }

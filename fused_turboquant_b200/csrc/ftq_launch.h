@@ -11,8 +11,11 @@
 
 namespace ftq {
 
+// which kernel encodes: a warp per vector; two vectors per octet and a quantiser table; an octet per vector
+enum class Encode { kFew, kTable, kAnyCodebook };
+
 #define FTQ_DECLARE_LAUNCHERS(DD)                                                              \
-    cudaError_t launch_encode_d##DD(int dtype, const EncodeJobs& jobs, int n_jobs, bool bulk,   \
+    cudaError_t launch_encode_d##DD(int dtype, const EncodeJobs& jobs, int n_jobs, Encode kind, \
                                     int n_layers, cudaStream_t stream);                         \
     cudaError_t launch_attn_split_d##DD(int bits_k, int bits_v, bool paged, const AttnParams& p, \
                                         int n_lb, cudaStream_t stream);                         \

@@ -276,11 +276,9 @@ struct ChunkPlan {
     }
 };
 
-// The device-side description of a plan over `units` units (n_regions = 0 for the fp32 kernels'
-// single split).
-ftq::SplitPlan make_split(const ChunkPlan& pl, int64_t units, bool tensor_core) {
+// The device-side description of a plan over `units` units.
+ftq::SplitPlan make_split(const ChunkPlan& pl, int64_t units) {
     ftq::SplitPlan sp{};
-    if (!tensor_core) return sp;
     auto put = [&](int k, int64_t first_unit, int64_t first_item, int chunks, int tokens) {
         sp.r[k].first_unit = static_cast<int>(first_unit);
         sp.r[k].first_item = static_cast<int>(first_item);
@@ -384,7 +382,7 @@ ChunkPlan plan_chunks_uniform(int B, int Hq, int Hkv, int d, int seq_len) {
 // lowest modelled cost wins.  Chunks hold at most 8192 tokens (short enough for the dynamic
 // hand-out of items to even out ragged batches; their block ids are staged in shared memory)
 // and at least 1024.
-// The planner both tensor-core kernels share.  Cost of a plan = waves of items over the CTA slots
+// The streaming kernel's planner.  Cost of a plan = waves of items over the CTA slots
 // x (pages of an item + the fixed cost of an item, in pages); the cheapest plan wins, the fewest
 // chunks among equals.  A plan has up to two regions: as many units as fill whole waves of the
 // grid are cut into few, long chunks; the remaining units into more, shorter ones that share the
@@ -488,12 +486,11 @@ cudaError_t dispatch_split(int d, int bk, int bv, bool paged, const ftq::AttnPar
     return cudaErrorInvalidValue;
 }
 
-cudaError_t dispatch_mma(int d, int bk, int bv, bool shared_lut, const ftq::AttnParams& p, int n_lb,
-                         cudaStream_t st, bool* merged) {
+cudaError_t dispatch_mma(int d, int bk, int bv, bool shared_lut, const ftq::AttnParams& p, cudaStream_t st) {
     switch (d) {
-        case 64: return ftq::launch_attn_mma_d64(bk, bv, shared_lut, p, n_lb, st, merged);
-        case 128: return ftq::launch_attn_mma_d128(bk, bv, shared_lut, p, n_lb, st, merged);
-        case 256: return ftq::launch_attn_mma_d256(bk, bv, shared_lut, p, n_lb, st, merged);
+        case 64: return ftq::launch_attn_mma_d64(bk, bv, shared_lut, p, st);
+        case 128: return ftq::launch_attn_mma_d128(bk, bv, shared_lut, p, st);
+        case 256: return ftq::launch_attn_mma_d256(bk, bv, shared_lut, p, st);
     }
     return cudaErrorInvalidValue;
 }
@@ -750,10 +747,9 @@ int ftq_qk_scores(const float* q_rot, const uint8_t* k_codes, const void* k_norm
 
 // The tail of a decode workspace holds the counters of the tensor-core kernels: a 256-byte header
 // (work-item counter, count of finished CTAs, the 64-bit epoch word) and, from byte 256 on, one
-// counter per (layer, sequence, KV head) unit for the in-kernel split-KV merge.  The
-// barrier-synchronised kernel's launcher zeroes the header with a memset node; the streaming
-// kernel clears the tail itself under a per-launch epoch (see AttnParams), so one call is one
-// node in the stream and needs nothing from the call before it.
+// counter per (layer, sequence, KV head) unit for the in-kernel split-KV merge.  The kernels clear the
+// tail themselves under a per-launch epoch (see AttnParams), so one call is one node in the stream (one
+// per 1024 sequences in the equal-share kernel) and needs nothing from the call before it.
 static unsigned long long next_epoch() {
     static std::atomic<unsigned long long> counter{[] {
         std::random_device rd;
@@ -970,16 +966,13 @@ int ftq_paged_decode_attn(const void* q, int q_dtype, void* out, int out_dtype,
         p.epoch = next_epoch();
         p.n_layers = n_layers;
         p.max_seq = max_seq_len;
-        if (streams) p.split = make_split(pl, p.n_units, true);
-        bool merged = false;
-        e = dispatch_mma(head_dim, bits_k, bits_v, shared_lut, p, n_layers * B, st, &merged);
-        if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_decode_attn launch");
-        if (merged) return FTQ_OK;  // the streaming kernel finishes the merge itself
-    } else {
-        e = cudaMemsetAsync(p.work_counter, 0, 256, st);   // the status word
-        if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_decode_attn status reset");
-        e = dispatch_split(head_dim, bits_k, bits_v, true, p, n_layers * B, st);
+        if (streams) p.split = make_split(pl, p.n_units);
+        e = dispatch_mma(head_dim, bits_k, bits_v, shared_lut, p, st);   // (merge included)
+        return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_paged_decode_attn launch");
     }
+    e = cudaMemsetAsync(p.work_counter, 0, 256, st);   // the status word
+    if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_decode_attn status reset");
+    e = dispatch_split(head_dim, bits_k, bits_v, true, p, n_layers * B, st);
     if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_decode_attn split launch");
     e = dispatch_merge(head_dim, out_dtype, p.partials, out, seq_lens, 0, B, Hq, pl.n_chunks,
                        pl.chunk_tokens, static_cast<int64_t>(n_layers) * B * Hq, p.signs, st);

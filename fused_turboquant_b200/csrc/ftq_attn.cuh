@@ -75,19 +75,18 @@ struct AttnParams {
     // Tensor-core kernels: how the (layer, sequence, KV head) units are cut into work items (see
     // SplitPlan).  The fp32 kernels use one split for all units: n_chunks / chunk_tokens above.
     SplitPlan split;
-    // Counters of the tensor-core path.  work_counter[0] = next work item.  The barrier-synchronised
-    // kernel has the host zero it before the launch.  The streaming kernel clears its counters
-    // itself: CTA 0 zeroes work_counter[0] (tickets), work_counter[1] (CTAs that have left) and
-    // the unit counters, then stores `epoch` (unique per launch, never 0) into the 64-bit word at
-    // work_counter + 2; everybody checks for it before the first atomic on a counter, and the
-    // last CTA to leave stores 0 there, so that a replay of the same launch does not find its
-    // own epoch.
+    // Counters of the tensor-core kernels, which clear them themselves: CTA 0 zeroes work_counter[0]
+    // (tickets of the streaming kernel), work_counter[1] (CTAs that have left) and the unit counters,
+    // then stores `epoch` (unique per call, never 0) into the 64-bit word at work_counter + 2;
+    // everybody checks for it before the first atomic on a counter, and the last CTA to leave stores 0
+    // there, so that a replay of the same launch, or the call's next launch, does not find its own
+    // epoch.
     // work_counter[4] is the call's status word (kStatus* bits, cleared with the counters): what
     // the kernels of this call met; the host reads it on request (ftq_paged_decode_status).
     // nullptr for the contiguous entry points.
     int* work_counter;
-    // streaming tensor-core kernel: it finishes the split-KV merge itself
-    int* unit_counter;          // [n_units = L*B*Hkv] chunks delivered per unit
+    // the tensor-core kernels finish the split-KV merge themselves
+    int* unit_counter;          // [n_units = L*B*Hkv] chunks or pieces delivered per unit
     int n_units;
     unsigned long long epoch;
     // equal-share tensor-core kernel: sequences b0 .. b0 + B - 1 of the batch's B_stride, n_layers

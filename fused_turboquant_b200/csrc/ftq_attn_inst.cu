@@ -71,13 +71,12 @@ constexpr bool use_stream_kernel() {
 }
 
 template <int BK, int BV, bool SHARED, int NH>
-static cudaError_t run_flow(const AttnParams& p_in, cudaStream_t stream, bool* merged) {
+static cudaError_t run_flow(const AttnParams& p_in, cudaStream_t stream) {
     using C = MmaCfg<FTQ_D, BK, BV, NH>;
     static_assert(C::SMEM_BYTES <= C::LIMIT, "shared memory budget");
     constexpr auto kern = attn_flow_kernel<FTQ_D, BK, BV, SHARED, NH>;
     cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
-    *merged = true;
     AttnParams p = p_in;
     // a CTA's share is at least one stage per warp: less would only cut units into more rows to merge
     p.min_share = C::WARPS * C::NP;
@@ -108,7 +107,7 @@ static cudaError_t run_flow(const AttnParams& p_in, cudaStream_t stream, bool* m
 }
 
 template <int BK, int BV, bool SHARED, int NH>
-static cudaError_t run_mma_nh(const AttnParams& p, int n_lb, cudaStream_t stream, bool* merged) {
+static cudaError_t run_mma_nh(const AttnParams& p, cudaStream_t stream) {
     constexpr int D = FTQ_D;
     if constexpr (use_stream_kernel<BK, BV, NH>()) {
         using S = StreamCfg<D, BK, BV, NH>;
@@ -129,62 +128,54 @@ static cudaError_t run_mma_nh(const AttnParams& p, int n_lb, cudaStream_t stream
         cfg.stream = stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-#ifdef FTQ_NO_PDL
-        attr[0].val.programmaticStreamSerializationAllowed = 0;
-#else
         attr[0].val.programmaticStreamSerializationAllowed = 1;
-#endif
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        *merged = true;
         return cudaLaunchKernelEx(&cfg, kern, p, static_cast<int>(items));
     } else {
-        return run_flow<BK, BV, SHARED, NH>(p, stream, merged);
+        return run_flow<BK, BV, SHARED, NH>(p, stream);
     }
 }
 
 template <int BK, int BV, bool SHARED>
-static cudaError_t run_mma(const AttnParams& p, int n_lb, cudaStream_t stream, bool* merged) {
-    return p.Hq / p.Hkv <= 4 ? run_mma_nh<BK, BV, SHARED, 1>(p, n_lb, stream, merged)
-                             : run_mma_nh<BK, BV, SHARED, 2>(p, n_lb, stream, merged);
+static cudaError_t run_mma(const AttnParams& p, cudaStream_t stream) {
+    return p.Hq / p.Hkv <= 4 ? run_mma_nh<BK, BV, SHARED, 1>(p, stream)
+                             : run_mma_nh<BK, BV, SHARED, 2>(p, stream);
 }
 
 // FTQ_ONLY_BITS=<b> (a development aid, never set by the build script) instantiates the
 // tensor-core kernels for bits_k = bits_v = b only, which cuts the compile time of an experiment.
 template <int BK>
-static cudaError_t mma_by_bv(int bv, bool shared_lut, const AttnParams& p, int n_lb,
-                             cudaStream_t stream, bool* merged) {
+static cudaError_t mma_by_bv(int bv, bool shared_lut, const AttnParams& p, cudaStream_t stream) {
 #ifdef FTQ_ONLY_BITS
     if (BK != FTQ_ONLY_BITS || bv != FTQ_ONLY_BITS) return cudaErrorInvalidValue;
     if constexpr (BK == FTQ_ONLY_BITS) {
-        return shared_lut ? run_mma<BK, BK, true>(p, n_lb, stream, merged)
-                          : run_mma<BK, BK, false>(p, n_lb, stream, merged);
+        return shared_lut ? run_mma<BK, BK, true>(p, stream)
+                          : run_mma<BK, BK, false>(p, stream);
     }
 #else
-    if (shared_lut && bv == BK) return run_mma<BK, BK, true>(p, n_lb, stream, merged);
+    if (shared_lut && bv == BK) return run_mma<BK, BK, true>(p, stream);
     switch (bv) {
-        case 2: return run_mma<BK, 2, false>(p, n_lb, stream, merged);
-        case 3: return run_mma<BK, 3, false>(p, n_lb, stream, merged);
-        case 4: return run_mma<BK, 4, false>(p, n_lb, stream, merged);
+        case 2: return run_mma<BK, 2, false>(p, stream);
+        case 3: return run_mma<BK, 3, false>(p, stream);
+        case 4: return run_mma<BK, 4, false>(p, stream);
     }
 #endif
     return cudaErrorInvalidValue;
 }
 
 cudaError_t FTQ_CAT(launch_attn_mma_d, FTQ_D)(int bits_k, int bits_v, bool shared_lut,
-                                              const AttnParams& p, int n_lb, cudaStream_t stream,
-                                              bool* merged) {
+                                              const AttnParams& p, cudaStream_t stream) {
     switch (bits_k) {
-        case 2: return mma_by_bv<2>(bits_v, shared_lut, p, n_lb, stream, merged);
-        case 3: return mma_by_bv<3>(bits_v, shared_lut, p, n_lb, stream, merged);
-        case 4: return mma_by_bv<4>(bits_v, shared_lut, p, n_lb, stream, merged);
+        case 2: return mma_by_bv<2>(bits_v, shared_lut, p, stream);
+        case 3: return mma_by_bv<3>(bits_v, shared_lut, p, stream);
+        case 4: return mma_by_bv<4>(bits_v, shared_lut, p, stream);
     }
     return cudaErrorInvalidValue;
 }
 
 // CTAs per SM of the streaming kernel where launch_attn_mma picks it for this configuration, 0
-// where it picks the barrier-synchronised kernel (the host plans the split of the context
-// differently for the two)
+// where it picks the equal-share kernel (which needs no plan of the host)
 template <int BK, int BV, int NH>
 static constexpr int stream_ctas() {
     return use_stream_kernel<BK, BV, NH>() ? StreamCfg<FTQ_D, BK, BV, NH>::CTAS_PER_SM : 0;

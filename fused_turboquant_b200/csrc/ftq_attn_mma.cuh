@@ -127,13 +127,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::
-            "r"(dst), "l"(src), "r"(bytes), "r"(bar)
-        : "memory");
-}
-// The same copy with an L2 policy: KV pages are read once per decode step, so L2 is told to drop
+// Bulk copy with an L2 policy: KV pages are read once per decode step, so L2 is told to drop
 // them first (measured on B200: +1.5 % on the Llama-shaped K4V4 batch).
 __device__ __forceinline__ uint64_t l2_evict_first_policy() {
     uint64_t pol;

@@ -20,7 +20,7 @@ enum class Encode { kFew, kTable, kAnyCodebook };
     cudaError_t launch_attn_split_d##DD(int bits_k, int bits_v, bool paged, const AttnParams& p, \
                                         int n_lb, cudaStream_t stream);                         \
     cudaError_t launch_attn_mma_d##DD(int bits_k, int bits_v, bool shared_lut, const AttnParams& p, \
-                                      int n_lb, cudaStream_t stream, bool* merged);            \
+                                      cudaStream_t stream);                                   \
     cudaError_t launch_attn_chunk_d##DD(int bits_k, int bits_v, const ChunkAttnParams& p, int B, \
                                         cudaStream_t stream);                                   \
     int attn_mma_stream_ctas_d##DD(int bits_k, int bits_v, int group);                          \

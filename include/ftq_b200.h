@@ -170,7 +170,8 @@ int ftq_paged_store(const void *key, const void *value, int dtype, int64_t n_tok
  * packed pool through the block table (no gather, no dense K/V).
  * Replaces FusedTurboQuantImpl._forward_decode (vllm_plugin/attention_impl.py:431-521:
  * gather_compressed_kv_batched -> randomized_hadamard(q) -> fused_qk_scores_rht ->
- * softmax -> gather + decode V -> matmul) with one split-KV kernel plus a merge.
+ * softmax -> gather + decode V -> matmul) with one split-KV kernel, which merges
+ * its splits itself (fp32 queries and GQA groups above 8: a second launch does).
  *   q   [n_layers, B, Hq, D] of q_dtype, NOT rotated (rotation is fused)
  *   out [n_layers, B, Hq, D] of out_dtype, original space
  *   block_table [B, max_blocks] int32 device; seq_lens [B] int32 device
@@ -207,9 +208,9 @@ int ftq_paged_decode_attn(const void *q, int q_dtype, void *out, int out_dtype,
  *     (ftq_decode_workspace_bytes tells) is rejected with FTQ_ERR_WORKSPACE;
  *   - all calls on one GPU share the array and it keeps whatever the last call
  *     left (every partial row that is read is written first by the same call,
- *     and the counters in its tail are cleared at the start of every call,
- *     by the kernel itself or by a memset node), so two calls that may run at the same time on one GPU
- *     (different streams) corrupt each other: serialise them;
+ *     and the counters in its tail are cleared at the start of every call), so
+ *     two calls that may run at the same time on one GPU (different streams)
+ *     corrupt each other: serialise them;
  *   - the device that owns q / out / pool must be the current device of the
  *     calling thread: the size check and the scratch address are per device;
  *   - the first call on each device looks up the array's device address

@@ -31,8 +31,8 @@ def _filled_pool(d, bk, bv, Hkv, seq_lens, seed=0, extra_blocks=8):
 
 @pytest.mark.parametrize("d,G,bk,bv,qdtype", [
     (128, 4, 4, 4, torch.bfloat16),   # streaming tensor-core kernel
-    (128, 8, 3, 3, torch.bfloat16),   # barrier-synchronised tensor-core kernel, two head halves
-    (256, 2, 4, 2, torch.bfloat16),   # ... head_dim 256
+    (128, 8, 3, 3, torch.bfloat16),   # equal-share tensor-core kernel, eight heads
+    (256, 2, 4, 2, torch.bfloat16),   # streaming, head_dim 256
     (128, 4, 4, 4, torch.float32),    # fp32 CUDA-core kernel
 ])
 def test_block_id_outside_the_pool_poisons_only_its_sequence(d, G, bk, bv, qdtype):

@@ -28,7 +28,7 @@ def _test_lib():
     return lib
 
 
-@pytest.mark.parametrize("G", [4, 8])   # streaming kernel / barrier-synchronised kernel
+@pytest.mark.parametrize("G", [4, 8])   # streaming kernel / equal-share kernel
 def test_an_expired_wait_poisons_its_rows_and_nothing_else(G):
     from fused_turboquant_b200 import PagedKVPool, _lib
     bad_lib, good_lib = _test_lib(), _lib.load()

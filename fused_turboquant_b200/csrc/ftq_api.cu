@@ -360,21 +360,24 @@ ChunkPlan plan_chunks(int B, int Hq, int Hkv, int d, int max_seq_len, int n_laye
 // those), but as few as fill the chip's slots (two CTAs per SM) in whole waves.  A CTA costs about
 // three tiles besides its own: tables, queries, the fold of its warps, its rows and their merge.
 ChunkPlan plan_chunks_uniform(int B, int Hq, int Hkv, int d, int seq_len) {
-    ChunkPlan pl = plan_chunks(B, Hq, Hkv, d, round_seq(seq_len), 1);
-    const int tile = ftq::kTilePages * ftq::kPageTokens;
-    const int tiles = (seq_len + tile - 1) / tile, most = pl.n_chunks;
-    const int64_t units = static_cast<int64_t>(B) * Hkv * pl.n_hpass, slots = ftq::sm_count() * 2;
-    int64_t best = INT64_MAX;
-    for (int n = 1; n <= most && n <= tiles; n++) {
-        const int per = (tiles + n - 1) / n, real = (tiles + per - 1) / per;
-        const int64_t cost = (units * real + slots - 1) / slots * (per + 3);
-        if (cost < best) {
-            best = cost;
-            pl.n_chunks = real;
-            pl.chunk_tokens = per * tile;
+    constexpr int tile = ftq::kTilePages * ftq::kPageTokens;   // (= what round_seq rounds to)
+    const int seq = round_seq(seq_len), slots = ftq::sm_count() * 2;
+    return remembered<ChunkPlan>({1, B, Hq, Hkv, d, seq, 1, slots}, [&] {
+        ChunkPlan pl = plan_chunks(B, Hq, Hkv, d, seq, 1);
+        const int tiles = seq / tile, most = pl.n_chunks;
+        const int64_t units = static_cast<int64_t>(B) * Hkv * pl.n_hpass;
+        int64_t best = INT64_MAX;
+        for (int n = 1; n <= most && n <= tiles; n++) {
+            const int per = (tiles + n - 1) / n, real = (tiles + per - 1) / per;
+            const int64_t cost = (units * real + slots - 1) / slots * (per + 3);
+            if (cost < best) {
+                best = cost;
+                pl.n_chunks = real;
+                pl.chunk_tokens = per * tile;
+            }
         }
-    }
-    return pl;
+        return pl;
+    });
 }
 
 // Chunking of the tensor-core path (persistent CTAs): few, large chunks keep the per-item

@@ -18,6 +18,7 @@ Nothing here falls back to PyTorch or the CPU.
 from __future__ import annotations
 
 import ctypes
+import functools
 import weakref
 
 import numpy as np
@@ -76,6 +77,11 @@ def packed_dim(head_dim: int, bits: int) -> int:
 def workspace_bytes(B: int, Hq: int, Hkv: int, head_dim: int, max_seq_len: int,
                     n_layers: int = 1) -> int:
     return int(_lib.load().ftq_decode_workspace_bytes(B, Hq, Hkv, head_dim, max_seq_len, n_layers))
+
+
+@functools.lru_cache(maxsize=None)
+def sm_count(device: torch.device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 def get_workspace(device: torch.device, nbytes: int) -> torch.Tensor:

@@ -170,7 +170,7 @@ class PagedKVPool:
                 block_table.dim() == 2 and block_table.shape[0] == B and seq_lens.shape == (B,)):
             return False
         tile = 32 if D == 256 else 64
-        return q_len >= 8 or B * H * -(-int(max_seq_len) // tile) <= 12 * 148
+        return q_len >= 8 or B * H * -(-int(max_seq_len) // tile) <= 12 * kernels.sm_count(q.device)
 
     def continuation_attention(self, q: torch.Tensor, block_table: torch.Tensor,
                                seq_lens: torch.Tensor, max_seq_len: int, scale: float | None = None,

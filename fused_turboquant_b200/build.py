@@ -22,15 +22,16 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libftq_b200.so")
 # A second library for ONE test (tests/test_gpu_wait_expiry.py): the same objects, except that the
-# head_dim-128 decode unit is compiled with FTQ_TEST_WAIT_EXPIRY (one page copy of one warp is
-# never issued and the poll limit is small), so that a bounded wait runs out and the give-up path
-# (NaN rows, status word, the context stays usable) executes.  Never loaded by the package.
+# head_dim-128 decode and chunk attention units are compiled with FTQ_TEST_WAIT_EXPIRY (one page copy of
+# one warp is never issued, one tile of one warp never reported, and the poll limits are small), so that
+# a bounded wait runs out and the give-up path (NaN rows, status word, the context stays usable)
+# executes.  Never loaded by the package.
 TEST_LIB_PATH = os.path.join(PKG_DIR, "libftq_b200_waittest.so")
 # The tensor-level host path (csrc/ftq_torch.cpp): a CPython module compiled with the host compiler
 # against torch's headers; it gets the C ABI's addresses at import and links nothing of ours.
 NATIVE_PATH = os.path.join(PKG_DIR, "_native.so")
-TEST_UNIT = ("ftq_attn_inst.cu", "attn_d128_waittest",
-             ["-DFTQ_D=128", "-DFTQ_ONLY_BITS=4", "-DFTQ_TEST_WAIT_EXPIRY"])
+TEST_UNITS = [(src, f"{tag}_waittest", ["-DFTQ_D=128", "-DFTQ_ONLY_BITS=4", "-DFTQ_TEST_WAIT_EXPIRY"])
+              for src, tag in (("ftq_attn_inst.cu", "attn_d128"), ("ftq_attn_chunk_inst.cu", "attn_chunk_d128"))]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -123,7 +124,7 @@ def _older(out: str, deps) -> bool:
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile and link what is missing or older than its own sources: the library, the wait-expiry test
     library, the host path."""
-    cuda_deps = set().union(*(_deps(os.path.join(CSRC, u[0])) for u in UNITS + [TEST_UNIT]))
+    cuda_deps = set().union(*(_deps(os.path.join(CSRC, u[0])) for u in UNITS + TEST_UNITS))
     cuda_stale = force or any(_older(l, cuda_deps) for l in (LIB_PATH, TEST_LIB_PATH))
     if force or _native_stale():
         _build_native()
@@ -144,10 +145,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return obj
 
     with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
-        objs = list(ex.map(compile_one, UNITS + [TEST_UNIT]))
-    test_obj = objs.pop()
-    for lib, members in ((LIB_PATH, objs),
-                         (TEST_LIB_PATH, [test_obj if o.endswith("attn_d128.o") else o for o in objs])):
+        objs = list(ex.map(compile_one, UNITS + TEST_UNITS))
+    test_objs = {o.replace("_waittest.o", ".o"): o for o in objs[len(UNITS):]}
+    objs = objs[:len(UNITS)]
+    for lib, members in ((LIB_PATH, objs), (TEST_LIB_PATH, [test_objs.get(o, o) for o in objs])):
         _run([nvcc, "-shared", *members, "-lcudart"], lib, f"link of {lib}")
     return LIB_PATH
 

@@ -21,13 +21,20 @@ static cudaError_t run_chunk(const ChunkAttnParams& p, int B, cudaStream_t strea
     return cudaGetLastError();
 }
 
+// FTQ_ONLY_BITS=<b>: bits_k = bits_v = b only (the wait-expiry test library)
 template <int BK>
 static cudaError_t chunk_by_bv(int bv, const ChunkAttnParams& p, int B, cudaStream_t stream) {
+#ifdef FTQ_ONLY_BITS
+    if constexpr (BK == FTQ_ONLY_BITS) {
+        if (bv == BK) return run_chunk<BK, BK>(p, B, stream);
+    }
+#else
     switch (bv) {
         case 2: return run_chunk<BK, 2>(p, B, stream);
         case 3: return run_chunk<BK, 3>(p, B, stream);
         case 4: return run_chunk<BK, 4>(p, B, stream);
     }
+#endif
     return cudaErrorInvalidValue;
 }
 

@@ -151,15 +151,17 @@ constexpr int kMbarSpinLimit = 1 << 6;
 #else
 constexpr int kMbarSpinLimit = 1 << 20;
 #endif
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {   // one poll
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (int i = 0; i < kMbarSpinLimit; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-    }
+    for (int i = 0; i < kMbarSpinLimit; i++)
+        if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {

@@ -83,3 +83,47 @@ def test_an_expired_wait_poisons_its_rows_and_nothing_else(G):
     again, rc, bits = run(good_lib)       # the context is as usable as before
     assert rc == 0 and bits == 0
     np.testing.assert_array_equal(again, good)
+
+
+def test_an_expired_wait_of_the_chunk_kernel_poisons_its_rows_and_nothing_else():
+    """One dequantising warp of CTA (0, 0, 0) does not report its second tile: the CTA gives up (its MMAs
+    drained, TMEM freed), the 256 rows it works on are NaN, the rest of the call is untouched."""
+    from fused_turboquant_b200 import PagedKVPool, _lib
+    bad_lib, good_lib = _test_lib(), _lib.load()
+    d, bits, Hkv, G, B, q_len, n = 128, 4, 2, 4, 2, 100, 2000
+    per = (n + 15) // 16
+    g = torch.Generator("cuda").manual_seed(9)
+    bt = torch.randperm(B * per, device="cuda", generator=g).int().view(B, per)
+    pool = PagedKVPool(B * per, Hkv, d, bits, bits, n_layers=1, device="cuda")
+    pos = torch.arange(n, device="cuda")
+    for b in range(B):
+        kv = torch.randn(2, n, Hkv, d, device="cuda", generator=g).bfloat16()
+        pool.store(kv[0], kv[1], bt[b, pos // 16].long() * 16 + pos % 16, layer=0)
+    q = torch.randn(B, q_len, Hkv * G, d, device="cuda", generator=g).bfloat16()
+    sl = torch.full((B,), n, dtype=torch.int32, device="cuda")
+    need = good_lib.ftq_paged_chunk_workspace_bytes(B, q_len, Hkv * G, Hkv, d, n)
+    ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+
+    def run(lib):
+        out = torch.full(q.shape, 7.0, dtype=torch.float32, device="cuda")
+        rc = lib.ftq_paged_chunk_attn(
+            p(q), _lib.BF16, p(out), _lib.F32, p(pool.pool[0]), pool.num_blocks, p(bt), per, p(sl), n, B,
+            q_len, Hkv * G, Hkv, d, bits, bits, _lib.fptr(pool.levels_k), _lib.fptr(pool.levels_v),
+            _lib.fptr(pool.signs), d ** -0.5, p(ws), ws.numel(), stream)
+        assert rc == 0, lib.ftq_last_error()
+        status = ctypes.c_int(-1)
+        rc = lib.ftq_paged_decode_status(p(ws), 1, Hkv * G, Hkv, d, n, 1, stream, ctypes.byref(status))
+        return out, rc, status.value
+
+    good, rc, status = run(good_lib)
+    assert rc == 0 and status == 0 and torch.isfinite(good).all()
+    got, rc, status = run(bad_lib)
+    assert rc == -5 and status == 2, (rc, status)
+    lost = torch.zeros(B, q_len, Hkv * G, dtype=torch.bool, device="cuda")
+    lost[0, :256 // G, :G] = True                 # two row tiles: 64 queries of KV head 0's group
+    assert torch.isnan(got[lost]).all()
+    assert torch.equal(got[~lost], good[~lost])
+    again, rc, status = run(good_lib)
+    assert rc == 0 and status == 0 and torch.equal(again, good)

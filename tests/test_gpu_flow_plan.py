@@ -60,3 +60,41 @@ def test_status_of_a_batch_above_one_launch():
         assert torch.equal(out[~rows], good[~rows])
     _run(pool, q, bt, sl, top)
     assert pool.decode_status() == 0
+
+
+# (batches that leave units cut by shares' ends, units within a share, and CTAs without work)
+BIG, SMALL = [5000, 3100, 4096, 77] * 12, [900, 33]
+
+
+def test_one_uninitialised_workspace_serves_calls_of_different_shapes():
+    """The kernel clears the counters in the workspace tail itself: garbage there is harmless, and so is
+    alternating between shapes whose tails lie at different places of one buffer."""
+    runs = []
+    for lens, seed in ((BIG, 1), (SMALL, 2)):
+        pool, bt, sl, q = _batch(lens, seed)
+        runs.append((pool, q, bt, sl, max(lens)))
+    need = max(p.workspace_bytes(q.shape[0], q.shape[1], top, 1) for p, q, _, _, top in runs)
+    ws = torch.randint(0, 256, (need,), dtype=torch.uint8, device="cuda")
+    ws[-8192:] = 0xFF
+    want = [_run(*r) for r in runs]
+    assert all(torch.isfinite(w).all() for w in want)
+    for i in (0, 1, 0, 1, 1, 0):
+        assert torch.equal(_run(*runs[i], ws=ws), want[i])
+
+
+@pytest.mark.parametrize("lens", [BIG, SMALL, [60] * 1100])
+def test_replays_of_a_captured_call(lens):
+    """A captured launch carries its epoch with it (both launches of 1100 sequences the same one)."""
+    pool, bt, sl, q = _batch(lens, 4)
+    qs = [q, q.flip(0).contiguous(), -q]
+    eager = [_run(pool, x, bt, sl, max(lens)) for x in qs]
+    q_static, out = q.clone(), torch.empty(q.shape, dtype=torch.float32, device="cuda")
+    ws = torch.empty(pool.workspace_bytes(q.shape[0], q.shape[1], max(lens), 1), dtype=torch.uint8, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        pool.decode_attention(q_static, bt, sl, max(lens), layer=0, out=out, workspace=ws)
+    for i in (1, 2, 0, 2):
+        q_static.copy_(qs[i])
+        graph.replay()
+        graph.replay()          # back to back: the second replay starts from the first one's leftovers
+        assert torch.equal(out, eager[i]), f"replay with query set {i}"

@@ -22,7 +22,7 @@
 // registers one tile ahead, looked up in the lane-replicated tables, written as fp16 tiles, two
 // stages), one warp that issues the MMAs: scores of tile i are issued before P.V of tile i - 1, so that
 // softmax, dequantisation and the tensor core overlap.  What bounds it: the softmax instructions
-// (about 8 per score); the MMAs take a tenth of the time.
+// (about 8 per score); the tensor pipe is busy a sixth of the time.
 //
 // The tiles of a row tile's causal range are cut into `splits` parts (grid.x); every CTA leaves its rows
 // (O, m, l) in the workspace and attn_merge_kernel finishes.

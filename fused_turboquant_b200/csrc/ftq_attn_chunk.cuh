@@ -32,6 +32,7 @@
 // a token of such a page.
 #pragma once
 
+#include <cfloat>
 #include <climits>
 
 #include "ftq_attn_mma.cuh"
@@ -189,6 +190,7 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;     // a wait ran out
     __shared__ int s_bad_pos;   // first token on a page whose block id is out of range
+    __shared__ int s_nan_pos;   // first token whose value norm is NaN
     const volatile int* const abort_now = &s_abort;
     const uint32_t bars = sbase + C::OFF_BAR;
     const uint32_t kv_full = bars, kv_empty = bars + 16, s_full = bars + 32, s_free = bars + 48,
@@ -214,7 +216,7 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
     }
     if (tid == 0) {
         s_abort = 0;
-        s_bad_pos = INT_MAX;
+        s_bad_pos = s_nan_pos = INT_MAX;
     }
     // ---- tables: an entry (the fp16 centroids of two adjacent codes) 32 times, bank = lane
     {
@@ -299,8 +301,7 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
                 const float4* vn = kn + KT / 4;
                 float mx = -INFINITY;
                 const int left = limit - (tile0 + it) * KT;   // tokens of this tile the row attends
-                const bool all_attended = __all_sync(0xffffffffu, left >= KT);
-                if (all_attended) {
+                if (__all_sync(0xffffffffu, left >= KT)) {
 #pragma unroll
                     for (int c = 0; c < KT; c += 4) {
                         const float4 n = kn[c / 4];
@@ -354,29 +355,16 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
                 }
                 const float m_use = m_run == -INFINITY ? 0.f : m_run;   // (nothing attended so far)
                 float l0 = 0.f, l1 = 0.f;
-                // A token that the row does not attend has weight zero whatever its value norm is: an
-                // infinite or NaN norm (a vector longer than fp16 holds, a slot of a rejected draft
-                // token) belongs to the later queries only.
-                auto weights = [&](auto whole) {
 #pragma unroll
-                    for (int c = 0; c < KT; c += 4) {
-                        float4 n = vn[c / 4];
-                        if constexpr (!decltype(whole)::value) {
-                            n.x = c < left ? n.x : 0.f;
-                            n.y = c + 1 < left ? n.y : 0.f;
-                            n.z = c + 2 < left ? n.z : 0.f;
-                            n.w = c + 3 < left ? n.w : 0.f;
-                        }
-                        const float p0 = fast_exp2(__uint_as_float(sr[c]) - m_use), p1 = fast_exp2(__uint_as_float(sr[c + 1]) - m_use);
-                        const float p2 = fast_exp2(__uint_as_float(sr[c + 2]) - m_use), p3 = fast_exp2(__uint_as_float(sr[c + 3]) - m_use);
-                        l0 += p0 + p1;
-                        l1 += p2 + p3;
-                        sr[c / 2] = f2h2_sat(p0 * n.x, p1 * n.y);
-                        sr[c / 2 + 1] = f2h2_sat(p2 * n.z, p3 * n.w);
-                    }
-                };
-                if (all_attended) weights(std::true_type{});
-                else weights(std::false_type{});
+                for (int c = 0; c < KT; c += 4) {
+                    const float4 n = vn[c / 4];   // (finite; tokens that the row does not attend have p = 0)
+                    const float p0 = fast_exp2(__uint_as_float(sr[c]) - m_use), p1 = fast_exp2(__uint_as_float(sr[c + 1]) - m_use);
+                    const float p2 = fast_exp2(__uint_as_float(sr[c + 2]) - m_use), p3 = fast_exp2(__uint_as_float(sr[c + 3]) - m_use);
+                    l0 += p0 + p1;
+                    l1 += p2 + p3;
+                    sr[c / 2] = f2h2_sat(p0 * n.x, p1 * n.y);
+                    sr[c / 2 + 1] = f2h2_sat(p2 * n.z, p3 * n.w);
+                }
                 l_run += l0 + l1;
 #pragma unroll
                 for (int c = 0; c < KT / 2; c += 16) tc_st16(tm + C::COL_P + c, sr + c);
@@ -493,8 +481,18 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
             put(sbase + C::OFF_K + st * C::KV_TILE, std::integral_constant<int, BK>{}, k0, tk);
             put(sbase + C::OFF_V + st * C::KV_TILE, std::integral_constant<int, BV>{}, v0, tv);
             if (gq == 0) {
+                // The weights of a tile are multiplied by its norms whether a row attends the token or not,
+                // so what 0 * norm must not turn into NaN is kept out of them: an infinite norm becomes the
+                // largest number, whose weights saturate like its own; a NaN makes the rows that attend it
+                // NaN at the end.  (Selecting by row in the softmax warps: 221 us instead of 205 for 8 queries
+                // over 131072 tokens, 32 / 8 heads of 128.)
+                float v = vn0;
+                if (!(fabsf(v) <= 65504.f)) {
+                    if (v != v) atomicMin(&s_nan_pos, (tile0 + it) * KT + t);
+                    v = v != v ? 0.f : copysignf(FLT_MAX, v);
+                }
                 norms[st * 2 * KT + t] = kn0;
-                norms[st * 2 * KT + KT + t] = vn0;
+                norms[st * 2 * KT + KT + t] = v;
             }
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
             __syncwarp();
@@ -550,11 +548,12 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
     __syncwarp();
     __syncthreads();
     const bool expired = s_abort != 0;
-    const int bad_pos = s_bad_pos;
-    if (expired || bad_pos != INT_MAX) {
+    const int bad_pos = s_bad_pos, poison = min(bad_pos, s_nan_pos);
+    if (expired || poison != INT_MAX) {
         for (int r = row0 + tid; r < row_end; r += C::THREADS)
-            if (expired || bad_pos < min(p.max_seq, limit0 + r / group)) partial_row(r)[D] = __int_as_float(0x7fc00000);
-        if (tid == 0) atomicOr(p.status, (expired ? kStatusWaitExpired : 0) | (bad_pos != INT_MAX ? kStatusBadBlock : 0));
+            if (expired || poison < min(p.max_seq, limit0 + r / group)) partial_row(r)[D] = __int_as_float(0x7fc00000);
+        if (tid == 0 && (expired || bad_pos != INT_MAX))
+            atomicOr(p.status, (expired ? kStatusWaitExpired : 0) | (bad_pos != INT_MAX ? kStatusBadBlock : 0));
     }
     if (warp == C::SM_WARPS + C::DQ_WARPS) {
         tc_fence_after();

@@ -115,6 +115,10 @@ def test_a_later_token_without_a_finite_value_norm_is_nobody_elses(d, bk, bv, gr
     pool.store(key, torch.full_like(key, bad), slots, layer=1)
     got = pool.continuation_attention(q, table, sl, n, layer=1)
     assert torch.equal(got[:, :-2], good[:, :-2])
+    if bad != bad:
+        assert torch.isnan(got[:, -2:]).all() and pool.decode_status() == 0
+    else:
+        assert torch.isfinite(got).all() and not torch.equal(got[:, -2:], good[:, -2:])
 
 
 def test_block_id_out_of_range_concerns_the_queries_that_attend_it():

@@ -24,7 +24,7 @@
 // softmax, dequantisation and the tensor core overlap.  What bounds it: the softmax instructions
 // (about 8 per score); the tensor pipe is busy a sixth of the time.
 //
-// The tiles of a row tile's causal range are cut into `splits` parts (grid.x); every CTA leaves its rows
+// The tiles of a row tile's causal range are cut into up to `splits` parts (grid.x); every CTA leaves its rows
 // (O, m, l) in the workspace and attn_merge_kernel finishes.
 //
 // Every wait is bounded; one that runs out makes the CTA's rows NaN and sets a bit of the status word.
@@ -45,7 +45,8 @@ struct ChunkAttnParams {
     const int32_t* block_table; // [B, max_blocks]
     const int32_t* seq_lens;    // [B], the new tokens included
     int64_t num_blocks;
-    int max_blocks, max_seq, q_len, Hq, Hkv, q_dtype, splits;
+    int max_blocks, max_seq, q_len, Hq, Hkv, q_dtype;
+    int splits, splits_even;    // parts of a context: rows per query vector and grid.x; used for even lengths
     float q_scale;              // softmax scale / (key table's scale) * log2(e) / sqrt(D)
     float inv_v_scale;
     float* partials;            // [B * q_len * Hq][splits][D + 4]
@@ -171,7 +172,25 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
     const int limit0 = p.seq_lens[b] - p.q_len + 1;
     const int reach = max(0, min(p.max_seq, limit0 + (row_end - 1) / group));
     const int all_tiles = (reach + KT - 1) / KT;
-    const int per = (all_tiles + p.splits - 1) / p.splits;
+    // parts: p.splits_even when the contexts are of about one length, else p.splits, of eight tiles or more
+    // (more than half of the longest on average is "about"; the host makes both the same number where it
+    // does not matter)
+    int parts = p.splits_even, per = 0;
+    if (p.splits != p.splits_even) {   // (grid-uniform; every warp looks for itself)
+        uint32_t longest = 0, sum = 0;   // in pages
+        for (int i = lane; i < static_cast<int>(gridDim.z); i += 32) {
+            const uint32_t n = (max(0, min(p.seq_lens[i], p.max_seq)) + kPageTokens - 1) / kPageTokens;
+            longest = max(longest, n);
+            sum += n;
+        }
+        longest = __reduce_max_sync(0xffffffffu, longest);
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (2ull * sum < static_cast<unsigned long long>(longest) * gridDim.z) {
+            parts = p.splits;
+            per = 8;
+        }
+    }
+    per = max(per, (all_tiles + parts - 1) / parts);
     const int tile0 = min(split * per, all_tiles), n_tiles = min(per, all_tiles - tile0);
     auto partial_row = [&](int r) {   // r: row of the unit
         const int i = r / group;

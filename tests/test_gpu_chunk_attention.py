@@ -132,3 +132,19 @@ def test_block_id_out_of_range_concerns_the_queries_that_attend_it():
     assert pool.decode_status() == 1
     assert torch.equal(out[:, :8], good[:, :8])
     assert torch.isnan(out[:, 8:]).all()
+
+
+@pytest.mark.parametrize("lens", [[20000, 300, 64, 1], [300] * 3 + [20000], [20000, 9000, 20000, 19000], [0, 20000, 10, 0]])
+@pytest.mark.parametrize("d,hkv,group", [(128, 8, 4), (256, 4, 2)])
+def test_contexts_of_different_lengths(d, hkv, group, lens):
+    """One long context among short ones is cut into more parts than contexts of one length."""
+    pool, table, sl, gen = _pool(d, 4, 4, hkv, lens, 11)
+    q_len, top = 9, 20000
+    q = torch.randn(len(lens), q_len, hkv * group, d, device="cuda", generator=gen).half()
+    got = pool.continuation_attention(q, table, sl, top, layer=1)
+    assert pool.decode_status() == 0
+    ref = pool.continuation_attention(q.float(), table, sl, top, layer=1)
+    dead = (sl[:, None] - q_len + 1 + torch.arange(q_len, device="cuda")[None]) <= 0
+    assert (got[dead] == 0).all()
+    err = (got.float() - ref).norm(dim=-1) / ref.norm(dim=-1).clamp_min(1e-6)
+    assert err[~dead].max().item() < 5e-3     # (as in test_matches_fp32_decode)

@@ -91,6 +91,15 @@ bool table_quantizer_takes(const ftq::EncodeJob& job) {
     return true;
 }
 
+// The same for the midpoints of a slot-format store (there a code counts midpoints <= y, and 0 may be one).
+bool table_takes_midpoints(const float* m, int n) {
+    for (int j = 0; j < n; j++) {
+        if (!(m[j] > -1.0f && m[j] < 1.0f) || (m[j] != 0.f && std::fabs(m[j]) < 1e-20f)) return false;
+        if (j > 0 && ftq::quant_cell(m[j]) == ftq::quant_cell(m[j - 1])) return false;
+    }
+    return true;
+}
+
 cudaError_t dispatch_encode(int d, int dtype, ftq::EncodeJobs& jobs, int n_jobs, int n_layers,
                             cudaStream_t st) {
     // vector indices are split into (token, head) with 31-bit arithmetic in the kernels (the
@@ -1367,6 +1376,20 @@ extern "C" int ftq_tq_store_layers(const void* key, const void* value, int dtype
                       (value_lloyd_max && value_bits == 4 ? ftq::kTqLloydMaxValues : 0) |
                       (n_layers << 8);
     cudaError_t e = cudaErrorInvalidValue;
+    // Many 16-bit vectors: the kernel with two vectors per lane (from 2048 of K and V it has a warp's worth for every
+    // SM; below, its table and its long chains show).  Other widths, Lloyd-Max value codes, fp32 inputs and codebooks
+    // that the table does not take: the octet kernel.
+    const bool many = n_vec * n_layers >= 2048 && n_vec < (1ll << 31) && dtype != FTQ_F32 && !key_mse8 &&
+                      (key_fp8 || key_bits == 3 || key_bits == 4) && (value_bits == 3 || value_bits == 4) &&
+                      !(vmode & ftq::kTqLloydMaxValues) && table_takes_midpoints(p.midpoints, nmid);
+    if (many) {
+        switch (head_dim) {
+            case 64: e = ftq::launch_tq_store2_d64(kb, value_bits, dtype, p, rotate_values != 0, n_vec, n_layers, st); break;
+            case 128: e = ftq::launch_tq_store2_d128(kb, value_bits, dtype, p, rotate_values != 0, n_vec, n_layers, st); break;
+            case 256: e = ftq::launch_tq_store2_d256(kb, value_bits, dtype, p, rotate_values != 0, n_vec, n_layers, st); break;
+        }
+        return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "tq_store launch");
+    }
     switch (head_dim) {
         case 64: e = ftq::launch_tq_store_d64(kb, value_bits, dtype, p, vmode, n_vec, t8, st); break;
         case 128: e = ftq::launch_tq_store_d128(kb, value_bits, dtype, p, vmode, n_vec, t8, st); break;

@@ -10,6 +10,9 @@
 #if !defined(FTQ_TQ_PART) || FTQ_TQ_PART == 1
 #define FTQ_TQ_DECODE 1
 #endif
+#ifdef FTQ_TQ_STORE
+#include "ftq_tq_v1_store2.cuh"
+#endif
 #if FTQ_D != 256 && defined(FTQ_TQ_DECODE)
 #include "ftq_tq_v1_fp8.cuh"
 #include "ftq_tq_v1_mma.cuh"
@@ -87,6 +90,44 @@ cudaError_t FTQ_CAT(launch_tq_store_d, FTQ_D)(int kb, int vb, int dtype, const T
         case 8:   // 8-bit Lloyd-Max codes with a table, FP8 keys without
             return mid8 ? store_by_vb<8, true>(vb, dtype, p, value_mode, n_vec, *mid8, stream)
                         : store_by_vb<8>(vb, dtype, p, value_mode, n_vec, none, stream);
+    }
+    return cudaErrorInvalidValue;
+}
+
+template <int KB, int VB, typename T, bool ROTV>
+static cudaError_t store2_run(const TqStore2Params& p, int n_layers, cudaStream_t stream) {
+    constexpr int threads = tq_store2_threads(FTQ_D), smem = encode2_smem_bytes(FTQ_D, threads / 32);
+    constexpr auto kern = tq_store2_kernel<FTQ_D, KB, VB, T, ROTV>;
+    const cudaError_t e = allow_smem<kern>(smem);
+    if (e != cudaSuccess) return e;
+    // one wave of CTAs, shared among the layers
+    const int64_t want = (p.n_vec + threads / 4 - 1) / (threads / 4);
+    const int64_t wave = static_cast<int64_t>(sm_count()) * (512 / threads);
+    const int64_t cap = (wave + n_layers - 1) / n_layers;
+    kern<<<dim3(static_cast<unsigned>(want < cap ? want : cap), n_layers), threads, smem, stream>>>(p);
+    return cudaGetLastError();
+}
+template <int KB, int VB>
+static cudaError_t store2_by_type(int dtype, const TqStore2Params& p, bool rot, int n_layers, cudaStream_t s) {
+    if (dtype == kBF16)
+        return rot ? store2_run<KB, VB, __nv_bfloat16, true>(p, n_layers, s) : store2_run<KB, VB, __nv_bfloat16, false>(p, n_layers, s);
+    if (dtype == kF16) return rot ? store2_run<KB, VB, __half, true>(p, n_layers, s) : store2_run<KB, VB, __half, false>(p, n_layers, s);
+    return cudaErrorInvalidValue;
+}
+template <int KB>
+static cudaError_t store2_by_vb(int vb, int dtype, const TqStore2Params& p, bool rot, int n_layers, cudaStream_t s) {
+    return vb == 3 ? store2_by_type<KB, 3>(dtype, p, rot, n_layers, s)
+           : vb == 4 ? store2_by_type<KB, 4>(dtype, p, rot, n_layers, s) : cudaErrorInvalidValue;
+}
+cudaError_t FTQ_CAT(launch_tq_store2_d, FTQ_D)(int kb, int vb, int dtype, const TqStoreParams& sp, bool rotate_v,
+                                              int64_t n_vec, int n_layers, cudaStream_t stream) {
+    TqStore2Params p{};
+    p.s = sp;
+    p.n_vec = static_cast<uint32_t>(n_vec);
+    switch (kb) {
+        case 3: return store2_by_vb<3>(vb, dtype, p, rotate_v, n_layers, stream);
+        case 4: return store2_by_vb<4>(vb, dtype, p, rotate_v, n_layers, stream);
+        case 8: return store2_by_vb<8>(vb, dtype, p, rotate_v, n_layers, stream);
     }
     return cudaErrorInvalidValue;
 }

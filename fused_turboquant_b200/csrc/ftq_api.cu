@@ -1415,6 +1415,19 @@ extern "C" int ftq_tq_decode(const void* q, int q_dtype, int B, int Hq, int Hkv,
                                 out_dtype, lse, prefix_out, prefix_dtype, prefix_lse, 1, 0, 0, stream);
 }
 
+// Workspace of the slot-format decode: [shares | page prefix sums | two row blocks per layer and share].  Where the rows
+// of all layers would take more than 64 MiB the layers are run in several groups.
+static size_t tq_rows_offset(int B) { return (256 + (static_cast<size_t>(B) + 1) * 4 + 255) / 256 * 256; }
+static size_t tq_layer_rows(int Hq, int head_dim) { return 2 * static_cast<size_t>(ftq::sm_count()) * Hq * (head_dim + 1) * 4; }
+static int tq_layers_per_launch(int Hq, int head_dim, int n_layers) {
+    const size_t fit = (64u << 20) / tq_layer_rows(Hq, head_dim);
+    return fit < 1 ? 1 : fit < static_cast<size_t>(n_layers) ? static_cast<int>(fit) : n_layers;
+}
+extern "C" size_t ftq_tq_decode_workspace_bytes(int B, int Hq, int head_dim, int n_layers) {
+    if (B < 0 || Hq <= 0 || n_layers <= 0 || !dim_ok(head_dim)) return 0;
+    return tq_rows_offset(B) + tq_layer_rows(Hq, head_dim) * tq_layers_per_launch(Hq, head_dim, n_layers);
+}
+
 extern "C" int ftq_tq_decode_layers(const void* q, int q_dtype, int B, int Hq, int Hkv, int head_dim,
                                     const uint8_t* kv_cache, int64_t stride_block, int64_t stride_pos,
                                     int64_t stride_head, int block_size, const int32_t* block_table,
@@ -1426,6 +1439,26 @@ extern "C" int ftq_tq_decode_layers(const void* q, int q_dtype, int B, int Hq, i
                                     const void* prefix_out, int prefix_dtype, const float* prefix_lse,
                                     int n_layers, int64_t cache_layer_stride, int64_t num_blocks,
                                     void* stream) {
+    return ftq_tq_decode_layers_ws(q, q_dtype, B, Hq, Hkv, head_dim, kv_cache, stride_block, stride_pos,
+                                   stride_head, block_size, block_table, max_blocks, seq_lens, kv_start_offset,
+                                   key_bits, value_bits, norm_correction, rotate_output, value_lloyd_max,
+                                   centroids_host, scale, num_kv_splits, mid_o, out, out_dtype, lse, prefix_out,
+                                   prefix_dtype, prefix_lse, n_layers, cache_layer_stride, num_blocks, nullptr, 0,
+                                   stream);
+}
+
+
+extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq, int Hkv, int head_dim,
+                                       const uint8_t* kv_cache, int64_t stride_block, int64_t stride_pos,
+                                       int64_t stride_head, int block_size, const int32_t* block_table,
+                                       int max_blocks, const int32_t* seq_lens,
+                                       const int32_t* kv_start_offset, int key_bits, int value_bits,
+                                       int norm_correction, int rotate_output, int value_lloyd_max,
+                                       const float* centroids_host, float scale, int num_kv_splits,
+                                       float* mid_o, void* out, int out_dtype, float* lse,
+                                       const void* prefix_out, int prefix_dtype, const float* prefix_lse,
+                                       int n_layers, int64_t cache_layer_stride, int64_t num_blocks,
+                                       void* workspace, size_t workspace_bytes, void* stream) {
     if (n_layers <= 0 || !even(cache_layer_stride) || num_blocks < 0)
         return fail(FTQ_ERR_INVALID, "bad n_layers / cache_layer_stride / num_blocks");
     const int B_seq = B;
@@ -1515,11 +1548,36 @@ extern "C" int ftq_tq_decode_layers(const void* q, int q_dtype, int B, int Hq, i
     const bool fp8 = key_fp8 && q_dtype != FTQ_F32 && group <= 8 && value_bits >= 2 && value_bits <= 4 &&
                      head_dim != 256 && aligned(kv_cache, 4) && strides % 4 == 0 &&
                      static_cast<int64_t>(B) * Hkv * num_kv_splits < (1ll << 31);
-    if (fp8) {
-        const int items = B * Hkv * num_kv_splits, nh = group <= 4 ? 1 : 2;
-        e = head_dim == 64 ? ftq::launch_tq_fp8_d64(value_bits, nh, p, items, st)
-                           : ftq::launch_tq_fp8_d128(value_bits, nh, p, items, st);
-    } else if (mma) {
+    // With a workspace, and pages of 16 slots that are one aligned span of memory for all KV heads, the kernel that
+    // streams whole pages (ftq_tq_v1_flow.cuh).
+    const int64_t slot = ftq_tq_slot_bytes(head_dim, key_bits, value_bits);
+    const bool flow = mma && workspace && workspace_bytes >= ftq_tq_decode_workspace_bytes(B_seq, Hq, head_dim, n_layers) &&
+                      aligned(workspace, 16) && aligned(kv_cache, 16) && stride_block % 16 == 0 &&
+                      cache_layer_stride % 16 == 0 && block_size % 16 == 0 && stride_head >= slot &&
+                      stride_pos == Hkv * stride_head && ftq::tq_flow_fits(Hkv, stride_pos, head_dim, key_bits, value_bits, group) &&
+                      num_kv_splits <= ftq::kTqFlowSplits && B_seq <= ftq::kFlowMaxSeqs &&
+                      static_cast<int64_t>(B_seq) * (static_cast<int64_t>(max_blocks) * (block_size / 16) + num_kv_splits) < (1ll << 30) &&
+                      static_cast<int64_t>(B) * Hq < (1ll << 31);
+    ftq::TqMergeParams mp{};
+    mp.mid_o = mid_o;
+    mp.out = out;
+    mp.lse = lse;
+    mp.n_rows = static_cast<int64_t>(B) * Hq;
+    mp.splits = num_kv_splits;
+    mp.rotate = rotate_output ? 1 : 0;
+    mp.rsqrt_d = p.rsqrt_d;
+    mp.prefix_out = prefix_out;
+    mp.prefix_dtype = prefix_dtype;
+    mp.prefix_lse = prefix_lse;
+    auto merge = [&]() {
+        switch (head_dim) {
+            case 64: return ftq::launch_tq_merge_d64(out_dtype, mp, st);
+            case 128: return ftq::launch_tq_merge_d128(out_dtype, mp, st);
+            case 256: return ftq::launch_tq_merge_d256(out_dtype, mp, st);
+        }
+        return cudaErrorInvalidValue;
+    };
+    if (mma) {
         // key centroids scaled for the smallest fp16 rounding error of the table (see
         // choose_k_scale).  With norm correction the factor cancels by itself (the centroid
         // vector is re-normalised with the scaled centroids); without, it goes into the
@@ -1527,6 +1585,54 @@ extern "C" int ftq_tq_decode_layers(const void* q, int q_dtype, int B, int Hq, i
         const float ks = choose_k_scale(centroids_host, key_bits, head_dim);
         for (int i = 0; i < (1 << key_bits); i++) p.centroids.v[i] *= ks;
         if (!p.norm_correction) p.scale = scale / ks;
+    }
+    if (flow) {
+        ftq::TqFlowParams fp{};
+        fp.d = p;
+        fp.min_share = static_cast<uint32_t>(ftq::kTqFlowWarps / Hkv);
+        fp.share = static_cast<uint32_t*>(workspace);
+        fp.prefix = reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) + 256);
+        fp.rows = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + tq_rows_offset(B_seq));
+        mp.share = fp.share;
+        mp.page_prefix = fp.prefix;
+        mp.rows = fp.rows;
+        mp.seq_lens = seq_lens;
+        mp.kv_start = kv_start_offset;
+        mp.Hq = Hq;
+        mp.B_seq = p.B_seq;
+        mp.div_hq = ftq::make_fastdiv(static_cast<uint32_t>(Hq));
+        mp.div_bseq = p.div_bseq;
+        const int nh = group <= 4 ? 1 : 2, per = tq_layers_per_launch(Hq, head_dim, n_layers);
+        const int64_t layer_rows = static_cast<int64_t>(B_seq) * Hq;
+        auto size_of = [](int dtype) { return dtype == FTQ_F32 ? 4 : 2; };
+        for (int l = 0; l < n_layers; l += per) {
+            const int n = n_layers - l < per ? n_layers - l : per;
+            const int64_t row0 = l * layer_rows;
+            fp.d.B = n * B_seq;
+            fp.d.q = static_cast<const uint8_t*>(q) + row0 * head_dim * size_of(q_dtype);
+            fp.d.kv_cache = kv_cache + l * cache_layer_stride;
+            fp.d.mid_o = mid_o + row0 * num_kv_splits * (head_dim + 1);
+            e = head_dim == 64 ? ftq::launch_tq_flow_d64(key_bits, value_bits, nh, fp, st)
+                               : ftq::launch_tq_flow_d128(key_bits, value_bits, nh, fp, st);
+            if (e != cudaSuccess) return cuda_fail(e, "tq_decode stage 1 launch");
+            mp.mid_o = mp.mid_out = fp.d.mid_o;
+            mp.out = static_cast<uint8_t*>(out) + row0 * head_dim * size_of(out_dtype);
+            mp.lse = lse ? lse + row0 : nullptr;
+            mp.n_rows = n * layer_rows;
+            if (prefix_out) {
+                mp.prefix_out = static_cast<const uint8_t*>(prefix_out) + row0 * head_dim * size_of(prefix_dtype);
+                mp.prefix_lse = prefix_lse + row0;
+            }
+            e = merge();
+            if (e != cudaSuccess) return cuda_fail(e, "tq_decode merge launch");
+        }
+        return FTQ_OK;
+    }
+    if (fp8) {
+        const int items = B * Hkv * num_kv_splits, nh = group <= 4 ? 1 : 2;
+        e = head_dim == 64 ? ftq::launch_tq_fp8_d64(value_bits, nh, p, items, st)
+                           : ftq::launch_tq_fp8_d128(value_bits, nh, p, items, st);
+    } else if (mma) {
         const int64_t items = static_cast<int64_t>(B) * Hkv * num_kv_splits;
         if (items >= (1ll << 31)) return fail(FTQ_ERR_INVALID, "too many (sequence, head, split) items");
         const int nh = group <= 4 ? 1 : 2;
@@ -1542,21 +1648,6 @@ extern "C" int ftq_tq_decode_layers(const void* q, int q_dtype, int B, int Hq, i
         }
     }
     if (e != cudaSuccess) return cuda_fail(e, "tq_decode stage 1 launch");
-    ftq::TqMergeParams mp{};
-    mp.mid_o = mid_o;
-    mp.out = out;
-    mp.lse = lse;
-    mp.n_rows = static_cast<int64_t>(B) * Hq;
-    mp.splits = num_kv_splits;
-    mp.rotate = rotate_output ? 1 : 0;
-    mp.rsqrt_d = p.rsqrt_d;
-    mp.prefix_out = prefix_out;
-    mp.prefix_dtype = prefix_dtype;
-    mp.prefix_lse = prefix_lse;
-    switch (head_dim) {
-        case 64: e = ftq::launch_tq_merge_d64(out_dtype, mp, st); break;
-        case 128: e = ftq::launch_tq_merge_d128(out_dtype, mp, st); break;
-        case 256: e = ftq::launch_tq_merge_d256(out_dtype, mp, st); break;
-    }
+    e = merge();
     return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "tq_decode merge launch");
 }

@@ -24,6 +24,8 @@
 
 namespace ftq {
 
+constexpr int kFlowMaxSeqs = 1024;       // sequences per launch (their prefix sums lie in shared memory)
+
 // How the tensor-core decode kernels cut the (layer, sequence, KV head) units into work items: up
 // to three regions of consecutive units, each with its own chunk length -- few long chunks for
 // the units that fill whole waves of the grid, shorter ones for the rest, sized so that the last

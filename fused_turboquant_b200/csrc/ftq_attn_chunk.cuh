@@ -138,9 +138,6 @@ __device__ __forceinline__ void tc_wait_ld(uint32_t* r) {
                  :: "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
 
 // Shared-memory matrix descriptor, 128-byte swizzle: `lead` and `stride` in bytes (K-major: stride =
 // distance of 8-row groups; MN-major: lead = distance of 64-element chunks, stride = of 8-k groups).

@@ -57,7 +57,6 @@
 namespace ftq {
 
 constexpr float kLog2e = 1.4426950408889634f, kLn2 = 0.6931471805599453f;
-constexpr int kFlowMaxSeqs = 1024;       // sequences per launch (their prefix sums lie in shared memory)
 
 // (not volatile: a pure function of its operands, so the compiler may interleave the MMAs
 // with the table lookups of later k-blocks)
@@ -126,6 +125,9 @@ __device__ __forceinline__ void mbar_fence_init() {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes)
                  : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
 }
 // Bulk copy with an L2 policy: KV pages are read once per decode step, so L2 is told to drop
 // them first (measured on B200: +1.5 % on the Llama-shaped K4V4 batch).

@@ -51,6 +51,21 @@ inline cudaError_t allow_smem(int bytes) {
     if (r == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
     return r;
 }
+// Launches a kernel that may start its set-up while the kernel before it drains (programmatic stream serialisation).
+template <typename P>
+inline cudaError_t launch_dependent(void (*kern)(P), unsigned grid, int threads, int smem, cudaStream_t stream, const P& p) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, p);
+}
 }  // namespace
 
 }  // namespace ftq

@@ -33,7 +33,7 @@ namespace {
 #define FTQ_BOUND(X)                                                                       \
     X(ftq_encode) X(ftq_decode_dense) X(ftq_rht) X(ftq_decode_workspace_bytes)             \
     X(ftq_flash_decode) X(ftq_paged_store) X(ftq_paged_decode_attn) X(ftq_tq_store_layers) \
-    X(ftq_tq_decode_layers) X(ftq_paged_chunk_workspace_bytes) X(ftq_paged_chunk_attn)
+    X(ftq_tq_decode_layers_ws) X(ftq_tq_decode_workspace_bytes) X(ftq_paged_chunk_workspace_bytes) X(ftq_paged_chunk_attn)
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
     FTQ_BOUND(X)
@@ -646,18 +646,20 @@ PyObject* tq_decode(PyObject* const* a) {
     const bool nc = as_bool(a[8]), rot = as_bool(a[9]), lloyd = as_bool(a[10]);
     const double scale = as_double(a[11]);
     void* st = stream_of(dev);
+    const at::Tensor ws = workspace(Py_None, dev, st, api.ftq_tq_decode_workspace_bytes(B, hq, d, L));
     int rc;
     {
         NoGil nogil;
-        rc = api.ftq_tq_decode_layers(
+        rc = api.ftq_tq_decode_layers_ws(
             ptr<void>(q), dtype_code(q.scalar_type()), B, hq, c.hkv, d, ptr(c.t), c.sb, c.sp, c.sh,
             c.block_size, ptr<int32_t>(bt), bt.size(1), ptr<int32_t>(sl), ks.defined() ? ptr<int32_t>(ks) : nullptr,
             kb, vb, nc, rot, lloyd, cent.p, static_cast<float>(scale), splits, mptr<float>(mid),
             mptr<void>(out), oc, lse.defined() ? mptr<float>(lse) : nullptr,
             po.defined() ? ptr<void>(po) : nullptr, po.defined() ? dtype_code(po.scalar_type()) : 0,
-            pl.defined() ? ptr<float>(pl) : nullptr, L, c.layer_stride, c.num_blocks, st);
+            pl.defined() ? ptr<float>(pl) : nullptr, L, c.layer_stride, c.num_blocks, mptr<void>(ws),
+            ws.numel(), st);
     }
-    check(rc, "ftq_tq_decode_layers");
+    check(rc, "ftq_tq_decode_layers_ws");
     if (a[14] != Py_None) return Py_NewRef(a[14]);
     return THPVariable_Wrap(out);
 }

@@ -465,6 +465,62 @@ struct TqDecodeParams {
     float* mid_o;  // [B, Hq, splits, D + 1]
 };
 
+// Token range of split sid of a sequence, and the 16-token pages that hold it.
+struct TqRange { int t0, t1; };
+__device__ __forceinline__ TqRange tq_split_range(int seq_len, int kv_start, int splits, int sid) {
+    const int split_len = (seq_len - kv_start + splits - 1) / splits;
+    const int t0 = kv_start + split_len * sid;
+    return {t0, min(t0 + split_len, seq_len)};
+}
+__device__ __forceinline__ int tq_range_pages(const TqRange& r) {
+    return r.t1 > r.t0 ? (r.t1 + kPageTokens - 1) / kPageTokens - r.t0 / kPageTokens : 0;
+}
+
+// Stage 1 with equal shares of pages (ftq_tq_v1_flow.cuh): its shared memory.
+constexpr int kTqFlowWarps = 16;                         // warps that compute; warp 16 fetches
+// (a whole warpgroup beside them: 640 threads get 96 registers each at launch, 512 of them take 112 and the
+// fetching warpgroup's 128 keep 32)
+constexpr int kTqFlowThreads = 32 * (kTqFlowWarps + 4);
+constexpr int kTqFlowRegs = 112, kTqFetchRegs = 32;
+constexpr int kTqFlowSlots = 64;                         // pages in the ring, at most
+constexpr int kTqFlowPieces = 4;                         // pieces announced ahead
+constexpr int kTqFlowBarriers = 2 * kTqFlowSlots + 2 * kTqFlowPieces + kTqFlowWarps;
+constexpr int kTqFlowSplits = 64;                        // (a CTA looks through a sequence's splits one by one)
+constexpr int kTqFlowSmem = 226 * 1024;
+// a warp's exchange slot, which also holds its rotated queries
+__host__ __device__ constexpr int tq_flow_xslot(int d, int nh) {
+    const int out = (nh == 1 ? d / 8 : d / 4) * 128, q = 4 * nh * (d + 4) * 4;
+    return ((out > q ? out : q) + 127) / 128 * 128;
+}
+// Does the ring hold at least two pages for every warp beside the tables and the small objects?
+inline bool tq_flow_fits(int Hkv, int64_t stride_pos, int d, int kb, int vb, int group) {
+    if (Hkv > kTqFlowWarps || kTqFlowWarps % Hkv != 0) return false;
+    const int64_t pitch = (kPageTokens * stride_pos + 127) / 128 * 128;
+    const int subs = kTqFlowWarps / Hkv;
+    const int tables = (kb == 4 ? 0 : 2 * (128 << (2 * kb))) + (vb == 4 ? 0 : 2 * (128 << (2 * vb)));
+    const int small = kTqFlowBarriers * 8 + kTqFlowSlots * 8 + kTqFlowWarps * 24 * 4 + (kFlowMaxSeqs + 4) * 4 + 1024;
+    const int xarea = kTqFlowWarps * tq_flow_xslot(d, group <= 4 ? 1 : 2);
+    // (worst case over where the 64 KB window of the byte table lies: what is in front of it and what is behind it)
+    for (int base : {16, 1024, 2048, 4096}) {
+        int64_t before = kb == 4 ? 65536 - base : 0, behind = kTqFlowSmem - 16 - before - (kb == 4 ? 65536 : 0);
+        for (int need : {tables, small, xarea}) {
+            if (need <= before) before -= need;
+            else behind -= need;
+        }
+        if (behind < 0 || (before / pitch + behind / pitch) / subs < 2) return false;
+    }
+    return true;
+}
+struct TqFlowParams {
+    TqDecodeParams d;
+    uint32_t min_share;   // pages of a share, at least
+    // workspace, read by the merge kernel: pages of a share (0: a wait ran out) and shares of a layer, pages of the
+    // sequences before b over all splits, row blocks
+    uint32_t* share;      // [2]
+    int* prefix;          // [B_seq + 1]
+    float* rows;          // [layers * shares][2][Hq][D + 1]
+};
+
 constexpr int kTqTileTokens = 64;
 
 // Row stride (bytes) of a staged tile whose rows hold `bytes` of codes read in lane slices of `nb`
@@ -884,7 +940,68 @@ struct TqMergeParams {
     const void* prefix_out;   // [n_rows, D] of prefix_dtype, original space
     int prefix_dtype;
     const float* prefix_lse;  // [n_rows]
+    // Stage 1 with equal shares: units that a share's end cuts lie in the workspace (nullable)
+    const uint32_t* share;
+    const int* page_prefix;
+    const float* rows;
+    float* mid_out;           // mid_o again: the rows of cut units are written here
+    const int32_t* seq_lens;
+    const int32_t* kv_start;  // nullable
+    int Hq, B_seq;
+    FastDiv div_hq, div_bseq;
 };
+
+// What is left of a row once its partials are summed up (weights relative to M, their sum l): normalise, rotate back,
+// merge the prefix in, store.  Every octet of the row holds the sums and stores its part.
+template <int D, typename OT, int OCTETS>
+__device__ __forceinline__ void tq_finish_row(const TqMergeParams& p, int64_t row, float (&a)[D / kOctet], float l, float M,
+                                              int lane, bool store) {
+    constexpr int E = D / kOctet;
+    const int t = lane & 7, o = (lane >> 3) & (OCTETS - 1);
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll
+    for (int r = 0; r < E; r++) a[r] *= inv;
+    if (p.rotate) {
+        octet_fwht<E>(a, lane);
+#pragma unroll
+        for (int k = 0; k < E; k++) a[k] *= p.rsqrt_d;
+    }
+    float lse = l > 0.f ? M + logf(l) : -INFINITY;
+    float w_own = 1.f, w_pre = 0.f;
+    const bool prefix = p.prefix_out != nullptr;
+    if (prefix) {
+        const float lp = p.prefix_lse[row];
+        const float lmax = fmaxf(lp, lse);
+        if (lmax == -INFINITY) {  // nothing attended on either side
+            w_own = 0.f;
+        } else {
+            const float ep = __expf(lp - lmax), eq = __expf(lse - lmax);
+            const float total = fmaxf(ep + eq, 1e-20f);
+            w_pre = ep / total;
+            w_own = eq / total;
+            lse = lmax + logf(ep + eq);
+        }
+    }
+    OT* orow = static_cast<OT*>(p.out) + row * D;
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        if (!store || (r & (OCTETS - 1)) != o) continue;
+        const int coord = p.rotate ? t + 8 * r : load_coord(t, r);
+        float v = a[r];
+        if (prefix) {
+            const int64_t at = row * D + coord;
+            const float pv = p.prefix_dtype == kF32 ? static_cast<const float*>(p.prefix_out)[at]
+                             : p.prefix_dtype == kF16
+                                 ? __half2float(static_cast<const __half*>(p.prefix_out)[at])
+                                 : __bfloat162float(static_cast<const __nv_bfloat16*>(p.prefix_out)[at]);
+            v = pv * w_pre + v * w_own;
+        }
+        if constexpr (sizeof(OT) == 4) orow[coord] = v;
+        else if constexpr (std::is_same<OT, __half>::value) orow[coord] = __float2half_rn(v);
+        else orow[coord] = __float2bfloat16_rn(v);
+    }
+    if (p.lse && t == 0 && o == 0 && store) p.lse[row] = lse;
+}
 
 // Merge the split partials of a (sequence, query head) row: softmax-weighted by lse, optionally
 // Hadamard-transform the result, optionally merge a prefix result in, cast and store.  mid_o rows with
@@ -895,11 +1012,8 @@ template <int D, typename OT, int OCTETS>
 __global__ void __launch_bounds__(128)
 tq_merge_kernel(const TqMergeParams p) {
     const float* __restrict__ mid_o = p.mid_o;
-    OT* __restrict__ out = static_cast<OT*>(p.out);
-    float* __restrict__ lse_out = p.lse;
     const int64_t n_rows = p.n_rows;
-    const int splits = p.splits, rotate = p.rotate;
-    const float rsqrt_d = p.rsqrt_d;
+    const int splits = p.splits;
     constexpr int E = D / kOctet;
     const int lane = threadIdx.x & 31;
     const int t = lane & 7, o = (lane >> 3) & (OCTETS - 1);
@@ -933,49 +1047,108 @@ tq_merge_kernel(const TqMergeParams p) {
 #pragma unroll
         for (int r = 0; r < E; r++) a[r] += __shfl_xor_sync(0xffffffffu, a[r], m);
     }
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-#pragma unroll
-    for (int r = 0; r < E; r++) a[r] *= inv;
-    if (rotate) {
-        octet_fwht<E>(a, lane);
-#pragma unroll
-        for (int k = 0; k < E; k++) a[k] *= rsqrt_d;
-    }
-    float lse = l > 0.f ? M + logf(l) : -INFINITY;
-    float w_own = 1.f, w_pre = 0.f;
-    const bool prefix = p.prefix_out != nullptr;
-    if (prefix) {
-        const float lp = p.prefix_lse[row];
-        const float lmax = fmaxf(lp, lse);
-        if (lmax == -INFINITY) {  // nothing attended on either side
-            w_own = 0.f;
-        } else {
-            const float ep = __expf(lp - lmax), eq = __expf(lse - lmax);
-            const float total = fmaxf(ep + eq, 1e-20f);
-            w_pre = ep / total;
-            w_own = eq / total;
-            lse = lmax + logf(ep + eq);
-        }
-    }
-    OT* orow = out + row * D;
-#pragma unroll
-    for (int r = 0; r < E; r++) {
-        if (at >= n_rows || (r & (OCTETS - 1)) != o) continue;   // (every octet of the row holds the result and stores its part)
-        const int coord = rotate ? t + 8 * r : load_coord(t, r);
-        float v = a[r];
-        if (prefix) {
-            const int64_t at = row * D + coord;
-            const float pv = p.prefix_dtype == kF32 ? static_cast<const float*>(p.prefix_out)[at]
-                             : p.prefix_dtype == kF16
-                                 ? __half2float(static_cast<const __half*>(p.prefix_out)[at])
-                                 : __bfloat162float(static_cast<const __nv_bfloat16*>(p.prefix_out)[at]);
-            v = pv * w_pre + v * w_own;
-        }
-        if constexpr (sizeof(OT) == 4) orow[coord] = v;
-        else if constexpr (std::is_same<OT, __half>::value) orow[coord] = __float2half_rn(v);
-        else orow[coord] = __float2bfloat16_rn(v);
-    }
-    if (lse_out && t == 0 && o == 0 && at < n_rows) lse_out[row] = lse;
+    tq_finish_row<D, OT, OCTETS>(p, row, a, l, M, lane, at < n_rows);
 }
 
+// The same for stage 1 with equal shares, where a split that a share's end cut lies in the workspace in pieces: they
+// are put together, written to mid_o and merged.  Two warps per row, an octet per split: the latency of its loads bounds
+// it (an octet that went through two splits one after the other, most of them cut, took 25 us for 1024 rows).
+template <int D, typename OT>
+__global__ void __launch_bounds__(128)
+tq_join_kernel(const __grid_constant__ TqMergeParams p) {
+    constexpr int E = D / kOctet;
+    __shared__ float part[2][kOctet][E + 2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 7;
+    const int which = warp >> 1, oct = 4 * (warp & 1) + (lane >> 3);
+    const int64_t at = static_cast<int64_t>(blockIdx.x) * 2 + which;
+    const int64_t row = at < p.n_rows ? at : p.n_rows - 1;
+    const uint32_t r = fast_div(static_cast<uint32_t>(row), p.div_hq);   // (layer, sequence)
+    const int h = static_cast<int>(static_cast<uint32_t>(row) - r * p.Hq);
+    const uint32_t layer = fast_div(r, p.div_bseq);
+    const int b = static_cast<int>(r - layer * p.B_seq);
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");   // stage 1 is complete
+    const uint32_t share = p.share[0];
+    const int64_t shares0 = static_cast<int64_t>(layer) * p.share[1];
+    const int len = p.seq_lens[b], start = p.kv_start ? p.kv_start[b] : 0;
+    uint32_t pos = static_cast<uint32_t>(p.page_prefix[b]);
+    float M = -INFINITY, l = 0.f, a[E];
+#pragma unroll
+    for (int i = 0; i < E; i++) a[i] = 0.f;
+    for (int s = 0; s < p.splits; s++) {
+        const uint32_t n = tq_range_pages(tq_split_range(len, start, p.splits, s));
+        if ((s & 7) == oct && n > 0 && share > 0) {
+            const uint32_t c0 = pos / share, c1 = (pos + n - 1) / share;
+            float* mid = p.mid_out + (row * p.splits + s) * (D + 1);
+            // (row block 0 is the piece the share starts with, 1 its last one)
+            auto piece = [&](uint32_t c) {
+                return c0 == c1 ? mid : p.rows + ((2 * (shares0 + c) + (c * share >= pos ? 0 : 1)) * p.Hq + h) * (D + 1);
+            };
+            float x[E], ms = -INFINITY, ls = 0.f;
+#pragma unroll
+            for (int i = 0; i < E; i++) x[i] = 0.f;
+            for (uint32_t c = c0; c <= c1; c++) {
+                const float* src = piece(c);
+                const float lse = __ldcg(src + D);
+                float y[E];
+#pragma unroll
+                for (int i = 0; i < E; i++) y[i] = __ldcg(src + load_coord(t, i));
+                const float m_new = fmaxf(ms, lse);
+                const float f0 = __expf(ms - m_new), f = __expf(lse - m_new);   // (a NaN stays one)
+                ls = fmaf(ls, f0, f);
+#pragma unroll
+                for (int i = 0; i < E; i++) x[i] = fmaf(x[i], f0, y[i] * f);
+                ms = m_new;
+            }
+            if (c0 != c1) {
+                const float inv = 1.f / ls;
+                const float lse = ms + logf(ls);
+#pragma unroll
+                for (int i = 0; i < E; i++) {
+                    x[i] *= inv;
+                    mid[load_coord(t, i)] = x[i];
+                }
+                if (t == 0) mid[D] = lse;
+                ms = lse;
+            }
+            const float m_new = fmaxf(M, ms);
+            const float f0 = __expf(M - m_new), f = c0 == c1 ? ls * __expf(ms - m_new) : __expf(ms - m_new);
+            l = fmaf(l, f0, f);
+#pragma unroll
+            for (int i = 0; i < E; i++) a[i] = fmaf(a[i], f0, x[i] * f);
+            M = m_new;
+        }
+        pos += n;
+    }
+    if (share == 0) {
+        l = __int_as_float(0x7fc00000);
+#pragma unroll
+        for (int i = 0; i < E; i++) a[i] = l;
+    }
+    // the octets of a warp, then the two warps
+    auto join = [&](float m_o, float l_o, auto other) {
+        const float m_new = fmaxf(M, m_o);
+        const float f0 = M == -INFINITY && l == 0.f ? 0.f : __expf(M - m_new);
+        const float f1 = m_o == -INFINITY && l_o == 0.f ? 0.f : __expf(m_o - m_new);
+        l = l * f0 + l_o * f1;
+#pragma unroll
+        for (int i = 0; i < E; i++) a[i] = a[i] * f0 + other(i) * f1;
+        M = m_new;
+    };
+#pragma unroll
+    for (int m = 8; m < 32; m <<= 1) {
+        const float m_o = __shfl_xor_sync(0xffffffffu, M, m), l_o = __shfl_xor_sync(0xffffffffu, l, m);
+        join(m_o, l_o, [&](int i) { return __shfl_xor_sync(0xffffffffu, a[i], m); });
+    }
+    if ((warp & 1) && lane < kOctet) {
+#pragma unroll
+        for (int i = 0; i < E; i++) part[which][t][i] = a[i];
+        part[which][t][E] = M;
+        part[which][t][E + 1] = l;
+    }
+    __syncthreads();
+    if (warp & 1) return;
+    join(part[which][t][E], part[which][t][E + 1], [&](int i) { return part[which][t][i]; });
+    tq_finish_row<D, OT, 4>(p, row, a, l, M, lane, at < p.n_rows);
+}
 }  // namespace ftq

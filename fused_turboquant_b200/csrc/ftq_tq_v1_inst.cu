@@ -14,6 +14,7 @@
 #include "ftq_tq_v1_store2.cuh"
 #endif
 #if FTQ_D != 256 && defined(FTQ_TQ_DECODE)
+#include "ftq_tq_v1_flow.cuh"
 #include "ftq_tq_v1_fp8.cuh"
 #include "ftq_tq_v1_mma.cuh"
 #endif
@@ -242,12 +243,50 @@ cudaError_t FTQ_CAT(launch_tq_mma_d, FTQ_D)(int kb, int vb, int nh, const TqDeco
     return cudaErrorInvalidValue;
 }
 
+template <int KB, int VB, int NH>
+static cudaError_t flow_run(const TqFlowParams& p, cudaStream_t stream) {
+#if FTQ_D != 256
+    constexpr auto kern = tq_flow_kernel<TqCodes<FTQ_D, KB, VB, NH>>;
+    const cudaError_t e = allow_smem<kern>(kTqFlowSmem);
+    if (e != cudaSuccess) return e;
+    // (its set-up, 64 KB of tables, overlaps the tail of the kernel before it)
+    return launch_dependent(kern, static_cast<unsigned>(sm_count()), kTqFlowThreads, kTqFlowSmem, stream, p);
+#else
+    return cudaErrorInvalidValue;
+#endif
+}
+template <int KB, int VB>
+static cudaError_t flow_by_nh(int nh, const TqFlowParams& p, cudaStream_t s) {
+    return nh == 1 ? flow_run<KB, VB, 1>(p, s) : flow_run<KB, VB, 2>(p, s);
+}
+template <int KB>
+static cudaError_t flow_by_vb(int vb, int nh, const TqFlowParams& p, cudaStream_t s) {
+    switch (vb) {
+        case 2: return flow_by_nh<KB, 2>(nh, p, s);
+        case 3: return flow_by_nh<KB, 3>(nh, p, s);
+        case 4: return flow_by_nh<KB, 4>(nh, p, s);
+    }
+    return cudaErrorInvalidValue;
+}
+cudaError_t FTQ_CAT(launch_tq_flow_d, FTQ_D)(int kb, int vb, int nh, const TqFlowParams& p, cudaStream_t stream) {
+    switch (kb) {
+        case 2: return flow_by_vb<2>(vb, nh, p, stream);
+        case 3: return flow_by_vb<3>(vb, nh, p, stream);
+        case 4: return flow_by_vb<4>(vb, nh, p, stream);
+    }
+    return cudaErrorInvalidValue;
+}
+
 template <typename OT>
 static cudaError_t run_tq_merge(const TqMergeParams& p, cudaStream_t stream) {
     // (as in the page-layout merge: a warp per row where there are few of them)
     if (p.n_rows <= 0) return cudaSuccess;
     const int octets = p.n_rows <= kWideMerge * sm_count() ? 4 : 1;
     const unsigned grid = static_cast<unsigned>((p.n_rows * octets + 15) / 16);
+    if (p.share) {
+        // (launched while stage 1 drains: it waits for stage 1's end itself)
+        return launch_dependent(tq_join_kernel<FTQ_D, OT>, static_cast<unsigned>((p.n_rows + 1) / 2), 128, 0, stream, p);
+    }
     if (octets == 4) tq_merge_kernel<FTQ_D, OT, 4><<<grid, 128, 0, stream>>>(p);
     else tq_merge_kernel<FTQ_D, OT, 1><<<grid, 128, 0, stream>>>(p);
     return cudaGetLastError();

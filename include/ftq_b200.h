@@ -415,6 +415,25 @@ int ftq_tq_decode_layers(const void *q, int q_dtype, int B, int Hq, int Hkv, int
                          int n_layers, int64_t cache_layer_stride, int64_t num_blocks,
                          void *stream);
 
+/*
+ * ftq_tq_decode_layers with scratch for stage 1: with it, batches of 16-bit queries over a
+ * [block, position, head, slot] cache whose blocks start on 16-byte boundaries are cut into equal
+ * shares of pages instead of (sequence, head, split) items.  Same results in mid_o and out.  The
+ * workspace (16-byte aligned, ftq_tq_decode_workspace_bytes(B, Hq, head_dim, n_layers) bytes, no initialisation)
+ * belongs to the call until it has run; NULL or a smaller one: ftq_tq_decode_layers.
+ */
+size_t ftq_tq_decode_workspace_bytes(int B, int Hq, int head_dim, int n_layers);
+int ftq_tq_decode_layers_ws(const void *q, int q_dtype, int B, int Hq, int Hkv, int head_dim,
+                            const uint8_t *kv_cache, int64_t stride_block, int64_t stride_pos,
+                            int64_t stride_head, int block_size, const int32_t *block_table,
+                            int max_blocks, const int32_t *seq_lens, const int32_t *kv_start_offset,
+                            int key_bits, int value_bits, int norm_correction, int rotate_output,
+                            int value_lloyd_max, const float *centroids_host, float scale,
+                            int num_kv_splits, float *mid_o, void *out, int out_dtype, float *lse,
+                            const void *prefix_out, int prefix_dtype, const float *prefix_lse,
+                            int n_layers, int64_t cache_layer_stride, int64_t num_blocks,
+                            void *workspace, size_t workspace_bytes, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1551,7 +1551,7 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
     // With a workspace, and pages of 16 slots that are one aligned span of memory for all KV heads, the kernel that
     // streams whole pages (ftq_tq_v1_flow.cuh).
     const int64_t slot = ftq_tq_slot_bytes(head_dim, key_bits, value_bits);
-    const bool flow = mma && workspace && workspace_bytes >= ftq_tq_decode_workspace_bytes(B_seq, Hq, head_dim, n_layers) &&
+    const bool flow = (mma || fp8) && workspace && workspace_bytes >= ftq_tq_decode_workspace_bytes(B_seq, Hq, head_dim, n_layers) &&
                       aligned(workspace, 16) && aligned(kv_cache, 16) && stride_block % 16 == 0 &&
                       cache_layer_stride % 16 == 0 && block_size % 16 == 0 && stride_head >= slot &&
                       stride_pos == Hkv * stride_head && ftq::tq_flow_fits(Hkv, stride_pos, head_dim, key_bits, value_bits, group) &&

@@ -497,7 +497,7 @@ inline bool tq_flow_fits(int Hkv, int64_t stride_pos, int d, int kb, int vb, int
     if (Hkv > kTqFlowWarps || kTqFlowWarps % Hkv != 0) return false;
     const int64_t pitch = (kPageTokens * stride_pos + 127) / 128 * 128;
     const int subs = kTqFlowWarps / Hkv;
-    const int tables = (kb == 4 ? 0 : 2 * (128 << (2 * kb))) + (vb == 4 ? 0 : 2 * (128 << (2 * vb)));
+    const int tables = kb == 8 ? 0 : (kb == 4 ? 0 : 2 * (128 << (2 * kb))) + (vb == 4 ? 0 : 2 * (128 << (2 * vb)));
     const int small = kTqFlowBarriers * 8 + kTqFlowSlots * 8 + kTqFlowWarps * 24 * 4 + (kFlowMaxSeqs + 4) * 4 + 1024;
     const int xarea = kTqFlowWarps * tq_flow_xslot(d, group <= 4 ? 1 : 2);
     // (worst case over where the 64 KB window of the byte table lies: what is in front of it and what is behind it)

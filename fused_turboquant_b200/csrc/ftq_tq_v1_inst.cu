@@ -243,21 +243,23 @@ cudaError_t FTQ_CAT(launch_tq_mma_d, FTQ_D)(int kb, int vb, int nh, const TqDeco
     return cudaErrorInvalidValue;
 }
 
-template <int KB, int VB, int NH>
-static cudaError_t flow_run(const TqFlowParams& p, cudaStream_t stream) {
 #if FTQ_D != 256
-    constexpr auto kern = tq_flow_kernel<TqCodes<FTQ_D, KB, VB, NH>>;
+template <class Engine>
+static cudaError_t flow_run(const TqFlowParams& p, cudaStream_t stream) {
+    constexpr auto kern = tq_flow_kernel<Engine>;
     const cudaError_t e = allow_smem<kern>(kTqFlowSmem);
     if (e != cudaSuccess) return e;
     // (its set-up, 64 KB of tables, overlaps the tail of the kernel before it)
     return launch_dependent(kern, static_cast<unsigned>(sm_count()), kTqFlowThreads, kTqFlowSmem, stream, p);
-#else
-    return cudaErrorInvalidValue;
-#endif
+}
+template <int KB, int VB, int NH>
+static cudaError_t flow_engine(const TqFlowParams& p, cudaStream_t s) {
+    if constexpr (KB == 8) return flow_run<TqFp8<FTQ_D, VB, NH, false>>(p, s);
+    else return flow_run<TqCodes<FTQ_D, KB, VB, NH>>(p, s);
 }
 template <int KB, int VB>
 static cudaError_t flow_by_nh(int nh, const TqFlowParams& p, cudaStream_t s) {
-    return nh == 1 ? flow_run<KB, VB, 1>(p, s) : flow_run<KB, VB, 2>(p, s);
+    return nh == 1 ? flow_engine<KB, VB, 1>(p, s) : flow_engine<KB, VB, 2>(p, s);
 }
 template <int KB>
 static cudaError_t flow_by_vb(int vb, int nh, const TqFlowParams& p, cudaStream_t s) {
@@ -268,12 +270,16 @@ static cudaError_t flow_by_vb(int vb, int nh, const TqFlowParams& p, cudaStream_
     }
     return cudaErrorInvalidValue;
 }
+#endif
 cudaError_t FTQ_CAT(launch_tq_flow_d, FTQ_D)(int kb, int vb, int nh, const TqFlowParams& p, cudaStream_t stream) {
+#if FTQ_D != 256
     switch (kb) {
         case 2: return flow_by_vb<2>(vb, nh, p, stream);
         case 3: return flow_by_vb<3>(vb, nh, p, stream);
         case 4: return flow_by_vb<4>(vb, nh, p, stream);
+        case 8: return flow_by_vb<8>(vb, nh, p, stream);   // FP8 keys
     }
+#endif
     return cudaErrorInvalidValue;
 }
 

@@ -509,18 +509,19 @@ cudaError_t dispatch_mma(int d, int bk, int bv, bool shared_lut, const ftq::Attn
 
 cudaError_t dispatch_merge(int d, int out_dtype, const float* partials, void* out,
                            const int32_t* seq_lens, int S, int B, int Hq, int n_chunks, int chunk_tokens,
-                           int64_t n_vec, const ftq::SignBits& signs, cudaStream_t st) {
+                           int64_t n_vec, const ftq::SignBits& signs, cudaStream_t st,
+                           const ftq::MergeStatus& status = {}) {
     const float r = rsqrt_dim(d);
     switch (d) {
         case 64:
             return ftq::launch_attn_merge_d64(out_dtype, partials, out, seq_lens, S, B, Hq, n_chunks,
-                                              chunk_tokens, n_vec, signs, r, st);
+                                              chunk_tokens, n_vec, signs, r, status, st);
         case 128:
             return ftq::launch_attn_merge_d128(out_dtype, partials, out, seq_lens, S, B, Hq, n_chunks,
-                                               chunk_tokens, n_vec, signs, r, st);
+                                               chunk_tokens, n_vec, signs, r, status, st);
         case 256:
             return ftq::launch_attn_merge_d256(out_dtype, partials, out, seq_lens, S, B, Hq, n_chunks,
-                                               chunk_tokens, n_vec, signs, r, st);
+                                               chunk_tokens, n_vec, signs, r, status, st);
     }
     return cudaErrorInvalidValue;
 }
@@ -648,13 +649,13 @@ int ftq_decode_dense(const uint8_t* packed, const void* norms, int norms_dtype, 
     const float r = rsqrt_dim(head_dim);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const unsigned grid = grid_for(n_vec, 32);
+    cudaError_t e = cudaErrorInvalidValue;
 #define FTQ_DD(DD, BB)                                                                          \
-    if (norms_dtype == FTQ_F16)                                                                 \
-        ftq::decode_dense_kernel<DD, BB, __half><<<grid, 256, 0, st>>>(                          \
-            packed, static_cast<const __half*>(norms), out, lv, sg, r, n_vec);                  \
-    else                                                                                        \
-        ftq::decode_dense_kernel<DD, BB, float><<<grid, 256, 0, st>>>(                           \
-            packed, static_cast<const float*>(norms), out, lv, sg, r, n_vec);
+    e = norms_dtype == FTQ_F16                                                                  \
+        ? ftq::launch_dependent(ftq::decode_dense_kernel<DD, BB, __half>, dim3(grid), 256, 0, st, packed, \
+                                static_cast<const __half*>(norms), out, lv, sg, r, n_vec)       \
+        : ftq::launch_dependent(ftq::decode_dense_kernel<DD, BB, float>, dim3(grid), 256, 0, st, packed, \
+                                static_cast<const float*>(norms), out, lv, sg, r, n_vec);
 #define FTQ_DB(DD)                                                                              \
     switch (bits) {                                                                             \
         case 2: FTQ_DD(DD, 2) break;                                                            \
@@ -668,7 +669,6 @@ int ftq_decode_dense(const uint8_t* packed, const void* norms, int norms_dtype, 
     }
 #undef FTQ_DB
 #undef FTQ_DD
-    cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_decode_dense launch");
 }
 
@@ -1246,11 +1246,13 @@ extern "C" int ftq_paged_chunk_attn(const void* q, int q_dtype, void* out, int o
     // finds the status word; the rows follow
     uint8_t* const ws = static_cast<uint8_t*>(workspace);
     const size_t head = ftq_decode_workspace_bytes(1, Hq, Hkv, head_dim, max_seq_len, 1);
-    p.status = reinterpret_cast<int*>(ws + head - counter_bytes(1, Hkv, 1)) + ftq::kStatusWord;
+    int* const counters = reinterpret_cast<int*>(ws + head - counter_bytes(1, Hkv, 1));
+    const ftq::MergeStatus status{counters + ftq::kStatusWord, reinterpret_cast<unsigned long long*>(counters + 8), next_epoch()};
+    p.errors = status.errors;
+    p.epoch = status.epoch;
     p.partials = reinterpret_cast<float*>(ws + (head + 255) / 256 * 256);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    cudaError_t e = cudaMemsetAsync(p.status, 0, sizeof(int), st);
-    if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_chunk_attn status reset");
+    cudaError_t e;
     switch (head_dim) {
         case 64: e = ftq::launch_attn_chunk_d64(bits_k, bits_v, p, B, st); break;
         case 128: e = ftq::launch_attn_chunk_d128(bits_k, bits_v, p, B, st); break;
@@ -1258,7 +1260,7 @@ extern "C" int ftq_paged_chunk_attn(const void* q, int q_dtype, void* out, int o
     }
     if (e != cudaSuccess) return cuda_fail(e, "ftq_paged_chunk_attn launch");
     e = dispatch_merge(head_dim, out_dtype, p.partials, out, nullptr, p.splits, B, Hq, p.splits, 1,
-                       static_cast<int64_t>(B) * q_len * Hq, p.signs, st);
+                       static_cast<int64_t>(B) * q_len * Hq, p.signs, st, status);
     return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_paged_chunk_attn merge launch");
 }
 

@@ -505,15 +505,26 @@ attn_split_kernel(const AttnParams p) {
 // chunk's row, and their sums are added up with shuffles.  What bounds it is the latency of the
 // rows' loads, so the loop has nothing that keeps the next row's loads from being issued.  (An octet
 // per vector with a branch per row took 23 us of the 65 us of a call with 128 vectors of 32 chunks.)
+// `st` (optional): the error words of the kernel before (their epoch: unique per launch) become the call's status word.
+struct MergeStatus {
+    int* status;
+    unsigned long long* errors;   // [2]: expired waits, bad block ids
+    unsigned long long epoch;
+};
 template <int D, typename OT, int OCTETS>
 __global__ void __launch_bounds__(128)
 attn_merge_kernel(const float* __restrict__ partials, OT* __restrict__ out,
                   const int32_t* __restrict__ seq_lens, int S, int B, int Hq, int n_chunks,
-                  int chunk_tokens, int64_t n_vec, SignBits signs, float rsqrt_d) {
+                  int chunk_tokens, int64_t n_vec, SignBits signs, float rsqrt_d, MergeStatus st) {
     constexpr int E = D / kOctet;
     constexpr int ROW = D + 4;
     const int lane = threadIdx.x & 31;
     const int t = lane & 7, o = (lane >> 3) & (OCTETS - 1);
+    after_previous_kernel();   // the rows are complete
+    if (st.status && blockIdx.x == 0 && threadIdx.x == 0) {
+        *st.status = (__ldcg(st.errors) == st.epoch ? kStatusWaitExpired : 0) | (__ldcg(st.errors + 1) == st.epoch ? kStatusBadBlock : 0);
+        st.errors[0] = st.errors[1] = 0ull;   // (a replayed launch has the same epoch)
+    }
     const int64_t at = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / (8 * OCTETS);
     const int64_t v = at < n_vec ? at : n_vec - 1;   // (octets left over repeat the last vector)
     const int b = static_cast<int>((v / Hq) % B);

@@ -50,7 +50,10 @@ struct ChunkAttnParams {
     float q_scale;              // softmax scale / (key table's scale) * log2(e) / sqrt(D)
     float inv_v_scale;
     float* partials;            // [B * q_len * Hq][splits][D + 4]
-    int* status;
+    // what went wrong (expired waits, bad block ids): a word holds `epoch` if it did; the merge kernel turns them into the
+    // call's status word
+    unsigned long long* errors;
+    unsigned long long epoch;
     Codebook lk, lv;            // scaled for their fp16 rounding
     SignBits signs;
 };
@@ -568,8 +571,8 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
     if (expired || poison != INT_MAX) {
         for (int r = row0 + tid; r < row_end; r += C::THREADS)
             if (expired || poison < min(p.max_seq, limit0 + r / group)) partial_row(r)[D] = __int_as_float(0x7fc00000);
-        if (tid == 0 && (expired || bad_pos != INT_MAX))
-            atomicOr(p.status, (expired ? kStatusWaitExpired : 0) | (bad_pos != INT_MAX ? kStatusBadBlock : 0));
+        if (tid == 0 && expired) __stcg(p.errors, p.epoch);
+        if (tid == 0 && bad_pos != INT_MAX) __stcg(p.errors + 1, p.epoch);
     }
     if (warp == C::SM_WARPS + C::DQ_WARPS) {
         tc_fence_after();

@@ -96,7 +96,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     };
 
     // the next kernel of the stream may start its own set-up as soon as every CTA got here
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    let_next_kernel_start();
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, tg = lane & 3;
@@ -172,7 +172,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
 
     // Everything up to here touched shared memory only.  From here on the kernel reads and writes
     // global memory that the kernel before it in the stream may still be using.
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    after_previous_kernel();
     unsigned long long* epoch_word = reinterpret_cast<unsigned long long*>(p.work_counter + 2);
     if (blockIdx.x == 0) {
         for (int i = tid; i < p.n_units; i += THREADS) p.unit_counter[i] = 0;

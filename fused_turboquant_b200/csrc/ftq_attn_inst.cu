@@ -207,35 +207,32 @@ int FTQ_CAT(attn_mma_stream_ctas_d, FTQ_D)(int bits_k, int bits_v, int group) {
 template <typename OT>
 static cudaError_t run_merge(const float* partials, void* out, const int32_t* seq_lens, int S, int B, int Hq,
                              int n_chunks, int chunk_tokens, int64_t n_vec, const SignBits& signs,
-                             float rsqrt_d, cudaStream_t stream) {
+                             float rsqrt_d, const MergeStatus& status, cudaStream_t stream) {
     // a warp per vector where there are few of them (kWideMerge), an octet where they fill the chip as
     // it is: 128 vectors of 32 chunks 23 -> 4 us with four octets, 8192 vectors of 4 chunks 6 -> 10 us
     const int octets = n_vec <= kWideMerge * sm_count() ? 4 : 1;
     const unsigned grid = static_cast<unsigned>((n_vec * octets + 15) / 16);
     if (n_vec <= 0) return cudaSuccess;
-    if (octets == 4)
-        attn_merge_kernel<FTQ_D, OT, 4><<<grid, 128, 0, stream>>>(
-            partials, static_cast<OT*>(out), seq_lens, S, B, Hq, n_chunks, chunk_tokens, n_vec, signs, rsqrt_d);
-    else
-        attn_merge_kernel<FTQ_D, OT, 1><<<grid, 128, 0, stream>>>(
-            partials, static_cast<OT*>(out), seq_lens, S, B, Hq, n_chunks, chunk_tokens, n_vec, signs, rsqrt_d);
-    return cudaGetLastError();
+    // (launched while the kernel before drains: it waits for that one's end itself)
+    return launch_dependent(octets == 4 ? attn_merge_kernel<FTQ_D, OT, 4> : attn_merge_kernel<FTQ_D, OT, 1>, grid, 128, 0, stream,
+                            partials, static_cast<OT*>(out), seq_lens, S, B, Hq, n_chunks, chunk_tokens, n_vec, signs, rsqrt_d, status);
 }
 
 cudaError_t FTQ_CAT(launch_attn_merge_d, FTQ_D)(int out_dtype, const float* partials, void* out,
                                                 const int32_t* seq_lens, int S, int B, int Hq,
                                                 int n_chunks, int chunk_tokens, int64_t n_vec,
-                                                const SignBits& signs, float rsqrt_d, cudaStream_t stream) {
+                                                const SignBits& signs, float rsqrt_d, const MergeStatus& status,
+                                                cudaStream_t stream) {
     switch (out_dtype) {
         case kF32:
             return run_merge<float>(partials, out, seq_lens, S, B, Hq, n_chunks, chunk_tokens, n_vec, signs,
-                                    rsqrt_d, stream);
+                                    rsqrt_d, status, stream);
         case kF16:
             return run_merge<__half>(partials, out, seq_lens, S, B, Hq, n_chunks, chunk_tokens, n_vec, signs,
-                                     rsqrt_d, stream);
+                                     rsqrt_d, status, stream);
         case kBF16:
             return run_merge<__nv_bfloat16>(partials, out, seq_lens, S, B, Hq, n_chunks, chunk_tokens, n_vec,
-                                            signs, rsqrt_d, stream);
+                                            signs, rsqrt_d, status, stream);
     }
     return cudaErrorInvalidValue;
 }

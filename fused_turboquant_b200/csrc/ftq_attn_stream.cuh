@@ -239,7 +239,7 @@ attn_stream_kernel(const AttnParams p, int n_items) {
     auto gptr = [&](uint32_t saddr) { return smem_raw + (saddr - sbase); };
 
     // the next kernel of the stream may start its own set-up as soon as every CTA got here
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    let_next_kernel_start();
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -327,7 +327,7 @@ attn_stream_kernel(const AttnParams p, int n_items) {
                   : ((BV == 4 ? (window | (SHARED_LUT ? 0u : 128u)) : tv_small) | (lane * 4));
     // Everything up to here touched shared memory only.  From here on the kernel reads and writes
     // global memory that the kernel before it in the stream may still be using (the workspace).
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    after_previous_kernel();
     unsigned long long* epoch_word = reinterpret_cast<unsigned long long*>(p.work_counter + 2);
     if (blockIdx.x == 0) {
         for (int i = tid; i < p.n_units; i += THREADS) p.unit_counter[i] = 0;

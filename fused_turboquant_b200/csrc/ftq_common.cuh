@@ -36,6 +36,13 @@ enum : int { kF32 = 0, kF16 = 1, kBF16 = 2 };
 
 __host__ __device__ constexpr int packed_dim(int d, int bits) { return d * bits / 8; }
 
+// ---------------------------------------------------------------- order of kernels in a stream
+// A kernel launched with programmatic stream serialisation starts while the one before drains; it touches global memory
+// after after_previous_kernel() only.  Every such kernel waits, so that what came before the previous one is complete too.
+// let_next_kernel_start(): that kernel's set-up may begin (its CTAs take the place of those that leave).
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // ---------------------------------------------------------------- tables
 
 // Small per-call tables, passed by value as kernel parameters (they live in

@@ -78,6 +78,8 @@ decode_dense_kernel(const uint8_t* __restrict__ packed, const NormT* __restrict_
     __shared__ float lut[kMaxLevels];
     if (threadIdx.x < kMaxLevels) lut[threadIdx.x] = levels.v[threadIdx.x];
     __syncthreads();
+    let_next_kernel_start();
+    after_previous_kernel();
 
     const int lane = threadIdx.x & 31;
     const int t = lane & 7;

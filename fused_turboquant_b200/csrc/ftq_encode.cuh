@@ -332,6 +332,8 @@ __device__ __forceinline__ void encode_body(const EncodeJobs& jobs, const Encode
 
 template <int D, typename T>
 __global__ void __launch_bounds__(256) encode_kernel(const __grid_constant__ EncodeJobs jobs) {
+    let_next_kernel_start();   // (a decode step's attention builds its tables meanwhile)
+    after_previous_kernel();
     const EncodeJob& job = jobs.job[blockIdx.z];
     switch (job.bits) {
         case 2: encode_body<D, 2, T>(jobs, job); break;
@@ -415,6 +417,8 @@ __device__ __forceinline__ void encode_octet_job(const EncodeJobs& jobs, const E
 
 template <int D, typename T>
 __global__ void __launch_bounds__(256) encode_octet_kernel(const __grid_constant__ EncodeJobs jobs) {
+    let_next_kernel_start();
+    after_previous_kernel();
     // (a body per job: its boundaries are constant operands)
     if (blockIdx.z == 0) encode_octet_job<D, T>(jobs, jobs.job[0]);
     else encode_octet_job<D, T>(jobs, jobs.job[1]);

@@ -176,6 +176,7 @@ __device__ __forceinline__ void encode2_body(const EncodeJobs& jobs, const Encod
         for (int i = 0; i < 16; i++) lut[c][(i + c) & 15] = make_float2(thr, base);
     }
     __syncthreads();
+    after_previous_kernel();
     const uint32_t lut_col = (lane & 15) * 8;
     float* slot = tbuf + (wip * 4 + sub) * SLOT;
 
@@ -404,6 +405,7 @@ encode2_kernel(const __grid_constant__ EncodeJobs jobs) {
     __shared__ __align__(128) QuantTable lut;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     float* tbuf = reinterpret_cast<float*>(smem_raw);                  // [warps][4][SLOT]
+    let_next_kernel_start();
     // A body per job: the fields of a job that is known at compile time are operands in the constant
     // bank, those of jobs.job[blockIdx.z] took registers and instructions inside the loop (524288 tokens,
     // K and V of 8 heads of 128: 1390 us, 1330 us so).

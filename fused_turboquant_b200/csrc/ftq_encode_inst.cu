@@ -25,24 +25,20 @@ static cudaError_t run(EncodeJobs jobs, int n_jobs, Encode kind, int n_layers, c
         const int64_t cap = static_cast<int64_t>(sm_count()) * (512 / threads) / n_jobs;
         const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), 1, n_jobs);
         jobs.n_layers = n_layers;
-        if (n_layers > 1) many<<<grid, threads, smem, stream>>>(jobs);
-        else one<<<grid, threads, smem, stream>>>(jobs);
-        return cudaGetLastError();
+        return launch_dependent(n_layers > 1 ? many : one, grid, threads, smem, stream, jobs);
     }
     if (kind == Encode::kAnyCodebook) {
         constexpr int threads = 256;                   // 8 warps, four vectors each
         const int64_t want = (n + threads / 8 - 1) / (threads / 8);
         const int64_t cap = static_cast<int64_t>(sm_count()) * 8;
         const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), n_layers, n_jobs);
-        encode_octet_kernel<FTQ_D, T><<<grid, threads, 0, stream>>>(jobs);
-        return cudaGetLastError();
+        return launch_dependent(encode_octet_kernel<FTQ_D, T>, grid, threads, 0, stream, jobs);
     }
     constexpr int threads = 128;                       // 4 warps, a vector each
     const int64_t want = (n + threads / 32 - 1) / (threads / 32);
     const int64_t cap = static_cast<int64_t>(sm_count()) * 64;
     const dim3 grid(static_cast<unsigned>(want < cap ? want : cap), n_layers, n_jobs);
-    encode_kernel<FTQ_D, T><<<grid, threads, 0, stream>>>(jobs);
-    return cudaGetLastError();
+    return launch_dependent(encode_kernel<FTQ_D, T>, grid, threads, 0, stream, jobs);
 }
 
 cudaError_t FTQ_CAT(launch_encode_d, FTQ_D)(int dtype, const EncodeJobs& jobs, int n_jobs, Encode kind,

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <utility>
 
 #include "ftq_attn_chunk.cuh"
 #include "ftq_encode2.cuh"
@@ -27,7 +28,8 @@ enum class Encode { kFew, kTable, kAnyCodebook };
     cudaError_t launch_attn_merge_d##DD(int out_dtype, const float* partials, void* out,        \
                                         const int32_t* seq_lens, int S, int B, int Hq,          \
                                         int n_chunks, int chunk_tokens, int64_t n_vec,          \
-                                        const SignBits& signs, float rsqrt_d, cudaStream_t stream);
+                                        const SignBits& signs, float rsqrt_d,               \
+                                        const MergeStatus& status, cudaStream_t stream);
 
 FTQ_DECLARE_LAUNCHERS(64)
 FTQ_DECLARE_LAUNCHERS(128)
@@ -52,10 +54,10 @@ inline cudaError_t allow_smem(int bytes) {
     return r;
 }
 // Launches a kernel that may start its set-up while the kernel before it drains (programmatic stream serialisation).
-template <typename P>
-inline cudaError_t launch_dependent(void (*kern)(P), unsigned grid, int threads, int smem, cudaStream_t stream, const P& p) {
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t stream, A&&... args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -64,7 +66,7 @@ inline cudaError_t launch_dependent(void (*kern)(P), unsigned grid, int threads,
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, p);
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 }  // namespace
 

@@ -1066,8 +1066,8 @@ tq_join_kernel(const __grid_constant__ TqMergeParams p) {
     const int h = static_cast<int>(static_cast<uint32_t>(row) - r * p.Hq);
     const uint32_t layer = fast_div(r, p.div_bseq);
     const int b = static_cast<int>(r - layer * p.B_seq);
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");   // stage 1 is complete
+    let_next_kernel_start();
+    after_previous_kernel();   // stage 1 is complete
     const uint32_t share = p.share[0];
     const int64_t shares0 = static_cast<int64_t>(layer) * p.share[1];
     const int len = p.seq_lens[b], start = p.kv_start ? p.kv_start[b] : 0;

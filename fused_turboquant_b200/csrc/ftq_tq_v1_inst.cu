@@ -105,8 +105,7 @@ static cudaError_t store2_run(const TqStore2Params& p, int n_layers, cudaStream_
     const int64_t want = (p.n_vec + threads / 4 - 1) / (threads / 4);
     const int64_t wave = static_cast<int64_t>(sm_count()) * (512 / threads);
     const int64_t cap = (wave + n_layers - 1) / n_layers;
-    kern<<<dim3(static_cast<unsigned>(want < cap ? want : cap), n_layers), threads, smem, stream>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(kern, dim3(static_cast<unsigned>(want < cap ? want : cap), n_layers), threads, smem, stream, p);
 }
 template <int KB, int VB>
 static cudaError_t store2_by_type(int dtype, const TqStore2Params& p, bool rot, int n_layers, cudaStream_t s) {

@@ -138,6 +138,8 @@ tq_store2_kernel(const __grid_constant__ TqStore2Params pp) {
         }
         __syncthreads();
     }
+    let_next_kernel_start();
+    after_previous_kernel();
     const uint32_t lut_col = (lane & 15) * 8;
     const u64 scale2 = pk2(p.rsqrt_d, p.rsqrt_d), cs2 = pk2(kCellScale, kCellScale), cm2 = pk2(kCellMagic, kCellMagic);
 

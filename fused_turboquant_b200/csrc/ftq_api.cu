@@ -1420,7 +1420,7 @@ extern "C" int ftq_tq_decode(const void* q, int q_dtype, int B, int Hq, int Hkv,
 // Workspace of the slot-format decode: [shares | page prefix sums | two row blocks per layer and share].  Where the rows
 // of all layers would take more than 64 MiB the layers are run in several groups.
 static size_t tq_rows_offset(int B) { return (256 + (static_cast<size_t>(B) + 1) * 4 + 255) / 256 * 256; }
-static size_t tq_layer_rows(int Hq, int head_dim) { return 2 * static_cast<size_t>(ftq::sm_count()) * Hq * (head_dim + 1) * 4; }
+static size_t tq_layer_rows(int Hq, int head_dim) { return 2 * static_cast<size_t>(ftq::sm_count()) * Hq * (head_dim + 2) * 4; }
 static int tq_layers_per_launch(int Hq, int head_dim, int n_layers) {
     const size_t fit = (64u << 20) / tq_layer_rows(Hq, head_dim);
     return fit < 1 ? 1 : fit < static_cast<size_t>(n_layers) ? static_cast<int>(fit) : n_layers;
@@ -1551,11 +1551,16 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
                      head_dim != 256 && aligned(kv_cache, 4) && strides % 4 == 0 &&
                      static_cast<int64_t>(B) * Hkv * num_kv_splits < (1ll << 31);
     // With a workspace, and pages of 16 slots that are one aligned span of memory for all KV heads, the kernel that
-    // streams whole pages (ftq_tq_v1_flow.cuh).
+    // streams whole pages (ftq_tq_v1_flow.cuh): at most two warps a KV head, so that a piece is many pages for each of them,
+    // and about as many (sequence, split) units as SMs, so that few of them are cut into more than two pieces, which the
+    // merge goes through one after the other.  Measured, items : shares in us, 8 splits, 4-bit codes: 32 x 8192 tokens of 8
+    // heads 182 : 122, 2 x 100 x 700 ragged 414 : 181, FP8 keys 16 x 4096 72 : 58; but 1 x 30000 45 : 148, 8 x 2000
+    // ragged 39 : 83, 6 x 64 x 1500 of 2 heads 139 : 198, 3 x 5000 of one head 23 : 43.
     const int64_t slot = ftq_tq_slot_bytes(head_dim, key_bits, value_bits);
-    const bool flow = (mma || fp8) && workspace && workspace_bytes >= ftq_tq_decode_workspace_bytes(B_seq, Hq, head_dim, n_layers) &&
+    const bool flow = (mma || (fp8 && (head_dim == 64 || group <= 4))) && workspace && workspace_bytes >= ftq_tq_decode_workspace_bytes(B_seq, Hq, head_dim, n_layers) &&
                       aligned(workspace, 16) && aligned(kv_cache, 16) && stride_block % 16 == 0 &&
                       cache_layer_stride % 16 == 0 && block_size % 16 == 0 && stride_head >= slot &&
+                      Hkv >= 8 && static_cast<int64_t>(B_seq) * num_kv_splits >= 128 &&
                       stride_pos == Hkv * stride_head && ftq::tq_flow_fits(Hkv, stride_pos, head_dim, key_bits, value_bits, group) &&
                       num_kv_splits <= ftq::kTqFlowSplits && B_seq <= ftq::kFlowMaxSeqs &&
                       static_cast<int64_t>(B_seq) * (static_cast<int64_t>(max_blocks) * (block_size / 16) + num_kv_splits) < (1ll << 30) &&

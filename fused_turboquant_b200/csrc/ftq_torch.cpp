@@ -646,7 +646,8 @@ PyObject* tq_decode(PyObject* const* a) {
     const bool nc = as_bool(a[8]), rot = as_bool(a[9]), lloyd = as_bool(a[10]);
     const double scale = as_double(a[11]);
     void* st = stream_of(dev);
-    const at::Tensor ws = workspace(Py_None, dev, st, api.ftq_tq_decode_workspace_bytes(B, hq, d, L));
+    // (a tensor of the call's own: a captured graph keeps its memory, whatever later calls need)
+    const at::Tensor ws = empty({static_cast<int64_t>(api.ftq_tq_decode_workspace_bytes(B, hq, d, L))}, at::kByte, dev);
     int rc;
     {
         NoGil nogil;

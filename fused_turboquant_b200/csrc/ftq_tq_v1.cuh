@@ -487,6 +487,8 @@ constexpr int kTqFlowPieces = 4;                         // pieces announced ahe
 constexpr int kTqFlowBarriers = 2 * kTqFlowSlots + 2 * kTqFlowPieces + kTqFlowWarps;
 constexpr int kTqFlowSplits = 64;                        // (a CTA looks through a sequence's splits one by one)
 constexpr int kTqFlowSmem = 226 * 1024;
+// FP8 keys: five to eight heads of 128 spill 280 bytes there and stay with the item kernel
+template <int D, int NH> constexpr bool kTqFlowFp8 = D == 64 || NH == 1;
 // a warp's exchange slot, which also holds its rotated queries
 __host__ __device__ constexpr int tq_flow_xslot(int d, int nh) {
     const int out = (nh == 1 ? d / 8 : d / 4) * 128, q = 4 * nh * (d + 4) * 4;
@@ -497,7 +499,7 @@ inline bool tq_flow_fits(int Hkv, int64_t stride_pos, int d, int kb, int vb, int
     if (Hkv > kTqFlowWarps || kTqFlowWarps % Hkv != 0) return false;
     const int64_t pitch = (kPageTokens * stride_pos + 127) / 128 * 128;
     const int subs = kTqFlowWarps / Hkv;
-    const int tables = kb == 8 ? 0 : (kb == 4 ? 0 : 2 * (128 << (2 * kb))) + (vb == 4 ? 0 : 2 * (128 << (2 * vb)));
+    const int tables = kb == 8 ? 0 : (kb == 4 ? 0 : 3 * (128 << (2 * kb))) + (vb == 4 ? 0 : 2 * (128 << (2 * vb)));
     const int small = kTqFlowBarriers * 8 + kTqFlowSlots * 8 + kTqFlowWarps * 24 * 4 + (kFlowMaxSeqs + 4) * 4 + 1024;
     const int xarea = kTqFlowWarps * tq_flow_xslot(d, group <= 4 ? 1 : 2);
     // (worst case over where the 64 KB window of the byte table lies: what is in front of it and what is behind it)
@@ -518,7 +520,7 @@ struct TqFlowParams {
     // sequences before b over all splits, row blocks
     uint32_t* share;      // [2]
     int* prefix;          // [B_seq + 1]
-    float* rows;          // [layers * shares][2][Hq][D + 1]
+    float* rows;          // [layers * shares][2][Hq][D + 2]: sums, base-2 reference maximum, sum of the weights
 };
 
 constexpr int kTqTileTokens = 64;
@@ -1080,39 +1082,43 @@ tq_join_kernel(const __grid_constant__ TqMergeParams p) {
         if ((s & 7) == oct && n > 0 && share > 0) {
             const uint32_t c0 = pos / share, c1 = (pos + n - 1) / share;
             float* mid = p.mid_out + (row * p.splits + s) * (D + 1);
-            // (row block 0 is the piece the share starts with, 1 its last one)
-            auto piece = [&](uint32_t c) {
-                return c0 == c1 ? mid : p.rows + ((2 * (shares0 + c) + (c * share >= pos ? 0 : 1)) * p.Hq + h) * (D + 1);
-            };
-            float x[E], ms = -INFINITY, ls = 0.f;
+            float x[E], ms;
+            if (c0 == c1) {
+                ms = __ldcg(mid + D);
 #pragma unroll
-            for (int i = 0; i < E; i++) x[i] = 0.f;
-            for (uint32_t c = c0; c <= c1; c++) {
-                const float* src = piece(c);
-                const float lse = __ldcg(src + D);
-                float y[E];
+                for (int i = 0; i < E; i++) x[i] = __ldcg(mid + load_coord(t, i));
+            } else {
+                // (row block 0 is the piece the share starts with, 1 its last one)
+                auto piece = [&](uint32_t c) {
+                    return p.rows + ((2 * (shares0 + c) + (c * share >= pos ? 0 : 1)) * p.Hq + h) * (D + 2);
+                };
+                float top = -INFINITY, ls = 0.f;
+#pragma unroll 4
+                for (uint32_t c = c0; c <= c1; c++) top = fmaxf(top, __ldcg(piece(c) + D));
 #pragma unroll
-                for (int i = 0; i < E; i++) y[i] = __ldcg(src + load_coord(t, i));
-                const float m_new = fmaxf(ms, lse);
-                const float f0 = __expf(ms - m_new), f = __expf(lse - m_new);   // (a NaN stays one)
-                ls = fmaf(ls, f0, f);
+                for (int i = 0; i < E; i++) x[i] = 0.f;
+#pragma unroll 2
+                for (uint32_t c = c0; c <= c1; c++) {
+                    const float* src = piece(c);
+                    float y[E];
 #pragma unroll
-                for (int i = 0; i < E; i++) x[i] = fmaf(x[i], f0, y[i] * f);
-                ms = m_new;
-            }
-            if (c0 != c1) {
+                    for (int i = 0; i < E; i++) y[i] = __ldcg(src + load_coord(t, i));
+                    const float f = fast_exp2(__ldcg(src + D) - top);
+                    ls = fmaf(__ldcg(src + D + 1), f, ls);   // (a NaN stays one)
+#pragma unroll
+                    for (int i = 0; i < E; i++) x[i] = fmaf(y[i], f, x[i]);
+                }
                 const float inv = 1.f / ls;
-                const float lse = ms + logf(ls);
+                ms = top * 0.6931471805599453f + logf(ls);
 #pragma unroll
                 for (int i = 0; i < E; i++) {
                     x[i] *= inv;
                     mid[load_coord(t, i)] = x[i];
                 }
-                if (t == 0) mid[D] = lse;
-                ms = lse;
+                if (t == 0) mid[D] = ms;
             }
             const float m_new = fmaxf(M, ms);
-            const float f0 = __expf(M - m_new), f = c0 == c1 ? ls * __expf(ms - m_new) : __expf(ms - m_new);
+            const float f0 = __expf(M - m_new), f = __expf(ms - m_new);
             l = fmaf(l, f0, f);
 #pragma unroll
             for (int i = 0; i < E; i++) a[i] = fmaf(a[i], f0, x[i] * f);

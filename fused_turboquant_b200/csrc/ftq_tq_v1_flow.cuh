@@ -34,13 +34,20 @@
 
 namespace ftq {
 
-__device__ __forceinline__ void mma_1688(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(b0));
+// mbar_wait that leaves the issue slots to the other warps between polls.  (Polls without a pause were a tenth of the
+// kernel's instructions; a poll with a suspend-time hint of 2 us slept that long whenever the copy had not arrived yet:
+// one sequence of 30000 tokens took 141 us.)
+__device__ __forceinline__ bool mbar_wait_idle(uint32_t bar, uint32_t parity) {
+    for (int i = 0; i < kMbarSpinLimit; i++) {
+        if (mbar_try_wait(bar, parity)) return true;
+        __nanosleep(32);
+    }
+    return false;
 }
-__device__ __forceinline__ void mma_1688_z(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};\n"
-        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a0), "r"(a1), "r"(b0), "f"(0.f));
+// A constant that stays in its register (an instruction has room for one immediate).
+__device__ __forceinline__ uint32_t in_register(uint32_t v) {
+    asm volatile("" : "+r"(v));
+    return v;
 }
 
 // What the warps of a CTA hear about a piece.
@@ -58,9 +65,8 @@ struct TqPiece {
 //   O^T: A rows = coordinates, k = (token, parity) for at most four heads, tokens for five to eight; the lane's tokens
 //      are 2 tg, 2 tg + 1, 2 tg + 8, 2 tg + 9; 4-bit codes: words g and g + 8 of the rows, else slices of
 //      D / 8 coordinates
-// A slot starts 0 or 2 bytes behind a word boundary.  4-bit rows are not realigned when all tokens of the
-// head start the same way (an even number of bytes per token is a multiple of 4): the codes are read as
-// the aligned words hold them, the two halves of the words at the ends put together, and the coordinates of the query
+// A head's slots start 0 or 2 bytes behind a word boundary, all alike (a token's bytes are a multiple of 4).  4-bit rows are not
+// realigned: the codes are read as the aligned words hold them, the two halves of the words at the ends put together, and the coordinates of the query
 // fragments and of the output follow.
 // Values are code * scale + zero, codes centred (see ftq_tq_v1_mma.cuh); norm correction by the key
 // tile's product with itself.
@@ -72,17 +78,21 @@ struct TqCodes {
     static constexpr int IWK = 2 * KB, IWV = 2 * VB;
     static constexpr int OFF_VC = PDK + 2, OFF_SC = PDK + 2 + PDV, USED = OFF_SC + 4;
     static constexpr bool WINDOW = KB == 4;                      // 64 KB byte table of the key centroids
-    static constexpr int TKS = KB == 4 ? 0 : (1 << IWK) * 128;   // small tables, aligned to their size
+    static constexpr int TKS = KB == 4 ? 0 : (1 << IWK) * 128;   // small tables, aligned to their size (keys: two)
     static constexpr int TVS = VB == 4 ? 0 : (1 << IWV) * 128;
     static constexpr int OL = NH == 1 ? D / 8 : D / 4;           // output floats of a lane
     static constexpr float kCtr = VB == 4 ? 8.f : 0.5f * ((1 << VB) - 1);
 
+    static constexpr int FLUSH = 0;
     uint32_t qb[NKB][2];
     float m_run[HL], l_run[HL], z_run[HL], oacc[OL / 4][4];
+    float s_ref, up;    // largest value scale so far as a power of two; weights are rounded times up
     uint32_t lk_lane, lv_lane;
-    int mis;        // (tokens alike) the head's slots start 2 * mis bytes behind a word boundary
+    uint32_t magic, c_sub, c_mul, c_add;   // of centred()
+    int mis;        // the head's slots start 2 * mis bytes behind a word boundary
 
-    // Key table: 32 copies of the fp16 centroids of two adjacent codes (byte-indexed rows are 256 bytes apart).
+    // Key tables: 32 copies of the fp16 centroids of two adjacent codes, and of the sum of their squares (byte-indexed: the
+    // halves of rows of 256 bytes).
     static __device__ __forceinline__ void init_tables(const TqDecodeParams& p, uint32_t* window, uint32_t* tk,
                                                        uint32_t* tv, int tid, int threads) {
         auto pack = [](float lo, float hi) {
@@ -92,8 +102,15 @@ struct TqCodes {
         for (int i = tid; i < (1 << IWK) * 32; i += threads) {
             const int e = i >> 5;
             const uint32_t two = pack(p.centroids.v[e & ((1 << KB) - 1)], p.centroids.v[e >> KB]);
-            if constexpr (KB == 4) window[e * 64 + (i & 31)] = two;
-            else tk[i] = two;
+            const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&two));
+            const uint32_t squares = __float_as_uint(fmaf(c.x, c.x, c.y * c.y));
+            if constexpr (KB == 4) {
+                window[e * 64 + (i & 31)] = two;
+                window[e * 64 + 32 + (i & 31)] = squares;
+            } else {
+                tk[i] = two;
+                tk[TKS / 4 + i] = squares;
+            }
         }
         for (int i = tid; i < TVS / 4; i += threads) {
             const int e = i >> 5;
@@ -104,6 +121,14 @@ struct TqCodes {
         lk_lane = (KB == 4 ? window : tk) | (lane * 4);
         lv_lane = tv | (lane * 4);
         mis = mis_;
+        auto twice = [](float x) {
+            const __half2 h = __floats2half2_rn(x, x);
+            return in_register(*reinterpret_cast<const uint32_t*>(&h));
+        };
+        magic = in_register(0x64006400u);
+        c_sub = twice(1024.f + kCtr);
+        c_mul = twice(0.0625f);
+        c_add = twice(-(64.f + kCtr));
     }
 
     // queries of the head's group, rotated and pre-scaled, in qs[4 * NH][D + 4]
@@ -149,6 +174,8 @@ struct TqCodes {
             m_run[h] = -INFINITY;
             l_run[h] = z_run[h] = 0.f;
         }
+        s_ref = 0.f;
+        up = 1.f;
 #pragma unroll
         for (int i = 0; i < OL / 4; i++)
 #pragma unroll
@@ -166,24 +193,14 @@ struct TqCodes {
 #pragma unroll
         for (int j = 0; j < NW; j++) out[j] = __funnelshift_r(w[j], w[j + 1], sh);
     }
-    // N words (first + STEP * j) of a row of 4-bit codes at `at`, realigned
-    template <int N, int STEP>
-    static __device__ __forceinline__ void load_words(uint32_t at, int first, uint32_t (&out)[N]) {
-        const uint32_t base = (at & ~3u) + 4 * first, sh = 8u * (at & 3u);
-#pragma unroll
-        for (int j = 0; j < N; j++) out[j] = __funnelshift_r(lds32(base + 4 * STEP * j), lds32(base + 4 * STEP * j + 4), sh);
-    }
-
-    // The head's slots of a page: token 0 at `page`, ts bytes apart; tokens [lo, hi) count.  ALIKE: all tokens start
-    // 2 * mis bytes behind a word boundary.
-    template <bool ALIKE>
+    // The head's slots of a page: token 0 at `page`, ts bytes (a multiple of 4) apart; tokens [lo, hi) count.
     __device__ __forceinline__ void page(uint32_t page, uint32_t ts, int lo, int hi, bool norm_correction, int lane) {
         const int g = lane >> 2, tg = lane & 3;
         uint32_t ka[KW], kb_[KW];
         float kna, knb;
         uint32_t sca, scb;     // scale | zero of the lane's two tokens
-        const uint32_t aligned = page & ~3u, rowa = (ALIKE ? aligned : page) + g * ts, rowb = rowa + 8 * ts;
-        if constexpr (ALIKE && KB == 4) {
+        const uint32_t rowa = (page & ~3u) + g * ts, rowb = rowa + 8 * ts;
+        if constexpr (KB == 4) {
             // words as they lie; word 0 gets the row's last two bytes in its lower half where the row starts in its
             // middle.  The word behind the codes holds those bytes and the norm, or the norm first.
             const uint32_t sel = mis && tg == 0 ? 0x3254u : 0x3210u, sel_n = mis ? 0x4432u : 0x4410u;
@@ -198,80 +215,61 @@ struct TqCodes {
             kna = half_bits_to_float(__byte_perm(xa, 0u, sel_n));
             knb = half_bits_to_float(__byte_perm(xb, 0u, sel_n));
         } else {
-            const uint32_t ra = ALIKE ? rowa + 2 * mis : rowa, rb = ALIKE ? rowb + 2 * mis : rowb;
-            if constexpr (KB == 4) {
-                load_words<KW, 4>(ra, tg, ka);
-                load_words<KW, 4>(rb, tg, kb_);
-            } else {
-                load_bytes<KSB>(ra + KSB * tg, ka);
-                load_bytes<KSB>(rb + KSB * tg, kb_);
-            }
+            const uint32_t ra = rowa + 2 * mis, rb = rowb + 2 * mis;
+            load_bytes<KSB>(ra + KSB * tg, ka);
+            load_bytes<KSB>(rb + KSB * tg, kb_);
             unsigned short na, nb;
             asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(na) : "r"(ra + PDK));
             asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(nb) : "r"(rb + PDK));
             kna = half_bits_to_float(na);
             knb = half_bits_to_float(nb);
         }
-        if constexpr (ALIKE) {
-            const uint32_t at = OFF_SC - 2 + 4 * mis, sh = mis ? 0u : 16u;
-            sca = __funnelshift_r(lds32(rowa + at), lds32(rowa + at + 4), sh);
-            scb = __funnelshift_r(lds32(rowb + at), lds32(rowb + at + 4), sh);
-        } else {
-            uint32_t w[1];
-            load_bytes<4>(rowa + OFF_SC, w);
-            sca = w[0];
-            load_bytes<4>(rowb + OFF_SC, w);
-            scb = w[0];
-        }
+        const uint32_t at = OFF_SC - 2 + 4 * mis, sh = mis ? 0u : 16u;
+        sca = __funnelshift_r(lds32(rowa + at), lds32(rowa + at + 4), sh);
+        scb = __funnelshift_r(lds32(rowb + at), lds32(rowb + at + 4), sh);
 
-        // ---- S = K.Q^T; with norm correction the key tile times itself: the diagonal holds sum c^2 per token
-        // (k = 8 steps: the operands of one are registers of the other as they stand, those of k = 16 would have to be
-        // moved together)
+        // ---- S = K.Q^T; with norm correction the sum of the squared centroids of the two tokens.  (From a second look-up per
+        // pair of codes: the key tile times itself, whose diagonal holds the sums, kept the tensor pipe as busy as the
+        // issue slots.)
         float c[2][4];
         if (norm_correction) {   // (uniform)
-            float na[4], nb[4];
-            scores<true>(ka, kb_, c, na, nb);
-            // (row g, column g) of the first product is held by lane (g, g >> 1), element g & 1;
-            // (row g + 8, column g) of the second one by the same lane, element 2 + (g & 1)
-            const float da = (g & 1) ? na[1] : na[0], db = (g & 1) ? nb[3] : nb[2];
-            const int src = (lane & ~3) | (g >> 1);
-            kna *= rsqrtf(__shfl_sync(0xffffffffu, da, src) + 1e-16f);
-            knb *= rsqrtf(__shfl_sync(0xffffffffu, db, src) + 1e-16f);
+            u64 n2 = pk2(0.f, 0.f);
+            scores<true>(ka, kb_, c, n2);
+            n2 = add2(n2, __shfl_xor_sync(0xffffffffu, n2, 1));
+            n2 = add2(n2, __shfl_xor_sync(0xffffffffu, n2, 2));
+            float na, nb;
+            upk2(n2, na, nb);
+            kna *= rsqrtf(na + 1e-16f);
+            knb *= rsqrtf(nb + 1e-16f);
         } else {
-            float na[4], nb[4];
-            scores<false>(ka, kb_, c, na, nb);
+            u64 n2 = 0;
+            scores<false>(ka, kb_, c, n2);
         }
 
-        if (lo <= 0 && hi >= kPageTokens) attend<ALIKE, true>(page, ts, lo, hi, lane, c, kna, knb, sca, scb);
-        else attend<ALIKE, false>(page, ts, lo, hi, lane, c, kna, knb, sca, scb);
+        if (lo <= 0 && hi >= kPageTokens) attend<true>(page, ts, lo, hi, lane, c, kna, knb, sca, scb);
+        else attend<false>(page, ts, lo, hi, lane, c, kna, knb, sca, scb);
     }
 
     template <bool NC>
-    __device__ __forceinline__ void scores(const uint32_t (&ka)[KW], const uint32_t (&kb_)[KW], float (&c)[2][4],
-                                           float (&na)[4], float (&nb)[4]) const {
+    __device__ __forceinline__ void scores(const uint32_t (&ka)[KW], const uint32_t (&kb_)[KW], float (&c)[2][4], u64& n2) const {
+        constexpr uint32_t SQ = KB == 4 ? 128u : TKS;   // from an entry to its squares
+        u64 other = pk2(0.f, 0.f);
 #pragma unroll
         for (int kb = 0; kb < NKB; kb++) {
-            const uint32_t a0 = lut32(entry_addr<IWK>(ka, 2 * kb, lk_lane));
-            const uint32_t a1 = lut32(entry_addr<IWK>(kb_, 2 * kb, lk_lane));
-            const uint32_t a2 = lut32(entry_addr<IWK>(ka, 2 * kb + 1, lk_lane));
-            const uint32_t a3 = lut32(entry_addr<IWK>(kb_, 2 * kb + 1, lk_lane));
+            const uint32_t e0 = entry_addr<IWK>(ka, 2 * kb, lk_lane), e1 = entry_addr<IWK>(kb_, 2 * kb, lk_lane);
+            const uint32_t e2 = entry_addr<IWK>(ka, 2 * kb + 1, lk_lane), e3 = entry_addr<IWK>(kb_, 2 * kb + 1, lk_lane);
+            const uint32_t a0 = lut32(e0), a1 = lut32(e1), a2 = lut32(e2), a3 = lut32(e3);
             if (kb < 2) mma_16816_z(c[kb & 1], a0, a1, a2, a3, qb[kb][0], qb[kb][1]);
             else mma_16816(c[kb & 1], a0, a1, a2, a3, qb[kb][0], qb[kb][1]);
             if constexpr (NC) {
-                if (kb == 0) {
-                    mma_1688_z(na, a0, a1, a0);   // columns = the tokens of rows 0..7
-                    mma_1688_z(nb, a0, a1, a1);   // columns = the tokens of rows 8..15
-                } else {
-                    mma_1688(na, a0, a1, a0);
-                    mma_1688(nb, a0, a1, a1);
-                }
-                mma_1688(na, a2, a3, a2);
-                mma_1688(nb, a2, a3, a3);
+                n2 = add2(n2, pk2(__uint_as_float(lut32(e0 + SQ)), __uint_as_float(lut32(e1 + SQ))));
+                other = add2(other, pk2(__uint_as_float(lut32(e2 + SQ)), __uint_as_float(lut32(e3 + SQ))));
             }
         }
+        if constexpr (NC) n2 = add2(n2, other);
     }
 
-    template <bool ALIKE, bool FULL>
+    template <bool FULL>
     __device__ __forceinline__ void attend(uint32_t page, uint32_t ts, int lo, int hi, int lane, const float (&c)[2][4],
                                            float kna, float knb, uint32_t sca, uint32_t scb) {
         const int g = lane >> 2, tg = lane & 3;
@@ -282,7 +280,8 @@ struct TqCodes {
         const float vsa = okA ? fa.x : 0.f, vsb = okB ? fb.x : 0.f;
         const float vza = okA ? fmaf(kCtr, fa.x, fa.y) : 0.f, vzb = okB ? fmaf(kCtr, fb.x, fb.y) : 0.f;
         float sa[HL], sb[HL];
-        bool above = false;
+        const float s_max = fmaxf(fabsf(vsa), fabsf(vsb));
+        bool above = s_max > s_ref;
 #pragma unroll
         for (int h = 0; h < HL; h++) {
             sa[h] = okA ? (c[0][h] + c[1][h]) * kna : -INFINITY;
@@ -290,6 +289,19 @@ struct TqCodes {
             above |= fmaxf(sa[h], sb[h]) > m_run[h];
         }
         if (__any_sync(0xffffffffu, above)) {
+            // the largest value scale, rounded up to a power of two, brought to 2^14: fp16 holds weights down to 2^-28 of the
+            // largest at full precision (a warp meets many pages under one reference maximum)
+            float top = s_max;
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 4));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 8));
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+            float shift = 1.f;
+            if (top > s_ref) {   // (warp-uniform)
+                s_ref = __uint_as_float((__float_as_uint(top) + 0x007fffffu) & 0x7f800000u);
+                const float was = up;
+                up = 16384.f / s_ref;
+                shift = up / was;
+            }
             float corr[HL];
 #pragma unroll
             for (int h = 0; h < HL; h++) {
@@ -306,33 +318,32 @@ struct TqCodes {
 #pragma unroll
             for (int i = 0; i < OL / 4; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) oacc[i][j] *= corr[j % HL];
+                for (int j = 0; j < 4; j++) oacc[i][j] *= corr[j % HL] * shift;
         }
         float wa[HL], wb[HL];
+        const float sua = vsa * up, sub = vsb * up;   // (exact)
 #pragma unroll
         for (int h = 0; h < HL; h++) {
             const float pa = fast_exp2(sa[h] - m_run[h]), pb = fast_exp2(sb[h] - m_run[h]);
             l_run[h] += pa + pb;
             z_run[h] = fmaf(pa, vza, fmaf(pb, vzb, z_run[h]));
-            wa[h] = pa * vsa;
-            wb[h] = pb * vsb;
+            wa[h] = pa * sua;
+            wb[h] = pb * sub;
         }
 
         // ---- O^T += V^T.P^T
         uint32_t v[4][VW];
-        const uint32_t vrow = (ALIKE ? page & ~3u : page) + 2 * tg * ts;
+        const uint32_t vrow = (page & ~3u) + 2 * tg * ts;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const uint32_t row = vrow + ((j & 1) + 8 * (j >> 1)) * ts;
-            if constexpr (ALIKE && VB == 4) {   // (as the keys; the values start OFF_VC = 2 mod 4 bytes into the slot)
+            if constexpr (VB == 4) {   // (as the keys; the values start OFF_VC = 2 mod 4 bytes into the slot)
                 const uint32_t at = row + OFF_VC - 2 + 4 * mis;
 #pragma unroll
                 for (int u = 0; u < VW; u++) v[j][u] = lds32(at + 4 * g + 32 * u);
                 v[j][0] = __byte_perm(v[j][0], lds32(at + PDV), !mis && g == 0 ? 0x3254u : 0x3210u);
-            } else if constexpr (VB == 4) {
-                load_words<VW, 8>(row + OFF_VC, g, v[j]);
             } else {
-                load_bytes<VSB>(row + (ALIKE ? 2 * mis : 0) + OFF_VC + VSB * g, v[j]);
+                load_bytes<VSB>(row + 2 * mis + OFF_VC + VSB * g, v[j]);
             }
         }
         auto pack = [](float lo, float hi) {
@@ -394,14 +405,12 @@ struct TqCodes {
     // The codes at bits 0, 4, 8, 12 of each 16-bit half of w, centred, as fp16 pairs: a nibble or-ed into the
     // mantissa of 1024 is 1024 + code (or 1024 + 16 code one nibble up), one packed subtraction or
     // multiply-add centres it exactly.
-    static __device__ __forceinline__ void centred(uint32_t w, uint32_t (&t)[4]) {
-        const uint32_t kMagic = 0x64006400u;
-        const __half2 sub = __floats2half2_rn(1024.f + kCtr, 1024.f + kCtr);
-        const __half2 mul = __floats2half2_rn(0.0625f, 0.0625f);
-        const __half2 add = __floats2half2_rn(-(64.f + kCtr), -(64.f + kCtr));
+    __device__ __forceinline__ void centred(uint32_t w, uint32_t (&t)[4]) const {
         const uint32_t w8 = w >> 8;
-        const uint32_t x[4] = {(w & 0x000F000Fu) | kMagic, (w & 0x00F000F0u) | kMagic,
-                               (w8 & 0x000F000Fu) | kMagic, (w8 & 0x00F000F0u) | kMagic};
+        const uint32_t x[4] = {(w & 0x000F000Fu) | magic, (w & 0x00F000F0u) | magic,
+                               (w8 & 0x000F000Fu) | magic, (w8 & 0x00F000F0u) | magic};
+        const __half2 sub = *reinterpret_cast<const __half2*>(&c_sub), mul = *reinterpret_cast<const __half2*>(&c_mul),
+                      add = *reinterpret_cast<const __half2*>(&c_add);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const __half2 h = *reinterpret_cast<const __half2*>(&x[i]);
@@ -420,7 +429,7 @@ struct TqCodes {
                 z_run[h] += __shfl_xor_sync(0xffffffffu, z_run[h], m);
             }
 #pragma unroll
-        for (int f = 0; f < OL; f++) xo[f * 32 + lane] = oacc[f >> 2][f & 3];
+        for (int f = 0; f < OL; f++) xo[f * 32 + lane] = oacc[f >> 2][f & 3] * (1.f / up);
         if (lane < 4) {
 #pragma unroll
             for (int h = 0; h < HL; h++) {
@@ -432,12 +441,12 @@ struct TqCodes {
     }
     // head and coordinate of output float f of lane ln
     static __device__ __forceinline__ int head_of(int f, int ln) { return NH == 1 ? ln & 3 : 2 * (ln & 3) + (f & 1); }
-    __device__ __forceinline__ int coord_of(int f, int ln, bool alike) const {
+    __device__ __forceinline__ int coord_of(int f, int ln) const {
         const int g = ln >> 2, tile = f >> 2, i = f & 3;
         if constexpr (VB == 4) {
             const int u = NH == 1 ? tile >> 1 : tile >> 2;
             const int nib = NH == 1 ? 2 * (tile & 1) + (i >> 1) + 4 * (i & 1) : 2 * (tile & 3) + (i >> 1);
-            return (8 * (g + 8 * u) + nib - (alike && !mis ? 4 : 0)) & (D - 1);
+            return (8 * (g + 8 * u) + nib - (mis ? 0 : 4)) & (D - 1);
         } else {
             return (D / 8) * g + (NH == 1 ? 4 * tile + i : 2 * tile + (i >> 1));
         }
@@ -465,7 +474,7 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
         free1 = a + bytes;
         return a;
     };
-    const uint32_t tk = E::TKS > 0 ? take(E::TKS, E::TKS) : 0, tv = E::TVS > 0 ? take(E::TVS, E::TVS) : 0;
+    const uint32_t tk = E::TKS > 0 ? take(2 * E::TKS, E::TKS) : 0, tv = E::TVS > 0 ? take(E::TVS, E::TVS) : 0;
     const uint32_t full = take(kTqFlowBarriers * 8, 128), empty = full + kTqFlowSlots * 8,
                    pfull = empty + kTqFlowSlots * 8, pempty = pfull + kTqFlowPieces * 8, folded = pempty + kTqFlowPieces * 8;
     TqPiece* pieces = reinterpret_cast<TqPiece*>(gptr(take(kTqFlowPieces * sizeof(TqPiece), 128)));
@@ -498,8 +507,8 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
         mbar_init(pempty + tid * 8, kTqFlowWarps);
     }
     mbar_fence_init();
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    let_next_kernel_start();
+    after_previous_kernel();
 
     // ---- prefix sums of the sequences' pages over all splits (also for the merge kernel)
     auto kv_start_of = [&](int b) { return p.kv_start ? p.kv_start[b] : 0; };
@@ -561,7 +570,7 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
         if (at < last) pos = at % n_shares * share;
         for (;;) {
             const int ps = pi % kTqFlowPieces;
-            if (pi >= kTqFlowPieces) ok = mbar_wait(pempty + ps * 8, ((pi / kTqFlowPieces) - 1) & 1) && ok;
+            if (pi >= kTqFlowPieces) ok = mbar_wait_idle(pempty + ps * 8, ((pi / kTqFlowPieces) - 1) & 1) && ok;
             TqPiece pc{};
             int b = 0, layer = 0, page0 = 0;
             if (ok && at < last) {
@@ -619,25 +628,25 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
                 }
                 int64_t id = __shfl_sync(0xffffffffu, ids, (i0 + lane) & 31);
                 const int i = i0 + lane;
-                const bool mine = lane < subs && i < pc.n;
                 const int k = sub_pages + i0 / subs, turn = k / per_sub, s = (k - turn * per_sub) * subs + lane;
-                // (a slot whose last copy has not arrived is not armed again)
-                bool free = !mine || turn == 0;
-                for (int spin = 0; spin < kMbarSpinLimit; spin++) {
-                    if (!free) free = mbar_try_wait(empty + s * 8, (turn - 1) & 1) && mbar_try_wait(full + s * 8, (turn - 1) & 1);
-                    if (__all_sync(0xffffffffu, free)) break;
-                    __nanosleep(50);
-                }
-                ok = __all_sync(0xffffffffu, free);
-                if (ok && mine) {
-                    const uint32_t tok = static_cast<uint32_t>(page0 + i) * kPageTokens;
-                    const uint32_t off = tok - fast_div(tok, p.div_block) * p.block_size;
-                    const bool bad = p.num_blocks > 0 && static_cast<uint64_t>(id) >= static_cast<uint64_t>(p.num_blocks);
-                    if (bad) id = 0;
-                    slot_info[s].y = 2 * turn + (bad ? 1 : 0);
-                    mbar_expect_tx(full + s * 8, bytes);
-                    bulk_g2s_hint(slot_info[s].x, kv_layer + id * p.stride_block + static_cast<int64_t>(off) * ts, bytes,
-                                  full + s * 8, policy);
+                const uint32_t tok = static_cast<uint32_t>(page0 + i) * kPageTokens;
+                const uint32_t off = tok - fast_div(tok, p.div_block) * p.block_size;
+                const bool bad = p.num_blocks > 0 && static_cast<uint64_t>(id) >= static_cast<uint64_t>(p.num_blocks);
+                if (bad) id = 0;
+                const uint8_t* const src = kv_layer + id * p.stride_block + static_cast<int64_t>(off) * ts;
+                // one after the other (polls of all of them at once were a quarter of the kernel's instructions)
+                for (int u = 0; u < subs && ok; u++) {
+                    const int s_u = __shfl_sync(0xffffffffu, s, u), turn_u = __shfl_sync(0xffffffffu, turn, u);
+                    if (i0 + u >= pc.n) break;
+                    // (a slot whose last copy has not arrived is not armed again)
+                    if (turn_u > 0)
+                        ok = mbar_wait_idle(empty + s_u * 8, (turn_u - 1) & 1) && mbar_wait(full + s_u * 8, (turn_u - 1) & 1);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (ok && lane == u) {
+                        slot_info[s].y = 2 * turn + (bad ? 1 : 0);
+                        mbar_expect_tx(full + s * 8, bytes);
+                        bulk_g2s_hint(slot_info[s].x, src, bytes, full + s * 8, policy);
+                    }
                 }
                 __syncwarp();
             }
@@ -664,17 +673,16 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
         __syncwarp();
         if (subs == 1) return;
         if (lane == 0) mbar_arrive(folded + head * 8);
-        if (!stalled && !mbar_wait(folded + head * 8, fold_par)) stalled = true;
+        if (!stalled && !mbar_wait_idle(folded + head * 8, fold_par)) stalled = true;
         fold_par ^= 1u;
     };
     E e;
-    const bool alike = (ts & 2u) == 0u;
-    e.init(window, tk, tv, lane, alike ? (my_off >> 1) & 1 : 0);
+    e.init(window, tk, tv, lane, (my_off >> 1) & 1);
     int s = sub;             // ring slot of the warp's next page, and the parity of its turn
     uint32_t par = 0;
     for (int pi = 0;; pi++) {
         const int ps = pi % kTqFlowPieces;
-        if (!mbar_wait(pfull + ps * 8, (pi / kTqFlowPieces) & 1)) {
+        if (!mbar_wait_idle(pfull + ps * 8, (pi / kTqFlowPieces) & 1)) {
             stalled = true;
             break;
         }
@@ -689,23 +697,23 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
         e.begin(qs, lane >> 2, lane & 3);
         __syncwarp();
         bool poison = false;
-        auto walk = [&](auto alike_tag) {
+        int seen = 0;
+        (void)seen;
         for (int i = sub; i < n; i += subs) {
-            if (!stalled && !mbar_wait(full + s * 8, par)) stalled = true;
+            if (!stalled && !mbar_wait_idle(full + s * 8, par)) stalled = true;
             const uint2 slot = lds64(slot_table + s * 8);
             poison |= (slot.y & 1u) != 0u;
             const uint32_t page = slot.x + my_off;
-            e.template page<decltype(alike_tag)::value>(page, ts, lo, hi, p.norm_correction != 0, lane);
+            e.page(page, ts, lo, hi, p.norm_correction != 0, lane);
             __syncwarp();
             if (lane == 0) mbar_arrive(empty + s * 8);
+            if constexpr (E::FLUSH > 0)
+                if (++seen % E::FLUSH == 0) e.flush(xchg(warp), lane);
             s += subs;
             if (s >= n_slots) { s = sub; par ^= 1u; }
             lo -= subs * kPageTokens;
             hi -= subs * kPageTokens;
         }
-        };
-        if (alike) walk(std::true_type{});
-        else walk(std::false_type{});
 
         // ---- the warps of the head put their states together
         head0 = static_cast<int64_t>(pc.row) * p.Hq + head * group;
@@ -731,11 +739,19 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
                 l = fmaf(xml[w * 24 + 8 + h], sc, l);
                 z = fmaf(xml[w * 24 + 16 + h], sc, z);
             }
-            float* dst = block < 0 ? p.mid_o + ((head0 + h) * p.splits + sid) * (D + 1)
-                                      : f.rows + (static_cast<int64_t>(block) * p.Hq + head * group + h) * (D + 1);
-            const int coord = e.coord_of(fo, ln, alike);
-            dst[coord] = (o + z) / l;
-            if (coord == 0) dst[D] = nan ? __int_as_float(0x7fc00000) : M * kLn2 + logf(l);
+            const int coord = e.coord_of(fo, ln);
+            if (block < 0) {
+                float* dst = p.mid_o + ((head0 + h) * p.splits + sid) * (D + 1);
+                dst[coord] = (o + z) / l;
+                if (coord == 0) dst[D] = nan ? __int_as_float(0x7fc00000) : M * kLn2 + logf(l);
+            } else {   // (sums, reference maximum and weight sum: nothing is rounded into a logarithm before the merge)
+                float* dst = f.rows + (static_cast<int64_t>(block) * p.Hq + head * group + h) * (D + 2);
+                dst[coord] = o + z;
+                if (coord == 0) {
+                    dst[D] = M;
+                    dst[D + 1] = nan ? __int_as_float(0x7fc00000) : l;
+                }
+            }
         }
         head_sync();
     }

@@ -59,6 +59,10 @@ struct TqFp8 {
     uint32_t qb[NH][NKB][2];
     float mul[HL], m_run[HL], l_run[HL], z_run[HL], oacc[NMT][2 * HL];   // [m-tile][row g or g + 8, head]
     float s_ref, up;   // largest value scale so far as a power of two; weights are split times up
+    // Sums over many pages in fp32 lose digits: a warp that goes through more than FLUSH of them adds up its sums of
+    // FLUSH pages in shared memory.  l_sum, z_sum, m_sum, up_sum: the other sums, and what the ones there are relative to.
+    static constexpr int FLUSH = WIDE ? 0 : 4;
+    float l_sum[HL], z_sum[HL], m_sum[HL], up_sum;
 
     static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
         const __half2 h = __floats2half2_rn(lo, hi);
@@ -122,7 +126,8 @@ struct TqFp8 {
         for (int h = 0; h < HL; h++) {
             mul[h] = qs[(HL * tg + h) * QROW + D];
             m_run[h] = -INFINITY;
-            l_run[h] = z_run[h] = 0.f;
+            l_run[h] = z_run[h] = l_sum[h] = z_sum[h] = 0.f;
+            m_sum[h] = -INFINITY;
         }
 #pragma unroll
         for (int mt = 0; mt < NMT; mt++)
@@ -130,6 +135,28 @@ struct TqFp8 {
             for (int i = 0; i < 2 * HL; i++) oacc[mt][i] = 0.f;
         s_ref = 0.f;
         up = 1.f;
+        up_sum = 0.f;   // (nothing there yet)
+    }
+    // adds the sums since the last time to those at xo[f * 32 + lane] (the lane's own)
+    __device__ __forceinline__ void flush(float* xo, int lane) {
+        const float ratio = up_sum > 0.f ? up / up_sum : 0.f;
+#pragma unroll
+        for (int h = 0; h < HL; h++) {
+            const float f = up_sum > 0.f ? fast_exp2(m_sum[h] - m_run[h]) : 0.f;
+            l_sum[h] = fmaf(l_sum[h], f, l_run[h]);
+            z_sum[h] = fmaf(z_sum[h], f, z_run[h]);
+            l_run[h] = z_run[h] = 0.f;
+            m_sum[h] = m_run[h];
+#pragma unroll
+            for (int mt = 0; mt < NMT; mt++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    float* at = xo + (mt * 2 * HL + j * HL + h) * 32 + lane;
+                    *at = up_sum > 0.f ? fmaf(*at, f * ratio, oacc[mt][j * HL + h]) : oacc[mt][j * HL + h];
+                    oacc[mt][j * HL + h] = 0.f;
+                }
+        }
+        up_sum = up;
     }
     // a lane's value slice (at the 4-byte aligned `at`, `sh` = 8 * the bytes it starts behind it)
     static __device__ __forceinline__ void load_slice(uint32_t at, uint32_t sh, uint32_t (&w)[VW]) {
@@ -142,7 +169,6 @@ struct TqFp8 {
     }
 
     // token 0 at `page`, `row` bytes apart; tokens [lo, hi) count
-    template <bool ALIKE>
     __device__ __forceinline__ void page(uint32_t page, uint32_t row, int lo, int hi, bool, int lane) {
         const int g = lane >> 2, tg = lane & 3;
         // ---- scores: chains of NKB / CH MMAs (an MMA's sum is truncated, the sums of the chains'
@@ -331,6 +357,21 @@ struct TqFp8 {
     }
     // the lane's state: OL floats at xo[f * 32 + lane], (m, l, z) of its heads at xml[0..2][8]
     __device__ __forceinline__ void publish(float* xo, float* xml, int lane, bool poison) {
+        if constexpr (FLUSH > 0) {
+            flush(xo, lane);
+#pragma unroll
+            for (int h = 0; h < HL; h++) {
+                l_run[h] = l_sum[h];
+                z_run[h] = z_sum[h];
+            }
+#pragma unroll
+            for (int f = 0; f < OL; f++) xo[f * 32 + lane] *= 1.f / up;
+        } else {
+#pragma unroll
+            for (int mt = 0; mt < NMT; mt++)
+#pragma unroll
+                for (int i = 0; i < 2 * HL; i++) xo[(mt * 2 * HL + i) * 32 + lane] = oacc[mt][i] * (1.f / up);
+        }
 #pragma unroll
         for (int h = 0; h < HL; h++)
 #pragma unroll
@@ -338,10 +379,6 @@ struct TqFp8 {
                 l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], m);
                 z_run[h] += __shfl_xor_sync(0xffffffffu, z_run[h], m);
             }
-#pragma unroll
-        for (int mt = 0; mt < NMT; mt++)
-#pragma unroll
-            for (int i = 0; i < 2 * HL; i++) xo[(mt * 2 * HL + i) * 32 + lane] = oacc[mt][i] * (1.f / up);
         if (lane < 4) {
 #pragma unroll
             for (int h = 0; h < HL; h++) {
@@ -353,7 +390,7 @@ struct TqFp8 {
     }
     // head and coordinate of output float f = (m-tile, row g or g + 8, head) of lane ln
     static __device__ __forceinline__ int head_of(int f, int ln) { return HL * (ln & 3) + f % HL; }
-    __device__ __forceinline__ int coord_of(int f, int ln, bool) const { return (D / 8) * (ln >> 2) + f / HL; }
+    __device__ __forceinline__ int coord_of(int f, int ln) const { return (D / 8) * (ln >> 2) + f / HL; }
 };
 
 template <int D, int VB, int NH>
@@ -476,7 +513,7 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
             copy_next();
             stage = stage + 1 == C::STAGES ? 0 : stage + 1;
 
-            e.template page<true>(page, C::ROWB, 0, it.t1 - it.t0 - pg * kPageTokens, false, lane);
+            e.page(page, C::ROWB, 0, it.t1 - it.t0 - pg * kPageTokens, false, lane);
         }
 
         // ---- fold the warps' states
@@ -497,7 +534,7 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
                 z = fmaf(xml[(w * 3 + 2) * 8 + h], s, z);
             }
             float* dst = mid_row(it, h);
-            const int coord = e.coord_of(f, ln, true);
+            const int coord = e.coord_of(f, ln);
             dst[coord] = (o + z) / l;
             if (coord == 0) dst[D] = any_bad ? __int_as_float(0x7fc00000) : M * kLn2 + logf(l);
         }

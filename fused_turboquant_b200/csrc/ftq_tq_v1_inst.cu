@@ -253,8 +253,9 @@ static cudaError_t flow_run(const TqFlowParams& p, cudaStream_t stream) {
 }
 template <int KB, int VB, int NH>
 static cudaError_t flow_engine(const TqFlowParams& p, cudaStream_t s) {
-    if constexpr (KB == 8) return flow_run<TqFp8<FTQ_D, VB, NH, false>>(p, s);
-    else return flow_run<TqCodes<FTQ_D, KB, VB, NH>>(p, s);
+    if constexpr (KB != 8) return flow_run<TqCodes<FTQ_D, KB, VB, NH>>(p, s);
+    else if constexpr (kTqFlowFp8<FTQ_D, NH>) return flow_run<TqFp8<FTQ_D, VB, NH, false>>(p, s);
+    else return cudaErrorInvalidValue;
 }
 template <int KB, int VB>
 static cudaError_t flow_by_nh(int nh, const TqFlowParams& p, cudaStream_t s) {

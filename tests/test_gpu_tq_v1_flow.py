@@ -56,16 +56,16 @@ def _compare(got, ref):
     np.testing.assert_allclose(l[np.isfinite(l_ref)], l_ref[np.isfinite(l_ref)], rtol=2e-3, atol=5e-3)
 
 
-SHAPES = [(128, 4, 4, 8, 4), (128, 4, 4, 4, 8), (128, 4, 4, 2, 7), (128, 4, 4, 1, 4), (128, 4, 4, 1, 8), (128, 4, 4, 16, 2),
-          (128, 3, 4, 8, 1), (128, 4, 3, 2, 4), (128, 3, 3, 8, 8), (128, 2, 2, 4, 4), (64, 4, 4, 8, 4), (64, 4, 4, 1, 5),
-          (64, 3, 3, 2, 7), (64, 3, 4, 4, 2), (64, 4, 2, 2, 8), (128, 4, 4, 3, 4)]   # (3 heads: the item kernel)
+SHAPES = [(128, 4, 4, 8, 4), (128, 4, 4, 8, 8), (128, 4, 4, 16, 2), (128, 3, 4, 8, 1), (128, 4, 3, 8, 4), (128, 3, 3, 8, 8),
+          (128, 2, 2, 16, 4), (64, 4, 4, 8, 4), (64, 4, 4, 16, 5), (64, 3, 3, 8, 7), (64, 3, 4, 8, 2), (64, 4, 2, 16, 8),
+          (128, 4, 4, 4, 4)]   # (four heads: the item kernel)
 
 
 @pytest.mark.parametrize("D,kb,vb,Hkv,G", SHAPES)
 def test_ragged(D, kb, vb, Hkv, G):
     cfg, cent, cache, bt, seq, q = _batch(D, kb, vb, Hkv, G, [1, 0, 15, 16, 17, 333, 2500, 64], seed=D + Hkv)
     start = torch.tensor([0, 0, 3, 16, 16, 100, 7, 64], dtype=torch.int32, device="cuda")
-    for splits, st in ((8, None), (3, start), (1, None)):
+    for splits, st in ((16, None), (19, start), (64, None), (3, start)):   # (3: the item kernel)
         _compare(_decode(q[0], cache[0], bt, seq, cent, cfg, splits, st),
                  _decode(q[0].float(), cache[0], bt, seq, cent, cfg, splits, st))
 
@@ -74,32 +74,32 @@ def test_ragged(D, kb, vb, Hkv, G):
 def test_block_sizes_padding_and_long_pieces(bs, pad, nc):
     """Blocks of several pages, slots longer than their contents, shares that cut splits of many pages."""
     cfg, cent, cache, bt, seq, q = _batch(128, 4, 4, 8, 4, [9001, 4000], bs=bs, pad=pad, nc=nc)
-    _compare(_decode(q[0], cache[0], bt, seq, cent, cfg, 2), _decode(q[0].float(), cache[0], bt, seq, cent, cfg, 2))
+    _compare(_decode(q[0], cache[0], bt, seq, cent, cfg, 64), _decode(q[0].float(), cache[0], bt, seq, cent, cfg, 64))
 
 
 def test_layers_in_several_launches():
     """64 query heads of 128: the workspace holds the rows of six layers, a call of eight is two launches."""
     cfg, cent, cache, bt, seq, q = _batch(128, 4, 4, 8, 8, [700, 90], layers=8)
-    o, m, l = _decode(q, cache, bt, seq, cent, cfg, 4)
+    o, m, l = _decode(q, cache, bt, seq, cent, cfg, 64)
     for i in range(8):
-        o1, m1, l1 = _decode(q[i], cache[i], bt, seq, cent, cfg, 4)
+        o1, m1, l1 = _decode(q[i], cache[i], bt, seq, cent, cfg, 64)
         assert np.array_equal(o[i], o1) and np.array_equal(m[i], m1) and np.array_equal(l[i], l1)
 
 
 def test_bad_block_poisons_its_rows_only():
     cfg, cent, cache, bt, seq, q = _batch(128, 4, 4, 8, 4, [500, 900, 130])
-    good, _, _ = _decode(q[0], cache[0], bt, seq, cent, cfg, 8)
+    good, _, _ = _decode(q[0], cache[0], bt, seq, cent, cfg, 64)
     bt[1, 20] = cache.shape[1] + 5
-    bt[2, 100 % bt.shape[1]] = -3 if bt.shape[1] > 9 else bt[2, 0]      # (beyond sequence 2's end: never read)
-    bad, _, _ = _decode(q[0], cache[0], bt, seq, cent, cfg, 8)
+    bt[2, 40] = -3                       # (beyond sequence 2's end: never read)
+    bad, _, _ = _decode(q[0], cache[0], bt, seq, cent, cfg, 64)
     assert np.isnan(bad[1]).all() and np.array_equal(bad[[0, 2]], good[[0, 2]])
 
 
 def test_captured_and_replayed():
     from fused_turboquant_b200 import tq_v1
     cfg, cent, cache, bt, seq, q = _batch(128, 4, 4, 8, 4, [500, 900, 130])
-    mid, out = torch.empty(3, 32, 8, 129, device="cuda"), torch.empty_like(q[0])
-    run = lambda: tq_v1.decode_attention(q[0], cache[0], bt, seq, cent, cfg, 128 ** -0.5, mid_o=mid, output=out)
+    mid, out = torch.empty(3, 32, 64, 129, device="cuda"), torch.empty_like(q[0])
+    run = lambda: tq_v1.decode_attention(q[0], cache[0], bt, seq, cent, cfg, 128 ** -0.5, num_kv_splits=64, mid_o=mid, output=out)
     run()
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g):

@@ -34,9 +34,9 @@
 
 namespace ftq {
 
-// mbar_wait that leaves the issue slots to the other warps between polls.  (Polls without a pause were a tenth of the
-// kernel's instructions; a poll with a suspend-time hint of 2 us slept that long whenever the copy had not arrived yet:
-// one sequence of 30000 tokens took 141 us.)
+// mbar_wait for the producer, with a pause between polls: it has time, the ring is some pages ahead, and its polls without one
+// were a tenth of the kernel's instructions.  (The warps that compute poll without: paused, FP8 keys of 16 x 4096 tokens took
+// 59 us instead of 54; suspended for up to 2 us by the poll itself, they slept that long whenever a copy was late.)
 __device__ __forceinline__ bool mbar_wait_idle(uint32_t bar, uint32_t parity) {
     for (int i = 0; i < kMbarSpinLimit; i++) {
         if (mbar_try_wait(bar, parity)) return true;
@@ -673,7 +673,7 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
         __syncwarp();
         if (subs == 1) return;
         if (lane == 0) mbar_arrive(folded + head * 8);
-        if (!stalled && !mbar_wait_idle(folded + head * 8, fold_par)) stalled = true;
+        if (!stalled && !mbar_wait(folded + head * 8, fold_par)) stalled = true;
         fold_par ^= 1u;
     };
     E e;
@@ -682,7 +682,7 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
     uint32_t par = 0;
     for (int pi = 0;; pi++) {
         const int ps = pi % kTqFlowPieces;
-        if (!mbar_wait_idle(pfull + ps * 8, (pi / kTqFlowPieces) & 1)) {
+        if (!mbar_wait(pfull + ps * 8, (pi / kTqFlowPieces) & 1)) {
             stalled = true;
             break;
         }
@@ -700,7 +700,7 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
         int seen = 0;
         (void)seen;
         for (int i = sub; i < n; i += subs) {
-            if (!stalled && !mbar_wait_idle(full + s * 8, par)) stalled = true;
+            if (!stalled && !mbar_wait(full + s * 8, par)) stalled = true;
             const uint2 slot = lds64(slot_table + s * 8);
             poison |= (slot.y & 1u) != 0u;
             const uint32_t page = slot.x + my_off;

@@ -12,7 +12,7 @@
 // page, with an online-softmax state of its own.  The warps of a head fold their states at the end of a
 // piece; nothing synchronises the whole CTA after the set-up.  (A warp that copied the slots of its own
 // pages word by word through registers spent 722 instructions a page and head on it: 32 x 8192 tokens of
-// 8 heads, 4-bit keys and values, took 182 us; this way 127.)
+// 8 heads, 4-bit keys and values, took 182 us; this way 122.)
 //
 // Work: the pages of a layer's (sequence, split) units lie in one line that is cut into equal shares, at most one per
 // SM, and the CTAs of the persistent grid take the shares of all layers in turn.  (Shares of single layers: a layer's
@@ -35,8 +35,8 @@
 namespace ftq {
 
 // mbar_wait for the producer, with a pause between polls: it has time, the ring is some pages ahead, and its polls without one
-// were a tenth of the kernel's instructions.  (The warps that compute poll without: paused, FP8 keys of 16 x 4096 tokens took
-// 59 us instead of 54; suspended for up to 2 us by the poll itself, they slept that long whenever a copy was late.)
+// were a tenth of the kernel's instructions.  (For the warps that compute a pause made no difference: 122.3 us with, 122.2
+// without for 32 x 8192 tokens.)
 __device__ __forceinline__ bool mbar_wait_idle(uint32_t bar, uint32_t parity) {
     for (int i = 0; i < kMbarSpinLimit; i++) {
         if (mbar_try_wait(bar, parity)) return true;

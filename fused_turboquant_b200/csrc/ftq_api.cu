@@ -1430,6 +1430,11 @@ extern "C" size_t ftq_tq_decode_workspace_bytes(int B, int Hq, int head_dim, int
     return tq_rows_offset(B) + tq_layer_rows(Hq, head_dim) * tq_layers_per_launch(Hq, head_dim, n_layers);
 }
 
+extern "C" int64_t ftq_tq_page_copy_bytes(int Hkv, int64_t stride_pos, int64_t stride_head, int head_dim, int key_bits, int value_bits) {
+    const int slot = ftq_tq_slot_bytes(head_dim, key_bits, value_bits);
+    return Hkv <= 0 || slot < 0 ? -1 : ftq::tq_page_copy_bytes(Hkv, stride_pos, stride_head, slot);
+}
+
 extern "C" int ftq_tq_decode_layers(const void* q, int q_dtype, int B, int Hq, int Hkv, int head_dim,
                                     const uint8_t* kv_cache, int64_t stride_block, int64_t stride_pos,
                                     int64_t stride_head, int block_size, const int32_t* block_table,
@@ -1596,6 +1601,7 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
     if (flow) {
         ftq::TqFlowParams fp{};
         fp.d = p;
+        fp.page_bytes = static_cast<uint32_t>(ftq::tq_page_copy_bytes(Hkv, stride_pos, stride_head, slot));
         fp.min_share = static_cast<uint32_t>(ftq::kTqFlowWarps / Hkv);
         fp.share = static_cast<uint32_t*>(workspace);
         fp.prefix = reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) + 256);

@@ -513,9 +513,16 @@ inline bool tq_flow_fits(int Hkv, int64_t stride_pos, int d, int kb, int vb, int
     }
     return true;
 }
+// Bytes of a page's copy: from its first slot to the last byte of the last slot's contents, rounded up to the 16 bytes that
+// a bulk copy goes by.  What lies behind the contents of the last slot belongs to the page only where the tensor says so (in a
+// view of wider slots it may be the end of the allocation); the last 16-byte unit always holds a byte of the page.
+inline int64_t tq_page_copy_bytes(int Hkv, int64_t stride_pos, int64_t stride_head, int64_t slot) {
+    return ((kPageTokens - 1) * stride_pos + (Hkv - 1) * stride_head + slot + 15) / 16 * 16;
+}
 struct TqFlowParams {
     TqDecodeParams d;
     uint32_t min_share;   // pages of a share, at least
+    uint32_t page_bytes;  // of a page's copy
     // workspace, read by the merge kernel: pages of a share (0: a wait ran out) and shares of a layer, pages of the
     // sequences before b over all splits, row blocks
     uint32_t* share;      // [2]

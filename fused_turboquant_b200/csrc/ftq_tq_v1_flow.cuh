@@ -485,8 +485,8 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
     float* xml = reinterpret_cast<float*>(gptr(take(kTqFlowWarps * 24 * 4, 128)));
     int* prefix = reinterpret_cast<int*>(gptr(take((kFlowMaxSeqs + 4) * 4, 128)));
     const uint32_t xarea = take(kTqFlowWarps * XSLOT, 128);
-    const uint32_t ts = static_cast<uint32_t>(p.stride_pos), bytes = kPageTokens * ts;
-    const uint32_t pitch = (bytes + 127) & ~127u;
+    const uint32_t ts = static_cast<uint32_t>(p.stride_pos), bytes = f.page_bytes;
+    const uint32_t pitch = (kPageTokens * ts + 127) & ~127u;
     free0 = (free0 + 127u) & ~127u;
     free1 = (free1 + 127u) & ~127u;
     const int n0 = end0 > free0 ? (end0 - free0) / pitch : 0;

@@ -77,6 +77,17 @@ def test_block_sizes_padding_and_long_pieces(bs, pad, nc):
     _compare(_decode(q[0], cache[0], bt, seq, cent, cfg, 64), _decode(q[0].float(), cache[0], bt, seq, cent, cfg, 64))
 
 
+def test_slots_at_an_offset_of_wider_ones():
+    """A view whose last page ends 16 bytes behind what a copy of whole slots would read.  (Compared with slots of the same
+    pitch, so that the order of the sums is the same.)"""
+    cfg, cent, cache, bt, seq, q = _batch(128, 4, 4, 8, 4, [1500, 16, 900], pad=26)   # slots of 160
+    slot = cfg.slot_size_aligned
+    view = torch.zeros_like(cache[0])[..., 16:16 + slot]
+    view.copy_(cache[0, ..., :slot])
+    for got, want in zip(_decode(q[0], view, bt, seq, cent, cfg, 64), _decode(q[0], cache[0], bt, seq, cent, cfg, 64)):
+        np.testing.assert_array_equal(got, want)
+
+
 def test_layers_in_several_launches():
     """64 query heads of 128: the workspace holds the rows of six layers, a call of eight is two launches."""
     cfg, cent, cache, bt, seq, q = _batch(128, 4, 4, 8, 8, [700, 90], layers=8)

@@ -78,3 +78,17 @@ def test_cpu_tensors_are_refused():
     with pytest.raises(RuntimeError):
         tq_v1.decode_attention(k, cache, torch.zeros(2, 1, dtype=torch.int32),
                                torch.ones(2, dtype=torch.int32), torch.linspace(-1, 1, 16), cfg, 0.1)
+
+
+@pytest.mark.parametrize("d,kb,vb", [(128, 4, 4), (128, 3, 4), (64, 3, 3), (64, 4, 2), (128, 8, 4), (64, 8, 3)])
+@pytest.mark.parametrize("hkv", [8, 16])
+def test_a_page_copy_ends_with_the_last_slots_contents(d, kb, vb, hkv):
+    """Slots that are a view of wider ones: the last page's copy ends in the 16-byte unit (no allocation ends inside one) that
+    holds the last byte of the cache's last slot, whatever lies behind it."""
+    from fused_turboquant_b200 import _lib
+    lib, slot = _lib.load(), tq_v1.TurboQuantSlotConfig(d, kb, vb).slot_size_aligned
+    for pad in (0, 2, 14, 16, 26, 64):
+        cache = torch.empty(3, 16, hkv, slot + pad, dtype=torch.uint8)[..., :slot]
+        last = sum((n - 1) * s for n, s in zip(cache.shape[1:], cache.stride()[1:])) + 1   # bytes of a page up to its last
+        n = lib.ftq_tq_page_copy_bytes(hkv, cache.stride(1), cache.stride(2), d, kb, vb)
+        assert n % 16 == 0 and last <= n < last + 16

@@ -93,9 +93,7 @@ __device__ __forceinline__ void tq_emit_columns(uint32_t (&w)[NCH], uint8_t* dst
 // (not inlined: hardly ever taken)
 template <int D, int KB, int VB, typename T, bool ROTV>
 __device__ __noinline__ void tq_store2_plain(const TqStoreParams& p, int64_t n_vec, int64_t base, int lane) {
-    tq_store_octets<D, KB, VB, T, ROTV, false, false>(p, n_vec, base, lane, nullptr);
-    __syncwarp();
-    tq_store_octets<D, KB, VB, T, ROTV, false, false>(p, n_vec, base + 4, lane, nullptr);
+    tq_store_octets<D, KB, VB, T, ROTV, false, false>(p, n_vec, base, 4, base + 8, lane, nullptr);
 }
 
 template <int D, int KB, int VB, typename T, bool ROTV>

@@ -44,6 +44,8 @@ UNITS = []
 for _d in (256, 128, 64):
     UNITS.append(("ftq_tq_v1_inst.cu", f"tq_v1_store_d{_d}", [f"-DFTQ_D={_d}", "-DFTQ_TQ_PART=0"]))
     UNITS.append(("ftq_tq_v1_inst.cu", f"tq_v1_decode_d{_d}", [f"-DFTQ_D={_d}", "-DFTQ_TQ_PART=1"]))
+    if _d != 256:   # (not for that size)
+        UNITS.append(("ftq_tq_v1_inst.cu", f"tq_v1_flow_d{_d}", [f"-DFTQ_D={_d}", "-DFTQ_TQ_PART=2"]))
 for _d in (256, 128, 64):
     UNITS.append(("ftq_attn_inst.cu", f"attn_d{_d}", [f"-DFTQ_D={_d}"]))
     UNITS.append(("ftq_attn_chunk_inst.cu", f"attn_chunk_d{_d}", [f"-DFTQ_D={_d}"]))

@@ -1636,7 +1636,7 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
                 mp.prefix_out = static_cast<const uint8_t*>(prefix_out) + row0 * head_dim * size_of(prefix_dtype);
                 mp.prefix_lse = prefix_lse + row0;
             }
-            e = merge();
+            e = head_dim == 64 ? ftq::launch_tq_join_d64(out_dtype, mp, st) : ftq::launch_tq_join_d128(out_dtype, mp, st);
             if (e != cudaSuccess) return cuda_fail(e, "tq_decode merge launch");
         }
         return FTQ_OK;

@@ -1064,109 +1064,4 @@ tq_merge_kernel(const TqMergeParams p) {
     tq_finish_row<D, OT, OCTETS>(p, out, lse_out, row, a, l, M, lane, at < n_rows);
 }
 
-// The same for stage 1 with equal shares, where a split that a share's end cut lies in the workspace in pieces: they
-// are put together, written to mid_o and merged.  Two warps per row, an octet per split: the latency of its loads bounds
-// it (an octet that went through two splits one after the other, most of them cut, took 25 us for 1024 rows).
-template <int D, typename OT>
-__global__ void __launch_bounds__(128)
-tq_join_kernel(const __grid_constant__ TqMergeParams p) {
-    constexpr int E = D / kOctet;
-    __shared__ float part[2][kOctet][E + 2];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 7;
-    const int which = warp >> 1, oct = 4 * (warp & 1) + (lane >> 3);
-    const int64_t at = static_cast<int64_t>(blockIdx.x) * 2 + which;
-    const int64_t row = at < p.n_rows ? at : p.n_rows - 1;
-    const uint32_t r = fast_div(static_cast<uint32_t>(row), p.div_hq);   // (layer, sequence)
-    const int h = static_cast<int>(static_cast<uint32_t>(row) - r * p.Hq);
-    const uint32_t layer = fast_div(r, p.div_bseq);
-    const int b = static_cast<int>(r - layer * p.B_seq);
-    let_next_kernel_start();
-    after_previous_kernel();   // stage 1 is complete
-    const uint32_t share = p.share[0];
-    const int64_t shares0 = static_cast<int64_t>(layer) * p.share[1];
-    const int len = p.seq_lens[b], start = p.kv_start ? p.kv_start[b] : 0;
-    uint32_t pos = static_cast<uint32_t>(p.page_prefix[b]);
-    float M = -INFINITY, l = 0.f, a[E];
-#pragma unroll
-    for (int i = 0; i < E; i++) a[i] = 0.f;
-    for (int s = 0; s < p.splits; s++) {
-        const uint32_t n = tq_range_pages(tq_split_range(len, start, p.splits, s));
-        if ((s & 7) == oct && n > 0 && share > 0) {
-            const uint32_t c0 = pos / share, c1 = (pos + n - 1) / share;
-            float* mid = p.mid_out + (row * p.splits + s) * (D + 1);
-            float x[E], ms;
-            if (c0 == c1) {
-                ms = __ldcg(mid + D);
-#pragma unroll
-                for (int i = 0; i < E; i++) x[i] = __ldcg(mid + load_coord(t, i));
-            } else {
-                // (row block 0 is the piece the share starts with, 1 its last one)
-                auto piece = [&](uint32_t c) {
-                    return p.rows + ((2 * (shares0 + c) + (c * share >= pos ? 0 : 1)) * p.Hq + h) * (D + 2);
-                };
-                float top = -INFINITY, ls = 0.f;
-#pragma unroll 4
-                for (uint32_t c = c0; c <= c1; c++) top = fmaxf(top, __ldcg(piece(c) + D));
-#pragma unroll
-                for (int i = 0; i < E; i++) x[i] = 0.f;
-#pragma unroll 2
-                for (uint32_t c = c0; c <= c1; c++) {
-                    const float* src = piece(c);
-                    float y[E];
-#pragma unroll
-                    for (int i = 0; i < E; i++) y[i] = __ldcg(src + load_coord(t, i));
-                    const float f = fast_exp2(__ldcg(src + D) - top);
-                    ls = fmaf(__ldcg(src + D + 1), f, ls);   // (a NaN stays one)
-#pragma unroll
-                    for (int i = 0; i < E; i++) x[i] = fmaf(y[i], f, x[i]);
-                }
-                const float inv = 1.f / ls;
-                ms = top * 0.6931471805599453f + logf(ls);
-#pragma unroll
-                for (int i = 0; i < E; i++) {
-                    x[i] *= inv;
-                    mid[load_coord(t, i)] = x[i];
-                }
-                if (t == 0) mid[D] = ms;
-            }
-            const float m_new = fmaxf(M, ms);
-            const float f0 = __expf(M - m_new), f = __expf(ms - m_new);
-            l = fmaf(l, f0, f);
-#pragma unroll
-            for (int i = 0; i < E; i++) a[i] = fmaf(a[i], f0, x[i] * f);
-            M = m_new;
-        }
-        pos += n;
-    }
-    if (share == 0) {
-        l = __int_as_float(0x7fc00000);
-#pragma unroll
-        for (int i = 0; i < E; i++) a[i] = l;
-    }
-    // the octets of a warp, then the two warps
-    auto join = [&](float m_o, float l_o, auto other) {
-        const float m_new = fmaxf(M, m_o);
-        const float f0 = M == -INFINITY && l == 0.f ? 0.f : __expf(M - m_new);
-        const float f1 = m_o == -INFINITY && l_o == 0.f ? 0.f : __expf(m_o - m_new);
-        l = l * f0 + l_o * f1;
-#pragma unroll
-        for (int i = 0; i < E; i++) a[i] = a[i] * f0 + other(i) * f1;
-        M = m_new;
-    };
-#pragma unroll
-    for (int m = 8; m < 32; m <<= 1) {
-        const float m_o = __shfl_xor_sync(0xffffffffu, M, m), l_o = __shfl_xor_sync(0xffffffffu, l, m);
-        join(m_o, l_o, [&](int i) { return __shfl_xor_sync(0xffffffffu, a[i], m); });
-    }
-    if ((warp & 1) && lane < kOctet) {
-#pragma unroll
-        for (int i = 0; i < E; i++) part[which][t][i] = a[i];
-        part[which][t][E] = M;
-        part[which][t][E + 1] = l;
-    }
-    __syncthreads();
-    if (warp & 1) return;
-    join(part[which][t][E], part[which][t][E + 1], [&](int i) { return part[which][t][i]; });
-    tq_finish_row<D, OT, 4>(p, static_cast<OT*>(p.out), p.lse, row, a, l, M, lane, at < p.n_rows);
-}
 }  // namespace ftq

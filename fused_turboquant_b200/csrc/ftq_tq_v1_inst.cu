@@ -1,6 +1,6 @@
 // Instantiates the vLLM-v1 slot-format kernels for one head_dim (FTQ_D).  FTQ_TQ_PART selects
-// what this object holds, so that the halves compile in parallel: 0 = the store kernels,
-// 1 = the decode kernels (fp32 split, tensor-core split, merge); undefined = both.
+// what this object holds, so that the parts compile in parallel: 0 = the store kernels, 1 = the decode
+// kernels (fp32 split, tensor-core split, merge), 2 = decode by shares of pages and its merge; undefined = all.
 #include "ftq_launch.h"
 #include "ftq_tq_v1.cuh"
 #include "ftq_tq_v1_launch.h"
@@ -10,11 +10,17 @@
 #if !defined(FTQ_TQ_PART) || FTQ_TQ_PART == 1
 #define FTQ_TQ_DECODE 1
 #endif
+#if !defined(FTQ_TQ_PART) || FTQ_TQ_PART == 2
+#define FTQ_TQ_FLOW 1
+#endif
 #ifdef FTQ_TQ_STORE
 #include "ftq_tq_v1_store2.cuh"
 #endif
-#if FTQ_D != 256 && defined(FTQ_TQ_DECODE)
+#if FTQ_D != 256 && defined(FTQ_TQ_FLOW)
 #include "ftq_tq_v1_flow.cuh"
+#include "ftq_tq_v1_fp8.cuh"
+#endif
+#if FTQ_D != 256 && defined(FTQ_TQ_DECODE)
 #include "ftq_tq_v1_fp8.cuh"
 #include "ftq_tq_v1_mma.cuh"
 #endif
@@ -242,6 +248,30 @@ cudaError_t FTQ_CAT(launch_tq_mma_d, FTQ_D)(int kb, int vb, int nh, const TqDeco
     return cudaErrorInvalidValue;
 }
 
+template <typename OT>
+static cudaError_t run_tq_merge(const TqMergeParams& p, cudaStream_t stream) {
+    // (as in the page-layout merge: a warp per row where there are few of them)
+    if (p.n_rows <= 0) return cudaSuccess;
+    const int octets = p.n_rows <= kWideMerge * sm_count() ? 4 : 1;
+    const unsigned grid = static_cast<unsigned>((p.n_rows * octets + 15) / 16);
+    if (octets == 4) tq_merge_kernel<FTQ_D, OT, 4><<<grid, 128, 0, stream>>>(p);
+    else tq_merge_kernel<FTQ_D, OT, 1><<<grid, 128, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t FTQ_CAT(launch_tq_merge_d, FTQ_D)(int out_dtype, const TqMergeParams& p,
+                                             cudaStream_t stream) {
+    switch (out_dtype) {
+        case kF32: return run_tq_merge<float>(p, stream);
+        case kF16: return run_tq_merge<__half>(p, stream);
+        case kBF16: return run_tq_merge<__nv_bfloat16>(p, stream);
+    }
+    return cudaErrorInvalidValue;
+}
+
+#endif  // FTQ_TQ_DECODE
+
+#ifdef FTQ_TQ_FLOW
 #if FTQ_D != 256
 template <class Engine>
 static cudaError_t flow_run(const TqFlowParams& p, cudaStream_t stream) {
@@ -270,6 +300,11 @@ static cudaError_t flow_by_vb(int vb, int nh, const TqFlowParams& p, cudaStream_
     }
     return cudaErrorInvalidValue;
 }
+// (launched while stage 1 drains: it waits for stage 1's end itself)
+template <typename OT>
+static cudaError_t join_run(const TqMergeParams& p, cudaStream_t stream) {
+    return launch_dependent(tq_join_kernel<FTQ_D, OT>, static_cast<unsigned>((p.n_rows + 1) / 2), 128, 0, stream, p);
+}
 #endif
 cudaError_t FTQ_CAT(launch_tq_flow_d, FTQ_D)(int kb, int vb, int nh, const TqFlowParams& p, cudaStream_t stream) {
 #if FTQ_D != 256
@@ -282,32 +317,16 @@ cudaError_t FTQ_CAT(launch_tq_flow_d, FTQ_D)(int kb, int vb, int nh, const TqFlo
 #endif
     return cudaErrorInvalidValue;
 }
-
-template <typename OT>
-static cudaError_t run_tq_merge(const TqMergeParams& p, cudaStream_t stream) {
-    // (as in the page-layout merge: a warp per row where there are few of them)
-    if (p.n_rows <= 0) return cudaSuccess;
-    const int octets = p.n_rows <= kWideMerge * sm_count() ? 4 : 1;
-    const unsigned grid = static_cast<unsigned>((p.n_rows * octets + 15) / 16);
-    if (p.share) {
-        // (launched while stage 1 drains: it waits for stage 1's end itself)
-        return launch_dependent(tq_join_kernel<FTQ_D, OT>, static_cast<unsigned>((p.n_rows + 1) / 2), 128, 0, stream, p);
-    }
-    if (octets == 4) tq_merge_kernel<FTQ_D, OT, 4><<<grid, 128, 0, stream>>>(p);
-    else tq_merge_kernel<FTQ_D, OT, 1><<<grid, 128, 0, stream>>>(p);
-    return cudaGetLastError();
-}
-
-cudaError_t FTQ_CAT(launch_tq_merge_d, FTQ_D)(int out_dtype, const TqMergeParams& p,
-                                             cudaStream_t stream) {
+cudaError_t FTQ_CAT(launch_tq_join_d, FTQ_D)(int out_dtype, const TqMergeParams& p, cudaStream_t stream) {
+#if FTQ_D != 256
     switch (out_dtype) {
-        case kF32: return run_tq_merge<float>(p, stream);
-        case kF16: return run_tq_merge<__half>(p, stream);
-        case kBF16: return run_tq_merge<__nv_bfloat16>(p, stream);
+        case kF32: return join_run<float>(p, stream);
+        case kF16: return join_run<__half>(p, stream);
+        case kBF16: return join_run<__nv_bfloat16>(p, stream);
     }
+#endif
     return cudaErrorInvalidValue;
 }
-
-#endif  // FTQ_TQ_DECODE
+#endif  // FTQ_TQ_FLOW
 
 }  // namespace ftq

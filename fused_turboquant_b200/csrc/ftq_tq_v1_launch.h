@@ -27,7 +27,8 @@ constexpr int kTqLloydMaxValues = 2;  // 4-bit values: Lloyd-Max codes against t
     cudaError_t launch_tq_fp8_d##DD(int vb, int nh, const TqDecodeParams& p, int n_items,           \
                                     cudaStream_t stream);                                         \
     cudaError_t launch_tq_flow_d##DD(int kb, int vb, int nh, const TqFlowParams& p, cudaStream_t stream); \
-    cudaError_t launch_tq_merge_d##DD(int out_dtype, const TqMergeParams& p, cudaStream_t stream);
+    cudaError_t launch_tq_merge_d##DD(int out_dtype, const TqMergeParams& p, cudaStream_t stream); \
+    cudaError_t launch_tq_join_d##DD(int out_dtype, const TqMergeParams& p, cudaStream_t stream);
 
 FTQ_DECLARE_TQ_LAUNCHERS(64)
 FTQ_DECLARE_TQ_LAUNCHERS(128)

@@ -1557,18 +1557,21 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
                      static_cast<int64_t>(B) * Hkv * num_kv_splits < (1ll << 31);
     // With a workspace, and pages of 16 slots that are one aligned span of memory for all KV heads, the kernel that
     // streams whole pages (ftq_tq_v1_flow.cuh): at most two warps a KV head, so that a piece is many pages for each of them,
-    // and about as many (sequence, split) units as SMs, so that few of them are cut into more than two pieces, which the
-    // merge goes through one after the other.  Measured, items : shares in us, 8 splits, 4-bit codes: 32 x 8192 tokens of 8
-    // heads 182 : 122, 2 x 100 x 700 ragged 414 : 181, FP8 keys 16 x 4096 72 : 58; but 1 x 30000 45 : 148, 8 x 2000
-    // ragged 39 : 83, 6 x 64 x 1500 of 2 heads 139 : 198, 3 x 5000 of one head 23 : 43.
+    // and from 128 (sequence, split) units of a layer on.  Measured over 175 batches of 128 to 1024 units of 8 and 16 heads, equal,
+    // ragged and with one long context among short ones, the shares took 0.32 to 1.02 of the items' time, 0.54 in the
+    // middle; in us, items : shares, 8 splits, 4-bit codes: 32 x 8192 tokens of 8 heads 182 : 116, 16 x 64 35 : 23, 64 of up to
+    // 16000 ragged 227 : 113, one of 16000 and 15 of 256 54 : 32, 2 x 64 in 64 splits 43 : 32.  The closest: 3-bit codes of groups of
+    // eight heads, 16 x 64, 33.1 : 33.8.  (Fewer units and fewer heads were slower by shares when their pieces were merged
+    // one after the other, and are not measured since.)
     const int64_t slot = ftq_tq_slot_bytes(head_dim, key_bits, value_bits);
+    const int piece_cost = ftq::tq_flow_piece_cost(Hkv);
     const bool flow = (mma || (fp8 && (head_dim == 64 || group <= 4))) && workspace && workspace_bytes >= ftq_tq_decode_workspace_bytes(B_seq, Hq, head_dim, n_layers) &&
                       aligned(workspace, 16) && aligned(kv_cache, 16) && stride_block % 16 == 0 &&
                       cache_layer_stride % 16 == 0 && block_size % 16 == 0 && stride_head >= slot &&
                       Hkv >= 8 && static_cast<int64_t>(B_seq) * num_kv_splits >= 128 &&
                       stride_pos == Hkv * stride_head && ftq::tq_flow_fits(Hkv, stride_pos, head_dim, key_bits, value_bits, group) &&
                       num_kv_splits <= ftq::kTqFlowSplits && B_seq <= ftq::kFlowMaxSeqs &&
-                      static_cast<int64_t>(B_seq) * (static_cast<int64_t>(max_blocks) * (block_size / 16) + num_kv_splits) < (1ll << 30) &&
+                      static_cast<int64_t>(B_seq) * (static_cast<int64_t>(max_blocks) * (block_size / 16) + num_kv_splits * (1 + piece_cost)) < (1ll << 30) &&
                       static_cast<int64_t>(B) * Hq < (1ll << 31);
     ftq::TqMergeParams mp{};
     mp.mid_o = mid_o;
@@ -1602,7 +1605,8 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
         ftq::TqFlowParams fp{};
         fp.d = p;
         fp.page_bytes = static_cast<uint32_t>(ftq::tq_page_copy_bytes(Hkv, stride_pos, stride_head, slot));
-        fp.min_share = static_cast<uint32_t>(ftq::kTqFlowWarps / Hkv);
+        fp.piece_cost = piece_cost;
+        fp.min_share = static_cast<uint32_t>(ftq::kTqFlowWarps / Hkv + piece_cost);
         fp.share = static_cast<uint32_t*>(workspace);
         fp.prefix = reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) + 256);
         fp.rows = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + tq_rows_offset(B_seq));
@@ -1613,6 +1617,7 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
         mp.kv_start = kv_start_offset;
         mp.Hq = Hq;
         mp.B_seq = p.B_seq;
+        mp.piece_cost = piece_cost;
         mp.div_hq = ftq::make_fastdiv(static_cast<uint32_t>(Hq));
         mp.div_bseq = p.div_bseq;
         const int nh = group <= 4 ? 1 : 2, per = tq_layers_per_launch(Hq, head_dim, n_layers);

@@ -489,6 +489,10 @@ constexpr int kTqFlowPieces = 4;                         // pieces announced ahe
 constexpr int kTqFlowBarriers = 2 * kTqFlowSlots + 2 * kTqFlowPieces + kTqFlowWarps;
 constexpr int kTqFlowSplits = 64;                        // (a CTA looks through a sequence's splits one by one)
 constexpr int kTqFlowSmem = 226 * 1024;
+// What a piece costs beside its pages, in pages of a CTA (four page visits of a warp; the rest of the line's unit is a page of all
+// heads, of which each head's warps take turns).  Over the batches named at the rule (ftq_api.cu) 0 / 2 / 3 / 4 / 6 visits
+// gave 1.16 / 1.41 / 1.48 / 1.50 / 1.50 times the items' speed, with a merge that was slower than it is now.
+inline int tq_flow_piece_cost(int Hkv) { return Hkv <= kTqFlowWarps ? 4 * (kTqFlowWarps / Hkv) : 4; }
 // FP8 keys: five to eight heads of 128 spill 280 bytes there and stay with the item kernel
 template <int D, int NH> constexpr bool kTqFlowFp8 = D == 64 || NH == 1;
 // a warp's exchange slot, which also holds its rotated queries
@@ -523,9 +527,10 @@ inline int64_t tq_page_copy_bytes(int Hkv, int64_t stride_pos, int64_t stride_he
 }
 struct TqFlowParams {
     TqDecodeParams d;
-    uint32_t min_share;   // pages of a share, at least
+    uint32_t min_share;   // places of a share, at least
+    int piece_cost;       // places that a unit takes beside those of its pages
     uint32_t page_bytes;  // of a page's copy
-    // workspace, read by the merge kernel: pages of a share (0: a wait ran out) and shares of a layer, pages of the
+    // workspace, read by the merge kernel: places of a share (0: a wait ran out) and shares of a layer, places of the
     // sequences before b over all splits, row blocks
     uint32_t* share;      // [2]
     int* prefix;          // [B_seq + 1]
@@ -958,7 +963,7 @@ struct TqMergeParams {
     float* mid_out;           // mid_o again: the rows of cut units are written here
     const int32_t* seq_lens;
     const int32_t* kv_start;  // nullable
-    int Hq, B_seq;
+    int Hq, B_seq, piece_cost;
     FastDiv div_hq, div_bseq;
 };
 

@@ -14,8 +14,11 @@
 // pages word by word through registers spent 722 instructions a page and head on it: 32 x 8192 tokens of
 // 8 heads, 4-bit keys and values, took 182 us; this way 122.)
 //
-// Work: the pages of a layer's (sequence, split) units lie in one line that is cut into equal shares, at most one per
-// SM, and the CTAs of the persistent grid take the shares of all layers in turn.  (Shares of single layers: a layer's
+// Work: the pages of a layer's (sequence, split) units lie in one line, each unit's behind piece_cost places without a page
+// (what a piece costs beside its pages: queries, the fold, the rows), and the line is cut into equal shares, at most one per
+// SM; a share's part of a unit that holds no page is no piece.  (Shares of pages alone gave the CTAs with the short contexts
+// of a ragged batch many times the pieces of the others: 64 sequences of 62 to 16000 tokens, 8 heads of 128, 4-bit codes, 242 us
+// and now 120 in this kernel.)  And the CTAs of the persistent grid take the shares of all layers in turn.  (Shares of single layers: a layer's
 // result does not depend on which others are in the call.)  A piece of a unit that a share's end cuts leaves its rows in the
 // workspace (two row blocks per share: its first and its last piece can be parts of units) and the merge kernel
 // puts them together; a whole unit's rows go to mid_o.  Splits keep their borders in tokens, pages the
@@ -507,10 +510,10 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
         mbar_init(pempty + tid * 8, kTqFlowWarps);
     }
     mbar_fence_init();
-    let_next_kernel_start();
     after_previous_kernel();
 
-    // ---- prefix sums of the sequences' pages over all splits (also for the merge kernel)
+    // ---- prefix sums of the sequences' places over all splits (also for the merge kernel)
+    const int cost = f.piece_cost;
     auto kv_start_of = [&](int b) { return p.kv_start ? p.kv_start[b] : 0; };
     if (warp == 0) {
         int carry = 0;
@@ -519,7 +522,10 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
             int x = 0;
             if (b < p.B_seq) {
                 const int len = p.seq_lens[b], start = kv_start_of(b);
-                for (int s = 0; s < p.splits; s++) x += tq_range_pages(tq_split_range(len, start, p.splits, s));
+                for (int s = 0; s < p.splits; s++) {
+                    const int n = tq_range_pages(tq_split_range(len, start, p.splits, s));
+                    x += n > 0 ? n + cost : 0;
+                }
             }
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -573,7 +579,7 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
             if (pi >= kTqFlowPieces) ok = mbar_wait_idle(pempty + ps * 8, ((pi / kTqFlowPieces) - 1) & 1) && ok;
             TqPiece pc{};
             int b = 0, layer = 0, page0 = 0;
-            if (ok && at < last) {
+            while (ok && at < last) {   // (until a part with pages)
                 layer = at / n_shares;
                 const uint32_t first = (at - layer * n_shares) * share, end = min(first + share, per_layer);
                 int r = pos;
@@ -590,20 +596,24 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
                 for (pc.sid = 0; pc.sid < p.splits; pc.sid++) {
                     rg = tq_split_range(len, start, p.splits, pc.sid);
                     n = tq_range_pages(rg);
-                    if (r < n) break;
-                    r -= n;
+                    const int places = n > 0 ? n + cost : 0;
+                    if (r < places) break;
+                    r -= places;
                 }
-                pc.n = min(n - r, static_cast<int>(end - pos));
+                const int stop = min(n + cost, r + static_cast<int>(end - pos));   // places [r, stop) of the unit
+                const int from = max(r - cost, 0);
+                pc.n = max(stop - cost, 0) - from;
                 pc.row = layer * p.B_seq + b;
-                pc.block = pc.n == n ? -1 : 2 * static_cast<int>(at) + (pos == first ? 0 : 1);
-                page0 = rg.t0 / kPageTokens + r;
+                pc.block = pc.n == n ? -1 : 2 * static_cast<int>(at) + (pos == first && r >= cost ? 0 : 1);
+                page0 = rg.t0 / kPageTokens + from;
                 pc.lo = rg.t0 - page0 * kPageTokens;
                 pc.hi = rg.t1 - page0 * kPageTokens;
-                pos += pc.n;
+                pos += stop - r;
                 if (pos == end) {
                     at++;
                     pos = at % n_shares * share;
                 }
+                if (pc.n > 0) break;
             }
             if (lane == 0) {
                 pieces[ps] = pc;
@@ -759,12 +769,17 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
 }
 
 // Stage 2 (tq_merge_kernel, ftq_tq_v1.cuh) where a split that a share's end cut lies in the workspace in pieces: they
-// are put together, written to mid_o and merged.  Two warps per row, an octet per split: the latency of its loads bounds
-// it (an octet that went through two splits one after the other, most of them cut, took 25 us for 1024 rows).
+// are put together, written to mid_o and merged.  Two warps per row, an octet per split, the eight octets side by side; the
+// pieces of a split kPieceBatch at a time (four took more registers: 4096 whole rows 23 us, 18 with two).  The latency of the
+// loads bounds it.  (While the octets of a warp took turns -- each looked through all splits for its own -- 64 rows of 64 splits
+// took 134 us, now 13; 512 rows of which 8 splits had 14 pieces each 74 us, now 12.)
+// Stage 1 does not let it start early: this kernel's CTAs would fill the first SMs that stage 1 leaves, many to an SM, and
+// wait there, and the few SMs then do all of its work (with one long context among short ones 55 us for the whole
+// call, 32 so).
 template <int D, typename OT>
 __global__ void __launch_bounds__(128)
 tq_join_kernel(const __grid_constant__ TqMergeParams p) {
-    constexpr int E = D / kOctet;
+    constexpr int E = D / kOctet, kPieceBatch = 2;
     __shared__ float part[2][kOctet][E + 2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 7;
     const int which = warp >> 1, oct = 4 * (warp & 1) + (lane >> 3);
@@ -776,61 +791,85 @@ tq_join_kernel(const __grid_constant__ TqMergeParams p) {
     const int b = static_cast<int>(r - layer * p.B_seq);
     let_next_kernel_start();
     after_previous_kernel();   // stage 1 is complete
-    const uint32_t share = p.share[0];
-    const int64_t shares0 = static_cast<int64_t>(layer) * p.share[1];
+    const uint32_t share = __ldcg(p.share);
+    const int64_t shares0 = static_cast<int64_t>(layer) * __ldcg(p.share + 1);
     const int len = p.seq_lens[b], start = p.kv_start ? p.kv_start[b] : 0;
-    uint32_t pos = static_cast<uint32_t>(p.page_prefix[b]);
+    uint32_t pos = static_cast<uint32_t>(__ldcg(p.page_prefix + b));
     float M = -INFINITY, l = 0.f, a[E];
 #pragma unroll
     for (int i = 0; i < E; i++) a[i] = 0.f;
-    for (int s = 0; s < p.splits; s++) {
-        const uint32_t n = tq_range_pages(tq_split_range(len, start, p.splits, s));
-        if ((s & 7) == oct && n > 0 && share > 0) {
-            const uint32_t c0 = pos / share, c1 = (pos + n - 1) / share;
-            float* mid = p.mid_out + (row * p.splits + s) * (D + 1);
-            float x[E], ms;
-            if (c0 == c1) {
-                ms = __ldcg(mid + D);
+    for (int s0 = 0; s0 < p.splits; s0 += kOctet) {
+        // lane t: pages of split s0 + t; its place in the line
+        const uint32_t pages = s0 + t < p.splits ? tq_range_pages(tq_split_range(len, start, p.splits, s0 + t)) : 0;
+        uint32_t upto = pages > 0 ? pages + p.piece_cost : 0;
 #pragma unroll
-                for (int i = 0; i < E; i++) x[i] = __ldcg(mid + load_coord(t, i));
-            } else {
-                // (row block 0 is the piece the share starts with, 1 its last one)
-                auto piece = [&](uint32_t c) {
-                    return p.rows + ((2 * (shares0 + c) + (c * share >= pos ? 0 : 1)) * p.Hq + h) * (D + 2);
-                };
-                float top = -INFINITY, ls = 0.f;
-#pragma unroll 4
-                for (uint32_t c = c0; c <= c1; c++) top = fmaxf(top, __ldcg(piece(c) + D));
-#pragma unroll
-                for (int i = 0; i < E; i++) x[i] = 0.f;
-#pragma unroll 2
-                for (uint32_t c = c0; c <= c1; c++) {
-                    const float* src = piece(c);
-                    float y[E];
-#pragma unroll
-                    for (int i = 0; i < E; i++) y[i] = __ldcg(src + load_coord(t, i));
-                    const float f = fast_exp2(__ldcg(src + D) - top);
-                    ls = fmaf(__ldcg(src + D + 1), f, ls);   // (a NaN stays one)
-#pragma unroll
-                    for (int i = 0; i < E; i++) x[i] = fmaf(y[i], f, x[i]);
-                }
-                const float inv = 1.f / ls;
-                ms = top * 0.6931471805599453f + logf(ls);
-#pragma unroll
-                for (int i = 0; i < E; i++) {
-                    x[i] *= inv;
-                    mid[load_coord(t, i)] = x[i];
-                }
-                if (t == 0) mid[D] = ms;
-            }
-            const float m_new = fmaxf(M, ms);
-            const float f0 = __expf(M - m_new), f = __expf(ms - m_new);
-            l = fmaf(l, f0, f);
-#pragma unroll
-            for (int i = 0; i < E; i++) a[i] = fmaf(a[i], f0, x[i] * f);
-            M = m_new;
+        for (int m = 1; m < kOctet; m <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, upto, m, kOctet);
+            if (t >= m) upto += y;
         }
-        pos += n;
+        const uint32_t n = __shfl_sync(0xffffffffu, pages, oct, kOctet);
+        const uint32_t first = pos + __shfl_sync(0xffffffffu, upto, oct, kOctet) - n;
+        pos += __shfl_sync(0xffffffffu, upto, kOctet - 1, kOctet);
+        if (n == 0 || share == 0) continue;
+        const uint32_t c0 = first / share, c1 = (first + n - 1) / share;
+        const bool cut = c0 != c1;
+        float* const mid = p.mid_out + (row * p.splits + s0 + oct) * (D + 1);
+        // (row block 0 is the piece the share starts with, 1 its last one)
+        auto source = [&](uint32_t c) {
+            return cut ? p.rows + ((2 * (shares0 + c) + (c * share >= first ? 0 : 1)) * p.Hq + h) * (D + 2) : mid;
+        };
+        const float* src = source(c0);
+        float x[E], ms = __ldcg(src + D), ls = cut ? __ldcg(src + D + 1) : 1.f;   // (a NaN stays one)
+#pragma unroll
+        for (int i = 0; i < E; i++) x[i] = __ldcg(src + load_coord(t, i));
+        for (uint32_t c = c0 + 1; c <= c1; c += kPieceBatch) {
+            float y[kPieceBatch][E], my[kPieceBatch], ly[kPieceBatch];
+#pragma unroll
+            for (int k = 0; k < kPieceBatch; k++) {
+                my[k] = -INFINITY;
+                ly[k] = 0.f;
+#pragma unroll
+                for (int i = 0; i < E; i++) y[k][i] = 0.f;
+                if (c + k <= c1) {
+                    src = source(c + k);
+                    my[k] = __ldcg(src + D);
+                    ly[k] = __ldcg(src + D + 1);
+#pragma unroll
+                    for (int i = 0; i < E; i++) y[k][i] = __ldcg(src + load_coord(t, i));
+                }
+            }
+            float top = ms;
+#pragma unroll
+            for (int k = 0; k < kPieceBatch; k++) top = fmaxf(top, my[k]);
+            const float f0 = fast_exp2(ms - top);
+            ls *= f0;
+#pragma unroll
+            for (int i = 0; i < E; i++) x[i] *= f0;
+#pragma unroll
+            for (int k = 0; k < kPieceBatch; k++) {
+                const float f = fast_exp2(my[k] - top);
+                ls = fmaf(ly[k], f, ls);
+#pragma unroll
+                for (int i = 0; i < E; i++) x[i] = fmaf(y[k][i], f, x[i]);
+            }
+            ms = top;
+        }
+        if (cut) {
+            const float inv = 1.f / ls;
+            ms = ms * kLn2 + logf(ls);
+#pragma unroll
+            for (int i = 0; i < E; i++) {
+                x[i] *= inv;
+                mid[load_coord(t, i)] = x[i];
+            }
+            if (t == 0) mid[D] = ms;
+        }
+        const float m_new = fmaxf(M, ms);
+        const float f0 = __expf(M - m_new), f = __expf(ms - m_new);
+        l = fmaf(l, f0, f);
+#pragma unroll
+        for (int i = 0; i < E; i++) a[i] = fmaf(a[i], f0, x[i] * f);
+        M = m_new;
     }
     if (share == 0) {
         l = __int_as_float(0x7fc00000);

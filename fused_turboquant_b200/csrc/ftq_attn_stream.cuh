@@ -533,10 +533,22 @@ attn_stream_kernel(const AttnParams p, int n_items) {
     }
     __syncthreads();
 
+    // The two looked for their items at the same time: warp 0, whose item held no tokens, may have drawn the ticket
+    // behind the last item while warp 1 has one.  The stream then starts with item number 1, as if number 0 had been done,
+    // and the end that its buffer says is that of number 2.
+    const int s0 = ctl[kCtlItem + 0] >= n_items && ctl[kCtlItem + 1] < n_items ? 1 : 0;
+    if (s0) {   // (the same for all threads)
+        if (tid == 0) {
+            ctl[kCtlReady] = 2;
+            ctl[kCtlReduced] = 0;
+        }
+        __syncthreads();
+    }
+
     // ---- per-warp stream state (all warp-uniform)
-    int gseq = 0;                       // item the next page request belongs to
-    int cseq = 0;                       // item number the arithmetic state belongs to
-    bool g_end = ctl[kCtlItem + 0] >= n_items;
+    int gseq = s0;                      // item the next page request belongs to
+    int cseq = s0;                      // item number the arithmetic state belongs to
+    bool g_end = ctl[kCtlItem + s0] >= n_items;
     bool deferred = false;              // a request was handed back: later ones must not overtake it
 
     // Pages of an item are dealt round-robin, except that the two service warps (warp 0 folds
@@ -554,7 +566,7 @@ attn_stream_kernel(const AttnParams p, int n_items) {
     bool test_drop = blockIdx.x == 0 && warp == 5;   // (see kMbarSpinLimit)
 #endif
     int g_next = g_first;                                   // next page of item gseq for this warp
-    int g_lim = g_end ? 0 : ctl[kCtlPages + 0];             // its page count (0: nothing to take)
+    int g_lim = g_end ? 0 : ctl[kCtlPages + s0];            // its page count (0: nothing to take)
     // request the next page of the stream into ring buffer rb; returns its index within item
     // gseq, -1 at the end of the stream, -2 when the request is handed back
     auto grab = [&](int rb) {
@@ -603,9 +615,9 @@ attn_stream_kernel(const AttnParams p, int n_items) {
     };
 
     // ---- per-item arithmetic state
-    int ntok_item = ctl[kCtlTokens + 0];
+    int ntok_item = ctl[kCtlTokens + s0];
     uint32_t qb[S::QSMEM ? 1 : NH][S::QSMEM ? 1 : NKB][2];
-    uint32_t qf_item = qfrag;  // fragment base of the current item (QSMEM)
+    uint32_t qf_item = qfrag + s0 * S::QFRAG_BYTES;  // fragment base of the current item (QSMEM)
     float m_run[NH], l_run[NH], oacc[NH][NMT][4];
     auto load_ctx = [&](int seq) {
         const int buf = seq & 1;

@@ -56,6 +56,8 @@ SIGNATURES = {
                                   _vp, _i, _i, _i, _i, _i, _fp, _c.c_float, _i, _vp, _vp, _i, _vp,
                                   _vp, _i, _vp, _i, _i64, _i64, _vp]),
     "ftq_tq_decode_workspace_bytes": (_sz, [_i, _i, _i, _i]),
+    "ftq_tq_decode_layers_workspace_bytes": (_sz, [_i, _i, _i, _i, _i, _vp, _i64, _i64, _i64, _i, _i, _i, _i,
+                                                   _i, _i, _i, _i64]),
     "ftq_tq_page_copy_bytes": (_i64, [_i, _i64, _i64, _i, _i, _i]),
     "ftq_tq_decode_layers_ws": (_i, [_vp, _i, _i, _i, _i, _i, _vp, _i64, _i64, _i64, _i, _vp, _i, _vp,
                                      _vp, _i, _i, _i, _i, _i, _fp, _c.c_float, _i, _vp, _vp, _i, _vp,

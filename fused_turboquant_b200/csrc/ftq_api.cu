@@ -1430,6 +1430,62 @@ extern "C" size_t ftq_tq_decode_workspace_bytes(int B, int Hq, int head_dim, int
     return tq_rows_offset(B) + tq_layer_rows(Hq, head_dim) * tq_layers_per_launch(Hq, head_dim, n_layers);
 }
 
+// Which stage 1 a slot-format decode takes: by tensor cores (mma: Lloyd-Max key codes, fp8: FP8 keys), and of those by shares of
+// pages where there is a workspace (flow).
+struct TqRoute { bool mma, fp8, flow; };
+static TqRoute tq_decode_route(int q_dtype, int B_seq, int Hq, int Hkv, int head_dim, const uint8_t* kv_cache, int64_t stride_block,
+                               int64_t stride_pos, int64_t stride_head, int block_size, int max_blocks, int key_bits,
+                               int value_bits, bool lloyd, int splits, int n_layers, int64_t cache_layer_stride) {
+    TqRoute r{};
+    const int group = Hq / Hkv;
+    const int64_t B = static_cast<int64_t>(B_seq) * n_layers;
+    // 16-bit queries with a GQA group of at most 8 take the tensor-core kernel (head_dim 64 / 128,
+    // key and uniform value codes of 2..4 bits); everything else the fp32 kernel
+    // (its copy loop reads whole aligned words: a cache that starts on an odd 2-byte boundary -- a
+    // view at an offset -- stays on the fp32 kernel, which reads 2-byte pieces)
+    r.mma = q_dtype != FTQ_F32 && group <= 8 && key_bits >= 2 && key_bits <= 4 && value_bits >= 2 &&
+                     value_bits != 8 && head_dim != 256 && aligned(kv_cache, 4) &&
+                     !lloyd;
+    // FP8 keys under the same conditions take a tensor-core kernel of fp32 precision; its copies are
+    // 4-byte words, so every slot has to start on one
+    const int64_t strides = stride_block | stride_pos | stride_head | cache_layer_stride;
+    r.fp8 = key_bits == 8 && q_dtype != FTQ_F32 && group <= 8 && value_bits >= 2 && value_bits <= 4 &&
+                     head_dim != 256 && aligned(kv_cache, 4) && strides % 4 == 0 &&
+                     static_cast<int64_t>(B) * Hkv * splits < (1ll << 31);
+    // With a workspace, and pages of 16 slots that are one aligned span of memory for all KV heads, the kernel that
+    // streams whole pages (ftq_tq_v1_flow.cuh): at most two warps a KV head, so that a piece is many pages for each of them,
+    // and from 128 (sequence, split) units of a layer on.  Measured over 175 batches of 128 to 1024 units of 8 and 16 heads, equal,
+    // ragged and with one long context among short ones, the shares took 0.32 to 1.02 of the items' time, 0.54 in the
+    // middle; in us, items : shares, 8 splits, 4-bit codes: 32 x 8192 tokens of 8 heads 182 : 116, 16 x 64 35 : 23, 64 of up to
+    // 16000 ragged 227 : 113, one of 16000 and 15 of 256 54 : 32, 2 x 64 in 64 splits 43 : 32.  The closest: 3-bit codes of groups of
+    // eight heads, 16 x 64, 33.1 : 33.8.  (Fewer units and fewer heads were slower by shares when their pieces were merged
+    // one after the other, and are not measured since.)
+    const int64_t slot = ftq_tq_slot_bytes(head_dim, key_bits, value_bits);
+    const int piece_cost = ftq::tq_flow_piece_cost(Hkv);
+    r.flow = (r.mma || (r.fp8 && (head_dim == 64 || group <= 4))) && aligned(kv_cache, 16) && stride_block % 16 == 0 &&
+             cache_layer_stride % 16 == 0 && block_size % 16 == 0 && stride_head >= slot && Hkv >= 8 &&
+             static_cast<int64_t>(B_seq) * splits >= 128 && stride_pos == Hkv * stride_head &&
+             ftq::tq_flow_fits(Hkv, stride_pos, head_dim, key_bits, value_bits, group) && splits <= ftq::kTqFlowSplits &&
+             B_seq <= ftq::kFlowMaxSeqs &&
+             static_cast<int64_t>(B_seq) * (static_cast<int64_t>(max_blocks) * (block_size / 16) + splits * (1 + piece_cost)) < (1ll << 30) &&
+             B * Hq < (1ll << 31);
+    return r;
+}
+
+extern "C" size_t ftq_tq_decode_layers_workspace_bytes(int q_dtype, int B, int Hq, int Hkv, int head_dim, const uint8_t* kv_cache,
+                                                       int64_t stride_block, int64_t stride_pos, int64_t stride_head,
+                                                       int block_size, int max_blocks, int key_bits, int value_bits,
+                                                       int value_lloyd_max, int num_kv_splits, int n_layers,
+                                                       int64_t cache_layer_stride) {
+    if (B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || n_layers <= 0 || !dim_ok(head_dim) || !dtype_ok(q_dtype) || block_size <= 0 ||
+        max_blocks <= 0 || num_kv_splits <= 0 || !tq_bits_ok(key_bits, value_bits))
+        return 0;
+    const bool flow = tq_decode_route(q_dtype, B, Hq, Hkv, head_dim, kv_cache, stride_block, stride_pos, stride_head, block_size,
+                                      max_blocks, key_bits, value_bits, value_lloyd_max && value_bits == 4, num_kv_splits,
+                                      n_layers, cache_layer_stride).flow;
+    return flow ? ftq_tq_decode_workspace_bytes(B, Hq, head_dim, n_layers) : 0;
+}
+
 extern "C" int64_t ftq_tq_page_copy_bytes(int Hkv, int64_t stride_pos, int64_t stride_head, int head_dim, int key_bits, int value_bits) {
     const int slot = ftq_tq_slot_bytes(head_dim, key_bits, value_bits);
     return Hkv <= 0 || slot < 0 ? -1 : ftq::tq_page_copy_bytes(Hkv, stride_pos, stride_head, slot);
@@ -1541,38 +1597,15 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
     p.mid_o = mid_o;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaErrorInvalidValue;
-    // 16-bit queries with a GQA group of at most 8 take the tensor-core kernel (head_dim 64 / 128,
-    // key and uniform value codes of 2..4 bits); everything else the fp32 kernel
     const int group = Hq / Hkv;
-    // (its copy loop reads whole aligned words: a cache that starts on an odd 2-byte boundary -- a
-    // view at an offset -- stays on the fp32 kernel, which reads 2-byte pieces)
-    const bool mma = q_dtype != FTQ_F32 && group <= 8 && key_bits >= 2 && key_bits <= 4 && value_bits >= 2 &&
-                     value_bits != 8 && head_dim != 256 && aligned(kv_cache, 4) &&
-                     !p.value_lloyd_max;
-    // FP8 keys under the same conditions take a tensor-core kernel of fp32 precision; its copies are
-    // 4-byte words, so every slot has to start on one
-    const int64_t strides = stride_block | stride_pos | stride_head | cache_layer_stride;
-    const bool fp8 = key_fp8 && q_dtype != FTQ_F32 && group <= 8 && value_bits >= 2 && value_bits <= 4 &&
-                     head_dim != 256 && aligned(kv_cache, 4) && strides % 4 == 0 &&
-                     static_cast<int64_t>(B) * Hkv * num_kv_splits < (1ll << 31);
-    // With a workspace, and pages of 16 slots that are one aligned span of memory for all KV heads, the kernel that
-    // streams whole pages (ftq_tq_v1_flow.cuh): at most two warps a KV head, so that a piece is many pages for each of them,
-    // and from 128 (sequence, split) units of a layer on.  Measured over 175 batches of 128 to 1024 units of 8 and 16 heads, equal,
-    // ragged and with one long context among short ones, the shares took 0.32 to 1.02 of the items' time, 0.54 in the
-    // middle; in us, items : shares, 8 splits, 4-bit codes: 32 x 8192 tokens of 8 heads 182 : 116, 16 x 64 35 : 23, 64 of up to
-    // 16000 ragged 227 : 113, one of 16000 and 15 of 256 54 : 32, 2 x 64 in 64 splits 43 : 32.  The closest: 3-bit codes of groups of
-    // eight heads, 16 x 64, 33.1 : 33.8.  (Fewer units and fewer heads were slower by shares when their pieces were merged
-    // one after the other, and are not measured since.)
+    const TqRoute route = tq_decode_route(q_dtype, B_seq, Hq, Hkv, head_dim, kv_cache, stride_block, stride_pos, stride_head,
+                                          block_size, max_blocks, key_bits, value_bits, p.value_lloyd_max, num_kv_splits,
+                                          n_layers, cache_layer_stride);
+    const bool mma = route.mma, fp8 = route.fp8;
+    const bool flow = route.flow && workspace && aligned(workspace, 16) &&
+                      workspace_bytes >= ftq_tq_decode_workspace_bytes(B_seq, Hq, head_dim, n_layers);
     const int64_t slot = ftq_tq_slot_bytes(head_dim, key_bits, value_bits);
     const int piece_cost = ftq::tq_flow_piece_cost(Hkv);
-    const bool flow = (mma || (fp8 && (head_dim == 64 || group <= 4))) && workspace && workspace_bytes >= ftq_tq_decode_workspace_bytes(B_seq, Hq, head_dim, n_layers) &&
-                      aligned(workspace, 16) && aligned(kv_cache, 16) && stride_block % 16 == 0 &&
-                      cache_layer_stride % 16 == 0 && block_size % 16 == 0 && stride_head >= slot &&
-                      Hkv >= 8 && static_cast<int64_t>(B_seq) * num_kv_splits >= 128 &&
-                      stride_pos == Hkv * stride_head && ftq::tq_flow_fits(Hkv, stride_pos, head_dim, key_bits, value_bits, group) &&
-                      num_kv_splits <= ftq::kTqFlowSplits && B_seq <= ftq::kFlowMaxSeqs &&
-                      static_cast<int64_t>(B_seq) * (static_cast<int64_t>(max_blocks) * (block_size / 16) + num_kv_splits * (1 + piece_cost)) < (1ll << 30) &&
-                      static_cast<int64_t>(B) * Hq < (1ll << 31);
     ftq::TqMergeParams mp{};
     mp.mid_o = mid_o;
     mp.out = out;

@@ -33,7 +33,7 @@ namespace {
 #define FTQ_BOUND(X)                                                                       \
     X(ftq_encode) X(ftq_decode_dense) X(ftq_rht) X(ftq_decode_workspace_bytes)             \
     X(ftq_flash_decode) X(ftq_paged_store) X(ftq_paged_decode_attn) X(ftq_tq_store_layers) \
-    X(ftq_tq_decode_layers_ws) X(ftq_tq_decode_workspace_bytes) X(ftq_paged_chunk_workspace_bytes) X(ftq_paged_chunk_attn)
+    X(ftq_tq_decode_layers_ws) X(ftq_tq_decode_layers_workspace_bytes) X(ftq_paged_chunk_workspace_bytes) X(ftq_paged_chunk_attn)
 struct Api {
 #define X(name) decltype(&::name) name = nullptr;
     FTQ_BOUND(X)
@@ -583,7 +583,7 @@ PyObject* tq_store(PyObject* const* a) {
 
 // tq_decode(query, kv_cache, block_table, seq_lens, kv_start_offset, centroids, key_bits, value_bits,
 //           norm_correction, v_rotate, v_lloyd_max, scale, num_kv_splits, mid_o, output, out_dtype,
-//           lse, prefix_output, prefix_lse, head_dim)
+//           lse, prefix_output, prefix_lse, head_dim, workspace)
 PyObject* tq_decode(PyObject* const* a) {
     at::Tensor q = supported(cuda_tensor(a[0], "query"));
     const bool layered = q.dim() == 4;
@@ -646,8 +646,22 @@ PyObject* tq_decode(PyObject* const* a) {
     const bool nc = as_bool(a[8]), rot = as_bool(a[9]), lloyd = as_bool(a[10]);
     const double scale = as_double(a[11]);
     void* st = stream_of(dev);
-    // (a tensor of the call's own: a captured graph keeps its memory, whatever later calls need)
-    const at::Tensor ws = empty({static_cast<int64_t>(api.ftq_tq_decode_workspace_bytes(B, hq, d, L))}, at::kByte, dev);
+    // Scratch of the kernel that streams whole pages: the caller's, or a tensor of the call's own (a captured graph keeps its
+    // memory, whatever later calls need).  Where that kernel is not taken nothing is allocated; without memory for it the
+    // item kernels run, which need none.
+    at::Tensor ws;
+    if (a[20] != Py_None) {
+        ws = tensor(a[20], "workspace");
+        if (ws.device() != dev || !ws.is_contiguous())
+            raise(PyExc_ValueError, "workspace must be a contiguous tensor on the query's device");
+    } else if (const size_t need = hq > 0 && c.hkv > 0 ? api.ftq_tq_decode_layers_workspace_bytes(
+                   dtype_code(q.scalar_type()), B, hq, c.hkv, d, ptr(c.t), c.sb, c.sp, c.sh, c.block_size, bt.size(1), kb, vb,
+                   lloyd, splits, L, c.layer_stride) : 0) {
+        try {
+            ws = empty({static_cast<int64_t>(need)}, at::kByte, dev);
+        } catch (const c10::OutOfMemoryError&) {
+        }
+    }
     int rc;
     {
         NoGil nogil;
@@ -657,8 +671,8 @@ PyObject* tq_decode(PyObject* const* a) {
             kb, vb, nc, rot, lloyd, cent.p, static_cast<float>(scale), splits, mptr<float>(mid),
             mptr<void>(out), oc, lse.defined() ? mptr<float>(lse) : nullptr,
             po.defined() ? ptr<void>(po) : nullptr, po.defined() ? dtype_code(po.scalar_type()) : 0,
-            pl.defined() ? ptr<float>(pl) : nullptr, L, c.layer_stride, c.num_blocks, mptr<void>(ws),
-            ws.numel(), st);
+            pl.defined() ? ptr<float>(pl) : nullptr, L, c.layer_stride, c.num_blocks,
+            ws.defined() ? mptr<void>(ws) : nullptr, ws.defined() ? ws.nbytes() : 0, st);
     }
     check(rc, "ftq_tq_decode_layers_ws");
     if (a[14] != Py_None) return Py_NewRef(a[14]);
@@ -706,7 +720,7 @@ PyMethodDef methods[] = {
     FTQ_ENTRY(rht, 3),
     FTQ_ENTRY(flash_decode, 15),
     FTQ_ENTRY(tq_store, 9),
-    FTQ_ENTRY(tq_decode, 20),
+    FTQ_ENTRY(tq_decode, 21),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_native", "Tensor-level host path over libftq_b200.so.",
                           -1, methods, nullptr, nullptr, nullptr, nullptr};

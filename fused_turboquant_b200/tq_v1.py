@@ -157,7 +157,8 @@ def decode_attention(query: torch.Tensor, kv_cache: torch.Tensor, block_table: t
                      output: torch.Tensor | None = None, lse: torch.Tensor | None = None,
                      out_dtype: torch.dtype | None = None, v_lloyd_max: bool = False,
                      prefix_output: torch.Tensor | None = None,
-                     prefix_lse: torch.Tensor | None = None) -> torch.Tensor:
+                     prefix_lse: torch.Tensor | None = None,
+                     workspace: torch.Tensor | None = None) -> torch.Tensor:
     """Decode attention of ``query`` ``[B, Hq, D]`` over the compressed cache; returns ``[B, Hq, D]``.
 
     All layers in one call: ``query`` ``[L, B, Hq, D]`` with ``kv_cache`` ``[L, num_blocks,
@@ -172,13 +173,21 @@ def decode_attention(query: torch.Tensor, kv_cache: torch.Tensor, block_table: t
 
     ``mid_o`` ``[B, Hq, num_kv_splits, D+1]`` fp32, ``output`` and ``lse`` ``[B, Hq]`` fp32 may be
     supplied (pre-allocated per layer, as the reference keeps them for CUDA-graph capture).
+    ``workspace``: scratch of ``decode_workspace_bytes(...)`` bytes that the call has to itself until it
+    has run; it is allocated per call where it is used and not given.  With a smaller one (an empty one), or
+    where there is no memory for it, the kernels that need none run, which can be slower.
     """
     _require_cuda(query, "query")
     _require_cuda(kv_cache, "kv_cache")
     return _lib.native().tq_decode(
         query, kv_cache, block_table, seq_lens, kv_start_offset, centroids, _key_bits(tq_config),
         tq_config.value_quant_bits, tq_config.norm_correction, v_rotate, v_lloyd_max, scale,
-        num_kv_splits, mid_o, output, out_dtype, lse, prefix_output, prefix_lse, tq_config.head_dim)
+        num_kv_splits, mid_o, output, out_dtype, lse, prefix_output, prefix_lse, tq_config.head_dim, workspace)
+
+
+def decode_workspace_bytes(batch: int, num_heads: int, head_dim: int, n_layers: int = 1) -> int:
+    """Bytes of ``workspace`` with which ``decode_attention`` allocates nothing, whatever the lengths."""
+    return _lib.load().ftq_tq_decode_workspace_bytes(batch, num_heads, head_dim, n_layers)
 
 
 def continuation_attention(query: torch.Tensor, kv_cache: torch.Tensor, block_table: torch.Tensor,

@@ -421,10 +421,17 @@ int ftq_tq_decode_layers(const void *q, int q_dtype, int B, int Hq, int Hkv, int
  * shares of pages instead of (sequence, head, split) items.  Same results in mid_o and out.  The
  * workspace (16-byte aligned, ftq_tq_decode_workspace_bytes(B, Hq, head_dim, n_layers) bytes, no initialisation)
  * belongs to the call until it has run; NULL or a smaller one: ftq_tq_decode_layers.
+ * ftq_tq_decode_layers_workspace_bytes: the same, 0 where the call would not use it.
  * ftq_tq_page_copy_bytes: what is read of 16 positions at once, from the first slot on (-1: bad arguments); it ends in the
  * 16-byte unit of the last slot's last byte.
  */
 size_t ftq_tq_decode_workspace_bytes(int B, int Hq, int head_dim, int n_layers);
+size_t ftq_tq_decode_layers_workspace_bytes(int q_dtype, int B, int Hq, int Hkv, int head_dim,
+                                            const uint8_t *kv_cache, int64_t stride_block,
+                                            int64_t stride_pos, int64_t stride_head, int block_size,
+                                            int max_blocks, int key_bits, int value_bits,
+                                            int value_lloyd_max, int num_kv_splits, int n_layers,
+                                            int64_t cache_layer_stride);
 int64_t ftq_tq_page_copy_bytes(int Hkv, int64_t stride_pos, int64_t stride_head, int head_dim,
                                int key_bits, int value_bits);
 int ftq_tq_decode_layers_ws(const void *q, int q_dtype, int B, int Hq, int Hkv, int head_dim,

@@ -1378,10 +1378,14 @@ extern "C" int ftq_tq_store_layers(const void* key, const void* value, int dtype
                       (value_lloyd_max && value_bits == 4 ? ftq::kTqLloydMaxValues : 0) |
                       (n_layers << 8);
     cudaError_t e = cudaErrorInvalidValue;
-    // Many 16-bit vectors: the kernel with two vectors per lane (from 2048 of K and V it has a warp's worth for every
-    // SM; below, its table and its long chains show).  Other widths, Lloyd-Max value codes, fp32 inputs and codebooks
-    // that the table does not take: the octet kernel.
-    const bool many = n_vec * n_layers >= 2048 && n_vec < (1ll << 31) && dtype != FTQ_F32 && !key_mse8 &&
+    // Many 16-bit vectors: the kernel with two vectors per lane.  Other widths, Lloyd-Max value codes, fp32 inputs and
+    // codebooks that the table does not take: the octet kernel.  Below the limits the table and the long chains of
+    // the two-vector kernel show; us, octets : pairs, called one after the other: heads of 128 and 4-bit codes 2048 vectors of K
+    // and V 8.2 : 4.2, 5120 8.2 : 5.3; heads of 64, 2048 6.1 : 4.3; heads of 256 (one CTA of 16 warps per SM) 4096 10.3 : 11.1,
+    // 5120 14.1 : 11.1, with FP8 keys 3200 8.2 : 9.6, 6144 10.3 : 9.7 and in a graph 8.2 : 9.5.  Layers of few vectors
+    // count together (256 layers of 8 vectors of 128: 7.6 : 4.2).
+    const int64_t many_from = head_dim < 256 ? 2048 : key_fp8 ? 12288 : 5120;
+    const bool many = n_vec * n_layers >= many_from && n_vec < (1ll << 31) && dtype != FTQ_F32 && !key_mse8 &&
                       (key_fp8 || key_bits == 3 || key_bits == 4) && (value_bits == 3 || value_bits == 4) &&
                       !(vmode & ftq::kTqLloydMaxValues) && table_takes_midpoints(p.midpoints, nmid);
     if (many) {

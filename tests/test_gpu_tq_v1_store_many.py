@@ -1,6 +1,6 @@
 """Slot-format store of many vectors (csrc/ftq_tq_v1_store2.cuh): byte for byte the cache that the oracle writes, and for
 what the oracle has no argument for (rotation in the kernel, NaN and infinities) the cache that the octet kernel writes, which
-calls of fewer than 2048 vectors take (tests/test_gpu_tq_v1.py pins that one)."""
+calls of fewer than 2048 vectors (heads of 256: 5120, FP8 keys 12288) take (tests/test_gpu_tq_v1.py pins that one)."""
 import numpy as np
 import pytest
 import torch
@@ -44,7 +44,8 @@ def _store(tq_v1, key, value, nb, cfg, mids, slots, rot, chunk):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_bytes(oracle, d, kb, vb, dtype):
     from fused_turboquant_b200 import TurboQuantMSE, tq_v1
-    n = 1031                             # 3093 vectors: neither whole warps of eight nor whole waves
+    # 3093 vectors, with heads of 256 12297: neither whole warps of eight nor whole waves
+    n = 1031 if d < 256 else 4099
     cfg = tq_v1.TurboQuantSlotConfig(d, kb, vb)
     _, mids = tq_v1.midpoints_of(TurboQuantMSE(d, bits=kb if kb < 8 else vb, device="cuda").quantizer.levels)
     nb = (n + BS - 1) // BS + 2

@@ -1459,10 +1459,10 @@ static TqRoute tq_decode_route(int q_dtype, int B_seq, int Hq, int Hkv, int head
     // With a workspace, and pages of 16 slots that are one aligned span of memory for all KV heads, the kernel that
     // streams whole pages (ftq_tq_v1_flow.cuh): at most two warps a KV head, so that a piece is many pages for each of them,
     // and from 128 (sequence, split) units of a layer on.  Measured over 175 batches of 128 to 1024 units of 8 and 16 heads, equal,
-    // ragged and with one long context among short ones, the shares took 0.32 to 1.02 of the items' time, 0.54 in the
+    // ragged and with one long context among short ones, the shares took 0.23 to 1.05 of the items' time, 0.56 in the
     // middle; in us, items : shares, 8 splits, 4-bit codes: 32 x 8192 tokens of 8 heads 182 : 116, 16 x 64 35 : 23, 64 of up to
-    // 16000 ragged 227 : 113, one of 16000 and 15 of 256 54 : 32, 2 x 64 in 64 splits 43 : 32.  The closest: 3-bit codes of groups of
-    // eight heads, 16 x 64, 33.1 : 33.8.  (Fewer units and fewer heads were slower by shares when their pieces were merged
+    // 16000 ragged 227 : 115, one of 16000 and 15 of 256 54 : 31, 2 x 64 in 64 splits 43 : 32.  The closest: 3-bit codes of groups of
+    // eight heads, 16 x 64, 33.1 : 34.6.  (Fewer units and fewer heads were slower by shares when their pieces were merged
     // one after the other, and are not measured since.)
     const int64_t slot = ftq_tq_slot_bytes(head_dim, key_bits, value_bits);
     const int piece_cost = ftq::tq_flow_piece_cost(Hkv);

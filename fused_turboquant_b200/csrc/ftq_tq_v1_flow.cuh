@@ -71,8 +71,12 @@ struct TqPiece {
 // A head's slots start 0 or 2 bytes behind a word boundary, all alike (a token's bytes are a multiple of 4).  4-bit rows are not
 // realigned: the codes are read as the aligned words hold them, the two halves of the words at the ends put together, and the coordinates of the query
 // fragments and of the output follow.
-// Values are code * scale + zero, codes centred (see ftq_tq_v1_mma.cuh); norm correction by the key
-// tile's product with itself.
+// Values are code * scale + zero, codes centred (see ftq_tq_v1_mma.cuh).
+// Precision: a rotated query is the sum of two fp16 numbers, hi + lo / 2^11, the lo parts in the columns that hold each of at
+// most four heads a second time, or by an MMA more for five to eight heads.  A warp has four times the pages of an item
+// kernel's warp under one reference maximum, and the weight of the token that sets it is the one that fp16 does not round; with
+// queries of one fp16 number the mean error against 64 bits was 1.03 to 1.08 of the item kernels' (splits of 128 to 1250 tokens),
+// with both it is 0.57 to 0.72 (32 x 2000 tokens 50.4 us and now 51.5).
 template <int D_, int KB, int VB, int NH_>
 struct TqCodes {
     static constexpr int D = D_, NH = NH_, HL = NH_, NKB = D / 16;
@@ -87,7 +91,9 @@ struct TqCodes {
     static constexpr float kCtr = VB == 4 ? 8.f : 0.5f * ((1 << VB) - 1);
 
     static constexpr int FLUSH = 0;
+    static constexpr float kLo = 2048.f, kInvLo = 1.f / 2048.f;
     uint32_t qb[NKB][2];
+    uint32_t q_lo;        // NH = 2: where the lane's lo parts are
     float m_run[HL], l_run[HL], z_run[HL], oacc[OL / 4][4];
     float s_ref, up;    // largest value scale so far as a power of two; weights are rounded times up
     uint32_t lk_lane, lv_lane;
@@ -159,8 +165,16 @@ struct TqCodes {
                 qs[hh * (D + 4) + t8 + 8 * k] = hv ? a[k] * p.rsqrt_d * (p.scale * kLog2e) : 0.f;
         }
     }
-    __device__ __forceinline__ void begin(const float* qs, int g, int tg) {
+    // (for five to eight heads the lo parts take the queries' place in qs)
+    __device__ __forceinline__ void begin(float* qs, int lane) {
+        const int g = lane >> 2, tg = lane & 3;
         const int head = NH == 1 ? g >> 1 : g;
+        auto pack = [](float lo, float hi) {
+            const __half2 h = __floats2half2_rn(lo, hi);
+            return *reinterpret_cast<const uint32_t*>(&h);
+        };
+        auto residual = [](float x) { return (x - __half2float(__float2half_rn(x))) * kLo; };
+        uint32_t lo[NKB][2];
 #pragma unroll
         for (int kb = 0; kb < NKB; kb++) {
             int coord = (D / 4) * tg + 4 * kb;
@@ -168,9 +182,21 @@ struct TqCodes {
                 coord = (8 * (tg + 4 * (kb >> 1)) + 4 * (kb & 1) - 4 * mis) & (D - 1);
             }
             const float4 q4 = *reinterpret_cast<const float4*>(qs + head * (D + 4) + coord);
-            const __half2 lo = __floats2half2_rn(q4.x, q4.y), hi = __floats2half2_rn(q4.z, q4.w);
-            qb[kb][0] = *reinterpret_cast<const uint32_t*>(&lo);
-            qb[kb][1] = *reinterpret_cast<const uint32_t*>(&hi);
+            qb[kb][0] = pack(q4.x, q4.y);
+            qb[kb][1] = pack(q4.z, q4.w);
+            lo[kb][0] = pack(residual(q4.x), residual(q4.y));
+            lo[kb][1] = pack(residual(q4.z), residual(q4.w));
+            if (NH == 1 && (g & 1)) {
+                qb[kb][0] = lo[kb][0];
+                qb[kb][1] = lo[kb][1];
+            }
+        }
+        if constexpr (NH == 2) {
+            __syncwarp();
+            uint2* const at = reinterpret_cast<uint2*>(qs) + lane;
+#pragma unroll
+            for (int kb = 0; kb < NKB; kb++) at[32 * kb] = make_uint2(lo[kb][0], lo[kb][1]);
+            q_lo = static_cast<uint32_t>(__cvta_generic_to_shared(at));
         }
 #pragma unroll
         for (int h = 0; h < HL; h++) {
@@ -234,7 +260,7 @@ struct TqCodes {
         // ---- S = K.Q^T; with norm correction the sum of the squared centroids of the two tokens.  (From a second look-up per
         // pair of codes: the key tile times itself, whose diagonal holds the sums, kept the tensor pipe as busy as the
         // issue slots.)
-        float c[2][4];
+        float c[NH + 1][4];   // (NH = 2: two chains of the hi parts and one of the lo parts)
         if (norm_correction) {   // (uniform)
             u64 n2 = pk2(0.f, 0.f);
             scores<true>(ka, kb_, c, n2);
@@ -254,7 +280,7 @@ struct TqCodes {
     }
 
     template <bool NC>
-    __device__ __forceinline__ void scores(const uint32_t (&ka)[KW], const uint32_t (&kb_)[KW], float (&c)[2][4], u64& n2) const {
+    __device__ __forceinline__ void scores(const uint32_t (&ka)[KW], const uint32_t (&kb_)[KW], float (&c)[NH + 1][4], u64& n2) const {
         constexpr uint32_t SQ = KB == 4 ? 128u : TKS;   // from an entry to its squares
         u64 other = pk2(0.f, 0.f);
 #pragma unroll
@@ -264,6 +290,11 @@ struct TqCodes {
             const uint32_t a0 = lut32(e0), a1 = lut32(e1), a2 = lut32(e2), a3 = lut32(e3);
             if (kb < 2) mma_16816_z(c[kb & 1], a0, a1, a2, a3, qb[kb][0], qb[kb][1]);
             else mma_16816(c[kb & 1], a0, a1, a2, a3, qb[kb][0], qb[kb][1]);
+            if constexpr (NH == 2) {
+                const uint2 lo = lds64(q_lo + 256 * kb);
+                if (kb == 0) mma_16816_z(c[NH], a0, a1, a2, a3, lo.x, lo.y);
+                else mma_16816(c[NH], a0, a1, a2, a3, lo.x, lo.y);
+            }
             if constexpr (NC) {
                 n2 = add2(n2, pk2(__uint_as_float(lut32(e0 + SQ)), __uint_as_float(lut32(e1 + SQ))));
                 other = add2(other, pk2(__uint_as_float(lut32(e2 + SQ)), __uint_as_float(lut32(e3 + SQ))));
@@ -273,7 +304,7 @@ struct TqCodes {
     }
 
     template <bool FULL>
-    __device__ __forceinline__ void attend(uint32_t page, uint32_t ts, int lo, int hi, int lane, const float (&c)[2][4],
+    __device__ __forceinline__ void attend(uint32_t page, uint32_t ts, int lo, int hi, int lane, const float (&c)[NH + 1][4],
                                            float kna, float knb, uint32_t sca, uint32_t scb) {
         const int g = lane >> 2, tg = lane & 3;
         // ---- online softmax (base-2 exponents), the lane's tokens g and g + 8
@@ -287,8 +318,9 @@ struct TqCodes {
         bool above = s_max > s_ref;
 #pragma unroll
         for (int h = 0; h < HL; h++) {
-            sa[h] = okA ? (c[0][h] + c[1][h]) * kna : -INFINITY;
-            sb[h] = okB ? (c[0][2 + h] + c[1][2 + h]) * knb : -INFINITY;
+            const float la = NH == 1 ? c[0][1] + c[1][1] : c[NH][h], lb = NH == 1 ? c[0][3] + c[1][3] : c[NH][2 + h];
+            sa[h] = okA ? fmaf(la, kInvLo, c[0][h] + c[1][h]) * kna : -INFINITY;
+            sb[h] = okB ? fmaf(lb, kInvLo, c[0][2 + h] + c[1][2 + h]) * knb : -INFINITY;
             above |= fmaxf(sa[h], sb[h]) > m_run[h];
         }
         if (__any_sync(0xffffffffu, above)) {
@@ -704,7 +736,7 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
         float* qs = xchg(warp);
         e.rotate(p, qs, head0, group, lane);
         __syncwarp();
-        e.begin(qs, lane >> 2, lane & 3);
+        e.begin(qs, lane);
         __syncwarp();
         bool poison = false;
         int seen = 0;

@@ -107,7 +107,8 @@ struct TqFp8 {
         for (int x = 0; x < NH; x++) rotate_four(p, qs, head0, group, lane, x);
     }
     // B fragments: column g = (head g >> 1, hi for an even g, lo for an odd one), or head g (hi, lo)
-    __device__ __forceinline__ void begin(const float* qs, int g, int tg) {
+    __device__ __forceinline__ void begin(const float* qs, int lane) {
+        const int g = lane >> 2, tg = lane & 3;
 #pragma unroll
         for (int kb = 0; kb < NKB; kb++) {
             const int coord = WIDE ? (D / 4) * tg + 4 * kb : 4 * (tg + 4 * kb);
@@ -417,7 +418,6 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
     constexpr int WARPS = C::WARPS;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, tg = lane & 3;
     const uint32_t ring = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw)) + warp * C::STAGES * C::PAGE;
     float* qs = reinterpret_cast<float*>(smem_raw + WARPS * C::STAGES * C::PAGE);   // [4 * NH][QROW]
     float* xo = qs + C::QS / 4;                                                    // [WARPS][OL][32]
@@ -502,7 +502,7 @@ tq_fp8_kernel(const TqDecodeParams p, int n_items) {
             Engine::rotate_four(p, qs, static_cast<int64_t>(it.b) * p.Hq + it.hkv * group, group, lane, warp);
         __syncthreads();
         Engine e;
-        e.begin(qs, g, tg);
+        e.begin(qs, lane);
         bool bad_block = false;
 
         for (int pg = warp; pg < it.n_pages; pg += WARPS) {

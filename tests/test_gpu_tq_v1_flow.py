@@ -34,13 +34,13 @@ def _batch(D, kb, vb, Hkv, G, lens, bs=16, pad=0, layers=1, nc=True, seed=0):
     return cfg, cent, cache, bt, torch.tensor(lens, dtype=torch.int32, device="cuda"), q
 
 
-def _decode(q, cache, bt, seq, cent, cfg, splits, start=None):
+def _decode(q, cache, bt, seq, cent, cfg, splits, start=None, **kw):
     from fused_turboquant_b200 import tq_v1
     lead, hq, d = q.shape[:-2], q.shape[-2], q.shape[-1]
     mid = torch.full((*lead, hq, splits, d + 1), 7.0, device="cuda")
     lse = torch.empty(*lead, hq, device="cuda")
     out = tq_v1.decode_attention(q, cache, bt, seq, cent, cfg, d ** -0.5, num_kv_splits=splits, kv_start_offset=start,
-                                 mid_o=mid, lse=lse, out_dtype=torch.float32)
+                                 mid_o=mid, lse=lse, out_dtype=torch.float32, **kw)
     return out.cpu().numpy(), mid.cpu().numpy(), lse.cpu().numpy()
 
 
@@ -123,3 +123,63 @@ def test_captured_and_replayed():
         g.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want)
+
+
+def _items():
+    """The workspace with which the item kernels run."""
+    return torch.empty(0, dtype=torch.uint8, device="cuda")
+
+
+def _float64(q, cache, bt, seq, cent, cfg):
+    """Attention over the cache's bytes in 64 bits: [B, Hq, D]."""
+    d, kb, vb, hkv = q.shape[-1], cfg.key_quant_bits, cfg.value_quant_bits, cache.shape[-2]
+    had = torch.ones(1, 1, dtype=torch.float64, device="cuda")
+    while had.shape[0] < d:
+        had = torch.cat([torch.cat([had, had], 1), torch.cat([had, -had], 1)], 0)
+    qr, out = q.double() @ (had / d ** 0.5), []
+
+    def codes(rows, bits):
+        b = (rows[..., None].int() >> torch.arange(8, device="cuda")) & 1
+        return (b.reshape(*rows.shape[:-1], d, bits) << torch.arange(bits, device="cuda")).sum(-1)
+    for b, n in enumerate(seq.tolist()):
+        rows = cache[bt[b].long()].reshape(-1, hkv, cache.shape[-1])[:n]
+        kc, vc = d * kb // 8, d * vb // 8
+        k = cent.cuda().double()[codes(rows[..., :kc], kb)]
+        norm = rows[..., kc:kc + 2].contiguous().view(torch.float16).double()
+        if cfg.norm_correction:
+            norm = norm / (k.norm(dim=-1, keepdim=True) ** 2 + 1e-16).sqrt()
+        meta = rows[..., kc + 2 + vc:kc + 6 + vc].contiguous().view(torch.float16).double()
+        v = codes(rows[..., kc + 2:kc + 2 + vc], vb).double() * meta[..., :1] + meta[..., 1:]
+        s = torch.einsum("hgd,nhd->hgn", qr[b].view(hkv, -1, d), k * norm) * d ** -0.5
+        out.append(torch.einsum("hgn,nhd->hgd", s.softmax(-1), v).reshape(-1, d))
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("D,kb,vb,Hkv,G,n,splits", [(128, 4, 4, 8, 4, 4096, 32), (128, 4, 4, 8, 8, 20000, 32), (128, 3, 3, 8, 4, 20000, 32),
+                                                    (64, 3, 4, 16, 2, 9000, 32), (128, 4, 4, 8, 4, 40000, 32)])
+def test_error_is_no_larger_than_the_item_kernels(D, kb, vb, Hkv, G, n, splits):
+    """Against 64 bits, where a warp adds up the pages of a split in one accumulator (up to 80 pages there)."""
+    cfg, cent, cache, bt, seq, q = _batch(D, kb, vb, Hkv, G, [n] * 4)
+    ref = _float64(q[0], cache[0], bt, seq, cent, cfg).cpu().numpy()
+    err = [(np.linalg.norm(_decode(q[0], cache[0], bt, seq, cent, cfg, splits, workspace=w)[0] - ref, axis=-1) /
+            np.linalg.norm(ref, axis=-1)).mean() for w in (None, _items())]
+    print(f"mean error: shares {err[0]:.3e}, items {err[1]:.3e}")
+    assert err[0] < 1.02 * err[1]     # (means over 128 rows and more of errors of the same size)
+
+
+@pytest.mark.parametrize("D,layers", [(128, 1), (64, 1), (128, 8)])   # (eight layers of 64 heads of 128: two launches)
+def test_rotation_and_prefix(D, layers):
+    """What the merge does after the sums, a sequence without tokens and one without a prefix among them."""
+    cfg, cent, cache, bt, seq, q = _batch(D, 4, 4, 8, 8 if layers > 1 else 4, [700, 0, 90, 333], layers=layers)
+    q, cache = (q, cache) if layers > 1 else (q[0], cache[0])
+    g = torch.Generator("cuda").manual_seed(5)
+    pre = torch.randn(q.shape, generator=g, device="cuda").bfloat16()
+    pre_lse = torch.randn(q.shape[:-1], generator=g, device="cuda") + 4.0
+    pre_lse[..., 2, :] = -float("inf")
+    for kw in (dict(v_rotate=True), dict(prefix_output=pre, prefix_lse=pre_lse),
+               dict(v_rotate=True, prefix_output=pre, prefix_lse=pre_lse)):
+        (o, _, l), (o_ref, _, l_ref) = (_decode(q, cache, bt, seq, cent, cfg, 32, workspace=w, **kw) for w in (None, _items()))
+        assert gate(o, o_ref) <= o.size // 300 and np.abs(o - o_ref).max() < 4e-3
+        assert np.array_equal(np.isneginf(l), np.isneginf(l_ref))
+        live = np.isfinite(l_ref)
+        np.testing.assert_allclose(l[live], l_ref[live], rtol=2e-3, atol=5e-3)

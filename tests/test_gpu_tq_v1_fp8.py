@@ -27,8 +27,17 @@ def _exact(q, cache, table, lens, d, vb, hkv, scale):
     return torch.stack(out)
 
 
+def _by_shares(q, cache, table, cfg, splits):
+    """Does the call take the kernel that streams whole pages?"""
+    from fused_turboquant_b200 import _lib
+    return _lib.load().ftq_tq_decode_layers_workspace_bytes(
+        _lib.BF16, q.shape[0], q.shape[1], cache.shape[2], q.shape[2], cache.data_ptr(), *cache.stride()[:3], cache.shape[1],
+        table.shape[1], cfg.key_quant_bits, cfg.value_quant_bits, 0, splits, 1, 0) > 0
+
+
 # (one token; less than a page; pages that not every warp has; remainders; groups on both sides of four;
-# splits without tokens; one and several layers of items per CTA)
+# splits without tokens; one and several layers of items per CTA.  The last six: 128 units and more of 8 and 16 heads, by shares of
+# pages, with unwritten slots in the pages that it reads whole)
 @pytest.mark.parametrize("d,vb,hkv,group,lens,splits,dtype", [
     (128, 4, 2, 4, [1, 15, 16, 17], 8, "bf16"),
     (128, 4, 8, 4, [1000, 4096, 333], 8, "bf16"),
@@ -37,6 +46,12 @@ def _exact(q, cache, table, lens, d, vb, hkv, scale):
     (64, 4, 4, 1, [129, 2000], 8, "fp16"),
     (64, 3, 2, 8, [40, 300], 3, "bf16"),
     (64, 2, 1, 3, [77] * 40, 16, "bf16"),
+    (128, 4, 8, 4, [1, 15, 16, 17, 700, 3000], 32, "bf16"),
+    (128, 3, 8, 1, [5, 9001], 64, "fp16"),
+    (128, 2, 16, 3, [513] * 8, 16, "bf16"),
+    (64, 4, 8, 7, [1000, 90], 64, "fp16"),
+    (64, 3, 16, 2, [40, 300, 5000, 1], 32, "bf16"),
+    (64, 2, 8, 8, [7000, 77, 16], 60, "bf16"),
 ])
 def test_fp32_precision(d, vb, hkv, group, lens, splits, dtype):
     from fused_turboquant_b200 import tq_v1
@@ -59,6 +74,7 @@ def test_fp32_precision(d, vb, hkv, group, lens, splits, dtype):
     sl = torch.tensor(lens, dtype=torch.int32, device="cuda")
     q = torch.randn(len(lens), hkv * group, d, device="cuda", generator=gen)
     q = q.to(torch.bfloat16 if dtype == "bf16" else torch.float16)
+    assert _by_shares(q, cache, table, cfg, splits) == (hkv >= 8 and len(lens) * splits >= 128)
 
     def run(x):
         out = torch.empty(x.shape, dtype=torch.float32, device="cuda")
@@ -99,11 +115,14 @@ def test_slots_off_the_word_stay_on_the_fp32_kernel():
     (4096, 8, 1e-4, 0.0, 10.0),     # small value scales
     (4096, 8, 1.0, 10.0, 1.0),      # a value channel that is never near zero
     (30000, 8, 1.0, 0.0, 10.0),     # 30 pages a warp
+    (4096, 32, 1.0, 0.0, 10.0),     # by shares of pages (groups of 128 up to four, of 64 up to eight), 8 pages a split
+    (16384, 32, 1.0, 0.0, 10.0),    # ... up to 16 pages a warp
+    (16384, 32, 1e-4, 10.0, 1.0),
 ])
 def test_error_is_no_larger_than_the_fp32_kernels(d, vb, group, n, splits, scale, shift, wide):
     from fused_turboquant_b200 import tq_v1
     gen = torch.Generator("cuda").manual_seed(d + vb + group + n)
-    hkv, B = (2 if n > 10000 else 8), 4
+    hkv, B = (2 if n > 20000 else 8), 4
     cfg = tq_v1.TurboQuantSlotConfig(d, 8, vb, norm_correction=True)
     per = (n + 15) // 16
     cache = torch.zeros(B * per, 16, hkv, cfg.slot_size_aligned, dtype=torch.uint8, device="cuda")
@@ -120,6 +139,7 @@ def test_error_is_no_larger_than_the_fp32_kernels(d, vb, group, n, splits, scale
         tq_v1.launch_store(kv[0].bfloat16(), kv[1].bfloat16(), cache, slots, None, cfg)
     sl = torch.full((B,), n, dtype=torch.int32, device="cuda")
     q = torch.randn(B, hkv * group, d, device="cuda", generator=gen).bfloat16()
+    assert _by_shares(q, cache, table, cfg, splits) == (splits == 32 and (d == 64 or group <= 4))
     ref = _exact(q, cache, table, sl, d, vb, hkv, d ** -0.5)
     err = []
     for x in (q, q.float()):

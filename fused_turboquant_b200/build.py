@@ -22,7 +22,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libftq_b200.so")
 # A second library for ONE test (tests/test_gpu_wait_expiry.py): the same objects, except that the
-# head_dim-128 decode and chunk attention units are compiled with FTQ_TEST_WAIT_EXPIRY (one page copy of
+# head_dim-128 decode, chunk attention and slot-format decode units are compiled with FTQ_TEST_WAIT_EXPIRY (one page copy of
 # one warp is never issued, one tile of one warp never reported, and the poll limits are small), so that
 # a bounded wait runs out and the give-up path (NaN rows, status word, the context stays usable)
 # executes.  Never loaded by the package.
@@ -30,8 +30,9 @@ TEST_LIB_PATH = os.path.join(PKG_DIR, "libftq_b200_waittest.so")
 # The tensor-level host path (csrc/ftq_torch.cpp): a CPython module compiled with the host compiler
 # against torch's headers; it gets the C ABI's addresses at import and links nothing of ours.
 NATIVE_PATH = os.path.join(PKG_DIR, "_native.so")
-TEST_UNITS = [(src, f"{tag}_waittest", ["-DFTQ_D=128", "-DFTQ_ONLY_BITS=4", "-DFTQ_TEST_WAIT_EXPIRY"])
-              for src, tag in (("ftq_attn_inst.cu", "attn_d128"), ("ftq_attn_chunk_inst.cu", "attn_chunk_d128"))]
+TEST_UNITS = [(src, f"{tag}_waittest", [*part, "-DFTQ_D=128", "-DFTQ_ONLY_BITS=4", "-DFTQ_TEST_WAIT_EXPIRY"])
+              for src, tag, part in (("ftq_attn_inst.cu", "attn_d128", ()), ("ftq_attn_chunk_inst.cu", "attn_chunk_d128", ()),
+                                     ("ftq_tq_v1_inst.cu", "tq_v1_flow_d128", ("-DFTQ_TQ_PART=2",)))]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

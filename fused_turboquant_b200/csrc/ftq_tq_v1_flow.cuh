@@ -687,6 +687,9 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
                     if (ok && lane == u) {
                         slot_info[s].y = 2 * turn + (bad ? 1 : 0);
                         mbar_expect_tx(full + s * 8, bytes);
+#ifdef FTQ_TEST_WAIT_EXPIRY
+                        if (blockIdx.x == 0 && sub_pages == 0 && i == 0) continue;   // (see kMbarSpinLimit)
+#endif
                         bulk_g2s_hint(slot_info[s].x, src, bytes, full + s * 8, policy);
                     }
                 }

@@ -306,8 +306,11 @@ static cudaError_t join_run(const TqMergeParams& p, cudaStream_t stream) {
     return launch_dependent(tq_join_kernel<FTQ_D, OT>, static_cast<unsigned>((p.n_rows + 1) / 2), 128, 0, stream, p);
 }
 #endif
+// FTQ_ONLY_BITS=<b>: key and value codes of b bits only (the wait-expiry test library)
 cudaError_t FTQ_CAT(launch_tq_flow_d, FTQ_D)(int kb, int vb, int nh, const TqFlowParams& p, cudaStream_t stream) {
-#if FTQ_D != 256
+#if defined(FTQ_ONLY_BITS)
+    if (kb == FTQ_ONLY_BITS && vb == FTQ_ONLY_BITS) return flow_by_nh<FTQ_ONLY_BITS, FTQ_ONLY_BITS>(nh, p, stream);
+#elif FTQ_D != 256
     switch (kb) {
         case 2: return flow_by_vb<2>(vb, nh, p, stream);
         case 3: return flow_by_vb<3>(vb, nh, p, stream);

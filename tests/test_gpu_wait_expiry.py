@@ -127,3 +127,42 @@ def test_an_expired_wait_of_the_chunk_kernel_poisons_its_rows_and_nothing_else()
     assert torch.equal(got[~lost], good[~lost])
     again, rc, status = run(good_lib)
     assert rc == 0 and status == 0 and torch.equal(again, good)
+
+
+@pytest.mark.parametrize("G", [4, 8])
+def test_an_expired_wait_of_the_slot_decode_by_shares_is_nan_everywhere(G):
+    """The first page of CTA 0 is announced but not copied: its warps and the producer give up, and the merge, which can
+    not know whose rows are missing, returns NaN for the call."""
+    from fused_turboquant_b200 import TurboQuantMSE, _lib, tq_v1
+    bad_lib, good_lib = _test_lib(), _lib.load()
+    d, Hkv, B, n, splits = 128, 8, 16, 700, 8
+    cfg = tq_v1.TurboQuantSlotConfig(d, 4, 4)
+    cent, mids = tq_v1.midpoints_of(TurboQuantMSE(d, bits=4, device="cuda").quantizer.levels)
+    g = torch.Generator("cuda").manual_seed(2)
+    per = (n + 15) // 16
+    bt = torch.randperm(B * per, device="cuda", generator=g).int().view(B, per)
+    cache = torch.zeros(B * per, 16, Hkv, cfg.slot_size_aligned, dtype=torch.uint8, device="cuda")
+    kv = torch.randn(2, B * per * 16, Hkv, d, device="cuda", generator=g).bfloat16()
+    tq_v1.launch_store(kv[0], kv[1], cache, torch.arange(B * per * 16, device="cuda"), mids, cfg)
+    q = torch.randn(B, Hkv * G, d, device="cuda", generator=g).bfloat16()
+    sl = torch.full((B,), n, dtype=torch.int32, device="cuda")
+    ws = torch.empty(tq_v1.decode_workspace_bytes(B, Hkv * G, d), dtype=torch.uint8, device="cuda")
+    mid = torch.empty(B, Hkv * G, splits, d + 1, device="cuda")
+    levels = cent.cpu().numpy().astype(np.float32)
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+
+    def run(lib):
+        out = torch.full(q.shape, 7.0, dtype=torch.float32, device="cuda")
+        rc = lib.ftq_tq_decode_layers_ws(
+            p(q), _lib.BF16, B, Hkv * G, Hkv, d, p(cache), *cache.stride()[:3], 16, p(bt), per, p(sl), None, 4, 4, 1, 0, 0,
+            _lib.fptr(levels), d ** -0.5, splits, p(mid), p(out), _lib.F32, None, None, 0, None, 1, 0, B * per, p(ws),
+            ws.numel(), stream)
+        assert rc == 0, lib.ftq_last_error()
+        torch.cuda.synchronize()
+        return out
+
+    good = run(good_lib)
+    assert torch.isfinite(good).all()
+    assert torch.isnan(run(bad_lib)).all()
+    assert torch.equal(run(good_lib), good)

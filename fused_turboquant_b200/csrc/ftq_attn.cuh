@@ -513,8 +513,8 @@ struct MergeStatus {
 };
 template <int D, typename OT, int OCTETS>
 __global__ void __launch_bounds__(128)
-attn_merge_kernel(const float* __restrict__ partials, OT* __restrict__ out,
-                  const int32_t* __restrict__ seq_lens, int S, int B, int Hq, int n_chunks,
+attn_merge_kernel(const float* partials, OT* __restrict__ out,   // (only the output is restrict: see load8)
+                  const int32_t* seq_lens, int S, int B, int Hq, int n_chunks,
                   int chunk_tokens, int64_t n_vec, SignBits signs, float rsqrt_d, MergeStatus st) {
     constexpr int E = D / kOctet;
     constexpr int ROW = D + 4;

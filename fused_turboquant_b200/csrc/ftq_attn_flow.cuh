@@ -285,7 +285,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         const int pg = (warp + (k0 + lane / NP) * WARPS) * NP + lane % NP;
         int id = 0;
         if (pg < it.n_pages) {
-            id = __ldg(p.block_table + static_cast<int64_t>(it.b) * p.max_blocks + it.page0 + pg);
+            id = p.block_table[static_cast<int64_t>(it.b) * p.max_blocks + it.page0 + pg];
             if (static_cast<uint32_t>(id) >= static_cast<uint64_t>(p.num_blocks)) {
                 id = 0;
                 s_bad[slot] = 1;

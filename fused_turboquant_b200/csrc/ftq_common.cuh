@@ -101,21 +101,23 @@ __device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u 
 __device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
 // Load 8 consecutive elements starting at p (16-byte aligned for 2-byte types,
-// 32-byte aligned for fp32) and widen to fp32.
+// 32-byte aligned for fp32) and widen to fp32.  Ordinary loads, as all of what another kernel may still be writing when
+// this one starts: those through the read-only path (__ldg, const __restrict__ arguments) are for memory that nobody
+// writes while the kernel lives, and may be moved to before the wait.
 template <typename T>
 __device__ __forceinline__ void load8(const T* p, float (&o)[8]);
 
 template <>
 __device__ __forceinline__ void load8<float>(const float* p, float (&o)[8]) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-    const float4 b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    const float4 a = *reinterpret_cast<const float4*>(p);
+    const float4 b = reinterpret_cast<const float4*>(p)[1];
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
     o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
 }
 
 template <>
 __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16* p, float (&o)[8]) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 a = *reinterpret_cast<const uint4*>(p);
     o[0] = bf16_lo(a.x); o[1] = bf16_hi(a.x);
     o[2] = bf16_lo(a.y); o[3] = bf16_hi(a.y);
     o[4] = bf16_lo(a.z); o[5] = bf16_hi(a.z);
@@ -124,7 +126,7 @@ __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16* p, flo
 
 template <>
 __device__ __forceinline__ void load8<__half>(const __half* p, float (&o)[8]) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint4 a = *reinterpret_cast<const uint4*>(p);
     const uint32_t w[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
     for (int j = 0; j < 4; j++) {

@@ -70,7 +70,7 @@ rht_kernel(const T* __restrict__ x, T* __restrict__ y, SignBits signs, float rsq
 // out = fwht(levels[code] * norm) * D^-1/2 * signs  (core/quantizer.py:191-205).
 template <int D, int BITS, typename NormT>
 __global__ void __launch_bounds__(256)
-decode_dense_kernel(const uint8_t* __restrict__ packed, const NormT* __restrict__ norms,
+decode_dense_kernel(const uint8_t* packed, const NormT* norms,   // (not restrict: see load8)
                     float* __restrict__ out, Codebook levels, SignBits signs, float rsqrt_d,
                     int64_t n_vec) {
     constexpr int E = D / kOctet;

@@ -59,12 +59,12 @@ template <> struct Raw8<float> { float4 a, b; };
 
 template <typename T>
 __device__ __forceinline__ void load_raw8(const T* p, Raw8<T>& r) {
-    r.v = __ldg(reinterpret_cast<const uint4*>(p));
+    r.v = *reinterpret_cast<const uint4*>(p);   // (see load8)
 }
 template <>
 __device__ __forceinline__ void load_raw8<float>(const float* p, Raw8<float>& r) {
-    r.a = __ldg(reinterpret_cast<const float4*>(p));
-    r.b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    r.a = *reinterpret_cast<const float4*>(p);
+    r.b = reinterpret_cast<const float4*>(p)[1];
 }
 template <typename T>
 __device__ __forceinline__ void widen8(const Raw8<T>& r, float (&o)[8]);

@@ -660,7 +660,7 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
             const uint8_t* const kv_layer = p.kv_cache + layer * p.cache_layer_stride;
             auto load_id = [&](int i) {
                 if (i >= pc.n) return 0;
-                return __ldg(btab + fast_div(static_cast<uint32_t>(page0 + i) * kPageTokens, p.div_block));
+                return btab[fast_div(static_cast<uint32_t>(page0 + i) * kPageTokens, p.div_block)];
             };
             int ids = 0, ids_next = load_id(lane);
             for (int i0 = 0; i0 < pc.n && ok; i0 += subs) {

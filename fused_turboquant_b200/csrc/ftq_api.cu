@@ -1647,16 +1647,17 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
         fp.share = static_cast<uint32_t*>(workspace);
         fp.prefix = reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) + 256);
         fp.rows = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + tq_rows_offset(B_seq));
-        mp.share = fp.share;
-        mp.page_prefix = fp.prefix;
-        mp.rows = fp.rows;
-        mp.seq_lens = seq_lens;
-        mp.kv_start = kv_start_offset;
-        mp.Hq = Hq;
-        mp.B_seq = p.B_seq;
-        mp.piece_cost = piece_cost;
-        mp.div_hq = ftq::make_fastdiv(static_cast<uint32_t>(Hq));
-        mp.div_bseq = p.div_bseq;
+        ftq::TqJoinParams jp{};
+        jp.share = fp.share;
+        jp.page_prefix = fp.prefix;
+        jp.rows = fp.rows;
+        jp.seq_lens = seq_lens;
+        jp.kv_start = kv_start_offset;
+        jp.Hq = Hq;
+        jp.B_seq = p.B_seq;
+        jp.piece_cost = piece_cost;
+        jp.div_hq = ftq::make_fastdiv(static_cast<uint32_t>(Hq));
+        jp.div_bseq = p.div_bseq;
         const int nh = group <= 4 ? 1 : 2, per = tq_layers_per_launch(Hq, head_dim, n_layers);
         const int64_t layer_rows = static_cast<int64_t>(B_seq) * Hq;
         auto size_of = [](int dtype) { return dtype == FTQ_F32 ? 4 : 2; };
@@ -1670,7 +1671,7 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
             e = head_dim == 64 ? ftq::launch_tq_flow_d64(key_bits, value_bits, nh, fp, st)
                                : ftq::launch_tq_flow_d128(key_bits, value_bits, nh, fp, st);
             if (e != cudaSuccess) return cuda_fail(e, "tq_decode stage 1 launch");
-            mp.mid_o = mp.mid_out = fp.d.mid_o;
+            mp.mid_o = jp.mid_out = fp.d.mid_o;
             mp.out = static_cast<uint8_t*>(out) + row0 * head_dim * size_of(out_dtype);
             mp.lse = lse ? lse + row0 : nullptr;
             mp.n_rows = n * layer_rows;
@@ -1678,7 +1679,8 @@ extern "C" int ftq_tq_decode_layers_ws(const void* q, int q_dtype, int B, int Hq
                 mp.prefix_out = static_cast<const uint8_t*>(prefix_out) + row0 * head_dim * size_of(prefix_dtype);
                 mp.prefix_lse = prefix_lse + row0;
             }
-            e = head_dim == 64 ? ftq::launch_tq_join_d64(out_dtype, mp, st) : ftq::launch_tq_join_d128(out_dtype, mp, st);
+            jp.m = mp;
+            e = head_dim == 64 ? ftq::launch_tq_join_d64(out_dtype, jp, st) : ftq::launch_tq_join_d128(out_dtype, jp, st);
             if (e != cudaSuccess) return cuda_fail(e, "tq_decode merge launch");
         }
         return FTQ_OK;

@@ -956,7 +956,11 @@ struct TqMergeParams {
     const void* prefix_out;   // [n_rows, D] of prefix_dtype, original space
     int prefix_dtype;
     const float* prefix_lse;  // [n_rows]
-    // Stage 1 with equal shares: units that a share's end cuts lie in the workspace (nullable)
+};
+// (a struct of its own: with these among its parameters the compiler made tq_merge_kernel 0.4 us slower)
+struct TqJoinParams {
+    TqMergeParams m;
+    // Stage 1 with equal shares: units that a share's end cuts lie in the workspace
     const uint32_t* share;
     const int* page_prefix;
     const float* rows;
@@ -966,59 +970,6 @@ struct TqMergeParams {
     int Hq, B_seq, piece_cost;
     FastDiv div_hq, div_bseq;
 };
-
-// What is left of a row once its partials are summed up (weights relative to M, their sum l): normalise, rotate back,
-// merge the prefix in, store.  Every octet of the row holds the sums and stores its part.  (The result overlaps none of what
-// the kernel reads; told so, the compiler took 0.5 us less for the merge: 4.2 instead of 4.7.)
-template <int D, typename OT, int OCTETS>
-__device__ __forceinline__ void tq_finish_row(const TqMergeParams& p, OT* __restrict__ out, float* __restrict__ lse_out,
-                                              int64_t row, float (&a)[D / kOctet], float l, float M, int lane, bool store) {
-    constexpr int E = D / kOctet;
-    const int t = lane & 7, o = (lane >> 3) & (OCTETS - 1);
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-#pragma unroll
-    for (int r = 0; r < E; r++) a[r] *= inv;
-    if (p.rotate) {
-        octet_fwht<E>(a, lane);
-#pragma unroll
-        for (int k = 0; k < E; k++) a[k] *= p.rsqrt_d;
-    }
-    float lse = l > 0.f ? M + logf(l) : -INFINITY;
-    float w_own = 1.f, w_pre = 0.f;
-    const bool prefix = p.prefix_out != nullptr;
-    if (prefix) {
-        const float lp = p.prefix_lse[row];
-        const float lmax = fmaxf(lp, lse);
-        if (lmax == -INFINITY) {  // nothing attended on either side
-            w_own = 0.f;
-        } else {
-            const float ep = __expf(lp - lmax), eq = __expf(lse - lmax);
-            const float total = fmaxf(ep + eq, 1e-20f);
-            w_pre = ep / total;
-            w_own = eq / total;
-            lse = lmax + logf(ep + eq);
-        }
-    }
-    OT* orow = out + row * D;
-#pragma unroll
-    for (int r = 0; r < E; r++) {
-        if (!store || (r & (OCTETS - 1)) != o) continue;
-        const int coord = p.rotate ? t + 8 * r : load_coord(t, r);
-        float v = a[r];
-        if (prefix) {
-            const int64_t at = row * D + coord;
-            const float pv = p.prefix_dtype == kF32 ? static_cast<const float*>(p.prefix_out)[at]
-                             : p.prefix_dtype == kF16
-                                 ? __half2float(static_cast<const __half*>(p.prefix_out)[at])
-                                 : __bfloat162float(static_cast<const __nv_bfloat16*>(p.prefix_out)[at]);
-            v = pv * w_pre + v * w_own;
-        }
-        if constexpr (sizeof(OT) == 4) orow[coord] = v;
-        else if constexpr (std::is_same<OT, __half>::value) orow[coord] = __float2half_rn(v);
-        else orow[coord] = __float2bfloat16_rn(v);
-    }
-    if (lse_out && t == 0 && o == 0 && store) lse_out[row] = lse;
-}
 
 // Merge the split partials of a (sequence, query head) row: softmax-weighted by lse, optionally
 // Hadamard-transform the result, optionally merge a prefix result in, cast and store.  mid_o rows with
@@ -1032,7 +983,8 @@ tq_merge_kernel(const TqMergeParams p) {
     OT* __restrict__ out = static_cast<OT*>(p.out);
     float* __restrict__ lse_out = p.lse;
     const int64_t n_rows = p.n_rows;
-    const int splits = p.splits;
+    const int splits = p.splits, rotate = p.rotate;
+    const float rsqrt_d = p.rsqrt_d;
     constexpr int E = D / kOctet;
     const int lane = threadIdx.x & 31;
     const int t = lane & 7, o = (lane >> 3) & (OCTETS - 1);
@@ -1066,7 +1018,49 @@ tq_merge_kernel(const TqMergeParams p) {
 #pragma unroll
         for (int r = 0; r < E; r++) a[r] += __shfl_xor_sync(0xffffffffu, a[r], m);
     }
-    tq_finish_row<D, OT, OCTETS>(p, out, lse_out, row, a, l, M, lane, at < n_rows);
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll
+    for (int r = 0; r < E; r++) a[r] *= inv;
+    if (rotate) {
+        octet_fwht<E>(a, lane);
+#pragma unroll
+        for (int k = 0; k < E; k++) a[k] *= rsqrt_d;
+    }
+    float lse = l > 0.f ? M + logf(l) : -INFINITY;
+    float w_own = 1.f, w_pre = 0.f;
+    const bool prefix = p.prefix_out != nullptr;
+    if (prefix) {
+        const float lp = p.prefix_lse[row];
+        const float lmax = fmaxf(lp, lse);
+        if (lmax == -INFINITY) {  // nothing attended on either side
+            w_own = 0.f;
+        } else {
+            const float ep = __expf(lp - lmax), eq = __expf(lse - lmax);
+            const float total = fmaxf(ep + eq, 1e-20f);
+            w_pre = ep / total;
+            w_own = eq / total;
+            lse = lmax + logf(ep + eq);
+        }
+    }
+    OT* orow = out + row * D;
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        if (at >= n_rows || (r & (OCTETS - 1)) != o) continue;   // (every octet of the row holds the result and stores its part)
+        const int coord = rotate ? t + 8 * r : load_coord(t, r);
+        float v = a[r];
+        if (prefix) {
+            const int64_t at = row * D + coord;
+            const float pv = p.prefix_dtype == kF32 ? static_cast<const float*>(p.prefix_out)[at]
+                             : p.prefix_dtype == kF16
+                                 ? __half2float(static_cast<const __half*>(p.prefix_out)[at])
+                                 : __bfloat162float(static_cast<const __nv_bfloat16*>(p.prefix_out)[at]);
+            v = pv * w_pre + v * w_own;
+        }
+        if constexpr (sizeof(OT) == 4) orow[coord] = v;
+        else if constexpr (std::is_same<OT, __half>::value) orow[coord] = __float2half_rn(v);
+        else orow[coord] = __float2bfloat16_rn(v);
+    }
+    if (lse_out && t == 0 && o == 0 && at < n_rows) lse_out[row] = lse;
 }
 
 }  // namespace ftq

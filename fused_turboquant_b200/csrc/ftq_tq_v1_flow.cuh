@@ -803,6 +803,59 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
     if (stalled && lane == 0) *f.share = 0u;
 }
 
+// What is left of a row once its partials are summed up (weights relative to M, their sum l): normalise, rotate back,
+// merge the prefix in, store.  Every octet of the row holds the sums and stores its part.  (As the end of
+// tq_merge_kernel, which has it in its body and its registers' number from that.)
+template <int D, typename OT, int OCTETS>
+__device__ __forceinline__ void tq_finish_row(const TqMergeParams& p, OT* __restrict__ out, float* __restrict__ lse_out,
+                                              int64_t row, float (&a)[D / kOctet], float l, float M, int lane, bool store) {
+    constexpr int E = D / kOctet;
+    const int t = lane & 7, o = (lane >> 3) & (OCTETS - 1);
+    const float inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll
+    for (int r = 0; r < E; r++) a[r] *= inv;
+    if (p.rotate) {
+        octet_fwht<E>(a, lane);
+#pragma unroll
+        for (int k = 0; k < E; k++) a[k] *= p.rsqrt_d;
+    }
+    float lse = l > 0.f ? M + logf(l) : -INFINITY;
+    float w_own = 1.f, w_pre = 0.f;
+    const bool prefix = p.prefix_out != nullptr;
+    if (prefix) {
+        const float lp = p.prefix_lse[row];
+        const float lmax = fmaxf(lp, lse);
+        if (lmax == -INFINITY) {  // nothing attended on either side
+            w_own = 0.f;
+        } else {
+            const float ep = __expf(lp - lmax), eq = __expf(lse - lmax);
+            const float total = fmaxf(ep + eq, 1e-20f);
+            w_pre = ep / total;
+            w_own = eq / total;
+            lse = lmax + logf(ep + eq);
+        }
+    }
+    OT* orow = out + row * D;
+#pragma unroll
+    for (int r = 0; r < E; r++) {
+        if (!store || (r & (OCTETS - 1)) != o) continue;
+        const int coord = p.rotate ? t + 8 * r : load_coord(t, r);
+        float v = a[r];
+        if (prefix) {
+            const int64_t at = row * D + coord;
+            const float pv = p.prefix_dtype == kF32 ? static_cast<const float*>(p.prefix_out)[at]
+                             : p.prefix_dtype == kF16
+                                 ? __half2float(static_cast<const __half*>(p.prefix_out)[at])
+                                 : __bfloat162float(static_cast<const __nv_bfloat16*>(p.prefix_out)[at]);
+            v = pv * w_pre + v * w_own;
+        }
+        if constexpr (sizeof(OT) == 4) orow[coord] = v;
+        else if constexpr (std::is_same<OT, __half>::value) orow[coord] = __float2half_rn(v);
+        else orow[coord] = __float2bfloat16_rn(v);
+    }
+    if (lse_out && t == 0 && o == 0 && store) lse_out[row] = lse;
+}
+
 // Stage 2 (tq_merge_kernel, ftq_tq_v1.cuh) where a split that a share's end cut lies in the workspace in pieces: they
 // are put together, written to mid_o and merged.  Two warps per row, an octet per split, the eight octets side by side; the
 // pieces of a split kPieceBatch at a time (four took more registers: 4096 whole rows 23 us, 18 with two).  The latency of the
@@ -813,13 +866,13 @@ tq_flow_kernel(const __grid_constant__ TqFlowParams f) {
 // call, 32 so).
 template <int D, typename OT>
 __global__ void __launch_bounds__(128)
-tq_join_kernel(const __grid_constant__ TqMergeParams p) {
+tq_join_kernel(const __grid_constant__ TqJoinParams p) {
     constexpr int E = D / kOctet, kPieceBatch = 2;
     __shared__ float part[2][kOctet][E + 2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 7;
     const int which = warp >> 1, oct = 4 * (warp & 1) + (lane >> 3);
     const int64_t at = static_cast<int64_t>(blockIdx.x) * 2 + which;
-    const int64_t row = at < p.n_rows ? at : p.n_rows - 1;
+    const int64_t row = at < p.m.n_rows ? at : p.m.n_rows - 1;
     const uint32_t r = fast_div(static_cast<uint32_t>(row), p.div_hq);   // (layer, sequence)
     const int h = static_cast<int>(static_cast<uint32_t>(row) - r * p.Hq);
     const uint32_t layer = fast_div(r, p.div_bseq);
@@ -833,9 +886,9 @@ tq_join_kernel(const __grid_constant__ TqMergeParams p) {
     float M = -INFINITY, l = 0.f, a[E];
 #pragma unroll
     for (int i = 0; i < E; i++) a[i] = 0.f;
-    for (int s0 = 0; s0 < p.splits; s0 += kOctet) {
+    for (int s0 = 0; s0 < p.m.splits; s0 += kOctet) {
         // lane t: pages of split s0 + t; its place in the line
-        const uint32_t pages = s0 + t < p.splits ? tq_range_pages(tq_split_range(len, start, p.splits, s0 + t)) : 0;
+        const uint32_t pages = s0 + t < p.m.splits ? tq_range_pages(tq_split_range(len, start, p.m.splits, s0 + t)) : 0;
         uint32_t upto = pages > 0 ? pages + p.piece_cost : 0;
 #pragma unroll
         for (int m = 1; m < kOctet; m <<= 1) {
@@ -848,7 +901,7 @@ tq_join_kernel(const __grid_constant__ TqMergeParams p) {
         if (n == 0 || share == 0) continue;
         const uint32_t c0 = first / share, c1 = (first + n - 1) / share;
         const bool cut = c0 != c1;
-        float* const mid = p.mid_out + (row * p.splits + s0 + oct) * (D + 1);
+        float* const mid = p.mid_out + (row * p.m.splits + s0 + oct) * (D + 1);
         // (row block 0 is the piece the share starts with, 1 its last one)
         auto source = [&](uint32_t c) {
             return cut ? p.rows + ((2 * (shares0 + c) + (c * share >= first ? 0 : 1)) * p.Hq + h) * (D + 2) : mid;
@@ -935,7 +988,7 @@ tq_join_kernel(const __grid_constant__ TqMergeParams p) {
     __syncthreads();
     if (warp & 1) return;
     join(part[which][t][E], part[which][t][E + 1], [&](int i) { return part[which][t][i]; });
-    tq_finish_row<D, OT, 4>(p, static_cast<OT*>(p.out), p.lse, row, a, l, M, lane, at < p.n_rows);
+    tq_finish_row<D, OT, 4>(p.m, static_cast<OT*>(p.m.out), p.m.lse, row, a, l, M, lane, at < p.m.n_rows);
 }
 
 }  // namespace ftq

@@ -302,8 +302,8 @@ static cudaError_t flow_by_vb(int vb, int nh, const TqFlowParams& p, cudaStream_
 }
 // (launched while stage 1 drains: it waits for stage 1's end itself)
 template <typename OT>
-static cudaError_t join_run(const TqMergeParams& p, cudaStream_t stream) {
-    return launch_dependent(tq_join_kernel<FTQ_D, OT>, static_cast<unsigned>((p.n_rows + 1) / 2), 128, 0, stream, p);
+static cudaError_t join_run(const TqJoinParams& p, cudaStream_t stream) {
+    return launch_dependent(tq_join_kernel<FTQ_D, OT>, static_cast<unsigned>((p.m.n_rows + 1) / 2), 128, 0, stream, p);
 }
 #endif
 // FTQ_ONLY_BITS=<b>: key and value codes of b bits only (the wait-expiry test library)
@@ -320,7 +320,7 @@ cudaError_t FTQ_CAT(launch_tq_flow_d, FTQ_D)(int kb, int vb, int nh, const TqFlo
 #endif
     return cudaErrorInvalidValue;
 }
-cudaError_t FTQ_CAT(launch_tq_join_d, FTQ_D)(int out_dtype, const TqMergeParams& p, cudaStream_t stream) {
+cudaError_t FTQ_CAT(launch_tq_join_d, FTQ_D)(int out_dtype, const TqJoinParams& p, cudaStream_t stream) {
 #if FTQ_D != 256
     switch (out_dtype) {
         case kF32: return join_run<float>(p, stream);

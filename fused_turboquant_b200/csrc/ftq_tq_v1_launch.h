@@ -28,7 +28,7 @@ constexpr int kTqLloydMaxValues = 2;  // 4-bit values: Lloyd-Max codes against t
                                     cudaStream_t stream);                                         \
     cudaError_t launch_tq_flow_d##DD(int kb, int vb, int nh, const TqFlowParams& p, cudaStream_t stream); \
     cudaError_t launch_tq_merge_d##DD(int out_dtype, const TqMergeParams& p, cudaStream_t stream); \
-    cudaError_t launch_tq_join_d##DD(int out_dtype, const TqMergeParams& p, cudaStream_t stream);
+    cudaError_t launch_tq_join_d##DD(int out_dtype, const TqJoinParams& p, cudaStream_t stream);
 
 FTQ_DECLARE_TQ_LAUNCHERS(64)
 FTQ_DECLARE_TQ_LAUNCHERS(128)

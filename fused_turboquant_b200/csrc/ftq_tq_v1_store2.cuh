@@ -4,8 +4,8 @@
 //
 // tq_store_kernel issues some 59 instructions per coordinate (15-way midpoint search by selects, scalar
 // butterflies with a shuffle per lane bit, two IEEE divisions), which bounds it: 16384 tokens of 8 heads of 128,
-// 4-bit keys and rotated 4-bit values in bf16, took 70 us.  This one issues 23 and takes 41.  Here a lane carries TWO vectors in packed fp32
-// pairs (each half an ordinary IEEE operation, in the same order), the transposition goes through shared memory,
+// 4-bit keys and rotated 4-bit values in bf16, took 70 us.  This one issues 23 and takes 38.  Here a lane carries TWO
+// vectors in packed fp32 pairs (each half an ordinary IEEE operation, in the same order), the transposition goes through shared memory,
 // and
 //  * x / den is q = x r (r the correctly rounded reciprocal) corrected twice with exact FMA residuals, which is
 //    the correctly rounded quotient as long as nothing underflows on the way;

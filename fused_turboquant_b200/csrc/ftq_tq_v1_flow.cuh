@@ -12,7 +12,7 @@
 // page, with an online-softmax state of its own.  The warps of a head fold their states at the end of a
 // piece; nothing synchronises the whole CTA after the set-up.  (A warp that copied the slots of its own
 // pages word by word through registers spent 722 instructions a page and head on it: 32 x 8192 tokens of
-// 8 heads, 4-bit keys and values, took 182 us; this way 122.)
+// 8 heads, 4-bit keys and values, took 182 us; this way 113.)
 //
 // Work: the pages of a layer's (sequence, split) units lie in one line, each unit's behind piece_cost places without a page
 // (what a piece costs beside its pages: queries, the fold, the rows), and the line is cut into equal shares, at most one per

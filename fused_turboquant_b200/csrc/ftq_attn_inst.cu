@@ -54,9 +54,9 @@ cudaError_t FTQ_CAT(launch_attn_split_d, FTQ_D)(int bits_k, int bits_v, bool pag
 
 // The streaming kernel (no CTA-wide barriers, merge included) serves the configurations in
 // which it was measured faster than the equal-share one: a 4-bit byte table (one CTA per SM) with
-// a GQA group of at most 4 -- 16 warps at head_dim 64 / 128, 8 warps at head_dim 256 (16 rings and
+// a GQA group of at most 4 -- 16 warps at head_dim 64 / 128, 12 or 8 at head_dim 256 (16 rings and
 // exchange slots do not fit beside the table there).  Measured on B200, streaming against equal
-// shares, store included: 879 : 1137 us for the ragged head_dim-256 K4V2 batch, 21.5 : 25.1 us for
+// shares, store included: 777 : 1137 us for the ragged head_dim-256 K4V2 batch, 21.5 : 25.1 us for
 // one sequence of 900 tokens, 142 : 141 us for 64 x 8192 tokens of 8 K4V4 heads.
 template <int BK, int BV, int NH>
 constexpr bool use_stream_kernel() {
@@ -66,7 +66,7 @@ constexpr bool use_stream_kernel() {
 #elif defined(FTQ_ALL_STREAM)
     return S::FITS;
 #else
-    return S::FITS && S::BYTE && NH == 1 && (S::WARPS == 16 || FTQ_D == 256);
+    return S::FITS && S::BYTE && NH == 1;
 #endif
 }
 

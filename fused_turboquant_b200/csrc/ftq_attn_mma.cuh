@@ -243,6 +243,19 @@ __device__ __forceinline__ uint32_t entry_addr(const uint32_t (&w)[NW], int pair
     }
 }
 
+// The sixteen 2-bit codes c0 .. c15 of a word as fp16 centroid pairs, without a table: a byte-permute picks
+// the two bytes of a centroid out of the eight of all four (`lo` = centroids 0 and 1, `hi` = 2 and 3).  Its
+// selector is 2c, 2c + 1, i.e. 0x22 * c + 0x10, for four codes at a time.  x[2i] = (c[i], c[i + 4]),
+// x[2i + 1] = (c[i + 8], c[i + 12]).
+__device__ __forceinline__ void select_pairs2(uint32_t w, uint32_t lo, uint32_t hi, uint32_t (&x)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t m = (w >> (2 * i)) & 0x03030303u;
+        x[2 * i] = __byte_perm(lo, hi, m * 0x22u + 0x10101010u);
+        x[2 * i + 1] = __byte_perm(lo, hi, (m * 0x22u + 0x10101010u) >> 16);
+    }
+}
+
 template <int D, int BK, int BV, int NH>
 struct MmaCfg {
     static constexpr int NKB = D / 16;                  // k-blocks of K.Q^T

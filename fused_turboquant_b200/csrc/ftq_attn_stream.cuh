@@ -62,7 +62,13 @@ struct StreamCfg {
     static constexpr bool BYTE = M::BYTE;
     static constexpr int PAGE_BYTES = M::PAGE_BYTES;
     static constexpr int RING = 2;
-    static constexpr bool QSMEM = D == 256;                       // query fragments stay in shared memory
+    // 2-bit values of heads of 256: one of the two words of a lane's slice goes to centroids by byte-permutes
+    // (select_pairs2), the other through the table: the first loads the ALU pipe (19 of its instructions for
+    // 16 codes), the second the shared-memory pipe (8 wavefronts).  Measured on the ragged batch of 256 x up to 32768
+    // tokens, 16 / 8 heads, K4V2, with 12 warps: 829 us by look-ups alone, 777 half and half, 895 by permutes
+    // alone.  At head_dim 128 a slice is one word: 144 us by permutes, 114 by look-ups (64 x 8192 tokens).
+    static constexpr int V2P = BV == 2 && D == 256 ? 1 : 0;
+
     static constexpr int QFRAG_BYTES = NH * NKB * 32 * 8;         // per metadata buffer
     static constexpr int QS_BYTES = 2 * 8 * (D + 16) * 4;         // fp32 rotated queries (2 scratch blocks)
     static constexpr int CTL_BYTES = 256 + 2 * 32 * 4;            // control words + per-warp addresses
@@ -117,11 +123,12 @@ struct StreamCfg {
         }
         return worst + 128;
     }
-    // one CTA per SM around a 64 KB byte table (16 warps when their rings and exchange slots fit
-    // beside it, else 8); two 8-warp CTAs per SM with the small tables of 3- and 2-bit codes
+    // one CTA per SM around a 64 KB byte table: as many warps as their rings and exchange slots fit beside it, in steps
+    // of one per scheduler (16 at head_dim 64 / 128; 12 or 8 at 256: 777 against 902 us for the ragged K4V2 batch
+    // above); two 8-warp CTAs per SM with the small tables of 3- and 2-bit codes
     static constexpr int CTAS_PER_SM = BYTE ? 1 : 2;
     static constexpr int LIMIT_CTA = BYTE ? LIMIT : LIMIT / 2 - 1024;
-    static constexpr int WARPS = (BYTE && need(16) <= LIMIT_CTA) ? 16 : 8;
+    static constexpr int WARPS = !BYTE ? 8 : need(16) <= LIMIT_CTA ? 16 : need(12) <= LIMIT_CTA ? 12 : 8;
     static constexpr int THREADS = 32 * WARPS;
     static constexpr int SMEM_BYTES = need(WARPS);
     static constexpr bool FITS = SMEM_BYTES <= LIMIT_CTA;
@@ -325,6 +332,12 @@ attn_stream_kernel(const AttnParams p, int n_items) {
     const uint32_t lv_lane =
         C::V2BYTE ? (window | 128u | ((lane & 15) * 8))
                   : ((BV == 4 ? (window | (SHARED_LUT ? 0u : 128u)) : tv_small) | (lane * 4));
+    uint32_t v2lo = 0, v2hi = 0;
+    if constexpr (S::V2P > 0) {
+        const __half2 a = __floats2half2_rn(p.lv_scaled.v[0], p.lv_scaled.v[1]), b = __floats2half2_rn(p.lv_scaled.v[2], p.lv_scaled.v[3]);
+        v2lo = *reinterpret_cast<const uint32_t*>(&a);
+        v2hi = *reinterpret_cast<const uint32_t*>(&b);
+    }
     // Everything up to here touched shared memory only.  From here on the kernel reads and writes
     // global memory that the kernel before it in the stream may still be using (the workspace).
     after_previous_kernel();
@@ -616,23 +629,20 @@ attn_stream_kernel(const AttnParams p, int n_items) {
 
     // ---- per-item arithmetic state
     int ntok_item = ctl[kCtlTokens + s0];
-    uint32_t qb[S::QSMEM ? 1 : NH][S::QSMEM ? 1 : NKB][2];
-    uint32_t qf_item = qfrag + s0 * S::QFRAG_BYTES;  // fragment base of the current item (QSMEM)
+    uint32_t qb[NH][NKB][2];
     float m_run[NH], l_run[NH], oacc[NH][NMT][4];
     auto load_ctx = [&](int seq) {
         const int buf = seq & 1;
         ntok_item = ctl[kCtlTokens + buf];
-        qf_item = qfrag + buf * S::QFRAG_BYTES;
-        if constexpr (!S::QSMEM) {
+        const uint32_t qf_item = qfrag + buf * S::QFRAG_BYTES;
 #pragma unroll
-            for (int hh = 0; hh < NH; hh++)
+        for (int hh = 0; hh < NH; hh++)
 #pragma unroll
-                for (int kb = 0; kb < NKB; kb++) {
-                    const uint2 v = lds64(qf_item + ((hh * NKB + kb) * 32 + lane) * 8);
-                    qb[hh][kb][0] = v.x;
-                    qb[hh][kb][1] = v.y;
-                }
-        }
+            for (int kb = 0; kb < NKB; kb++) {
+                const uint2 v = lds64(qf_item + ((hh * NKB + kb) * 32 + lane) * 8);
+                qb[hh][kb][0] = v.x;
+                qb[hh][kb][1] = v.y;
+            }
     };
     auto reset_state = [&]() {
 #pragma unroll
@@ -690,15 +700,8 @@ attn_stream_kernel(const AttnParams p, int n_items) {
             const uint32_t a3 = lut32(entry_addr<C::IWK>(r.k[1], 2 * kb + 1, lk_lane));
 #pragma unroll
             for (int hh = 0; hh < NH; hh++) {
-                uint32_t b0, b1;
-                if constexpr (S::QSMEM) {
-                    const uint2 qv = lds64(qf_item + ((hh * NKB + kb) * 32 + lane) * 8);
-                    b0 = qv.x; b1 = qv.y;
-                } else {
-                    b0 = qb[hh][kb][0]; b1 = qb[hh][kb][1];
-                }
-                if (kb < 2) mma_16816_z(c[hh][kb & 1], a0, a1, a2, a3, b0, b1);
-                else mma_16816(c[hh][kb & 1], a0, a1, a2, a3, b0, b1);
+                if (kb < 2) mma_16816_z(c[hh][kb & 1], a0, a1, a2, a3, qb[hh][kb][0], qb[hh][kb][1]);
+                else mma_16816(c[hh][kb & 1], a0, a1, a2, a3, qb[hh][kb][0], qb[hh][kb][1]);
             }
         }
     };
@@ -774,11 +777,20 @@ attn_stream_kernel(const AttnParams p, int n_items) {
 
     auto pv_accum = [&](const uint32_t (&v)[4][(C::VSB + 3) / 4], const uint32_t (&pb)[NH][2][2]) {
 #pragma unroll
-        for (int ks = 0; ks < 2; ks++)
+        for (int ks = 0; ks < 2; ks++) {
+            uint32_t xs[S::V2P + 1][2][8];
+#pragma unroll
+            for (int w = 0; w < S::V2P; w++) {
+                select_pairs2(v[2 * ks][w], v2lo, v2hi, xs[w][0]);
+                select_pairs2(v[2 * ks + 1][w], v2lo, v2hi, xs[w][1]);
+            }
 #pragma unroll
             for (int mt = 0; mt < NMT; mt++) {
                 uint32_t a0, a1, a2, a3;
-                if constexpr (C::V2BYTE) {
+                if (mt < 4 * S::V2P) {
+                    a0 = xs[mt / 4][0][2 * (mt % 4)]; a1 = xs[mt / 4][0][2 * (mt % 4) + 1];
+                    a2 = xs[mt / 4][1][2 * (mt % 4)]; a3 = xs[mt / 4][1][2 * (mt % 4) + 1];
+                } else if constexpr (C::V2BYTE) {
                     const uint2 lo = lut64(entry_addr<8>(v[2 * ks], mt, lv_lane));
                     const uint2 hi = lut64(entry_addr<8>(v[2 * ks + 1], mt, lv_lane));
                     a0 = lo.x; a1 = lo.y; a2 = hi.x; a3 = hi.y;
@@ -792,6 +804,7 @@ attn_stream_kernel(const AttnParams p, int n_items) {
                 for (int hh = 0; hh < NH; hh++)
                     mma_16816(oacc[hh][mt], a0, a1, a2, a3, pb[hh][ks][0], pb[hh][ks][1]);
             }
+        }
     };
 
     // ---- fold service for item number seq (warp 0, after it has published its own state): fold
@@ -906,14 +919,15 @@ attn_stream_kernel(const AttnParams p, int n_items) {
         }
         if (!stalled && !wait_ge(kCtlReduced, seq - 1)) stalled = true;
         float* xml = reinterpret_cast<float*>(my_xchg + 32 * C::STATE_F4);
+        auto out_of = [&](int hh, int mt, int i) { return mt < 4 * S::V2P ? oacc[hh][4 * (mt / 4) + i][mt % 4] : oacc[hh][mt][i]; };
 #pragma unroll
         for (int hh = 0; hh < NH; hh++) {
             if (m_run[hh] != -INFINITY) {  // (warp-uniform per head half: the reference is shared)
 #pragma unroll
                 for (int mt = 0; mt < NMT; mt++)
                     my_xchg[(hh * NMT + mt) * 32 + lane] = make_float4(
-                        oacc[hh][mt][0] * p.inv_v_scale, oacc[hh][mt][1] * p.inv_v_scale,
-                        oacc[hh][mt][2] * p.inv_v_scale, oacc[hh][mt][3] * p.inv_v_scale);
+                        out_of(hh, mt, 0) * p.inv_v_scale, out_of(hh, mt, 1) * p.inv_v_scale,
+                        out_of(hh, mt, 2) * p.inv_v_scale, out_of(hh, mt, 3) * p.inv_v_scale);
             }
             if (g == 0) {
                 xml[(hh * 2 + 0) * 4 + tg] = stalled ? __int_as_float(0x7fc00000) : m_run[hh];
@@ -945,7 +959,7 @@ attn_stream_kernel(const AttnParams p, int n_items) {
     // independent and sit in one straight-line block.  One register set serves both: the
     // values of a page are read from its ring buffer only after P.V of the page before has
     // consumed the value registers, and the buffer is released after that read.
-    constexpr bool kPipelined = NH == 1 && !S::QSMEM;
+    constexpr bool kPipelined = NH == 1;
     Regs r;
     uint32_t pb[NH][2][2];
     float c[NH][2][4];

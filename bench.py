@@ -822,9 +822,7 @@ def main():
         value = total_bytes_step / (ms_step * 1e-3) / 1e9
         bytes_call = s.bytes_layer * s.layers_per_call
         traffic, traffic_src = load_traffic(args.workload, s.layers_per_call)
-        # one kernel per call (merge and counter reset inside): the streaming kernel for 4-bit keys
-        # with a GQA group of at most 4, the equal-share kernel for the other configurations
-        stream = w["bk"] == 4 and w["Hq"] // w["Hkv"] <= 4
+        # (one kernel per call: merge and counter reset inside)
         # Duration of the kernel's launch.  Where a step is nothing but such calls back to back, it is
         # the timed region divided by its launches (gaps between launches included).  Otherwise (a
         # collective inside the step) it is the event-timed duration of one call, timed call by call.
@@ -846,8 +844,7 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_src,
                          "peak_source": peak_src, "frac_of_nominal_8000": achieved / 8000.0,
-                         "kernel": ("attn_stream_kernel" if stream else "attn_flow_kernel")
-                                   + " (one ftq_paged_decode_attn call = this one kernel)"
+                         "kernel": "attn_flow_kernel (one ftq_paged_decode_attn call = this one kernel)"
                                    + ", %d layer(s)" % s.layers_per_call,
                          "bytes_per_launch": bytes_call, "ms_per_launch": launch_ms,
                          "ms_per_call_timed_alone": call_ms},

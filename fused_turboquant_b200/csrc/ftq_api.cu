@@ -270,50 +270,7 @@ float choose_k_scale(const float* levels, int bits, int head_dim) {
 
 struct ChunkPlan {
     int chunk_tokens, n_chunks, n_hpass;
-    // tensor-core kernels: units from bulk_units on are cut into tail_chunks chunks of
-    // tail_chunk_tokens instead, and the last tail_b_units of them into one chunk more
-    // (bulk_units < 0: one split for all units)
-    int64_t bulk_units = -1;
-    int tail_chunks = 0, tail_chunk_tokens = 0;
-    int64_t tail_b_units = 0;
-    int tail_b_chunks = 0, tail_b_chunk_tokens = 0;
-    int row_chunks() const {
-        int m = n_chunks;
-        if (tail_chunks > m) m = tail_chunks;
-        if (tail_b_units > 0 && tail_b_chunks > m) m = tail_b_chunks;
-        return m;
-    }
 };
-
-// The device-side description of a plan over `units` units.
-ftq::SplitPlan make_split(const ChunkPlan& pl, int64_t units) {
-    ftq::SplitPlan sp{};
-    auto put = [&](int k, int64_t first_unit, int64_t first_item, int chunks, int tokens) {
-        sp.r[k].first_unit = static_cast<int>(first_unit);
-        sp.r[k].first_item = static_cast<int>(first_item);
-        sp.r[k].chunks = chunks;
-        sp.r[k].chunk_tokens = tokens;
-        sp.r[k].div_chunks = ftq::make_fastdiv(static_cast<uint32_t>(chunks));
-    };
-    const int64_t bulk = pl.bulk_units >= 0 ? pl.bulk_units : units;
-    put(0, 0, 0, pl.n_chunks, pl.chunk_tokens);
-    sp.n_regions = 1;
-    int64_t items = bulk * pl.n_chunks;
-    if (bulk < units) {
-        const int64_t a_units = units - bulk - pl.tail_b_units;
-        if (a_units > 0) {
-            put(sp.n_regions++, bulk, items, pl.tail_chunks, pl.tail_chunk_tokens);
-            items += a_units * pl.tail_chunks;
-        }
-        if (pl.tail_b_units > 0) {
-            put(sp.n_regions++, bulk + a_units, items, pl.tail_b_chunks, pl.tail_b_chunk_tokens);
-            items += pl.tail_b_units * pl.tail_b_chunks;
-        }
-    }
-    sp.row_chunks = pl.row_chunks();
-    sp.total_items = static_cast<int>(items);
-    return sp;
-}
 
 // Plans are pure functions of a few sizes, and finding one walks up to a thousand candidates (up
 // to 60 us on the host for a 128k context): each thread keeps the last ones it made.  Contexts are
@@ -389,103 +346,10 @@ ChunkPlan plan_chunks_uniform(int B, int Hq, int Hkv, int d, int seq_len) {
     });
 }
 
-// Chunking of the tensor-core path (persistent CTAs): few, large chunks keep the per-item
-// fixed costs small, more chunks fill the last wave of CTA slots better; the plan with the
-// lowest modelled cost wins.  Chunks hold at most 8192 tokens (short enough for the dynamic
-// hand-out of items to even out ragged batches; their block ids are staged in shared memory)
-// and at least 1024.
-// The streaming kernel's planner.  Cost of a plan = waves of items over the CTA slots
-// x (pages of an item + the fixed cost of an item, in pages); the cheapest plan wins, the fewest
-// chunks among equals.  A plan has up to two regions: as many units as fill whole waves of the
-// grid are cut into few, long chunks; the remaining units into more, shorter ones that share the
-// last wave.  Items are handed out bulk first, so the short ones also even out the CTAs'
-// different speeds.
-ChunkPlan plan_two_regions(int64_t units, int64_t slots, int max_seq_len, double item_cost) {
-    ChunkPlan pl;
-    pl.n_hpass = 1;
-    const int seq = max_seq_len > 0 ? max_seq_len : 1;
-    const int c_min = (seq + 8191) / 8192;
-    const int c_max = (seq + 1023) / 1024 > c_min ? (seq + 1023) / 1024 : c_min;
-    auto split = [&](int nc, int* ct, int* real) {
-        int t = ((seq + nc - 1) / nc + 63) / 64 * 64;
-        if (t > 8192) t = 8192;
-        *ct = t;
-        *real = (seq + t - 1) / t;
-    };
-    double best = -1.0;
-    for (int nc1 = c_min; nc1 <= c_max && nc1 < c_min + 64; nc1++) {
-        int ct1, r1;
-        split(nc1, &ct1, &r1);
-        const double cost1 = ct1 / 16.0 + item_cost;
-        // one split for all units
-        const double uniform = static_cast<double>((units * r1 + slots - 1) / slots) * cost1;
-        if (best < 0.0 || uniform < best * (1.0 - 1e-9)) {
-            best = uniform;
-            pl.chunk_tokens = ct1; pl.n_chunks = r1;
-            pl.bulk_units = -1; pl.tail_chunks = 0; pl.tail_chunk_tokens = 0;
-        }
-        // whole waves of this split, the rest of the units cut finer
-        const int64_t full = units * r1 / slots;
-        const int64_t bulk = full * slots / r1;
-        if (full == 0 || bulk >= units) continue;
-        for (int nc2 = nc1 + 1; nc2 <= c_max && nc2 <= nc1 + 16; nc2++) {
-            int ct2, r2;
-            split(nc2, &ct2, &r2);
-            if (r2 <= r1) continue;
-            const int64_t tail_waves = ((units - bulk) * r2 + slots - 1) / slots;
-            const double cost = static_cast<double>(full) * cost1 +
-                                static_cast<double>(tail_waves) * (ct2 / 16.0 + item_cost);
-            if (cost < best * (1.0 - 1e-9)) {
-                best = cost;
-                pl.chunk_tokens = ct1; pl.n_chunks = r1;
-                pl.bulk_units = bulk; pl.tail_chunks = r2; pl.tail_chunk_tokens = ct2;
-            }
-        }
-    }
-    // The CTAs differ in speed by a few percent on identical items (measured), and a last wave
-    // with fewer items than CTAs leaves the fastest ones idle.  So some of the tail units get
-    // one chunk more, enough for the last wave to hold an item for every CTA: the ticket order
-    // hands the longer items to the CTAs that arrive first and the shorter ones to the late ones.
-    pl.tail_b_units = 0;
-    if (pl.bulk_units >= 0) {
-        const int64_t tail_units = units - pl.bulk_units;
-        const int64_t items = tail_units * pl.tail_chunks;
-        const int64_t missing = (items + slots - 1) / slots * slots - items;
-        int ct3, r3;
-        split(pl.tail_chunks + 1, &ct3, &r3);
-        if (missing > 0 && missing <= tail_units && r3 == pl.tail_chunks + 1 && r3 <= c_max) {
-            pl.tail_b_units = missing;
-            pl.tail_b_chunks = r3;
-            pl.tail_b_chunk_tokens = ct3;
-        }
-    }
-    return pl;
-}
-
-// The streaming kernel.  Measured on B200 (Llama-shaped K4V4 batches of 37..111
-// sequences, forced chunk counts): an item costs about 74 pages on top of its own pages (the
-// service warps' smaller page share, the publish / fold / prepare hand-overs), so long chunks
-// pay -- but whole waves of them rarely match the unit count, hence the two regions.
-ChunkPlan plan_chunks_stream(int B, int Hkv, int max_seq_len, int n_layers, int ctas_per_sm) {
-    const int seq = round_seq(max_seq_len), slots = ftq::sm_count() * ctas_per_sm;
-    return remembered<ChunkPlan>({2, B, 0, Hkv, 0, seq, n_layers, slots}, [&] {
-        return plan_two_regions(static_cast<int64_t>(B) * Hkv * n_layers, slots, seq, 74.0);
-    });
-}
-
-int attn_mma_stream_ctas(int d, int bits_k, int bits_v, int group) {
-    switch (d) {
-        case 64: return ftq::attn_mma_stream_ctas_d64(bits_k, bits_v, group);
-        case 128: return ftq::attn_mma_stream_ctas_d128(bits_k, bits_v, group);
-        case 256: return ftq::attn_mma_stream_ctas_d256(bits_k, bits_v, group);
-    }
-    return 0;
-}
-
 bool use_mma_path(int Hq, int Hkv, int q_dtype) { return Hq / Hkv <= 8 && q_dtype != FTQ_F32; }
 
 size_t partial_bytes(const ChunkPlan& pl, int B, int Hq, int d, int n_layers) {
-    return static_cast<size_t>(n_layers) * B * Hq * pl.row_chunks() * (d + 4) * sizeof(float);
+    return static_cast<size_t>(n_layers) * B * Hq * pl.n_chunks * (d + 4) * sizeof(float);
 }
 
 cudaError_t dispatch_split(int d, int bk, int bv, bool paged, const ftq::AttnParams& p, int n_lb,
@@ -783,14 +647,8 @@ size_t ftq_decode_workspace_bytes(int B, int Hq, int Hkv, int head_dim, int max_
     // the larger of the paths' needs, so one buffer serves whichever kernel runs
     const int seq = round_seq(max_seq_len);
     return remembered<size_t>({0, B, Hq, Hkv, head_dim, seq, n_layers, ftq::sm_count()}, [&] {
-        size_t n = 0;
-        for (const ChunkPlan& pl : {plan_chunks(B, Hq, Hkv, head_dim, seq, n_layers),
-                                    plan_chunks_stream(B, Hkv, seq, n_layers, 1),
-                                    plan_chunks_stream(B, Hkv, seq, n_layers, 2)}) {
-            const size_t m = partial_bytes(pl, B, Hq, head_dim, n_layers);
-            n = m > n ? m : n;
-        }
-        // the equal-share kernel (groups of at most 8): two blocks of rows per CTA, at most two CTAs per SM
+        const size_t n = partial_bytes(plan_chunks(B, Hq, Hkv, head_dim, seq, n_layers), B, Hq, head_dim, n_layers);
+        // the equal-share kernel (groups of at most 8): two blocks of rows for each half of a CTA, one CTA per SM
         const size_t flow = Hq / Hkv > 8 ? 0 : static_cast<size_t>(ftq::sm_count()) * 4 * (Hq / Hkv) * (head_dim + 4) * sizeof(float);
         return flow > n ? flow : n;
     }) + counter_bytes(B, Hkv, n_layers);
@@ -926,11 +784,7 @@ int ftq_paged_decode_attn(const void* q, int q_dtype, void* out, int out_dtype,
     // 16-bit queries with a GQA group of at most 8 take the tensor-core kernel; fp32 queries
     // (and larger groups) take the fp32 kernel.
     const bool mma = use_mma_path(Hq, Hkv, q_dtype);
-    const int stream_ctas = mma ? attn_mma_stream_ctas(head_dim, bits_k, bits_v, Hq / Hkv) : 0;
-    const bool streams = stream_ctas > 0;
-    const ChunkPlan pl = streams ? plan_chunks_stream(B, Hkv, max_seq_len, n_layers, stream_ctas)
-                         : mma   ? ChunkPlan{}
-                                 : plan_chunks(B, Hq, Hkv, head_dim, round_seq(max_seq_len), n_layers);
+    const ChunkPlan pl = mma ? ChunkPlan{} : plan_chunks(B, Hq, Hkv, head_dim, round_seq(max_seq_len), n_layers);
     const size_t need = ftq_decode_workspace_bytes(B, Hq, Hkv, head_dim, max_seq_len, n_layers);
     if (!workspace || workspace_bytes < need)
         return fail(FTQ_ERR_WORKSPACE, "workspace needs %zu bytes, got %zu", need, workspace_bytes);
@@ -972,13 +826,10 @@ int ftq_paged_decode_attn(const void* q, int q_dtype, void* out, int out_dtype,
         p.out = out;
         p.out_dtype = out_dtype;
         p.num_blocks = num_blocks;
-        p.div_hkv = ftq::make_fastdiv(static_cast<uint32_t>(Hkv));
-        p.div_b = ftq::make_fastdiv(static_cast<uint32_t>(B));
         p.n_units = n_layers * B * Hkv;
         p.epoch = next_epoch();
         p.n_layers = n_layers;
         p.max_seq = max_seq_len;
-        if (streams) p.split = make_split(pl, p.n_units);
         e = dispatch_mma(head_dim, bits_k, bits_v, shared_lut, p, st);   // (merge included)
         return e == cudaSuccess ? FTQ_OK : cuda_fail(e, "ftq_paged_decode_attn launch");
     }

@@ -26,33 +26,6 @@ namespace ftq {
 
 constexpr int kFlowMaxSeqs = 1024;       // sequences per launch (their prefix sums lie in shared memory)
 
-// How the tensor-core decode kernels cut the (layer, sequence, KV head) units into work items: up
-// to three regions of consecutive units, each with its own chunk length -- few long chunks for
-// the units that fill whole waves of the grid, shorter ones for the rest, sized so that the last
-// wave has an item for every CTA (the longer ones first: the CTAs that arrive last get the short
-// ones).  Items are numbered region by region: item = r.first_item + (unit - r.first_unit) *
-// r.chunks + chunk.  A unit owns row_chunks chunk rows of the partials buffer whatever its region.
-struct SplitRegion {
-    int first_unit, first_item, chunks, chunk_tokens;
-    FastDiv div_chunks;
-};
-struct SplitPlan {
-    SplitRegion r[3];
-    int n_regions, row_chunks, total_items;
-};
-__host__ __device__ __forceinline__ const SplitRegion& region_of_item(const SplitPlan& s, int item) {
-    int k = 0;
-    if (s.n_regions > 1 && item >= s.r[1].first_item) k = 1;
-    if (s.n_regions > 2 && item >= s.r[2].first_item) k = 2;
-    return s.r[k];
-}
-__host__ __device__ __forceinline__ const SplitRegion& region_of_unit(const SplitPlan& s, int unit) {
-    int k = 0;
-    if (s.n_regions > 1 && unit >= s.r[1].first_unit) k = 1;
-    if (s.n_regions > 2 && unit >= s.r[2].first_unit) k = 2;
-    return s.r[k];
-}
-
 struct AttnParams {
     const void* q;              // [L*B, Hq, D]
     // paged source
@@ -74,31 +47,25 @@ struct AttnParams {
     int cp16;                   // contiguous source: every span 16-byte aligned
     int chunk_tokens, n_chunks, n_hpass;
     float* partials;            // [L*B*Hq][row_chunks][D + 4]
-    // Tensor-core kernels: how the (layer, sequence, KV head) units are cut into work items (see
-    // SplitPlan).  The fp32 kernels use one split for all units: n_chunks / chunk_tokens above.
-    SplitPlan split;
-    // Counters of the tensor-core kernels, which clear them themselves: CTA 0 zeroes work_counter[0]
-    // (tickets of the streaming kernel), work_counter[1] (CTAs that have left) and the unit counters,
-    // then stores `epoch` (unique per call, never 0) into the 64-bit word at work_counter + 2;
-    // everybody checks for it before the first atomic on a counter, and the last CTA to leave stores 0
-    // there, so that a replay of the same launch, or the call's next launch, does not find its own
-    // epoch.
+    // Counters of the tensor-core kernel, which clears them itself: CTA 0 zeroes work_counter[1]
+    // (CTAs that have left) and the unit counters, then stores `epoch` (unique per call, never 0) into
+    // the 64-bit word at work_counter + 2; everybody checks for it before the first atomic on a
+    // counter, and the last CTA to leave stores 0 there, so that a replay of the same launch, or the
+    // call's next launch, does not find its own epoch.
     // work_counter[4] is the call's status word (kStatus* bits, cleared with the counters): what
     // the kernels of this call met; the host reads it on request (ftq_paged_decode_status).
     // nullptr for the contiguous entry points.
     int* work_counter;
-    // the tensor-core kernels finish the split-KV merge themselves
-    int* unit_counter;          // [n_units = L*B*Hkv] chunks or pieces delivered per unit
+    // the tensor-core kernel finishes the split-KV merge itself
+    int* unit_counter;          // [n_units = L*B*Hkv] pieces delivered per unit
     int n_units;
     unsigned long long epoch;
-    // equal-share tensor-core kernel: sequences b0 .. b0 + B - 1 of the batch's B_stride, n_layers
-    // layers; context lengths are cut to max_seq; pages per CTA at least min_share; a unit's counter
-    // holds 16 bits for each warp that finishes pieces
+    // tensor-core kernel: sequences b0 .. b0 + B - 1 of the batch's B_stride, n_layers layers; context
+    // lengths are cut to max_seq; places per share at least min_share
     int n_layers, b0, B_stride, max_seq, min_share;
     void* out;                  // [L*B, Hq, D]
     int out_dtype;
     int64_t num_blocks;         // block ids are checked against it
-    FastDiv div_hkv, div_b;     // divisions by Hkv, B
     Codebook lk, lv;
     SignBits signs;
     float rsqrt_d;

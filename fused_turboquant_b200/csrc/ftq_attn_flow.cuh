@@ -5,15 +5,20 @@
 // rotation of hf/fused_cache.py:579-581 and the page-table walk of vllm_plugin/cache_ops.py:151-205
 // folded in).  This file: how the work is split and put together again.
 //
-// The pages of all (layer, sequence, KV head) units lie in one line, unit after unit, and CTA c of
-// the persistent grid takes pages [c * share, (c + 1) * share): all CTAs have the same amount of
-// work whatever the lengths of the sequences are, a CTA's share crosses unit borders in at most
-// units / CTAs + 2 pieces, and a unit is cut only where a share ends.  (Cutting every unit into
-// equal chunks instead left the last wave of chunks up to half empty and paid the fixed cost of a
-// piece -- rotate the queries, fold the warps' states, about as long as 30 pages -- for every
-// chunk: 24 layers of 32 x 4096 tokens, 14 / 2 heads of 64, 3 bits, 173 us against 149 here; 4 x 131072,
-// 64 / 8 heads of 128, 189 against 155.)  The partition needs the
-// prefix sums of the page counts, which every CTA computes from seq_lens at its start.
+// One CTA per SM holds the dequantisation tables; its threads are two halves, each of which walks a share of the work
+// on its own (own queries, page rings, barriers): while one half folds, merges or waits for a piece's first pages, the
+// other one computes.  "CTA" below means such a half.
+//
+// The (layer, sequence, KV head) units lie in one line of places, unit after unit, a place for each page and PIECE more
+// for each unit, and CTA c of the persistent grid takes places [c * share, (c + 1) * share): all CTAs have the same amount
+// of work whatever the lengths of the sequences are, and a unit is cut only where a share ends.  PIECE is what a piece
+// costs on its own (rotate the queries, fold the warps' states, the first pages' latency).  Without it the CTAs whose
+// shares held many short sequences were the last by far: 40 sequences log-uniform up to 4000 tokens, 32 / 8 heads of 128,
+// K3V3, 59 -> 25 us; 100 up to 1000, 64 / 8 heads, K4V4, 85 -> 33.  (20 to 40 places measure alike, 8 and 60 up to half as
+// much again.)  The partition needs the prefix sums of the places, which every CTA computes from seq_lens at its start.
+// This kernel took the place of one that streamed pages across work items without CTA-wide barriers, tickets handing
+// out the items: 64 x 8192 tokens of 32 / 8 heads of 128, K4V4, 137 us there and 123 to 132 here, 24 sequences
+// log-uniform up to 30000 tokens 78 and 44, the ragged batch of 256 up to 32768, heads of 256, K4V2, 777 and 739.
 //
 // A piece is walked by the CTA's warps in stages of NP consecutive pages, dealt round-robin.  A
 // warp keeps RING stages in flight (1-D bulk copies, TMA); block ids are read straight from the
@@ -21,10 +26,13 @@
 // requested before this piece's states are folded.
 //
 // Pieces of a cut unit leave (O, m, l) rows in the workspace (two row blocks per CTA: a CTA's first
-// and last piece can be parts of units) and count themselves in; whoever arrives last merges the
-// rows, rotates back (core/hadamard.py:93-100) and stores.  A unit that one piece covers is
+// and last piece can be parts of units).  When its share is done a CTA counts them in; whoever arrives last
+// merges the rows, rotates back (core/hadamard.py:93-100) and stores.  A unit that one piece covers is
 // finished from shared memory.  Nobody waits for anybody.  The counters are cleared by CTA 0 under
 // the launch's epoch, as described at AttnParams.
+//
+// CLUSTER: few units with short contexts.  A cluster of CTAs has one unit, each half a part of its pages; the parts' (O,
+// m, l) stay in shared memory, and after a cluster barrier a warp per head merges them from there.
 //
 // Every wait is bounded (mbar_wait, the epoch); a wait that runs out turns the unit's rows into NaN
 // and sets a bit of the status word.  Block ids outside [0, num_blocks) are never dereferenced.
@@ -38,15 +46,112 @@ constexpr int kEpochSpinLimit = 1 << 22;
 
 // A piece of a CTA's share: pages [page0, page0 + n_pages) of one unit (n_pages = 0: none left).
 struct FlowPiece {
-    int64_t unit_start;   // first page of the unit on the line of all pages
+    int64_t unit_start;   // first place of the unit on the line of all places
     int64_t next;         // where the next piece starts
     int unit_pages, layer, b, hkv, page0, n_pages, tokens;
+    bool first;           // the share starts with it
 };
 
-template <int D, int BK, int BV, bool SHARED_LUT, int NH>
-__global__ void __launch_bounds__(MmaCfg<D, BK, BV, NH>::THREADS, MmaCfg<D, BK, BV, NH>::CTAS_PER_SM)
+template <int D, int BK, int BV, int NH, bool CLUSTER = false>
+struct FlowCfg : MmaCfg<D, BK, BV, NH> {
+    using M = MmaCfg<D, BK, BV, NH>;
+    static constexpr bool H8 = NH == 2;       // eight heads in the N dimension (see the fragment maps)
+    static constexpr int HL = H8 ? 2 : 1;     // heads whose softmax state a lane keeps: HL * tg + {0 ..}
+    static constexpr int NPB = H8 ? 1 : 2;    // P.V steps per page
+    // Lane (g, tg) reads slice g of page tokens 4tg .. 4tg + 3, one row per instruction.  Rows of whole
+    // power-of-two sizes put the quad's four rows (4 rows apart) on the same banks: each lane then
+    // starts at another of its four tokens.  24- and 48-byte rows (3 bits, head_dim 64 / 128) are
+    // apart as they are -- rotated they collide (20 extra wavefronts per page at head_dim 64).
+    static constexpr bool ROT = !(BV == 3 && D <= 128);
+    // per-warp ring of stages filled by bulk copies (TMA), one mbarrier per stage; a stage holds the
+    // NP consecutive pages a warp works on at a time
+    static constexpr int RING = 2;
+    // what a half (see attn_flow_kernel) has of its own: the queries; the folded piece, the warps' (m, l), mbarriers,
+    // ring addresses
+    static constexpr int QS_BYTES = 4 * NH * (D + 16) * 4;
+    __host__ __device__ static constexpr int misc_bytes(int warps) {
+        return 4 * NH * (D + 4) * 4 + warps * XML + warps * RING * 8 + warps * 4 + 64;
+    }
+    // a warp's share of the merge exchange area: its (O, m, l)
+    static constexpr int XSLOT = 32 * M::STATE_F4 * 16, XML = NH * 2 * 4 * 4;
+    static constexpr int PREFIX_BYTES = (kFlowMaxSeqs + 4) * 4;
+    // Objects are placed first-fit before / after the 64 KB-aligned table window, large ones first: every warp's ring, the
+    // exchange areas where they have their own space (`sep`: the first pages of the NEXT item can then
+    // already be copied into the rings while the merge runs; else a warp's share lies in its ring,
+    // which is idle during the merge), the queries, the misc blocks, the prefix sums.  Bytes needed from `base`.
+    __host__ __device__ static constexpr int ring_bytes(int np, bool sep) {
+        const int ring = RING * np * M::PAGE_BYTES;
+        return ((sep || ring > XSLOT ? ring : XSLOT) + 127) / 128 * 128;
+    }
+    __host__ __device__ static constexpr int plan(int halves, int warps, int np, bool sep, int base) {
+        int free0 = base, free1 = (base + 65535) / 65536 * 65536;
+        const int end0 = free1;
+        free1 += 65536;
+        const int n = halves * (warps + 3) + 1;
+        for (int i = 0; i < n; i++) {
+            const int k = i - halves * warps;
+            const int bytes = k < 0 ? ring_bytes(np, sep) : k < halves ? (sep ? warps * XSLOT : 0) : k < 2 * halves ? QS_BYTES
+                              : k < 3 * halves ? misc_bytes(warps) : PREFIX_BYTES;
+            const int a0 = (free0 + 127) / 128 * 128;
+            if (a0 + bytes <= end0) free0 = a0 + bytes;
+            else free1 = (free1 + 127) / 128 * 128 + bytes;
+        }
+        return (free1 > free0 ? free1 : free0) - base;
+    }
+    __host__ __device__ static constexpr int need(int halves, int warps, int np, bool sep) {
+        int worst = 0;
+        const int bases[5] = {0, 16, 1024, 2048, 4096};
+        for (int i = 0; i < 5; i++) {
+            const int n = plan(halves, warps, np, sep, bases[i]);
+            worst = n > worst ? n : worst;
+        }
+        return worst + 128;
+    }
+    static constexpr int LIMIT = 226 * 1024;   // (1 KB for the kernel's static shared memory)
+    // A CTA per SM, as two halves that share the tables and nothing else: one half's barriers and folds overlap with the
+    // other's pages.  Warps of a half: 8 of 128 registers where 3-bit codes or 2-bit keys keep the ALU pipe busy, 6 of 168
+    // otherwise (64 x 8192 tokens, two layers of 32 / 8 heads of 128, K4V4: 258 us with 8, 238 with 6; 4 x 131072, 64 / 8
+    // heads, K3V3: 134 with 8, 138 with 6); heads of 256: 6 (ragged K4V2 batch of 256 up to 32768 tokens: 802 with 8, 739
+    // with 6), in groups of five to eight 4 of 255.  A cluster's CTA at head_dim 256 is one half.
+    static constexpr int HALVES = D == 256 && CLUSTER ? 1 : 2;
+    static constexpr int WARPS = CLUSTER ? (D == 256 && NH == 1 ? 12 : 8) : D == 256 ? (NH == 1 ? 6 : 4) : BK == 4 && BV != 3 ? 6 : 8;
+    // places of the line that a unit takes beyond one for each page (see above)
+    static constexpr int PIECE = 28;
+    // two pages per stage wherever their rings leave the warp count alone (a cluster's parts are a few pages long)
+    static constexpr int NP = !CLUSTER && need(HALVES, WARPS, 2, false) <= LIMIT ? 2 : 1;
+    static constexpr int STAGE_BYTES = NP * M::PAGE_BYTES;
+    static constexpr int THREADS = 32 * WARPS;
+    static constexpr bool SEP = need(HALVES, WARPS, NP, true) <= LIMIT;
+    static constexpr int SMEM_BYTES = need(HALVES, WARPS, NP, SEP);
+    // the codes' look-ups: keys in column 0 of the window, values in column 1, or both in the same tables
+    template <bool SHARED>
+    using WinK = Window<BK, SHARED && BK == 3>;
+    template <bool SHARED>
+    using WinV = Window<BV, SHARED && BV == 3>;
+};
+
+__device__ __forceinline__ uint32_t atom_add_acq_rel(int* p, int v) {
+    uint32_t old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;\n" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ float2 ld_cluster2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];\n" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+template <int D, int BK, int BV, bool SHARED_LUT, int NH, bool CLUSTER>
+__global__ void __launch_bounds__(FlowCfg<D, BK, BV, NH, CLUSTER>::HALVES * FlowCfg<D, BK, BV, NH, CLUSTER>::THREADS, 1)
 attn_flow_kernel(const __grid_constant__ AttnParams p) {
-    using C = MmaCfg<D, BK, BV, NH>;
+    using C = FlowCfg<D, BK, BV, NH, CLUSTER>;
+    using WK = typename C::template WinK<SHARED_LUT>;
+    using WV = typename C::template WinV<SHARED_LUT>;
     constexpr int NKB = C::NKB, NMT = C::NMT, WARPS = C::WARPS, THREADS = C::THREADS, NP = C::NP;
     constexpr int E = D / kOctet;
     constexpr int ROW = D + 4;
@@ -54,14 +159,10 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
 
     extern __shared__ __align__(16) uint8_t smem_raw[];
     const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw));
-    // ---- carve shared memory (addresses in the shared window): the byte table needs a
+    // ---- carve shared memory (addresses in the shared window): the tables need a
     // 64 KB-aligned window; the other objects go first-fit before or after it
-    uint32_t window = 0, free0 = sbase, end0 = sbase, free1 = sbase;
-    if constexpr (C::BYTE) {
-        window = (sbase + 65535u) & ~65535u;
-        end0 = window;
-        free1 = window + 65536u;
-    }
+    const uint32_t window = (sbase + 65535u) & ~65535u, end0 = window;
+    uint32_t free0 = sbase, free1 = window + 65536u;
     auto take = [&](uint32_t bytes) {
         uint32_t a = (free0 + 127u) & ~127u;
         if (a + bytes <= end0) { free0 = a + bytes; return a; }
@@ -70,35 +171,55 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         return a;
     };
     auto gptr = [&](uint32_t saddr) { return smem_raw + (saddr - sbase); };
-    const uint32_t misc = take(C::MISC_BYTES + WARPS * C::XML);
-    uint32_t tk_small = 0, tv_small = 0, cur_addr = misc;
-    if constexpr (C::SMALL_ALIGN > 0) {
-        cur_addr = (misc + C::SMALL_ALIGN - 1) & ~static_cast<uint32_t>(C::SMALL_ALIGN - 1);
-        if (C::TKS >= C::TVS) { tk_small = cur_addr; tv_small = cur_addr + C::TKS; }
-        else { tv_small = cur_addr; tk_small = cur_addr + C::TVS; }
-        cur_addr += C::TKS + C::TVS;
-        if (SHARED_LUT) tv_small = tk_small;
-    }
-    cur_addr = (cur_addr + 15u) & ~15u;
-    float* qs = reinterpret_cast<float*>(gptr(cur_addr));             // [8][D + 16] rotated queries
-    float* folded = qs + 8 * (D + 16);                                // [4 * NH][ROW] the piece's (O, m, l)
-    int* prefix = reinterpret_cast<int*>(folded + 4 * NH * ROW);      // [B + 1] page counts, summed up
-    float* xml = reinterpret_cast<float*>(prefix + kFlowMaxSeqs + 4); // [WARPS][2][4 * NH]
-    const uint32_t bars = cur_addr + 8 * (D + 16) * 4 + 4 * NH * ROW * 4 + (kFlowMaxSeqs + 4) * 4 +
-                          WARPS * C::XML;                             // [WARPS][RING] x 8 bytes
+    const int half = C::HALVES > 1 ? static_cast<int>(threadIdx.x) / THREADS : 0;
+    uint32_t rings[WARPS], xarea = 0, qs_at = 0, misc_of[C::HALVES];
+    auto take_mine = [&](uint32_t& mine, uint32_t bytes) {   // one for each half
+#pragma unroll
+        for (int h = 0; h < C::HALVES; h++) {
+            const uint32_t a = take(bytes);
+            if (h == half) mine = a;
+        }
+    };
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) take_mine(rings[w], C::ring_bytes(NP, C::SEP));
+    if constexpr (C::SEP) take_mine(xarea, WARPS * C::XSLOT);
+    take_mine(qs_at, C::QS_BYTES);
+#pragma unroll
+    for (int h = 0; h < C::HALVES; h++) misc_of[h] = take(C::misc_bytes(WARPS));
+    const uint32_t misc = half == 0 ? misc_of[0] : misc_of[C::HALVES - 1];
+    int* prefix = reinterpret_cast<int*>(gptr(take(C::PREFIX_BYTES)));   // [B + 1] page counts, summed up
+    float* qs = reinterpret_cast<float*>(gptr(qs_at));                // [4 * NH][D + 16] rotated queries
+    float* folded = reinterpret_cast<float*>(gptr(misc));             // [4 * NH][ROW] the piece's (O, m, l)
+    float* xml = folded + 4 * NH * ROW;                               // [WARPS][2][4 * NH]
+    const uint32_t bars = misc + 4 * NH * ROW * 4 + WARPS * C::XML;   // [WARPS][RING] x 8 bytes
     uint32_t* ring_at = reinterpret_cast<uint32_t*>(gptr(bars + WARPS * C::RING * 8));  // [WARPS]
-    const uint32_t xarea = C::SEP ? take(WARPS * C::XSLOT) : 0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < WARPS; w++) ring_at[w] = take(C::ring_bytes(NP, C::SEP));
+    const int tid = static_cast<int>(threadIdx.x) - half * THREADS;
+    if (tid == 0) {
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) ring_at[w] = rings[w];
+    }
     // warp w's share of the merge exchange area
     auto xchg = [&](int w) {
         return reinterpret_cast<float4*>(gptr(C::SEP ? xarea + w * C::XSLOT : ring_at[w]));
     };
+    // the half's barrier
+    auto sync_half = [&]() {
+        if constexpr (C::HALVES == 1) __syncthreads();
+        else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + half), "n"(THREADS) : "memory");
+    };
 
     // the next kernel of the stream may start its own set-up as soon as every CTA got here
     let_next_kernel_start();
-    const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
+    // This half among all halves of the grid.  A cluster: its unit's part `cta` of `ctas`.
+    int cta = half * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x), ctas = C::HALVES * static_cast<int>(gridDim.x);
+    uint32_t rank = 0, cluster_size = 1;
+    if constexpr (CLUSTER) {
+        asm("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+        asm("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(cluster_size));
+        cta = static_cast<int>(rank) * C::HALVES + half;
+        ctas = static_cast<int>(cluster_size) * C::HALVES;
+    }
     const int g = lane >> 2, tg = lane & 3;
     const bool odd = g & 1;
     const int group = p.Hq / p.Hkv;  // <= 4 * NH
@@ -133,33 +254,22 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             const __half2 h = __floats2half2_rn(__shfl_sync(0xffffffffu, lev, lo), __shfl_sync(0xffffffffu, lev, hi));
             return *reinterpret_cast<const uint32_t*>(&h);
         };
-        if constexpr (C::BYTE) {
-            uint32_t* tb = reinterpret_cast<uint32_t*>(gptr(window));
+        uint32_t* tb = reinterpret_cast<uint32_t*>(gptr(window));
+        auto entry = [&](float lev, int bits, int column, int e) {   // the lane's copy in row e
+            if (bits == 4) return pair(lev, e & 15, e >> 4);
+            if (bits == 3) return pair(lev, e >> (2 * column) & 7, e >> (2 * column + 3) & 7);
+            const uint32_t x = pair(lev, e & 3, (e >> 2) & 3), y = pair(lev, (e >> 4) & 3, e >> 6);
+            return (lane & 1) ? y : x;
+        };
 #pragma unroll 4
-            for (int e = warp; e < 256; e += WARPS) {
-                if constexpr (BK == 4) tb[e * 64 + lane] = pair(lev_k, e & 15, e >> 4);
-                if constexpr (BV == 4 && !SHARED_LUT) tb[e * 64 + 32 + lane] = pair(lev_v, e & 15, e >> 4);
-                if constexpr (C::V2BYTE) {
-                    const uint32_t x = pair(lev_v, e & 3, (e >> 2) & 3), y = pair(lev_v, (e >> 4) & 3, e >> 6);
-                    tb[e * 64 + 32 + lane] = (lane & 1) ? y : x;
-                }
-            }
-        }
-        if constexpr (BK != 4) {
-            uint32_t* t = reinterpret_cast<uint32_t*>(gptr(tk_small));
-            for (int e = warp; e < (1 << C::IWK); e += WARPS)
-                t[e * 32 + lane] = pair(lev_k, e & ((1 << BK) - 1), e >> BK);
-        }
-        if constexpr (BV != 4 && !SHARED_LUT && !C::V2BYTE) {
-            uint32_t* t = reinterpret_cast<uint32_t*>(gptr(tv_small));
-            for (int e = warp; e < (1 << C::IWV); e += WARPS)
-                t[e * 32 + lane] = pair(lev_v, e & ((1 << BV) - 1), e >> BV);
+        for (int e = threadIdx.x / 32; e < 256; e += C::HALVES * WARPS) {
+            tb[e * 64 + lane] = entry(lev_k, BK, 0, e);
+            if constexpr (SHARED_LUT && BK == 3) tb[e * 64 + 32 + lane] = entry(lev_k, 3, 1, e);   // (by the high six bits)
+            else if constexpr (!SHARED_LUT) tb[e * 64 + 32 + lane] = entry(lev_v, BV, 0, e);
         }
     }
-    const uint32_t lk_lane = (BK == 4 ? window : tk_small) | (lane * 4);
-    const uint32_t lv_lane =
-        C::V2BYTE ? (window | 128u | ((lane & 15) * 8))
-                  : ((BV == 4 ? (window | (SHARED_LUT ? 0u : 128u)) : tv_small) | (lane * 4));
+    const uint32_t lk_lane = window | (BK == 2 ? (lane & 15) * 8 : lane * 4);
+    const uint32_t lv_lane = window | (SHARED_LUT ? 0u : 128u) | (BV == 2 ? (lane & 15) * 8 : lane * 4);
     // one mbarrier per ring buffer (a single arrival + the copies' bytes)
     const uint32_t my_bars = bars + warp * C::RING * 8;
     if (lane == 0) {
@@ -167,7 +277,8 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         for (int r = 0; r < C::RING; r++) mbar_init(my_bars + r * 8, 1);
     }
     mbar_fence_init();
-    __shared__ int s_bad[3];   // by piece number mod 3: a block id of the piece was out of range
+    __shared__ int s_bads[C::HALVES][3];   // by piece number mod 3: a block id of the piece was out of range
+    int* s_bad = s_bads[half];
     if (tid < 3) s_bad[tid] = 0;
 
     // Everything up to here touched shared memory only.  From here on the kernel reads and writes
@@ -175,31 +286,41 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     after_previous_kernel();
     unsigned long long* epoch_word = reinterpret_cast<unsigned long long*>(p.work_counter + 2);
     if (blockIdx.x == 0) {
-        for (int i = tid; i < p.n_units; i += THREADS) p.unit_counter[i] = 0;
-        if (tid == 0) {
+        if constexpr (!CLUSTER)
+            for (int i = threadIdx.x; i < p.n_units; i += C::HALVES * THREADS) p.unit_counter[i] = 0;
+        if (threadIdx.x == 0) {
             p.work_counter[1] = 0;
             if (p.b0 == 0) p.work_counter[kStatusWord] = 0;   // (the call's: its later launches add to it)
         }
     }
     // prefix sums of the page counts (lengths beyond the host's bound are cut to it)
     auto tokens_of = [&](int b) { return max(0, min(p.seq_lens[b], p.max_seq)); };
-    if (warp == 0) {
+    if (!CLUSTER && threadIdx.x < 32) {
         int carry = 0;
-        for (int b0 = 0; b0 < p.B; b0 += 32) {
-            const int b = b0 + lane;
-            int x = b < p.B ? (tokens_of(b) + kPageTokens - 1) / kPageTokens : 0;
+        for (int b0 = 0; b0 < p.B; b0 += 128) {
+            int x[4];      // (their loads do not wait for one another)
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, d);
-                if (lane >= d) x += y;
+            for (int k = 0; k < 4; k++) {
+                const int b = b0 + 32 * k + lane;
+                x[k] = b < p.B ? (tokens_of(b) + kPageTokens - 1) / kPageTokens : 0;
+                if (x[k] > 0) x[k] += C::PIECE;
             }
-            if (b < p.B) prefix[b + 1] = carry + x;
-            carry += __shfl_sync(0xffffffffu, x, 31);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, x[k], d);
+                    if (lane >= d) x[k] += y;
+                }
+                const int b = b0 + 32 * k + lane;
+                if (b < p.B) prefix[b + 1] = carry + x[k];
+                carry += __shfl_sync(0xffffffffu, x[k], 31);
+            }
         }
         if (lane == 0) prefix[0] = 0;
     }
     __syncthreads();
-    if (blockIdx.x == 0 && tid == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
         __threadfence();
         asm volatile("st.release.gpu.global.u64 [%0], %1;\n" ::"l"(epoch_word), "l"(p.epoch) : "memory");
     }
@@ -219,16 +340,41 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         stalled = true;
     };
 
+    // a CTA has left (run by one warp)
+    auto leave = [&]() {
+        await_epoch();
+        if (lane == 0 && atomicAdd(p.work_counter + 1, 1) == static_cast<int>(gridDim.x) - 1) {
+            __threadfence();
+            asm volatile("st.release.gpu.global.u64 [%0], %1;\n" ::"l"(epoch_word), "l"(0ull) : "memory");
+        }
+    };
+
     // ---- this CTA's share of the pages, and the piece that starts at a given page
-    const int per_layer = prefix[p.B] * p.Hkv;
+    const int per_layer = CLUSTER ? 1 : prefix[p.B] * p.Hkv;
     const int64_t total = static_cast<int64_t>(per_layer) * p.n_layers;
-    int64_t share = (total + gridDim.x - 1) / gridDim.x;
+    int64_t share = (total + ctas - 1) / ctas;
     share = share > p.min_share ? share : p.min_share;
-    const int64_t first = share * blockIdx.x;
+    const int64_t first = share * cta;
     const int64_t end = first + share < total ? first + share : total;
     auto locate = [&](int64_t pos) {
         FlowPiece it{};
         it.next = pos;
+        if constexpr (CLUSTER) {   // one piece: part `cta` of the cluster's unit
+            if (pos != 0) return it;
+            const int unit = static_cast<int>(blockIdx.x / cluster_size), per_lay = p.B * p.Hkv;
+            it.layer = unit / per_lay;
+            const int r = unit - it.layer * per_lay;
+            it.b = r / p.Hkv;
+            it.hkv = r - it.b * p.Hkv;
+            const int tokens = tokens_of(it.b);
+            it.unit_pages = (tokens + kPageTokens - 1) / kPageTokens;
+            const int per = (it.unit_pages + ctas - 1) / ctas;
+            it.page0 = cta * per;
+            it.n_pages = max(0, min(per, it.unit_pages - it.page0));
+            it.tokens = min(tokens - it.page0 * kPageTokens, it.n_pages * kPageTokens);
+            it.next = 1;
+            return it;
+        }
         if (pos >= end) return it;
         int r;
         if (p.n_layers == 1) {
@@ -244,26 +390,28 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             if (prefix[mid] * p.Hkv <= r) lo = mid; else hi = mid;
         }
         it.b = lo;
-        it.unit_pages = prefix[lo + 1] - prefix[lo];
+        const int places = prefix[lo + 1] - prefix[lo];
+        it.unit_pages = places - C::PIECE;
         r -= prefix[lo] * p.Hkv;
-        it.hkv = r / it.unit_pages;
-        it.page0 = r - it.hkv * it.unit_pages;
-        it.unit_start = pos - it.page0;
+        it.hkv = r / places;
+        const int at = r - it.hkv * places;
+        it.unit_start = pos - at;
         const int64_t room = end - pos;
-        it.n_pages = it.unit_pages - it.page0;
-        if (it.n_pages > room) it.n_pages = static_cast<int>(room);
+        const int to = places - at > room ? at + static_cast<int>(room) : places;
+        // (a share that ends among a unit's extra places has none of its pages: 0, and the share's end)
+        it.page0 = max(at - C::PIECE, 0);
+        it.n_pages = max(to - C::PIECE, 0) - it.page0;
         it.tokens = min(tokens_of(lo) - it.page0 * kPageTokens, it.n_pages * kPageTokens);
-        it.next = pos + it.n_pages;
+        it.first = pos == first;
+        it.next = pos + (to - at);
         return it;
     };
     // The pieces of the share, by number mod 3: this one, the next one and the one after are known (one
     // thread looks for them, between two barriers).
-    __shared__ FlowPiece s_piece[3];
-    if (tid == 0) {
-        s_piece[0] = locate(first);
-        s_piece[1] = locate(s_piece[0].next);
-    }
-    __syncthreads();
+    __shared__ FlowPiece s_pieces[C::HALVES][3];
+    FlowPiece* s_piece = s_pieces[half];
+    if (tid == 0) s_piece[0] = locate(CLUSTER ? 0 : first);
+    sync_half();
 
     // ---- pages: block ids and bulk copies
     const uint32_t my_ring = ring_at[warp];
@@ -272,7 +420,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     uint32_t phase = 0;   // bit r = parity the next wait on ring buffer r expects
     int ring_it = 0;      // stages this warp has taken from its ring so far (buffer = ring_it % RING)
 #ifdef FTQ_TEST_WAIT_EXPIRY
-    bool test_drop = blockIdx.x == 0 && warp == 5;
+    bool test_drop = blockIdx.x == 0 && half == 0 && warp == 5;
 #endif
     // stages of a piece that are this warp's: warp, warp + WARPS, ...
     auto my_stages = [&](const FlowPiece& it) {
@@ -329,14 +477,14 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         const int t8 = lane & 7, o = lane >> 3;
         const int hh = (warp - w0) * 4 + o;
         const bool hv = hh < group;
-        const int64_t qoff = (head_row(it) + (hv ? hh : 0)) * D;
+        const uint8_t* src = static_cast<const uint8_t*>(p.q) + (head_row(it) + (hv ? hh : 0)) * (D * 2);
         float a[E];
 #pragma unroll
         for (int i = 0; i < E / 8; i++) {
             float tmp[8];
-            const int64_t eo = qoff + 8 * (t8 + 8 * i);
-            if (p.q_dtype == kBF16) load8<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.q) + eo, tmp);
-            else load8<__half>(static_cast<const __half*>(p.q) + eo, tmp);
+            const uint8_t* at = src + 16 * (t8 + 8 * i);
+            if (p.q_dtype == kBF16) load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(at), tmp);
+            else load8<__half>(reinterpret_cast<const __half*>(at), tmp);
 #pragma unroll
             for (int c = 0; c < 8; c++)
                 a[8 * i + c] = __uint_as_float(
@@ -350,8 +498,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
 
     // ---- per-piece arithmetic state of a lane: query fragments, softmax state of heads
     // HL*tg + {0 .. HL-1}, O[head][(D/8)*g .. + D/8)
-    uint32_t qb[C::QSMEM ? 1 : NKB][2];
-    const uint32_t qfrag = static_cast<uint32_t>(__cvta_generic_to_shared(qs));   // [kb][lane] x 8 bytes (QSMEM)
+    uint32_t qb[NKB][2];
     float m_run[HL], l_run[HL], oacc[NO][4];
 
     // a lane's slices of the staged page at `page`
@@ -371,24 +518,25 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
 
     // S = K.Q^T of NP pages (two accumulator chains each)
     auto qk_scores = [&](const uint32_t (&k)[C::NP][2][C::KW], float (&c)[C::NP][2][4]) {
+        typename WK::template Run<C::KW> run[NP][2];
 #pragma unroll
-        for (int kb = 0; kb < NKB; kb++) {
-            uint32_t b0, b1;
-            if constexpr (C::QSMEM) {
-                const uint2 qv = lds64(qfrag + (kb * 32 + lane) * 8);
-                b0 = qv.x; b1 = qv.y;
-            } else {
-                b0 = qb[kb][0]; b1 = qb[kb][1];
+        for (int i = 0; i < NP; i++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+#pragma unroll
+                for (int j = 0; j < C::KW; j++) run[i][r].w[j] = k[i][r][j];
+                WK::shift(run[i][r]);
             }
 #pragma unroll
+        for (int kb = 0; kb < NKB; kb++) {
+#pragma unroll
             for (int i = 0; i < NP; i++) {
-                const uint32_t a0 = lut32(entry_addr<C::IWK>(k[i][0], 2 * kb, lk_lane));
-                const uint32_t a1 = lut32(entry_addr<C::IWK>(k[i][1], 2 * kb, lk_lane));
-                const uint32_t a2 = lut32(entry_addr<C::IWK>(k[i][0], 2 * kb + 1, lk_lane));
-                const uint32_t a3 = lut32(entry_addr<C::IWK>(k[i][1], 2 * kb + 1, lk_lane));
+                uint32_t a0, a1, a2, a3;
+                WK::pairs(run[i][0], kb, lk_lane, a0, a2);
+                WK::pairs(run[i][1], kb, lk_lane, a1, a3);
                 // (the first MMA of each of the two accumulator chains starts from zero)
-                if (kb < 2) mma_16816_z(c[i][kb & 1], a0, a1, a2, a3, b0, b1);
-                else mma_16816(c[i][kb & 1], a0, a1, a2, a3, b0, b1);
+                if (kb < 2) mma_16816_z(c[i][kb & 1], a0, a1, a2, a3, qb[kb][0], qb[kb][1]);
+                else mma_16816(c[i][kb & 1], a0, a1, a2, a3, qb[kb][0], qb[kb][1]);
             }
         }
     };
@@ -502,40 +650,38 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         }
     };
 
-    // values of the code pairs (coordinates (D/8)g + 2 * pair + {0, 1}) of register v[j]
-    auto v_pairs = [&](const uint32_t (&v)[C::VW], int mt, uint32_t& x, uint32_t& y) {
-        if constexpr (C::V2BYTE) {
-            const uint2 e = lut64(entry_addr<8>(v, mt, lv_lane));   // byte mt = pairs 2mt, 2mt + 1
-            x = e.x; y = e.y;
-        } else {
-            x = lut32(entry_addr<C::IWV>(v, 2 * mt, lv_lane));
-            y = lut32(entry_addr<C::IWV>(v, 2 * mt + 1, lv_lane));
-        }
-    };
     auto pv_accum = [&](const uint32_t (&v)[4][C::VW], const uint32_t (&pb)[C::NPB][2]) {
+        typename WV::template Run<C::VW> run[4];
         if constexpr (H8) {
-            // O^T += V^T.P^T : rows = coordinates (D/8)g + 2mt, + 1, k = tokens
+            // O^T += V^T.P^T : rows = coordinates (D/8)g + 2f, + 1, k = tokens: the codes of two tokens merged
+            // into pairs before the look-up (exchanging the looked-up values took a byte-permute per look-up)
+            WV::merge(v[0], v[1], run[0], run[1]);
+            WV::merge(v[2], v[3], run[2], run[3]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) WV::shift(run[j]);
 #pragma unroll
             for (int m2 = 0; m2 < NMT; m2++) {
                 uint32_t x[4], y[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) v_pairs(v[j], m2, x[j], y[j]);
-                mma_16816(oacc[2 * m2], __byte_perm(x[0], x[1], 0x5410u), __byte_perm(x[0], x[1], 0x7632u),
-                          __byte_perm(x[2], x[3], 0x5410u), __byte_perm(x[2], x[3], 0x7632u),
-                          pb[0][0], pb[0][1]);
-                mma_16816(oacc[2 * m2 + 1], __byte_perm(y[0], y[1], 0x5410u),
-                          __byte_perm(y[0], y[1], 0x7632u), __byte_perm(y[2], y[3], 0x5410u),
-                          __byte_perm(y[2], y[3], 0x7632u), pb[0][0], pb[0][1]);
+                for (int j = 0; j < 4; j++) WV::pairs(run[j], m2, lv_lane, x[j], y[j]);
+                mma_16816(oacc[2 * m2], x[0], x[1], x[2], x[3], pb[0][0], pb[0][1]);
+                mma_16816(oacc[2 * m2 + 1], y[0], y[1], y[2], y[3], pb[0][0], pb[0][1]);
             }
         } else {
             // rows = d-pairs (D/16)*g + 2*mt + {0,1}, k = (token, parity)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+#pragma unroll
+                for (int i = 0; i < C::VW; i++) run[j].w[i] = v[j][i];
+                WV::shift(run[j]);
+            }
 #pragma unroll
             for (int ks = 0; ks < 2; ks++)
 #pragma unroll
                 for (int mt = 0; mt < NMT; mt++) {
                     uint32_t a0, a1, a2, a3;
-                    v_pairs(v[2 * ks], mt, a0, a1);
-                    v_pairs(v[2 * ks + 1], mt, a2, a3);
+                    WV::pairs(run[2 * ks], mt, lv_lane, a0, a1);
+                    WV::pairs(run[2 * ks + 1], mt, lv_lane, a2, a3);
                     mma_16816(oacc[mt], a0, a1, a2, a3, pb[ks][0], pb[ks][1]);
                 }
         }
@@ -544,13 +690,34 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     // warps that fold the per-warp states; when enough warps are left over they rotate the next
     // piece's queries at the same time
     constexpr int NRED = (NO <= WARPS - 2) ? NO : WARPS;
-    constexpr int FINISH = NH;   // warps that finish a piece (four heads each)
+    // warps that finish a piece (four heads each): the last ones, which have the fewest stages
+    constexpr int FIN0 = WARPS - NH;
 
-    // Finish warp w's heads of a folded piece: normalise, rotate back and store when the piece is the
-    // whole unit; else put its rows beside the unit's others, and finish the unit when they were the
-    // last ones missing.
+    // Rows (O, m, l) [group][ROW] of a half's pieces that are parts of units: block 0 the piece its share starts with, 1 its
+    // last one.
+    auto row_of = [&](int64_t c, int block) { return p.partials + (2 * c + block) * group * ROW; };
+    __shared__ FlowPiece s_cuts[C::HALVES][2];
+    __shared__ int s_part[C::HALVES][2];      // parts of the unit when this half is the last of them, else 0
+    FlowPiece* s_cut = s_cuts[half];
+    int* s_parts = s_part[half];
+    if (tid < 2) s_cut[tid].n_pages = 0;
+    // a finished head's coordinates t + 8 k
+    auto store_head = [&](const FlowPiece& it, int h, int t, const float (&a)[E]) {
+        const int64_t at = (head_row(it) + h) * D;
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const float r = a[k] * p.rsqrt_d;
+            const float s = __uint_as_float(__float_as_uint(r) ^ sign_mask(p.signs, t + 8 * k));
+            const int64_t idx = at + t + 8 * k;
+            if (p.out_dtype == kBF16) static_cast<__nv_bfloat16*>(p.out)[idx] = __float2bfloat16_rn(s);
+            else if (p.out_dtype == kF16) static_cast<__half*>(p.out)[idx] = __float2half_rn(s);
+            else static_cast<float*>(p.out)[idx] = s;
+        }
+    };
+    // Finish warp w's heads of a folded piece: normalise, rotate back and store when the piece is the whole unit; else
+    // leave its rows in the workspace, for merge_units.
     auto finish_piece = [&](const FlowPiece& it, bool first_of_cta) {
-        const int t = lane & 7, h = warp * 4 + (lane >> 3);
+        const int t = lane & 7, h = (warp - FIN0) * 4 + (lane >> 3);
         const bool valid = h < group;
         const float* row0 = folded + (valid ? h : 0) * ROW;
         float a[E];
@@ -561,82 +728,138 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             a[8 * i] = u.x; a[8 * i + 1] = u.y; a[8 * i + 2] = u.z; a[8 * i + 3] = u.w;
             a[8 * i + 4] = v.x; a[8 * i + 5] = v.y; a[8 * i + 6] = v.z; a[8 * i + 7] = v.w;
         }
-        float m = row0[D], l = row0[D + 1];
-        bool nan = m != m;
-        const int64_t c0 = it.unit_start / share, c1 = (it.unit_start + it.unit_pages - 1) / share;
-        if (c0 != c1) {
-            // row block 0 of a CTA: the piece its share starts with; 1: its last one
-            auto row_of = [&](int64_t c, int block) {
-                return p.partials + ((2 * c + block) * group + (valid ? h : 0)) * ROW;
-            };
-            float* mine = row_of(blockIdx.x, first_of_cta ? 0 : 1);
+        const float m = row0[D], l = row0[D + 1];
+        if (it.page0 != 0 || it.n_pages != it.unit_pages) {
             if (valid) {
+                float* mine = row_of(cta, first_of_cta ? 0 : 1) + h * ROW;
 #pragma unroll
                 for (int i = 0; i < E / 8; i++) {
                     float4* dst = reinterpret_cast<float4*>(mine + 8 * (t + 8 * i));
                     __stcg(dst, make_float4(a[8 * i], a[8 * i + 1], a[8 * i + 2], a[8 * i + 3]));
                     __stcg(dst + 1, make_float4(a[8 * i + 4], a[8 * i + 5], a[8 * i + 6], a[8 * i + 7]));
                 }
-                if (t == 0) {
-                    __stcg(mine + D, m);
-                    __stcg(mine + D + 1, l);
-                }
+                if (t == 0) __stcg(reinterpret_cast<float2*>(mine + D), make_float2(m, l));
             }
-            __threadfence();
-            __syncwarp();
-            await_epoch();
-            uint32_t old = 0;   // (16 bits of the unit's counter for each finishing warp)
-            if (lane == 0) {
-                const int64_t unit = (static_cast<int64_t>(it.layer) * p.B + it.b) * p.Hkv + it.hkv;
-                old = static_cast<uint32_t>(atomicAdd(p.unit_counter + unit, 1 << (16 * warp))) >> (16 * warp) & 0xffffu;
-            }
-            if (__shfl_sync(0xffffffffu, old, 0) != static_cast<uint32_t>(c1 - c0)) return;
-            __threadfence();
-            // (the order of the sum is the order of the CTAs, whoever merges)
-            m = -INFINITY;
-            for (int64_t c = c0; c <= c1; c++) {
-                const float mc = __ldcg(row_of(c, c * share >= it.unit_start ? 0 : 1) + D);
-                nan |= mc != mc;   // (fmaxf drops a NaN operand)
-                m = fmaxf(m, mc);
-            }
-            l = 0.f;
-#pragma unroll
-            for (int r = 0; r < E; r++) a[r] = 0.f;
-            for (int64_t c = c0; c <= c1; c++) {
-                const float* row = row_of(c, c * share >= it.unit_start ? 0 : 1);
-                const float f = fast_exp2(__ldcg(row + D) - m);
-                l = fmaf(__ldcg(row + D + 1), f, l);
-#pragma unroll
-                for (int i = 0; i < E / 4; i++) {
-                    const float4 x = __ldcg(reinterpret_cast<const float4*>(row + 8 * (t + 8 * (i / 2))) + (i & 1));
-                    a[4 * i] = fmaf(x.x, f, a[4 * i]);
-                    a[4 * i + 1] = fmaf(x.y, f, a[4 * i + 1]);
-                    a[4 * i + 2] = fmaf(x.z, f, a[4 * i + 2]);
-                    a[4 * i + 3] = fmaf(x.w, f, a[4 * i + 3]);
-                }
-            }
+            if (tid == FIN0 * 32) s_cut[first_of_cta ? 0 : 1] = it;
+            return;
         }
         float inv = l > 0.f ? 1.f / l : 0.f;
+        if (m != m) inv = __int_as_float(0x7fc00000);
+#pragma unroll
+        for (int r = 0; r < E; r++) a[r] *= inv;
+        octet_fwht<E>(a, lane);
+        if (valid) store_head(it, h, t, a);
+    };
+
+    // A head of a unit from its n parts' rows (O, m, l), by S = 1, 2 or 4 octets of a warp (sub = which of them), each of
+    // which adds up parts sub, sub + S, ...: the order of the sums depends on n and S alone.  `row` gives the row of a
+    // part, `load2` / `load4` read from it.  All lanes of the warp run it together, with S in common; a lane of an octet
+    // without a head has n = 0.
+    auto merge_head = [&](const FlowPiece& it, int h, int n, int S, int sub, auto row, auto load2, auto load4) {
+        const int t = lane & 7;
+        float M = -INFINITY, L = 0.f, a[E];
+        bool nan = false;
+#pragma unroll
+        for (int r = 0; r < E; r++) a[r] = 0.f;
+        // two rows of an octet at a time; the first ones are on their way while the maximum is looked for
+        float4 x[2][E / 4];
+        float2 ml[2];
+        auto load = [&](int i0) {
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int i = i0 + u * S;
+                ml[u] = make_float2(-INFINITY, 0.f);
+                if (i < n) {
+                    const auto r = row(i);
+                    ml[u] = load2(r, D);
+#pragma unroll
+                    for (int c = 0; c < E / 4; c++) x[u][c] = load4(r, 8 * (t + 8 * (c / 2)) + 4 * (c & 1));
+                }
+            }
+        };
+        load(sub);
+        for (int i = sub * kOctet + t; i < n; i += S * kOctet) {
+            const float m = load2(row(i), D).x;
+            nan |= m != m;   // (fmaxf drops a NaN operand)
+            M = fmaxf(M, m);
+        }
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const float mo = __shfl_xor_sync(0xffffffffu, M, s);
+            const bool no = __shfl_xor_sync(0xffffffffu, static_cast<int>(nan), s) != 0;
+            if (s < kOctet * S) {
+                M = fmaxf(M, mo);
+                nan |= no;
+            }
+        }
+        for (int i0 = sub;;) {
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (ml[u].x == -INFINITY) continue;   // (none, or a part without pages: its O is not written)
+                const float f = fast_exp2(ml[u].x - M);
+                L = fmaf(ml[u].y, f, L);
+#pragma unroll
+                for (int c = 0; c < E / 4; c++) {
+                    a[4 * c] = fmaf(x[u][c].x, f, a[4 * c]);
+                    a[4 * c + 1] = fmaf(x[u][c].y, f, a[4 * c + 1]);
+                    a[4 * c + 2] = fmaf(x[u][c].z, f, a[4 * c + 2]);
+                    a[4 * c + 3] = fmaf(x[u][c].w, f, a[4 * c + 3]);
+                }
+            }
+            i0 += 2 * S;
+            if (i0 >= n) break;
+            load(i0);
+        }
+        __syncwarp();
+        for (int s = kOctet; s < kOctet * S; s <<= 1) {
+            L += __shfl_xor_sync(0xffffffffu, L, s);
+#pragma unroll
+            for (int r = 0; r < E; r++) a[r] += __shfl_xor_sync(0xffffffffu, a[r], s);
+        }
+        float inv = L > 0.f ? 1.f / L : 0.f;   // (a sequence without tokens: zero)
         if (nan) inv = __int_as_float(0x7fc00000);
 #pragma unroll
         for (int r = 0; r < E; r++) a[r] *= inv;
         octet_fwht<E>(a, lane);
-        if (valid) {
-            const int64_t at = (head_row(it) + h) * D;
-#pragma unroll
-            for (int k = 0; k < E; k++) {
-                const float r = a[k] * p.rsqrt_d;
-                const float s = __uint_as_float(__float_as_uint(r) ^ sign_mask(p.signs, t + 8 * k));
-                const int64_t idx = at + t + 8 * k;
-                if (p.out_dtype == kBF16) static_cast<__nv_bfloat16*>(p.out)[idx] = __float2bfloat16_rn(s);
-                else if (p.out_dtype == kF16) static_cast<__half*>(p.out)[idx] = __float2half_rn(s);
-                else static_cast<float*>(p.out)[idx] = s;
+        if (sub == 0 && h < group) store_head(it, h, t, a);
+    };
+
+    // The cut units of this share (its first and its last piece), once all its pieces are done: whoever is the last to get
+    // here with a unit puts it together, all heads at the same time.  Under load a dependent access to L2 takes 1 to 2 us,
+    // so the chain is kept short: rows -> counter (2.4 us) -> rows and maxima together (2.4 us, 6 with a head per warp and
+    // the maxima first).  In the loop, by the warps that finish pieces, it held up the half's other warps.
+    auto merge_units = [&]() {
+        if (tid < 2) {
+            const FlowPiece& it = s_cut[tid];
+            int n = 0;
+            if (it.n_pages > 0) {
+                await_epoch();
+                // (release: the rows that the half wrote before the barrier; acquire: those of the others)
+                const uint32_t old = atom_add_acq_rel(p.unit_counter + (static_cast<int64_t>(it.layer) * p.B + it.b) * p.Hkv + it.hkv, 1);
+                const int parts = static_cast<int>((it.unit_start + C::PIECE + it.unit_pages - 1) / share - (it.unit_start + C::PIECE) / share) + 1;
+                if (static_cast<int>(old) == parts - 1) n = parts;
             }
+            s_parts[tid] = n;
         }
+        sync_half();
+        const int n0 = s_parts[0], n1 = s_parts[1], heads0 = n0 ? group : 0, heads = heads0 + (n1 ? group : 0);
+        if (heads == 0) return;
+        // octets a head: all heads of both units at the same time (the same S when this half has only one to merge: who
+        // merges must not change the order of the sums)
+        const int S = 2 * group <= WARPS ? 4 : group <= WARPS ? 2 : 1;
+        const int octet = warp * 4 + (lane >> 3), k = octet / S;
+        const bool second = k >= heads0;
+        const FlowPiece& it = s_cut[second];
+        const int h = k >= heads ? group : second ? k - heads0 : k;
+        const int64_t c0 = (it.unit_start + C::PIECE) / share;
+        merge_head(it, h, k >= heads ? 0 : second ? n1 : n0, S, octet % S,
+                   [&](int i) { return row_of(c0 + i, (c0 + i) * share >= it.unit_start ? 0 : 1) + h * ROW; },
+                   [](const float* r, int at) { return __ldcg(reinterpret_cast<const float2*>(r + at)); },
+                   [](const float* r, int at) { return __ldcg(reinterpret_cast<const float4*>(r + at)); });
     };
 
     // sequences without tokens: no CTA meets their units, their outputs are zero (softmax over nothing)
-    for (int i = blockIdx.x; i < p.n_layers * p.B; i += gridDim.x) {
+    for (int i = CLUSTER ? p.n_layers * p.B : cta; i < p.n_layers * p.B; i += ctas) {
         const int layer = i / p.B, b = i - layer * p.B;
         if (prefix[b + 1] != prefix[b]) continue;
         const int per_seq = p.Hq * D;
@@ -654,7 +877,14 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     bool any = false, prev_first = true;   // a folded piece is waiting; it was the CTA's first
     if (s_piece[0].n_pages > 0) {
         ids = load_ids(s_piece[0], 0, 0);
-        rotate_queries(s_piece[0], 0);
+        const int n = my_stages(s_piece[0]);
+#pragma unroll
+        for (int r = 0; r < C::RING; r++)
+            if (r < n) issue_stage(head_base(s_piece[0]), ids, s_piece[0].n_pages, r, r);
+        primed = true;
+        rotate_queries(s_piece[0], FIN0);
+        if (tid == 0) s_piece[1] = locate(s_piece[0].next);
+        if (!CLUSTER && tid < 2) await_epoch();   // (while the first pages are on their way)
     }
     while (s_piece[slot].n_pages > 0) {
         const FlowPiece& cur = s_piece[slot];
@@ -663,7 +893,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         const int n_mine = my_stages(cur);
         const uint8_t* base = head_base(cur);
         ids_next = load_ids(cur, IDS, slot);
-        __syncthreads();         // C: queries, the next piece visible; `folded` holds the piece before
+        sync_half();         // C: queries, the next piece visible; `folded` holds the piece before
         int ids_piece = 0;       // first batch of the next piece
         if (s_piece[slot1].n_pages > 0) ids_piece = load_ids(s_piece[slot1], 0, slot1);
         // (a warp whose wait has run out requests nothing any more: the mbarrier of the lost copy
@@ -678,43 +908,16 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
 
         // Q^T fragments: column n = g is head g >> 1 (NH = 1) or g (NH = 2); k-block kb covers
         // coordinates (D/4)*tg + 4*kb + {0,1} (b0) and + {2,3} (b1)
-        if constexpr (!C::QSMEM) {
 #pragma unroll
-            for (int kb = 0; kb < NKB; kb++) {
-                const float4 q4 = *reinterpret_cast<const float4*>(
-                    qs + qs_index(H8 ? g : g >> 1, (D / 4) * tg + 4 * kb));
-                const __half2 lo = __floats2half2_rn(q4.x, q4.y);
-                const __half2 hi = __floats2half2_rn(q4.z, q4.w);
-                qb[kb][0] = *reinterpret_cast<const uint32_t*>(&lo);
-                qb[kb][1] = *reinterpret_cast<const uint32_t*>(&hi);
-            }
-        } else {
-            // shared-memory copy of the fragments, in place of the fp32 queries, which nobody reads
-            // again before the next piece's are rotated
-            constexpr int NE = NKB * 32, PER = (NE + THREADS - 1) / THREADS;
-            uint2 frag[PER];
-#pragma unroll
-            for (int i = 0; i < PER; i++) {
-                const int e = tid + i * THREADS;
-                const int ln = e & 31, kb = e >> 5;
-                if (e < NE) {
-                    const float4 q4 = *reinterpret_cast<const float4*>(
-                        qs + qs_index(H8 ? ln >> 2 : ln >> 3, (D / 4) * (ln & 3) + 4 * kb));
-                    const __half2 lo = __floats2half2_rn(q4.x, q4.y);
-                    const __half2 hi = __floats2half2_rn(q4.z, q4.w);
-                    frag[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo),
-                                         *reinterpret_cast<const uint32_t*>(&hi));
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < PER; i++) {
-                const int e = tid + i * THREADS;
-                if (e < NE) reinterpret_cast<uint2*>(qs)[e] = frag[i];
-            }
-            __syncthreads();
+        for (int kb = 0; kb < NKB; kb++) {
+            const float4 q4 = *reinterpret_cast<const float4*>(
+                qs + qs_index(H8 ? g : g >> 1, (D / 4) * tg + 4 * kb));
+            const __half2 lo = __floats2half2_rn(q4.x, q4.y);
+            const __half2 hi = __floats2half2_rn(q4.z, q4.w);
+            qb[kb][0] = *reinterpret_cast<const uint32_t*>(&lo);
+            qb[kb][1] = *reinterpret_cast<const uint32_t*>(&hi);
         }
-        if (any && warp < FINISH) finish_piece(s_piece[slot2], prev_first);
+        if (any && warp >= FIN0) finish_piece(s_piece[slot2], prev_first);
 
 #pragma unroll
         for (int i = 0; i < HL; i++) { m_run[i] = -INFINITY; l_run[i] = 0.f; }
@@ -791,7 +994,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
 #pragma unroll
             for (int i = 0; i < HL; i++) m_run[i] = __int_as_float(0x7fc00000);
         }
-        __syncthreads();  // A: every warp is done with the ring, the queries and `folded`
+        sync_half();  // A: every warp is done with the ring, the queries and `folded`
 #pragma unroll
         for (int mt = 0; mt < NO; mt++)
             // (the factor that undoes the scaling of the value centroids is applied once per piece)
@@ -805,7 +1008,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
                 xml[(warp * 2 + 1) * (4 * NH) + HL * tg + i] = l_run[i];
             }
         }
-        __syncthreads();  // B: all states are published
+        sync_half();  // B: all states are published
         if (warp < NRED) {
             const bool bad = s_bad[slot] != 0;
             for (int j = tid; j < NO * 32; j += NRED * 32) {
@@ -871,13 +1074,47 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             s_bad[slot2] = 0;
         }
         any = true;
-        prev_first = cur.unit_start + cur.page0 == first;
+        prev_first = cur.first;
         slot = slot1;
         __syncwarp();
         if (s_piece[slot].n_pages == 0) break;
     }
-    __syncthreads();
-    if (any && warp < FINISH) finish_piece(s_piece[slot == 0 ? 2 : slot - 1], prev_first);
+    if constexpr (CLUSTER) {
+        // every part's (O, m, l) lies in its CTA's `folded`: a warp per head adds them up over distributed shared memory
+        if (!any && tid < 4 * NH) {   // a part without pages
+            folded[tid * ROW + D] = -INFINITY;
+            folded[tid * ROW + D + 1] = 0.f;
+        }
+        if (stalled) {
+            await_epoch();
+            if (lane == 0) atomicOr(p.work_counter + kStatusWord, kStatusWaitExpired);
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        const int all = static_cast<int>(threadIdx.x) / 32;      // warp of the CTA
+        const int h = static_cast<int>(rank) + all * static_cast<int>(cluster_size);
+        if (h < group) {
+            merge_head(s_piece[0], h, ctas, 4, lane >> 3,
+                       [&](int i) {
+                           const int r = i / C::HALVES, hf = i - r * C::HALVES;
+                           uint32_t at;
+                           asm("mapa.shared::cluster.u32 %0, %1, %2;\n"
+                               : "=r"(at) : "r"((hf == 0 ? misc_of[0] : misc_of[C::HALVES - 1]) + h * ROW * 4), "r"(r));
+                           return at;
+                       },
+                       [](uint32_t r, int at) { return ld_cluster2(r + at * 4); },
+                       [](uint32_t r, int at) { return ld_cluster4(r + at * 4); });
+        }
+        // the last CTA takes the epoch out, see below; nobody leaves while its rows are being read
+        if (threadIdx.x / 32 == C::HALVES * WARPS - 1) leave();
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        return;
+    }
+    sync_half();
+    if (any && warp >= FIN0) {
+        finish_piece(s_piece[slot == 0 ? 2 : slot - 1], prev_first);
+    }
+    sync_half();
+    merge_units();
     if (stalled) {
         await_epoch();
         if (lane == 0) atomicOr(p.work_counter + kStatusWord, kStatusWaitExpired);
@@ -885,13 +1122,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     // the last CTA to leave takes the epoch out of the workspace: a replay of this very launch (a
     // captured graph) must not find its own epoch there before CTA 0 has cleared the counters
     __syncthreads();
-    if (warp == 0) {
-        await_epoch();
-        if (lane == 0 && atomicAdd(p.work_counter + 1, 1) == static_cast<int>(gridDim.x) - 1) {
-            __threadfence();
-            asm volatile("st.release.gpu.global.u64 [%0], %1;\n" ::"l"(epoch_word), "l"(0ull) : "memory");
-        }
-    }
+    if (threadIdx.x < 32) leave();
 }
 
 }  // namespace ftq

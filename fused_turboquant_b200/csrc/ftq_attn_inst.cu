@@ -1,7 +1,8 @@
 // Instantiates the split-KV decode attention kernels for one head_dim (FTQ_D).
 #include "ftq_attn_flow.cuh"
-#include "ftq_attn_stream.cuh"
 #include "ftq_launch.h"
+
+#include <atomic>
 
 #ifndef FTQ_D
 #error "compile with -DFTQ_D=64, 128 or 256"
@@ -52,33 +53,15 @@ cudaError_t FTQ_CAT(launch_attn_split_d, FTQ_D)(int bits_k, int bits_v, bool pag
                  : by_bk<false>(bits_k, bits_v, p, n_lb, stream);
 }
 
-// The streaming kernel (no CTA-wide barriers, merge included) serves the configurations in
-// which it was measured faster than the equal-share one: a 4-bit byte table (one CTA per SM) with
-// a GQA group of at most 4 -- 16 warps at head_dim 64 / 128, 12 or 8 at head_dim 256 (16 rings and
-// exchange slots do not fit beside the table there).  Measured on B200, streaming against equal
-// shares, store included: 777 : 1137 us for the ragged head_dim-256 K4V2 batch, 21.5 : 25.1 us for
-// one sequence of 900 tokens, 142 : 141 us for 64 x 8192 tokens of 8 K4V4 heads.
-template <int BK, int BV, int NH>
-constexpr bool use_stream_kernel() {
-    using S = StreamCfg<FTQ_D, BK, BV, NH>;
-#if defined(FTQ_NO_STREAM)
-    return false;
-#elif defined(FTQ_ALL_STREAM)
-    return S::FITS;
-#else
-    return S::FITS && S::BYTE && NH == 1;
-#endif
-}
-
 template <int BK, int BV, bool SHARED, int NH>
 static cudaError_t run_flow(const AttnParams& p_in, cudaStream_t stream) {
-    using C = MmaCfg<FTQ_D, BK, BV, NH>;
+    using C = FlowCfg<FTQ_D, BK, BV, NH>;
     static_assert(C::SMEM_BYTES <= C::LIMIT, "shared memory budget");
-    constexpr auto kern = attn_flow_kernel<FTQ_D, BK, BV, SHARED, NH>;
+    constexpr auto kern = attn_flow_kernel<FTQ_D, BK, BV, SHARED, NH, false>;
     cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     AttnParams p = p_in;
-    // a CTA's share is at least one stage per warp: less would only cut units into more rows to merge
+    // a share is at least one stage per warp: less would only cut units into more rows to merge
     p.min_share = C::WARPS * C::NP;
     p.B_stride = p_in.B;
     for (p.b0 = 0; p.b0 < p_in.B; p.b0 += kFlowMaxSeqs) {
@@ -88,10 +71,10 @@ static cudaError_t run_flow(const AttnParams& p_in, cudaStream_t stream) {
         p.n_units = p.n_layers * p.B * p.Hkv;
         const int64_t most = static_cast<int64_t>(p.n_units) * ((static_cast<int64_t>(p.max_seq) + kPageTokens - 1) / kPageTokens);
         const int64_t want = (most + p.min_share - 1) / p.min_share;
-        const int64_t slots = static_cast<int64_t>(sm_count()) * C::CTAS_PER_SM;
+        const int64_t slots = sm_count();
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(static_cast<unsigned>(want < 1 ? 1 : want < slots ? want : slots));
-        cfg.blockDim = dim3(C::THREADS);
+        cfg.blockDim = dim3(C::HALVES * C::THREADS);
         cfg.dynamicSmemBytes = C::SMEM_BYTES;
         cfg.stream = stream;
         // (programmatic stream serialisation: the tables are built while the kernel before drains)
@@ -106,35 +89,77 @@ static cudaError_t run_flow(const AttnParams& p_in, cudaStream_t stream) {
     return cudaSuccess;
 }
 
+// Clusters of `size` CTAs of the kernel that the device holds at a time (asked once per device and size).
+template <auto kern>
+static int clusters_at_a_time(int size, int threads, int smem) {
+    static std::atomic<int> known[64][3];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const int slot = size == 8 ? 0 : size == 4 ? 1 : 2;   // (a size of one is not asked for)
+    if (dev < 64) {
+        const int n = known[dev][slot].load(std::memory_order_relaxed);
+        if (n) return n - 1;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(size) * 64);
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {static_cast<unsigned>(size), 1, 1};
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        n = 0;
+    }
+    if (dev < 64) known[dev][slot].store(n + 1, std::memory_order_relaxed);
+    return n;
+}
+
+// Few units with short contexts (at most one per SM): a cluster of 8, 4, 2 CTAs or one CTA per unit, as many as the device
+// holds at a time, whose parts are put together over distributed shared memory.  Rows in the workspace, a fence, a
+// counter and the rows again are a chain of 6 to 8 us at the end of the equal-share kernel; here it is 2.  Measured as
+// steps (store included, equal shares : clusters; 32 / 8 heads of 128, K3V3, bounded by the host at 12): 1 x 900
+// tokens 23 : 11.7, 1 x 8000 25 : 16, 9 x 5000 ragged 30 : 22, 18 x 3000 30 : 26 us.
+// kClusterPages is the longest part of a half: what the longest sequence of a ragged batch takes (30 us) while the
+// equal shares would even it out.  Returns cudaErrorNotSupported where equal shares are the better ones.
+constexpr int kClusterPages = 192;
+template <int BK, int BV, bool SHARED, int NH>
+static cudaError_t run_cluster(const AttnParams& p_in, cudaStream_t stream) {
+    using C = FlowCfg<FTQ_D, BK, BV, NH, true>;
+    static_assert(C::SMEM_BYTES <= C::LIMIT, "shared memory budget");
+    constexpr auto kern = attn_flow_kernel<FTQ_D, BK, BV, SHARED, NH, true>;
+    const int pages = (p_in.max_seq + kPageTokens - 1) / kPageTokens;
+    if (p_in.n_units > sm_count() || pages > kClusterPages * 8 * C::HALVES) return cudaErrorNotSupported;
+    cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+    int size = 8;
+    while (size > 1 && clusters_at_a_time<kern>(size, C::HALVES * C::THREADS, C::SMEM_BYTES) < p_in.n_units) size /= 2;
+    if (pages > kClusterPages * size * C::HALVES) return cudaErrorNotSupported;
+    AttnParams p = p_in;
+    p.b0 = 0;
+    p.B_stride = p_in.B;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(p.n_units * size));
+    cfg.blockDim = dim3(C::HALVES * C::THREADS);
+    cfg.dynamicSmemBytes = C::SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim = {static_cast<unsigned>(size), 1, 1};
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
 template <int BK, int BV, bool SHARED, int NH>
 static cudaError_t run_mma_nh(const AttnParams& p, cudaStream_t stream) {
-    constexpr int D = FTQ_D;
-    if constexpr (use_stream_kernel<BK, BV, NH>()) {
-        using S = StreamCfg<D, BK, BV, NH>;
-        constexpr auto kern = attn_stream_kernel<D, BK, BV, SHARED, NH>;
-        cudaError_t e = allow_smem<kern>(S::SMEM_BYTES);
-        if (e != cudaSuccess) return e;
-        const int64_t items = p.split.total_items;
-        const int64_t slots = static_cast<int64_t>(sm_count()) * S::CTAS_PER_SM;
-        const unsigned grid = static_cast<unsigned>(items < slots ? items : slots);
-        // One node per call: the kernel clears its own counters.  Programmatic stream
-        // serialisation lets the set-up of this launch (tables in shared memory) run while the
-        // kernel before it in the stream drains; the kernel waits for that kernel's completion
-        // (griddepcontrol.wait) before it touches anything in global memory.
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(S::THREADS);
-        cfg.dynamicSmemBytes = S::SMEM_BYTES;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kern, p, static_cast<int>(items));
-    } else {
-        return run_flow<BK, BV, SHARED, NH>(p, stream);
-    }
+    const cudaError_t e = run_cluster<BK, BV, SHARED, NH>(p, stream);
+    return e != cudaErrorNotSupported ? e : run_flow<BK, BV, SHARED, NH>(p, stream);
 }
 
 template <int BK, int BV, bool SHARED>
@@ -172,36 +197,6 @@ cudaError_t FTQ_CAT(launch_attn_mma_d, FTQ_D)(int bits_k, int bits_v, bool share
         case 4: return mma_by_bv<4>(bits_v, shared_lut, p, stream);
     }
     return cudaErrorInvalidValue;
-}
-
-// CTAs per SM of the streaming kernel where launch_attn_mma picks it for this configuration, 0
-// where it picks the equal-share kernel (which needs no plan of the host)
-template <int BK, int BV, int NH>
-static constexpr int stream_ctas() {
-    return use_stream_kernel<BK, BV, NH>() ? StreamCfg<FTQ_D, BK, BV, NH>::CTAS_PER_SM : 0;
-}
-template <int BK>
-static int stream_ctas_by_bv(int bv, int nh) {
-#ifdef FTQ_ONLY_BITS
-    if (BK != FTQ_ONLY_BITS || bv != FTQ_ONLY_BITS) return 0;
-    return nh == 1 ? stream_ctas<BK, BK, 1>() : stream_ctas<BK, BK, 2>();
-#else
-    switch (bv) {
-        case 2: return nh == 1 ? stream_ctas<BK, 2, 1>() : stream_ctas<BK, 2, 2>();
-        case 3: return nh == 1 ? stream_ctas<BK, 3, 1>() : stream_ctas<BK, 3, 2>();
-        case 4: return nh == 1 ? stream_ctas<BK, 4, 1>() : stream_ctas<BK, 4, 2>();
-    }
-    return 0;
-#endif
-}
-int FTQ_CAT(attn_mma_stream_ctas_d, FTQ_D)(int bits_k, int bits_v, int group) {
-    const int nh = group <= 4 ? 1 : 2;
-    switch (bits_k) {
-        case 2: return stream_ctas_by_bv<2>(bits_v, nh);
-        case 3: return stream_ctas_by_bv<3>(bits_v, nh);
-        case 4: return stream_ctas_by_bv<4>(bits_v, nh);
-    }
-    return 0;
 }
 
 template <typename OT>

@@ -1,6 +1,5 @@
-// What the tensor-core kernels of paged decode attention share (ftq_attn_flow.cuh: equal
-// shares of pages per CTA; ftq_attn_stream.cuh: streaming warps): whole
-// 16-token pages arrive in a per-warp ring by 1-D bulk copies (TMA), every lane
+// Arithmetic of the tensor-core kernel of paged decode attention (ftq_attn_flow.cuh); its look-ups, MMAs and
+// copies serve the slot-format and chunk kernels too.  Whole 16-token pages arrive in a per-warp ring by 1-D bulk copies (TMA), every lane
 // copies its slices to registers, the codes are dequantised through a
 // bank-conflict-free shared-memory table and feed warp-level m16n8k16 fp16 MMAs
 // (fp32 accumulate).  With a GQA
@@ -16,12 +15,10 @@
 // by it): a common rounding bias of the centroids would otherwise add up over
 // all coordinates into one output element through the inverse rotation.
 //
-// Tables: an entry holds the fp16 centroids of two adjacent codes, replicated
-// for the 32 lanes so that bank = lane (no conflicts whatever the codes are).
-// 4-bit codes index by byte: the table occupies a 64 KB-aligned window with
-// 256-byte rows, so that the address is one byte-permute -- the code byte
-// dropped into bits 8..15 of the lane's base address.  3- and 2-bit codes use
-// 128-byte rows in a table aligned to its own size (shift + and/or).
+// Tables: an entry holds the fp16 centroids of two adjacent codes, replicated for the 32 lanes so that
+// bank = lane (no conflicts whatever the codes are); struct Window below says how codes of 4, 3 and 2 bits find
+// their entry.  (The slot-format kernels' 3- and 2-bit codes use 128-byte rows in a table aligned to its own
+// size: shift + and/or, entry_addr.)
 //
 // Fragment maps for one 16-token page (lane = 4*g + tg), GQA group <= 4 (NH = 1):
 //   S = K.Q^T :  A = K [16 tokens x 16 coords]: rows g / g+8 = page tokens rho(g) / rho(g)+2,
@@ -41,10 +38,9 @@
 //                (rho(0..7) + 2) straight into the B registers of P.V: head g, tokens 4tg, 4tg + 1
 //                (4tg + 2, 4tg + 3);
 //   O^T += V^T.P^T with k = token:  A[row g / g+8 = coordinate (D/8)g + 2mt / + 1][k = token]: the
-//                pairs of two tokens' look-ups are exchanged with two byte-permutes;
+//                codes of two tokens are merged into pairs before the look-up (Window::merge);
 //                C[coordinate pair][heads 2tg, 2tg + 1].
-//   Against two passes of the 4-head map this halves the MMAs and the softmax bookkeeping for one
-//   byte-permute per value look-up.
+//   Against two passes of the 4-head map this halves the MMAs and the softmax bookkeeping.
 // In both maps a lane dequantises the K slices (D/4 coordinates) of two tokens and the V
 // slices (D/8 coordinates) of four tokens per page, all contiguous bytes, every
 //   code exactly once per KV head.
@@ -77,9 +73,10 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
 // Lookup in a dequantisation table: the tables never change after the CTA-wide barrier that
 // follows their construction and every address derives from page data read after that barrier,
 // so the load may be scheduled freely (not volatile).
+template <int OFFSET = 0>
 __device__ __forceinline__ uint32_t lut32(uint32_t addr) {
     uint32_t v;
-    asm("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(addr));
+    asm("ld.shared.b32 %0, [%1+%2];\n" : "=r"(v) : "r"(addr), "n"(OFFSET));
     return v;
 }
 
@@ -243,18 +240,74 @@ __device__ __forceinline__ uint32_t entry_addr(const uint32_t (&w)[NW], int pair
     }
 }
 
-// The sixteen 2-bit codes c0 .. c15 of a word as fp16 centroid pairs, without a table: a byte-permute picks
-// the two bytes of a centroid out of the eight of all four (`lo` = centroids 0 and 1, `hi` = 2 and 3).  Its
-// selector is 2c, 2c + 1, i.e. 0x22 * c + 0x10, for four codes at a time.  x[2i] = (c[i], c[i + 4]),
-// x[2i + 1] = (c[i + 8], c[i + 12]).
-__device__ __forceinline__ void select_pairs2(uint32_t w, uint32_t lo, uint32_t hi, uint32_t (&x)[8]) {
+// A dequantisation window: 256 rows of 256 bytes, each row the 32-fold copies of two entries ("columns" of 128
+// bytes), indexed by a whole byte of the packed codes: the address of a look-up is ONE byte-permute, the byte dropped
+// into bits 8..15 of the lane's base address.
+//   4-bit codes: a byte is a pair of codes.
+//   2-bit codes: a byte is four codes, an entry eight bytes (sixteen copies).
+//   3-bit codes: a pair is six of a byte's bits.  Of the four pairs in 24 bits, the first is the low six bits of byte 0
+//     and the last the high six of byte 2; of the codes shifted right by four, the second is the high six of byte 0
+//     and the third the low six of byte 1.  With both columns (BOTH: one codebook for keys and values; column 0 by the
+//     low six bits, column 1 by the high six) that is one shift and four byte-permutes for four look-ups, with
+//     the low six bits alone three shifts.
+// The ALU pipe bounds the 3-bit page loop (64 % busy when a shift and an and-or, three instructions where a pair
+// straddles words, made an index): 24 layers of 32 x 4096 tokens, 14 / 2 heads of 64, 152 -> 139 us, 4 x 131072, 64 / 8
+// heads of 128, 159 -> 138 us by these tables and `merge` alone.
+template <int BITS, bool BOTH>
+struct Window {
+    static constexpr int NS = BITS != 3 ? 0 : BOTH ? 1 : 3;   // shifted copies of the codes
+    template <int NW>
+    struct Run {              // consecutive codes of a lane: NW words
+        uint32_t w[NW];
+        uint32_t s[NS > 0 ? NS : 1][NW];
+    };
+    template <int NW>
+    static __device__ __forceinline__ void shift(Run<NW>& r) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const uint32_t m = (w >> (2 * i)) & 0x03030303u;
-        x[2 * i] = __byte_perm(lo, hi, m * 0x22u + 0x10101010u);
-        x[2 * i + 1] = __byte_perm(lo, hi, (m * 0x22u + 0x10101010u) >> 16);
+        for (int k = 0; k < NS; k++)
+#pragma unroll
+            for (int j = 0; j < NW; j++) {
+                const int sh = BOTH ? 4 : 6 - 2 * k;
+                r.s[k][j] = j + 1 < NW ? __funnelshift_r(r.w[j], r.w[j + 1], sh) : r.w[j] >> sh;
+            }
     }
-}
+    // centroids of the code pairs 2i and 2i + 1
+    template <int NW>
+    static __device__ __forceinline__ void pairs(const Run<NW>& r, int i, uint32_t base, uint32_t& x, uint32_t& y) {
+        auto at = [&](const uint32_t (&w)[NW], int byte) {
+            return __byte_perm(w[byte >> 2], base, 0x7604u | (static_cast<uint32_t>(byte & 3) << 4));
+        };
+        if constexpr (BITS == 4) {
+            x = lut32(at(r.w, 2 * i));
+            y = lut32(at(r.w, 2 * i + 1));
+        } else if constexpr (BITS == 2) {
+            const uint2 e = lut64(at(r.w, i));
+            x = e.x; y = e.y;
+        } else if (i % 2 == 0) {
+            const int b = 3 * (i / 2);
+            x = lut32(at(r.w, b));
+            y = BOTH ? lut32<128>(at(r.s[0], b)) : lut32(at(r.s[0], b));
+        } else {
+            const int b = 3 * (i / 2);
+            x = lut32(at(r.s[BOTH ? 0 : 1], b + 1));
+            y = BOTH ? lut32<128>(at(r.w, b + 2)) : lut32(at(r.s[BOTH ? 0 : 2], b + 2));
+        }
+    }
+    // codes of two tokens, a and b, merged into the pairs (a[2f], b[2f]) and (a[2f + 1], b[2f + 1])
+    template <int NW>
+    static __device__ __forceinline__ void merge(const uint32_t (&a)[NW], const uint32_t (&b)[NW], Run<NW>& even, Run<NW>& odd) {
+#pragma unroll
+        for (int j = 0; j < NW; j++) {
+            uint32_t m = 0;      // the bits of the even codes
+#pragma unroll
+            for (int i = 0; i < 32; i++) m |= (32 * j + i) % (2 * BITS) < BITS ? 1u << i : 0u;
+            const uint32_t up = j > 0 && BITS == 3 ? __funnelshift_l(b[j > 0 ? j - 1 : 0], b[j], BITS) : b[j] << BITS;
+            const uint32_t down = j + 1 < NW && BITS == 3 ? __funnelshift_r(a[j], a[j + 1 < NW ? j + 1 : j], BITS) : a[j] >> BITS;
+            even.w[j] = (a[j] & m) | (up & ~m);
+            odd.w[j] = (down & m) | (b[j] & ~m);
+        }
+    }
+};
 
 template <int D, int BK, int BV, int NH>
 struct MmaCfg {
@@ -263,84 +316,11 @@ struct MmaCfg {
     static constexpr int PDK = packed_dim(D, BK), PDV = packed_dim(D, BV);
     static constexpr int KSB = PDK / 4, VSB = PDV / 8;  // slice bytes per lane
     static constexpr int KW = (KSB + 3) / 4, VW = (VSB + 3) / 4;   // ... in words
-    static constexpr int IWK = 2 * BK, IWV = 2 * BV;    // table index width (two codes)
-    static constexpr bool BYTE = BK == 4 || BV == 4;    // a 64 KB byte-indexed window is used
     static constexpr int OFF_KN = kPageTokens * PDK;
     static constexpr int OFF_VC = OFF_KN + 2 * kPageTokens;
     static constexpr int OFF_VN = OFF_VC + kPageTokens * PDV;
     static constexpr int PAGE_BYTES = OFF_VN + 2 * kPageTokens;
-    // small (non-byte) tables, each aligned to its own size
-    static constexpr int TKS = BK == 4 ? 0 : (1 << IWK) * 128;
-    // 2-bit values next to 4-bit keys: the upper half of every row of the key's byte window holds,
-    // 16 times, the FOUR centroids of a value byte (8 bytes), so one byte-permute + one 8-byte
-    // load dequantise four codes (instead of shift/and + two 4-byte loads)
-    static constexpr bool V2BYTE = BK == 4 && BV == 2;
-    static constexpr int TVS = (BV == 4 || V2BYTE) ? 0 : (1 << IWV) * 128;
-    static constexpr int SMALL_ALIGN = TKS > TVS ? TKS : TVS;
-    static constexpr int SMALL_BYTES = TKS + TVS + SMALL_ALIGN;  // incl. alignment slack
     static constexpr int STATE_F4 = NH * NMT;                    // float4 items per lane
-    static constexpr bool H8 = NH == 2;       // eight heads in the N dimension (see the fragment maps)
-    static constexpr int HL = H8 ? 2 : 1;     // heads whose softmax state a lane keeps: HL * tg + {0 ..}
-    static constexpr int NPB = H8 ? 1 : 2;    // P.V steps per page
-    // Lane (g, tg) reads slice g of page tokens 4tg .. 4tg + 3, one row per instruction.  Rows of whole
-    // power-of-two sizes put the quad's four rows (4 rows apart) on the same banks: each lane then
-    // starts at another of its four tokens.  24- and 48-byte rows (3 bits, head_dim 64 / 128) are
-    // apart as they are -- rotated they collide (20 extra wavefronts per page at head_dim 64).
-    static constexpr bool ROT = !(BV == 3 && D <= 128);
-    // per-warp ring of stages filled by bulk copies (TMA), one mbarrier per stage; a stage holds the
-    // NP consecutive pages a warp works on at a time
-    static constexpr int RING = 2;
-    // tables, queries, the folded piece, prefix sums, mbarriers, ring addresses
-    static constexpr int MISC_BYTES = SMALL_BYTES + 8 * (D + 16) * 4 + 4 * NH * (D + 4) * 4 +
-                                      (kFlowMaxSeqs + 4) * 4 + 16 * RING * 8 + 16 * 4 + 64;
-    // a warp's share of the merge exchange area: its (O, m, l)
-    static constexpr int XSLOT = 32 * STATE_F4 * 16, XML = NH * 2 * 4 * 4;
-    // Objects are placed first-fit before / after the 64 KB-aligned table window: the misc block, the
-    // exchange area where it has its own space (`sep`: the first pages of the NEXT item can then
-    // already be copied into the rings while the merge runs; else a warp's share lies in its ring,
-    // which is idle during the merge), and every warp's ring.  Bytes needed from `base`.
-    __host__ __device__ static constexpr int ring_bytes(int np, bool sep) {
-        const int ring = RING * np * PAGE_BYTES;
-        return ((sep || ring > XSLOT ? ring : XSLOT) + 127) / 128 * 128;
-    }
-    __host__ __device__ static constexpr int plan(int warps, int np, bool sep, int base) {
-        int free0 = base, end0 = base, free1 = base;
-        if (BYTE) {
-            end0 = (base + 65535) / 65536 * 65536;
-            free1 = end0 + 65536;
-        }
-        const int n = warps + (sep ? 2 : 1);
-        for (int i = 0; i < n; i++) {
-            const int bytes = i == 0 ? MISC_BYTES + warps * XML : (sep && i == 1) ? warps * XSLOT : ring_bytes(np, sep);
-            const int a0 = (free0 + 127) / 128 * 128;
-            if (a0 + bytes <= end0) free0 = a0 + bytes;
-            else free1 = (free1 + 127) / 128 * 128 + bytes;
-        }
-        return (free1 > free0 ? free1 : free0) - base;
-    }
-    __host__ __device__ static constexpr int need(int warps, int np, bool sep) {
-        int worst = 0;
-        const int bases[5] = {0, 16, 1024, 2048, 4096};
-        for (int i = 0; i < 5; i++) {
-            const int n = plan(warps, np, sep, bases[i]);
-            worst = n > worst ? n : worst;
-        }
-        return worst + 128;
-    }
-    static constexpr int CTAS_PER_SM = BYTE ? 1 : 2;
-    static constexpr int LIMIT = BYTE ? 227 * 1024 : 227 * 1024 / CTAS_PER_SM - 1024;
-    // head_dim 256 keeps the query fragments in shared memory (one 8-byte load per k-block and
-    // stage) instead of 32 registers, which lets it run 16 warps per SM like head_dim 128
-    // wherever 16 page rings fit next to the byte table
-    static constexpr int WARPS = (BYTE && D <= 128 && need(16, 1, false) <= LIMIT) ? 16 : 8;
-    // two pages per stage wherever their rings leave the warp count alone
-    static constexpr int NP = need(WARPS, 2, false) <= LIMIT ? 2 : 1;
-    static constexpr int STAGE_BYTES = NP * PAGE_BYTES;
-    // (an 8-warp CTA that owns its SM has 255 registers per thread and keeps them in registers)
-    static constexpr bool QSMEM = D == 256 && !(BYTE && WARPS == 8);
-    static constexpr int THREADS = 32 * WARPS;
-    static constexpr bool SEP = need(WARPS, NP, true) <= LIMIT;
-    static constexpr int SMEM_BYTES = need(WARPS, NP, SEP);
 };
 
 // One page worth of packed data in registers (per lane).

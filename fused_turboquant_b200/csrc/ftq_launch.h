@@ -24,7 +24,6 @@ enum class Encode { kFew, kTable, kAnyCodebook };
                                       cudaStream_t stream);                                   \
     cudaError_t launch_attn_chunk_d##DD(int bits_k, int bits_v, const ChunkAttnParams& p, int B, \
                                         cudaStream_t stream);                                   \
-    int attn_mma_stream_ctas_d##DD(int bits_k, int bits_v, int group);                          \
     cudaError_t launch_attn_merge_d##DD(int out_dtype, const float* partials, void* out,        \
                                         const int32_t* seq_lens, int S, int B, int Hq,          \
                                         int n_chunks, int chunk_tokens, int64_t n_vec,          \

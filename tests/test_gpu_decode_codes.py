@@ -1,0 +1,112 @@
+"""The tensor-core decode kernel over every pair of code widths (how codes become centroids differs with the width of the
+keys, of the values, whether both share a codebook, the head size and the GQA group) and over its two ways to split
+a batch: a cluster of CTAs per (sequence, KV head) unit, equal shares of all units."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from test_gpu_guards import _filled_pool
+from test_gpu_stream_plan import _oracle_bad
+
+pytestmark = pytest.mark.gpu
+
+# at the edges of a page, of a stage of two pages, of a round of all warps
+LENS = [1, 15, 17, 32, 33, 255, 513, 16 * 24 + 1]
+
+
+def _decode(pool, bt, lens, q):
+    out = torch.empty(q.shape, dtype=torch.float32, device="cuda")
+    pool.decode_attention(q, torch.from_numpy(bt).cuda(), torch.tensor(lens, dtype=torch.int32).cuda(), max(lens), layer=0, out=out)
+    torch.cuda.synchronize()
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("times", [1, 10])      # 16 units: clusters; 160 units: equal shares
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("group", [3, 7])
+@pytest.mark.parametrize("bk", [2, 3, 4])
+@pytest.mark.parametrize("bv", [2, 3, 4])
+def test_code_widths(oracle, d, group, bk, bv, times):
+    lens = LENS * times
+    pool, bt, key, val, _, _ = _filled_pool(d, bk, bv, 2, lens, seed=d + bk + bv)
+    g = torch.Generator("cpu").manual_seed(group)
+    q = torch.randn(len(lens), 2 * group, d, generator=g).bfloat16().cuda()
+    got = _decode(pool, bt, lens, q)
+    assert np.isfinite(got).all()
+    which = sorted({*range(8), *range(len(lens) - 8, len(lens))})
+    # (the gate is that of the 16-bit operands: 1e-3 + 2e-3 |ref|)
+    assert _oracle_bad(oracle, pool, key, val, q, np.array(lens), got, d, bk, bv, which) == 0
+
+
+@pytest.mark.parametrize("n_seq", [1, 7, 9, 16, 17, 36, 38, 74, 75])
+def test_cluster_sizes(oracle, n_seq):
+    """Two KV heads: 2 to 150 units, i.e. clusters of 8, 4, 2 and 1 CTAs and equal shares; sequences without tokens,
+    with fewer pages than a cluster has parts, and the longest at the end."""
+    d, group, bits = 128, 4, 4
+    lens = [([0, 1, 130, 16, 900][i % 5]) for i in range(n_seq - 1)] + [3000]
+    pool, bt, key, val, _, _ = _filled_pool(d, bits, bits, 2, lens, seed=n_seq)
+    g = torch.Generator("cpu").manual_seed(n_seq)
+    q = torch.randn(n_seq, 2 * group, d, generator=g).bfloat16().cuda()
+    got = _decode(pool, bt, lens, q)
+    np.testing.assert_array_equal(got, _decode(pool, bt, lens, q))
+    for b, n in enumerate(lens):
+        assert n or (got[b] == 0).all()
+    which = [b for b, n in enumerate(lens) if n][-6:]
+    assert _oracle_bad(oracle, pool, key, val, q, np.array(lens), got, d, bits, bits, which) == 0
+
+
+@pytest.mark.parametrize("times", [1, 30])
+def test_a_block_id_outside_the_pool(times):
+    """Its sequence comes back as NaN, the others as before, and the status word says so (30 times: equal shares)."""
+    lens = [700, 1300, 90] * times
+    pool, bt, *_, used = _filled_pool(128, 4, 4, 2, lens)
+    q = torch.randn(len(lens), 8, 128, generator=torch.Generator("cpu").manual_seed(5)).bfloat16().cuda()
+    good = _decode(pool, bt, lens, q)
+    assert pool.decode_status() == 0
+    pool.num_blocks = used           # (eight blocks more are allocated)
+    bad = bt.copy()
+    bad[1, 3] = used + 2
+    got = _decode(pool, bad, lens, q)
+    assert np.isnan(got[1]).all() and pool.decode_status() == 1
+    rest = [b for b in range(len(lens)) if b != 1]
+    np.testing.assert_array_equal(got[rest], good[rest])
+
+
+@pytest.mark.parametrize("G", [4, 8])
+def test_an_expired_wait_of_equal_shares(G):
+    """The give-up path with a batch that is cut into equal shares: 160 units (see test_gpu_wait_expiry.py)."""
+    from test_gpu_wait_expiry import _test_lib
+
+    from fused_turboquant_b200 import _lib
+    d, bits, Hkv, lens = 128, 4, 2, [4096] * 80
+    pool, bt, *_ = _filled_pool(d, bits, bits, Hkv, lens)
+    q = torch.randn(len(lens), Hkv * G, d, generator=torch.Generator("cpu").manual_seed(9)).bfloat16().cuda()
+    sl, table = torch.tensor(lens, dtype=torch.int32).cuda(), torch.from_numpy(bt).cuda()
+    ws = torch.empty(pool.workspace_bytes(len(lens), Hkv * G, 4096, 1), dtype=torch.uint8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+
+    def run(lib):
+        out = torch.full(q.shape, 7.0, dtype=torch.float32, device="cuda")
+        rc = lib.ftq_paged_decode_attn(
+            p(q), _lib.BF16, p(out), _lib.F32, p(pool.pool[0]), pool.num_blocks, pool.layer_stride, 1, p(table),
+            table.shape[1], p(sl), 4096, len(lens), Hkv * G, Hkv, d, bits, bits, _lib.fptr(pool.levels_k),
+            _lib.fptr(pool.levels_v), _lib.fptr(pool.signs), d ** -0.5, p(ws), ws.numel(), stream)
+        assert rc == 0, lib.ftq_last_error()
+        status = ctypes.c_int(-1)
+        rc = lib.ftq_paged_decode_status(p(ws), len(lens), Hkv * G, Hkv, d, 4096, 1, stream, ctypes.byref(status))
+        return out.cpu().numpy(), rc, status.value
+
+    good, rc, status = run(_lib.load())
+    assert (rc, status) == (0, 0) and np.isfinite(good).all()
+    got, rc, status = run(_test_lib())
+    assert (rc, status) == (-5, 2)
+    units = got.reshape(len(lens), Hkv, G, d)
+    poisoned = np.isnan(units).any(axis=(2, 3))
+    assert poisoned.sum() == 1 and np.isnan(units[poisoned]).all()
+    np.testing.assert_array_equal(units[~poisoned], good.reshape(units.shape)[~poisoned])
+    again, rc, status = run(_lib.load())
+    assert (rc, status) == (0, 0)
+    np.testing.assert_array_equal(again, good)

@@ -693,6 +693,7 @@ int ftq_flash_decode(const void* q, int q_dtype, int q_is_rotated, const uint8_t
     if (rc) return rc;
     rc = pack_levels(levels_v_host, bits_v, &p.lv);
     if (rc) return rc;
+    p.shared_table = bits_k == bits_v && memcmp(p.lk.v, p.lv.v, sizeof(float) << bits_k) == 0;
     rc = pack_signs(signs_host, head_dim, &p.signs);
     if (rc) return rc;
     const int pdk = ftq::packed_dim(head_dim, bits_k), pdv = ftq::packed_dim(head_dim, bits_v);
@@ -794,6 +795,7 @@ int ftq_paged_decode_attn(const void* q, int q_dtype, void* out, int out_dtype,
     if (rc) return rc;
     rc = pack_levels(levels_v_host, bits_v, &p.lv);
     if (rc) return rc;
+    p.shared_table = bits_k == bits_v && memcmp(p.lk.v, p.lv.v, sizeof(float) << bits_k) == 0;
     rc = pack_signs(signs_host, head_dim, &p.signs);
     if (rc) return rc;
     p.q = q;

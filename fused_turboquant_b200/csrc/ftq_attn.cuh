@@ -67,6 +67,7 @@ struct AttnParams {
     int out_dtype;
     int64_t num_blocks;         // block ids are checked against it
     Codebook lk, lv;
+    int shared_table;           // fp32 kernel: keys and values have the same codebook
     SignBits signs;
     float rsqrt_d;
     // tensor-core path: V centroids pre-multiplied by v_scale before the fp16 rounding
@@ -146,7 +147,21 @@ __device__ __forceinline__ uint32_t extract_code(const uint32_t (&w)[NWORDS], in
     return __funnelshift_r(w[lo], w[lo + 1 < NWORDS ? lo + 1 : lo], sh) & mask;
 }
 
+// Shared-memory byte offset (entry * 128) of the table entry for code pair `pair`
+// of a slice: bits [pair*IW, pair*IW + IW) of the little-endian stream in w[].
+template <int IW, int NW>
+__device__ __forceinline__ uint32_t pair_index(const uint32_t (&w)[NW], int pair) {
+    constexpr uint32_t mask = ((1u << IW) - 1u) << 7;
+    const int bo = pair * IW;
+    const int j = bo >> 5, sh = bo & 31;
+    uint32_t x;
+    if (sh + IW <= 32) x = sh >= 7 ? (w[j] >> (sh - 7)) : (w[j] << (7 - sh));
+    else x = __funnelshift_r(w[j], w[j + 1 < NW ? j + 1 : j], sh - 7);
+    return x & mask;
+}
+
 constexpr int kTilePages = 4;
+constexpr int kTileRing = 2;       // buffers of a page of a warp (three measure alike)
 constexpr int kAttnThreads = 128;
 
 template <int D>
@@ -155,6 +170,13 @@ struct AttnCfg {
     static constexpr int GH = 64 / E;  // query heads per pass: 8 / 4 / 2 for D = 64 / 128 / 256
 };
 
+// Bound by instruction issue and its latencies at two CTAs of four warps per SM (some 230 registers a thread hold the
+// queries and the accumulators; three CTAs of 168 spill: 32.7 us in place of 24.6 below).  So: a pair of codes is one
+// look-up of an 8-byte entry (extracting and looking up each code took four instructions), the octet's dot products
+// are added up in a tree that leaves every lane one head (a third of the shuffles, a quarter of the exponentials), and
+// every warp fetches its own pages without a barrier of the CTA in the loop.  4 x 4001 tokens, 32 / 8 heads of 128,
+// K4V4, contiguous: 32.8 -> 28.6 -> 24.6 us with its merge; 16 x 3000, 8 / 8 heads 108 -> 52; paged, 16 x 2000, 32 / 8
+// heads, with the store 66 -> 56.  Each sum is made in the order it had.
 // PAGED: pages come from the pool through the block table; otherwise they are
 // cut from contiguous [B,Hkv,S,*] tensors (cp.async granule 16 bytes when every
 // span is 16-byte aligned, p.cp16, else 4).
@@ -175,13 +197,15 @@ attn_split_kernel(const AttnParams p) {
     // the tile ring doubles as the cross-warp merge area once the loop is over
     constexpr int MERGE_BYTES = 4 * GH * (D + 2) * 4;
     constexpr int RING_BYTES =
-        ((2 * TILE_BYTES > MERGE_BYTES ? 2 * TILE_BYTES : MERGE_BYTES) + 15) / 16 * 16;
+        ((kTileRing * TILE_BYTES > MERGE_BYTES ? kTileRing * TILE_BYTES : MERGE_BYTES) + 15) / 16 * 16;
 
     extern __shared__ __align__(16) uint8_t smem_raw[];
     uint8_t* tiles = smem_raw;                                   // RING_BYTES
     float* qs = reinterpret_cast<float*>(smem_raw + RING_BYTES);      // [GH][D]
-    float* lutk = qs + GH * D;
-    float* lutv = lutk + kMaxLevels;
+    // dequantisation tables: an entry is the two centroids of a pair of codes, sixteen copies of it a row, so that a half
+    // warp's 8-byte look-ups never meet in a bank
+    constexpr int TAB_K = RING_BYTES + GH * D * 4, TK_BYTES = (1 << (2 * BK)) * 128;
+    const int tab_v = TAB_K + (p.shared_table ? 0 : TK_BYTES);
 
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -216,14 +240,15 @@ attn_split_kernel(const AttnParams p) {
     const int32_t* btab = PAGED ? p.block_table + static_cast<int64_t>(b) * p.max_blocks : nullptr;
     const int64_t cbase = (static_cast<int64_t>(b) * p.Hkv + hkv) * p.S;
 
-    bool bad_block = false;  // (every thread walks the same block ids)
-    auto issue_tile = [&](int ti, int buf) {
-        uint8_t* dst = tiles + buf * TILE_BYTES;
-#pragma unroll
-        for (int pi = 0; pi < kTilePages; pi++) {
-            const int ts = t0 + ti * (kTilePages * kPageTokens) + pi * kPageTokens;
-            if (ts >= t1) break;
-            uint8_t* pd = dst + pi * PAGE_BYTES;
+    // A warp's page of tile ti (tokens t0 + 64 ti + 16 warp ..) on its way to the warp's buffer: nobody else reads it, so
+    // the loop has no barrier of the whole CTA.  The norms of a contiguous source lie on 2-byte boundaries: a lane keeps
+    // the one it loads until the page is waited for.
+    bool bad_block = false;
+    uint16_t norm[kTileRing] = {};
+    auto issue_page = [&](int ti, int buf) {
+        const int ts = t0 + ti * (kTilePages * kPageTokens) + warp * kPageTokens;
+        if (ts < t1) {
+            uint8_t* pd = tiles + buf * TILE_BYTES + warp * PAGE_BYTES;
             if constexpr (PAGED) {
                 // a block id outside the pool is never dereferenced: block 0 stands in and the
                 // chunk's result is replaced by NaN below
@@ -233,40 +258,42 @@ attn_split_kernel(const AttnParams p) {
                     bad_block = true;
                 }
                 const uint8_t* src = pool + (blk * p.Hkv + hkv) * PAGE_BYTES;
-                stage_span<16>(pd, src, PAGE_BYTES, PAGE_BYTES, tid, kAttnThreads);
+                stage_span<16>(pd, src, PAGE_BYTES, PAGE_BYTES, lane, 32);
             } else {
                 const int ntok = min(kPageTokens, t1 - ts);
                 if (p.cp16) {
                     stage_span<16>(pd, p.k_codes + (cbase + ts) * PDK, kPageTokens * PDK,
-                                   ntok * PDK, tid, kAttnThreads);
+                                   ntok * PDK, lane, 32);
                     stage_span<16>(pd + OFF_VC, p.v_codes + (cbase + ts) * PDV, kPageTokens * PDV,
-                                   ntok * PDV, tid, kAttnThreads);
+                                   ntok * PDV, lane, 32);
                 } else {
                     stage_span<4>(pd, p.k_codes + (cbase + ts) * PDK, kPageTokens * PDK,
-                                  ntok * PDK, tid, kAttnThreads);
+                                  ntok * PDK, lane, 32);
                     stage_span<4>(pd + OFF_VC, p.v_codes + (cbase + ts) * PDV, kPageTokens * PDV,
-                                  ntok * PDV, tid, kAttnThreads);
+                                  ntok * PDV, lane, 32);
                 }
-                if (tid < 2 * kPageTokens) {
-                    const int tk = tid & (kPageTokens - 1);
-                    const bool isv = tid >= kPageTokens;
-                    const uint16_t* nsrc = isv ? p.v_norms : p.k_norms;
-                    const uint16_t val = tk < ntok ? nsrc[cbase + ts + tk] : uint16_t(0);
-                    reinterpret_cast<uint16_t*>(pd + (isv ? OFF_VN : OFF_KN))[tk] = val;
-                }
+                const int tk = lane & (kPageTokens - 1);
+                norm[buf] = tk < ntok ? (lane >= kPageTokens ? p.v_norms : p.k_norms)[cbase + ts + tk] : uint16_t(0);
             }
         }
         cp_async_commit();
     };
 
     const int n_tiles = (t1 - t0 + kTilePages * kPageTokens - 1) / (kTilePages * kPageTokens);
-    issue_tile(0, 0);
+#pragma unroll
+    for (int i = 0; i < kTileRing - 1; i++) issue_page(i, i);
 
     // ---- prologue: tables and the rotated, pre-scaled queries of this pass
-    if (tid < kMaxLevels) {
-        lutk[tid] = p.lk.v[tid];
-        lutv[tid] = p.lv.v[tid];
-    }
+    auto build = [&](int at, const Codebook& levels, int bits) {
+        // (a thread's two copies of an entry: one 16-byte store)
+        for (int i = tid; i < 8 << (2 * bits); i += kAttnThreads) {
+            const int e = i >> 3;
+            const float lo = levels.v[e & ((1 << bits) - 1)], hi = levels.v[e >> bits];
+            *reinterpret_cast<float4*>(smem_raw + at + i * 16) = make_float4(lo, hi, lo, hi);
+        }
+    };
+    build(TAB_K, p.lk, BK);
+    if (!p.shared_table) build(tab_v, p.lv, BV);
     {
         const int hh = warp * 4 + o;  // one octet rotates one query head (GH <= 8 < 16 octets)
         const bool hv = hh < nh;
@@ -314,31 +341,45 @@ attn_split_kernel(const AttnParams p) {
         for (int i = 0; i < EP; i++)
             qr[h][i] = pk2(qs[h * D + t * E + 2 * i], qs[h * D + t * E + 2 * i + 1]);
 
-    float m_run[GH], l_run[GH];
+    // Softmax state of ONE head, that of the lane: the dot products of an octet's lanes are added up in a tree that leaves
+    // each lane with a head of its own (for fewer heads than lanes, several with the same).
+    constexpr int HB = GH == 8 ? 3 : GH == 4 ? 2 : 1;      // bits of a lane's number that say its head
+    int my_head = 0;
 #pragma unroll
-    for (int h = 0; h < GH; h++) {
-        m_run[h] = -INFINITY;
-        l_run[h] = 0.f;
+    for (int i = 0; i < HB; i++) my_head |= ((t >> i) & 1) << (HB - 1 - i);
+    auto lane_of = [&](int h) {   // a lane of this octet with head h
+        int r = lane & 24;
+#pragma unroll
+        for (int i = 0; i < HB; i++) r |= ((h >> (HB - 1 - i)) & 1) << i;
+        return r;
+    };
+    float m_run = -INFINITY, l_run = 0.f;
+#pragma unroll
+    for (int h = 0; h < GH; h++)
 #pragma unroll
         for (int i = 0; i < EP; i++) acc[h][i] = pk2(0.f, 0.f);
-    }
+    // centroids of the lane's code pair `pair`
+    const uint32_t col = (lane & 15) * 8;
+    auto look_up = [&](int at, uint32_t index) { return *reinterpret_cast<const u64*>(smem_raw + at + (index | col)); };
 
-    // ---- main loop over 64-token tiles, double buffered
-    for (int ti = 0; ti < n_tiles; ti++) {
-        if (ti + 1 < n_tiles) {
-            issue_tile(ti + 1, (ti + 1) & 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
+    // ---- main loop over 64-token tiles, a page per warp
+    for (int ti0 = 0; ti0 < n_tiles; ti0 += kTileRing) {
+#pragma unroll
+      for (int buf = 0; buf < kTileRing; buf++) {     // (buffer numbers known to the compiler: `norm` stays in registers)
+        const int ti = ti0 + buf;
+        if (ti >= n_tiles) break;
+        issue_page(ti + kTileRing - 1, (buf + kTileRing - 1) % kTileRing);
+        cp_async_wait<kTileRing - 1>();
+        uint8_t* page = tiles + buf * TILE_BYTES + warp * PAGE_BYTES;
+        if constexpr (!PAGED)
+            reinterpret_cast<uint16_t*>(page + (lane >= kPageTokens ? OFF_VN : OFF_KN))[lane & (kPageTokens - 1)] = norm[buf];
+        __syncwarp();
 
         const int ts = t0 + ti * (kTilePages * kPageTokens) + warp * kPageTokens;
         if (ts < t1) {  // warp-uniform
             const int ntok = min(kPageTokens, t1 - ts);
-            const uint8_t* page = tiles + (ti & 1) * TILE_BYTES + warp * PAGE_BYTES;
 
-            float sc[4][GH];
+            float sc[4];
 #pragma unroll
             for (int step = 0; step < 4; step++) {
                 const int tk = step * 4 + o;
@@ -348,8 +389,8 @@ attn_split_kernel(const AttnParams p) {
                     __half2float(reinterpret_cast<const __half*>(page + OFF_KN)[tk]);
                 u64 kv[EP];
 #pragma unroll
-                for (int i = 0; i < EP; i++)
-                    kv[i] = pk2(lutk[extract_code<BK>(w, 2 * i)], lutk[extract_code<BK>(w, 2 * i + 1)]);
+                for (int i = 0; i < EP; i++) kv[i] = look_up(TAB_K, pair_index<2 * BK>(w, i));
+                float d[GH];
 #pragma unroll
                 for (int h = 0; h < GH; h++) {
                     u64 d2 = pk2(0.f, 0.f);
@@ -357,35 +398,49 @@ attn_split_kernel(const AttnParams p) {
                     for (int i = 0; i < EP; i++) d2 = fma2(qr[h][i], kv[i], d2);
                     float d0, d1;
                     upk2(d2, d0, d1);
-                    float d = d0 + d1;
-                    d += __shfl_xor_sync(0xffffffffu, d, 1);
-                    d += __shfl_xor_sync(0xffffffffu, d, 2);
-                    d += __shfl_xor_sync(0xffffffffu, d, 4);
-                    sc[step][h] = tk < ntok ? d * kn : -INFINITY;
+                    d[h] = d0 + d1;
                 }
+#pragma unroll
+                for (int i = 0; i < 3; i++) {
+                    const int n = GH >> (i + 1);
+                    if (n > 0) {
+                        const bool up = (t >> i) & 1;   // this lane keeps the upper half of the heads
+#pragma unroll
+                        for (int k = 0; k < (n > 0 ? n : 1); k++) {
+                            const float give = up ? d[k] : d[k + n], keep = up ? d[k + n] : d[k];
+                            d[k] = keep + __shfl_xor_sync(0xffffffffu, give, 1 << i);
+                        }
+                    } else {
+                        d[0] += __shfl_xor_sync(0xffffffffu, d[0], 1 << i);
+                    }
+                }
+                sc[step] = tk < ntok ? d[0] * kn : -INFINITY;
             }
 
-            float wp[4][GH];
+            float mx = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+            // (a maximum that stays leaves the accumulators as they are: the factor is one)
+            if (__any_sync(0xffffffffu, !(mx <= m_run))) {
+                const float m_new = fmaxf(m_run, mx);  // finite: token 0 of the page is valid
+                const float corr = m_run == -INFINITY ? 0.f : __expf(m_run - m_new);
+                m_run = m_new;
+                l_run *= corr;
 #pragma unroll
-            for (int h = 0; h < GH; h++) {
-                float mx = fmaxf(fmaxf(sc[0][h], sc[1][h]), fmaxf(sc[2][h], sc[3][h]));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                const float m_new = fmaxf(m_run[h], mx);  // finite: token 0 of the page is valid
-                const float corr = m_run[h] == -INFINITY ? 0.f : __expf(m_run[h] - m_new);
-                m_run[h] = m_new;
-                float ls = 0.f;
+                for (int h = 0; h < GH; h++) {
+                    const float c = __shfl_sync(0xffffffffu, corr, lane_of(h));
+                    const u64 corr2 = pk2(c, c);
 #pragma unroll
-                for (int step = 0; step < 4; step++) {
-                    const float pe = sc[step][h] == -INFINITY ? 0.f : __expf(sc[step][h] - m_new);
-                    ls += pe;
-                    wp[step][h] = pe;
+                    for (int i = 0; i < EP; i++) acc[h][i] = mul2(acc[h][i], corr2);
                 }
-                l_run[h] = l_run[h] * corr + ls;
-                const u64 corr2 = pk2(corr, corr);
-#pragma unroll
-                for (int i = 0; i < EP; i++) acc[h][i] = mul2(acc[h][i], corr2);
             }
+            float wp[4], ls = 0.f;
+#pragma unroll
+            for (int step = 0; step < 4; step++) {
+                wp[step] = sc[step] == -INFINITY ? 0.f : __expf(sc[step] - m_run);
+                ls += wp[step];
+            }
+            l_run += ls;
 
 #pragma unroll
             for (int step = 0; step < 4; step++) {
@@ -394,36 +449,37 @@ attn_split_kernel(const AttnParams p) {
                 // pool pages store a V row with its halves exchanged for tokens with bit 1 set
                 const int vt = PAGED ? (t ^ ((tk & 2) << 1)) : t;
                 load_code_bytes<NBV>(page + OFF_VC + tk * PDV + vt * NBV, w);
-                const float vn = tk < ntok
-                    ? __half2float(reinterpret_cast<const __half*>(page + OFF_VN)[tk]) : 0.f;
+                const float vn = __half2float(reinterpret_cast<const __half*>(page + OFF_VN)[tk]);
+                const float wgt = tk < ntok ? wp[step] * vn : 0.f;
                 u64 vv[EP];
 #pragma unroll
-                for (int i = 0; i < EP; i++)
-                    vv[i] = pk2(lutv[extract_code<BV>(w, 2 * i)], lutv[extract_code<BV>(w, 2 * i + 1)]);
+                for (int i = 0; i < EP; i++) vv[i] = look_up(tab_v, pair_index<2 * BV>(w, i));
 #pragma unroll
                 for (int h = 0; h < GH; h++) {
-                    const float wgt = tk < ntok ? wp[step][h] * vn : 0.f;
-                    const u64 wgt2 = pk2(wgt, wgt);
+                    const float wh = __shfl_sync(0xffffffffu, wgt, lane_of(h));
+                    const u64 wgt2 = pk2(wh, wh);
 #pragma unroll
                     for (int i = 0; i < EP; i++) acc[h][i] = fma2(wgt2, vv[i], acc[h][i]);
                 }
             }
         }
-        __syncthreads();
+        __syncwarp();   // (the buffer is requested again in the next round)
+      }
     }
 
     // ---- combine the 4 octets of each warp, then the 4 warps through shared memory
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 8);
+    l_run += __shfl_xor_sync(0xffffffffu, l_run, 16);
 #pragma unroll
     for (int h = 0; h < GH; h++) {
-        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 8);
-        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 16);
 #pragma unroll
         for (int i = 0; i < EP; i++) {
             acc[h][i] = add2(acc[h][i], __shfl_xor_sync(0xffffffffu, acc[h][i], 8));
             acc[h][i] = add2(acc[h][i], __shfl_xor_sync(0xffffffffu, acc[h][i], 16));
         }
     }
-    float* wacc = reinterpret_cast<float*>(tiles);   // [4][GH][D]   (tiles are free now)
+    bad_block = __syncthreads_or(bad_block) != 0;    // (nobody reads the tiles any more)
+    float* wacc = reinterpret_cast<float*>(tiles);   // [4][GH][D]
     float* wm = wacc + 4 * GH * D;                   // [4][GH]
     float* wl = wm + 4 * GH;                         // [4][GH]
     if (o == 0) {
@@ -432,10 +488,10 @@ attn_split_kernel(const AttnParams p) {
 #pragma unroll
             for (int i = 0; i < EP; i++)
                 *reinterpret_cast<u64*>(wacc + (warp * GH + h) * D + t * E + 2 * i) = acc[h][i];
-            if (t == 0) {
-                wm[warp * GH + h] = m_run[h];
-                wl[warp * GH + h] = l_run[h];
-            }
+        }
+        if (t < GH) {   // (the lanes with the heads' first copies)
+            wm[warp * GH + my_head] = m_run;
+            wl[warp * GH + my_head] = l_run;
         }
     }
     __syncthreads();

@@ -18,11 +18,14 @@ static cudaError_t run_split(const AttnParams& p, int n_lb, cudaStream_t stream)
     constexpr int GH = AttnCfg<D>::GH;
     constexpr int page = kPageTokens * (packed_dim(D, BK) + packed_dim(D, BV) + 4);
     constexpr int merge = 4 * GH * (D + 2) * 4;
-    constexpr int ring = ((2 * kTilePages * page > merge ? 2 * kTilePages * page : merge) + 15) / 16 * 16;
-    constexpr int smem = ring + (GH * D + 2 * kMaxLevels) * 4;
-    static_assert(smem <= 48 * 1024, "shared memory budget");
+    constexpr int ring = ((kTileRing * kTilePages * page > merge ? kTileRing * kTilePages * page : merge) + 15) / 16 * 16;
+    constexpr int tk = (1 << (2 * BK)) * 128, tv = (1 << (2 * BV)) * 128;
+    constexpr int smem = ring + GH * D * 4 + tk;
+    constexpr auto kern = attn_split_kernel<D, BK, BV, PAGED>;
+    const cudaError_t e = allow_smem<kern>(smem + tv);
+    if (e != cudaSuccess) return e;
     const dim3 grid(p.n_chunks, p.Hkv * p.n_hpass, n_lb);
-    attn_split_kernel<D, BK, BV, PAGED><<<grid, kAttnThreads, smem, stream>>>(p);
+    kern<<<grid, kAttnThreads, smem + (p.shared_table ? 0 : tv), stream>>>(p);
     return cudaGetLastError();
 }
 

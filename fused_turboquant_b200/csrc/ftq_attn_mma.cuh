@@ -214,19 +214,6 @@ __device__ __forceinline__ void lds_slice(uint32_t addr, uint32_t sh, uint32_t (
     }
 }
 
-// Shared-memory byte offset (entry * 128) of the table entry for code pair `pair`
-// of a slice: bits [pair*IW, pair*IW + IW) of the little-endian stream in w[].
-template <int IW, int NW>
-__device__ __forceinline__ uint32_t pair_index(const uint32_t (&w)[NW], int pair) {
-    constexpr uint32_t mask = ((1u << IW) - 1u) << 7;
-    const int bo = pair * IW;
-    const int j = bo >> 5, sh = bo & 31;
-    uint32_t x;
-    if (sh + IW <= 32) x = sh >= 7 ? (w[j] >> (sh - 7)) : (w[j] << (7 - sh));
-    else x = __funnelshift_r(w[j], w[j + 1 < NW ? j + 1 : j], sh - 7);
-    return x & mask;
-}
-
 // Shared-memory address of the table entry for code pair `pair` of a slice.
 //   IW == 8 (4-bit): lane_base = window | table half | lane*4; the code byte becomes byte 1.
 //   IW  < 8        : lane_base = table | lane*4; entry * 128 is or-ed in.

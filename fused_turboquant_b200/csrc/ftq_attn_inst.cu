@@ -122,25 +122,27 @@ static int clusters_at_a_time(int size, int threads, int smem) {
 }
 
 // Few units with short contexts (at most one per SM): a cluster of 8, 4, 2 CTAs or one CTA per unit, as many as the device
-// holds at a time, whose parts are put together over distributed shared memory.  Rows in the workspace, a fence, a
-// counter and the rows again are a chain of 6 to 8 us at the end of the equal-share kernel; here it is 2.  Measured as
-// steps (store included, equal shares : clusters; 32 / 8 heads of 128, K3V3, bounded by the host at 12): 1 x 900
-// tokens 23 : 11.7, 1 x 8000 25 : 16, 9 x 5000 ragged 30 : 22, 18 x 3000 30 : 26 us.
-// kClusterPages is the longest part of a half: what the longest sequence of a ragged batch takes (30 us) while the
-// equal shares would even it out.  Returns cudaErrorNotSupported where equal shares are the better ones.
-constexpr int kClusterPages = 192;
+// holds at a time, whose parts are put together over distributed shared memory.  Rows in the workspace, a counter and
+// the rows again are a chain of 5 us at the end of the equal-share kernel, and few long units have many rows; a
+// cluster's merge takes 2 us, but leaves SMs idle where the units do not fill them and cannot even out a ragged batch.
+// Steps (store included) by clusters : equal shares, parts of 40, 100 and 185 pages: 8 units of 128 coordinates, K4V4,
+// in clusters of 8 16.3 : 22.3, 24.7 : 27.2, 37.0 : 30.9 us; 4 units, K3V3 17.4 : 25.6, 26.6 : 36.2, 39.2 : 35.1; 48
+// units in clusters of 2 16.5 : 19.1, 24.9 : 24.1, 36.6 : 31.0; 104 units, one CTA each, 16.9 : 19.6, 25.3 : 24.5, 37.0 :
+// 31.3, ragged 36.0 : 19.9.  So the lines, in pages of a half's part:
+constexpr int kClusterPages8 = 112, kClusterPages = 72;
+// Returns cudaErrorNotSupported where equal shares are the better ones.
 template <int BK, int BV, bool SHARED, int NH>
 static cudaError_t run_cluster(const AttnParams& p_in, cudaStream_t stream) {
     using C = FlowCfg<FTQ_D, BK, BV, NH, true>;
     static_assert(C::SMEM_BYTES <= C::LIMIT, "shared memory budget");
     constexpr auto kern = attn_flow_kernel<FTQ_D, BK, BV, SHARED, NH, true>;
     const int pages = (p_in.max_seq + kPageTokens - 1) / kPageTokens;
-    if (p_in.n_units > sm_count() || pages > kClusterPages * 8 * C::HALVES) return cudaErrorNotSupported;
+    if (p_in.n_units > sm_count() || pages > kClusterPages8 * 8 * C::HALVES) return cudaErrorNotSupported;
     cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     int size = 8;
     while (size > 1 && clusters_at_a_time<kern>(size, C::HALVES * C::THREADS, C::SMEM_BYTES) < p_in.n_units) size /= 2;
-    if (pages > kClusterPages * size * C::HALVES) return cudaErrorNotSupported;
+    if (pages > (size == 8 ? kClusterPages8 : kClusterPages) * size * C::HALVES) return cudaErrorNotSupported;
     AttnParams p = p_in;
     p.b0 = 0;
     p.B_stride = p_in.B;

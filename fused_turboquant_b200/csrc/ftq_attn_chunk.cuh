@@ -19,10 +19,13 @@
 // fp16 rotated queries, fp16 weights, fp32 accumulation, fp32 softmax.
 //
 // Warps: SLOTS x 4 softmax warps, KT * D / 1024 dequantising warps (codes of a tile are loaded into
-// registers one tile ahead, looked up in the lane-replicated tables, written as fp16 tiles, two
+// registers one tile ahead, looked up in the lane-replicated tables, written as fp16 tiles, three
 // stages), one warp that issues the MMAs: scores of tile i are issued before P.V of tile i - 1, so that
-// softmax, dequantisation and the tensor core overlap.  What bounds it: the softmax instructions
-// (about 8 per score); the tensor pipe is busy a sixth of the time.
+// softmax, dequantisation and the tensor core overlap.  What bounds it is that last warp's line of work: by the clock
+// of a CTA (4 x 64 queries over 4096 tokens, 32 / 8 heads of 128, K4V4) a tile of 64 tokens and 256 rows took 4200 cycles,
+// 1000 of them waiting for the tile, 1780 for the scores' sixteen MMAs, 1250 for P.V's eight; now 3060, with a third
+// stage and operands in uniform registers.  61.5 -> 53.4 us with its merge, 50.9 with the queries' loads side by side and the
+// tables built while the kernel before drains; 2 x 512 queries 172 -> 130.
 //
 // The tiles of a row tile's causal range are cut into up to `splits` parts (grid.x); every CTA leaves its rows
 // (O, m, l) in the workspace and attn_merge_kernel finishes.
@@ -73,16 +76,19 @@ struct ChunkCfg {
     static constexpr int OFF_VN = OFF_VC + kPageTokens * PDV;
     static constexpr int PAGE_BYTES = OFF_VN + 2 * kPageTokens;
     static constexpr int TK_BYTES = (1 << (2 * BK)) * 128, TV_BYTES = (1 << (2 * BV)) * 128;
-    // shared memory, 1024-byte aligned parts: Q tiles, K and V tiles (2 stages), tables, norms, barriers
+    // K and V tiles: with two, a tile was dequantised (1000 cycles) after P.V of the tile before the last and before its own
+    // scores, i.e. in series with the tensor core
+    static constexpr int STAGES = 3;
+    // shared memory, 1024-byte aligned parts: Q tiles, K and V tiles, tables, norms, barriers
     static constexpr int Q_TILE = 128 * D * 2, KV_TILE = KT * D * 2;
     static constexpr int OFF_Q = 0;
     static constexpr int OFF_K = OFF_Q + SLOTS * Q_TILE;
-    static constexpr int OFF_V = OFF_K + 2 * KV_TILE;
-    static constexpr int OFF_TK = OFF_V + 2 * KV_TILE;
+    static constexpr int OFF_V = OFF_K + STAGES * KV_TILE;
+    static constexpr int OFF_TK = OFF_V + STAGES * KV_TILE;
     static constexpr int OFF_TV = OFF_TK + TK_BYTES;
-    static constexpr int OFF_NORM = OFF_TV + TV_BYTES;     // [2 stages][2][KT] floats
-    static constexpr int OFF_BAR = OFF_NORM + 4 * KT * 4;
-    static constexpr int USED = OFF_BAR + 128 + 1024;      // (1024: alignment of the base)
+    static constexpr int OFF_NORM = OFF_TV + TV_BYTES;     // [STAGES][2][KT] floats
+    static constexpr int OFF_BAR = OFF_NORM + STAGES * 2 * KT * 4;
+    static constexpr int USED = OFF_BAR + 160 + 1024;      // (1024: alignment of the base)
     // one CTA per SM: a second one would only wait for TMEM
     static constexpr int SMEM_BYTES = USED > 120 * 1024 ? USED : 120 * 1024;
     // TMEM columns of a slot: O (fp32), S (fp32), P (fp16 pairs)
@@ -106,17 +112,20 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tc_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
+// (Run by a whole warp, whose lane `one` issues: the operands are uniform registers, and code that only one lane
+// runs has to move each of them there.  Shared-memory descriptors as lower and upper halves; the upper one is
+// common to both operands.)
+__device__ __forceinline__ void tc_mma_ss(bool one, uint32_t d, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc, bool acc) {
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
-        "r"(static_cast<uint32_t>(acc)) : "memory");
+        "{\n.reg .pred p, q;\n.reg .b64 da, db;\nmov.b64 da, {%1, %3};\nmov.b64 db, {%2, %3};\nsetp.ne.b32 p, %5, 0;\n"
+        "setp.ne.b32 q, %6, 0;\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n}\n" ::"r"(d), "r"(a), "r"(b),
+        "r"(hi), "r"(idesc), "r"(static_cast<uint32_t>(acc)), "r"(static_cast<uint32_t>(one)) : "memory");
 }
-__device__ __forceinline__ void tc_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool acc) {
+__device__ __forceinline__ void tc_mma_ts(bool one, uint32_t d, uint32_t a, uint32_t b, uint32_t hi, uint32_t idesc, bool acc) {
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d), "r"(a), "l"(b), "r"(idesc),
-        "r"(static_cast<uint32_t>(acc)) : "memory");
+        "{\n.reg .pred p, q;\n.reg .b64 db;\nmov.b64 db, {%2, %3};\nsetp.ne.b32 p, %5, 0;\n"
+        "setp.ne.b32 q, %6, 0;\n@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n}\n" ::"r"(d), "r"(a), "r"(b),
+        "r"(hi), "r"(idesc), "r"(static_cast<uint32_t>(acc)), "r"(static_cast<uint32_t>(one)) : "memory");
 }
 // 32 lanes x 16 columns of 32 bits, one row per lane
 __device__ __forceinline__ void tc_ld16(uint32_t addr, uint32_t* r) {
@@ -142,13 +151,9 @@ __device__ __forceinline__ void tc_wait_ld(uint32_t* r) {
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
-// Shared-memory matrix descriptor, 128-byte swizzle: `lead` and `stride` in bytes (K-major: stride =
-// distance of 8-row groups; MN-major: lead = distance of 64-element chunks, stride = of 8-k groups).
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr, uint32_t lead, uint32_t stride) {
-    return static_cast<uint64_t>((addr & 0x3ffffu) >> 4) | (static_cast<uint64_t>(lead >> 4) << 16) |
-           (static_cast<uint64_t>(stride >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-
+// Shared-memory matrix descriptor, 128-byte swizzle: bits 0-13 address / 16, 16-29 the distance of 64-element chunks / 16
+// (MN-major; K-major: unused), 32-45 of 8-row (K-major) or 8-k (MN-major) groups / 16, 46 set, 61-63 = 2.  Addresses are
+// below 256 KB.
 template <int D, int BK, int BV>
 __global__ void __launch_bounds__(ChunkCfg<D, BK, BV>::THREADS, 1)
 attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
@@ -158,7 +163,23 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
     const uint32_t raw = static_cast<uint32_t>(__cvta_generic_to_shared(smem_raw));
     const uint32_t sbase = (raw + 1023u) & ~1023u;
     uint8_t* const smem = smem_raw + (sbase - raw);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+
+    // ---- tables: an entry (the fp16 centroids of two adjacent codes) 32 times, bank = lane
+    {
+        auto build = [&](int off, int bits, const Codebook& cb) {
+            uint32_t* t = reinterpret_cast<uint32_t*>(smem + off);
+            const float lev = cb.v[lane & 15];
+            for (int e = warp; e < (1 << (2 * bits)); e += C::THREADS / 32) {
+                const __half2 h = __floats2half2_rn(__shfl_sync(0xffffffffu, lev, e & ((1 << bits) - 1)),
+                                                    __shfl_sync(0xffffffffu, lev, e >> bits));
+                t[e * 32 + lane] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+        };
+        build(C::OFF_TK, BK, p.lk);
+        build(C::OFF_TV, BV, p.lv);
+    }
+    after_previous_kernel();    // (nothing in global memory was touched so far)
 
     // ---- what this CTA works on
     const int group = p.Hq / p.Hkv, rows = p.q_len * group;
@@ -212,17 +233,20 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
     __shared__ int s_nan_pos;   // first token whose value norm is NaN
     const volatile int* const abort_now = &s_abort;
     const uint32_t bars = sbase + C::OFF_BAR;
-    const uint32_t kv_full = bars, kv_empty = bars + 16, s_full = bars + 32, s_free = bars + 48,
-                   p_full = bars + 64, o_done = bars + 80,   // two of each
-                   drained = bars + 96;
+    constexpr int NST = C::STAGES;
+    const uint32_t kv_full = bars, kv_empty = bars + 32,                    // NST of each
+                   s_full = bars + 64, s_free = bars + 80, p_full = bars + 96, o_done = bars + 112,   // two of each
+                   drained = bars + 128;
     if (warp == C::SM_WARPS + C::DQ_WARPS) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(
                          static_cast<uint32_t>(__cvta_generic_to_shared(&s_tmem))) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
         if (lane == 0) {
-            for (int i = 0; i < 2; i++) {
+            for (int i = 0; i < NST; i++) {
                 mbar_init(kv_full + 8 * i, C::DQ_WARPS);
                 mbar_init(kv_empty + 8 * i, 1);
+            }
+            for (int i = 0; i < 2; i++) {
                 mbar_init(s_full + 8 * i, 1);
                 mbar_init(s_free + 8 * i, 4);
                 mbar_init(p_full + 8 * i, 4);
@@ -237,33 +261,29 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
         s_abort = 0;
         s_bad_pos = s_nan_pos = INT_MAX;
     }
-    // ---- tables: an entry (the fp16 centroids of two adjacent codes) 32 times, bank = lane
-    {
-        auto build = [&](int off, int bits, const Codebook& cb) {
-            uint32_t* t = reinterpret_cast<uint32_t*>(smem + off);
-            const float lev = cb.v[lane & 15];
-            for (int e = warp; e < (1 << (2 * bits)); e += C::THREADS / 32) {
-                const __half2 h = __floats2half2_rn(__shfl_sync(0xffffffffu, lev, e & ((1 << bits) - 1)),
-                                                    __shfl_sync(0xffffffffu, lev, e >> bits));
-                t[e * 32 + lane] = *reinterpret_cast<const uint32_t*>(&h);
-            }
-        };
-        build(C::OFF_TK, BK, p.lk);
-        build(C::OFF_TV, BV, p.lv);
-    }
-    // ---- queries: rotated, scaled, fp16, K-major with 128-byte swizzle; an octet per row
-    for (int r4 = warp * 4; r4 < n_slots * 128; r4 += C::THREADS / 8) {
-        const int r = r4 + (lane >> 3), t8 = lane & 7, gr = row0 + r;
-        const bool valid = gr < rows;
-        const int i = valid ? gr / group : 0, h = valid ? gr - i * group : 0;
+    // ---- queries: rotated, scaled, fp16, K-major with 128-byte swizzle; an octet per row, all rows' loads first
+    constexpr int PER = C::THREADS / 8, ROUNDS = (SLOTS * 128 + PER - 1) / PER;
+    uint4 raw_q[ROUNDS][E / 8];
+#pragma unroll
+    for (int j = 0; j < ROUNDS; j++) {
+        const int gr = row0 + j * PER + (tid >> 3);
+        const int i = gr < row_end ? gr / group : 0, h = gr < row_end ? gr - i * group : 0;
         const int64_t qoff = ((static_cast<int64_t>(b) * p.q_len + i) * p.Hq + hkv * group + h) * D;
+#pragma unroll
+        for (int k = 0; k < E / 8; k++)
+            raw_q[j][k] = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.q) + qoff + 8 * ((lane & 7) + 8 * k));
+    }
+#pragma unroll
+    for (int j = 0; j < ROUNDS; j++) {
+        const int r = j * PER + (tid >> 3), t8 = lane & 7;
+        if (j * PER + 4 * warp >= n_slots * 128) continue;   // (warp-uniform)
+        const bool valid = row0 + r < rows;
         float a[E];
 #pragma unroll
         for (int k = 0; k < E / 8; k++) {
             float tmp[8];
-            const int64_t eo = qoff + 8 * (t8 + 8 * k);
-            if (p.q_dtype == kBF16) load8<__nv_bfloat16>(static_cast<const __nv_bfloat16*>(p.q) + eo, tmp);
-            else load8<__half>(static_cast<const __half*>(p.q) + eo, tmp);
+            if (p.q_dtype == kBF16) load8<__nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(&raw_q[j][k]), tmp);
+            else load8<__half>(reinterpret_cast<const __half*>(&raw_q[j][k]), tmp);
 #pragma unroll
             for (int c = 0; c < 8; c++)
                 a[8 * k + c] = __uint_as_float(
@@ -272,16 +292,18 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
         octet_fwht<E>(a, lane);
         const int slot = r >> 7, rr = r & 127;
         uint8_t* dst = smem + C::OFF_Q + slot * C::Q_TILE + rr * 128 + 2 * t8;
+        if (r < n_slots * 128) {
 #pragma unroll
-        for (int k = 0; k < E; k++) {   // coordinate t8 + 8 k: 16-byte chunk k & 7 of 64-coordinate chunk k / 8
-            const __half v = __float2half_rn(valid ? a[k] * p.q_scale : 0.f);
-            *reinterpret_cast<__half*>(dst + (k >> 3) * (128 * 128) + (((k & 7) ^ (rr & 7)) << 4)) = v;
+            for (int k = 0; k < E; k++) {   // coordinate t8 + 8 k: 16-byte chunk k & 7 of 64-coordinate chunk k / 8
+                const __half v = __float2half_rn(valid ? a[k] * p.q_scale : 0.f);
+                *reinterpret_cast<__half*>(dst + (k >> 3) * (128 * 128) + (((k & 7) ^ (rr & 7)) << 4)) = v;
+            }
         }
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
 
     // bounded wait; false: give up (somebody's wait ran out)
     auto wait = [&](uint32_t bar, uint32_t parity) {
@@ -304,8 +326,8 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
             float m_run = -INFINITY, l_run = 0.f;
             bool alive = true;
             for (int it = 0; it < n_tiles; it++) {
-                const int st = it & 1;
-                alive = wait(kv_full + 8 * st, it >> 1) && wait(s_full + 8 * slot, it);
+                const int st = it % NST;
+                alive = wait(kv_full + 8 * st, it / NST) && wait(s_full + 8 * slot, it);
                 if (!__all_sync(0xffffffffu, alive)) break;
                 tc_fence_after();
                 uint32_t sr[KT];
@@ -486,7 +508,7 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
         int id = page_id(0), id_next = page_id(1);
         load(0, id);
         for (int it = 0; it < n_tiles; it++) {
-            const int st = it & 1;
+            const int st = it % NST;
             uint32_t k0[BK], v0[BV];
 #pragma unroll
             for (int i = 0; i < BK; i++) k0[i] = kw[i];
@@ -495,7 +517,7 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
             const float kn0 = kn, vn0 = vn;
             load(it + 1, id_next);
             id_next = page_id(it + 2);
-            bool alive = it < 2 || wait(kv_empty + 8 * st, (it >> 1) - 1);
+            bool alive = it < NST || wait(kv_empty + 8 * st, it / NST - 1);
             if (!__all_sync(0xffffffffu, alive)) break;
             put(sbase + C::OFF_K + st * C::KV_TILE, std::integral_constant<int, BK>{}, k0, tk);
             put(sbase + C::OFF_V + st * C::KV_TILE, std::integral_constant<int, BV>{}, v0, tv);
@@ -520,47 +542,56 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
 #endif
             if (lane == 0) mbar_arrive(kv_full + 8 * st);
         }
-    } else if (lane == 0) {
+    } else {
         // ================= the MMAs
+        const bool one = lane == 0;
         constexpr uint32_t kIdescS = (1u << 4) | (static_cast<uint32_t>(KT / 8) << 17) | (8u << 24);
         constexpr uint32_t kIdescO = (1u << 4) | (1u << 16) | (static_cast<uint32_t>(D / 8) << 17) | (8u << 24);
+        // descriptors: the upper halves are constants, the lower ones a base and a constant
+        constexpr uint32_t kHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+        constexpr uint32_t kLeadK = (16u >> 4) << 16, kLeadV = (static_cast<uint32_t>(KT * 128) >> 4) << 16;
+        const uint32_t q_lo = ((sbase + C::OFF_Q) >> 4) | kLeadK, k_lo = ((sbase + C::OFF_K) >> 4) | kLeadK,
+                       v_lo = ((sbase + C::OFF_V) >> 4) | kLeadV;
         auto pv = [&](int it) {
-            const int st = it & 1;
+            const int st = it % NST;
+            const uint32_t v = v_lo + st * (C::KV_TILE >> 4);
             for (int s = 0; s < n_slots; s++) {
-                if (!wait(p_full + 8 * s, it)) return false;
+                if (!__all_sync(0xffffffffu, wait(p_full + 8 * s, it))) return false;
                 tc_fence_after();
                 const uint32_t tm = tmem + s * C::COLS;
 #pragma unroll
                 for (int ks = 0; ks < KT / 16; ks++)
-                    tc_mma_ts(tm, tm + C::COL_P + 8 * ks,
-                              sw128_desc(sbase + C::OFF_V + st * C::KV_TILE + ks * 2048, KT * 128, 1024),
-                              kIdescO, it > 0 || ks > 0);
-                tc_commit(o_done + 8 * s);
+                    tc_mma_ts(one, tm, tm + C::COL_P + 8 * ks, v + ks * (2048 >> 4), kHi, kIdescO, it > 0 || ks > 0);
+                if (one) tc_commit(o_done + 8 * s);
+                __syncwarp();
             }
-            tc_commit(kv_empty + 8 * st);
+            if (one) tc_commit(kv_empty + 8 * st);
+            __syncwarp();
             return true;
         };
         bool ok = true;
         for (int it = 0; it < n_tiles && ok; it++) {
-            const int st = it & 1;
-            ok = wait(kv_full + 8 * st, it >> 1);
+            const int st = it % NST;
+            const uint32_t k = k_lo + st * (C::KV_TILE >> 4);
+            ok = __all_sync(0xffffffffu, wait(kv_full + 8 * st, it / NST));
             for (int s = 0; s < n_slots && ok; s++) {
-                if (it > 0) ok = wait(s_free + 8 * s, it - 1);
+                if (it > 0) ok = __all_sync(0xffffffffu, wait(s_free + 8 * s, it - 1));
                 if (!ok) break;
                 tc_fence_after();
+                const uint32_t q = q_lo + s * (C::Q_TILE >> 4);
 #pragma unroll
                 for (int kb = 0; kb < D / 16; kb++)
-                    tc_mma_ss(tmem + s * C::COLS + C::COL_S,
-                              sw128_desc(sbase + C::OFF_Q + s * C::Q_TILE + (kb >> 2) * (128 * 128) + (kb & 3) * 32, 16, 1024),
-                              sw128_desc(sbase + C::OFF_K + st * C::KV_TILE + (kb >> 2) * (KT * 128) + (kb & 3) * 32, 16, 1024),
-                              kIdescS, kb > 0);
-                tc_commit(s_full + 8 * s);
+                    tc_mma_ss(one, tmem + s * C::COLS + C::COL_S, q + ((kb >> 2) * (128 * 128) + (kb & 3) * 32) / 16,
+                              k + ((kb >> 2) * (KT * 128) + (kb & 3) * 32) / 16, kHi, kIdescS, kb > 0);
+                if (one) tc_commit(s_full + 8 * s);
+                __syncwarp();
             }
             if (ok && it > 0) ok = pv(it - 1);
         }
         if (ok) ok = pv(n_tiles - 1);
         if (!ok) {   // nothing may be in flight when TMEM is given back
-            tc_commit(drained);
+            if (one) tc_commit(drained);
+            __syncwarp();
             for (int i = 0; i < kDrainSpinLimit && !mbar_try_wait(drained, 0); i++) {}
         }
     }

@@ -17,8 +17,8 @@ static cudaError_t run_chunk(const ChunkAttnParams& p, int B, cudaStream_t strea
     const cudaError_t e = allow_smem<kern>(C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     const int rows = p.q_len * (p.Hq / p.Hkv), tiles = (rows + 128 * C::SLOTS - 1) / (128 * C::SLOTS);
-    kern<<<dim3(p.splits, p.Hkv * tiles, B), C::THREADS, C::SMEM_BYTES, stream>>>(p);
-    return cudaGetLastError();
+    // (the tables are built while the kernel before drains)
+    return launch_dependent(kern, dim3(p.splits, p.Hkv * tiles, B), C::THREADS, C::SMEM_BYTES, stream, p);
 }
 
 // FTQ_ONLY_BITS=<b>: bits_k = bits_v = b only (the wait-expiry test library)

@@ -99,13 +99,14 @@ struct FlowCfg : MmaCfg<D, BK, BV, NH> {
         return (free1 > free0 ? free1 : free0) - base;
     }
     __host__ __device__ static constexpr int need(int halves, int warps, int np, bool sep) {
-        int worst = 0;
-        const int bases[5] = {0, 16, 1024, 2048, 4096};
-        for (int i = 0; i < 5; i++) {
-            const int n = plan(halves, warps, np, sep, bases[i]);
+        // (wherever the dynamic part starts in the first 4 KB: all bases with the same next 128-byte boundary place alike, and
+        // the first of them needs the most)
+        int worst = plan(halves, warps, np, sep, 0);
+        for (int base = 16; base <= 4096; base += 128) {
+            const int n = plan(halves, warps, np, sep, base);
             worst = n > worst ? n : worst;
         }
-        return worst + 128;
+        return worst;
     }
     static constexpr int LIMIT = 226 * 1024;   // (1 KB for the kernel's static shared memory)
     // A CTA per SM, as two halves that share the tables and nothing else: one half's barriers and folds overlap with the

@@ -34,15 +34,21 @@
 // CLUSTER: few units with short contexts.  A cluster of CTAs has one unit, each half a part of its pages; the parts' (O,
 // m, l) stay in shared memory, and after a cluster barrier a warp per head merges them from there.
 //
-// Every wait is bounded (mbar_wait, the epoch); a wait that runs out turns the unit's rows into NaN
-// and sets a bit of the status word.  Block ids outside [0, num_blocks) are never dereferenced.
+// Every wait is bounded and run by whole warps (mbar_wait, the epoch); one that runs out turns the rows of the units that it
+// was for into NaN and sets a bit of the status word.  Block ids outside [0, num_blocks) are never dereferenced.
 #pragma once
 
 #include "ftq_attn_mma.cuh"
 
 namespace ftq {
 
+#ifdef FTQ_TEST_WAIT_EXPIRY
+constexpr int kEpochSpinLimit = 1 << 8;
+// Set by a test of the give-up path: CTA 0 does not publish its epoch (and every page copy is issued).
+__device__ int test_withhold_epoch = 0;
+#else
 constexpr int kEpochSpinLimit = 1 << 22;
+#endif
 
 // A piece of a CTA's share: pages [page0, page0 + n_pages) of one unit (n_pages = 0: none left).
 struct FlowPiece {
@@ -321,29 +327,37 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         if (lane == 0) prefix[0] = 0;
     }
     __syncthreads();
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+#ifdef FTQ_TEST_WAIT_EXPIRY
+    const bool publish = test_withhold_epoch == 0;
+#else
+    constexpr bool publish = true;
+#endif
+    if (blockIdx.x == 0 && threadIdx.x == 0 && publish) {
         __threadfence();
         asm volatile("st.release.gpu.global.u64 [%0], %1;\n" ::"l"(epoch_word), "l"(p.epoch) : "memory");
     }
-    bool stalled = false; // a wait of this warp ran out: no more waiting, its results become NaN
-    bool epoch_seen = false;
-    // the counters and the status word are valid once CTA 0 has published this launch's epoch (by the
-    // time anybody asks it has normally been there for long)
+    bool stalled = false;   // a wait for a page ran out: no more waiting, the warp's results become NaN
+    // The counters and the status word are valid once CTA 0 has published this launch's epoch (by the time anybody asks it
+    // has normally been there for long).  Run by a whole warp: its lane 0 asks, and all its lanes learn what came of it.
     auto await_epoch = [&]() {
-        if (epoch_seen) return;
-        epoch_seen = true;
-        for (int i = 0; i < kEpochSpinLimit; i++) {
-            unsigned long long v;
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(epoch_word) : "memory");
-            if (v == p.epoch) return;
-            __nanosleep(100);
-        }
-        stalled = true;
+        bool seen = false;
+        if (lane == 0)
+            for (int i = 0; i < kEpochSpinLimit && !seen; i++) {
+                unsigned long long v;
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(epoch_word) : "memory");
+                seen = v == p.epoch;
+                if (!seen) __nanosleep(100);
+            }
+        return __any_sync(0xffffffffu, seen) != 0;
     };
+    // a half with pieces asks once, by its first warp, before them
+    __shared__ bool s_epochs_lost[C::HALVES];
+    bool& s_epoch_lost = s_epochs_lost[half];
 
-    // a CTA has left (run by one warp)
-    auto leave = [&]() {
-        await_epoch();
+    // a CTA has left (run by one warp; `asked`: its half has)
+    auto leave = [&](bool asked) {
+        const bool lost = asked ? s_epoch_lost : !await_epoch();
+        if (lane == 0 && lost) atomicOr(p.work_counter + kStatusWord, kStatusWaitExpired);
         if (lane == 0 && atomicAdd(p.work_counter + 1, 1) == static_cast<int>(gridDim.x) - 1) {
             __threadfence();
             asm volatile("st.release.gpu.global.u64 [%0], %1;\n" ::"l"(epoch_word), "l"(0ull) : "memory");
@@ -421,7 +435,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     uint32_t phase = 0;   // bit r = parity the next wait on ring buffer r expects
     int ring_it = 0;      // stages this warp has taken from its ring so far (buffer = ring_it % RING)
 #ifdef FTQ_TEST_WAIT_EXPIRY
-    bool test_drop = blockIdx.x == 0 && half == 0 && warp == 5;
+    bool test_drop = blockIdx.x == 0 && half == 0 && warp == 5 && publish;
 #endif
     // stages of a piece that are this warp's: warp, warp + WARPS, ...
     auto my_stages = [&](const FlowPiece& it) {
@@ -833,8 +847,9 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         if (tid < 2) {
             const FlowPiece& it = s_cut[tid];
             int n = 0;
-            if (it.n_pages > 0) {
-                await_epoch();
+            if (it.n_pages > 0 && s_epoch_lost) {
+                n = -1;   // (not counted: nobody else becomes the last one)
+            } else if (it.n_pages > 0) {
                 // (release: the rows that the half wrote before the barrier; acquire: those of the others)
                 const uint32_t old = atom_add_acq_rel(p.unit_counter + (static_cast<int64_t>(it.layer) * p.B + it.b) * p.Hkv + it.hkv, 1);
                 const int parts = static_cast<int>((it.unit_start + C::PIECE + it.unit_pages - 1) / share - (it.unit_start + C::PIECE) / share) + 1;
@@ -843,7 +858,17 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             s_parts[tid] = n;
         }
         sync_half();
-        const int n0 = s_parts[0], n1 = s_parts[1], heads0 = n0 ? group : 0, heads = heads0 + (n1 ? group : 0);
+#pragma unroll 1
+        for (int cut = 0; cut < 2; cut++) {
+            if (s_parts[cut] >= 0) continue;
+            const int64_t at = head_row(s_cut[cut]) * D;
+#pragma unroll 1
+            for (int i = tid; i < group * D; i += THREADS) {
+                if (p.out_dtype == kF32) static_cast<float*>(p.out)[at + i] = __int_as_float(0x7fc00000);
+                else static_cast<uint16_t*>(p.out)[at + i] = 0x7fff;   // (a NaN in fp16 and in bf16)
+            }
+        }
+        const int n0 = max(s_parts[0], 0), n1 = max(s_parts[1], 0), heads0 = n0 ? group : 0, heads = heads0 + (n1 ? group : 0);
         if (heads == 0) return;
         // octets a head: all heads of both units at the same time (the same S when this half has only one to merge: who
         // merges must not change the order of the sums)
@@ -885,7 +910,10 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         primed = true;
         rotate_queries(s_piece[0], FIN0);
         if (tid == 0) s_piece[1] = locate(s_piece[0].next);
-        if (!CLUSTER && tid < 2) await_epoch();   // (while the first pages are on their way)
+        if (!CLUSTER && warp == 0) {   // (while the first pages are on their way)
+            const bool seen = await_epoch();
+            if (lane == 0) s_epoch_lost = !seen;
+        }
     }
     while (s_piece[slot].n_pages > 0) {
         const FlowPiece& cur = s_piece[slot];
@@ -1064,10 +1092,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
                     }
                 }
             }
-            if (bad && tid == 0) {
-                await_epoch();
-                atomicOr(p.work_counter + kStatusWord, kStatusBadBlock);
-            }
+            if (!CLUSTER && bad && tid == 0) atomicOr(p.work_counter + kStatusWord, kStatusBadBlock);
         }
         if (s_piece[slot1].n_pages > 0) rotate_queries(s_piece[slot1], NRED < WARPS ? NRED : 0);
         if (tid == THREADS - 1) {
@@ -1086,9 +1111,9 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             folded[tid * ROW + D] = -INFINITY;
             folded[tid * ROW + D + 1] = 0.f;
         }
-        if (stalled) {
+        if (stalled || (warp == 0 && s_bad[0])) {
             await_epoch();
-            if (lane == 0) atomicOr(p.work_counter + kStatusWord, kStatusWaitExpired);
+            if (lane == 0) atomicOr(p.work_counter + kStatusWord, (stalled ? kStatusWaitExpired : 0) | (s_bad[0] ? kStatusBadBlock : 0));
         }
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
         const int all = static_cast<int>(threadIdx.x) / 32;      // warp of the CTA
@@ -1106,7 +1131,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
                        [](uint32_t r, int at) { return ld_cluster4(r + at * 4); });
         }
         // the last CTA takes the epoch out, see below; nobody leaves while its rows are being read
-        if (threadIdx.x / 32 == C::HALVES * WARPS - 1) leave();
+        if (threadIdx.x / 32 == C::HALVES * WARPS - 1) leave(false);
         asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
         return;
     }
@@ -1116,14 +1141,11 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     }
     sync_half();
     merge_units();
-    if (stalled) {
-        await_epoch();
-        if (lane == 0) atomicOr(p.work_counter + kStatusWord, kStatusWaitExpired);
-    }
+    if (lane == 0 && (stalled || (any && warp == 0 && s_epoch_lost))) atomicOr(p.work_counter + kStatusWord, kStatusWaitExpired);
     // the last CTA to leave takes the epoch out of the workspace: a replay of this very launch (a
     // captured graph) must not find its own epoch there before CTA 0 has cleared the counters
     __syncthreads();
-    if (threadIdx.x < 32) leave();
+    if (threadIdx.x < 32) leave(any);
 }
 
 }  // namespace ftq

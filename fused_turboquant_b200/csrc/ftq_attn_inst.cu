@@ -56,6 +56,12 @@ cudaError_t FTQ_CAT(launch_attn_split_d, FTQ_D)(int bits_k, int bits_v, bool pag
                  : by_bk<false>(bits_k, bits_v, p, n_lb, stream);
 }
 
+#if defined(FTQ_TEST_WAIT_EXPIRY)
+extern "C" int ftq_test_withhold_epoch(int on) {   // (see ftq_attn_flow.cuh)
+    return static_cast<int>(cudaMemcpyToSymbol(test_withhold_epoch, &on, sizeof(on)));
+}
+#endif
+
 template <int BK, int BV, bool SHARED, int NH>
 static cudaError_t run_flow(const AttnParams& p_in, cudaStream_t stream) {
     using C = FlowCfg<FTQ_D, BK, BV, NH>;

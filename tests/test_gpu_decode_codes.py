@@ -110,3 +110,49 @@ def test_an_expired_wait_of_equal_shares(G):
     again, rc, status = run(_lib.load())
     assert (rc, status) == (0, 0)
     np.testing.assert_array_equal(again, good)
+
+
+@pytest.mark.parametrize("G", [4, 8])
+@pytest.mark.parametrize("n_seq", [3, 80])      # clusters, equal shares
+def test_an_epoch_that_nobody_sees(G, n_seq):
+    """CTA 0 does not publish its epoch (in the test library): nobody may use the counters of the cut units, which come back
+    as NaN; units that one half or one cluster has finished need none and are as ever."""
+    from test_gpu_wait_expiry import _test_lib
+
+    from fused_turboquant_b200 import _lib
+    d, Hkv, lens = 128, 2, [4096 - 1000 * (i % 3) for i in range(n_seq)]
+    pool, bt, *_ = _filled_pool(d, 4, 4, Hkv, lens)
+    q = torch.randn(n_seq, Hkv * G, d, generator=torch.Generator("cpu").manual_seed(9)).bfloat16().cuda()
+    sl, table = torch.tensor(lens, dtype=torch.int32).cuda(), torch.from_numpy(bt).cuda()
+    ws = torch.empty(pool.workspace_bytes(n_seq, Hkv * G, 4096, 1), dtype=torch.uint8, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+
+    def run(lib):
+        out = torch.full(q.shape, 7.0, dtype=torch.float32, device="cuda")
+        rc = lib.ftq_paged_decode_attn(
+            p(q), _lib.BF16, p(out), _lib.F32, p(pool.pool[0]), pool.num_blocks, pool.layer_stride, 1, p(table),
+            table.shape[1], p(sl), 4096, n_seq, Hkv * G, Hkv, d, 4, 4, _lib.fptr(pool.levels_k),
+            _lib.fptr(pool.levels_v), _lib.fptr(pool.signs), d ** -0.5, p(ws), ws.numel(), stream)
+        assert rc == 0, lib.ftq_last_error()
+        status = ctypes.c_int(-1)
+        rc = lib.ftq_paged_decode_status(p(ws), n_seq, Hkv * G, Hkv, d, 4096, 1, stream, ctypes.byref(status))
+        return out.cpu().numpy().reshape(n_seq, Hkv, G, d), rc, status.value
+
+    good, rc, status = run(_lib.load())
+    assert (rc, status) == (0, 0) and np.isfinite(good).all()
+    lib = _test_lib()
+    assert lib.ftq_test_withhold_epoch(1) == 0
+    try:
+        got, rc, status = run(lib)
+    finally:
+        assert lib.ftq_test_withhold_epoch(0) == 0
+    assert (rc, status) == (-5, 2)
+    poisoned = np.isnan(got).any(axis=(2, 3))
+    assert np.isnan(got[poisoned]).all()
+    np.testing.assert_array_equal(got[~poisoned], good[~poisoned])
+    # (160 units of up to 284 places on 296 halves: shares are shorter than most units)
+    assert poisoned.sum() > poisoned.size // 2 if n_seq == 80 else not poisoned.any()
+    again, rc, status = run(_lib.load())
+    assert (rc, status) == (0, 0)
+    np.testing.assert_array_equal(again, good)

@@ -448,21 +448,22 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
         // the pool stores a V row with its halves exchanged for tokens with bit 1 set
         const int k_off = tok * C::PDK + gq * 4 * BK;
         const int v_off = C::OFF_VC + tok * C::PDV + (gq ^ ((tok & 2) ? C::NG / 2 : 0)) * 4 * BV;
+        // (ordinary loads: the kernel before this one may have written what they read, see load8)
         auto page_id = [&](int it) {
             const int pg = ((tile0 + it) * KT + t) / kPageTokens;
-            return it < n_tiles && pg < n_pages ? __ldg(btab + pg) : -1;
+            return it < n_tiles && pg < n_pages ? btab[pg] : -1;
         };
         auto words = [&](const uint8_t* src, auto bits, uint32_t* w) {
             constexpr int NB = decltype(bits)::value;
             if constexpr (NB == 4) {
-                const uint4 x = __ldg(reinterpret_cast<const uint4*>(src));
+                const uint4 x = *reinterpret_cast<const uint4*>(src);
                 w[0] = x.x; w[1] = x.y; w[2] = x.z; w[3] = x.w;
             } else if constexpr (NB == 2) {
-                const uint2 x = __ldg(reinterpret_cast<const uint2*>(src));
+                const uint2 x = *reinterpret_cast<const uint2*>(src);
                 w[0] = x.x; w[1] = x.y;
             } else {
 #pragma unroll
-                for (int i = 0; i < NB; i++) w[i] = __ldg(reinterpret_cast<const uint32_t*>(src) + i);
+                for (int i = 0; i < NB; i++) w[i] = reinterpret_cast<const uint32_t*>(src)[i];
             }
         };
         uint32_t kw[BK], vw[BV];
@@ -483,8 +484,8 @@ attn_chunk_kernel(const __grid_constant__ ChunkAttnParams p) {
             words(page + k_off, std::integral_constant<int, BK>{}, kw);
             words(page + v_off, std::integral_constant<int, BV>{}, vw);
             if (gq == 0) {
-                kn = __half2float(__ldg(reinterpret_cast<const __half*>(page + C::OFF_KN) + tok));
-                vn = __half2float(__ldg(reinterpret_cast<const __half*>(page + C::OFF_VN) + tok));
+                kn = __half2float(reinterpret_cast<const __half*>(page + C::OFF_KN)[tok]);
+                vn = __half2float(reinterpret_cast<const __half*>(page + C::OFF_VN)[tok]);
             }
         };
         const uint32_t tk = sbase + C::OFF_TK + lane * 4, tv = sbase + C::OFF_TV + lane * 4;

@@ -59,3 +59,13 @@ def test_outputs_appear_complete(outputs):
     """Nothing is written under an output's own name: a process that has it loaded keeps its file."""
     build.build(force=True)
     assert not set(outputs) & {build.LIB_PATH, build.TEST_LIB_PATH, build.NATIVE_PATH}
+
+
+@pytest.mark.parametrize("name", sorted(n for n in os.listdir(build.CSRC) if n.endswith(".cuh")))
+def test_kernels_launched_early_do_not_load_through_the_read_only_path(name):
+    """A kernel that waits for the one before it lives while that one writes: what it reads may not go through the cache
+    that is not kept coherent (ftq_common.cuh: load8)."""
+    with open(os.path.join(build.CSRC, name)) as f:
+        code = "\n".join(line.split("//")[0] for line in f)
+    if name != "ftq_common.cuh" and "after_previous_kernel()" in code:
+        assert "__ldg" not in code and "ld.global.nc" not in code

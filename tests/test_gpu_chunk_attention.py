@@ -148,3 +148,30 @@ def test_contexts_of_different_lengths(d, hkv, group, lens):
     assert (got[dead] == 0).all()
     err = (got.float() - ref).norm(dim=-1) / ref.norm(dim=-1).clamp_min(1e-6)
     assert err[~dead].max().item() < 5e-3     # (as in test_matches_fp32_decode)
+
+
+@pytest.mark.parametrize("d,bits,lens", [(128, 4, [64, 300]), (64, 3, [1500]), (256, 2, [40] * 4)])
+def test_reads_what_the_store_before_it_has_just_written(d, bits, lens):
+    """The same pages stored anew and attended, time after time without a pause (the kernel is launched while the store
+    drains), against the same calls one at a time."""
+    pool, table, sl, gen = _pool(d, bits, bits, 2, lens, 13)
+    q_len, n = 8, sum(lens)
+    q = torch.randn(len(lens), q_len, 8, d, device="cuda", generator=gen).half()
+    pos = torch.cat([torch.arange(k, device="cuda") for k in lens])
+    row = torch.repeat_interleave(torch.arange(len(lens), device="cuda"), sl.long())
+    slots = table[row, pos // 16].long() * 16 + pos % 16
+    kv = torch.randn(30, 2, n, 2, d, device="cuda", generator=gen).half()
+
+    def run(pause):
+        out = []
+        for key, value in kv:
+            pool.store(key, value, slots, layer=1)
+            pause()
+            out.append(pool.continuation_attention(q, table, sl, max(lens), layer=1))
+            pause()
+        return torch.stack(out)
+
+    want = run(torch.cuda.synchronize)
+    assert torch.isfinite(want).all() and not torch.equal(want[0], want[1])
+    for _ in range(10):
+        assert torch.equal(run(lambda: None), want)

@@ -1018,11 +1018,11 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 8);
             l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 16);
         }
-        // a warp whose copy never arrived poisons its state (NaN propagates to the output)
-        if (stalled) {
+        // A warp whose copy never arrived poisons its state (NaN propagates to the output), and so does a score that is not
+        // a number: it is in the sum of the weights, but no maximum knows it, and a warp without any other looks empty.
 #pragma unroll
-            for (int i = 0; i < HL; i++) m_run[i] = __int_as_float(0x7fc00000);
-        }
+        for (int i = 0; i < HL; i++)
+            if (stalled || l_run[i] != l_run[i]) m_run[i] = __int_as_float(0x7fc00000);
         sync_half();  // A: every warp is done with the ring, the queries and `folded`
 #pragma unroll
         for (int mt = 0; mt < NO; mt++)

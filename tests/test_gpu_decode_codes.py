@@ -156,3 +156,25 @@ def test_an_epoch_that_nobody_sees(G, n_seq):
     again, rc, status = run(_lib.load())
     assert (rc, status) == (0, 0)
     np.testing.assert_array_equal(again, good)
+
+
+@pytest.mark.parametrize("times", [1, 40])      # clusters, equal shares
+@pytest.mark.parametrize("d,bk,bv,G", [(128, 4, 4, 4), (128, 3, 3, 8), (64, 2, 3, 7), (256, 4, 2, 2)])
+@pytest.mark.parametrize("pages", ["first", "last", "all"])
+def test_keys_that_are_not_numbers(times, d, bk, bv, G, pages):
+    """Pages of nothing but NaN key norms are not taken for pages without tokens: the (sequence, KV head) they belong to is
+    NaN, the others are as before."""
+    lens = [1, 16, 17, 40, 200, 700] * times
+    pool, bt, *_ = _filled_pool(d, bk, bv, 2, lens)
+    q = torch.randn(len(lens), 2 * G, d, generator=torch.Generator("cpu").manual_seed(5)).bfloat16().cuda()
+    good = _decode(pool, bt, lens, q).reshape(len(lens), 2, G, d)
+    for b in range(0, len(lens), 2):
+        last = (lens[b] + 15) // 16
+        for page in {"first": [0], "last": [last - 1], "all": range(last)}[pages]:
+            norms = pool.pool[0, int(bt[b, page]), 1, 2 * d * bk:2 * d * bk + 32]
+            norms.copy_(torch.full((16,), float("nan"), dtype=torch.float16).view(torch.uint8))
+    got = _decode(pool, bt, lens, q).reshape(good.shape)
+    assert np.isnan(got[::2, 1]).all()
+    np.testing.assert_array_equal(got[:, 0], good[:, 0])
+    np.testing.assert_array_equal(got[1::2], good[1::2])
+    assert pool.decode_status() == 0

@@ -490,7 +490,8 @@ attn_split_kernel(const AttnParams p) {
                 *reinterpret_cast<u64*>(wacc + (warp * GH + h) * D + t * E + 2 * i) = acc[h][i];
         }
         if (t < GH) {   // (the lanes with the heads' first copies)
-            wm[warp * GH + my_head] = m_run;
+            // (a score that is not a number is in the sum of the weights, but no maximum knows it)
+            wm[warp * GH + my_head] = l_run != l_run ? l_run : m_run;
             wl[warp * GH + my_head] = l_run;
         }
     }
@@ -512,10 +513,8 @@ attn_split_kernel(const AttnParams p) {
         }
         prow[h * prow_head_stride + d] = a;
         if (d == 0) {
-            if (bad_block) {
-                M = __int_as_float(0x7fc00000);
-                if (h == 0 && p.work_counter) atomicOr(p.work_counter + kStatusWord, kStatusBadBlock);
-            }
+            if (bad_block && h == 0 && p.work_counter) atomicOr(p.work_counter + kStatusWord, kStatusBadBlock);
+            if (bad_block || l != l) M = __int_as_float(0x7fc00000);
             prow[h * prow_head_stride + D] = M;
             prow[h * prow_head_stride + D + 1] = l;
         }

@@ -178,3 +178,37 @@ def test_keys_that_are_not_numbers(times, d, bk, bv, G, pages):
     np.testing.assert_array_equal(got[:, 0], good[:, 0])
     np.testing.assert_array_equal(got[1::2], good[1::2])
     assert pool.decode_status() == 0
+
+
+@pytest.mark.parametrize("d,bk,bv,G", [(128, 4, 4, 4), (64, 2, 3, 12), (256, 4, 2, 1)])
+@pytest.mark.parametrize("S", [1, 16, 40, 700])
+@pytest.mark.parametrize("where", ["first page", "all"])
+def test_keys_that_are_not_numbers_fp32(d, bk, bv, G, S, where):
+    """The same for the fp32 kernel, from contiguous tensors and from the pool: one (sequence, KV head) is NaN."""
+    from fused_turboquant_b200 import TurboQuantMSE, kernels
+    g = torch.Generator("cuda").manual_seed(S)
+    x = torch.randn(2, 2, 2, S, d, device="cuda", generator=g)
+    tk, tv = TurboQuantMSE(d, bits=bk, device="cuda"), TurboQuantMSE(d, bits=bv, device="cuda")
+    k, v = tk.encode(x[0]), tv.encode(x[1])
+    q = torch.randn(2, 2 * G, 1, d, device="cuda", generator=g)
+    n = min(16, S) if where == "first page" else S
+
+    def flash():
+        return kernels.flash_decode_compressed(
+            q, k.indices, k.norms, v.indices, v.norms, tk.quantizer.levels, tv.quantizer.levels, tk.rotation.signs,
+            d ** -0.5, bk, bv).reshape(2, 2, G, d)
+    good = flash()
+    k.norms[1, 0, :n] = float("nan")
+    got = flash()
+    assert torch.isnan(got[1, 0]).all()
+    assert torch.equal(got[0], good[0]) and torch.equal(got[1, 1], good[1, 1])
+
+    pool, bt, *_ = _filled_pool(d, bk, bv, 2, [S, S])
+    good = _decode(pool, bt, [S, S], q[:, :, 0]).reshape(2, 2, G, d)
+    for page in range((n + 15) // 16):
+        norms = pool.pool[0, int(bt[1, page]), 0, 2 * d * bk:2 * d * bk + 32]
+        norms.copy_(torch.full((16,), float("nan"), dtype=torch.float16).view(torch.uint8))
+    got = _decode(pool, bt, [S, S], q[:, :, 0]).reshape(2, 2, G, d)
+    assert np.isnan(got[1, 0]).all() and pool.decode_status() == 0
+    np.testing.assert_array_equal(got[0], good[0])
+    np.testing.assert_array_equal(got[1, 1], good[1, 1])

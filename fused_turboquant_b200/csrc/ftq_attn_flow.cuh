@@ -15,7 +15,7 @@
 // costs on its own (rotate the queries, fold the warps' states, the first pages' latency).  Without it the CTAs whose
 // shares held many short sequences were the last by far: 40 sequences log-uniform up to 4000 tokens, 32 / 8 heads of 128,
 // K3V3, 59 -> 25 us; 100 up to 1000, 64 / 8 heads, K4V4, 85 -> 33.  (20 to 40 places measure alike, 8 and 60 up to half as
-// much again.)  The partition needs the prefix sums of the places, which every CTA computes from seq_lens at its start.
+// much again.)  Batches of short units are not cut at all (WHOLE below).  The partition needs the prefix sums of the places, which every CTA computes from seq_lens at its start.
 // This kernel took the place of one that streamed pages across work items without CTA-wide barriers, tickets handing
 // out the items: 64 x 8192 tokens of 32 / 8 heads of 128, K4V4, 137 us there and 123 to 132 here, 24 sequences
 // log-uniform up to 30000 tokens 78 and 44, the ragged batch of 256 up to 32768, heads of 256, K4V2, 777 and 739.
@@ -124,6 +124,11 @@ struct FlowCfg : MmaCfg<D, BK, BV, NH> {
     static constexpr int WARPS = CLUSTER ? (D == 256 && NH == 1 ? 12 : 8) : D == 256 ? (NH == 1 ? 6 : 4) : BK == 4 && BV != 3 ? 6 : 8;
     // places of the line that a unit takes beyond one for each page (see above)
     static constexpr int PIECE = 28;
+    // Where the longest unit has no more pages than this, none is cut: it belongs to the half in whose share it starts.  A
+    // half walks them in less time than the merge of a cut unit takes (200 sequences of up to 400 tokens, 32 / 8 heads of
+    // 128, K4V4: 31.5 -> 30.1 us; 60 of 300 17.7 -> 15.8; 224 units of 118 11.2 -> 9.5).  At 48 pages 300 units of 600 tokens, a few
+    // more than there are halves, take 20.3 us in place of 19.2; heads of 256 at 32 pages 344 of 468 30.0 in place of 27.8.
+    static constexpr int WHOLE = D == 256 ? 24 : 32;
     // two pages per stage wherever their rings leave the warp count alone (a cluster's parts are a few pages long)
     static constexpr int NP = !CLUSTER && need(HALVES, WARPS, 2, false) <= LIMIT ? 2 : 1;
     static constexpr int STAGE_BYTES = NP * M::PAGE_BYTES;
@@ -303,13 +308,14 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     // prefix sums of the page counts (lengths beyond the host's bound are cut to it)
     auto tokens_of = [&](int b) { return max(0, min(p.seq_lens[b], p.max_seq)); };
     if (!CLUSTER && threadIdx.x < 32) {
-        int carry = 0;
+        int carry = 0, longest = 0;
         for (int b0 = 0; b0 < p.B; b0 += 128) {
             int x[4];      // (their loads do not wait for one another)
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 const int b = b0 + 32 * k + lane;
                 x[k] = b < p.B ? (tokens_of(b) + kPageTokens - 1) / kPageTokens : 0;
+                longest = max(longest, x[k]);
                 if (x[k] > 0) x[k] += C::PIECE;
             }
 #pragma unroll
@@ -324,7 +330,11 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
                 carry += __shfl_sync(0xffffffffu, x[k], 31);
             }
         }
-        if (lane == 0) prefix[0] = 0;
+        longest = __reduce_max_sync(0xffffffffu, longest);
+        if (lane == 0) {
+            prefix[0] = 0;
+            prefix[kFlowMaxSeqs + 1] = longest;
+        }
     }
     __syncthreads();
 #ifdef FTQ_TEST_WAIT_EXPIRY
@@ -369,6 +379,10 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     const int64_t total = static_cast<int64_t>(per_layer) * p.n_layers;
     int64_t share = (total + ctas - 1) / ctas;
     share = share > p.min_share ? share : p.min_share;
+    const int longest = CLUSTER ? 0 : prefix[kFlowMaxSeqs + 1];
+    const bool whole = !CLUSTER && longest <= C::WHOLE;
+    if (whole && total == static_cast<int64_t>(longest + C::PIECE) * p.n_units)   // (all alike: as many to each)
+        share = static_cast<int64_t>((p.n_units + ctas - 1) / ctas) * (longest + C::PIECE);
     const int64_t first = share * cta;
     const int64_t end = first + share < total ? first + share : total;
     auto locate = [&](int64_t pos) {
@@ -411,13 +425,19 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         it.hkv = r / places;
         const int at = r - it.hkv * places;
         it.unit_start = pos - at;
+        it.first = pos == first;
+        if (whole) {     // this half's if it starts in its share
+            it.n_pages = at == 0 ? it.unit_pages : 0;
+            it.tokens = tokens_of(lo);
+            it.next = pos + (places - at);
+            return it;
+        }
         const int64_t room = end - pos;
         const int to = places - at > room ? at + static_cast<int>(room) : places;
         // (a share that ends among a unit's extra places has none of its pages: 0, and the share's end)
         it.page0 = max(at - C::PIECE, 0);
         it.n_pages = max(to - C::PIECE, 0) - it.page0;
         it.tokens = min(tokens_of(lo) - it.page0 * kPageTokens, it.n_pages * kPageTokens);
-        it.first = pos == first;
         it.next = pos + (to - at);
         return it;
     };
@@ -425,7 +445,10 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     // thread looks for them, between two barriers).
     __shared__ FlowPiece s_pieces[C::HALVES][3];
     FlowPiece* s_piece = s_pieces[half];
-    if (tid == 0) s_piece[0] = locate(CLUSTER ? 0 : first);
+    if (tid == 0) {
+        s_piece[0] = locate(CLUSTER ? 0 : first);
+        if (whole && s_piece[0].n_pages == 0) s_piece[0] = locate(s_piece[0].next);   // (the share starts inside a unit)
+    }
     sync_half();
 
     // ---- pages: block ids and bulk copies

@@ -212,3 +212,59 @@ def test_keys_that_are_not_numbers_fp32(d, bk, bv, G, S, where):
     assert np.isnan(got[1, 0]).all() and pool.decode_status() == 0
     np.testing.assert_array_equal(got[0], good[0])
     np.testing.assert_array_equal(got[1, 1], good[1, 1])
+
+
+def _time_of_calls(pool, bt, lens, q):
+    """Microseconds of a call among twenty in a graph, the least of ten replays."""
+    table, sl = torch.from_numpy(bt).cuda(), torch.tensor(lens, dtype=torch.int32).cuda()
+    out = torch.empty_like(q)
+    ws = torch.empty(pool.workspace_bytes(q.shape[0], q.shape[1], max(lens), 1), dtype=torch.uint8, device="cuda")
+    call = lambda: pool.decode_attention(q, table, sl, max(lens), layer=0, out=out, workspace=ws)
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(20):
+            call()
+    times = []
+    for _ in range(10):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        graph.replay()
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b) * 50)
+    return min(times)
+
+
+def test_many_short_sequences_use_the_whole_device():
+    """Twice the units of a device of 148 SMs, a page each, in equal shares: not much more than one unit per SM in clusters
+    (three times as much where their pages alone sized the grid)."""
+    times = []
+    for n_seq in (140, 280):
+        pool, bt, *_ = _filled_pool(64, 4, 3, 1, [8] * n_seq)
+        times.append(_time_of_calls(pool, bt, [8] * n_seq, torch.randn(n_seq, 4, 64, device="cuda").bfloat16()))
+    assert times[1] < 2 * times[0], times
+
+
+@pytest.mark.parametrize("longest", [24 * 16, 24 * 16 + 1, 32 * 16, 32 * 16 + 1])
+@pytest.mark.parametrize("mix", ["alike", "ragged", "mostly empty"])
+@pytest.mark.parametrize("d,bits,group,n_seq", [(128, 4, 4, 80), (64, 3, 8, 100), (256, 4, 1, 75), (128, 4, 4, 400)])
+def test_short_units_are_not_cut(d, bits, group, n_seq, mix, longest):
+    """150 to 800 units on either side of the lengths (24 pages for heads of 256, else 32) from which units are cut, alike (as many to each half) and ragged (shares
+    that start inside a unit, that hold none, and sequences without tokens), against the fp32 kernel."""
+    r = np.random.default_rng(n_seq)
+    lens = np.full(n_seq, longest) if mix == "alike" else r.integers(1, longest + 1, n_seq)
+    if mix == "mostly empty":
+        lens[r.random(n_seq) < 0.7] = 0
+    lens[n_seq // 2] = longest
+    lens = [int(n) for n in lens]
+    pool, bt, *_ = _filled_pool(d, bits, bits, 2, lens, seed=n_seq)
+    q = torch.randn(n_seq, 2 * group, d, generator=torch.Generator("cpu").manual_seed(3)).bfloat16().cuda()
+    got, ref = _decode(pool, bt, lens, q), _decode(pool, bt, lens, q.float())
+    np.testing.assert_array_equal(got, _decode(pool, bt, lens, q))
+    some = np.array(lens) > 0
+    assert (got[~some] == 0).all()
+    # 16-bit operands: 3e-4 in the middle of a call, the bar is that of test_gpu_stream_plan.py
+    err = np.linalg.norm(got - ref, axis=-1)[some] / np.linalg.norm(ref, axis=-1)[some]
+    assert err.max() < 1e-2

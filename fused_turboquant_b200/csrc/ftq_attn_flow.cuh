@@ -58,6 +58,12 @@ struct FlowPiece {
     bool first;           // the share starts with it
 };
 
+// A half's share: places [first, end) of the line; all shares but the last have `share` places.
+struct FlowShare {
+    int64_t first, end, share;
+    bool whole;           // units are not cut (see FlowCfg::WHOLE): a half has those that start in its share
+};
+
 template <int D, int BK, int BV, int NH, bool CLUSTER = false>
 struct FlowCfg : MmaCfg<D, BK, BV, NH> {
     using M = MmaCfg<D, BK, BV, NH>;
@@ -375,16 +381,30 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     };
 
     // ---- this CTA's share of the pages, and the piece that starts at a given page
-    const int per_layer = CLUSTER ? 1 : prefix[p.B] * p.Hkv;
-    const int64_t total = static_cast<int64_t>(per_layer) * p.n_layers;
-    int64_t share = (total + ctas - 1) / ctas;
-    share = share > p.min_share ? share : p.min_share;
-    const int longest = CLUSTER ? 0 : prefix[kFlowMaxSeqs + 1];
-    const bool whole = !CLUSTER && longest <= C::WHOLE;
-    if (whole && total == static_cast<int64_t>(longest + C::PIECE) * p.n_units)   // (all alike: as many to each)
-        share = static_cast<int64_t>((p.n_units + ctas - 1) / ctas) * (longest + C::PIECE);
-    const int64_t first = share * cta;
-    const int64_t end = first + share < total ? first + share : total;
+    // (in shared memory: two threads of a half use it between pieces, and the page loop needs the registers)
+    __shared__ FlowShare s_shares[C::HALVES];
+    FlowShare& mine = s_shares[half];
+    if (!CLUSTER && tid == 0) {
+        const int64_t total = static_cast<int64_t>(prefix[p.B] * p.Hkv) * p.n_layers;
+        int64_t share = (total + ctas - 1) / ctas;
+        const int longest = prefix[kFlowMaxSeqs + 1];
+        // (the parts of a unit are walked side by side but merged by one half: the square root is where a few long units
+        // balance the two.  One sequence of 131072 tokens, 4 / 1 heads of 128, K4V4, 38.6 -> 25.0 us, in 171 parts in place of
+        // 293; two ragged ones of 37397, 14 / 2 heads 32.9 -> 22.5; half of it 29.7 and 27.7)
+        constexpr int ROUND = WARPS * NP;      // (a stage of each warp: the share's pages take whole rounds)
+        const int least = max(ROUND, static_cast<int>(0.8f * sqrtf(static_cast<float>(longest))) / ROUND * ROUND);
+        share = share > least ? share : least;
+        mine.whole = longest <= C::WHOLE;
+        // all alike: as many to each, unless that is half as much again (400 units of 100 tokens on 296 halves 15.0 -> 13.9 us,
+        // 302 of 8 12.4 and 13.4)
+        const int each = (p.n_units + ctas - 1) / ctas;
+        if (mine.whole && total == static_cast<int64_t>(longest + C::PIECE) * p.n_units &&
+            (each == 1 || 2 * each * ctas <= 3 * p.n_units))
+            share = static_cast<int64_t>(each) * (longest + C::PIECE);
+        mine.share = share;
+        mine.first = share * cta;
+        mine.end = mine.first + share < total ? mine.first + share : total;
+    }
     auto locate = [&](int64_t pos) {
         FlowPiece it{};
         it.next = pos;
@@ -404,12 +424,13 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             it.next = 1;
             return it;
         }
-        if (pos >= end) return it;
+        if (pos >= mine.end) return it;
         int r;
         if (p.n_layers == 1) {
             it.layer = 0;
             r = static_cast<int>(pos);
         } else {
+            const int per_layer = prefix[p.B] * p.Hkv;
             it.layer = static_cast<int>(pos / per_layer);
             r = static_cast<int>(pos - static_cast<int64_t>(it.layer) * per_layer);
         }
@@ -419,20 +440,28 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             if (prefix[mid] * p.Hkv <= r) lo = mid; else hi = mid;
         }
         it.b = lo;
-        const int places = prefix[lo + 1] - prefix[lo];
-        it.unit_pages = places - C::PIECE;
+        int places = prefix[lo + 1] - prefix[lo];
         r -= prefix[lo] * p.Hkv;
         it.hkv = r / places;
-        const int at = r - it.hkv * places;
-        it.unit_start = pos - at;
-        it.first = pos == first;
-        if (whole) {     // this half's if it starts in its share
-            it.n_pages = at == 0 ? it.unit_pages : 0;
-            it.tokens = tokens_of(lo);
-            it.next = pos + (places - at);
-            return it;
+        int at = r - it.hkv * places;
+        if (mine.whole && at > 0) {   // (a share that starts inside a unit: with the next one, if that is in it)
+            pos += places - at;
+            it.next = pos;
+            if (pos >= mine.end) return it;
+            at = 0;
+            if (++it.hkv == p.Hkv) {
+                it.hkv = 0;
+                do {
+                    if (++lo == p.B) { lo = 0; it.layer++; }
+                    places = prefix[lo + 1] - prefix[lo];
+                } while (places == 0);
+                it.b = lo;
+            }
         }
-        const int64_t room = end - pos;
+        it.unit_pages = places - C::PIECE;
+        it.unit_start = pos - at;
+        it.first = pos == mine.first;
+        const int64_t room = mine.whole ? places : mine.end - pos;
         const int to = places - at > room ? at + static_cast<int>(room) : places;
         // (a share that ends among a unit's extra places has none of its pages: 0, and the share's end)
         it.page0 = max(at - C::PIECE, 0);
@@ -445,10 +474,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     // thread looks for them, between two barriers).
     __shared__ FlowPiece s_pieces[C::HALVES][3];
     FlowPiece* s_piece = s_pieces[half];
-    if (tid == 0) {
-        s_piece[0] = locate(CLUSTER ? 0 : first);
-        if (whole && s_piece[0].n_pages == 0) s_piece[0] = locate(s_piece[0].next);   // (the share starts inside a unit)
-    }
+    if (tid == 0) s_piece[0] = locate(CLUSTER ? 0 : mine.first);
     sync_half();
 
     // ---- pages: block ids and bulk copies
@@ -799,12 +825,13 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         bool nan = false;
 #pragma unroll
         for (int r = 0; r < E; r++) a[r] = 0.f;
-        // two rows of an octet at a time; the first ones are on their way while the maximum is looked for
-        float4 x[2][E / 4];
-        float2 ml[2];
+        // AHEAD rows of an octet at a time; the first ones are on their way while the maximum is looked for
+        constexpr int AHEAD = D == 256 && NH == 1 ? 2 : 4;      // (as many as the registers hold)
+        float4 x[AHEAD][E / 4];
+        float2 ml[AHEAD];
         auto load = [&](int i0) {
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
+            for (int u = 0; u < AHEAD; u++) {
                 const int i = i0 + u * S;
                 ml[u] = make_float2(-INFINITY, 0.f);
                 if (i < n) {
@@ -816,10 +843,15 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             }
         };
         load(sub);
-        for (int i = sub * kOctet + t; i < n; i += S * kOctet) {
-            const float m = load2(row(i), D).x;
-            nan |= m != m;   // (fmaxf drops a NaN operand)
-            M = fmaxf(M, m);
+        for (int i = sub * kOctet + t; i < n; i += 4 * S * kOctet) {
+            float m[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) m[u] = i + u * S * kOctet < n ? load2(row(i + u * S * kOctet), D).x : -INFINITY;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                nan |= m[u] != m[u];   // (fmaxf drops a NaN operand)
+                M = fmaxf(M, m[u]);
+            }
         }
 #pragma unroll
         for (int s = 1; s < 32; s <<= 1) {
@@ -832,7 +864,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         }
         for (int i0 = sub;;) {
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
+            for (int u = 0; u < AHEAD; u++) {
                 if (ml[u].x == -INFINITY) continue;   // (none, or a part without pages: its O is not written)
                 const float f = fast_exp2(ml[u].x - M);
                 L = fmaf(ml[u].y, f, L);
@@ -844,7 +876,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
                     a[4 * c + 3] = fmaf(x[u][c].w, f, a[4 * c + 3]);
                 }
             }
-            i0 += 2 * S;
+            i0 += AHEAD * S;
             if (i0 >= n) break;
             load(i0);
         }
@@ -870,6 +902,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         if (tid < 2) {
             const FlowPiece& it = s_cut[tid];
             int n = 0;
+            const int64_t share = mine.share;
             if (it.n_pages > 0 && s_epoch_lost) {
                 n = -1;   // (not counted: nobody else becomes the last one)
             } else if (it.n_pages > 0) {
@@ -891,20 +924,30 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
                 else static_cast<uint16_t*>(p.out)[at + i] = 0x7fff;   // (a NaN in fp16 and in bf16)
             }
         }
-        const int n0 = max(s_parts[0], 0), n1 = max(s_parts[1], 0), heads0 = n0 ? group : 0, heads = heads0 + (n1 ? group : 0);
-        if (heads == 0) return;
-        // octets a head: all heads of both units at the same time (the same S when this half has only one to merge: who
-        // merges must not change the order of the sums)
-        const int S = 2 * group <= WARPS ? 4 : group <= WARPS ? 2 : 1;
-        const int octet = warp * 4 + (lane >> 3), k = octet / S;
-        const bool second = k >= heads0;
-        const FlowPiece& it = s_cut[second];
-        const int h = k >= heads ? group : second ? k - heads0 : k;
-        const int64_t c0 = (it.unit_start + C::PIECE) / share;
-        merge_head(it, h, k >= heads ? 0 : second ? n1 : n0, S, octet % S,
-                   [&](int i) { return row_of(c0 + i, (c0 + i) * share >= it.unit_start ? 0 : 1) + h * ROW; },
-                   [](const float* r, int at) { return __ldcg(reinterpret_cast<const float2*>(r + at)); },
-                   [](const float* r, int at) { return __ldcg(reinterpret_cast<const float4*>(r + at)); });
+        // Octets a head: from the number of parts alone, not from whether this half has one unit to merge or both, so that who
+        // merges does not change the order of the sums.  Units of few parts together, all heads of both at the same time;
+        // one of many (few long sequences) by itself, its rows over all octets.
+        constexpr int FEW = 8;
+        auto octets = [&](int heads) { return 4 * heads <= 4 * WARPS ? 4 : 2 * heads <= 4 * WARPS ? 2 : 1; };
+        int n0 = max(s_parts[0], 0), n1 = max(s_parts[1], 0);
+        while (n0 + n1 > 0) {
+            const int a0 = n0, a1 = n0 > 0 && max(n0, n1) > FEW ? 0 : n1;
+            const int S = octets(max(a0, a1) > FEW ? group : 2 * group);
+            const int heads0 = a0 ? group : 0, heads = heads0 + (a1 ? group : 0);
+            const int octet = warp * 4 + (lane >> 3), k = octet / S;
+            const bool second = k >= heads0;
+            const FlowPiece& it = s_cut[second];
+            const int h = k >= heads ? group : second ? k - heads0 : k;
+            const int64_t share = mine.share, c0 = (it.unit_start + C::PIECE) / share;
+            merge_head(it, h, k >= heads ? 0 : second ? a1 : a0, S, octet % S,
+                       [&](int i) { return row_of(c0 + i, (c0 + i) * share >= it.unit_start ? 0 : 1) + h * ROW; },
+                       // (ordinary loads, behind the acquire and the barrier: a lane's two halves of 32 bytes are one sector, which
+                       // L1 keeps from one to the other.  2 x 50554 tokens, 16 / 2 heads of 128, K3V4: 39.5 -> 30.7 us)
+                       [](const float* r, int at) { return *reinterpret_cast<const float2*>(r + at); },
+                       [](const float* r, int at) { return *reinterpret_cast<const float4*>(r + at); });
+            n0 = 0;
+            n1 -= a1;
+        }
     };
 
     // sequences without tokens: no CTA meets their units, their outputs are zero (softmax over nothing)

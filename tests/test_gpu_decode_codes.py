@@ -268,3 +268,28 @@ def test_short_units_are_not_cut(d, bits, group, n_seq, mix, longest):
     # 16-bit operands: 3e-4 in the middle of a call, the bar is that of test_gpu_stream_plan.py
     err = np.linalg.norm(got - ref, axis=-1)[some] / np.linalg.norm(ref, axis=-1)[some]
     assert err.max() < 1e-2
+
+
+@pytest.mark.parametrize("d,bits,group", [(128, 4, 8), (128, 3, 5), (64, 4, 7), (64, 2, 1), (256, 4, 8), (256, 3, 3)])
+@pytest.mark.parametrize("n_seq,top", [(1, 40000), (3, 20000), (40, 12000)])
+def test_units_of_many_parts(d, bits, group, n_seq, top):
+    """Few long sequences, cut into more parts than a merge takes up at a time, among sequences of a few parts and of one; two
+    runs of the same call are the same whoever merges what."""
+    lens = [max(1, top // (1 + 7 * (i % 5))) for i in range(n_seq)]
+    pool, bt, *_ = _filled_pool(d, bits, bits, 1, lens, seed=top)
+    q = torch.randn(n_seq, group, d, generator=torch.Generator("cpu").manual_seed(3)).bfloat16().cuda()
+    got, ref = _decode(pool, bt, lens, q), _decode(pool, bt, lens, q.float())
+    for _ in range(5):
+        np.testing.assert_array_equal(got, _decode(pool, bt, lens, q))
+    err = np.linalg.norm(got - ref, axis=-1) / np.linalg.norm(ref, axis=-1)
+    assert err.max() < 1e-2        # (16-bit operands, as above)
+
+
+def test_the_merge_of_many_parts_keeps_up_with_the_heads():
+    """Eight heads of a long sequence against four: the pages are the same, the rows to merge twice as many (1.8 times the time
+    with an octet a head, two rows at a time)."""
+    lens, times = [131072], []
+    pool, bt, *_ = _filled_pool(128, 4, 4, 1, lens)
+    for group in (4, 8):
+        times.append(_time_of_calls(pool, bt, lens, torch.randn(1, group, 128, device="cuda").bfloat16()))
+    assert times[1] < 1.5 * times[0], times

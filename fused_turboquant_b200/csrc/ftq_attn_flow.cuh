@@ -220,10 +220,19 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
     auto xchg = [&](int w) {
         return reinterpret_cast<float4*>(gptr(C::SEP ? xarea + w * C::XSLOT : ring_at[w]));
     };
-    // the half's barrier
+    // the half's barrier, and the cluster's.  (`bar.sync` and `.aligned` want whole warps to arrive together, and lanes that
+    // have parted -- one of them asked for the epoch, some wrote rows -- need not have met again by themselves)
     auto sync_half = [&]() {
-        if constexpr (C::HALVES == 1) __syncthreads();
-        else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + half), "n"(THREADS) : "memory");
+        if constexpr (C::HALVES == 1) {
+            __syncthreads();
+        } else {
+            __syncwarp();
+            asm volatile("bar.sync %0, %1;\n" ::"r"(1 + half), "n"(THREADS) : "memory");
+        }
+    };
+    auto sync_cluster = [&]() {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
     };
 
     // the next kernel of the stream may start its own set-up as soon as every CTA got here
@@ -1027,7 +1036,8 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         for (int k = 0; k < n_mine; k++) {
             const int rb = ring_it % C::RING;
             ring_it++;
-            if (!stalled && !mbar_wait(my_bars + rb * 8, (phase >> rb) & 1u)) stalled = true;
+            // (every lane polls; the vote brings them together again for the MMAs and makes one answer of theirs)
+            if (!stalled) stalled = !__all_sync(0xffffffffu, mbar_wait(my_bars + rb * 8, (phase >> rb) & 1u));
             phase ^= 1u << rb;
             const uint32_t page = my_ring + rb * C::STAGE_BYTES;
             uint32_t kw[C::NP][2][C::KW], v[4][C::VW], pb[C::NP][C::NPB][2];
@@ -1181,7 +1191,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             await_epoch();
             if (lane == 0) atomicOr(p.work_counter + kStatusWord, (stalled ? kStatusWaitExpired : 0) | (s_bad[0] ? kStatusBadBlock : 0));
         }
-        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        sync_cluster();
         const int all = static_cast<int>(threadIdx.x) / 32;      // warp of the CTA
         const int h = static_cast<int>(rank) + all * static_cast<int>(cluster_size);
         if (h < group) {
@@ -1198,7 +1208,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
         }
         // the last CTA takes the epoch out, see below; nobody leaves while its rows are being read
         if (threadIdx.x / 32 == C::HALVES * WARPS - 1) leave(false);
-        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        sync_cluster();
         return;
     }
     sync_half();

@@ -69,3 +69,22 @@ def test_kernels_launched_early_do_not_load_through_the_read_only_path(name):
         code = "\n".join(line.split("//")[0] for line in f)
     if name != "ftq_common.cuh" and "after_previous_kernel()" in code:
         assert "__ldg" not in code and "ld.global.nc" not in code
+
+
+@pytest.mark.parametrize("name", sorted(n for n in os.listdir(build.CSRC) if n.endswith(".cuh")))
+def test_warps_are_whole_before_aligned_barriers(name):
+    """`bar.sync` and `barrier.cluster ... .aligned` are undefined for a warp whose lanes arrive apart, and inline assembly
+    does not bring them together: the statement before is a __syncwarp()."""
+    with open(os.path.join(build.CSRC, name)) as f:
+        code = [line.split("//")[0].strip() for line in f]
+    code = [line for line in code if line]
+    for before, line in zip(code, code[1:]):
+        if "asm volatile(\"bar.sync" in line or ("barrier.cluster" in line and ".aligned" in line):
+            assert before == "__syncwarp();", line
+
+
+def test_a_wait_for_pages_has_one_answer_for_the_warp():
+    """What follows it in the decode kernel (shuffles, MMAs, page requests) is run by all lanes or by none."""
+    with open(os.path.join(build.CSRC, "ftq_attn_flow.cuh")) as f:
+        waits = [line for line in f if "mbar_wait(my_bars" in line]
+    assert waits and all("__all_sync(0xffffffffu, mbar_wait(" in line for line in waits)

@@ -293,3 +293,23 @@ def test_the_merge_of_many_parts_keeps_up_with_the_heads():
     for group in (4, 8):
         times.append(_time_of_calls(pool, bt, lens, torch.randn(1, group, 128, device="cuda").bfloat16()))
     assert times[1] < 1.5 * times[0], times
+
+
+@pytest.mark.parametrize("over", [0, 1])         # clusters up to here, equal shares from one token more on
+@pytest.mark.parametrize("d,group,n_seq,line", [
+    (64, 7, 4, 112 * 8 * 2), (128, 4, 4, 112 * 8 * 2), (64, 4, 13, 72 * 4 * 2), (128, 8, 74, 72 * 2), (256, 2, 4, 112 * 8)])
+def test_the_lines_between_clusters_and_equal_shares(oracle, d, group, n_seq, line, over):
+    """Two KV heads; line = pages of the longest context (pages of a half's part, CTAs, halves), the others far shorter:
+    parts without pages, shares that end among a unit's extra places, halves without pages."""
+    bits = 4
+    lens = [([16, 0, 700, 1, 33, 16 * 28][i % 6]) for i in range(n_seq - 1)] + [line * 16 + over]
+    pool, bt, key, val, _, _ = _filled_pool(d, bits, bits, 2, lens, seed=n_seq)
+    g = torch.Generator("cpu").manual_seed(n_seq + d)
+    q = torch.randn(n_seq, 2 * group, d, generator=g).bfloat16().cuda()
+    got = _decode(pool, bt, lens, q)
+    assert np.isfinite(got).all()
+    np.testing.assert_array_equal(got, _decode(pool, bt, lens, q))
+    for b, n in enumerate(lens):
+        assert n or (got[b] == 0).all()
+    which = [b for b, n in enumerate(lens) if n][-6:]
+    assert _oracle_bad(oracle, pool, key, val, q, np.array(lens), got, d, bits, bits, which) == 0

@@ -622,7 +622,7 @@ int ftq_qk_scores(const float* q_rot, const uint8_t* k_codes, const void* k_norm
 }
 
 // The tail of a decode workspace holds the counters of the tensor-core kernels: a 256-byte header
-// (work-item counter, count of finished CTAs, the 64-bit epoch word) and, from byte 256 on, one
+// (word 1 the count of finished CTAs, words 2 and 3 the 64-bit epoch, word 4 the status) and, from byte 256 on, one
 // counter per (layer, sequence, KV head) unit for the in-kernel split-KV merge.  The kernels clear the
 // tail themselves under a per-launch epoch (see AttnParams), so one call is one node in the stream (one
 // per 1024 sequences in the equal-share kernel) and needs nothing from the call before it.

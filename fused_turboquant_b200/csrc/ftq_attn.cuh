@@ -46,7 +46,9 @@ struct AttnParams {
     int q_dtype;                // kF32 / kF16 / kBF16
     int cp16;                   // contiguous source: every span 16-byte aligned
     int chunk_tokens, n_chunks, n_hpass;
-    float* partials;            // [L*B*Hq][row_chunks][D + 4]
+    // rows (O, m, l): attn_split_kernel [L*B*Hq][n_chunks][D + 4]; attn_flow_kernel [halves of the grid][2][group][D + 4],
+    // the pieces of cut units at the start and the end of each half's share
+    float* partials;
     // Counters of the tensor-core kernel, which clears them itself: CTA 0 zeroes work_counter[1]
     // (CTAs that have left) and the unit counters, then stores `epoch` (unique per call, never 0) into
     // the 64-bit word at work_counter + 2; everybody checks for it before the first atomic on a

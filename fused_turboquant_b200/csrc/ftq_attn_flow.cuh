@@ -15,18 +15,20 @@
 // costs on its own (rotate the queries, fold the warps' states, the first pages' latency).  Without it the CTAs whose
 // shares held many short sequences were the last by far: 40 sequences log-uniform up to 4000 tokens, 32 / 8 heads of 128,
 // K3V3, 59 -> 25 us; 100 up to 1000, 64 / 8 heads, K4V4, 85 -> 33.  (20 to 40 places measure alike, 8 and 60 up to half as
-// much again.)  Batches of short units are not cut at all (WHOLE below).  The partition needs the prefix sums of the places, which every CTA computes from seq_lens at its start.
+// much again.)  Batches of short units are not cut at all (WHOLE below).  The partition needs the prefix sums of the
+// places, which every CTA computes from seq_lens at its start.
 // This kernel took the place of one that streamed pages across work items without CTA-wide barriers, tickets handing
-// out the items: 64 x 8192 tokens of 32 / 8 heads of 128, K4V4, 137 us there and 123 to 132 here, 24 sequences
-// log-uniform up to 30000 tokens 78 and 44, the ragged batch of 256 up to 32768, heads of 256, K4V2, 777 and 739.
+// out the items.  In turn on one device, us there and here: 64 x 8192 tokens of 32 / 8 heads of 128, K4V4, 140 and 135
+// (runs of one side differ by 3 %), 24 sequences log-uniform up to 30000 tokens 64 and 35, 4 x 131072, 64 / 8 heads, K3V3,
+// 159 and 139, the ragged batch of 256 up to 32768, 16 / 8 heads of 256, K4V2, 877 and 781.
 //
 // A piece is walked by the CTA's warps in stages of NP consecutive pages, dealt round-robin.  A
 // warp keeps RING stages in flight (1-D bulk copies, TMA); block ids are read straight from the
 // block table, a batch of 32 per warp, one batch ahead.  The first stages of the next piece are
 // requested before this piece's states are folded.
 //
-// Pieces of a cut unit leave (O, m, l) rows in the workspace (two row blocks per CTA: a CTA's first
-// and last piece can be parts of units).  When its share is done a CTA counts them in; whoever arrives last
+// Pieces of a cut unit leave (O, m, l) rows in the workspace (two row blocks per half: a share's first
+// and last piece can be parts of units).  When its share is done a half counts them in; whoever arrives last
 // merges the rows, rotates back (core/hadamard.py:93-100) and stores.  A unit that one piece covers is
 // finished from shared memory.  Nobody waits for anybody.  The counters are cleared by CTA 0 under
 // the launch's epoch, as described at AttnParams.
@@ -205,7 +207,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
 #pragma unroll
     for (int h = 0; h < C::HALVES; h++) misc_of[h] = take(C::misc_bytes(WARPS));
     const uint32_t misc = half == 0 ? misc_of[0] : misc_of[C::HALVES - 1];
-    int* prefix = reinterpret_cast<int*>(gptr(take(C::PREFIX_BYTES)));   // [B + 1] page counts, summed up
+    int* prefix = reinterpret_cast<int*>(gptr(take(C::PREFIX_BYTES)));   // [B + 1] places, summed up
     float* qs = reinterpret_cast<float*>(gptr(qs_at));                // [4 * NH][D + 16] rotated queries
     float* folded = reinterpret_cast<float*>(gptr(misc));             // [4 * NH][ROW] the piece's (O, m, l)
     float* xml = folded + 4 * NH * ROW;                               // [WARPS][2][4 * NH]
@@ -320,7 +322,7 @@ attn_flow_kernel(const __grid_constant__ AttnParams p) {
             if (p.b0 == 0) p.work_counter[kStatusWord] = 0;   // (the call's: its later launches add to it)
         }
     }
-    // prefix sums of the page counts (lengths beyond the host's bound are cut to it)
+    // prefix sums of the places (lengths beyond the host's bound are cut to it)
     auto tokens_of = [&](int b) { return max(0, min(p.seq_lens[b], p.max_seq)); };
     if (!CLUSTER && threadIdx.x < 32) {
         int carry = 0, longest = 0;
